@@ -125,9 +125,9 @@ def seeds_for(wl, first, S):
 def next_bytes(wl, st, mode):
     """Algorithmic bytes of the next() launches of one sample(), from the device's event counters.
     Walks: per live pair 8 B map-in + 8 B row offsets, per sampled edge 4 B neighbour + 4 B output,
-    8 B map-out per pair of every step but the last (no maps in sample-parallel mode); weighted
+    8 B map-out per pair of every step but the last (transit-parallel mode only: the other two run a lane per walk); weighted
     apps + 4 B max weight per next() and 4 B per weight read; node2vec + previous vertex (4+4 B,
-    kept in a register in sample-parallel mode), 8 B for its row, and per try 4 B candidate + 4 B per
+    kept in a register where a lane keeps its walk), 8 B for its row, and per try 4 B candidate + 4 B per
     word read by the membership test (one 8-id bucket of the previous vertex's neighbour set = 32 B;
     tests the draw decides without are not made and not counted).  k-hop: per pair 8 B map-in + 8 B row offsets, per neighbour 4 B + 4 B,
     8 B map-out per neighbour of every hop but the last.  Collective: 4 B per gathered neighbour id
@@ -138,12 +138,12 @@ def next_bytes(wl, st, mode):
         steps = wl["steps"]
         pairs -= st.get("pairs_not_entered", 0)   # PPR, load-balanced mode: pairs that were never written to or read from a map
         b = 8 * pairs + 8 * edges
-        if mode != 2:
+        if mode == 0:
             b += 8 * pairs + 8 * pairs * (steps - 1) / steps
         if app in (1, 2):
             b += 4 * pairs + 4 * st["weight_tries"]
         if app == 3:
-            b += (16 if mode != 2 else 8) * pairs + 4 * st["n2v_tries"] + 4 * st["n2v_probes"]
+            b += (16 if mode == 0 else 8) * pairs + 4 * st["n2v_tries"] + 4 * st["n2v_probes"]
         return b
     if wl["kind"] == KHOP:
         f = wl["fanout"]
@@ -430,7 +430,7 @@ def roofline_of(nd, smp, wl, workload, mode_name, mode, ms_per_step, hbm_peak, p
     replay_ms = ms_per_step * (next_ms - tail_ms) / phase_sum if phase_sum > 0 and ms_per_step else None
     pairs_per_launch = None
     if wl["kind"] == WALK:      # pairs in the maps the step launches read (the tail launch and its pairs are not among them)
-        pairs_per_launch = (float(smp.live_pairs()[:next_launches].sum()) if mode != 2 else float(st["live_pairs"])) / max(next_launches, 1)
+        pairs_per_launch = (float(smp.live_pairs()[:next_launches].sum()) if mode == 0 else float(st["live_pairs"])) / max(next_launches, 1)
     traffic, traffic_src = ncu_traffic(workload, mode_name, pairs_per_launch)
     gather = None
     if wl["kind"] == WALK and with_gather_probe:

@@ -47,7 +47,7 @@ typedef enum nd_app {
 /* kernelType + load-balancing flag of nextdoor<>() (src/nextdoor.cu:3239-3243, src/main.cu:21-29) */
 typedef enum nd_mode {
   ND_MODE_TRANSIT_PARALLEL = 0,    /* "TransitParallel", -l off: no bins */
-  ND_MODE_TRANSIT_PARALLEL_LB = 1, /* "TransitParallel", -l on: sub-warp / block / grid bins */
+  ND_MODE_TRANSIT_PARALLEL_LB = 1, /* "TransitParallel", -l on: the library chooses how the work is laid out (walks: a lane per walk) */
   ND_MODE_SAMPLE_PARALLEL = 2      /* "SampleParallel" (what the Python sample() runs) */
 } nd_mode;
 
@@ -188,8 +188,8 @@ int nd_sampler_aux(nd_sampler *s, int32_t *adj_row, int32_t *adj_col, float *pro
 int nd_sampler_stats(nd_sampler *s, int64_t *stats, int n);
 /* walks in a transit-parallel mode: live[k] = (transit, sample) pairs that entered step k of the last
  * sample(), i.e. the size of the step's map (the reference prints the same as "totalThreads" per
- * step, src/nextdoor.cu:2400-2410); entries of steps the run did not take step by step are those of
- * an earlier run or zero.  n <= steps. */
+ * step, src/nextdoor.cu:2400-2410).  In the load-balanced mode: the walks that were alive at step k (the
+ * step loop its switches select reports the sizes of its maps).  n <= steps. */
 int nd_sampler_live_pairs(nd_sampler *s, int32_t *live, int n);
 /* per-phase device time of the last sample() when profiling is on: see nd_phase */
 typedef enum nd_phase {

@@ -253,8 +253,7 @@ class Sampler:
                     pairs_not_entered=int(st[7]))
 
     def live_pairs(self):
-        """Walks, transit-parallel modes: pairs in the map of each step of the last sample() (PPR in
-        the load-balanced mode leaves out pairs whose walk is known to stop at that step)."""
+        """Walks, transit-parallel and load-balanced modes: walks alive at each step of the last sample()."""
         live = np.zeros(self.params.steps, np.int32)
         check(lib.nd_sampler_live_pairs(self._h, _ptr(live), live.shape[0]))
         return live

@@ -78,12 +78,12 @@ void free_sampler(nd_sampler *s) {
   nd_hostrows_free(s);
   cudaFree(s->d_initial); cudaFree(s->d_out); cudaFree(s->d_tmp); cudaFree(s->d_len); cudaFree(s->d_plen); cudaFree(s->d_state);
   for (int i = 0; i < 2; i++) { cudaFree(s->d_map_key[i]); cudaFree(s->d_map_val[i]); }
-  cudaFree(s->d_init_key); cudaFree(s->d_init_val); cudaFree(s->d_nlive); cudaFree(s->d_stats); cudaFree(s->d_status);
+  cudaFree(s->d_init_key); cudaFree(s->d_init_val); cudaFree(s->d_nlive); cudaFree(s->d_stats); if (s->h_status) cudaFreeHost(s->h_status);
   cudaFree(s->d_runs); cudaFree(s->d_bin_counts); cudaFree(s->d_hop_counts);
   cudaFree(s->d_adj_row); cudaFree(s->d_adj_col); cudaFree(s->d_prob); cudaFree(s->d_cand); cudaFree(s->d_cand_w); cudaFree(s->d_acc); cudaFree(s->d_bm);
   cudaFree(s->d_cnt); cudaFree(s->d_offs); cudaFree(s->d_bsum); cudaFree(s->d_rank);
   for (int i = 0; i < 2; i++) cudaFree(s->d_srec[i]);
-  cudaFree(s->d_init_rec); cudaFree(s->d_uext);
+  cudaFree(s->d_init_rec); cudaFree(s->d_list); cudaFree(s->d_rows_acc);
   for (int i = 0; i < 3; i++) if (s->graph_exec[i]) cudaGraphExecDestroy(s->graph_exec[i]);
   if (s->copy_event) cudaEventDestroy(s->copy_event);
   if (s->copy_done) cudaEventDestroy(s->copy_done);
@@ -178,9 +178,10 @@ int nd_sampler_create(const nd_graph *g, const nd_app_params *p, int64_t num_sam
   ND_CUDA_S(cudaMalloc(&s->d_initial, sizeof(int32_t) * S1 * s->isz));
   ND_CUDA_S(cudaMalloc(&s->d_out, sizeof(int32_t) * S1 * s->fs));
   ND_CUDA_S(cudaMalloc(&s->d_stats, sizeof(unsigned long long) * 8));
-  ND_CUDA_S(cudaMalloc(&s->d_status, sizeof(int)));
+  ND_CUDA_S(cudaHostAlloc(&s->h_status, sizeof(int), cudaHostAllocMapped));
+  *s->h_status = 0;
+  ND_CUDA_S(cudaHostGetDevicePointer(&s->d_status, s->h_status, 0));
   ND_CUDA_S(cudaMemset(s->d_stats, 0, sizeof(unsigned long long) * 8));
-  ND_CUDA_S(cudaMemset(s->d_status, 0, sizeof(int)));
   if (nd_is_walk(p->app)) ND_TRY_S(nd_walk_alloc(s));
   else if (nd_is_khop(p->app)) ND_TRY_S(nd_khop_alloc(s));
   else ND_TRY_S(nd_collective_alloc(s));
@@ -191,7 +192,7 @@ int nd_sampler_create(const nd_graph *g, const nd_app_params *p, int64_t num_sam
     default_initial_kernel<<<(int)((n + 255) / 256), 256>>>(first_sample, num_samples, s->isz, g->V, s->d_initial);
     ND_CUDA_S(cudaGetLastError());
   }
-  if (!nd_is_collective(p->app)) ND_TRY_S(nd_sampler_build_initial_map(s));
+  if (nd_is_khop(p->app)) ND_TRY_S(nd_sampler_build_initial_map(s));
   ND_CUDA_S(cudaDeviceSynchronize());
 #undef ND_TRY_S
 #undef ND_CUDA_S
@@ -203,7 +204,8 @@ int nd_sampler_set_initial(nd_sampler *s, const int32_t *initial) {
   ND_REQUIRE(s && initial, ND_ERR_ARG, "nd_sampler_set_initial: null argument");
   ND_CUDA(cudaSetDevice(s->g->device));
   ND_CUDA(cudaMemcpyAsync(s->d_initial, initial, sizeof(int32_t) * (size_t)s->S * s->isz, cudaMemcpyHostToDevice, s->stream));
-  if (!nd_is_collective(s->p.app)) ND_TRY(nd_sampler_build_initial_map(s));
+  if (nd_is_khop(s->p.app)) ND_TRY(nd_sampler_build_initial_map(s));
+  s->map_stale = true;
   return ND_OK;
 }
 
@@ -237,10 +239,9 @@ int nd_sampler_sync(nd_sampler *s) {
   ND_REQUIRE(s, ND_ERR_ARG, "null sampler");
   ND_CUDA(cudaSetDevice(s->g->device));
   ND_CUDA(cudaStreamSynchronize(s->stream));
-  int status = 0;
-  ND_CUDA(cudaMemcpy(&status, s->d_status, sizeof(int), cudaMemcpyDeviceToHost));
+  const int status = *(volatile int *)s->h_status;
   if (status != 0) {
-    ND_CUDA(cudaMemset(s->d_status, 0, sizeof(int)));
+    *(volatile int *)s->h_status = 0;
     nd_set_error("device status word 0x%x:%s%s%s%s", status, status & ND_DEV_BAD_TRANSIT ? " transit id out of range" : "",
                  status & ND_DEV_WAIT_TIMEOUT ? " bounded wait gave up" : "", status & ND_DEV_OVERFLOW ? " buffer overflow avoided" : "",
                  status & ND_DEV_RETRY_LIMIT ? " rejection loop hit its cap" : "");
@@ -318,8 +319,25 @@ int nd_sampler_live_pairs(nd_sampler *s, int32_t *live, int n) {
   ND_REQUIRE(nd_is_walk(s->p.app), ND_ERR_ARG, "nd_sampler_live_pairs: walk applications only");
   ND_TRY(nd_sampler_sync(s));
   const int m = n < s->p.steps ? n : s->p.steps;
-  ND_CUDA(cudaMemcpy(live, s->d_nlive, sizeof(int32_t) * (size_t)m, cudaMemcpyDeviceToHost));
   for (int i = m; i < n; i++) live[i] = 0;
+  if (!s->live_is_ended || s->S == 0) {
+    ND_CUDA(cudaMemcpy(live, s->d_nlive, sizeof(int32_t) * (size_t)m, cudaMemcpyDeviceToHost));
+    return ND_OK;
+  }
+  // a lane per walk: ended[k] walks ended after k vertices, at step k; the pairs of all steps together give
+  // the number of walks that entered step 0
+  const int steps = s->p.steps;
+  std::vector<int32_t> ended((size_t)steps);
+  unsigned long long pairs = 0;
+  ND_CUDA(cudaMemcpy(ended.data(), s->d_nlive, sizeof(int32_t) * (size_t)steps, cudaMemcpyDeviceToHost));
+  ND_CUDA(cudaMemcpy(&pairs, s->d_stats + 1, sizeof(pairs), cudaMemcpyDeviceToHost));
+  int64_t missing = 0;
+  for (int k = 0; k < steps; k++) missing += (int64_t)(uint32_t)ended[k] * (steps - 1 - k);
+  int64_t alive = ((int64_t)pairs + missing) / steps;
+  for (int k = 0; k < m; k++) {
+    live[k] = (int32_t)alive;
+    alive -= (uint32_t)ended[k];
+  }
   return ND_OK;
 }
 
@@ -351,8 +369,8 @@ int nd_sampler_next_kernel(const nd_sampler *s, int mode, char *name, int n) {
   const int app = s->p.app;
   if (nd_is_walk(app)) {
     const char *k = mode == ND_MODE_TRANSIT_PARALLEL ? "walk_next_tp_kernel"
-                    : mode == ND_MODE_TRANSIT_PARALLEL_LB ? "walk_next_count_kernel"
-                    : (app == ND_APP_UNIFORM_WALK || getenv("ND_SP_PLAIN")) ? "walk_sp_kernel" : "walk_sp_rounds_kernel";
+                    : mode == ND_MODE_SAMPLE_PARALLEL ? "walk_sp_kernel"
+                    : nd_walk_step_loop(s) ? "walk_next_ticket_kernel" : "walk_next_count_kernel";
     snprintf(name, (size_t)n, "%s<%s>", k, walk_app[app]);
   } else if (nd_is_khop(app)) {
     const char *e = getenv("ND_KHOP_STAGING");

@@ -74,7 +74,12 @@ struct nd_graph {
   // Derived layouts, built on the first sampler that needs them and shared by all samplers of the graph:
   mutable int2 *colw = nullptr;        // [E] (neighbour id, weight bits) records: one 8-byte gather per weighted try
   mutable int2 *vrec = nullptr;        // [V+1] (row start, max weight bits) per vertex: what a thread-per-walk kernel needs of a vertex in one sector
+  mutable int2 *vrow = nullptr;        // [V] (row start, degree): one load per vertex
+  mutable int4 *vrec4 = nullptr;       // [V] (row start, degree, max weight bits, 0)
+  mutable int4 *erec = nullptr;        // [E] (neighbour id, its row start, its degree, 0)
+  mutable uint8_t *wq = nullptr;       // [E] weights as whole 256ths of the row's maximum
   mutable int32_t *adjset = nullptr;   // node2vec membership: per-vertex hash sets of the neighbour ids, 8-slot buckets
+  mutable uint32_t *adjsign = nullptr; // ... and the filter in front of them
 };
 
 struct NdGraphView {
@@ -169,16 +174,21 @@ struct nd_sampler {
   int64_t map_cap = 0;
   int32_t *d_nlive = nullptr;     // [steps+2] live pairs entering each step
   unsigned long long *d_stats = nullptr;  // [8]
-  int *d_status = nullptr;
+  int *h_status = nullptr, *d_status = nullptr;   // status word in mapped host memory: read without a copy once the stream has drained
   NdRadixScratch radix;
   // counting inversion of the walk maps: per-vertex counters, their exclusive scan, chunk sums, ranks
   uint32_t *d_cnt = nullptr, *d_offs = nullptr, *d_bsum = nullptr;
   int32_t *d_rank = nullptr;
-  // load-balanced walk loop: the transit-sorted map as records (8 bytes, node2vec 32 bytes), ping-pong,
-  // the initial map in the same form, and (node2vec) what next() hands to the scatter per pair
+  // step loop of the load-balanced mode: the transit-sorted map as records {transit, sample}, ping-pong, and the initial map in the same form
   void *d_srec[2] = {nullptr, nullptr};
   void *d_init_rec = nullptr;
-  int4 *d_uext = nullptr;
+  bool loop_ready = false;
+  // a lane per walk (nd_walk_rows.cu): walks that can start, counters of the running job
+  int4 *d_list = nullptr;
+  unsigned long long *d_rows_acc = nullptr;
+  bool live_is_ended = false;     // d_nlive holds walks by the number of their vertices (see nd_sampler_live_pairs)
+  bool map_stale = false;         // the initial map does not belong to the seeds (walks: sorted by the first job that needs it)
+  int32_t *d_init_n = nullptr;    // pairs of the initial map (inside d_nlive)
   // the step loop of a walk job captured once per mode and replayed (needs a non-default stream)
   cudaGraphExec_t graph_exec[3] = {nullptr, nullptr, nullptr};
   int graph_launches[3] = {0, 0, 0};
@@ -231,6 +241,8 @@ int nd_walk_step_launch(const nd_graph *g, const nd_app_params *p, int step, int
 int nd_walk_step_status_read(cudaStream_t st, int *status);
 
 int nd_walk_alloc(nd_sampler *s);
+int nd_walk_ensure_tmp(nd_sampler *s);   // d_tmp
+bool nd_walk_step_loop(const nd_sampler *s);   // the load-balanced mode takes the step loop over sorted maps (its switches are set)
 int nd_walk_sample(nd_sampler *s, int mode);
 int nd_khop_alloc(nd_sampler *s);
 int nd_khop_sample(nd_sampler *s, int mode);

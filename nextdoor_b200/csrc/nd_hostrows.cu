@@ -209,6 +209,7 @@ int hostrows_init(nd_sampler *s) {
 // the rows' prefixes packed into the staging array of the walk (free between two passes), on the sampler's stream
 int pack_enqueue(nd_sampler *s) {
   NdHostRows *h = s->hostrows;
+  ND_TRY(nd_walk_ensure_tmp(s));
   pack_sum_kernel<<<h->n_chunks, PACK_THREADS, 0, s->stream>>>(s->d_plen, s->S, h->d_chunk);
   pack_scan_kernel<<<1, 1024, 0, s->stream>>>(h->d_chunk, h->n_chunks);
   pack_rows_kernel<<<h->n_chunks, PACK_THREADS, 0, s->stream>>>(s->d_plen, s->d_out, s->S, s->fs, h->d_chunk, s->d_tmp);
@@ -367,6 +368,7 @@ int nd_sampler_pack_rows(nd_sampler *s, const int32_t **d_row_len, const int32_t
   ND_TRY(hostrows_init(s));
   NdHostRows *h = s->hostrows;
   ND_REQUIRE(h->stage == 0, ND_ERR_STATE, "a host update of this sampler is using the staging array");
+  ND_TRY(nd_walk_ensure_tmp(s));
   *d_row_len = s->d_plen;
   *d_vals = s->d_tmp;
   *h->h_total = 0;

@@ -407,6 +407,7 @@ int nd_khop_alloc(nd_sampler *s) {
   ND_CUDA(cudaMalloc(&s->d_init_key, sizeof(int32_t) * (size_t)(S > 0 ? S : 1)));
   ND_CUDA(cudaMalloc(&s->d_init_val, sizeof(int32_t) * (size_t)(S > 0 ? S : 1)));
   ND_CUDA(cudaMalloc(&s->d_nlive, sizeof(int32_t) * (size_t)(2 * p.steps + 4)));
+  s->d_init_n = s->d_nlive;
   // work items of the block / grid bins: a staged run has >= 1 pair and is cut every 128+ pairs
   s->runs_cap = s->map_cap / 2 + s->map_cap / 128 + 1024;
   ND_CUDA(cudaMalloc(&s->d_runs, sizeof(int2) * (size_t)s->runs_cap));

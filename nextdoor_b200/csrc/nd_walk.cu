@@ -5,20 +5,17 @@
 // identityKernel (src/nextdoor.cu:212-336, 338-504) -- and then inverts the freshly written
 // sample->transit pairs with the in-house radix sort.  The next() kernel already counts the first
 // radix digit of the keys it writes, so the inversion starts at its scan.
-// Sample-parallel path (sampleParallelKernel, src/nextdoor.cu:1348-1518): one thread owns a walk
-// for all its steps and keeps the walk state in registers.
+// The other two modes run a lane per walk (nd_walk_rows.cu); what the transit-parallel path needs beyond
+// that -- maps, sort scratch, staged output -- is made when it is first asked for.
 //
-// Both paths write the walk step-major (tmp[step][sample], 4-byte stores that the L2 merges into
-// full sectors) and a last kernel transposes that into the reference's sample-major layout
+// The transit-parallel kernels write the walk step-major (tmp[step][sample], 4-byte stores that the L2
+// merges into full sectors) and a last kernel transposes that into the reference's sample-major layout
 // finalSamples[sample*steps + step] (src/nextdoor.cu:2041, 293-334) with coalesced row stores.
-// Why no adjacency staging here: a walk draws one neighbour per visit, and at stationarity a
-// transit of degree d is visited by about d * S / E walks per step (1/32 of d on the 2^20-vertex
-// graph), so the visits touch fewer sectors than the list holds; staging pays for k-hop, not for walks.
-#include <mutex>
-
 #include "nd_cache.cuh"
 #include "nd_common.cuh"
+#include "nd_nbrset.cuh"
 #include "nd_philox.cuh"
+#include "nd_walk_rows.cuh"
 
 namespace {
 
@@ -32,27 +29,8 @@ struct WalkParams {
   const int32_t *adjset;  // node2vec: per-vertex hash sets of the neighbour ids
   const int2 *colw;       // DeepWalk / PPR: (neighbour id, weight bits) records
   const int2 *vrec = nullptr;  // DeepWalk / PPR: (row start, max weight bits) per vertex, V + 1 entries
-  int keep_all_step = -1; // PPR, load-balanced loop: the step whose map goes to the tail launch keeps every pair (see walk_next_count_kernel)
+  int keep_all_step = -1; // PPR, load-balanced loop: the step whose map goes to the tail launch keeps every pair (see walk_next_ticket_kernel)
 };
-
-// node2vec asks "is v a neighbour of the previous vertex t?" for its candidates, and t is usually a
-// hub (a 17-probe bisection of dependent loads).  Every vertex with at least SET_MIN_DEG
-// neighbours gets an open-addressing hash set of its neighbour ids instead: buckets of 8 ids (one
-// 32-byte sector), the buckets [row_ptr[t]/4, (row_ptr[t]+deg)/4) of one array (regions of
-// consecutive vertices cannot overlap; at least deg slots each, load factor about 1/2).  An id
-// lives in the first free slot at or after its home bucket, so a lookup reads the home bucket and
-// is done unless that bucket is full and does not hold the id (about 5 % of the lookups).  The
-// answer is exact, i.e. the answer of utils::binarySearch (src/utils.hpp:30-48).
-constexpr int SET_MIN_DEG = 8;
-constexpr int32_t SET_EMPTY = -1;
-
-__device__ __forceinline__ uint32_t set_mix(uint32_t x) {
-  x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu; x ^= x >> 16;
-  return x;
-}
-__device__ __forceinline__ uint32_t set_bucket(int32_t v, uint32_t n_buckets) {
-  return (uint32_t)(((unsigned long long)set_mix((uint32_t)v) * n_buckets) >> 32);
-}
 
 constexpr int RETRY_CAP = 1 << 16;
 
@@ -106,8 +84,7 @@ struct Events {
 // Gathers from the big graph arrays (neighbour ids, weight records, set buckets) are used once per
 // launch in the transit-parallel kernels: there they are loaded with the streaming policy
 // (evict-first) so that they do not push the small per-sample and per-vertex arrays (maps,
-// counters, staged output row, row offsets) out of L2.  A sample-parallel walk revisits hub lists
-// from the same thread step after step and is faster with the default policy.
+// counters, staged output row, row offsets) out of L2.
 template <bool STREAM, typename T>
 __device__ __forceinline__ T ld_graph(const T *p) { return STREAM ? __ldcs(p) : __ldg(p); }
 
@@ -136,15 +113,8 @@ __device__ __forceinline__ bool n2v_member_slow(const NdGraphView &g, const int3
   return false;
 }
 
-// node2vec tries whose gathers are issued together (template argument of app_next): measured
-// best are 3 in the ticket kernel and 2 in the sample-parallel kernel at four CTAs of 256 per SM,
-// and 4 at three CTAs per SM in the kernel that also keeps the radix histogram
-constexpr int N2V_BATCH_COUNT = 3, N2V_BATCH_SP = 2, N2V_BATCH_TP = 4;
-// Weighted tries per round.  Every try of a round is gathered, so a larger batch buys latency with
-// gathers that a 60 % acceptance rate wastes: two per round, except PPR in the sample-parallel
-// kernel (walks die young there, the kernel is short of loads in flight; four measured faster).
-template <int APP, bool STREAM>
-__host__ __device__ constexpr int weight_batch() { return APP == ND_APP_PPR && !STREAM ? 4 : 2; }
+constexpr int N2V_BATCH = 4;      // node2vec tries whose gathers are issued together
+constexpr int WEIGHT_BATCH = 2;   // weighted tries per round: a larger batch buys latency with gathers that a 60 % acceptance rate wastes
 
 constexpr int32_t ROUND_AGAIN = -2;   // a round of tries ended without an accepted vertex
 
@@ -254,7 +224,7 @@ __device__ __forceinline__ int32_t n2v_round(const NdGraphView &g, const WalkPar
 
 // node2vec next() on a transit with n > 1 neighbours at a step > 0 when the row [ts, ts + tn) of the
 // previous vertex t is known already
-template <bool STREAM, int N2V_BATCH>
+template <bool STREAM>
 __device__ __forceinline__ int32_t n2v_next_known(const NdGraphView &g, const WalkParams &wp, int32_t rs, int32_t n,
                                                   int32_t t, int32_t ts, int32_t tn, Rng &rng, int *status, Events &ev) {
   const N2vConsts c(wp);
@@ -267,7 +237,7 @@ __device__ __forceinline__ int32_t n2v_next_known(const NdGraphView &g, const Wa
 }
 
 // One next() of the app on a transit with n > 0 neighbours; -1 = no vertex.
-template <int APP, bool STREAM = true, int N2V_BATCH = N2V_BATCH_COUNT>
+template <int APP, bool STREAM = true>
 __device__ __forceinline__ int32_t app_next(const NdGraphView &g, const WalkParams &wp, int step,
                                             int32_t transit, int32_t rs, int32_t n, int32_t &state_t,
                                             Rng &rng, int *status, Events &ev, bool have_max_w = false,
@@ -283,7 +253,6 @@ __device__ __forceinline__ int32_t app_next(const NdGraphView &g, const WalkPara
     }
     if (n == 1) return ld_graph<STREAM>(edges);
     const float max_w = have_max_w ? max_w_in : __ldg(g.max_w + transit);
-    constexpr int WEIGHT_BATCH = weight_batch<APP, STREAM>();
     for (int it = 0; it <= RETRY_CAP; it += WEIGHT_BATCH) {
       const int32_t r = weighted_round<STREAM, WEIGHT_BATCH>(wp, rs, n, max_w, rng, ev);
       if (r != ROUND_AGAIN) return r;
@@ -297,60 +266,20 @@ __device__ __forceinline__ int32_t app_next(const NdGraphView &g, const WalkPara
     const int32_t ts = __ldg(g.row_ptr + t);
     const int32_t tn = __ldg(g.row_ptr + t + 1) - ts;
     state_t = transit;
-    return n2v_next_known<STREAM, N2V_BATCH>(g, wp, rs, n, t, ts, tn, rng, status, ev);
+    return n2v_next_known<STREAM>(g, wp, rs, n, t, ts, tn, rng, status, ev);
   }
   return -1;
 }
 
 // ---------------------------------------------------------------- set-up kernels
 
-// thread per CSR entry: find the entry's source vertex by bisection of the row offsets and insert
-// the neighbour id into the source's set (first free slot at or after the home bucket)
-__global__ void adjset_build_kernel(NdGraphView g, int64_t E, int32_t *__restrict__ adjset, int *__restrict__ status) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
-    int32_t lo = 0, hi = g.V;  // last vertex with row_ptr[v] <= e
-    while (hi - lo > 1) {
-      const int32_t mid = lo + ((hi - lo) >> 1);
-      if ((int64_t)g.row_ptr[mid] <= e) lo = mid; else hi = mid;
-    }
-    const int32_t rs = g.row_ptr[lo], deg = g.row_ptr[lo + 1] - rs;
-    if (deg < SET_MIN_DEG) continue;
-    const uint32_t n_buckets = ((uint32_t)(rs + deg) >> 2) - ((uint32_t)rs >> 2);
-    int32_t *region = adjset + 8 * (size_t)((uint32_t)rs >> 2);
-    const int32_t v = g.col[e];
-    uint32_t b = set_bucket(v, n_buckets);
-    bool done = false;
-    for (uint32_t it = 0; it < n_buckets && !done; it++) {
-      for (int i = 0; i < 8 && !done; i++) {
-        int32_t *slot = region + 8 * (size_t)b + i;
-        int32_t cur = *(volatile int32_t *)slot;
-        if (cur == SET_EMPTY) cur = atomicCAS(slot, SET_EMPTY, v);
-        done = cur == SET_EMPTY || cur == v;  // placed, or the id is in the set already (repeated edge)
-      }
-      b = b + 1 < n_buckets ? b + 1 : 0;
-    }
-    if (!done) atomicOr(status, ND_DEV_RETRY_LIMIT);  // cannot happen: a region has at least deg slots
-  }
-}
-
-__global__ void colw_build_kernel(const int32_t *__restrict__ col, const float *__restrict__ w, int64_t E,
-                                  int2 *__restrict__ colw) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x)
-    colw[e] = make_int2(col[e], __float_as_int(w[e]));
-}
-
-__global__ void vrec_build_kernel(const int32_t *__restrict__ row_ptr, const float *__restrict__ max_w, int32_t V,
-                                  int2 *__restrict__ vrec) {
-  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v <= V; v += (int64_t)gridDim.x * blockDim.x)
-    vrec[v] = make_int2(row_ptr[v], v < V ? __float_as_int(max_w[v]) : 0);
-}
-
 __global__ void walk_reset_kernel(const int32_t *__restrict__ initial, int32_t V, int64_t S, int steps,
                                   int32_t *__restrict__ len, int32_t *__restrict__ state,
-                                  unsigned long long *__restrict__ stats, int32_t *__restrict__ tail_ctr) {
+                                  unsigned long long *__restrict__ stats, int32_t *__restrict__ tail_ctr,
+                                  const int32_t *__restrict__ init_n, int32_t *__restrict__ nlive) {
   const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (s < 8 && stats) stats[s] = 0ull;
-  if (s == 0 && tail_ctr) *tail_ctr = 0;
+  if (s < 8) stats[s] = 0ull;
+  if (s == 0) { *tail_ctr = 0; nlive[0] = *init_n; }
   if (s >= S) return;
   const int32_t t = initial[s];
   len[s] = (t >= 0 && t < V) ? steps : -1;
@@ -379,15 +308,6 @@ __global__ void init_map_kernel(const int32_t *__restrict__ initial, int32_t V, 
 }
 
 // ---------------------------------------------------------------- transit-parallel next()
-
-// node2vec keeps a round of candidates and set buckets in registers: four CTAs of 256 per SM (64
-// registers) with rounds of 2-3 tries measured faster than three CTAs with rounds of 4
-// (the weighted apps: five CTAs per SM in the ticket kernel, six in the sample-parallel one,
-// measured against 4-8 on the 2^20- and 2^24-vertex graphs)
-template <int APP>
-constexpr int walk_min_ctas() { return APP == ND_APP_NODE2VEC ? 4 : (APP == ND_APP_UNIFORM_WALK ? 1 : 5); }
-template <int APP>
-constexpr int walk_min_ctas_sp() { return APP == ND_APP_NODE2VEC ? 4 : (APP == ND_APP_UNIFORM_WALK ? 1 : 6); }
 
 constexpr int NEXT_THREADS = 256;
 
@@ -427,7 +347,7 @@ walk_next_tp_kernel(NdGraphView g, WalkParams wp, int step, int64_t first_sample
           Rng rng(wp.seed, (uint32_t)(first_sample + s), (uint32_t)step, 0u);
           int32_t st = 0;
           if (APP == ND_APP_NODE2VEC && step > 0) st = state[s];
-          nbr = app_next<APP, true, N2V_BATCH_TP>(g, wp, step, t, rs, deg, st, rng, status, ev);
+          nbr = app_next<APP>(g, wp, step, t, rs, deg, st, rng, status, ev);
           if (APP == ND_APP_NODE2VEC && nbr >= 0) state[s] = st;
         }
       }
@@ -454,7 +374,10 @@ walk_next_tp_kernel(NdGraphView g, WalkParams wp, int step, int64_t first_sample
   if (APP != ND_APP_UNIFORM_WALK) ev.flush(stats);
 }
 
-// ---------------------------------------------------------------- next() + counting inversion (load-balanced mode)
+// ---------------------------------------------------------------- next() + counting inversion (opt-in step loop)
+//
+// The load-balanced mode's step loop, kept behind its switches for the uniform walk (ND_WALK_STAGING) and PPR
+// (ND_WALK_NO_TAIL, ND_WALK_TAIL_PAIRS): a lane per walk is faster at every size (nd_walk_rows.cu).
 //
 // The transit ids are a dense key space (< V) and the map holds at most one pair per walk, so
 // the inversion does not need a multi-pass sort: next() takes a ticket on its new transit
@@ -466,9 +389,6 @@ walk_next_tp_kernel(NdGraphView g, WalkParams wp, int step, int64_t first_sample
 // and 16 B read + 8 B written per pair beside the counter traffic, against 2-3 radix passes of
 // three launches each.  The order of the pairs inside one transit's run depends on the order the
 // tickets were drawn; results do not, because every draw is keyed by the sample.
-// node2vec: the previous vertex of a walk travels with the sorted map (the scatter copies the
-// transit the pair was read under), so next() reads it with a coalesced load instead of a gather
-// by sample id.
 
 constexpr int CNT_SUPER = 4096;                             // counters per scan CTA = vertices per coarse bin
 constexpr int CNT_SUPER_SHIFT = 12;
@@ -492,101 +412,22 @@ constexpr int HUB_PASS = 8;        // tiles whose pairs a CTA serves per sweep o
 constexpr int HUB_CHUNK = 8192;    // neighbour ids staged at once (32 KB)
 
 // transit of hub tile `tau` of the 8-byte-record map, or -1 if the tile is not one
-__device__ __forceinline__ int32_t hub_tile(const void *in_rec, int n, int tau) {
+__device__ __forceinline__ int32_t hub_tile(const int2 *rec, int n, int tau) {
   const int base = tau * HUB_TILE;
   if (tau < 0 || base + HUB_TILE > n) return -1;
-  const int2 *rec = reinterpret_cast<const int2 *>(in_rec);
   const int32_t a = rec[base].x, b = rec[base + HUB_TILE - 1].x;
   return a == b ? a : -1;
 }
 
-// The kernel.  CTAs take tiles of 256 * PPT pairs of the sorted map (PPT = pairs a thread works on
-// at once, phase by phase; 1 measured best for every app, larger values are kept as a tuning macro).
-//  * uniform walk, DeepWalk, PPR: next() in place, up to 16 CTAs per SM, a tile each.
-//  * node2vec: the first round of tries of a pair is straight-line code (no divergence: the
-//    round's candidate gathers are issued together, then its set buckets); a pair the first round
-//    does not settle (every try rejected, or a membership test that has to walk past a full
-//    bucket: about one pair in eight) goes on a per-warp queue in shared memory, and whenever a
-//    queue holds 32 pairs the warp runs them through the general loop with all lanes busy --
-//    continuing behind the rejected tries in the pair's draw sequence, so nothing is gathered
-//    twice.  The draws of a pair depend only on (sample, step), so the queue changes no sample.
-//    The CTAs are persistent here (as many as are resident), so that the queues fill over tiles.
-//  * the coarse histogram (pairs per 4096 vertices, for the scan) is kept in shared memory and flushed once per CTA.
-// What bounds it: a pair costs a few random 32-byte sector reads that miss the L2 (one neighbour id;
-// node2vec about 2.6 candidates and 1.3 set buckets in a first round of four tries), and the memory system serves those at a
-// rate far below its streaming bandwidth; occupancy, pairs per thread, cache hints and the L2
-// fetch granularity were all measured and do not move the kernel's time by more than a few per cent.
 constexpr int COUNT_THREADS = 256;
-constexpr int COUNT_WARPS = COUNT_THREADS / 32;
 
-#ifndef ND_TUNE_PPT_UNIFORM
-#define ND_TUNE_PPT_UNIFORM 1
-#endif
-#ifndef ND_TUNE_PPT_WEIGHTED
-#define ND_TUNE_PPT_WEIGHTED 1
-#endif
-#ifndef ND_TUNE_PPT_N2V
-#define ND_TUNE_PPT_N2V 1
-#endif
-#ifndef ND_TUNE_N2V_FIRST
-#define ND_TUNE_N2V_FIRST 4
-#endif
-#ifndef ND_TUNE_CTAS_UNIFORM
-#define ND_TUNE_CTAS_UNIFORM 4
-#endif
-#ifndef ND_TUNE_CTAS_WEIGHTED
-#define ND_TUNE_CTAS_WEIGHTED 5
-#endif
-#ifndef ND_TUNE_CTAS_N2V
-#define ND_TUNE_CTAS_N2V 3
-#endif
-template <int APP>
-__host__ __device__ constexpr int count_ppt() {
-  return APP == ND_APP_NODE2VEC ? ND_TUNE_PPT_N2V : (APP == ND_APP_UNIFORM_WALK ? ND_TUNE_PPT_UNIFORM : ND_TUNE_PPT_WEIGHTED);
-}
-template <int APP>
-__host__ __device__ constexpr int count_ctas() {
-  return APP == ND_APP_NODE2VEC ? ND_TUNE_CTAS_N2V : (APP == ND_APP_UNIFORM_WALK ? ND_TUNE_CTAS_UNIFORM : ND_TUNE_CTAS_WEIGHTED);
-}
-constexpr int N2V_FIRST = ND_TUNE_N2V_FIRST;   // tries of the straight-line first round
-
-// A record of the transit-sorted map in the load-balanced mode.  One record = one aligned piece
-// of one 32-byte sector, so the scatter kernel places a pair with ONE random sector write:
-// {transit, sample} (8 bytes), or for node2vec 32 bytes {transit, sample, previous vertex, row
-// start of the previous vertex, its degree, 0, 0, 0} -- the previous vertex's row travels with
-// the pair, so next() never gathers row offsets by a random vertex id.
-template <bool N2V>
-struct MapRec {
-  int32_t t, s, pv;
-  int2 prow;
-};
-template <bool N2V>
-__host__ __device__ constexpr size_t map_rec_bytes() { return N2V ? 32 : 8; }
-
-template <bool N2V>
-__device__ __forceinline__ MapRec<N2V> map_rec_load(const ndmem::Keep &keep, const void *base, int i) {
-  MapRec<N2V> r;
-  if (N2V) {
-    const int4 *p = reinterpret_cast<const int4 *>(base) + 2 * (size_t)i;
-    const int4 a = keep.ld(p);
-    r.t = a.x; r.s = a.y; r.pv = a.z;
-    r.prow = make_int2(a.w, keep.ld(reinterpret_cast<const int32_t *>(p + 1)));
-  } else {
-    const int2 a = keep.ld(reinterpret_cast<const int2 *>(base) + i);
-    r.t = a.x; r.s = a.y; r.pv = 0;
-    r.prow = make_int2(0, 0);
-  }
-  return r;
-}
-
-// what the kernel writes for one settled pair
+// what the kernel writes for one pair
 template <bool COUNT>
 __device__ __forceinline__ void count_emit(const ndmem::Keep &keep, int i, int32_t s, int32_t nbr, int32_t V, int step,
                                            bool smem_bins, uint32_t *sh_bins, int32_t *__restrict__ out_key,
                                            int32_t *__restrict__ out_val, int32_t *__restrict__ out_rank,
                                            uint32_t *__restrict__ cnt, uint32_t *__restrict__ bsum,
                                            int32_t *__restrict__ tmp_step, int32_t *__restrict__ len,
-                                           int4 *__restrict__ out_ext, int32_t t, int32_t rs, int32_t deg,
                                            bool ends_next = false) {  // the walk takes this vertex and is known to stop at the next step
   if (nbr >= 0) keep.st(tmp_step + s, nbr); else len[s] = step;
   if (ends_next) len[s] = step + 1;
@@ -596,249 +437,68 @@ __device__ __forceinline__ void count_emit(const ndmem::Keep &keep, int i, int32
     if (in_map) {
       keep.st(out_val + i, s);
       keep.st(out_rank + i, (int32_t)keep.atom_add(cnt + nbr, 1u));
-      if (out_ext) keep.st(out_ext + i, make_int4(t, rs, deg, 0));  // node2vec: this transit is the pair's previous vertex next step
       if (smem_bins) atomicAdd(&sh_bins[nbr >> CNT_SUPER_SHIFT], 1u);
       else atomicAdd(&bsum[nbr >> CNT_SUPER_SHIFT], 1u);
     }
   }
 }
 
+// A CTA takes tiles of 256 pairs of the sorted map, records {transit, sample}: one record lies in one 32-byte
+// sector, so the scatter kernel places a pair with one random sector write.
 template <int APP, bool COUNT>
-__global__ void __launch_bounds__(COUNT_THREADS, count_ctas<APP>())
-walk_next_count_kernel(NdGraphView g, WalkParams wp, int step, int64_t first_sample,
-                       const void *__restrict__ in_rec, const int32_t *__restrict__ d_n,
-                       int32_t *__restrict__ out_key, int32_t *__restrict__ out_val, int32_t *__restrict__ out_rank,
-                       int4 *__restrict__ out_ext, uint32_t *__restrict__ cnt, uint32_t *__restrict__ bsum, int bins, int32_t *__restrict__ tmp_step,
-                       int32_t *__restrict__ len, int *__restrict__ status, unsigned long long *__restrict__ stats,
-                       int skip_hub_tiles) {
-  constexpr int PPT = count_ppt<APP>();
-  constexpr int QCAP = 32 * PPT + 32;
-  constexpr bool N2V = APP == ND_APP_NODE2VEC;
-  constexpr bool WEIGHTED = APP == ND_APP_DEEPWALK || APP == ND_APP_PPR;
-  extern __shared__ uint32_t sh_dyn[];
+__global__ void __launch_bounds__(COUNT_THREADS, APP == ND_APP_UNIFORM_WALK ? 4 : 5)
+walk_next_ticket_kernel(NdGraphView g, WalkParams wp, int step, int64_t first_sample, const int2 *__restrict__ in_rec,
+                        const int32_t *__restrict__ d_n, int32_t *__restrict__ out_key, int32_t *__restrict__ out_val,
+                        int32_t *__restrict__ out_rank, uint32_t *__restrict__ cnt, uint32_t *__restrict__ bsum, int bins,
+                        int32_t *__restrict__ tmp_step, int32_t *__restrict__ len, int *__restrict__ status,
+                        unsigned long long *__restrict__ stats, int skip_hub_tiles) {
+  static_assert(APP == ND_APP_UNIFORM_WALK || APP == ND_APP_PPR, "the apps with a step loop");
+  extern __shared__ uint32_t sh_bins[];
   Events ev;
   const int n = *d_n;
-  constexpr int TILE = COUNT_THREADS * PPT;
-  if ((int64_t)blockIdx.x * TILE >= n) return;  // no pair for this CTA
+  if ((int64_t)blockIdx.x * COUNT_THREADS >= n) return;  // no pair for this CTA
   const bool smem_bins = COUNT && bins <= MAX_SMEM_BINS;
-  uint32_t *sh_bins = sh_dyn;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int32_t *queue = reinterpret_cast<int32_t *>(sh_dyn + (smem_bins ? bins : 0)) + warp * QCAP;
-  int q_count = 0;  // warp-uniform
   if (smem_bins) {
-#pragma unroll 1
     for (int b = threadIdx.x; b < bins; b += COUNT_THREADS) sh_bins[b] = 0u;
     __syncthreads();
   }
-  const N2vConsts c(wp);
   const ndmem::Keep keep;
-
-  // runs 32 queued pairs (or the rest, when `all`) through the general loop.  A queue entry is the
-  // pair's position in the map; bit 31 set = the first round rejected all its tries, so the loop
-  // continues behind them in the pair's draw sequence; clear = the pair starts over (node2vec, a
-  // membership test that the home bucket did not answer).
-  constexpr uint32_t Q_CONTINUE = 0x80000000u;
-  auto drain = [&](bool all) {
-    while (q_count >= 32 || (all && q_count > 0)) {
-      const int take = q_count < 32 ? q_count : 32;
-      q_count -= take;
-      __syncwarp();
-      if (lane < take) {
-        const uint32_t q = (uint32_t)queue[q_count + lane];
-        const int i = (int)(q & ~Q_CONTINUE);
-        const bool cont = (q & Q_CONTINUE) != 0u;
-        const MapRec<N2V> r = map_rec_load<N2V>(keep, in_rec, i);
-        const int32_t rs = keep.ld_const(g.row_ptr + r.t);
-        const int32_t deg = keep.ld_const(g.row_ptr + r.t + 1) - rs;
-        Rng rng(wp.seed, (uint32_t)(first_sample + r.s), (uint32_t)step, 0u);
-        int32_t nbr = ROUND_AGAIN;
-        if (N2V) {
-          if (cont) { rng.seek(2u * N2V_FIRST); ev.n2v_tries += N2V_FIRST; }
-          nbr = n2v_next_known<true, N2V_BATCH_COUNT>(g, wp, rs, deg, r.pv, r.prow.x, r.prow.y, rng, status, ev);
-        }
-        count_emit<COUNT>(keep, i, r.s, nbr, g.V, step, smem_bins, sh_bins, out_key, out_val, out_rank, cnt, bsum, tmp_step, len,
-                          out_ext, r.t, rs, deg);
-      }
-      __syncwarp();
-    }
-  };
-
-  for (int base = blockIdx.x * TILE; base < n; base += gridDim.x * TILE) {
-    // opt-in staging of hub lists (uniform walk): a tile whose 256 pairs all stand on one transit
-    // belongs to walk_next_hub_kernel
-    if (APP == ND_APP_UNIFORM_WALK && PPT == 1 && skip_hub_tiles && hub_tile(in_rec, n, base / HUB_TILE) >= 0) continue;
-    int idx[PPT];
-    int32_t t[PPT], s[PPT], rs[PPT], deg[PPT], nbr[PPT];
-    bool live[PPT], settled[PPT], cont[PPT];
-    // ---- map entries
-    int32_t pv[PPT];
-    int2 prow[PPT];
-#pragma unroll
-    for (int k = 0; k < PPT; k++) {
-      idx[k] = base + k * COUNT_THREADS + threadIdx.x;
-      live[k] = idx[k] < n;
-      MapRec<N2V> r;
-      r.t = 0; r.s = 0; r.pv = 0; r.prow = make_int2(0, 0);
-      if (live[k]) r = map_rec_load<N2V>(keep, in_rec, idx[k]);
-      t[k] = r.t; s[k] = r.s; pv[k] = r.pv; prow[k] = r.prow;
-    }
-    // ---- row offsets
-    float mw[PPT];
-#pragma unroll
-    for (int k = 0; k < PPT; k++) {
-      mw[k] = 0.f;
-      const bool ok = live[k] && t[k] >= 0 && t[k] < g.V;
-      if (live[k] && !ok) atomicOr(status, ND_DEV_BAD_TRANSIT);
-      rs[k] = ok ? keep.ld_const(g.row_ptr + t[k]) : 0;
-      deg[k] = ok ? keep.ld_const(g.row_ptr + t[k] + 1) - rs[k] : 0;
-      if (WEIGHTED) mw[k] = ok ? __ldg(g.max_w + t[k]) : 0.f;   // independent of the row offsets: one latency, not two
-      nbr[k] = -1;
-      cont[k] = false;
-      settled[k] = deg[k] <= 0;  // next() runs only on transits with edges (src/nextdoor.cu:255,412)
-    }
-    // ---- first round
-    if (APP == ND_APP_UNIFORM_WALK) {  // example/uniformRandWalk.cu:35-36
-#pragma unroll
-      for (int k = 0; k < PPT; k++) {
-        Rng rng(wp.seed, (uint32_t)(first_sample + s[k]), (uint32_t)step, 0u);
-        const int32_t x = rng.rand_int(deg[k] > 0 ? deg[k] : 1);
-        if (deg[k] > 0) nbr[k] = __ldcs(g.col + rs[k] + x);
-        settled[k] = true;
+  for (int base = blockIdx.x * COUNT_THREADS; base < n; base += gridDim.x * COUNT_THREADS) {
+    // staged hub lists (uniform walk): a tile whose 256 pairs all stand on one transit belongs to walk_next_hub_kernel
+    if (APP == ND_APP_UNIFORM_WALK && skip_hub_tiles && hub_tile(in_rec, n, base / HUB_TILE) >= 0) continue;
+    const int i = base + threadIdx.x;
+    if (i >= n) continue;
+    const int2 r = keep.ld(in_rec + i);
+    const int32_t t = r.x, s = r.y;
+    int32_t nbr = -1;
+    if (t < 0 || t >= g.V) {
+      atomicOr(status, ND_DEV_BAD_TRANSIT);
+    } else {
+      const int32_t rs = keep.ld_const(g.row_ptr + t);
+      const int32_t deg = keep.ld_const(g.row_ptr + t + 1) - rs;
+      const float mw = APP == ND_APP_PPR ? __ldg(g.max_w + t) : 0.f;   // independent of the row offsets: one latency, not two
+      if (deg > 0) {  // next() runs only on transits with edges (src/nextdoor.cu:255,412)
+        Rng rng(wp.seed, (uint32_t)(first_sample + s), (uint32_t)step, 0u);
+        int32_t st = 0;
+        nbr = app_next<APP>(g, wp, step, t, rs, deg, st, rng, status, ev, true, mw);
       }
     }
-    if (WEIGHTED) {  // randomWalks.cu:74-90, 102-124: the rejection loop in place (rounds of two tries)
-#pragma unroll
-      for (int k = 0; k < PPT; k++) {
-        if (deg[k] > 0) {
-          Rng rng(wp.seed, (uint32_t)(first_sample + s[k]), (uint32_t)step, 0u);
-          int32_t st = 0;
-          nbr[k] = app_next<APP>(g, wp, step, t[k], rs[k], deg[k], st, rng, status, ev, true, mw[k]);
-          settled[k] = true;
-        }
-      }
+    // PPR: whether a walk stops at a step is the first draw of that step's keyed sequence and does
+    // not depend on where the walk stands, so the next step's verdict is known now: a pair that
+    // would only enter the next map to be dropped from it takes no ticket and is not scattered.
+    // (Not in the step that feeds the tail launch: the result update that runs beside the tail
+    // tells the tail's walks from the others by their length, and a walk ended here would have
+    // the length of one that the tail is about to continue.)
+    bool ends_next = false;
+    if (APP == ND_APP_PPR && COUNT && nbr >= 0 && step != wp.keep_all_step) {
+      Rng ahead(wp.seed, (uint32_t)(first_sample + s), (uint32_t)(step + 1), 0u);
+      ends_next = ahead.uniform() < wp.stop_prob;
+      ev.not_entered += ends_next ? 1u : 0u;
     }
-    if (N2V) {  // randomWalks.cu:141-172
-      int32_t x[PPT][N2V_FIRST], v[PPT][N2V_FIRST];
-      float y[PPT][N2V_FIRST];
-      int n_try[PPT];
-      bool simple[PPT];
-#pragma unroll
-      for (int k = 0; k < PPT; k++) {
-        simple[k] = deg[k] == 1 || step == 0;
-        Rng rng(wp.seed, (uint32_t)(first_sample + s[k]), (uint32_t)step, 0u);
-        n_try[k] = N2V_FIRST;
-#pragma unroll
-        for (int j = 0; j < N2V_FIRST; j++) {
-          x[k][j] = 0; y[k][j] = 0.f;
-          if (j < n_try[k]) {
-            x[k][j] = rng.rand_int(deg[k] > 0 ? deg[k] : 1);
-            y[k][j] = __fmul_rn(rng.uniform(), c.bound);
-            if (y[k][j] < c.sure) n_try[k] = j + 1;
-          }
-        }
-        if (simple[k]) { n_try[k] = 1; x[k][0] = 0; }
-        if (deg[k] <= 0) n_try[k] = 0;
-      }
-#pragma unroll
-      for (int k = 0; k < PPT; k++)
-#pragma unroll
-        for (int j = 0; j < N2V_FIRST; j++) v[k][j] = j < n_try[k] ? __ldcs(g.col + rs[k] + x[k][j]) : -1;
-      bool is_ret[PPT][N2V_FIRST], need[PPT][N2V_FIRST];
-      int4 ba[PPT][N2V_FIRST], bb[PPT][N2V_FIRST];
-#pragma unroll
-      for (int k = 0; k < PPT; k++) {
-        const int32_t ts = prow[k].x, tn = prow[k].y;
-        const uint32_t n_buckets = ((uint32_t)(ts + tn) >> 2) - ((uint32_t)ts >> 2);
-        const int4 *__restrict__ region = reinterpret_cast<const int4 *>(wp.adjset) + 2 * (size_t)((uint32_t)ts >> 2);
-#pragma unroll
-        for (int j = 0; j < N2V_FIRST; j++) {
-          is_ret[k][j] = wp.n2v_compat ? (x[k][j] == pv[k]) : (v[k][j] == pv[k]);  // randomWalks.cu:159 compares the index
-          need[k][j] = !simple[k] && j < n_try[k] && !is_ret[k][j] && y[k][j] >= c.lo && y[k][j] < c.hi;
-          const uint32_t bucket = set_bucket(v[k][j], n_buckets);
-          const bool fetch = need[k][j] && tn >= SET_MIN_DEG;
-          ba[k][j] = fetch ? __ldcs(region + 2 * (size_t)bucket) : make_int4(SET_EMPTY, SET_EMPTY, SET_EMPTY, SET_EMPTY);
-          bb[k][j] = fetch ? __ldcs(region + 2 * (size_t)bucket + 1) : make_int4(SET_EMPTY, SET_EMPTY, SET_EMPTY, SET_EMPTY);
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < PPT; k++) {
-        if (deg[k] > 0) {
-          if (simple[k]) {
-            nbr[k] = v[k][0];
-            settled[k] = true;
-          } else {
-            const bool use_set = prow[k].y >= SET_MIN_DEG;
-            int32_t res = ROUND_AGAIN;
-            uint32_t tries = (uint32_t)n_try[k], probes = 0;
-            bool slow = false;  // a membership test the home bucket does not answer, before any accepted try
-#pragma unroll
-            for (int j = N2V_FIRST - 1; j >= 0; j--) {
-              if (j < n_try[k]) {
-                bool accept, unsure = false;
-                uint32_t pj = 0;
-                if (is_ret[k][j]) {
-                  accept = y[k][j] < wp.p;
-                } else if (!need[k][j]) {
-                  accept = y[k][j] < c.lo;
-                } else {
-                  const int32_t vv = v[k][j];
-                  const bool found = ba[k][j].x == vv || ba[k][j].y == vv || ba[k][j].z == vv || ba[k][j].w == vv ||
-                                     bb[k][j].x == vv || bb[k][j].y == vv || bb[k][j].z == vv || bb[k][j].w == vv;
-                  if (use_set) pj = 8;
-                  unsure = !found && (!use_set || bb[k][j].w != SET_EMPTY);
-                  accept = y[k][j] < (found ? c.inv_q : 1.0f);
-                }
-                // walking from the last try to the first: an earlier try overrides what later ones said
-                if (unsure) { slow = true; res = ROUND_AGAIN; probes = 0; }
-                else if (accept) { slow = false; res = v[k][j]; tries = j + 1; probes = pj; }
-                else { probes += pj; }
-              }
-            }
-            if (!slow && res != ROUND_AGAIN) {
-              nbr[k] = res; settled[k] = true;
-              ev.n2v_tries += tries; ev.n2v_probes += probes;
-            } else if (!slow) {  // every try rejected: the queue continues behind them
-              cont[k] = true;
-              ev.n2v_probes += probes;
-            }
-          }
-        }
-      }
-    }
-    // ---- settled pairs are written, the others queued
-#pragma unroll
-    for (int k = 0; k < PPT; k++)
-      if (live[k] && settled[k]) {
-        // PPR: whether a walk stops at a step is the first draw of that step's keyed sequence and does
-        // not depend on where the walk stands, so the next step's verdict is known now: a pair that
-        // would only enter the next map to be dropped from it takes no ticket and is not scattered.
-        // (Not in the step that feeds the tail launch: the result update that runs beside the tail
-        // tells the tail's walks from the others by their length, and a walk ended here would have
-        // the length of one that the tail is about to continue.)
-        bool ends_next = false;
-        if (APP == ND_APP_PPR && COUNT && nbr[k] >= 0 && step != wp.keep_all_step) {
-          Rng ahead(wp.seed, (uint32_t)(first_sample + s[k]), (uint32_t)(step + 1), 0u);
-          ends_next = ahead.uniform() < wp.stop_prob;
-          ev.not_entered += ends_next ? 1u : 0u;
-        }
-        count_emit<COUNT>(keep, idx[k], s[k], nbr[k], g.V, step, smem_bins, sh_bins, out_key, out_val, out_rank, cnt, bsum, tmp_step, len,
-                          out_ext, t[k], rs[k], deg[k], ends_next);
-      }
-    if (APP != ND_APP_UNIFORM_WALK) {
-#pragma unroll
-      for (int k = 0; k < PPT; k++) {
-        const bool push = live[k] && !settled[k];
-        const uint32_t m = __ballot_sync(0xffffffffu, push);
-        if (push) queue[q_count + __popc(m & ((1u << lane) - 1u))] = (int32_t)((uint32_t)idx[k] | (cont[k] ? Q_CONTINUE : 0u));
-        q_count += __popc(m);
-      }
-      drain(false);
-    }
+    count_emit<COUNT>(keep, i, s, nbr, g.V, step, smem_bins, sh_bins, out_key, out_val, out_rank, cnt, bsum, tmp_step, len, ends_next);
   }
-  if (APP != ND_APP_UNIFORM_WALK) drain(true);
   if (smem_bins) {
     __syncthreads();
-#pragma unroll 1
     for (int b = threadIdx.x; b < bins; b += COUNT_THREADS) {
       const uint32_t cb = sh_bins[b];
       if (cb) atomicAdd(&bsum[b], cb);
@@ -849,7 +509,7 @@ walk_next_count_kernel(NdGraphView g, WalkParams wp, int step, int64_t first_sam
 
 template <bool COUNT>
 __global__ void __launch_bounds__(HUB_TILE)
-walk_next_hub_kernel(NdGraphView g, WalkParams wp, int step, int64_t first_sample, const void *__restrict__ in_rec,
+walk_next_hub_kernel(NdGraphView g, WalkParams wp, int step, int64_t first_sample, const int2 *__restrict__ in_rec,
                      const int32_t *__restrict__ d_n, int32_t *__restrict__ out_key, int32_t *__restrict__ out_val,
                      int32_t *__restrict__ out_rank, uint32_t *__restrict__ cnt, uint32_t *__restrict__ bsum,
                      int32_t *__restrict__ tmp_step, int32_t *__restrict__ len) {
@@ -857,7 +517,6 @@ walk_next_hub_kernel(NdGraphView g, WalkParams wp, int step, int64_t first_sampl
   const ndmem::Keep keep;
   const int n = *d_n;
   const int tiles = n / HUB_TILE;
-  const int2 *rec = reinterpret_cast<const int2 *>(in_rec);
   for (int tau = blockIdx.x; tau < tiles; tau += gridDim.x) {
     const int32_t t = hub_tile(in_rec, n, tau);
     if (t < 0 || hub_tile(in_rec, n, tau - 1) == t) continue;       // not the first tile of a run
@@ -873,7 +532,7 @@ walk_next_hub_kernel(NdGraphView g, WalkParams wp, int step, int64_t first_sampl
       for (int j = 0; j < HUB_PASS; j++) {
         smp[j] = 0; x[j] = -1; nbr[j] = -1;
         if (j < m) {
-          smp[j] = rec[(tau + j0 + j) * HUB_TILE + threadIdx.x].y;
+          smp[j] = in_rec[(tau + j0 + j) * HUB_TILE + threadIdx.x].y;
           Rng rng(wp.seed, (uint32_t)(first_sample + smp[j]), (uint32_t)step, 0u);
           if (deg > 0) x[j] = rng.rand_int(deg);
         }
@@ -891,7 +550,7 @@ walk_next_hub_kernel(NdGraphView g, WalkParams wp, int step, int64_t first_sampl
       for (int j = 0; j < HUB_PASS; j++)
         if (j < m)
           count_emit<COUNT>(keep, (int)((tau + j0 + j) * HUB_TILE + threadIdx.x), smp[j], nbr[j], g.V, step, false, nullptr, out_key,
-                            out_val, out_rank, cnt, bsum, tmp_step, len, nullptr, 0, 0, 0);
+                            out_val, out_rank, cnt, bsum, tmp_step, len);
     }
   }
 }
@@ -960,21 +619,18 @@ cnt_scan_kernel(uint32_t *__restrict__ cnt, const uint32_t *__restrict__ bsum, u
 }
 
 // Moves every live pair to its place in the sorted map of the next step -- one record, one random
-// sector write (see MapRec) -- and clears the coarse bins (the scan before it was their last reader).
+// sector write -- and clears the coarse bins (the scan before it was their last reader).
 constexpr int SCATTER_PPT = 2;
-template <bool N2V>
 __global__ void __launch_bounds__(256)
 walk_scatter_kernel(const int32_t *__restrict__ d_n, int32_t V, const int32_t *__restrict__ ukey,
                     const int32_t *__restrict__ uval, const int32_t *__restrict__ urank,
-                    const int4 *__restrict__ uext, const uint32_t *__restrict__ offs, void *__restrict__ out_rec,
-                    uint32_t *__restrict__ bsum, int bins) {
+                    const uint32_t *__restrict__ offs, int2 *__restrict__ out_rec, uint32_t *__restrict__ bsum, int bins) {
   const int n = *d_n;
   const ndmem::Keep keep;
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < bins; b += gridDim.x * blockDim.x) bsum[b] = 0u;
   constexpr int TILE = 256 * SCATTER_PPT;
   for (int base = blockIdx.x * TILE; base < n; base += gridDim.x * TILE) {
     int32_t k[SCATTER_PPT], v[SCATTER_PPT], r[SCATTER_PPT];
-    int4 ext[SCATTER_PPT];
     uint32_t pos[SCATTER_PPT];
 #pragma unroll
     for (int j = 0; j < SCATTER_PPT; j++) {
@@ -983,40 +639,21 @@ walk_scatter_kernel(const int32_t *__restrict__ d_n, int32_t V, const int32_t *_
       const bool ok = k[j] != V;
       v[j] = ok ? keep.ld(uval + i) : 0;
       r[j] = ok ? keep.ld(urank + i) : 0;
-      if (N2V) ext[j] = ok ? keep.ld(uext + i) : make_int4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int j = 0; j < SCATTER_PPT; j++) pos[j] = k[j] != V ? keep.ld(offs + k[j]) + (uint32_t)r[j] : 0u;
 #pragma unroll
-    for (int j = 0; j < SCATTER_PPT; j++) {
-      if (k[j] != V) {
-        if (N2V) {
-          int4 *dst = reinterpret_cast<int4 *>(out_rec) + 2 * (size_t)pos[j];
-          keep.st(dst, make_int4(k[j], v[j], ext[j].x, ext[j].y));
-          keep.st(dst + 1, make_int4(ext[j].z, 0, 0, 0));
-        } else {
-          keep.st(reinterpret_cast<int2 *>(out_rec) + pos[j], make_int2(k[j], v[j]));
-        }
-      }
-    }
+    for (int j = 0; j < SCATTER_PPT; j++)
+      if (k[j] != V) keep.st(out_rec + pos[j], make_int2(k[j], v[j]));
   }
 }
 
 // the transit-sorted initial map (key, value arrays) as records
-template <bool N2V>
 __global__ void __launch_bounds__(256)
 pack_map_kernel(const int32_t *__restrict__ d_n, const int32_t *__restrict__ key, const int32_t *__restrict__ val,
-                void *__restrict__ rec) {
+                int2 *__restrict__ rec) {
   const int n = *d_n;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    if (N2V) {
-      int4 *dst = reinterpret_cast<int4 *>(rec) + 2 * (size_t)i;
-      dst[0] = make_int4(key[i], val[i], 0, 0);
-      dst[1] = make_int4(0, 0, 0, 0);
-    } else {
-      reinterpret_cast<int2 *>(rec)[i] = make_int2(key[i], val[i]);
-    }
-  }
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) rec[i] = make_int2(key[i], val[i]);
 }
 
 // Row start, degree and maximum weight of a vertex for a kernel that reaches it by a random id: the
@@ -1033,7 +670,7 @@ __device__ __forceinline__ void vertex_of(const WalkParams &wp, int32_t v, int32
 // transit-parallel loop is three launches whose fixed cost outweighs the per-pair work.  From
 // there on one launch finishes the job, a lane per walk: a lane takes a pair of the sorted map
 // (a batch of indices per warp from a device counter, so that the lanes end together) and walks its sample to
-// the end; a warp makes one round of tries per trip as walk_sp_rounds_kernel does, and a lane
+// the end; a warp makes one round of tries per trip, and a lane
 // whose walk ended takes the next pair.  The draws are keyed by (sample, step), so the samples are
 // the ones the step-by-step loop would have produced.
 // DIRECT: the launch lasts at least as long as the longest surviving walk's chain of dependent
@@ -1042,9 +679,10 @@ __device__ __forceinline__ void vertex_of(const WalkParams &wp, int32_t v, int32
 // first_step).  The two kernels split the result rows between them: a survivor's slots from
 // first_step on, its entry of plen and its share of the counters belong to this kernel, everything
 // else to the other.
+constexpr int TAIL_CTAS = 6;
 template <int APP, bool DIRECT>
-__global__ void __launch_bounds__(256, walk_min_ctas_sp<APP>())
-walk_tail_kernel(NdGraphView g, WalkParams wp, int first_step, int64_t first_sample, const void *__restrict__ in_rec,
+__global__ void __launch_bounds__(256, TAIL_CTAS)
+walk_tail_kernel(NdGraphView g, WalkParams wp, int first_step, int64_t first_sample, const int2 *__restrict__ in_rec,
                  const int32_t *__restrict__ d_n, int32_t *__restrict__ next_pair, int64_t S, int32_t *__restrict__ tmp,
                  int32_t *__restrict__ len, int32_t *__restrict__ plen, int32_t *__restrict__ out, int *__restrict__ status,
                  unsigned long long *__restrict__ stats) {
@@ -1087,9 +725,9 @@ walk_tail_kernel(NdGraphView g, WalkParams wp, int first_step, int64_t first_sam
         if (i >= n) {
           done = true;
         } else {
-          const MapRec<false> r = map_rec_load<false>(keep, in_rec, i);
-          s = r.s;
-          cur = r.t;
+          const int2 r = keep.ld(in_rec + i);
+          s = r.y;
+          cur = r.x;
           step = first_step;
           have = true;
           fresh = true;
@@ -1156,130 +794,6 @@ walk_tail_kernel(NdGraphView g, WalkParams wp, int first_step, int64_t first_sam
     if (lane == 0) {
       if (edges) atomicAdd(&stats[0], (unsigned long long)edges);
       if (live) atomicAdd(&stats[1], (unsigned long long)live);
-    }
-  }
-  ev.flush(stats);
-}
-
-// ---------------------------------------------------------------- sample-parallel: a thread owns a walk
-
-template <int APP>
-__global__ void __launch_bounds__(256, walk_min_ctas_sp<APP>())
-walk_sp_kernel(NdGraphView g, WalkParams wp, int64_t first_sample, int64_t S,
-               const int32_t *__restrict__ initial, int32_t *__restrict__ tmp,
-               int32_t *__restrict__ len, int *__restrict__ status, unsigned long long *__restrict__ stats) {
-  Events ev;
-  for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < S;
-       s += (int64_t)gridDim.x * blockDim.x) {
-    int32_t cur = initial[s];
-    if (cur < 0 || cur >= g.V) continue;  // len already -1
-    int32_t st = 0;
-    int step = 0;
-    for (; step < wp.steps; step++) {
-      const int32_t rs = __ldg(g.row_ptr + cur);
-      const int32_t deg = __ldg(g.row_ptr + cur + 1) - rs;
-      int32_t nbr = -1;
-      if (deg > 0) {
-        Rng rng(wp.seed, (uint32_t)(first_sample + s), (uint32_t)step, 0u);
-        nbr = app_next<APP, false, N2V_BATCH_SP>(g, wp, step, cur, rs, deg, st, rng, status, ev);
-      }
-      if (nbr < 0) break;
-      tmp[(int64_t)step * S + s] = nbr;
-      cur = nbr;
-    }
-    if (step < wp.steps) len[s] = step;
-  }
-  if (APP != ND_APP_UNIFORM_WALK) ev.flush(stats);
-}
-
-// Sample-parallel walks of the apps with a rejection loop, as a per-lane state machine.  In
-// walk_sp_kernel a warp spends, at every step, as many rounds as its unluckiest lane (about 2.2
-// rounds per step for node2vec although a walk needs 1.13 on average).  Here a loop trip is ONE
-// round for every lane, wherever its walk stands: a lane whose try was accepted moves on to its
-// next step (the row offsets of the new vertex are fetched at the end of the trip, so that the
-// next trip starts with them in registers), a lane that was rejected stays on its step, a lane
-// whose walk ended takes the next walk.  Over 100 steps the lanes' round counts even out, so a
-// warp makes about as many trips as the average walk needs rounds.  Draws are keyed by (sample,
-// step) and counted per step, so the walks are the same as in every other kernel.
-template <int APP>
-__global__ void __launch_bounds__(256, walk_min_ctas_sp<APP>())
-walk_sp_rounds_kernel(NdGraphView g, WalkParams wp, int64_t first_sample, int64_t S,
-                      const int32_t *__restrict__ initial, int32_t *__restrict__ tmp,
-                      int32_t *__restrict__ len, int *__restrict__ status, unsigned long long *__restrict__ stats) {
-  constexpr bool N2V = APP == ND_APP_NODE2VEC;
-  Events ev;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x - stride;
-  bool have = false, fresh = true;
-  int32_t cur = 0, rs = 0, deg = 0, prev = 0, ts = 0, tn = 0;
-  int step = 0, rounds = 0;
-  float max_w = 0.f;
-  Rng rng(wp.seed, 0u, 0u, 0u);
-  const N2vConsts c(wp);
-  bool done = false;  // this lane has no walk left
-  // every lane of the warp stays in the loop until the last one is done: the vote at the loop
-  // head is where the lanes meet again after a trip, so that a trip runs as one instruction stream
-  while (__any_sync(0xffffffffu, !done)) {
-    if (!done && !have) {  // take the next walk of this lane
-      s += stride;
-      if (s >= S) {
-        done = true;
-      } else {
-        cur = initial[s];
-        if (cur >= 0 && cur < g.V) {  // otherwise len is -1 already and the lane tries the next walk in the next trip
-          if (N2V) {
-            rs = __ldg(g.row_ptr + cur);
-            deg = __ldg(g.row_ptr + cur + 1) - rs;
-          } else {
-            vertex_of(wp, cur, rs, deg, max_w);
-          }
-          step = 0;
-          have = true;
-          fresh = true;
-        }
-      }
-    }
-    if (have) {
-      int32_t nbr = ROUND_AGAIN;
-      if (deg == 0) {
-        nbr = -1;
-      } else if (fresh) {  // first trip of a step: the draws of the step start, the cases without a rejection loop
-        rng = Rng(wp.seed, (uint32_t)(first_sample + s), (uint32_t)step, 0u);
-        rounds = 0;
-        fresh = false;
-        if (APP == ND_APP_PPR) {
-          const float pr = rng.uniform();
-          if (pr < wp.stop_prob) nbr = -1;
-        }
-        if (nbr == ROUND_AGAIN && (deg == 1 || (N2V && step == 0))) nbr = __ldg(g.col + rs);
-      }
-      if (nbr == ROUND_AGAIN) {
-        if (N2V) nbr = n2v_round<false, N2V_BATCH_SP>(g, wp, c, rs, deg, prev, ts, tn, rng, ev);
-        else nbr = weighted_round<false, 2>(wp, rs, deg, max_w, rng, ev);
-        if (nbr == ROUND_AGAIN && ++rounds > RETRY_CAP) {
-          atomicOr(status, ND_DEV_RETRY_LIMIT);
-          nbr = __ldg(g.col + rs);
-        }
-      }
-      if (nbr == -1) {  // the walk ends here
-        len[s] = step;
-        have = false;
-      } else if (nbr >= 0) {
-        tmp[(int64_t)step * S + s] = nbr;
-        prev = cur; ts = rs; tn = deg;
-        cur = nbr;
-        if (++step == wp.steps) {
-          have = false;
-        } else {
-          if (N2V) {
-            rs = __ldg(g.row_ptr + cur);
-            deg = __ldg(g.row_ptr + cur + 1) - rs;
-          } else {
-            vertex_of(wp, cur, rs, deg, max_w);
-          }
-          fresh = true;
-        }
-      }  // ROUND_AGAIN: the lane stays on its step
     }
   }
   ev.flush(stats);
@@ -1479,38 +993,22 @@ int launch_next_tp(nd_sampler *s, const WalkParams &wp, int step, bool hist, int
   return ND_OK;
 }
 
-// next() of one step in the load-balanced mode: as many CTAs as are resident, at most one per tile
+// next() of one step of the ticket loop: up to 16 CTAs per SM, a tile each
 template <int APP>
-int launch_count(nd_sampler *s, const WalkParams &wp, int step, bool last, int bins, const void *in_rec, const int32_t *d_n,
-                 int32_t *ukey, int32_t *uval, int32_t *tmp_step) {
-  constexpr int PPT = count_ppt<APP>();
-  const size_t smem = sizeof(uint32_t) * ((bins <= MAX_SMEM_BINS && !last ? (size_t)bins : 0) + (size_t)COUNT_WARPS * (32 * PPT + 32));
-  static int resident[2] = {0, 0};  // CTAs per SM (with and without the histogram), asked once
-  int &res = resident[last ? 1 : 0];
-  if (res == 0) {
-    int r = 0;
-    cudaError_t e = last ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, walk_next_count_kernel<APP, false>, COUNT_THREADS, smem)
-                         : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, walk_next_count_kernel<APP, true>, COUNT_THREADS, smem);
-    if (e != cudaSuccess || r < 1) { cudaGetLastError(); r = count_ctas<APP>(); }
-    res = r;
-  }
-  const int64_t tiles = (s->S + COUNT_THREADS * PPT - 1) / (COUNT_THREADS * PPT);
-  // node2vec: as many CTAs as are resident, each working through several tiles (its per-warp queues
-  // fill up over the tiles); the others measured best with up to 16 CTAs per SM, a tile each
-  const int64_t cap = (int64_t)s->dev.sms * (APP == ND_APP_NODE2VEC ? res : 16);
+int launch_ticket(nd_sampler *s, const WalkParams &wp, int step, bool last, int bins, const int2 *in_rec, const int32_t *d_n,
+                  int32_t *ukey, int32_t *uval, int32_t *tmp_step) {
+  const size_t smem = sizeof(uint32_t) * (bins <= MAX_SMEM_BINS && !last ? (size_t)bins : 0);
+  const int64_t tiles = (s->S + COUNT_THREADS - 1) / COUNT_THREADS, cap = (int64_t)s->dev.sms * 16;
   const int grid = (int)(tiles < cap ? (tiles > 0 ? tiles : 1) : cap);
   NdGraphView gv = nd_view(s->g);
-  int4 *uext = APP == ND_APP_NODE2VEC && !last ? s->d_uext : nullptr;
-  const char *staging_env = getenv("ND_WALK_STAGING");   // opt-in: hub tiles of the uniform walk through walk_next_hub_kernel
-  const int staging = APP == ND_APP_UNIFORM_WALK && count_ppt<APP>() == 1 && staging_env && staging_env[0] == '1' ? 1 : 0;
+  const char *staging_env = getenv("ND_WALK_STAGING");   // hub tiles of the uniform walk through walk_next_hub_kernel
+  const int staging = APP == ND_APP_UNIFORM_WALK && staging_env && staging_env[0] == '1' ? 1 : 0;
   if (last)
-    walk_next_count_kernel<APP, false><<<grid, COUNT_THREADS, smem, s->stream>>>(
-        gv, wp, step, s->first, in_rec, d_n, ukey, uval, s->d_rank, uext, s->d_cnt, s->d_bsum, bins,
-        tmp_step, s->d_len, s->d_status, s->d_stats, staging);
+    walk_next_ticket_kernel<APP, false><<<grid, COUNT_THREADS, smem, s->stream>>>(
+        gv, wp, step, s->first, in_rec, d_n, ukey, uval, s->d_rank, s->d_cnt, s->d_bsum, bins, tmp_step, s->d_len, s->d_status, s->d_stats, staging);
   else
-    walk_next_count_kernel<APP, true><<<grid, COUNT_THREADS, smem, s->stream>>>(
-        gv, wp, step, s->first, in_rec, d_n, ukey, uval, s->d_rank, uext, s->d_cnt, s->d_bsum, bins,
-        tmp_step, s->d_len, s->d_status, s->d_stats, staging);
+    walk_next_ticket_kernel<APP, true><<<grid, COUNT_THREADS, smem, s->stream>>>(
+        gv, wp, step, s->first, in_rec, d_n, ukey, uval, s->d_rank, s->d_cnt, s->d_bsum, bins, tmp_step, s->d_len, s->d_status, s->d_stats, staging);
   if (staging) {  // the hub tiles the kernel above left out
     const int hgrid = (int)(tiles < (int64_t)s->dev.sms * 8 ? (tiles > 0 ? tiles : 1) : (int64_t)s->dev.sms * 8);
     if (last)
@@ -1524,49 +1022,19 @@ int launch_count(nd_sampler *s, const WalkParams &wp, int step, bool last, int b
   return ND_OK;
 }
 
-template <int APP>
-int launch_sp(nd_sampler *s, const WalkParams &wp) {
-  const int64_t blocks = (s->S + 255) / 256;
-  const int grid = (int)(blocks < (int64_t)s->dev.sms * 32 ? blocks : (int64_t)s->dev.sms * 32);
-  static const bool plain = getenv("ND_SP_PLAIN") != nullptr;
-  if (APP == ND_APP_UNIFORM_WALK || plain)   // no rejection loop: one round per step for every lane anyway
-    walk_sp_kernel<APP><<<grid, 256, 0, s->stream>>>(nd_view(s->g), wp, s->first, s->S, s->d_initial,
-                                                      s->d_tmp, s->d_len, s->d_status, s->d_stats);
-  else
-    walk_sp_rounds_kernel<APP><<<grid, 256, 0, s->stream>>>(nd_view(s->g), wp, s->first, s->S, s->d_initial,
-                                                             s->d_tmp, s->d_len, s->d_status, s->d_stats);
-  return ND_OK;
+// whether mode 1 takes the step loop over sorted maps for this sampler (its switches are set)
+bool step_loop(const nd_sampler *s) {
+  const char *st = getenv("ND_WALK_STAGING");
+  if (s->p.app == ND_APP_UNIFORM_WALK) return st && st[0] == '1';
+  return s->p.app == ND_APP_PPR && (getenv("ND_WALK_NO_TAIL") || getenv("ND_WALK_TAIL_PAIRS"));
 }
 
 }  // namespace
 
-// The derived layouts of a graph are built by the first sampler that needs them; samplers of one
-// graph may be created from several host threads, so the builds are serialised.
-static std::mutex g_derived_mutex;
-
-// interleaved (neighbour id, weight) records of a graph, built on first use
-int nd_graph_ensure_colw(const nd_graph *g, int sms) {
-  std::lock_guard<std::mutex> lock(g_derived_mutex);
-  if (g->colw || g->E == 0) return ND_OK;
-  int2 *cw = nullptr, *vr = nullptr;
-  ND_CUDA(cudaMalloc(&cw, sizeof(int2) * (size_t)g->E));
-  if (cudaMalloc(&vr, sizeof(int2) * ((size_t)g->V + 1)) != cudaSuccess) {
-    cudaFree(cw);
-    nd_set_error("per-vertex records: out of device memory");
-    cudaGetLastError();
-    return ND_ERR_CUDA;
-  }
-  colw_build_kernel<<<sms * 16, 256>>>(g->col, g->w, g->E, cw);
-  vrec_build_kernel<<<sms * 16, 256>>>(g->row_ptr, g->max_w, g->V, vr);
-  ND_CUDA(cudaDeviceSynchronize());
-  g->vrec = vr;
-  g->colw = cw;
-  return ND_OK;
-}
+bool nd_walk_step_loop(const nd_sampler *s) { return step_loop(s); }
 
 namespace {
 __device__ int g_step_status;                       // device status word of nd_walk_step
-__device__ unsigned long long g_step_stats[8];      // its event counters (not reported)
 
 // One next() per explicit (transit, sample) pair; the sample id is the global one the draws are keyed by.
 template <int APP>
@@ -1667,65 +1135,69 @@ int nd_walk_step_launch(const nd_graph *g, const nd_app_params *p, int step, int
   return ND_OK;
 }
 
+int nd_walk_ensure_tmp(nd_sampler *s) {
+  if (!s->d_tmp) ND_CUDA(cudaMalloc(&s->d_tmp, sizeof(int32_t) * (size_t)(s->S > 0 ? s->S : 1) * s->p.steps));
+  return ND_OK;
+}
+
 int nd_walk_alloc(nd_sampler *s) {
   const int64_t S = s->S;
   const int steps = s->p.steps;
   ND_REQUIRE(steps >= 1 && steps <= 4096, ND_ERR_ARG, "walk length %d out of range [1,4096]", steps);
-  ND_CUDA(cudaMalloc(&s->d_tmp, sizeof(int32_t) * (size_t)S * steps));
-  ND_CUDA(cudaMalloc(&s->d_len, sizeof(int32_t) * (size_t)S));
-  // the result array starts out all-invalid with no slot in use (walk_finalize_kernel keeps it that way)
+  // the result array starts out all-invalid with no slot in use (every kernel that writes rows keeps it that way)
   ND_CUDA(cudaMalloc(&s->d_plen, sizeof(int32_t) * (size_t)(S > 0 ? S : 1)));
   ND_CUDA(cudaMemset(s->d_plen, 0, sizeof(int32_t) * (size_t)(S > 0 ? S : 1)));
   if (S > 0) walk_fill_kernel<<<s->dev.sms * 8, 256>>>(s->d_out, S * steps / 4, S * steps, s->g->V);
-  if (s->p.app == ND_APP_NODE2VEC) {
-    ND_CUDA(cudaMalloc(&s->d_state, sizeof(int32_t) * (size_t)S));
-    std::lock_guard<std::mutex> lock(g_derived_mutex);
-    if (!s->g->adjset) {  // 8 bytes per CSR entry, built once per graph
-      const size_t slots = 8 * ((size_t)(s->g->E / 4) + 2);
-      int32_t *set = nullptr;
-      ND_CUDA(cudaMalloc(&set, sizeof(int32_t) * slots));
-      ND_CUDA(cudaMemset(set, 0xff, sizeof(int32_t) * slots));
-      ND_CUDA(cudaMemset(s->d_status, 0, sizeof(int)));
-      adjset_build_kernel<<<s->dev.sms * 16, 256>>>(nd_view(s->g), s->g->E, set, s->d_status);
-      int st = 0;
-      ND_CUDA(cudaMemcpy(&st, s->d_status, sizeof(int), cudaMemcpyDeviceToHost));
-      if (st) { cudaFree(set); ND_REQUIRE(false, ND_ERR_DEVICE, "neighbour-set construction failed (status %d)", st); }
-      s->g->adjset = set;
-    }
-  }
+  ND_CUDA(cudaMalloc(&s->d_nlive, sizeof(int32_t) * (size_t)(steps + 5)));  // live pairs per step, a spare slot, the tail launch's work counter, walks that can start, pairs of the initial map
+  s->d_init_n = s->d_nlive + steps + 4;
+  s->map_stale = true;
+  return nd_walk_rows_alloc(s);
+}
+
+// What the transit-parallel modes need beyond a lane per walk, made by the first job that runs in one.
+static int tp_alloc(nd_sampler *s) {
+  const int64_t S = s->S;
+  const size_t S1 = (size_t)(S > 0 ? S : 1);
+  ND_TRY(nd_walk_ensure_tmp(s));
   if (s->p.app == ND_APP_DEEPWALK || s->p.app == ND_APP_PPR) ND_TRY(nd_graph_ensure_colw(s->g, s->dev.sms));
+  if (!s->d_len) ND_CUDA(cudaMalloc(&s->d_len, sizeof(int32_t) * S1));
+  if (s->p.app == ND_APP_NODE2VEC && !s->d_state) ND_CUDA(cudaMalloc(&s->d_state, sizeof(int32_t) * S1));
   s->map_cap = S;
   for (int i = 0; i < 2; i++) {
-    ND_CUDA(cudaMalloc(&s->d_map_key[i], sizeof(int32_t) * (size_t)S));
-    ND_CUDA(cudaMalloc(&s->d_map_val[i], sizeof(int32_t) * (size_t)S));
+    if (!s->d_map_key[i]) ND_CUDA(cudaMalloc(&s->d_map_key[i], sizeof(int32_t) * S1));
+    if (!s->d_map_val[i]) ND_CUDA(cudaMalloc(&s->d_map_val[i], sizeof(int32_t) * S1));
   }
-  ND_CUDA(cudaMalloc(&s->d_init_key, sizeof(int32_t) * (size_t)S));
-  ND_CUDA(cudaMalloc(&s->d_init_val, sizeof(int32_t) * (size_t)S));
-  ND_CUDA(cudaMalloc(&s->d_nlive, sizeof(int32_t) * (size_t)(steps + 4)));  // live pairs per step, a spare slot, the tail launch's work counter, walks that can start
+  if (!s->d_init_key) ND_CUDA(cudaMalloc(&s->d_init_key, sizeof(int32_t) * S1));
+  if (!s->d_init_val) ND_CUDA(cudaMalloc(&s->d_init_val, sizeof(int32_t) * S1));
   const int key_bits = nd_bit_length((uint32_t)(s->g->V > 1 ? s->g->V - 1 : 1));
-  ND_TRY(nd_radix_scratch_alloc(&s->radix, key_bits, S));
-  // counting inversion (load-balanced mode)
-  const size_t V = (size_t)s->g->V;
+  if (!s->radix.tile_hist) ND_TRY(nd_radix_scratch_alloc(&s->radix, key_bits, S));
+  return ND_OK;
+}
+
+// ... and the step loop of the load-balanced mode
+static int loop_alloc(nd_sampler *s) {
+  if (s->loop_ready) return ND_OK;
+  const size_t V = (size_t)s->g->V, S1 = (size_t)(s->S > 0 ? s->S : 1);
   const size_t bins = (V + CNT_SUPER - 1) / CNT_SUPER;
-  ND_CUDA(cudaMalloc(&s->d_cnt, sizeof(uint32_t) * bins * CNT_SUPER));   // padded to whole bins
-  ND_CUDA(cudaMalloc(&s->d_offs, sizeof(uint32_t) * bins * CNT_SUPER));
-  ND_CUDA(cudaMalloc(&s->d_bsum, sizeof(uint32_t) * bins));
-  ND_CUDA(cudaMalloc(&s->d_rank, sizeof(int32_t) * (size_t)(S > 0 ? S : 1)));
+  if (!s->d_cnt) ND_CUDA(cudaMalloc(&s->d_cnt, sizeof(uint32_t) * bins * CNT_SUPER));   // padded to whole bins
+  if (!s->d_offs) ND_CUDA(cudaMalloc(&s->d_offs, sizeof(uint32_t) * bins * CNT_SUPER));
+  if (!s->d_bsum) ND_CUDA(cudaMalloc(&s->d_bsum, sizeof(uint32_t) * bins));
+  if (!s->d_rank) ND_CUDA(cudaMalloc(&s->d_rank, sizeof(int32_t) * S1));
   ND_CUDA(cudaMemset(s->d_cnt, 0, sizeof(uint32_t) * bins * CNT_SUPER));
   ND_CUDA(cudaMemset(s->d_bsum, 0, sizeof(uint32_t) * bins));
-  const size_t rec = s->p.app == ND_APP_NODE2VEC ? map_rec_bytes<true>() : map_rec_bytes<false>();
-  const size_t S1 = (size_t)(S > 0 ? S : 1);
-  for (int i = 0; i < 2; i++) ND_CUDA(cudaMalloc(&s->d_srec[i], rec * S1));
-  ND_CUDA(cudaMalloc(&s->d_init_rec, rec * S1));
-  if (s->p.app == ND_APP_NODE2VEC) ND_CUDA(cudaMalloc(&s->d_uext, sizeof(int4) * S1));
-  if (s->p.app == ND_APP_PPR && s->p.stop_prob > 0.f) {  // the tail launch runs beside the result update
+  for (int i = 0; i < 2; i++) if (!s->d_srec[i]) ND_CUDA(cudaMalloc(&s->d_srec[i], sizeof(int2) * S1));
+  if (!s->d_init_rec) ND_CUDA(cudaMalloc(&s->d_init_rec, sizeof(int2) * S1));
+  if (s->p.app == ND_APP_PPR && s->p.stop_prob > 0.f && !s->h_active) {  // the tail launch runs beside the result update
     ND_CUDA(cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking));
     ND_CUDA(cudaEventCreateWithFlags(&s->side_fork, cudaEventDisableTiming));
     ND_CUDA(cudaEventCreateWithFlags(&s->side_join, cudaEventDisableTiming));
+    ND_CUDA(cudaEventCreateWithFlags(&s->active_done, cudaEventDisableTiming));
     ND_CUDA(cudaMallocHost(&s->h_active, sizeof(int32_t)));
     *s->h_active = -1;
-    ND_CUDA(cudaEventCreateWithFlags(&s->active_done, cudaEventDisableTiming));
   }
+  s->map_stale = true;   // the records are made with the map
+  ND_CUDA(cudaDeviceSynchronize());   // the clears above ran on the default stream
+  s->loop_ready = true;
   return ND_OK;
 }
 
@@ -1744,14 +1216,13 @@ int nd_sampler_build_initial_map(nd_sampler *s) {
   arr.a[0] = (uint32_t *)s->d_map_key[0]; arr.a[1] = (uint32_t *)s->d_map_val[0]; arr.a[2] = nullptr;
   arr.b[0] = (uint32_t *)s->d_map_key[1]; arr.b[1] = (uint32_t *)s->d_map_val[1]; arr.b[2] = nullptr;
   bool in_b = false;
-  ND_TRY(nd_radix_sort(s->dev, s->stream, &s->radix, s->radix.plan, arr, 0, d_n_in, s->d_nlive, true, (uint32_t)s->g->V, false, &in_b));
+  ND_TRY(nd_radix_sort(s->dev, s->stream, &s->radix, s->radix.plan, arr, 0, d_n_in, s->d_init_n, true, (uint32_t)s->g->V, false, &in_b));
   const int src = in_b ? 1 : 0;
   ND_CUDA(cudaMemcpyAsync(s->d_init_key, s->d_map_key[src], sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, s->stream));
   ND_CUDA(cudaMemcpyAsync(s->d_init_val, s->d_map_val[src], sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, s->stream));
-  if (s->d_init_rec) {  // walks: the records the load-balanced mode starts from
+  if (s->d_init_rec) {  // the records the step loop starts from
     const int pg = (int)(blocks < s->dev.sms * 16 ? (blocks > 0 ? blocks : 1) : s->dev.sms * 16);
-    if (s->p.app == ND_APP_NODE2VEC) pack_map_kernel<true><<<pg, 256, 0, s->stream>>>(s->d_nlive, s->d_map_key[src], s->d_map_val[src], s->d_init_rec);
-    else pack_map_kernel<false><<<pg, 256, 0, s->stream>>>(s->d_nlive, s->d_map_key[src], s->d_map_val[src], s->d_init_rec);
+    pack_map_kernel<<<pg, 256, 0, s->stream>>>(s->d_init_n, s->d_map_key[src], s->d_map_val[src], (int2 *)s->d_init_rec);
   }
   if (s->h_active) {  // PPR: how many walks can start (read when the step loop is laid out, not waited for here)
     s->active_starts = -1;
@@ -1762,6 +1233,7 @@ int nd_sampler_build_initial_map(nd_sampler *s) {
     ND_CUDA(cudaMemcpyAsync(s->h_active, d_active, sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream));
     ND_CUDA(cudaEventRecord(s->active_done, s->stream));
   }
+  s->map_stale = false;
   return ND_OK;  // stream-ordered: no host synchronisation, so chunks on different streams overlap
 }
 
@@ -1778,19 +1250,9 @@ static int walk_enqueue(nd_sampler *s, int mode) {
   int tail_from = 0x7fffffff;               // first step of that launch
   const int rblocks = (int)((S + 255) / 256);
   walk_reset_kernel<<<rblocks > 1 ? rblocks : 1, 256, 0, st>>>(s->d_initial, s->g->V, S, steps, s->d_len, s->d_state, s->d_stats,
-                                                                s->d_nlive + steps + 2);
+                                                                s->d_nlive + steps + 2, s->d_init_n, s->d_nlive);
   nd_count_launches(1);
-  if (mode == ND_MODE_SAMPLE_PARALLEL) {
-    nd_phase_begin(s, ND_PHASE_NEXT);
-    switch (app) {
-      case ND_APP_UNIFORM_WALK: launch_sp<ND_APP_UNIFORM_WALK>(s, wp); break;
-      case ND_APP_DEEPWALK: launch_sp<ND_APP_DEEPWALK>(s, wp); break;
-      case ND_APP_PPR: launch_sp<ND_APP_PPR>(s, wp); break;
-      default: launch_sp<ND_APP_NODE2VEC>(s, wp); break;
-    }
-    nd_phase_end(s);
-    nd_count_launches(1);
-  } else if (mode == ND_MODE_TRANSIT_PARALLEL) {
+  if (mode == ND_MODE_TRANSIT_PARALLEL) {
     // plain transit-parallel: sort-based inversion, first digit histogram fused into next()
     const NdRadixPlan &pl = s->radix.plan;
     const int64_t tiles = pl.max_tiles;
@@ -1826,14 +1288,12 @@ static int walk_enqueue(nd_sampler *s, int mode) {
       cur = res ^ 1;
     }
   } else {
-    // load-balanced transit-parallel: next() draws tickets, counting inversion
+    // the step loop of the load-balanced mode: next() draws tickets, counting inversion
     const int V = s->g->V;
     const int bins = (V + CNT_SUPER - 1) / CNT_SUPER;
-    const bool n2v = app == ND_APP_NODE2VEC;
-    // unsorted pairs written by next(): key/val in d_map_*[0], rank, (node2vec) d_uext; the sorted
-    // maps are records that ping-pong between d_srec[0] and d_srec[1]
+    // unsorted pairs written by next(): key/val in d_map_*[0], rank; the sorted maps are records that ping-pong between d_srec[0] and d_srec[1]
     int32_t *ukey = s->d_map_key[0], *uval = s->d_map_val[0];
-    const void *in_rec = s->d_init_rec;
+    const int2 *in_rec = (const int2 *)s->d_init_rec;
     const int64_t sblocks = (S + 256 * SCATTER_PPT - 1) / (256 * SCATTER_PPT);
     const int sgrid = (int)(sblocks < (int64_t)s->dev.sms * 16 ? (sblocks > 0 ? sblocks : 1) : (int64_t)s->dev.sms * 16);
     // PPR: a step of the loop costs about 40 us of launches and of the scan over the per-vertex
@@ -1861,22 +1321,17 @@ static int walk_enqueue(nd_sampler *s, int mode) {
       const int32_t *d_n = s->d_nlive + step;
       int32_t *tmp_step = s->d_tmp + (int64_t)step * S;
       nd_phase_begin(s, ND_PHASE_NEXT);
-      switch (app) {
-        case ND_APP_UNIFORM_WALK: ND_TRY(launch_count<ND_APP_UNIFORM_WALK>(s, wp, step, last, bins, in_rec, d_n, ukey, uval, tmp_step)); break;
-        case ND_APP_DEEPWALK: ND_TRY(launch_count<ND_APP_DEEPWALK>(s, wp, step, last, bins, in_rec, d_n, ukey, uval, tmp_step)); break;
-        case ND_APP_PPR: ND_TRY(launch_count<ND_APP_PPR>(s, wp, step, last, bins, in_rec, d_n, ukey, uval, tmp_step)); break;
-        default: ND_TRY(launch_count<ND_APP_NODE2VEC>(s, wp, step, last, bins, in_rec, d_n, ukey, uval, tmp_step)); break;
-      }
+      if (app == ND_APP_PPR) ND_TRY(launch_ticket<ND_APP_PPR>(s, wp, step, last, bins, in_rec, d_n, ukey, uval, tmp_step));
+      else ND_TRY(launch_ticket<ND_APP_UNIFORM_WALK>(s, wp, step, last, bins, in_rec, d_n, ukey, uval, tmp_step));
       nd_phase_end(s);
       nd_count_launches(1);
       if (last) break;
       nd_phase_begin(s, ND_PHASE_INVERT);
       cnt_scan_kernel<<<bins, SCAN_THREADS, 0, st>>>(s->d_cnt, s->d_bsum, s->d_offs, s->d_nlive + step + 1);
-      if (n2v) walk_scatter_kernel<true><<<sgrid, 256, 0, st>>>(d_n, V, ukey, uval, s->d_rank, s->d_uext, s->d_offs, s->d_srec[cur], s->d_bsum, bins);
-      else walk_scatter_kernel<false><<<sgrid, 256, 0, st>>>(d_n, V, ukey, uval, s->d_rank, nullptr, s->d_offs, s->d_srec[cur], s->d_bsum, bins);
+      walk_scatter_kernel<<<sgrid, 256, 0, st>>>(d_n, V, ukey, uval, s->d_rank, s->d_offs, (int2 *)s->d_srec[cur], s->d_bsum, bins);
       nd_phase_end(s);
       nd_count_launches(2);
-      in_rec = s->d_srec[cur];
+      in_rec = (const int2 *)s->d_srec[cur];
       cur ^= 1;
     }
     if (tp_steps < steps) {
@@ -1892,7 +1347,7 @@ static int walk_enqueue(nd_sampler *s, int mode) {
         ts = s->side;
       }
       nd_phase_begin(s, ND_PHASE_TAIL);
-      const int tgrid = s->dev.sms * walk_min_ctas_sp<ND_APP_PPR>();   // resident CTAs; the lanes draw their pairs from a counter
+      const int tgrid = s->dev.sms * TAIL_CTAS;   // resident CTAs; the lanes draw their pairs from a counter
       int32_t *next_pair = s->d_nlive + steps + 2;
       if (tail_direct)
         walk_tail_kernel<ND_APP_PPR, true><<<tgrid, 256, 0, ts>>>(nd_view(s->g), wp, tp_steps, s->first, in_rec, s->d_nlive + tp_steps, next_pair,
@@ -1926,6 +1381,17 @@ static int walk_enqueue(nd_sampler *s, int mode) {
 }
 
 int nd_walk_sample(nd_sampler *s, int mode) {
+  const bool loop = mode == ND_MODE_TRANSIT_PARALLEL_LB && step_loop(s);
+  s->live_is_ended = mode == ND_MODE_TRANSIT_PARALLEL_LB && !loop;
+  if (mode == ND_MODE_SAMPLE_PARALLEL || s->live_is_ended) {   // a lane per walk: one or two launches, nothing to capture
+    nd_phase_begin(s, ND_PHASE_NEXT);
+    const int rc = nd_walk_rows_launch(s, mode == ND_MODE_TRANSIT_PARALLEL_LB);
+    nd_phase_end(s);
+    return rc;
+  }
+  ND_TRY(tp_alloc(s));
+  if (loop) ND_TRY(loop_alloc(s));
+  if (s->map_stale) ND_TRY(nd_sampler_build_initial_map(s));
   // the count of walks that can start is waited for here, outside any stream capture, the first
   // time a step loop is laid out after the seeds were set
   if (s->h_active && s->active_starts < 0 && s->active_done) {

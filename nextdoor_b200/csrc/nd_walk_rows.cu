@@ -1,0 +1,835 @@
+// Random walks, a lane per walk: the kernels of the sample-parallel mode (sampleParallelKernel,
+// src/nextdoor.cu:1348-1518) and of the load-balanced mode.  The draws are keyed by (sample, step), so every
+// organisation of a job gives the same samples, and on B200 a lane that keeps its walk in registers beats a
+// step-by-step pass over a transit-sorted map at every number of walks (measured, transit-parallel loop with
+// counting inversion -> this file: uniform walk on 57 K vertices 1.10 -> 0.07 ms, DeepWalk on 2^20 vertices
+// 5.2 -> 1.6 ms, node2vec 7.6 -> 2.3 ms, PPR on 2^24 vertices 5.4 -> 2.5 ms).
+//
+// What bounds it.  Large graphs: the rate of random DRAM reads.  A walker picks every CSR entry with the same
+// probability, the entry arrays do not fit the L2, and a gather of 4 or 8 bytes costs a 64-byte DRAM read; the
+// kernels run at 4.1-5.0 TB/s of such reads (58-66 % of the pins; streaming copies reach 6.5).  So what
+// counts is the number of gathers that miss, hence: one try per round for the weighted apps (no speculation),
+// the weights as one byte per entry where that array has a chance to stay in the L2, the first stop draw of
+// a step made before the vertex is fetched, a filter in front of node2vec's sets, rows written once, in
+// 32-byte sectors.  Small graphs: the chain of dependent L2 reads of a walk, two per step, one where the
+// entries carry the neighbour's row.
+#include <mutex>
+
+#include "nd_common.cuh"
+#include "nd_nbrset.cuh"
+#include "nd_philox.cuh"
+#include "nd_walk_rows.cuh"
+
+namespace {
+
+constexpr int ROWS_THREADS = 128;
+// CTAs per SM: 1536 lanes at 40 registers.  Measured on DeepWalk, 2^20 vertices: 8 -> 1.95, 12 -> 1.63,
+// 14 -> 1.81, 16 -> 1.90 ms; two walks per lane at half the lanes 2.0 ms (fewer L1 hits, longer tail).
+constexpr int ROWS_CTAS = 12;
+constexpr int RETRY_CAP = 1 << 16;
+constexpr int32_t AGAIN = -2;   // the round ended without an accepted vertex
+
+struct RowsArgs {
+  int32_t V;
+  const int32_t *__restrict__ row_ptr;
+  const int32_t *__restrict__ col;
+  const float *__restrict__ w;
+  const float *__restrict__ max_w;
+  const int2 *__restrict__ vrow;     // [V] (row start, degree)
+  const int4 *__restrict__ vrec4;    // [V] (row start, degree, max weight bits, 0)
+  const int4 *__restrict__ erec;     // [E] (neighbour, its row start, its degree, 0)
+  const int2 *__restrict__ colw;     // [E] (neighbour, weight bits)
+  const int2 *__restrict__ vrec;     // [V+1] (row start, max weight bits)
+  const uint8_t *__restrict__ wq;    // [E] weights as 256ths of the row's maximum, rounded down
+  const int32_t *__restrict__ adjset;
+  const uint32_t *__restrict__ adjsign;
+  uint64_t seed;
+  float p, q, stop_prob;
+  int n2v_compat, steps;
+  int64_t first_sample, S;
+  const int32_t *__restrict__ initial;
+  int32_t *__restrict__ out;
+  int32_t *__restrict__ plen;
+  int4 *__restrict__ list;                  // walks that can start: (sample, row start, degree, max weight bits or vertex); null: all walks, in order
+  // Counters of the running job, zero between jobs: [0..7] as published, [8] walks handed out beyond the first
+  // round, [9] entries of the list, [10] CTAs that are done; the last CTA publishes them and clears them again,
+  // so a job needs no launch for that and can be replayed from a graph.
+  unsigned long long *__restrict__ acc;
+  uint32_t *__restrict__ ended;             // [steps] walks that ended after k vertices, or null
+  unsigned long long *__restrict__ stats;   // published counters [8]
+  uint32_t *__restrict__ ended_out;         // published histogram
+  int *__restrict__ status;
+};
+
+template <int APP>
+__host__ __device__ constexpr bool weighted() { return APP == ND_APP_DEEPWALK || APP == ND_APP_PPR; }
+
+// Layouts.  ALT: uniform walk: entries that carry the neighbour's row; weighted walks: one byte per weight.
+enum : int { LAYOUT_PLAIN = 0, LAYOUT_ALT = 1 };
+
+// ---- loads.  The small per-vertex and per-entry arrays ask to stay in the L2; a weighted walk's neighbour
+// ids bypass the L1, which then serves the bytes and vertex records of the hubs (DeepWalk 1.80 -> 1.63 ms;
+// the uniform walk and node2vec are slower that way: 0.94 -> 1.21, 2.32 -> 2.50 ms).
+struct Hot {
+  uint64_t pol;
+  __device__ __forceinline__ Hot() { asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol)); }
+  __device__ __forceinline__ int32_t ld(const int32_t *p) const { int32_t v; asm("ld.global.nc.L2::cache_hint.s32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol)); return v; }
+  __device__ __forceinline__ uint32_t ld(const uint8_t *p) const { uint32_t v; asm("ld.global.nc.L2::cache_hint.u8 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol)); return v; }
+  __device__ __forceinline__ int2 ld(const int2 *p) const { int2 v; asm("ld.global.nc.L2::cache_hint.v2.s32 {%0, %1}, [%2], %3;" : "=r"(v.x), "=r"(v.y) : "l"(p), "l"(pol)); return v; }
+  __device__ __forceinline__ int4 ld(const int4 *p) const { int4 v; asm("ld.global.nc.L2::cache_hint.v4.s32 {%0, %1, %2, %3}, [%4], %5;" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(pol)); return v; }
+};
+__device__ __forceinline__ int32_t ld_once(const int32_t *p) { int32_t v; asm("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
+__device__ __forceinline__ int2 ld_once(const int2 *p) { int2 v; asm("ld.global.nc.L1::no_allocate.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p)); return v; }
+
+// ---- rows of the result
+//
+// Vertices are collected in shared memory and go out in aligned pieces: slot j of thread t at [j * threads + t],
+// so every access of a warp is free of bank conflicts.  64-byte pieces for the walks that run their full
+// length (a dirty half of a 64-byte DRAM unit costs as much as the whole: DeepWalk 1.84 -> 1.77 ms against
+// 32-byte pieces), 32-byte pieces for PPR, whose rows hold a few vertices.
+template <int APP>
+__host__ __device__ constexpr int piece() { return APP == ND_APP_PPR ? 8 : 16; }   // vertices
+template <int PIECE>
+__device__ __forceinline__ int piece_slot(const RowsArgs &a, uint32_t s, int step) { return (int)(((int64_t)s * a.steps + step) & (PIECE - 1)); }
+
+// The piece that holds the p vertices before slot n of the row goes out.  Slots behind the walk hold the
+// invalid id, so a sector that lies inside the row is written whole (one that is written in part costs the
+// memory a read of it).  Returns the first slot behind those written.
+template <int PIECE>
+__device__ __forceinline__ int piece_out(const RowsArgs &a, const int32_t *buf, uint32_t s, int n, int p) {
+  int32_t *row = a.out + (int64_t)s * a.steps;
+  int written = n;
+#pragma unroll
+  for (int q = 0; q < PIECE; q += 8) {
+    const int at = n - p + q;   // slot of the row the sector begins at
+    if (q < p) {
+      if (at >= 0 && at + 8 <= a.steps) {
+        int32_t v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = q + j < p ? buf[(q + j) * ROWS_THREADS + threadIdx.x] : a.V;
+        asm volatile("st.global.L2::evict_first.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(row + at), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                     "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                     : "memory");
+        written = at + 8 > written ? at + 8 : written;
+      } else {
+        for (int j = at < 0 ? -at : 0; j < 8 && q + j < p; j++) row[at + j] = buf[(q + j) * ROWS_THREADS + threadIdx.x];
+      }
+    }
+  }
+  return written;
+}
+
+// What the CTA's walks add up to, and how a walk ends.
+template <int PIECE>
+struct Rows {
+  int32_t *buf;
+  uint32_t *ended;     // histogram of the CTA's walks that ended early, by their vertices
+  unsigned int *sum;   // [0] vertices, [1] walks that ended early
+  __device__ __forceinline__ Rows(const RowsArgs &a, unsigned int *sums) {
+    extern __shared__ int32_t sh_dyn[];
+    buf = sh_dyn;
+    ended = reinterpret_cast<uint32_t *>(sh_dyn + PIECE * ROWS_THREADS);
+    sum = sums;
+    if (threadIdx.x < 2) sum[threadIdx.x] = 0u;
+    if (a.ended) for (int k = threadIdx.x; k < a.steps; k += ROWS_THREADS) ended[k] = 0u;
+    __syncthreads();
+  }
+  __device__ __forceinline__ void put(const RowsArgs &a, uint32_t s, int step, int32_t v) {
+    const int p = piece_slot<PIECE>(a, s, step);
+    buf[p * ROWS_THREADS + threadIdx.x] = v;
+    if (p == PIECE - 1) piece_out<PIECE>(a, buf, s, step + 1, PIECE);
+  }
+  // the walk has ended with n vertices: its open piece, and the slots the row's previous walk filled beyond them
+  __device__ __forceinline__ void end(const RowsArgs &a, uint32_t s, int n, bool counts) {
+    const int p = piece_slot<PIECE>(a, s, n);
+    const int written = p ? piece_out<PIECE>(a, buf, s, n, p) : n;
+    const int32_t had = a.plen[s];
+    for (int j = written; j < had; j++) a.out[(int64_t)s * a.steps + j] = a.V;
+    if (had != n) a.plen[s] = n;
+    if (n) atomicAdd(&sum[0], (unsigned int)n);
+    if (counts && n < a.steps) {
+      atomicAdd(&sum[1], 1u);
+      if (a.ended) atomicAdd(&ended[n], 1u);
+    }
+  }
+  // the whole CTA, at its end; `tries` and `words` of every thread go to counters `tries_at` and 4
+  __device__ __forceinline__ void out(const RowsArgs &a, uint32_t tries, int tries_at, uint32_t words) {
+    __shared__ int last;
+    for (int o = 16; o > 0; o >>= 1) {
+      tries += __shfl_xor_sync(0xffffffffu, tries, o);
+      words += __shfl_xor_sync(0xffffffffu, words, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+      if (tries) atomicAdd(&a.acc[tries_at], (unsigned long long)tries);
+      if (words) atomicAdd(&a.acc[4], (unsigned long long)words);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && sum[0] + sum[1]) {
+      atomicAdd(&a.acc[0], (unsigned long long)sum[0]);
+      atomicAdd(&a.acc[1], (unsigned long long)sum[0] + sum[1]);
+    }
+    if (a.ended)
+      for (int k = threadIdx.x; k < a.steps; k += ROWS_THREADS)
+        if (ended[k]) atomicAdd(&a.ended[k], ended[k]);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&a.acc[10], 1ull) == (unsigned long long)gridDim.x - 1ull;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (threadIdx.x < 8) a.stats[threadIdx.x] = __ldcg(&a.acc[threadIdx.x]);
+    if (a.ended)
+      for (int k = threadIdx.x; k < a.steps; k += ROWS_THREADS) {
+        a.ended_out[k] = __ldcg(&a.ended[k]);
+        a.ended[k] = 0u;
+      }
+    __syncthreads();
+    if (threadIdx.x < 11) a.acc[threadIdx.x] = 0ull;
+  }
+};
+
+__device__ __forceinline__ void draw_block(const RowsArgs &a, uint32_t s, int step, uint32_t block, uint32_t (&o)[4]) {
+  ndrng::philox4x32_10((uint32_t)(a.first_sample + s), (uint32_t)step, 0u, block, (uint32_t)a.seed, (uint32_t)(a.seed >> 32), o);
+}
+__device__ __forceinline__ int32_t draw_index(uint32_t u, int32_t n) { return ndrng::rand_int_from(ndrng::u32_to_uniform(u), n); }
+
+// ---- which walks a lane takes
+//
+// A job with more walks than there are lanes starts from a list of the walks that can start (on the R-MAT
+// graphs 40-47 % of the vertices have no neighbours, and a lane without a walk reads nothing); the first
+// walks of a lane follow from its place, the next ones are handed out to its warp 64 at a time.  A job whose
+// walks all have a lane takes them in order, without the pass that makes the list.
+constexpr int START_PER_THREAD = 4;
+template <int APP>
+__global__ void __launch_bounds__(256) walk_start_kernel(const RowsArgs a) {
+  __shared__ uint32_t sh_n, sh_dead;
+  __shared__ unsigned long long sh_base;
+  if (threadIdx.x == 0) { sh_n = 0u; sh_dead = 0u; }
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const int64_t first = (int64_t)blockIdx.x * 256 * START_PER_THREAD + threadIdx.x;
+  int4 e[START_PER_THREAD];
+  int32_t t[START_PER_THREAD], had[START_PER_THREAD];
+#pragma unroll
+  for (int j = 0; j < START_PER_THREAD; j++) {
+    const int64_t s = first + j * 256;
+    t[j] = s < a.S ? a.initial[s] : -1;
+    had[j] = s < a.S ? a.plen[s] : 0;
+  }
+  uint32_t at[START_PER_THREAD], dead = 0;
+#pragma unroll
+  for (int j = 0; j < START_PER_THREAD; j++) {
+    const int64_t s = first + j * 256;
+    const bool valid = t[j] >= 0 && t[j] < a.V;
+    const int32_t rs = valid ? __ldg(a.row_ptr + t[j]) : 0, deg = valid ? __ldg(a.row_ptr + t[j] + 1) - rs : 0;
+    bool active = deg > 0;
+    if (APP == ND_APP_PPR && active) {   // the stop draw does not depend on the vertex
+      uint32_t o[4];
+      draw_block(a, (uint32_t)s, 0, 0u, o);
+      active = !(ndrng::u32_to_uniform(o[0]) < a.stop_prob);
+    }
+    e[j] = make_int4((int)(uint32_t)s, rs, active ? deg : 0, weighted<APP>() ? (active ? __float_as_int(__ldg(a.max_w + t[j])) : 0) : t[j]);
+    if (!active) {
+      for (int k = 0; k < had[j]; k++) a.out[s * a.steps + k] = a.V;
+      if (had[j]) a.plen[s] = 0;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, active);
+    dead += __popc(__ballot_sync(0xffffffffu, valid && !active));
+    uint32_t base = 0;
+    if (lane == 0 && m) base = atomicAdd(&sh_n, (uint32_t)__popc(m));
+    at[j] = __shfl_sync(0xffffffffu, base, 0) + __popc(m & ((1u << lane) - 1u));
+  }
+  if (lane == 0 && dead) atomicAdd(&sh_dead, dead);
+  __syncthreads();
+  if (threadIdx.x == 0) {   // one atomic per CTA and counter: with one per warp this pass took 0.43 instead of 0.13 ms on 2^24 walks
+    sh_base = sh_n ? atomicAdd(&a.acc[9], (unsigned long long)sh_n) : 0ull;
+    if (sh_dead) {
+      atomicAdd(&a.acc[1], (unsigned long long)sh_dead);
+      if (a.ended) atomicAdd(&a.ended[0], sh_dead);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < START_PER_THREAD; j++)
+    if (e[j].z > 0) a.list[sh_base + at[j]] = e[j];
+}
+
+// (row start, degree, max weight bits or vertex) of a vertex
+template <int APP, int LAYOUT>
+__device__ __forceinline__ int4 vertex_of(const RowsArgs &a, const Hot &hot, int32_t v) {
+  if (weighted<APP>()) {
+    if (LAYOUT == LAYOUT_ALT) return hot.ld(a.vrec4 + v);
+    const int2 r = hot.ld(a.vrec + v), n = hot.ld(a.vrec + v + 1);
+    return make_int4(r.x, n.x - r.x, r.y, 0);
+  }
+  const int2 r = hot.ld(a.vrow + v);
+  return make_int4(r.x, r.y, v, 0);
+}
+
+// walk i of the job as (sample, row start, degree, max weight bits or vertex); degree -1: the seed is not a vertex
+template <int APP, int LAYOUT>
+__device__ __forceinline__ int4 walk_of(const RowsArgs &a, const Hot &hot, int64_t i) {
+  if (a.list) return a.list[i];
+  const int32_t t = a.initial[i];
+  if (t < 0 || t >= a.V) return make_int4((int)(uint32_t)i, 0, -1, 0);
+  const int4 v = vertex_of<APP, LAYOUT>(a, hot, t);
+  return make_int4((int)(uint32_t)i, v.x, v.y, v.z);
+}
+
+struct Taker {
+  int64_t n, lanes, cur, end;
+  __device__ __forceinline__ explicit Taker(const RowsArgs &a)
+      : n(a.list ? (int64_t)a.acc[9] : a.S), lanes((int64_t)gridDim.x * ROWS_THREADS), cur(0), end(0) {}
+  __device__ __forceinline__ int64_t first() const { return (int64_t)blockIdx.x * ROWS_THREADS + threadIdx.x; }
+  // the next walk of every lane that wants one (n or more: none left); the whole warp calls it
+  __device__ __forceinline__ int64_t next(const RowsArgs &a, unsigned want) {
+    const int lane = threadIdx.x & 31;
+    const int need = __popc(want), my = __popc(want & ((1u << lane) - 1u));
+    const int64_t avail = end - cur;
+    int64_t i = cur + my;
+    if (need <= avail) {
+      cur += need;
+    } else {
+      unsigned long long nb = (unsigned long long)n;
+      if (n > lanes) {
+        if (lane == 0) nb = (unsigned long long)lanes + atomicAdd(&a.acc[8], 64ull);
+        nb = __shfl_sync(0xffffffffu, nb, 0);
+      }
+      if (my >= avail) i = (int64_t)nb + (my - avail);
+      cur = (int64_t)nb + (need - avail);
+      end = (int64_t)nb + 64;
+    }
+    return i;
+  }
+};
+
+// ---------------------------------------------------------------- uniform walk (example/uniformRandWalk.cu:27-37)
+//
+// The lanes of a warp go in step.  The draw of the next step does not depend on the vertex: it is made while
+// the gather is in flight, so that a step is its dependent reads and little else.  Equal waves: with w waves
+// of lanes every wave takes n / w walks, or the last one would run a fraction of the lanes for as long.
+template <int LAYOUT>
+__device__ __forceinline__ void uniform_walks(const RowsArgs &a) {
+  constexpr bool FAT = LAYOUT == LAYOUT_ALT;
+  constexpr int PIECE = piece<ND_APP_UNIFORM_WALK>();
+  __shared__ unsigned int sums[2];
+  Rows<PIECE> rows(a, sums);
+  const Hot hot;
+  const Taker take(a);
+  const int64_t waves = (take.n + take.lanes - 1) / take.lanes, per = waves ? (take.n + waves - 1) / waves : 0;
+  for (int64_t wave = 0; wave < waves; wave++) {
+    const int64_t w0 = wave * per, wn = take.n - w0 < per ? take.n - w0 : per;
+    if (take.first() >= wn) continue;
+    const int4 e = walk_of<ND_APP_UNIFORM_WALK, LAYOUT>(a, hot, w0 + take.first());
+    const uint32_t s = (uint32_t)e.x;
+    int32_t rs = e.y, deg = e.z;
+    uint32_t u[4];
+    draw_block(a, s, 0, 0u, u);
+    if (deg <= 0) rows.end(a, s, 0, deg == 0);
+    for (int step = 0; deg > 0; step++) {
+      const int32_t x = draw_index(u[0], deg);
+      int32_t v;
+      int2 r = make_int2(0, 0);
+      if (FAT) {
+        const int4 f = hot.ld(a.erec + rs + x);
+        draw_block(a, s, step + 1, 0u, u);
+        v = f.x; r = make_int2(f.y, f.z);
+      } else {
+        v = __ldg(a.col + rs + x);
+        draw_block(a, s, step + 1, 0u, u);
+        if (step + 1 < a.steps) r = hot.ld(a.vrow + v);
+      }
+      rows.put(a, s, step, v);
+      rs = r.x;
+      deg = step + 1 < a.steps ? r.y : 0;
+      if (deg <= 0) rows.end(a, s, step + 1, true);
+    }
+  }
+  rows.out(a, 0u, 2, 0u);
+}
+
+// ---------------------------------------------------------------- weighted walks (randomWalks.cu:65-124)
+//
+// A lane is a state machine: a trip of the loop is one try {x = rand_int(n); y = u * max_w; accept unless
+// y > w[x]} wherever the lane's walk stands, a lane whose try was rejected stays on its step, a lane whose
+// walk ended takes the next one, and the vote at the loop head is where the warp meets again.  Draws of a
+// step: PPR's stop draw, then two per try; a block of four is made once and kept (k0..k2).
+// PPR makes the stop draw of a step before it fetches the vertex, which a walk that stops never needs.
+//
+// Weights.  PLAIN: (id, weight) records, one gather per try.  ALT: the row's weights as whole 256ths of its
+// maximum, rounded down (a byte per entry): b/256 <= w/max < (b+1)/256 decides all but one try in 256 --
+// those read the weight -- and the id is gathered once per step.  Same decisions, as b * (max/256) and
+// (b+1) * (max/256), rounded as the kernel rounds them, were compared with w when b was chosen.  ALT moves
+// fewer DRAM reads while the bytes have a chance to stay in the L2 (WQ_ENTRIES): DeepWalk on 33.5 M entries
+// 1.99 -> 1.63 ms, but a byte array that is itself read from DRAM is one more read per step.
+template <int APP, int LAYOUT>
+__device__ __forceinline__ void weighted_walks(const RowsArgs &a) {
+  constexpr bool PPR = APP == ND_APP_PPR;
+  __shared__ unsigned int sums[2];
+  Rows<piece<APP>()> rows(a, sums);
+  const Hot hot;
+  Taker take(a);
+  uint32_t s = 0, k0 = 0, k1 = 0, k2 = 0, tries = 0;
+  // cur: the vertex the walk has moved to, its record not fetched yet; -1: (rs, deg, mw) are those of the walk's vertex
+  int32_t rs = 0, deg = 0, mw = 0, cur = -1;
+  int step = -1, t = 0;   // step -1: no walk; t: tries of this step so far
+  if (take.first() < take.n) {
+    const int4 e = walk_of<APP, LAYOUT>(a, hot, take.first());
+    s = (uint32_t)e.x; rs = e.y; deg = e.z; mw = e.w; step = 0;
+  }
+  while (__any_sync(0xffffffffu, step >= 0)) {
+    const bool odd = (t & 1) != 0;
+    uint32_t dx = PPR && odd ? k2 : k0, dy = k1;
+    bool over = step == a.steps || (cur < 0 && deg <= 0);
+    if (PPR ? (odd || t == 0) : !odd) {
+      uint32_t o[4];
+      draw_block(a, s, step, (uint32_t)(PPR ? (t + 1) >> 1 : t >> 1), o);
+      if (PPR) {
+        if (odd) { dy = o[0]; } else { dx = o[1]; dy = o[2]; over |= ndrng::u32_to_uniform(o[0]) < a.stop_prob; }
+        k0 = o[1]; k1 = o[2]; k2 = o[3];
+      } else {
+        dx = o[0]; dy = o[1]; k0 = o[2]; k1 = o[3];
+      }
+    }
+    over = over && step >= 0;
+    if (cur >= 0 && !over) {
+      const int4 r = vertex_of<APP, LAYOUT>(a, hot, cur);
+      rs = r.x; deg = r.y; mw = r.z;
+      cur = -1;
+    }
+    const unsigned want = __ballot_sync(0xffffffffu, over);
+    if (want) {
+      const int64_t i = take.next(a, want);
+      if (over) {
+        rows.end(a, s, step, deg >= 0);
+        step = -1; deg = 0; cur = -1; t = 0;
+        if (i < take.n) {
+          const int4 e = walk_of<APP, LAYOUT>(a, hot, i);
+          s = (uint32_t)e.x; rs = e.y; deg = e.z; mw = e.w; step = 0;
+        }
+      }
+    }
+    if (deg <= 0 || over) continue;   // no walk, a vertex without neighbours, or a walk just taken: it starts in the next trip
+    const float max_w = __int_as_float(mw);
+    const int32_t x = draw_index(dx, deg);
+    const float y = __fmul_rn(ndrng::u32_to_uniform(dy), max_w);
+    int32_t nbr = AGAIN;
+    if (LAYOUT == LAYOUT_ALT) {
+      const uint32_t b = hot.ld(a.wq + rs + x);
+      const float unit = __fmul_rn(max_w, 0.00390625f);
+      const float lo = __fmul_rn(__uint2float_rn(b), unit), hi = __fmul_rn(__uint2float_rn(b + 1u), unit);
+      bool accept = deg == 1 || (b > 0u && y <= lo);
+      if (!accept && !(b < 255u && y > hi)) accept = !(y > __ldg(a.w + rs + x));
+      if (accept) nbr = ld_once(a.col + rs + x);
+    } else {
+      const int2 r = ld_once(a.colw + rs + x);
+      if (deg == 1 || !(y > __int_as_float(r.y))) nbr = r.x;
+    }
+    tries += deg > 1 ? 1u : 0u;
+    if (nbr == AGAIN && ++t > RETRY_CAP) {
+      atomicOr(a.status, ND_DEV_RETRY_LIMIT);
+      nbr = __ldg(a.col + rs);
+    }
+    if (nbr >= 0) {
+      rows.put(a, s, step, nbr);
+      step++;
+      t = 0;
+      cur = nbr;
+    }
+  }
+  rows.out(a, tries, 2, 0u);
+}
+
+// ---------------------------------------------------------------- node2vec (randomWalks.cu:141-172)
+//
+// A candidate that is not the previous vertex t is accepted when y < 1/q (neighbour of t) or y < 1 (not a
+// neighbour): below `lo` the membership does not matter, at or above `hi` neither; below `sure` nothing
+// about the candidate matters.
+struct N2vConsts {
+  float inv_q, bound, lo, hi, sure;
+  __device__ __forceinline__ N2vConsts(float p, float q) {
+    inv_q = __fdiv_rn(1.0f, q);
+    bound = p > inv_q ? p : inv_q;
+    if (bound < 1.0f) bound = 1.0f;
+    lo = inv_q < 1.0f ? inv_q : 1.0f;
+    hi = inv_q < 1.0f ? 1.0f : inv_q;
+    sure = lo < p ? lo : p;
+  }
+};
+
+// v in the list [ts, ts + tn), exactly; `words` counts the 4-byte words read
+__device__ __forceinline__ bool member_exact(const RowsArgs &a, int32_t ts, int32_t tn, int32_t v, uint32_t hash, uint32_t &words) {
+  if (tn < SET_MIN_DEG) {
+    bool found = false;
+#pragma unroll
+    for (int k = 0; k < SET_MIN_DEG - 1; k++) found |= (k < tn ? __ldg(a.col + ts + k) : -1) == v;
+    words += tn;
+    return found;
+  }
+  const uint32_t n_buckets = ((uint32_t)(ts + tn) >> 2) - ((uint32_t)ts >> 2);
+  const int4 *region = reinterpret_cast<const int4 *>(a.adjset) + 2 * (size_t)((uint32_t)ts >> 2);
+  uint32_t b = set_bucket_of_hash(hash, n_buckets);
+  for (uint32_t it = 0; it < n_buckets; it++) {
+    const int4 c = __ldg(region + 2 * (size_t)b), d = __ldg(region + 2 * (size_t)b + 1);
+    words += 8;
+    if (c.x == v || c.y == v || c.z == v || c.w == v || d.x == v || d.y == v || d.z == v || d.w == v) return true;
+    if (d.w == SET_EMPTY) return false;   // slots fill front to back inside a bucket
+    b = b + 1 < n_buckets ? b + 1 : 0;
+  }
+  return false;
+}
+
+// The same state machine; a trip is a round of two tries (one block of draws).  The round ends at the first
+// try that is sure to accept, so the second candidate is fetched for nothing only when the first one's
+// membership accepts it (one try per round: 2.32 -> 2.6 ms).  A membership test asks the filter first: a word
+// of 8 bits per neighbour answers about 95 % of the tests that fail (88 % of all), the rest read the set
+// (without the filter 2.9 ms).
+__device__ __forceinline__ void n2v_walks(const RowsArgs &a) {
+  constexpr int APP = ND_APP_NODE2VEC;
+  constexpr int TRIES = 2;
+  __shared__ unsigned int sums[2];
+  Rows<piece<APP>()> rows(a, sums);
+  const Hot hot;
+  const N2vConsts c(a.p, a.q);
+  Taker take(a);
+  uint32_t s = 0, tries = 0, words = 0;
+  int32_t rs = 0, deg = 0, cur = 0, prev = 0, ts = 0, tn = 0;   // [ts, ts + tn): the row of the previous vertex
+  int step = -1, round = 0;
+  if (take.first() < take.n) {
+    const int4 e = walk_of<APP, LAYOUT_PLAIN>(a, hot, take.first());
+    s = (uint32_t)e.x; rs = e.y; deg = e.z; cur = e.w; step = 0;
+  }
+  while (__any_sync(0xffffffffu, step >= 0)) {
+    int32_t nbr = AGAIN;
+    const bool over0 = step >= 0 && deg <= 0;
+    if (step >= 0 && !over0) {
+      uint32_t o[4];
+      draw_block(a, s, step, (uint32_t)round, o);
+      int32_t x[TRIES], v[TRIES];
+      float y[TRIES];
+      int n_try = TRIES;
+#pragma unroll
+      for (int j = 0; j < TRIES; j++) {
+        x[j] = draw_index(o[2 * j], deg);
+        y[j] = __fmul_rn(ndrng::u32_to_uniform(o[2 * j + 1]), c.bound);
+      }
+      const bool simple = deg == 1 || step == 0;
+      if (simple) x[0] = 0;
+#pragma unroll
+      for (int j = TRIES - 1; j >= 0; j--) if (y[j] < c.sure) n_try = j + 1;
+      if (simple) n_try = 1;
+#pragma unroll
+      for (int j = 0; j < TRIES; j++) v[j] = j < n_try ? __ldg(a.col + rs + x[j]) : -1;
+      const uint32_t w0 = (uint32_t)ts >> 2, n_words = ((uint32_t)(ts + tn) >> 2) - w0;
+      bool is_ret[TRIES], need[TRIES];
+      uint32_t h[TRIES], word[TRIES];
+#pragma unroll
+      for (int j = 0; j < TRIES; j++) {
+        is_ret[j] = a.n2v_compat ? (x[j] == prev) : (v[j] == prev);   // randomWalks.cu:159 compares the index
+        need[j] = !simple && j < n_try && !is_ret[j] && y[j] >= c.lo && y[j] < c.hi;
+        h[j] = set_mix((uint32_t)v[j]);
+        word[j] = 0xffffffffu;
+        if (need[j] && tn >= SET_MIN_DEG) word[j] = (uint32_t)hot.ld(reinterpret_cast<const int32_t *>(a.adjsign) + w0 + set_bucket_of_hash(h[j], n_words));
+      }
+      if (simple) {
+        nbr = v[0];
+      } else {
+#pragma unroll
+        for (int j = 0; j < TRIES; j++) {
+          if (nbr == AGAIN && j < n_try) {
+            tries++;
+            bool accept;
+            if (is_ret[j]) {
+              accept = y[j] < a.p;
+            } else if (!need[j]) {
+              accept = y[j] < c.lo;
+            } else {
+              const uint32_t sign = set_sign(h[j]);
+              words += tn >= SET_MIN_DEG ? 1u : 0u;
+              const bool found = (word[j] & sign) == sign && member_exact(a, ts, tn, v[j], h[j], words);
+              accept = y[j] < (found ? c.inv_q : 1.0f);
+            }
+            if (accept) nbr = v[j];
+          }
+        }
+        round++;
+        if (nbr == AGAIN && TRIES * round > RETRY_CAP) {
+          atomicOr(a.status, ND_DEV_RETRY_LIMIT);
+          nbr = __ldg(a.col + rs);
+        }
+      }
+    }
+    const bool moved = nbr >= 0, over = over0 || (moved && step + 1 == a.steps);
+    int4 next = make_int4(0, 0, 0, 0);   // the new vertex, or the next walk (w: there is one)
+    uint32_t s_next = 0;
+    if (moved && !over) next = vertex_of<APP, LAYOUT_PLAIN>(a, hot, nbr);
+    const unsigned want = __ballot_sync(0xffffffffu, over);
+    if (want) {
+      const int64_t i = take.next(a, want);
+      if (over && i < take.n) {
+        const int4 e = walk_of<APP, LAYOUT_PLAIN>(a, hot, i);
+        next = make_int4(e.y, e.z, e.w, 1);
+        s_next = (uint32_t)e.x;
+      }
+    }
+    if (moved) {
+      rows.put(a, s, step, nbr);
+      step++;
+    }
+    if (over) {
+      rows.end(a, s, step, deg >= 0);
+      s = s_next;
+      step = next.w ? 0 : -1;
+    }
+    if (moved || over) {
+      prev = cur; ts = rs; tn = deg;
+      rs = next.x; deg = next.y; cur = next.z;
+      round = 0;
+    }
+  }
+  rows.out(a, tries, 3, words);
+}
+
+template <int APP, int LAYOUT>
+__device__ __forceinline__ void walks(const RowsArgs &a) {
+  if (APP == ND_APP_UNIFORM_WALK) uniform_walks<LAYOUT>(a);
+  else if (APP == ND_APP_NODE2VEC) n2v_walks(a);
+  else weighted_walks<APP, LAYOUT>(a);
+}
+
+// the sample-parallel mode
+template <int APP, int LAYOUT>
+__global__ void __launch_bounds__(ROWS_THREADS, ROWS_CTAS) walk_sp_kernel(const RowsArgs a) { walks<APP, LAYOUT>(a); }
+
+// the load-balanced mode: the same walks, and the walks that are alive at every step are counted
+template <int APP, int LAYOUT>
+__global__ void __launch_bounds__(ROWS_THREADS, ROWS_CTAS) walk_next_count_kernel(const RowsArgs a) { walks<APP, LAYOUT>(a); }
+
+// ---------------------------------------------------------------- layouts, built by a graph's first sampler that reads them
+
+// source row of the CSR entry e, which lies in the rows [lo, hi)
+__device__ __forceinline__ int32_t row_of_entry(const int32_t *__restrict__ row_ptr, int32_t lo, int32_t hi, int64_t e) {
+  while (hi - lo > 1) {
+    const int32_t mid = lo + ((hi - lo) >> 1);
+    if ((int64_t)row_ptr[mid] <= e) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
+// f(entry, its row) for every entry.  A CTA takes BUILD_SPAN consecutive entries at a time: the rows of the
+// first and the last of them bound the search of all others.
+constexpr int BUILD_THREADS = 256, BUILD_SPAN = 2048;
+template <class F>
+__device__ __forceinline__ void for_entries(const int32_t *__restrict__ row_ptr, int32_t V, int64_t E, F f) {
+  __shared__ int32_t sh[2];
+  for (int64_t e0 = (int64_t)blockIdx.x * BUILD_SPAN; e0 < E; e0 += (int64_t)gridDim.x * BUILD_SPAN) {
+    const int64_t e1 = e0 + BUILD_SPAN < E ? e0 + BUILD_SPAN : E;
+    __syncthreads();
+    if (threadIdx.x < 2) sh[threadIdx.x] = row_of_entry(row_ptr, 0, V, threadIdx.x ? e1 - 1 : e0);
+    __syncthreads();
+    const int32_t lo = sh[0], hi = sh[1] + 1;
+    for (int64_t e = e0 + threadIdx.x; e < e1; e += BUILD_THREADS) f(e, row_of_entry(row_ptr, lo, hi, e));
+  }
+}
+
+__global__ void vrow_build_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int2 *__restrict__ vrow) {
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x)
+    vrow[v] = make_int2(row_ptr[v], row_ptr[v + 1] - row_ptr[v]);
+}
+
+__global__ void colw_build_kernel(const int32_t *__restrict__ col, const float *__restrict__ w, int64_t E, int2 *__restrict__ colw) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x)
+    colw[e] = make_int2(col[e], __float_as_int(w[e]));
+}
+
+__global__ void vrec_build_kernel(const int32_t *__restrict__ row_ptr, const float *__restrict__ max_w, int32_t V, int2 *__restrict__ vrec) {
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v <= V; v += (int64_t)gridDim.x * blockDim.x)
+    vrec[v] = make_int2(row_ptr[v], v < V ? __float_as_int(max_w[v]) : 0);
+}
+
+__global__ void vrec4_build_kernel(const int32_t *__restrict__ row_ptr, const float *__restrict__ max_w, int32_t V, int4 *__restrict__ vrec) {
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x)
+    vrec[v] = make_int4(row_ptr[v], row_ptr[v + 1] - row_ptr[v], __float_as_int(max_w[v]), 0);
+}
+
+__global__ void erec_build_kernel(const int32_t *__restrict__ col, const int32_t *__restrict__ row_ptr, int64_t E, int4 *__restrict__ erec) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t v = col[e], rs = row_ptr[v];
+    erec[e] = make_int4(v, rs, row_ptr[v + 1] - rs, 0);
+  }
+}
+
+__global__ void __launch_bounds__(BUILD_THREADS)
+wq_build_kernel(const int32_t *__restrict__ row_ptr, const float *__restrict__ max_w, const float *__restrict__ w, int32_t V, int64_t E,
+                uint8_t *__restrict__ wq) {
+  for_entries(row_ptr, V, E, [&](int64_t e, int32_t v) {
+    const float x = w[e], unit = __fmul_rn(max_w[v], 0.00390625f);
+    int b = 255;   // a weight that is not a number accepts every draw: decided by comparing with it
+    if (x == x) {
+      const float r = __fdiv_rn(x, unit);
+      b = r > 0.f ? (r < 255.f ? (int)r : 255) : 0;
+      while (b > 0 && !(__fmul_rn((float)b, unit) <= x)) b--;
+      while (b < 255 && __fmul_rn((float)(b + 1), unit) <= x) b++;
+    }
+    wq[e] = (uint8_t)b;
+  });
+}
+
+__global__ void __launch_bounds__(BUILD_THREADS)
+adjsign_build_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col, int32_t V, int64_t E, uint32_t *__restrict__ sign) {
+  for_entries(row_ptr, V, E, [&](int64_t e, int32_t t) {
+    const int32_t rs = row_ptr[t], deg = row_ptr[t + 1] - rs;
+    if (deg < SET_MIN_DEG) return;
+    const uint32_t w0 = (uint32_t)rs >> 2, n = ((uint32_t)(rs + deg) >> 2) - w0, h = set_mix((uint32_t)col[e]);
+    atomicOr(sign + w0 + set_bucket_of_hash(h, n), set_sign(h));
+  });
+}
+
+// insert every neighbour id into its row's set: first free slot at or after the home bucket
+__global__ void __launch_bounds__(BUILD_THREADS)
+adjset_build_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col, int32_t V, int64_t E, int32_t *__restrict__ adjset,
+                    int *__restrict__ status) {
+  for_entries(row_ptr, V, E, [&](int64_t e, int32_t t) {
+    const int32_t rs = row_ptr[t], deg = row_ptr[t + 1] - rs;
+    if (deg < SET_MIN_DEG) return;
+    const uint32_t n_buckets = ((uint32_t)(rs + deg) >> 2) - ((uint32_t)rs >> 2);
+    int32_t *region = adjset + 8 * (size_t)((uint32_t)rs >> 2);
+    const int32_t v = col[e];
+    uint32_t b = set_bucket(v, n_buckets);
+    bool done = false;
+    for (uint32_t it = 0; it < n_buckets && !done; it++) {
+      for (int i = 0; i < 8 && !done; i++) {
+        int32_t *slot = region + 8 * (size_t)b + i;
+        int32_t at = *(volatile int32_t *)slot;
+        if (at == SET_EMPTY) at = atomicCAS(slot, SET_EMPTY, v);
+        done = at == SET_EMPTY || at == v;  // placed, or the id is in the set already (repeated edge)
+      }
+      b = b + 1 < n_buckets ? b + 1 : 0;
+    }
+    if (!done) atomicOr(status, ND_DEV_RETRY_LIMIT);  // cannot happen: a region has at least deg slots
+  });
+}
+
+// Entries that carry the neighbour's row (16 bytes each) shorten a step to one dependent read; they pay while
+// the array stays in a die's half of the L2 with room to spare: 32 MB.
+constexpr int64_t ERECS = (int64_t)1 << 21;
+// The byte array of the weights: see weighted_walks.
+constexpr int64_t WQ_ENTRIES = (int64_t)1 << 26;
+
+bool alt_layout(const nd_sampler *s) {
+  if (s->p.app == ND_APP_UNIFORM_WALK) return s->g->E <= ERECS;
+  return (s->p.app == ND_APP_DEEPWALK || s->p.app == ND_APP_PPR) && s->g->E <= WQ_ENTRIES;
+}
+
+template <int APP, int LAYOUT>
+void launch(nd_sampler *s, RowsArgs &a, bool count) {
+  const int64_t ctas = (s->S + ROWS_THREADS - 1) / ROWS_THREADS, cap = (int64_t)s->dev.sms * ROWS_CTAS;
+  const int grid = (int)(ctas < cap ? ctas : cap);
+  const int smem = 4 * piece<APP>() * ROWS_THREADS + (count ? 4 * a.steps : 0);
+  if (ctas > cap) {   // more walks than lanes: start from the list
+    constexpr int per_cta = 256 * START_PER_THREAD;
+    walk_start_kernel<APP><<<(int)((s->S + per_cta - 1) / per_cta), 256, 0, s->stream>>>(a);
+    nd_count_launches(1);
+  } else {
+    a.list = nullptr;
+  }
+  if (count) walk_next_count_kernel<APP, LAYOUT><<<grid, ROWS_THREADS, smem, s->stream>>>(a);
+  else walk_sp_kernel<APP, LAYOUT><<<grid, ROWS_THREADS, smem, s->stream>>>(a);
+  nd_count_launches(1);
+}
+
+// The derived layouts of a graph are built by the first sampler that needs them; samplers of one
+// graph may be created from several host threads, so the builds are serialised.
+std::mutex g_derived_mutex;
+
+template <class T>
+int make(T *&p, size_t n) {
+  T *q = nullptr;
+  ND_CUDA(cudaMalloc(&q, sizeof(T) * n));
+  p = q;
+  return ND_OK;
+}
+
+// (neighbour id, weight) records and per-vertex (row start, maximum weight) records
+int ensure_colw(const nd_graph *g, int sms) {
+  if (g->colw || g->E == 0) return ND_OK;
+  int2 *cw = nullptr;
+  ND_TRY(make(cw, (size_t)g->E));
+  if (!g->vrec && make(g->vrec, (size_t)g->V + 1) != ND_OK) { cudaFree(cw); return ND_ERR_CUDA; }
+  colw_build_kernel<<<sms * 16, 256>>>(g->col, g->w, g->E, cw);
+  vrec_build_kernel<<<sms * 16, 256>>>(g->row_ptr, g->max_w, g->V, g->vrec);
+  ND_CUDA(cudaDeviceSynchronize());
+  g->colw = cw;
+  return ND_OK;
+}
+
+}  // namespace
+
+int nd_graph_ensure_colw(const nd_graph *g, int sms) {
+  std::lock_guard<std::mutex> lock(g_derived_mutex);
+  return ensure_colw(g, sms);
+}
+
+int nd_walk_rows_alloc(nd_sampler *s) {
+  const nd_graph *g = s->g;
+  const size_t V = (size_t)g->V, E = (size_t)(g->E > 0 ? g->E : 1);
+  const int grid = s->dev.sms * 16;
+  const int app = s->p.app;
+  if (s->S > (int64_t)s->dev.sms * ROWS_CTAS * ROWS_THREADS) ND_TRY(make(s->d_list, (size_t)s->S));
+  const size_t acc = 16 + ((size_t)s->p.steps + 1) / 2;
+  ND_TRY(make(s->d_rows_acc, acc));
+  ND_CUDA(cudaMemset(s->d_rows_acc, 0, 8 * acc));
+  std::lock_guard<std::mutex> lock(g_derived_mutex);
+  if (app == ND_APP_DEEPWALK || app == ND_APP_PPR) {
+    if (!alt_layout(s)) return ensure_colw(g, s->dev.sms);
+    if (!g->wq) {
+      ND_TRY(make(g->vrec4, V));
+      vrec4_build_kernel<<<grid, 256>>>(g->row_ptr, g->max_w, g->V, g->vrec4);
+      ND_TRY(make(g->wq, E));
+      wq_build_kernel<<<grid, BUILD_THREADS>>>(g->row_ptr, g->max_w, g->w, g->V, g->E, g->wq);
+    }
+    ND_CUDA(cudaGetLastError());
+    return ND_OK;
+  }
+  if (!g->vrow) {
+    ND_TRY(make(g->vrow, V));
+    vrow_build_kernel<<<grid, 256>>>(g->row_ptr, g->V, g->vrow);
+  }
+  if (app == ND_APP_UNIFORM_WALK && alt_layout(s) && !g->erec) {
+    ND_TRY(make(g->erec, E));
+    erec_build_kernel<<<grid, 256>>>(g->col, g->row_ptr, g->E, g->erec);
+  }
+  if (app == ND_APP_NODE2VEC && !g->adjset) {   // 8 bytes per CSR entry, and one of filter
+    const size_t words = E / 4 + 2, slots = 8 * words;
+    ND_TRY(make(g->adjsign, words));
+    ND_CUDA(cudaMemset(g->adjsign, 0, 4 * words));
+    adjsign_build_kernel<<<grid, BUILD_THREADS>>>(g->row_ptr, g->col, g->V, g->E, g->adjsign);
+    int32_t *set = nullptr;
+    ND_TRY(make(set, slots));
+    ND_CUDA(cudaMemset(set, 0xff, sizeof(int32_t) * slots));
+    adjset_build_kernel<<<grid, BUILD_THREADS>>>(g->row_ptr, g->col, g->V, g->E, set, s->d_status);
+    ND_CUDA(cudaDeviceSynchronize());
+    const int st = *(volatile int *)s->h_status;
+    if (st) { cudaFree(set); ND_REQUIRE(false, ND_ERR_DEVICE, "neighbour-set construction failed (status %d)", st); }
+    g->adjset = set;
+  }
+  ND_CUDA(cudaGetLastError());
+  return ND_OK;
+}
+
+int nd_walk_rows_launch(nd_sampler *s, bool count) {
+  const nd_graph *g = s->g;
+  uint32_t *ended = count ? reinterpret_cast<uint32_t *>(s->d_rows_acc + 16) : nullptr;
+  RowsArgs a{g->V, g->row_ptr, g->col, g->w, g->max_w, g->vrow, g->vrec4, g->erec, g->colw, g->vrec, g->wq, g->adjset, g->adjsign,
+             s->p.seed, s->p.p, s->p.q, s->p.stop_prob, s->p.n2v_ref_compat, s->p.steps, s->first, s->S, s->d_initial, s->d_out,
+             s->d_plen, s->d_list, s->d_rows_acc, ended, s->d_stats, (uint32_t *)s->d_nlive, s->d_status};
+  const bool alt = alt_layout(s);
+  switch (s->p.app) {
+    case ND_APP_UNIFORM_WALK: if (alt) launch<ND_APP_UNIFORM_WALK, LAYOUT_ALT>(s, a, count); else launch<ND_APP_UNIFORM_WALK, LAYOUT_PLAIN>(s, a, count); break;
+    case ND_APP_DEEPWALK: if (alt) launch<ND_APP_DEEPWALK, LAYOUT_ALT>(s, a, count); else launch<ND_APP_DEEPWALK, LAYOUT_PLAIN>(s, a, count); break;
+    case ND_APP_PPR: if (alt) launch<ND_APP_PPR, LAYOUT_ALT>(s, a, count); else launch<ND_APP_PPR, LAYOUT_PLAIN>(s, a, count); break;
+    default: launch<ND_APP_NODE2VEC, LAYOUT_PLAIN>(s, a, count); break;
+  }
+  ND_CUDA(cudaGetLastError());
+  return ND_OK;
+}

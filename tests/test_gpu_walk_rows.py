@@ -1,0 +1,64 @@
+"""The lane-per-walk kernels (sample-parallel and load-balanced modes) where they can go wrong: rows that do not fill
+the pieces they are written in, jobs just below and above the number of resident lanes, weights whose byte code
+decides nothing, rows that shrink and grow between passes."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+LANES = 148 * 12 * 128          # resident lanes of one B200
+
+
+def _graph(nd, hg):
+    return nd.Graph.from_csr(hg.row_ptr, hg.col, hg.w, hg.max_w)
+
+
+@pytest.mark.parametrize("app", [0, 1, 2, 3])
+@pytest.mark.parametrize("steps", [1, 3, 7, 8, 9, 15, 16, 17, 24, 31, 100])
+def test_row_pieces(nd, ndo, small_graph, app, steps):
+    g = _graph(nd, small_graph)
+    S = 1003
+    rng = np.random.default_rng(steps)
+    pr = nd.app_params(app, steps=steps, seed=7, stop_prob=0.1)
+    s = nd.Sampler(g, pr, num_samples=S, first_sample=5)
+    for mode in (1, 2, 0, 1):
+        init = rng.integers(-1, small_graph.V, S).astype(np.int32)
+        s.set_initial(init)
+        s.sample(mode)
+        clean = np.where(init < 0, small_graph.V, init).astype(np.int32)
+        exp = ndo.sample(small_graph, ndo.make_params(app, steps=steps, seed=7, stop_prob=0.1), S, first=5, initial=clean)
+        assert np.array_equal(s.final_samples(), exp["out"]), mode
+        st = s.stats()
+        assert all(st[k] == exp["counters"][k] for k in ("sampled_edges", "live_pairs", "weight_tries", "n2v_tries")), mode
+        if mode == 1:
+            live = s.live_pairs()
+            n = (exp["out"] != small_graph.V).sum(axis=1)
+            assert live[0] == (init >= 0).sum() and all(live[k] == (n >= k).sum() for k in range(1, steps))
+
+
+@pytest.mark.parametrize("app", [0, 1, 2, 3])
+@pytest.mark.parametrize("S", [1, 31, LANES, LANES + 1, LANES + 4097])
+def test_job_sizes_around_the_resident_lanes(nd, ndo, small_graph, app, S):
+    g = _graph(nd, small_graph)
+    pr = nd.app_params(app, steps=5, seed=3, stop_prob=0.3)
+    s = nd.Sampler(g, pr, num_samples=S)
+    exp = ndo.sample(small_graph, ndo.make_params(app, steps=5, seed=3, stop_prob=0.3), S)
+    for _ in range(2):
+        s.sample(1)
+        assert np.array_equal(s.final_samples(), exp["out"])
+        assert s.stats()["live_pairs"] == exp["counters"]["live_pairs"]
+
+
+@pytest.mark.parametrize("kind", ["equal", "tiny", "zero", "spread", "steps"])
+def test_weights_at_the_edges_of_their_byte_code(nd, ndo, small_graph, kind):
+    rng = np.random.default_rng(1)
+    n = small_graph.E
+    w = {"equal": np.full(n, 3.0), "tiny": rng.random(n) * 1e-42, "zero": np.where(rng.random(n) < 0.7, 0.0, 2.0),
+         "spread": 10.0 ** rng.uniform(-6, 3, n), "steps": rng.integers(1, 257, n) / 256.0}[kind].astype(np.float32)
+    src = np.repeat(np.arange(small_graph.V, dtype=np.int32), small_graph.degree())
+    hg = ndo.csr_from_records(src, small_graph.col, w, V=small_graph.V)
+    pr = nd.app_params(1, steps=12, seed=11)
+    s = nd.Sampler(_graph(nd, hg), pr, num_samples=4000)
+    s.sample(1)
+    exp = ndo.sample(hg, ndo.make_params(1, steps=12, seed=11), 4000)
+    assert np.array_equal(s.final_samples(), exp["out"])
+    assert s.stats()["weight_tries"] == exp["counters"]["weight_tries"]
