@@ -153,7 +153,7 @@ def next_bytes(wl, st, mode):
             n *= k
             tot += n
         last_share = n / tot
-        return (16 if mode != 2 else 8) * pairs + 8 * edges + (8 * edges * (1 - last_share) if mode != 2 else 0)
+        return (16 if mode == 0 else 8) * pairs + 8 * edges + (8 * edges * (1 - last_share) if mode == 0 else 0)
     return (8 if app == 9 else 4) * st["union_ids"] + 8 * st["union_unique"] + 8 * edges
 
 

@@ -6,9 +6,11 @@
 #include <string.h>
 
 #include "nd_common.cuh"
+#include "nd_khop_rows.cuh"
 #include "nd_philox.cuh"
 
 #include <atomic>
+#include <mutex>
 
 static thread_local char g_err[512] = "";
 static std::atomic<long long> g_launches{0};
@@ -52,7 +54,51 @@ void nd_phase_end(nd_sampler *s) {
   cudaEventRecord(s->timer.ev.back(), s->stream);
 }
 
+// Status words of the samplers: 4-byte slots of mapped, portable host pages.  Pinning memory costs a
+// millisecond or two, more than the rest of a small sampler, so the pages are shared: the first stays for the
+// life of the process, another one is returned when its last slot is free.
 namespace {
+
+constexpr int STATUS_SLOTS = 1024;
+struct StatusPage {
+  int *words = nullptr;
+  std::vector<int> free_slots;
+};
+std::mutex g_status_mutex;
+std::vector<StatusPage> g_status_pages;
+
+int status_word_get(int **host, int **dev) {
+  std::lock_guard<std::mutex> lock(g_status_mutex);
+  size_t k = 0;
+  while (k < g_status_pages.size() && g_status_pages[k].free_slots.empty()) k++;
+  if (k == g_status_pages.size()) {
+    StatusPage pg;
+    ND_CUDA(cudaHostAlloc(&pg.words, sizeof(int) * STATUS_SLOTS, cudaHostAllocMapped | cudaHostAllocPortable));
+    for (int i = STATUS_SLOTS - 1; i >= 0; i--) pg.free_slots.push_back(i);
+    g_status_pages.push_back(pg);
+  }
+  int *w = g_status_pages[k].words + g_status_pages[k].free_slots.back();
+  ND_CUDA(cudaHostGetDevicePointer(dev, w, 0));
+  g_status_pages[k].free_slots.pop_back();
+  *w = 0;
+  *host = w;
+  return ND_OK;
+}
+
+void status_word_put(int *host) {
+  if (!host) return;
+  std::lock_guard<std::mutex> lock(g_status_mutex);
+  for (size_t k = 0; k < g_status_pages.size(); k++) {
+    StatusPage &pg = g_status_pages[k];
+    if (host < pg.words || host >= pg.words + STATUS_SLOTS) continue;
+    pg.free_slots.push_back((int)(host - pg.words));
+    if (k > 0 && pg.free_slots.size() == (size_t)STATUS_SLOTS) {
+      cudaFreeHost(pg.words);
+      g_status_pages.erase(g_status_pages.begin() + (long)k);
+    }
+    return;
+  }
+}
 
 __global__ void philox_uniform_kernel(uint64_t seed, int64_t n, const uint32_t *__restrict__ t4, float *__restrict__ out) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -78,7 +124,7 @@ void free_sampler(nd_sampler *s) {
   nd_hostrows_free(s);
   cudaFree(s->d_initial); cudaFree(s->d_out); cudaFree(s->d_tmp); cudaFree(s->d_len); cudaFree(s->d_plen); cudaFree(s->d_state);
   for (int i = 0; i < 2; i++) { cudaFree(s->d_map_key[i]); cudaFree(s->d_map_val[i]); }
-  cudaFree(s->d_init_key); cudaFree(s->d_init_val); cudaFree(s->d_nlive); cudaFree(s->d_stats); if (s->h_status) cudaFreeHost(s->h_status);
+  cudaFree(s->d_init_key); cudaFree(s->d_init_val); cudaFree(s->d_nlive); cudaFree(s->d_stats); status_word_put(s->h_status);
   cudaFree(s->d_runs); cudaFree(s->d_bin_counts); cudaFree(s->d_hop_counts);
   cudaFree(s->d_adj_row); cudaFree(s->d_adj_col); cudaFree(s->d_prob); cudaFree(s->d_cand); cudaFree(s->d_cand_w); cudaFree(s->d_acc); cudaFree(s->d_bm);
   cudaFree(s->d_cnt); cudaFree(s->d_offs); cudaFree(s->d_bsum); cudaFree(s->d_rank);
@@ -178,9 +224,7 @@ int nd_sampler_create(const nd_graph *g, const nd_app_params *p, int64_t num_sam
   ND_CUDA_S(cudaMalloc(&s->d_initial, sizeof(int32_t) * S1 * s->isz));
   ND_CUDA_S(cudaMalloc(&s->d_out, sizeof(int32_t) * S1 * s->fs));
   ND_CUDA_S(cudaMalloc(&s->d_stats, sizeof(unsigned long long) * 8));
-  ND_CUDA_S(cudaHostAlloc(&s->h_status, sizeof(int), cudaHostAllocMapped));
-  *s->h_status = 0;
-  ND_CUDA_S(cudaHostGetDevicePointer(&s->d_status, s->h_status, 0));
+  ND_TRY_S(status_word_get(&s->h_status, &s->d_status));
   ND_CUDA_S(cudaMemset(s->d_stats, 0, sizeof(unsigned long long) * 8));
   if (nd_is_walk(p->app)) ND_TRY_S(nd_walk_alloc(s));
   else if (nd_is_khop(p->app)) ND_TRY_S(nd_khop_alloc(s));
@@ -192,7 +236,6 @@ int nd_sampler_create(const nd_graph *g, const nd_app_params *p, int64_t num_sam
     default_initial_kernel<<<(int)((n + 255) / 256), 256>>>(first_sample, num_samples, s->isz, g->V, s->d_initial);
     ND_CUDA_S(cudaGetLastError());
   }
-  if (nd_is_khop(p->app)) ND_TRY_S(nd_sampler_build_initial_map(s));
   ND_CUDA_S(cudaDeviceSynchronize());
 #undef ND_TRY_S
 #undef ND_CUDA_S
@@ -204,8 +247,7 @@ int nd_sampler_set_initial(nd_sampler *s, const int32_t *initial) {
   ND_REQUIRE(s && initial, ND_ERR_ARG, "nd_sampler_set_initial: null argument");
   ND_CUDA(cudaSetDevice(s->g->device));
   ND_CUDA(cudaMemcpyAsync(s->d_initial, initial, sizeof(int32_t) * (size_t)s->S * s->isz, cudaMemcpyHostToDevice, s->stream));
-  if (nd_is_khop(s->p.app)) ND_TRY(nd_sampler_build_initial_map(s));
-  s->map_stale = true;
+  s->map_stale = true;   // the transit-parallel modes sort the initial map when they next run
   return ND_OK;
 }
 
@@ -373,9 +415,9 @@ int nd_sampler_next_kernel(const nd_sampler *s, int mode, char *name, int n) {
                     : nd_walk_step_loop(s) ? "walk_next_ticket_kernel" : "walk_next_count_kernel";
     snprintf(name, (size_t)n, "%s<%s>", k, walk_app[app]);
   } else if (nd_is_khop(app)) {
-    const char *e = getenv("ND_KHOP_STAGING");
-    const bool staged = mode == ND_MODE_TRANSIT_PARALLEL_LB && e && e[0] == '1';
-    snprintf(name, (size_t)n, "%s", staged ? "khop_bin_kernel + khop_pairs_kernel + khop_staged_kernel" : "khop_pairs_kernel");
+    const bool staged = mode == ND_MODE_TRANSIT_PARALLEL_LB && nd_khop_staging();
+    snprintf(name, (size_t)n, "%s", staged ? "khop_bin_kernel + khop_pairs_kernel + khop_staged_kernel"
+                                   : mode != ND_MODE_TRANSIT_PARALLEL && nd_khop_rows_fits(s) ? "khop_rows_kernel" : "khop_pairs_kernel");
   } else if (app == ND_APP_FASTGCN_REF || app == ND_APP_LADIES_REF) {
     snprintf(name, (size_t)n, "coll_ref_kernel");
   } else {

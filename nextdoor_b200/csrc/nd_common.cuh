@@ -233,6 +233,7 @@ void nd_phase_end(nd_sampler *s);
 
 // ---------------------------------------------------------------- per-family entry points
 int nd_graph_ensure_colw(const nd_graph *g, int sms);
+int nd_graph_ensure_vrow(const nd_graph *g, int sms);
 int nd_walk_step_packed_launch(const nd_graph *g, const nd_app_params *p, int step, int64_t n, const uint64_t *d_in,
                                uint64_t *d_out, cudaStream_t st);
 int nd_walk_step_launch(const nd_graph *g, const nd_app_params *p, int step, int64_t n, const int32_t *d_transits,
@@ -246,6 +247,7 @@ bool nd_walk_step_loop(const nd_sampler *s);   // the load-balanced mode takes t
 int nd_walk_sample(nd_sampler *s, int mode);
 int nd_khop_alloc(nd_sampler *s);
 int nd_khop_sample(nd_sampler *s, int mode);
+bool nd_khop_staging();   // ND_KHOP_STAGING=1: the load-balanced mode bins transits and stages lists
 int nd_collective_alloc(nd_sampler *s);
 int nd_collective_sample(nd_sampler *s, int mode);
 const char *nd_collective_kernel_name(const nd_sampler *s);  // union path of the importance samplers

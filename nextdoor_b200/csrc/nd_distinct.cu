@@ -8,6 +8,7 @@
 // in shared memory, flags the first element of every run of equal ids, ranks the flags with a
 // shared-memory scan and writes the survivors back in one coalesced pass.
 #include "nd_common.cuh"
+#include "nd_warp_sort.cuh"
 
 namespace {
 
@@ -85,7 +86,6 @@ template <int E>
 __global__ void __launch_bounds__(DTHREADS)
 distinct_warp_kernel(int32_t *__restrict__ data, int64_t n_segments, int32_t seg_len, int32_t seg_stride,
                      int32_t invalid, int32_t *__restrict__ counts, int32_t counts_stride) {
-  constexpr int P = 32 * E;
   const int lane = threadIdx.x & 31;
   const int64_t seg = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   if (seg >= n_segments) return;  // whole warps leave together
@@ -101,51 +101,8 @@ distinct_warp_kernel(int32_t *__restrict__ data, int64_t n_segments, int32_t seg
     }
     v[e] = x;
   }
-#pragma unroll
-  for (int size = 2; size <= P; size <<= 1) {
-#pragma unroll
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      if (stride >= E) {
-        const int ls = stride / E;
-        const bool lower = (lane & ls) == 0;
-#pragma unroll
-        for (int e = 0; e < E; e++) {
-          const int32_t other = __shfl_xor_sync(0xffffffffu, v[e], ls);
-          const bool up = (((lane * E + e) & size) == 0);
-          v[e] = (lower == up) ? min(v[e], other) : max(v[e], other);
-        }
-      } else {
-#pragma unroll
-        for (int e = 0; e < E; e++) {
-          if ((e & stride) == 0) {
-            const bool up = (((lane * E + e) & size) == 0);
-            const int32_t a = v[e], b = v[e + stride];
-            if ((a > b) == up) { v[e] = b; v[e + stride] = a; }
-          }
-        }
-      }
-    }
-  }
-  int32_t before = __shfl_up_sync(0xffffffffu, v[E - 1], 1);  // last id of the lane to the left
-  bool head[E];
-  int cnt = 0;
-#pragma unroll
-  for (int e = 0; e < E; e++) {
-    const int32_t prev = e == 0 ? before : v[e - 1];
-    head[e] = v[e] != 0x7fffffff && ((lane == 0 && e == 0) || v[e] != prev);
-    cnt += head[e] ? 1 : 0;
-  }
-  int inc = cnt;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += t;
-  }
-  const int uniq = __shfl_sync(0xffffffffu, inc, 31);
-  int pos = inc - cnt;
-#pragma unroll
-  for (int e = 0; e < E; e++)
-    if (head[e]) base[pos++] = v[e];
+  warp_sort<E>(v);
+  const int uniq = warp_unique_store<E>(v, base);
   for (int i = uniq + lane; i < seg_len; i += 32) base[i] = invalid;
   if (lane == 0 && counts) counts[seg * (int64_t)counts_stride] = uniq;
 }

@@ -19,6 +19,10 @@
 // list length (staging must cost fewer sectors than the gathers it replaces).  Nothing returns
 // to the host between steps: counts and work lists stay on the device.
 //
+// The sample-parallel and load-balanced modes run a warp per sample (nd_khop_rows.cu) unless the row is too
+// long for shared memory or ND_KHOP_STAGING=1 asks for the bins; what the transit-parallel path needs beyond
+// that is made when it is first asked for.
+//
 // Output layout: child j of parent slot i of hop k is written at prefix_k + i*stepSize(k) + j and
 // its draws are keyed by slot i*stepSize(k) + j.  The reference hands out positions inside
 // [prefix_k, prefix_k + n_k) with an atomic counter (src/nextdoor.cu:295-305), so any order
@@ -26,6 +30,7 @@
 #include <cstdlib>
 
 #include "nd_common.cuh"
+#include "nd_khop_rows.cuh"
 #include "nd_philox.cuh"
 
 namespace {
@@ -399,29 +404,44 @@ int nd_khop_alloc(nd_sampler *s) {
   const int64_t S = s->S;
   s->map_cap = S * cap;
   ND_REQUIRE(s->map_cap * 32 < ((int64_t)1 << 31), ND_ERR_RANGE, "%lld (transit, sample) pairs per step do not fit int32 pair ids", (long long)s->map_cap);
-  const size_t mc = (size_t)(s->map_cap > 0 ? s->map_cap : 1);
-  for (int i = 0; i < 2; i++) {
-    ND_CUDA(cudaMalloc(&s->d_map_key[i], sizeof(int32_t) * mc));
-    ND_CUDA(cudaMalloc(&s->d_map_val[i], sizeof(int32_t) * mc));
-  }
-  ND_CUDA(cudaMalloc(&s->d_init_key, sizeof(int32_t) * (size_t)(S > 0 ? S : 1)));
-  ND_CUDA(cudaMalloc(&s->d_init_val, sizeof(int32_t) * (size_t)(S > 0 ? S : 1)));
   ND_CUDA(cudaMalloc(&s->d_nlive, sizeof(int32_t) * (size_t)(2 * p.steps + 4)));
   s->d_init_n = s->d_nlive;
+  s->map_stale = true;
+  if (p.app == ND_APP_KHOP_DISTINCT) ND_CUDA(cudaMalloc(&s->d_hop_counts, sizeof(int32_t) * (size_t)(S > 0 ? S : 1) * p.steps));
+  return nd_khop_rows_alloc(s);
+}
+
+// maps, sort scratch, bins: for the transit-parallel path
+static int tp_alloc(nd_sampler *s) {
+  if (s->loop_ready) return ND_OK;
+  const nd_app_params &p = s->p;
+  const int64_t S = s->S;
+  const size_t mc = (size_t)(s->map_cap > 0 ? s->map_cap : 1);
+  for (int i = 0; i < 2; i++) {
+    if (!s->d_map_key[i]) ND_CUDA(cudaMalloc(&s->d_map_key[i], sizeof(int32_t) * mc));
+    if (!s->d_map_val[i]) ND_CUDA(cudaMalloc(&s->d_map_val[i], sizeof(int32_t) * mc));
+  }
+  if (!s->d_init_key) ND_CUDA(cudaMalloc(&s->d_init_key, sizeof(int32_t) * (size_t)(S > 0 ? S : 1)));
+  if (!s->d_init_val) ND_CUDA(cudaMalloc(&s->d_init_val, sizeof(int32_t) * (size_t)(S > 0 ? S : 1)));
   // work items of the block / grid bins: a staged run has >= 1 pair and is cut every 128+ pairs
   s->runs_cap = s->map_cap / 2 + s->map_cap / 128 + 1024;
-  ND_CUDA(cudaMalloc(&s->d_runs, sizeof(int2) * (size_t)s->runs_cap));
-  ND_CUDA(cudaMalloc(&s->d_bin_counts, sizeof(int32_t) * 4 * (size_t)p.steps));
-  ND_CUDA(cudaMalloc(&s->d_state, (size_t)s->g->V + 16));  // per-transit bin flags (kernelTypeForTransit, src/nextdoor.cu:2309)
-  if (p.app == ND_APP_KHOP_DISTINCT) ND_CUDA(cudaMalloc(&s->d_hop_counts, sizeof(int32_t) * (size_t)(S > 0 ? S : 1) * p.steps));
+  if (!s->d_runs) ND_CUDA(cudaMalloc(&s->d_runs, sizeof(int2) * (size_t)s->runs_cap));
+  if (!s->d_bin_counts) ND_CUDA(cudaMalloc(&s->d_bin_counts, sizeof(int32_t) * 4 * (size_t)p.steps));
+  if (!s->d_state) ND_CUDA(cudaMalloc(&s->d_state, (size_t)s->g->V + 16));  // per-transit bin flags (kernelTypeForTransit, src/nextdoor.cu:2309)
   const int key_bits = nd_bit_length((uint32_t)(s->g->V > 1 ? s->g->V - 1 : 1));
-  ND_TRY(nd_radix_scratch_alloc(&s->radix, key_bits, s->map_cap > S ? s->map_cap : S));
+  if (!s->radix.tile_hist) ND_TRY(nd_radix_scratch_alloc(&s->radix, key_bits, s->map_cap > S ? s->map_cap : S));
   // host-known sizes of the unsorted child maps, kept on the device for the sort
   std::vector<int32_t> full((size_t)p.steps + 1, 0);
   int64_t m = S;
   for (int k = 0; k < p.steps; k++) { m *= p.fanout[k]; full[k] = (int32_t)(k < p.steps - 1 ? m : 0); }
   ND_CUDA(cudaMemcpy(s->d_nlive + p.steps + 2, full.data(), sizeof(int32_t) * (size_t)p.steps, cudaMemcpyHostToDevice));
+  s->loop_ready = true;
   return ND_OK;
+}
+
+bool nd_khop_staging() {
+  const char *e = getenv("ND_KHOP_STAGING");
+  return e && e[0] == '1';
 }
 
 int nd_khop_sample(nd_sampler *s, int mode) {
@@ -429,10 +449,19 @@ int nd_khop_sample(nd_sampler *s, int mode) {
   // B200 it measured slower than the plain pairs kernel in every configuration tried (2^21-vertex
   // R-MAT graph; 262,144 and 2,097,152 seeds; with and without replacement: 9-25 % slower): the
   // lists that are short enough to stage and hot enough to pay are served by the 126 MB L2 anyway.
-  // So the load-balanced mode runs the plain transit-parallel kernels unless ND_KHOP_STAGING=1.
-  if (mode == ND_MODE_TRANSIT_PARALLEL_LB) {
-    const char *e = getenv("ND_KHOP_STAGING");
-    if (!(e && e[0] == '1')) mode = ND_MODE_TRANSIT_PARALLEL;
+  // And a warp per sample is faster than either, at every number of samples: it runs unless
+  // ND_KHOP_STAGING=1 or the row does not fit.
+  const bool staging = mode == ND_MODE_TRANSIT_PARALLEL_LB && nd_khop_staging();
+  if (mode != ND_MODE_TRANSIT_PARALLEL && !staging && nd_khop_rows_fits(s)) {
+    nd_phase_begin(s, ND_PHASE_NEXT);
+    const int rc = nd_khop_rows_launch(s);
+    nd_phase_end(s);
+    return rc;
+  }
+  if (mode == ND_MODE_TRANSIT_PARALLEL_LB && !staging) mode = ND_MODE_TRANSIT_PARALLEL;
+  if (mode != ND_MODE_SAMPLE_PARALLEL) {
+    ND_TRY(tp_alloc(s));
+    if (s->map_stale) ND_TRY(nd_sampler_build_initial_map(s));
   }
   const nd_app_params &p = s->p;
   const int64_t S = s->S;

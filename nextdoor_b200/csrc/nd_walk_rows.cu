@@ -763,7 +763,19 @@ int ensure_colw(const nd_graph *g, int sms) {
   return ND_OK;
 }
 
+int ensure_vrow(const nd_graph *g, int sms) {
+  if (g->vrow) return ND_OK;
+  ND_TRY(make(g->vrow, (size_t)g->V));
+  vrow_build_kernel<<<sms * 16, 256>>>(g->row_ptr, g->V, g->vrow);
+  return ND_OK;
+}
+
 }  // namespace
+
+int nd_graph_ensure_vrow(const nd_graph *g, int sms) {
+  std::lock_guard<std::mutex> lock(g_derived_mutex);
+  return ensure_vrow(g, sms);
+}
 
 int nd_graph_ensure_colw(const nd_graph *g, int sms) {
   std::lock_guard<std::mutex> lock(g_derived_mutex);
@@ -772,7 +784,7 @@ int nd_graph_ensure_colw(const nd_graph *g, int sms) {
 
 int nd_walk_rows_alloc(nd_sampler *s) {
   const nd_graph *g = s->g;
-  const size_t V = (size_t)g->V, E = (size_t)(g->E > 0 ? g->E : 1);
+  const size_t E = (size_t)(g->E > 0 ? g->E : 1);
   const int grid = s->dev.sms * 16;
   const int app = s->p.app;
   if (s->S > (int64_t)s->dev.sms * ROWS_CTAS * ROWS_THREADS) ND_TRY(make(s->d_list, (size_t)s->S));
@@ -783,7 +795,7 @@ int nd_walk_rows_alloc(nd_sampler *s) {
   if (app == ND_APP_DEEPWALK || app == ND_APP_PPR) {
     if (!alt_layout(s)) return ensure_colw(g, s->dev.sms);
     if (!g->wq) {
-      ND_TRY(make(g->vrec4, V));
+      ND_TRY(make(g->vrec4, (size_t)g->V));
       vrec4_build_kernel<<<grid, 256>>>(g->row_ptr, g->max_w, g->V, g->vrec4);
       ND_TRY(make(g->wq, E));
       wq_build_kernel<<<grid, BUILD_THREADS>>>(g->row_ptr, g->max_w, g->w, g->V, g->E, g->wq);
@@ -791,10 +803,7 @@ int nd_walk_rows_alloc(nd_sampler *s) {
     ND_CUDA(cudaGetLastError());
     return ND_OK;
   }
-  if (!g->vrow) {
-    ND_TRY(make(g->vrow, V));
-    vrow_build_kernel<<<grid, 256>>>(g->row_ptr, g->V, g->vrow);
-  }
+  ND_TRY(ensure_vrow(g, s->dev.sms));
   if (app == ND_APP_UNIFORM_WALK && alt_layout(s) && !g->erec) {
     ND_TRY(make(g->erec, E));
     erec_build_kernel<<<grid, 256>>>(g->col, g->row_ptr, g->E, g->erec);
