@@ -86,6 +86,8 @@ int nd_graph_from_csr(int device, int32_t V, int64_t E, const int32_t *row_ptr, 
  * done on the device: n 12-byte records {int32 src, int32 dst, float32 w} in host memory are
  * sorted by (src, dst, w) with the library's radix sort; vertex count = max id + 1; duplicates kept. */
 int nd_graph_from_edge_records(int device, int64_t n, const void *records, nd_graph **out);
+/* the same from three host arrays */
+int nd_graph_from_edges(int device, int64_t n, const int32_t *src, const int32_t *dst, const float *w, nd_graph **out);
 /* loadGraph(file, "edge-list", "binary") (src/nextdoor.cu:1845-1891) */
 int nd_graph_load_edge_list_binary(int device, const char *path, nd_graph **out);
 /* loadGraph(file, type, format) with all three formats of the reference (src/nextdoor.cu:1845-1891):

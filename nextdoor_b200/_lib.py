@@ -55,6 +55,7 @@ _SIGS = {
     "nd_launch_count": (C.c_int64, []),
     "nd_graph_from_csr": (C.c_int, [C.c_int, C.c_int32, C.c_int64, VP, VP, VP, VP, C.POINTER(VP)]),
     "nd_graph_from_edge_records": (C.c_int, [C.c_int, C.c_int64, VP, C.POINTER(VP)]),
+    "nd_graph_from_edges": (C.c_int, [C.c_int, C.c_int64, VP, VP, VP, C.POINTER(VP)]),
     "nd_graph_load_edge_list_binary": (C.c_int, [C.c_int, C.c_char_p, C.POINTER(VP)]),
     "nd_graph_load": (C.c_int, [C.c_int, C.c_char_p, C.c_char_p, C.c_char_p, C.POINTER(VP)]),
     "nd_graph_rmat": (C.c_int, [C.c_int, C.c_int32, C.c_int64, C.c_uint64, C.POINTER(VP)]),

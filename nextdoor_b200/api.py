@@ -96,10 +96,11 @@ class Graph:
 
     @classmethod
     def from_edge_records(cls, src, dst, w, device=0):
-        rec = np.empty(len(src), dtype=[("s", "<i4"), ("d", "<i4"), ("w", "<f4")])
-        rec["s"], rec["d"], rec["w"] = src, dst, w
+        n = len(src)
+        src, dst, w = (np.ascontiguousarray(np.broadcast_to(np.asarray(x).astype(t, copy=False), (n,)))
+                       for x, t in ((src, np.int32), (dst, np.int32), (w, np.float32)))
         h = C.c_void_p()
-        check(lib.nd_graph_from_edge_records(device, rec.shape[0], _ptr(rec), C.byref(h)))
+        check(lib.nd_graph_from_edges(device, n, _ptr(src), _ptr(dst), _ptr(w), C.byref(h)))
         return cls(h, device)
 
     @classmethod

@@ -6,6 +6,7 @@
 #include <string.h>
 
 #include "nd_common.cuh"
+#include "nd_host.h"
 #include "nd_khop_rows.cuh"
 #include "nd_philox.cuh"
 
@@ -230,7 +231,7 @@ int nd_sampler_create(const nd_graph *g, const nd_app_params *p, int64_t num_sam
   else if (nd_is_khop(p->app)) ND_TRY_S(nd_khop_alloc(s));
   else ND_TRY_S(nd_collective_alloc(s));
   if (initial) {
-    ND_CUDA_S(cudaMemcpy(s->d_initial, initial, sizeof(int32_t) * (size_t)num_samples * s->isz, cudaMemcpyHostToDevice));
+    ND_TRY_S(nd_copy_to_device(g->device, s->d_initial, initial, sizeof(int32_t) * (size_t)num_samples * s->isz));
   } else if (num_samples > 0) {
     const int64_t n = num_samples * s->isz;
     default_initial_kernel<<<(int)((n + 255) / 256), 256>>>(first_sample, num_samples, s->isz, g->V, s->d_initial);
@@ -240,6 +241,7 @@ int nd_sampler_create(const nd_graph *g, const nd_app_params *p, int64_t num_sam
 #undef ND_TRY_S
 #undef ND_CUDA_S
   *out = s;
+  nd_objects_add(1);
   return ND_OK;
 }
 
@@ -296,8 +298,7 @@ int nd_sampler_final_samples(nd_sampler *s, int32_t *out) {
   ND_REQUIRE(s && (out || s->S == 0), ND_ERR_ARG, "nd_sampler_final_samples: null argument");
   ND_REQUIRE(s->sampled, ND_ERR_STATE, "final samples requested before sample()");
   ND_TRY(nd_sampler_sync(s));
-  if (s->S > 0) ND_CUDA(cudaMemcpy(out, s->d_out, sizeof(int32_t) * (size_t)s->S * s->fs, cudaMemcpyDeviceToHost));
-  return ND_OK;
+  return nd_copy_to_host(s->g->device, out, s->d_out, sizeof(int32_t) * (size_t)s->S * s->fs);
 }
 
 int nd_sampler_final_samples_async(nd_sampler *s, int32_t *out, void *copy_stream) {
@@ -338,12 +339,13 @@ int nd_sampler_aux(nd_sampler *s, int32_t *adj_row, int32_t *adj_col, float *pro
   if (nd_is_collective(s->p.app)) {
     const int L = s->p.fanout[0], B = s->p.batch;
     const size_t n = (size_t)s->S * s->p.steps * (B > L ? B : L) * L;
-    if (adj_row) ND_CUDA(cudaMemcpy(adj_row, s->d_adj_row, 4 * n, cudaMemcpyDeviceToHost));
-    if (adj_col) ND_CUDA(cudaMemcpy(adj_col, s->d_adj_col, 4 * n, cudaMemcpyDeviceToHost));
-    if (prob && s->d_prob) ND_CUDA(cudaMemcpy(prob, s->d_prob, 4 * (size_t)s->S * s->fs, cudaMemcpyDeviceToHost));
+    const int dev = s->g->device;
+    if (adj_row) ND_TRY(nd_copy_to_host(dev, adj_row, s->d_adj_row, 4 * n));
+    if (adj_col) ND_TRY(nd_copy_to_host(dev, adj_col, s->d_adj_col, 4 * n));
+    if (prob && s->d_prob) ND_TRY(nd_copy_to_host(dev, prob, s->d_prob, 4 * (size_t)s->S * s->fs));
   }
   if (hop_counts && s->d_hop_counts)
-    ND_CUDA(cudaMemcpy(hop_counts, s->d_hop_counts, 4 * (size_t)s->S * s->p.steps, cudaMemcpyDeviceToHost));
+    ND_TRY(nd_copy_to_host(s->g->device, hop_counts, s->d_hop_counts, 4 * (size_t)s->S * s->p.steps));
   return ND_OK;
 }
 
@@ -431,6 +433,7 @@ int nd_sampler_destroy(nd_sampler *s) {
   cudaSetDevice(s->g->device);
   cudaStreamSynchronize(s->stream);
   free_sampler(s);
+  nd_objects_add(-1);
   return ND_OK;
 }
 

@@ -71,6 +71,7 @@ struct nd_graph {
   int32_t *col = nullptr;
   float *w = nullptr;
   float *max_w = nullptr;
+  void *block = nullptr;        // the one allocation the four arrays lie in, or null: an allocation each
   // Derived layouts, built on the first sampler that needs them and shared by all samplers of the graph:
   mutable int2 *colw = nullptr;        // [E] (neighbour id, weight bits) records: one 8-byte gather per weighted try
   mutable int2 *vrec = nullptr;        // [V+1] (row start, max weight bits) per vertex: what a thread-per-walk kernel needs of a vertex in one sector
@@ -116,6 +117,8 @@ struct NdRadixScratch {
 };
 
 NdRadixPlan nd_radix_plan(int key_bits, int64_t max_n);
+size_t nd_radix_scratch_bytes(int64_t max_n);
+void nd_radix_scratch_place(NdRadixScratch *s, const NdRadixPlan &plan, void *at);
 int nd_radix_scratch_alloc(NdRadixScratch *s, int key_bits, int64_t max_n);
 void nd_radix_scratch_free(NdRadixScratch *s);
 

@@ -7,15 +7,20 @@
 // The records are sorted by (src, dst, weight) with three stable LSD sorts of the in-house radix
 // sort (weight bits, then dst, then src), row offsets come from the boundaries of the sorted src
 // array, and the sorted dst / weight arrays become col / w in place.
+#include <fcntl.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <sys/stat.h>
+#include <unistd.h>
 
 #include <algorithm>
+#include <atomic>
 #include <string>
 #include <vector>
 
 #include "nd_common.cuh"
+#include "nd_host.h"
 #include "nd_philox.cuh"
 
 namespace {
@@ -31,18 +36,60 @@ __device__ __forceinline__ float key_to_float(uint32_t k) {
 
 struct Rec12 { int32_t s, d; float w; };
 
+// What the build needs to know of the records: largest id, whether one is negative, and which bits of the
+// weight keys differ between records (all others need no sorting).
+struct RecordFacts {
+  int32_t max_id;
+  int32_t bad;
+  uint32_t key_and, key_or;
+};
+
+__device__ __forceinline__ void facts_out(RecordFacts *facts, int32_t m, bool bad, uint32_t ka, uint32_t ko) {
+  for (int o = 16; o > 0; o >>= 1) {
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    ka &= __shfl_xor_sync(0xffffffffu, ka, o);
+    ko |= __shfl_xor_sync(0xffffffffu, ko, o);
+  }
+  bad = __any_sync(0xffffffffu, bad);
+  if ((threadIdx.x & 31) == 0) {
+    if (m >= 0) atomicMax(&facts->max_id, m);
+    if (bad) atomicOr(&facts->bad, 1);
+    atomicAnd(&facts->key_and, ka);
+    atomicOr(&facts->key_or, ko);
+  }
+}
+
 __global__ void unpack_records_kernel(const Rec12 *__restrict__ rec, int64_t n, uint32_t *__restrict__ src,
-                                      uint32_t *__restrict__ dst, uint32_t *__restrict__ wk,
-                                      int32_t *__restrict__ max_id, int *__restrict__ status) {
+                                      uint32_t *__restrict__ dst, uint32_t *__restrict__ wk, RecordFacts *__restrict__ facts) {
   int32_t m = -1;
+  bool bad = false;
+  uint32_t ka = 0xffffffffu, ko = 0u;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const Rec12 r = rec[i];
-    if (r.s < 0 || r.d < 0) atomicOr(status, ND_DEV_BAD_TRANSIT);
-    src[i] = (uint32_t)r.s; dst[i] = (uint32_t)r.d; wk[i] = float_to_key(r.w);
+    const uint32_t k = float_to_key(r.w);
+    src[i] = (uint32_t)r.s; dst[i] = (uint32_t)r.d; wk[i] = k;
+    bad |= r.s < 0 || r.d < 0;
     m = max(m, max(r.s, r.d));
+    ka &= k; ko |= k;
   }
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m >= 0) atomicMax(max_id, m);
+  facts_out(facts, m, bad, ka, ko);
+}
+
+// the same for records that arrive as three arrays: the weights become their keys in place
+__global__ void unpack_arrays_kernel(int64_t n, const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst,
+                                     uint32_t *__restrict__ wk, RecordFacts *__restrict__ facts) {
+  int32_t m = -1;
+  bool bad = false;
+  uint32_t ka = 0xffffffffu, ko = 0u;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t s = (int32_t)src[i], d = (int32_t)dst[i];
+    const uint32_t k = float_to_key(__uint_as_float(wk[i]));
+    wk[i] = k;
+    bad |= s < 0 || d < 0;
+    m = max(m, max(s, d));
+    ka &= k; ko |= k;
+  }
+  facts_out(facts, m, bad, ka, ko);
 }
 
 // R-MAT (a,b,c,d) = (.57,.19,.19,.05).  Undirected edge e, attempt t: Philox counter
@@ -86,18 +133,18 @@ __global__ void rmat_kernel(int32_t V, int scale, int64_t M, uint64_t seed, uint
   }
 }
 
-// row_ptr from the sorted src array: element i closes the rows (src[i-1], src[i]]
-__global__ void row_ptr_kernel(const uint32_t *__restrict__ src, int64_t n, int32_t V, int32_t *__restrict__ row_ptr) {
+// The sorted records become the CSR: row_ptr (element i closes the rows (src[i-1], src[i]]), col, w.
+__global__ void csr_from_sorted_kernel(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst, const uint32_t *__restrict__ wk,
+                                       int64_t n, int32_t V, int32_t *__restrict__ row_ptr, int32_t *__restrict__ col, float *__restrict__ w) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t lo = i == 0 ? 0 : (int64_t)src[i - 1] + 1;
     const int64_t hi = i == n ? V : (int64_t)src[i];
     for (int64_t v = lo; v <= hi; v++) row_ptr[v] = (int32_t)i;
+    if (i < n) {
+      col[i] = (int32_t)dst[i];
+      w[i] = key_to_float(wk[i]);
+    }
   }
-}
-
-__global__ void weights_back_kernel(uint32_t *__restrict__ wk, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    wk[i] = __float_as_uint(key_to_float(wk[i]));
 }
 
 // Vertex::max_weight (src/graph.hpp:71-80) starts from 0, so only positive weights can raise it
@@ -199,52 +246,82 @@ int grid_for(int64_t n, int threads, int sms) {
   return (int)(b > 0 ? b : 1);
 }
 
-// sorted SoA records (device, already (src,dst,wkey) in a[]) -> graph
-int build_from_soa(int device, int64_t n, int32_t V, uint32_t *a[3], uint32_t *b[3], cudaStream_t st, nd_graph **out) {
-  NdDeviceInfo dev;
-  ND_TRY(nd_device_info(device, &dev));
-  ND_REQUIRE(n < ((int64_t)1 << 31), ND_ERR_RANGE, "%lld edges do not fit the int32 edge index of the CSR", (long long)n);
-  NdRadixScratch scr;
-  ND_TRY(nd_radix_scratch_alloc(&scr, 32, n));
-  int32_t *d_n = nullptr;
-  ND_CUDA(cudaMalloc(&d_n, sizeof(int32_t)));
+// Device memory of a build in one allocation:
+// the records twice -- (src, dst, weight key) and the sort's other side --, the sort's histograms, small words.
+// 32 bytes of padding behind every array.
+struct BuildScratch {
+  unsigned char *base = nullptr;
+  uint32_t *a[3], *b[3];
+  Rec12 *rec;                // over b: 12-byte records before they are unpacked into a
+  NdRadixScratch radix;
+  RecordFacts *facts;
+  int32_t *d_n, *d_max_degree;
+  int device = 0;
+  ~BuildScratch() { nd_pool_free(device, base); }
+};
+
+int build_scratch(BuildScratch *s, int device, int64_t n) {
+  s->device = device;
+  const size_t words = ((size_t)(n > 0 ? n : 1) + 8 + 63) & ~(size_t)63;
+  const NdRadixPlan pl = nd_radix_plan(32, n);
+  const size_t radix = nd_radix_scratch_bytes(n);
+  ND_TRY(nd_pool_alloc(device, (void **)&s->base, 24 * words + radix + 256));
+  for (int w = 0; w < 3; w++) { s->a[w] = (uint32_t *)s->base + w * words; s->b[w] = (uint32_t *)s->base + (3 + w) * words; }
+  s->rec = (Rec12 *)s->b[0];
+  unsigned char *p = s->base + 24 * words;
+  s->facts = (RecordFacts *)p;
+  s->d_n = (int32_t *)(p + 64);
+  s->d_max_degree = (int32_t *)(p + 128);
+  nd_radix_scratch_place(&s->radix, pl, p + 256);
+  const RecordFacts none{-1, 0, 0xffffffffu, 0u};
   const int32_t n32 = (int32_t)n;
-  ND_CUDA(cudaMemcpyAsync(d_n, &n32, sizeof(int32_t), cudaMemcpyHostToDevice, st));
+  ND_CUDA(cudaMemset(p + 128, 0, radix + 128));
+  ND_CUDA(cudaMemcpy(s->facts, &none, sizeof(none), cudaMemcpyHostToDevice));
+  ND_CUDA(cudaMemcpy(s->d_n, &n32, sizeof(n32), cudaMemcpyHostToDevice));
+  return ND_OK;
+}
+
+// records in bs->a (weights as keys) -> graph; key bits outside [lo_bit, hi_bit) are the same in all records
+int build_from_soa(const NdDeviceInfo &dev, int64_t n, int32_t V, BuildScratch *bs, int lo_bit, int hi_bit, nd_graph **out) {
+  ND_REQUIRE(n < ((int64_t)1 << 31), ND_ERR_RANGE, "%lld edges do not fit the int32 edge index of the CSR", (long long)n);
   const int vbits = nd_bit_length((uint32_t)(V > 1 ? V - 1 : 1));
   const int key_word[3] = {2, 1, 0};
-  const int key_bits[3] = {32, vbits, vbits};
-  uint32_t *cur[3] = {a[0], a[1], a[2]}, *oth[3] = {b[0], b[1], b[2]};
+  const int key_bits[3] = {hi_bit - lo_bit, vbits, vbits};
+  uint32_t *cur[3] = {bs->a[0], bs->a[1], bs->a[2]}, *oth[3] = {bs->b[0], bs->b[1], bs->b[2]};
   for (int k = 0; k < 3; k++) {
+    if (n < 2 || key_bits[k] <= 0) continue;
     NdSortArrays arr;
     arr.nwords = 3;
     for (int w = 0; w < 3; w++) { arr.a[w] = cur[w]; arr.b[w] = oth[w]; }
     bool in_b = false;
-    const NdRadixPlan pl = nd_radix_plan(key_bits[k], n);
-    ND_TRY(nd_radix_sort(dev, st, &scr, pl, arr, key_word[k], d_n, nullptr, false, 0u, false, &in_b));
+    NdRadixPlan pl = nd_radix_plan(key_bits[k], n);
+    if (k == 0) for (int p = 0; p < pl.passes; p++) pl.shift[p] += lo_bit;
+    ND_TRY(nd_radix_sort(dev, nullptr, &bs->radix, pl, arr, key_word[k], bs->d_n, nullptr, false, 0u, false, &in_b));
     if (in_b) for (int w = 0; w < 3; w++) { uint32_t *t = cur[w]; cur[w] = oth[w]; oth[w] = t; }
   }
+  // one block: row offsets, ids and weights (32 bytes of padding for the 16-byte staging windows), maximum weights
+  auto round = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  const size_t o_col = round(4 * ((size_t)V + 1)), o_w = o_col + round(4 * ((size_t)n + 8)), o_max = o_w + round(4 * ((size_t)n + 8)), all = o_max + round(4 * (size_t)V);
+  unsigned char *block = nullptr;
+  ND_TRY(nd_pool_alloc(dev.device, (void **)&block, all));
   nd_graph *g = new nd_graph();
-  g->device = device; g->V = V; g->E = n;
-  ND_CUDA(cudaMalloc(&g->row_ptr, sizeof(int32_t) * ((size_t)V + 1)));
-  row_ptr_kernel<<<grid_for(n + 1, 256, dev.sms), 256, 0, st>>>(cur[0], n, V, g->row_ptr);
-  weights_back_kernel<<<grid_for(n, 256, dev.sms), 256, 0, st>>>(cur[2], n);
-  ND_CUDA(cudaMalloc(&g->max_w, sizeof(float) * (size_t)V));
-  ND_CUDA(cudaMemsetAsync(g->max_w, 0, sizeof(float) * (size_t)V, st));
-  if (n > 0)
-    max_weight_kernel<<<grid_for(n, 256, dev.sms), 256, 0, st>>>(g->row_ptr, cur[0], (const float *)cur[2], V, n, (int32_t *)g->max_w);
-  ND_CUDA(cudaGetLastError());
-  ND_CUDA(cudaStreamSynchronize(st));
-  // keep the buffers that hold the sorted dst / weights as col / w (they carry 32 bytes of
-  // padding for the 16-byte staging windows); release the rest
-  g->col = (int32_t *)cur[1];
-  g->w = (float *)cur[2];
-  ND_CUDA(cudaMemset(g->col + n, 0, sizeof(int32_t) * 8));
-  ND_CUDA(cudaMemset(g->w + n, 0, sizeof(float) * 8));
-  cudaFree(cur[0]);
-  for (int w = 0; w < 3; w++) cudaFree(oth[w]);
-  nd_radix_scratch_free(&scr);
-  cudaFree(d_n);
-  ND_TRY(nd_graph_finish(g, st));
+  g->device = dev.device; g->V = V; g->E = n; g->block = block;
+  g->row_ptr = (int32_t *)block; g->col = (int32_t *)(block + o_col); g->w = (float *)(block + o_w); g->max_w = (float *)(block + o_max);
+  auto build = [&]() -> int {
+    ND_CUDA(cudaMemsetAsync(g->col + n, 0, sizeof(int32_t) * 8));
+    ND_CUDA(cudaMemsetAsync(g->w + n, 0, sizeof(float) * 8));
+    ND_CUDA(cudaMemsetAsync(g->max_w, 0, sizeof(float) * (size_t)V));
+    csr_from_sorted_kernel<<<grid_for(n + 1, 256, dev.sms), 256>>>(cur[0], cur[1], cur[2], n, V, g->row_ptr, g->col, g->w);
+    if (n > 0) max_weight_kernel<<<grid_for(n, 256, dev.sms), 256>>>(g->row_ptr, cur[0], g->w, V, n, (int32_t *)g->max_w);
+    max_degree_kernel<<<grid_for(V, 256, dev.sms), 256>>>(g->row_ptr, V, bs->d_max_degree);
+    nd_count_launches(3);
+    ND_CUDA(cudaGetLastError());
+    ND_CUDA(cudaMemcpy(&g->max_degree, bs->d_max_degree, sizeof(int32_t), cudaMemcpyDeviceToHost));
+    return ND_OK;
+  };
+  const int rc = build();
+  if (rc != ND_OK) { nd_pool_free(dev.device, block); delete g; return rc; }
+  nd_objects_add(1);
   *out = g;
   return ND_OK;
 }
@@ -288,14 +365,15 @@ int nd_graph_from_csr(int device, int32_t V, int64_t E, const int32_t *row_ptr, 
   ND_CUDA(cudaMemset(g->w + E, 0, sizeof(float) * 8));
   ND_CUDA(cudaMemcpy(g->row_ptr, row_ptr, sizeof(int32_t) * ((size_t)V + 1), cudaMemcpyHostToDevice));
   if (E > 0) {
-    ND_CUDA(cudaMemcpy(g->col, col, sizeof(int32_t) * (size_t)E, cudaMemcpyHostToDevice));
-    ND_CUDA(cudaMemcpy(g->w, w, sizeof(float) * (size_t)E, cudaMemcpyHostToDevice));
+    ND_TRY(nd_copy_to_device(device, g->col, col, sizeof(int32_t) * (size_t)E));
+    ND_TRY(nd_copy_to_device(device, g->w, w, sizeof(float) * (size_t)E));
   }
   if (max_w) {
     ND_CUDA(cudaMalloc(&g->max_w, sizeof(float) * (size_t)V));
     ND_CUDA(cudaMemcpy(g->max_w, max_w, sizeof(float) * (size_t)V, cudaMemcpyHostToDevice));
   }
   ND_TRY(nd_graph_finish(g, nullptr));
+  nd_objects_add(1);
   *out = g;
   return ND_OK;
 }
@@ -306,55 +384,71 @@ int nd_graph_from_edge_records(int device, int64_t n, const void *records, nd_gr
   return from_edge_records_min_v(device, n, records, 0, out);
 }
 
-// min_v: lower bound of the vertex count (the adjacency-list format numbers vertices by line,
-// including lines without edges)
+// the facts of the unpacked records decide the rest of the build; min_v: lower bound of the vertex count (the
+// adjacency-list format numbers vertices by line, including lines without edges)
+static int build_from_facts(const NdDeviceInfo &dev, int64_t n, int32_t min_v, BuildScratch *bs, nd_graph **out) {
+  RecordFacts f;
+  ND_CUDA(cudaGetLastError());
+  ND_CUDA(cudaMemcpy(&f, bs->facts, sizeof(f), cudaMemcpyDeviceToHost));
+  ND_REQUIRE(f.bad == 0 && f.max_id != 0x7fffffff, ND_ERR_RANGE, "edge records hold a negative or out-of-range vertex id");
+  int32_t V = f.max_id + 1 > 0 ? f.max_id + 1 : 1;  // vertex count = max id + 1 (src/graph.hpp:131-142)
+  if (V < min_v) V = min_v;
+  const uint32_t differ = f.key_and ^ f.key_or;
+  int lo = 0, hi = nd_bit_length(differ);
+  while (lo < hi && !((differ >> lo) & 1u)) lo++;
+  return build_from_soa(dev, n, V, bs, n > 0 ? lo : 0, n > 0 ? hi : 0, out);
+}
+
 static int from_edge_records_min_v(int device, int64_t n, const void *records, int32_t min_v, nd_graph **out) {
   ND_REQUIRE(out && (records || n == 0) && n >= 0, ND_ERR_ARG, "nd_graph_from_edge_records: bad argument");
   ND_REQUIRE(n < ((int64_t)1 << 31), ND_ERR_RANGE, "%lld edges do not fit the int32 edge index of the CSR", (long long)n);
   ND_CUDA(cudaSetDevice(device));
   NdDeviceInfo dev;
   ND_TRY(nd_device_info(device, &dev));
-  const size_t cap = (size_t)(n > 0 ? n : 1);
-  Rec12 *d_rec = nullptr;
-  uint32_t *a[3], *b[3];
-  ND_CUDA(cudaMalloc(&d_rec, sizeof(Rec12) * cap));
-  for (int w = 0; w < 3; w++) { ND_CUDA(cudaMalloc(&a[w], 4 * (cap + 8))); ND_CUDA(cudaMalloc(&b[w], 4 * (cap + 8))); }
-  int32_t *d_max = nullptr;
-  int *d_status = nullptr;
-  ND_CUDA(cudaMalloc(&d_max, sizeof(int32_t)));
-  ND_CUDA(cudaMalloc(&d_status, sizeof(int)));
-  ND_CUDA(cudaMemset(d_max, 0xff, sizeof(int32_t)));
-  ND_CUDA(cudaMemset(d_status, 0, sizeof(int)));
-  ND_CUDA(cudaMemcpy(d_rec, records, sizeof(Rec12) * (size_t)n, cudaMemcpyHostToDevice));
-  unpack_records_kernel<<<grid_for(n, 256, dev.sms), 256>>>(d_rec, n, a[0], a[1], a[2], d_max, d_status);
-  int32_t max_id = -1;
-  int status = 0;
-  ND_CUDA(cudaMemcpy(&max_id, d_max, sizeof(int32_t), cudaMemcpyDeviceToHost));
-  ND_CUDA(cudaMemcpy(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost));
-  cudaFree(d_rec); cudaFree(d_max); cudaFree(d_status);
-  if (status != 0 || max_id == 0x7fffffff) {
-    for (int w = 0; w < 3; w++) { cudaFree(a[w]); cudaFree(b[w]); }
-    nd_set_error("edge records hold a negative or out-of-range vertex id");
-    return ND_ERR_RANGE;
-  }
-  int32_t V = max_id + 1 > 0 ? max_id + 1 : 1;  // vertex count = max id + 1 (src/graph.hpp:131-142)
-  if (V < min_v) V = min_v;
-  return build_from_soa(device, n, V, a, b, nullptr, out);
+  BuildScratch bs;
+  ND_TRY(build_scratch(&bs, device, n));
+  ND_TRY(nd_copy_to_device(device, bs.rec, records, sizeof(Rec12) * (size_t)n));
+  unpack_records_kernel<<<grid_for(n, 256, dev.sms), 256>>>(bs.rec, n, bs.a[0], bs.a[1], bs.a[2], bs.facts);
+  nd_count_launches(1);
+  return build_from_facts(dev, n, min_v, &bs, out);
+}
+
+int nd_graph_from_edges(int device, int64_t n, const int32_t *src, const int32_t *dst, const float *w, nd_graph **out) {
+  ND_REQUIRE(out && ((src && dst && w) || n == 0) && n >= 0, ND_ERR_ARG, "nd_graph_from_edges: bad argument");
+  ND_REQUIRE(n < ((int64_t)1 << 31), ND_ERR_RANGE, "%lld edges do not fit the int32 edge index of the CSR", (long long)n);
+  ND_CUDA(cudaSetDevice(device));
+  NdDeviceInfo dev;
+  ND_TRY(nd_device_info(device, &dev));
+  BuildScratch bs;
+  ND_TRY(build_scratch(&bs, device, n));
+  const void *from[3] = {src, dst, w};
+  for (int k = 0; k < 3; k++) ND_TRY(nd_copy_to_device(device, bs.a[k], from[k], 4 * (size_t)n));
+  unpack_arrays_kernel<<<grid_for(n, 256, dev.sms), 256>>>(n, bs.a[0], bs.a[1], bs.a[2], bs.facts);
+  nd_count_launches(1);
+  return build_from_facts(dev, n, 0, &bs, out);
 }
 
 int nd_graph_load_edge_list_binary(int device, const char *path, nd_graph **out) {
   ND_REQUIRE(path && out, ND_ERR_ARG, "nd_graph_load_edge_list_binary: bad argument");
-  FILE *fp = fopen(path, "rb");
-  if (!fp) { nd_set_error("File '%s' not found", path); return ND_ERR_IO; }
-  fseek(fp, 0, SEEK_END);
-  const long fsize = ftell(fp);
-  fseek(fp, 0, SEEK_SET);
-  const int64_t n = fsize / 12;
-  std::vector<char> buf((size_t)(n * 12 > 0 ? n * 12 : 1));
-  const size_t got = fread(buf.data(), 1, (size_t)(n * 12), fp);
-  fclose(fp);
-  if (got != (size_t)(n * 12)) { nd_set_error("short read on '%s'", path); return ND_ERR_IO; }
-  return nd_graph_from_edge_records(device, n, buf.data(), out);
+  const int fd = open(path, O_RDONLY);
+  if (fd < 0) { nd_set_error("File '%s' not found", path); return ND_ERR_IO; }
+  struct stat st;
+  const int64_t n = fstat(fd, &st) == 0 ? (int64_t)st.st_size / 12 : -1;
+  char *buf = n >= 0 ? (char *)malloc((size_t)(n * 12 > 0 ? n * 12 : 1)) : nullptr;
+  std::atomic<bool> ok{buf != nullptr};
+  if (buf)   // the workers read (and first touch) a range each
+    nd_host_ranges(n * 12, nd_host_threads(), [&](int, int64_t at, int64_t end) {
+      while (at < end) {
+        const ssize_t got = pread(fd, buf + at, (size_t)(end - at), (off_t)at);
+        if (got <= 0) { ok = false; return; }
+        at += got;
+      }
+    });
+  close(fd);
+  if (!ok) { free(buf); nd_set_error("short read on '%s'", path); return ND_ERR_IO; }
+  const int rc = nd_graph_from_edge_records(device, n, buf, out);
+  free(buf);
+  return rc;
 }
 
 // Text edge list (Graph::load_from_edge_list_txt, src/graph.hpp:162-254): whitespace-separated
@@ -437,14 +531,13 @@ int nd_graph_rmat(int device, int32_t V, int64_t M, uint64_t seed, nd_graph **ou
   ND_CUDA(cudaSetDevice(device));
   NdDeviceInfo dev;
   ND_TRY(nd_device_info(device, &dev));
-  const size_t cap = (size_t)(2 * M);
-  uint32_t *a[3], *b[3];
-  for (int w = 0; w < 3; w++) { ND_CUDA(cudaMalloc(&a[w], 4 * (cap + 8))); ND_CUDA(cudaMalloc(&b[w], 4 * (cap + 8))); }
+  BuildScratch bs;
+  ND_TRY(build_scratch(&bs, device, 2 * M));
   int scale = 0;
   while (((int64_t)1 << scale) < V) scale++;
-  rmat_kernel<<<grid_for(M, 256, dev.sms), 256>>>(V, scale, M, seed, a[0], a[1], a[2]);
+  rmat_kernel<<<grid_for(M, 256, dev.sms), 256>>>(V, scale, M, seed, bs.a[0], bs.a[1], bs.a[2]);
   ND_CUDA(cudaGetLastError());
-  return build_from_soa(device, 2 * M, V, a, b, nullptr, out);
+  return build_from_soa(dev, 2 * M, V, &bs, 0, 32, out);
 }
 
 int nd_graph_info(const nd_graph *g, int32_t *V, int64_t *E, int32_t *max_degree, int *device) {
@@ -459,10 +552,10 @@ int nd_graph_info(const nd_graph *g, int32_t *V, int64_t *E, int32_t *max_degree
 int nd_graph_to_host(const nd_graph *g, int32_t *row_ptr, int32_t *col, float *w, float *max_w) {
   ND_REQUIRE(g, ND_ERR_ARG, "null graph");
   ND_CUDA(cudaSetDevice(g->device));
-  if (row_ptr) ND_CUDA(cudaMemcpy(row_ptr, g->row_ptr, sizeof(int32_t) * ((size_t)g->V + 1), cudaMemcpyDeviceToHost));
-  if (col && g->E) ND_CUDA(cudaMemcpy(col, g->col, sizeof(int32_t) * (size_t)g->E, cudaMemcpyDeviceToHost));
-  if (w && g->E) ND_CUDA(cudaMemcpy(w, g->w, sizeof(float) * (size_t)g->E, cudaMemcpyDeviceToHost));
-  if (max_w) ND_CUDA(cudaMemcpy(max_w, g->max_w, sizeof(float) * (size_t)g->V, cudaMemcpyDeviceToHost));
+  if (row_ptr) ND_TRY(nd_copy_to_host(g->device, row_ptr, g->row_ptr, sizeof(int32_t) * ((size_t)g->V + 1)));
+  if (col && g->E) ND_TRY(nd_copy_to_host(g->device, col, g->col, sizeof(int32_t) * (size_t)g->E));
+  if (w && g->E) ND_TRY(nd_copy_to_host(g->device, w, g->w, sizeof(float) * (size_t)g->E));
+  if (max_w) ND_TRY(nd_copy_to_host(g->device, max_w, g->max_w, sizeof(float) * (size_t)g->V));
   return ND_OK;
 }
 
@@ -479,9 +572,11 @@ int nd_graph_device_ptrs(const nd_graph *g, const int32_t **row_ptr, const int32
 int nd_graph_destroy(nd_graph *g) {
   if (!g) return ND_OK;
   cudaSetDevice(g->device);
-  cudaFree(g->row_ptr); cudaFree(g->col); cudaFree(g->w); cudaFree(g->max_w);
+  if (g->block) nd_pool_free(g->device, g->block);
+  else { cudaFree(g->row_ptr); cudaFree(g->col); cudaFree(g->w); cudaFree(g->max_w); }
   cudaFree(g->colw); cudaFree(g->vrec); cudaFree(g->vrow); cudaFree(g->vrec4); cudaFree(g->erec); cudaFree(g->wq); cudaFree(g->adjset); cudaFree(g->adjsign);
   delete g;
+  nd_objects_add(-1);
   return ND_OK;
 }
 

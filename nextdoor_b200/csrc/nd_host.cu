@@ -1,0 +1,341 @@
+// Worker threads and staged host <-> device copies.
+//
+// A copy between the device and pageable memory runs at 10 GB/s up and 19 GB/s down on this box (one driver
+// thread copies to or from its own pinned buffer, and faults in a fresh destination page by page); PCIe moves
+// 53-55.  Here the pieces of a large copy go through a ring of pinned buffers that several workers fill or empty
+// at once: 31-35 GB/s into memory that is there, 15-20 into fresh pages (pieces of 512 KB 27, of 2 MB 36 but
+// slow to start; non-temporal stores and a second stream gain nothing).  One copy at a time uses the ring; a second one, and small ones, take the plain call.
+#include "nd_host.h"
+
+#include <stdlib.h>
+#include <string.h>
+#include <unistd.h>
+
+#include <algorithm>
+#include <atomic>
+#include <chrono>
+#include <condition_variable>
+#include <deque>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+#include "nd_common.cuh"
+
+// ---------------------------------------------------------------- workers
+
+static void nd_host_idle();
+
+namespace {
+
+struct Job {
+  const std::function<void(int)> *task;
+  int n;
+  std::atomic<int> next{0}, done{0};
+};
+
+struct Pool {
+  std::mutex m;
+  std::condition_variable work, finished;
+  std::deque<Job *> jobs;      // with tasks nobody has taken
+  int workers = 0, idle = 0;
+  pid_t pid = 0;               // threads do not survive a fork
+};
+Pool *g_pool = nullptr;        // never destroyed: a worker may outlive the static objects
+std::mutex g_pool_mutex;
+
+Pool *pool() {
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  if (!g_pool || g_pool->pid != getpid()) {
+    g_pool = new Pool();
+    g_pool->pid = getpid();
+  }
+  return g_pool;
+}
+
+void worker(Pool *p) {
+  std::unique_lock<std::mutex> lock(p->m);
+  for (;;) {
+    if (p->jobs.empty()) {
+      p->idle++;
+      const bool woken = p->work.wait_for(lock, std::chrono::seconds(1), [&] { return !p->jobs.empty(); });
+      p->idle--;
+      if (!woken) {
+        const bool last = --p->workers == 0;
+        lock.unlock();
+        if (last) nd_host_idle();
+        return;
+      }
+    }
+    Job *job = p->jobs.front();
+    const int i = job->next.fetch_add(1, std::memory_order_relaxed);   // under the lock: the job is alive while it is in the queue
+    if (i >= job->n - 1) p->jobs.pop_front();
+    if (i >= job->n) continue;
+    const int n = job->n;
+    lock.unlock();
+    (*job->task)(i);
+    const bool last = job->done.fetch_add(1, std::memory_order_acq_rel) + 1 == n;   // after this the job may be gone
+    lock.lock();
+    if (last) p->finished.notify_all();
+  }
+}
+
+}  // namespace
+
+int nd_host_threads() {
+  if (const char *e = getenv("ND_HOST_THREADS")) {
+    const int n = atoi(e);
+    if (n >= 1) return n < 256 ? n : 256;
+  }
+  const unsigned hc = std::thread::hardware_concurrency();
+  return hc == 0 ? 4 : (hc > 32 ? 32 : (int)hc);
+}
+
+void nd_host_run(int n, const std::function<void(int)> &task, const std::function<void()> &own) {
+  if (n <= 0 || (n == 1 && !own)) {
+    if (own) own();
+    if (n == 1) task(0);
+    return;
+  }
+  Pool *p = pool();
+  Job job;
+  job.task = &task;
+  job.n = n;
+  {
+    std::lock_guard<std::mutex> lock(p->m);
+    p->jobs.push_back(&job);
+    const int want = std::min(own ? n : n - 1, nd_host_threads() - 1) - p->idle;
+    for (int k = 0; k < want && p->workers < 256; k++) {
+      try {
+        std::thread(worker, p).detach();
+        p->workers++;
+      } catch (...) {   // out of threads: the caller does it
+        break;
+      }
+    }
+  }
+  p->work.notify_all();
+  if (own) own();
+  for (;;) {   // the caller's share
+    const int i = job.next.fetch_add(1, std::memory_order_relaxed);
+    if (i >= n) break;
+    task(i);
+    job.done.fetch_add(1, std::memory_order_acq_rel);
+  }
+  std::unique_lock<std::mutex> lock(p->m);
+  p->jobs.erase(std::remove(p->jobs.begin(), p->jobs.end(), &job), p->jobs.end());
+  p->finished.wait(lock, [&] { return job.done.load(std::memory_order_acquire) == n; });
+}
+
+// ---------------------------------------------------------------- staged copies
+
+namespace {
+
+constexpr size_t PIECE = (size_t)1 << 20;   // 1 MB: twenty microseconds on the wire
+constexpr int RING = 8;                    // pinned pieces
+constexpr size_t STAGED_MIN = (size_t)2 << 20;   // below this the plain call is as fast
+
+struct Ring {
+  std::mutex m;                 // one copy at a time
+  unsigned char *pinned = nullptr;
+  int device = -1;              // of the stream and the events
+  cudaStream_t stream = nullptr;
+  cudaEvent_t done[RING] = {};  // the piece's transfer
+};
+Ring g_ring;
+std::mutex g_objects_mutex;
+int g_objects = 0;
+std::atomic<bool> g_exiting{false};   // the process is on its way out: leave the driver alone
+
+void ring_device_free() {
+  if (g_ring.stream) cudaStreamDestroy(g_ring.stream);
+  g_ring.stream = nullptr;
+  for (cudaEvent_t &e : g_ring.done) { if (e) cudaEventDestroy(e); e = nullptr; }
+  g_ring.device = -1;
+}
+
+// under g_ring.m, with `device` current
+bool ring_ready(int device) {
+  if (!g_ring.pinned && cudaHostAlloc(&g_ring.pinned, PIECE * RING, cudaHostAllocPortable) != cudaSuccess) {
+    cudaGetLastError();
+    g_ring.pinned = nullptr;
+    return false;
+  }
+  static const int once = atexit([] { g_exiting.store(true); });
+  (void)once;
+  if (g_ring.device == device) return true;
+  ring_device_free();
+  bool ok = cudaStreamCreateWithFlags(&g_ring.stream, cudaStreamNonBlocking) == cudaSuccess;
+  for (int i = 0; i < RING && ok; i++) ok = cudaEventCreateWithFlags(&g_ring.done[i], cudaEventDisableTiming) == cudaSuccess;
+  if (!ok) { cudaGetLastError(); ring_device_free(); return false; }
+  g_ring.device = device;
+  return true;
+}
+
+bool pageable(const void *p) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return true; }
+  return at.type == cudaMemoryTypeUnregistered;
+}
+
+// Piece k of the copy uses slot k % RING.  The caller alone talks to the driver (threads that wait for
+// events get in each other's way): it enqueues the pieces in order and publishes how many
+// transfers are over.  The workers move pieces between the slots and the user's memory; the caller does so when
+// none of them has got on for a while, so the copy ends without them too.
+int staged(unsigned char *host, unsigned char *dev, size_t bytes, bool up) {
+  const size_t pieces = (bytes + PIECE - 1) / PIECE;
+  std::vector<std::atomic<char>> moved(pieces);   // the host side of the piece is done
+  std::atomic<size_t> over{0};                    // transfers that are complete
+  std::atomic<size_t> next{0};                    // next piece to move
+  std::atomic<bool> stop{false};
+  auto size = [&](size_t k) { return k + 1 < pieces ? PIECE : bytes - k * PIECE; };
+  // up: the slot's last transfer is over; down: the piece's own is
+  auto movable = [&](size_t k) { return up ? k < over.load(std::memory_order_acquire) + RING : k < over.load(std::memory_order_acquire); };
+  auto move = [&](size_t k) {
+    unsigned char *slot = g_ring.pinned + (k % RING) * PIECE;
+    if (up) memcpy(slot, host + k * PIECE, size(k));
+    else memcpy(host + k * PIECE, slot, size(k));
+    moved[k].store(1, std::memory_order_release);
+  };
+  std::atomic<int> helpers{0};                    // workers at it
+  auto mover = [&] {
+    helpers.fetch_add(1);
+    for (;;) {
+      const size_t k = next.fetch_add(1);
+      if (k >= pieces) return;
+      for (int spins = 0; !movable(k); spins++) {
+        if (stop.load(std::memory_order_relaxed)) return;
+        if (spins > 500) std::this_thread::yield();
+      }
+      move(k);
+    }
+  };
+  cudaError_t err = cudaSuccess;
+  auto driver = [&] {
+    size_t sent = 0, done = 0;
+    auto last = std::chrono::steady_clock::now();
+    while (done < pieces) {
+      if (sent < pieces && sent < done + RING && (up ? moved[sent].load(std::memory_order_acquire) != 0 : sent < RING || moved[sent - RING].load(std::memory_order_acquire) != 0)) {
+        unsigned char *slot = g_ring.pinned + (sent % RING) * PIECE;
+        err = up ? cudaMemcpyAsync(dev + sent * PIECE, slot, size(sent), cudaMemcpyHostToDevice, g_ring.stream)
+                 : cudaMemcpyAsync(slot, dev + sent * PIECE, size(sent), cudaMemcpyDeviceToHost, g_ring.stream);
+        if (err == cudaSuccess) err = cudaEventRecord(g_ring.done[sent % RING], g_ring.stream);
+        if (err != cudaSuccess) return;
+        sent++;
+        last = std::chrono::steady_clock::now();
+        continue;
+      }
+      if (done < sent) {
+        const cudaError_t q = cudaEventQuery(g_ring.done[done % RING]);
+        if (q == cudaSuccess) {
+          over.store(++done, std::memory_order_release);
+          last = std::chrono::steady_clock::now();
+          continue;
+        }
+        if (q != cudaErrorNotReady) { err = q; return; }
+      }
+      // (waking a worker takes as long as moving a piece or two: until one is there the caller moves)
+      if (helpers.load(std::memory_order_relaxed) > 0 && std::chrono::steady_clock::now() - last < std::chrono::microseconds(200)) continue;
+      size_t k = next.load();
+      if (k < pieces && movable(k) && next.compare_exchange_strong(k, k + 1)) move(k);
+    }
+  };
+  // five keep up with the wire (more help where the destination is fresh memory, 15 -> 20 GB/s, but take longer to wake)
+  const int movers = (int)std::min<size_t>(std::min<size_t>(pieces, 5), (size_t)std::max(1, nd_host_threads() - 1));
+  nd_host_run(movers, [&](int) { mover(); }, [&] {
+    driver();
+    stop.store(err != cudaSuccess);
+  });
+  cudaError_t e = cudaStreamSynchronize(g_ring.stream);   // nothing of the ring is in flight, whatever happened
+  if (err != cudaSuccess) e = err;
+  cudaGetLastError();   // a query that was not ready counts as an error of the thread
+  ND_REQUIRE(e == cudaSuccess, ND_ERR_CUDA, "staged copy of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+  return ND_OK;
+}
+
+int copy(int device, void *dst, const void *src, size_t bytes, bool up) {
+  if (bytes == 0) return ND_OK;
+  ND_CUDA(cudaSetDevice(device));
+  if (bytes >= STAGED_MIN && nd_host_threads() > 2 && pageable(up ? src : dst)) {
+    std::unique_lock<std::mutex> lock(g_ring.m, std::try_to_lock);
+    if (lock.owns_lock() && ring_ready(device))
+      return up ? staged((unsigned char *)const_cast<void *>(src), (unsigned char *)dst, bytes, true)
+                : staged((unsigned char *)dst, (unsigned char *)const_cast<void *>(src), bytes, false);
+  }
+  ND_CUDA(cudaMemcpy(dst, src, bytes, up ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost));
+  return ND_OK;
+}
+
+}  // namespace
+
+int nd_copy_to_host(int device, void *dst, const void *src, size_t bytes) { return copy(device, dst, src, bytes, false); }
+int nd_copy_to_device(int device, void *dst, const void *src, size_t bytes) { return copy(device, dst, src, bytes, true); }
+
+// ---------------------------------------------------------------- device memory pool
+
+namespace {
+constexpr uint64_t POOL_KEEP = (uint64_t)1 << 30;
+std::mutex g_pools_mutex;
+std::vector<cudaMemPool_t> g_pools;   // by device, made at the first allocation
+
+int pool_of(int device, cudaMemPool_t *pool) {
+  std::lock_guard<std::mutex> lock(g_pools_mutex);
+  if ((size_t)device >= g_pools.size()) g_pools.resize((size_t)device + 1, nullptr);
+  if (!g_pools[(size_t)device]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t p = nullptr;
+    ND_CUDA(cudaMemPoolCreate(&p, &props));
+    uint64_t keep = POOL_KEEP;
+    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    g_pools[(size_t)device] = p;
+  }
+  *pool = g_pools[(size_t)device];
+  return ND_OK;
+}
+}  // namespace
+
+int nd_pool_alloc(int device, void **p, size_t bytes) {
+  cudaMemPool_t pool = nullptr;
+  ND_TRY(pool_of(device, &pool));
+  ND_CUDA(cudaMallocFromPoolAsync(p, bytes, pool, nullptr));
+  return ND_OK;
+}
+
+void nd_pool_free(int device, void *p) {
+  if (!p) return;
+  cudaSetDevice(device);
+  cudaDeviceSynchronize();   // as cudaFree: no stream uses it any more
+  cudaFreeAsync(p, nullptr);
+}
+
+void nd_objects_add(int n) {
+  std::lock_guard<std::mutex> lock(g_objects_mutex);
+  g_objects += n;
+  if (g_objects > 0) return;
+  std::lock_guard<std::mutex> pools(g_pools_mutex);
+  int now = 0;
+  cudaGetDevice(&now);
+  for (size_t d = 0; d < g_pools.size(); d++)
+    if (g_pools[d]) {
+      cudaSetDevice((int)d);
+      cudaStreamSynchronize(nullptr);
+      cudaMemPoolTrimTo(g_pools[d], 0);
+    }
+  cudaSetDevice(now);
+}
+
+// The last worker ends, a second after the last work: without graphs and samplers the ring goes too.
+static void nd_host_idle() {
+  {
+    std::lock_guard<std::mutex> lock(g_objects_mutex);
+    if (g_objects > 0) return;
+  }
+  std::unique_lock<std::mutex> ring(g_ring.m, std::try_to_lock);
+  if (!ring.owns_lock() || g_exiting.load()) return;
+  ring_device_free();
+  if (g_ring.pinned) cudaFreeHost(g_ring.pinned);
+  g_ring.pinned = nullptr;
+}

@@ -1,0 +1,37 @@
+// Host side of the library: worker threads and staged transfers between pageable memory and the device.
+#pragma once
+
+#include <stddef.h>
+#include <stdint.h>
+
+#include <functional>
+
+// Host threads of the library's own work (ND_HOST_THREADS, default the hardware threads, at most 32).
+int nd_host_threads();
+
+// Runs task(0) .. task(n - 1) on the caller and the library's workers and returns when all are done; the caller runs
+// `own` first, while workers may be at the tasks already.  Tasks must not wait for one another.  Workers are
+// started when there is work for them, at most nd_host_threads() - 1, and end after a second without any; a
+// worker that cannot be started is done without.  Several threads may call it at the same time.
+void nd_host_run(int n, const std::function<void(int)> &task, const std::function<void()> &own = nullptr);
+
+// fn(range, first, end) on `threads` contiguous ranges of [0, count)
+template <class F>
+void nd_host_ranges(int64_t count, int threads, F fn) {
+  if (threads > count) threads = count > 0 ? (int)count : 1;
+  nd_host_run(threads, [&](int t) { fn(t, count * t / threads, count * (t + 1) / threads); });
+}
+
+// Blocking copies on a stream of their own: everything the copy depends on has to be complete.
+int nd_copy_to_host(int device, void *dst, const void *src, size_t bytes);
+int nd_copy_to_device(int device, void *dst, const void *src, size_t bytes);
+
+// Device memory that is kept for the next allocation when it is freed, up to POOL_KEEP bytes per device while graphs
+// or samplers are alive (a cudaMalloc / cudaFree pair of a large block costs 0.5 to 30 ms, by the box).  Allocation
+// and release are ordered like work on the default stream; the release waits for the device.
+int nd_pool_alloc(int device, void **p, size_t bytes);
+void nd_pool_free(int device, void *p);
+
+// Graphs and samplers alive: without any, the pool keeps nothing, and the staging memory of the
+// copies is returned when the workers end.
+void nd_objects_add(int n);

@@ -12,12 +12,10 @@
 // previous update of that array.  Three calls, so that the caller can overlap them with the next
 // job's sampling: begin (enqueue) -> fetch (lengths have landed: enqueue the vertices) -> finish
 // (vertices have landed: write the rows).
-#include <stdlib.h>
-
-#include <thread>
 #include <vector>
 
 #include "nd_common.cuh"
+#include "nd_host.h"
 
 struct NdHostRows {
   int32_t *h_len = nullptr;     // pinned [S]: the rows' lengths of the job being copied
@@ -153,35 +151,6 @@ pack_rows_kernel(const int32_t *__restrict__ plen, const int32_t *__restrict__ o
 // positions in the packed array are 32-bit
 bool packable(const nd_sampler *s) { return s->S * (int64_t)s->fs < ((int64_t)1 << 32); }
 
-int host_threads() {
-  if (const char *e = getenv("ND_HOST_THREADS")) {
-    const int n = atoi(e);
-    if (n >= 1) return n < 256 ? n : 256;
-  }
-  const unsigned hc = std::thread::hardware_concurrency();
-  return hc == 0 ? 4 : (hc > 32 ? 32 : (int)hc);
-}
-
-// runs fn(t, first_row, end_row) on `threads` contiguous row ranges; a range whose thread cannot be
-// started (the process is out of threads) is run by the caller, so nothing escapes the C boundary
-template <class F>
-void for_row_ranges(int64_t S, int threads, F fn) {
-  if (threads > S) threads = S > 0 ? (int)S : 1;
-  std::vector<std::thread> pool;
-  pool.reserve((size_t)threads);
-  int started = 1;
-  for (; started < threads; started++) {
-    try {
-      pool.emplace_back(fn, started, S * started / threads, S * (started + 1) / threads);
-    } catch (...) {
-      break;
-    }
-  }
-  fn(0, (int64_t)0, S / threads);
-  for (int t = started; t < threads; t++) fn(t, S * t / threads, S * (t + 1) / threads);
-  for (auto &th : pool) th.join();
-}
-
 // staging state of a sampler, made at the first use
 int hostrows_init(nd_sampler *s) {
   if (s->hostrows) return ND_OK;
@@ -189,7 +158,7 @@ int hostrows_init(nd_sampler *s) {
   NdHostRows *h = s->hostrows;
   const size_t S1 = (size_t)(s->S > 0 ? s->S : 1);
   h->n_chunks = (int)((S1 + PACK_ROWS - 1) / PACK_ROWS);
-  h->threads = host_threads();
+  h->threads = nd_host_threads();
   cudaError_t e = cudaMallocHost(&h->h_len, sizeof(int32_t) * S1);
   if (e == cudaSuccess) e = cudaMallocHost(&h->h_total, sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMalloc(&h->d_chunk, sizeof(uint32_t) * ((size_t)h->n_chunks + 1));
@@ -242,7 +211,7 @@ extern "C" {
 int nd_host_fill_int32(int32_t *dst, int64_t n, int32_t value) {
   ND_REQUIRE(dst || n == 0, ND_ERR_ARG, "nd_host_fill_int32: null destination");
   ND_REQUIRE(n >= 0, ND_ERR_ARG, "nd_host_fill_int32: negative length");
-  for_row_ranges(n, host_threads(), [=](int, int64_t a, int64_t b) {
+  nd_host_ranges(n, nd_host_threads(), [=](int, int64_t a, int64_t b) {
     for (int64_t i = a; i < b; i++) dst[i] = value;
   });
   return ND_OK;
@@ -288,7 +257,7 @@ int nd_sampler_host_update_fetch(nd_sampler *s) {
   ND_CUDA(cudaEventSynchronize(h->len_done));
   std::vector<int64_t> part((size_t)h->threads, 0);
   const int32_t *len = h->h_len;
-  for_row_ranges(s->S, h->threads, [&](int t, int64_t a, int64_t b) {
+  nd_host_ranges(s->S, h->threads, [&](int t, int64_t a, int64_t b) {
     int64_t sum = 0;
     for (int64_t i = a; i < b; i++) sum += len[i];
     part[(size_t)t] = sum;
@@ -330,20 +299,20 @@ int nd_sampler_host_update_finish(nd_sampler *s, int64_t *values_copied) {
   const int steps = s->fs;
   const int32_t invalid = s->g->V;
   if (h->dense) {  // the whole array came over as it is: only the lengths are left to note
-    for_row_ranges(s->S, h->threads, [=](int, int64_t a, int64_t b) {
+    nd_host_ranges(s->S, h->threads, [=](int, int64_t a, int64_t b) {
       for (int64_t i = a; i < b; i++) row_len[i] = len[i];
     });
     return ND_OK;
   }
   // every thread needs the position of its first row in the packed array: the ranges' sums again
   std::vector<int64_t> part((size_t)h->threads + 1, 0);
-  for_row_ranges(s->S, h->threads, [&](int t, int64_t a, int64_t b) {
+  nd_host_ranges(s->S, h->threads, [&](int t, int64_t a, int64_t b) {
     int64_t sum = 0;
     for (int64_t i = a; i < b; i++) sum += len[i];
     part[(size_t)t + 1] = sum;
   });
   for (size_t t = 1; t < part.size(); t++) part[t] += part[t - 1];
-  for_row_ranges(s->S, h->threads, [&, out, row_len, len, vals](int t, int64_t a, int64_t b) {
+  nd_host_ranges(s->S, h->threads, [&, out, row_len, len, vals](int t, int64_t a, int64_t b) {
     const int32_t *src = vals + part[(size_t)t];
     for (int64_t i = a; i < b; i++) {
       const int32_t now = len[i], had = row_len[i];

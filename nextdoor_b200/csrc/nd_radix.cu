@@ -319,14 +319,24 @@ NdRadixPlan nd_radix_plan(int key_bits, int64_t max_n) {
 
 // The scratch is sized for the widest digit any plan over max_n pairs may pick, so one allocation
 // serves sorts on keys of different widths (transit ids, edge endpoints, weight bits).
-int nd_radix_scratch_alloc(NdRadixScratch *s, int key_bits, int64_t max_n) {
-  s->plan = nd_radix_plan(key_bits, max_n);
-  s->cap_bins = 1 << nd_radix_max_digit(max_n);
-  s->bytes = sizeof(uint32_t) * ((size_t)s->cap_bins * s->plan.max_tiles + 8 * (size_t)s->cap_bins);
-  void *p = nullptr;
-  ND_CUDA(cudaMalloc(&p, s->bytes));
-  s->tile_hist = (uint32_t *)p;
+size_t nd_radix_scratch_bytes(int64_t max_n) {
+  const size_t bins = (size_t)1 << nd_radix_max_digit(max_n);
+  return sizeof(uint32_t) * (bins * (size_t)nd_radix_plan(1, max_n).max_tiles + 8 * bins);
+}
+
+// histograms in `at`: nd_radix_scratch_bytes(plan.max_n) bytes of cleared device memory
+void nd_radix_scratch_place(NdRadixScratch *s, const NdRadixPlan &plan, void *at) {
+  s->plan = plan;
+  s->cap_bins = 1 << nd_radix_max_digit(plan.max_n);
+  s->bytes = nd_radix_scratch_bytes(plan.max_n);
+  s->tile_hist = (uint32_t *)at;
   s->ghist = s->tile_hist + (size_t)s->cap_bins * s->plan.max_tiles;
+}
+
+int nd_radix_scratch_alloc(NdRadixScratch *s, int key_bits, int64_t max_n) {
+  void *p = nullptr;
+  ND_CUDA(cudaMalloc(&p, nd_radix_scratch_bytes(max_n)));
+  nd_radix_scratch_place(s, nd_radix_plan(key_bits, max_n), p);
   ND_CUDA(cudaMemset(s->ghist, 0, sizeof(uint32_t) * 8 * s->cap_bins));
   return ND_OK;
 }

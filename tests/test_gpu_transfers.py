@@ -1,0 +1,68 @@
+"""Results and graphs through the staged copies: sizes around a piece and around the size below which the plain copy
+is used, odd addresses, pinned destinations, several threads at once; the loader with weights that do not differ."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+MB = 1 << 20
+
+
+@pytest.mark.parametrize("nbytes", [4, 2 * MB - 4, 2 * MB, 2 * MB + 4, 9 * MB - 4, 9 * MB + 4, 41 * MB])
+def test_final_samples_of_every_size(nd, small_graph, nbytes):
+    import torch
+    from nextdoor_b200 import dist as nd_dist
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    s = nd.Sampler(g, nd.app_params(0, steps=1, seed=2), num_samples=nbytes // 4)
+    s.sample()
+    exp = nd_dist.device_samples(s).cpu().numpy()
+    assert np.array_equal(s.final_samples(), exp)
+    raw = np.zeros(nbytes + 64, np.uint8)
+    for off in (0, 4, 60):
+        out = raw[off:off + nbytes].view(np.int32)
+        out[:] = -9
+        s.final_samples(out)
+        assert np.array_equal(out, exp.reshape(-1))
+    pinned = torch.full((nbytes // 4,), -9, dtype=torch.int32).pin_memory().numpy()
+    s.final_samples(pinned)
+    assert np.array_equal(pinned, exp.reshape(-1))
+
+
+def test_several_threads_copy_at_once(nd, small_graph):
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    samplers = [nd.Sampler(g, nd.app_params(0, steps=10, seed=k), num_samples=300_000) for k in range(4)]
+    for s in samplers:
+        s.sample()
+    exp = [s.final_samples() for s in samplers]
+    wrong = []
+
+    def work(k):
+        for _ in range(5):
+            if not np.array_equal(samplers[k].final_samples(), exp[k]):
+                wrong.append(k)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+
+
+@pytest.mark.parametrize("n", [0, 1, 2, 1000, 300_000])
+@pytest.mark.parametrize("weights", ["same", "two", "low bits", "signs", "random"])
+def test_loader_sorts_by_all_bits_that_differ(nd, ndo, n, weights):
+    rng = np.random.default_rng(n)
+    V = 700
+    src, dst = rng.integers(0, V, n).astype(np.int32), rng.integers(0, V // 8, n).astype(np.int32)
+    w = {"same": np.full(n, 1.5), "two": rng.choice([1.0, 1.0 + 2.0 ** -23], n), "low bits": 1.0 + rng.integers(0, 4, n) * 2.0 ** -22,
+         "signs": rng.choice([-2.0, -1.0, 1.0, 2.0], n), "random": rng.random(n) * 4 + 1}[weights].astype(np.float32)
+    g = nd.Graph.from_edge_records(src, dst, w)
+    row_ptr, col, got_w, max_w = g.to_host()
+    order = np.lexsort((w, dst, src))
+    assert np.array_equal(col, dst[order]) and np.array_equal(got_w, w[order])
+    assert np.array_equal(np.diff(row_ptr), np.bincount(src, minlength=g.V)[: g.V])
+    exp_max = np.zeros(g.V, np.float32)
+    np.maximum.at(exp_max, src, w)
+    assert np.array_equal(max_w, exp_max)
