@@ -127,7 +127,7 @@ void free_sampler(nd_sampler *s) {
   for (int i = 0; i < 2; i++) { cudaFree(s->d_map_key[i]); cudaFree(s->d_map_val[i]); }
   cudaFree(s->d_init_key); cudaFree(s->d_init_val); cudaFree(s->d_nlive); cudaFree(s->d_stats); status_word_put(s->h_status);
   cudaFree(s->d_runs); cudaFree(s->d_bin_counts); cudaFree(s->d_hop_counts);
-  cudaFree(s->d_adj_row); cudaFree(s->d_adj_col); cudaFree(s->d_prob); cudaFree(s->d_cand); cudaFree(s->d_cand_w); cudaFree(s->d_acc); cudaFree(s->d_bm);
+  cudaFree(s->d_adj_row); cudaFree(s->d_adj_col); cudaFree(s->d_prob); cudaFree(s->d_cand); cudaFree(s->d_cand_w); cudaFree(s->d_bm);
   cudaFree(s->d_cnt); cudaFree(s->d_offs); cudaFree(s->d_bsum); cudaFree(s->d_rank);
   for (int i = 0; i < 2; i++) cudaFree(s->d_srec[i]);
   cudaFree(s->d_init_rec); cudaFree(s->d_list); cudaFree(s->d_rows_acc);

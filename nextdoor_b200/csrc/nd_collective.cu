@@ -27,79 +27,182 @@
 #include <cstdlib>
 #include <vector>
 
-#include "nd_common.cuh"
-#include "nd_philox.cuh"
+#include "nd_collective.cuh"
 
 namespace {
 
 using ndrng::Rng;
 constexpr int CTHREADS = 256;
 
-struct CollParams {
-  uint64_t seed;
-  int64_t first_sample;
-  int32_t V, fs, L, B, stride, step, ntr;
-  int app;
+// ---------------------------------------------------------------- reference semantics: uniform over V
+//
+// A layer's vertices are drawn from the whole graph, whatever the transits are, so all layers of a pass are drawn
+// first and all their (transit, layer) pairs are probed together: the transits' lists are flattened over the
+// CTA, every entry asks a filter of the layer's ids in shared memory, and the few that pass look for the id.
+// A list longer than PROBE_RATIO times the layer is bisected for every id instead.  (One bisection per
+// (transit, slot) pair, 205 M of them for 10,000 samples of 5 x 64 x 64 on 57 K vertices: 1.04 ms, now 0.57.)
+// What is left is the 1.6 GB of adjacency entries, in 16-byte stores.
+constexpr int FILTER_WORDS = 256;   // 8192 bits per layer
+constexpr int PROBE_RATIO = 8;
+
+struct RefLayout {
+  int per_pass;                                                        // layers drawn and probed together
+  uint32_t off_ids, off_tr, off_rs, off_deg, off_pre, off_filter, off_flags;    // bytes
+  uint32_t bytes;
+  int flag_words;                                                      // per transit
 };
 
-__device__ __forceinline__ const int32_t *transits_of(const CollParams &cp, const int32_t *initial, const int32_t *out, int64_t s) {
-  return cp.step == 0 ? initial + s * cp.B : out + s * cp.fs + (int64_t)(cp.step - 1) * cp.L;
-}
-
-__device__ __forceinline__ bool has_edge_logn(const NdGraphView &g, int32_t src, int32_t dst) {
-  int32_t l = __ldg(g.row_ptr + src), r = __ldg(g.row_ptr + src + 1) - 1;
-  while (l <= r) {
-    const int32_t m = l + (r - l) / 2;
-    const int32_t e = __ldg(g.col + m);
-    if (e == dst) return true;
-    if (e < dst) l = m + 1; else r = m - 1;
-  }
-  return false;
-}
-
-// adjacency entries of one layer of one sample: (row,col) = (i,j) where transit i -- vertex j is an edge
-__device__ __forceinline__ void emit_adjacency(const NdGraphView &g, const CollParams &cp, const int32_t *tr,
-                                               const int32_t *layer, int32_t *arow, int32_t *acol) {
-  for (int e = threadIdx.x; e < cp.stride; e += blockDim.x) {
-    const int i = e / cp.L, j = e - i * cp.L;
-    int32_t ri = -1, cj = -1;
-    if (i < cp.ntr) {
-      const int32_t t = tr[i], v = layer[j];
-      if (t >= 0 && t < cp.V && v >= 0 && v < cp.V && has_edge_logn(g, t, v)) { ri = i; cj = j; }
-    }
-    arow[e] = ri;
-    acol[e] = cj;
+static RefLayout ref_layout(int steps, int B, int L) {
+  RefLayout r;
+  const int ntr = B > L ? B : L;
+  r.flag_words = (L + 31) / 32;
+  for (r.per_pass = steps;; r.per_pass--) {
+    const uint32_t k = (uint32_t)r.per_pass, nt = k * (uint32_t)ntr;
+    uint32_t off = 0;
+    r.off_ids = off; off += 4u * (k + 1u) * (uint32_t)L;   // the layer before the pass too: its transits
+    r.off_tr = off; off += 4u * nt;
+    r.off_rs = off; off += 4u * nt;
+    r.off_deg = off; off += 4u * nt;
+    r.off_pre = off; off += 4u * (nt + 1u);
+    r.off_filter = off; off += 4u * k * FILTER_WORDS;
+    r.off_flags = off; off += 4u * nt * (uint32_t)r.flag_words;
+    r.bytes = off;
+    if (r.per_pass == 1 || off <= 24u * 1024u) return r;
   }
 }
 
-// ---------------------------------------------------------------- reference semantics: uniform over V
 __global__ void __launch_bounds__(CTHREADS)
-coll_ref_kernel(NdGraphView g, CollParams cp, int steps, int64_t S, const int32_t *__restrict__ initial, int32_t *out,
+coll_ref_kernel(NdGraphView g, CollParams cp, RefLayout lay, int steps, int64_t S, const int32_t *__restrict__ initial, int32_t *__restrict__ out,
                 int32_t *__restrict__ adj_row, int32_t *__restrict__ adj_col, unsigned long long *__restrict__ stats) {
-  __shared__ int32_t sh_tr[1024];
-  __shared__ int32_t sh_layer[1024];
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ uint32_t red[CTHREADS / 32];
+  int32_t *ids = reinterpret_cast<int32_t *>(sm + lay.off_ids);
+  int32_t *tr = reinterpret_cast<int32_t *>(sm + lay.off_tr), *rs = reinterpret_cast<int32_t *>(sm + lay.off_rs), *deg_of = reinterpret_cast<int32_t *>(sm + lay.off_deg);
+  __shared__ int heavy;   // transits whose lists are bisected: the first entries of tr
+  uint32_t *pre = reinterpret_cast<uint32_t *>(sm + lay.off_pre);
+  uint32_t *filter = reinterpret_cast<uint32_t *>(sm + lay.off_filter), *flags = reinterpret_cast<uint32_t *>(sm + lay.off_flags);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, L = cp.L;
   for (int64_t s = blockIdx.x; s < S; s += gridDim.x) {
-    for (int step = 0; step < steps; step++) {
-      cp.step = step;
-      cp.ntr = step == 0 ? cp.B : cp.L;
-      const int32_t *tr = transits_of(cp, initial, out, s);
-      for (int i = threadIdx.x; i < cp.ntr; i += CTHREADS) sh_tr[i] = tr[i];
-      for (int j = threadIdx.x; j < cp.L; j += CTHREADS) {
-        Rng rng(cp.seed, (uint32_t)(cp.first_sample + s), (uint32_t)step, (uint32_t)j);
+    for (int k0 = 0; k0 < steps; k0 += lay.per_pass) {
+      const int kn = min(lay.per_pass, steps - k0);
+      // transits of the pass, back to back: the batch (first layer of the sample), then the layers before
+      const int n0 = k0 == 0 ? cp.B : L, nt = n0 + (kn - 1) * L;
+      __syncthreads();   // the pass before has written its entries
+      if (tid == 0) heavy = 0;
+      if (k0 > 0) for (int j = tid; j < L; j += CTHREADS) ids[j] = ids[lay.per_pass * L + j];
+      for (int i = tid; i < kn * FILTER_WORDS; i += CTHREADS) filter[i] = 0u;
+      for (int i = tid; i < nt * lay.flag_words; i += CTHREADS) flags[i] = 0u;
+      __syncthreads();
+      for (int q = tid; q < kn * L; q += CTHREADS) {
+        const int k = q / L, j = q - k * L;
+        Rng rng(cp.seed, (uint32_t)(cp.first_sample + s), (uint32_t)(k0 + k), (uint32_t)j);
         const int32_t id = rng.rand_int(cp.V);
-        sh_layer[j] = id;
-        out[s * cp.fs + (int64_t)step * cp.L + j] = id;
+        ids[L + q] = id;
+        out[s * cp.fs + (int64_t)k0 * L + q] = id;
+        atomicOr(filter + k * FILTER_WORDS + (((uint32_t)id >> 5) & (FILTER_WORDS - 1)), 1u << (id & 31));
       }
       __syncthreads();
-      const int64_t a = (s * steps + step) * (int64_t)cp.stride;
-      emit_adjacency(g, cp, sh_tr, sh_layer, adj_row + a, adj_col + a);
+      // rows of the transits; exclusive prefix of the lengths that are streamed
+      uint32_t carry = 0;
+      for (int i0 = 0; i0 < nt; i0 += CTHREADS) {
+        const int i = i0 + tid;
+        uint32_t n = 0;
+        if (i < nt) {
+          const int32_t t = i < n0 ? (k0 == 0 ? initial[s * cp.B + i] : ids[i]) : ids[L + (i - n0)];
+          int32_t at = 0, deg = 0;
+          if (t >= 0 && t < cp.V) { at = __ldg(g.row_ptr + t); deg = __ldg(g.row_ptr + t + 1) - at; }
+          if (deg > PROBE_RATIO * L) {   // bisected
+            const int h = atomicAdd(&heavy, 1);
+            tr[h] = i;
+          }
+          rs[i] = at;
+          deg_of[i] = deg;
+          n = deg > PROBE_RATIO * L ? 0u : (uint32_t)deg;
+        }
+        uint32_t inc = n;
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= o) inc += t;
+        }
+        if (lane == 31) red[warp] = inc;
+        __syncthreads();
+        uint32_t before = carry + inc - n, all = 0;
+        for (int w = 0; w < CTHREADS / 32; w++) {
+          if (w < warp) before += red[w];
+          all += red[w];
+        }
+        if (i < nt) pre[i] = before;
+        carry += all;
+        __syncthreads();
+      }
+      // the entries of the short lists; a thread's loads are independent
+      constexpr int LOADS = 4;
+      for (uint32_t f0 = (uint32_t)tid; f0 < carry; f0 += CTHREADS * LOADS) {
+        int32_t v[LOADS];
+        int at[LOADS];
+#pragma unroll
+        for (int j = 0; j < LOADS; j++) {
+          const uint32_t f = f0 + (uint32_t)(j * CTHREADS);
+          v[j] = -1; at[j] = 0;
+          if (f < carry) {
+            int lo = 0, hi = nt - 1;   // last transit with pre <= f
+            while (lo < hi) {
+              const int mid = (lo + hi + 1) >> 1;
+              if (pre[mid] <= f) lo = mid; else hi = mid - 1;
+            }
+            at[j] = lo;
+            v[j] = __ldg(g.col + rs[lo] + (int32_t)(f - pre[lo]));
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < LOADS; j++) {
+          if (v[j] < 0) continue;
+          const int k = at[j] < n0 ? 0 : 1 + (at[j] - n0) / L;
+          if (!((filter[k * FILTER_WORDS + (((uint32_t)v[j] >> 5) & (FILTER_WORDS - 1))] >> (v[j] & 31)) & 1u)) continue;
+          const int32_t *layer = ids + L + k * L;
+          for (int q = 0; q < L; q++)
+            if (layer[q] == v[j]) atomicOr(flags + at[j] * lay.flag_words + (q >> 5), 1u << (q & 31));
+        }
+      }
+      const int nheavy = heavy;
+      for (int q = tid; q < nheavy * L; q += CTHREADS) {
+        const int i = tr[q / L], j = q % L, k = i < n0 ? 0 : 1 + (i - n0) / L;
+        const int32_t id = ids[L + k * L + j];
+        int32_t lo = rs[i], hi = rs[i] + deg_of[i];
+        while (lo < hi) {
+          const int32_t m = lo + ((hi - lo) >> 1);
+          if (__ldg(g.col + m) < id) lo = m + 1; else hi = m;
+        }
+        if (lo < rs[i] + deg_of[i] && __ldg(g.col + lo) == id) atomicOr(flags + i * lay.flag_words + (j >> 5), 1u << (j & 31));
+      }
       __syncthreads();
+      // adjacency entries: (row, col) = (i, j) where transit i -- vertex j is an edge
+      for (int k = 0; k < kn; k++) {
+        const int first = k == 0 ? 0 : n0 + (k - 1) * L, n = k == 0 ? n0 : L;
+        const int64_t a = (s * steps + k0 + k) * (int64_t)cp.stride;
+        auto set = [&](int i, int j) { return i < n && ((flags[(first + i) * lay.flag_words + (j >> 5)] >> (j & 31)) & 1u); };
+        if ((L & 3) == 0) {
+          int4 *ar = reinterpret_cast<int4 *>(adj_row + a), *ac = reinterpret_cast<int4 *>(adj_col + a);
+          for (int q = tid; q < cp.stride / 4; q += CTHREADS) {
+            const int i = 4 * q / L, j = 4 * q - i * L;
+            const uint32_t b = i < n ? (flags[(first + i) * lay.flag_words + (j >> 5)] >> (j & 31)) & 15u : 0u;
+            __stcs(ar + q, make_int4(b & 1u ? i : -1, b & 2u ? i : -1, b & 4u ? i : -1, b & 8u ? i : -1));
+            __stcs(ac + q, make_int4(b & 1u ? j : -1, b & 2u ? j + 1 : -1, b & 4u ? j + 2 : -1, b & 8u ? j + 3 : -1));
+          }
+        } else {
+          for (int e = tid; e < cp.stride; e += CTHREADS) {
+            const int i = e / L, j = e - i * L;
+            const bool b = set(i, j);
+            adj_row[a + e] = b ? i : -1;
+            adj_col[a + e] = b ? j : -1;
+          }
+        }
+      }
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    stats[0] = (unsigned long long)S * steps * cp.L;
-    stats[1] = (unsigned long long)S * (cp.B + (unsigned long long)(steps - 1) * cp.L);
-  }
+  if (blockIdx.x == 0 && tid < 8)
+    stats[tid] = tid == 0 ? (unsigned long long)S * steps * cp.L
+                 : tid == 1 ? (unsigned long long)S * (cp.B + (unsigned long long)(steps - 1) * cp.L) : 0ull;
 }
 
 // ---------------------------------------------------------------- importance sampling pipeline
@@ -262,349 +365,6 @@ coll_sample_kernel(NdGraphView g, CollParams cp, int steps, int64_t s0, int64_t 
   }
 }
 
-// ---------------------------------------------------------------- importance sampling, bitmap path
-//
-// When a bit per vertex fits the CTA's shared memory (V up to about 1.4 M with 227 KB), the union
-// of a sample's neighbour lists needs no sort: one CTA per sample streams the transits' lists and
-// sets the neighbours' bits; a popcount scan over groups of BM_GROUP_WORDS words ranks every set
-// bit, which is the candidate's index in the sorted unique union; the candidates' weights are
-// summed per group and scanned in fp64, and a draw bisects the group sums and then walks the one
-// group its target falls into.  FastGCN weights are recomputed from the row offsets where they are
-// needed; LADIES accumulates its terms per candidate rank in a global fp64 array (one V-entry
-// region per CTA) during a second pass over the lists.  No host round trip, no chunking: one
-// launch per layer for all samples.  Sums are fp64, so they agree with the sorted sequential
-// order to ~1e-16 (FastGCN's integer weights sum exactly).
-constexpr int BM_THREADS = 1024;
-constexpr int BM_GROUP_WORDS = 16;   // 512 candidates per group
-constexpr int BM_BIG_LIST = 4096;    // lists at least this long are streamed by the whole CTA
-
-// The bitmap, the group prefix counts and the group CDF make the "big" part (about V/8 + 3V/128
-// bytes); it lives in shared memory when the whole layout fits the CTA's opt-in shared memory
-// (graphs up to about 1.4 M vertices) and otherwise in a per-CTA slice of a global scratch array
-// (glob_bytes > 0), where the same code runs on L2-resident words.  The small part (transits,
-// layer, row sums, reduction scratch) is always in shared memory.
-struct BmLayout {
-  int words, groups;
-  uint32_t off_gcdf, off_gpref;                        // inside the big part (the bitmap is at 0)
-  uint32_t off_tr, off_layer, off_rowsum, off_red;     // inside shared memory
-  uint32_t bytes;                                      // dynamic shared memory of the launch
-  uint32_t glob_bytes;                                 // per-CTA slice of the global scratch, 0 = big part in shared memory
-};
-
-__device__ __forceinline__ void bm_mark(uint32_t *bm, int32_t v) {
-  const uint32_t bit = 1u << (v & 31);
-  uint32_t *wp = bm + ((uint32_t)v >> 5);
-  if (!(*(volatile uint32_t *)wp & bit)) atomicOr(wp, bit);  // hub lists overlap: most bits are set already
-}
-
-__device__ __forceinline__ uint32_t bm_rank(const uint32_t *bm, const uint32_t *gpref, int32_t v) {
-  const uint32_t word = (uint32_t)v >> 5, grp = word / BM_GROUP_WORDS;
-  uint32_t r = gpref[grp];
-  for (uint32_t k = grp * BM_GROUP_WORDS; k < word; k++) r += __popc(bm[k]);
-  return r + __popc(bm[word] & ((1u << (v & 31)) - 1u));
-}
-
-// Streams one neighbour list with STRIDE cooperating threads: sets the neighbours' bits and, for
-// LADIES, adds the weights to the caller's partial row sum.  The body of the list is read as
-// 16-byte vectors (the arrays are 256-byte aligned, so entry rs + head is 16-byte aligned for
-// head = (4 - rs % 4) % 4), BM_VEC vectors in flight per thread; head and tail entries one by one.
-constexpr int BM_UNROLL = 8;   // scalar loads in flight per thread (second LADIES pass)
-constexpr int BM_VEC = 4;      // 16-byte loads in flight per thread
-template <bool LADIES, int STRIDE>
-__device__ __forceinline__ void bm_stream(const NdGraphView &g, uint32_t *bm, int32_t rs, int32_t deg, int me, double &part) {
-  const int32_t *__restrict__ col = g.col + rs;
-  const float *__restrict__ wts = g.w + rs;
-  int head = (4 - (rs & 3)) & 3;
-  if (head > deg) head = deg;
-  if (me < head) {
-    bm_mark(bm, __ldg(col + me));
-    if (LADIES) part += (double)__ldg(wts + me);
-  }
-  const int n4 = (deg - head) >> 2;
-  const int4 *__restrict__ col4 = reinterpret_cast<const int4 *>(col + head);
-  const float4 *__restrict__ w4 = reinterpret_cast<const float4 *>(wts + head);
-  for (int e0 = me; e0 < n4; e0 += STRIDE * BM_VEC) {
-    int4 v[BM_VEC];
-    float4 w[BM_VEC];
-#pragma unroll
-    for (int k = 0; k < BM_VEC; k++) {
-      const int e = e0 + k * STRIDE;
-      v[k] = e < n4 ? __ldg(col4 + e) : make_int4(-1, -1, -1, -1);
-      if (LADIES) w[k] = e < n4 ? __ldg(w4 + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-#pragma unroll
-    for (int k = 0; k < BM_VEC; k++) {
-      if (v[k].x >= 0) { bm_mark(bm, v[k].x); bm_mark(bm, v[k].y); bm_mark(bm, v[k].z); bm_mark(bm, v[k].w); }
-      if (LADIES) part += ((double)w[k].x + (double)w[k].y) + ((double)w[k].z + (double)w[k].w);
-    }
-  }
-  for (int e = head + (n4 << 2) + me; e < deg; e += STRIDE) {
-    bm_mark(bm, __ldg(col + e));
-    if (LADIES) part += (double)__ldg(wts + e);
-  }
-}
-
-// LADIES second pass over one list: (w / rowsum)^2 of every entry added to its candidate's accumulator
-template <int STRIDE>
-__device__ __forceinline__ void bm_accumulate(const NdGraphView &g, const uint32_t *bm, const uint32_t *gpref, double *acc,
-                                              int32_t rs, int32_t deg, int me, float rowsum) {
-  for (int e0 = me; e0 < deg; e0 += STRIDE * BM_UNROLL) {
-    int32_t v[BM_UNROLL];
-    float w[BM_UNROLL];
-#pragma unroll
-    for (int k = 0; k < BM_UNROLL; k++) {
-      const int e = e0 + k * STRIDE;
-      v[k] = e < deg ? __ldg(g.col + rs + e) : -1;
-      w[k] = e < deg ? __ldg(g.w + rs + e) : 0.f;
-    }
-#pragma unroll
-    for (int k = 0; k < BM_UNROLL; k++) {
-      if (v[k] >= 0) {
-        const float r = __fdiv_rn(w[k], rowsum);
-        atomicAdd(acc + bm_rank(bm, gpref, v[k]), (double)__fmul_rn(r, r));
-      }
-    }
-  }
-}
-
-template <bool LADIES>
-__device__ __forceinline__ float bm_weight(const NdGraphView &g, const double *acc, int32_t v, uint32_t rank) {
-  if (LADIES) return (float)acc[rank];
-  const float d = __int2float_rn(__ldg(g.row_ptr + v + 1) - __ldg(g.row_ptr + v));
-  return __fmul_rn(d, d);
-}
-
-// exclusive (uint32) or inclusive (double) scan of a shared array by the whole CTA: every thread
-// owns a contiguous chunk, the chunk totals are scanned through warp shuffles
-__device__ __forceinline__ uint32_t bm_scan_u32(uint32_t *a, int n, uint32_t *red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int per = (n + BM_THREADS - 1) / BM_THREADS;
-  const int b = threadIdx.x * per, e = b + per < n ? b + per : n;
-  uint32_t sum = 0;
-  for (int i = b; i < e; i++) sum += a[i];
-  uint32_t inc = sum;
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += t;
-  }
-  if (lane == 31) red[warp] = inc;
-  __syncthreads();
-  uint32_t base = inc - sum;
-  for (int w = 0; w < warp; w++) base += red[w];
-  uint32_t total = 0;
-  for (int w = 0; w < BM_THREADS / 32; w++) total += red[w];
-  for (int i = b; i < e; i++) { const uint32_t c = a[i]; a[i] = base; base += c; }
-  __syncthreads();
-  return total;
-}
-
-__device__ __forceinline__ void bm_scan_f64(double *a, int n, double *red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int per = (n + BM_THREADS - 1) / BM_THREADS;
-  const int b = threadIdx.x * per, e = b + per < n ? b + per : n;
-  double sum = 0.0;
-  for (int i = b; i < e; i++) sum += a[i];
-  double inc = sum;
-  for (int o = 1; o < 32; o <<= 1) {
-    const double t = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += t;
-  }
-  if (lane == 31) red[warp] = inc;
-  __syncthreads();
-  double base = inc - sum;
-  for (int w = 0; w < warp; w++) base += red[w];
-  for (int i = b; i < e; i++) { base += a[i]; a[i] = base; }
-  __syncthreads();
-}
-
-template <bool LADIES>
-__global__ void __launch_bounds__(BM_THREADS, 1)
-coll_bitmap_kernel(NdGraphView g, CollParams cp, int steps, int64_t S, BmLayout lay, unsigned char *__restrict__ gscratch,
-                   const int32_t *__restrict__ initial, int32_t *out, double *__restrict__ acc_all, int32_t *__restrict__ adj_row,
-                   int32_t *__restrict__ adj_col, float *__restrict__ prob, unsigned long long *__restrict__ stats) {
-  extern __shared__ __align__(16) unsigned char bm_smem[];
-  unsigned char *big = lay.glob_bytes ? gscratch + (size_t)blockIdx.x * lay.glob_bytes : bm_smem;
-  uint32_t *bm = reinterpret_cast<uint32_t *>(big);
-  double *gcdf = reinterpret_cast<double *>(big + lay.off_gcdf);
-  uint32_t *gpref = reinterpret_cast<uint32_t *>(big + lay.off_gpref);
-  int32_t *sh_tr = reinterpret_cast<int32_t *>(bm_smem + lay.off_tr);
-  int32_t *sh_layer = reinterpret_cast<int32_t *>(bm_smem + lay.off_layer);
-  float *sh_rowsum = reinterpret_cast<float *>(bm_smem + lay.off_rowsum);
-  double *red = reinterpret_cast<double *>(bm_smem + lay.off_red);   // 32 doubles
-  uint32_t *red_u = reinterpret_cast<uint32_t *>(red + 32);           // 32 words
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  double *acc = LADIES ? acc_all + (size_t)blockIdx.x * (size_t)cp.V : nullptr;
-  unsigned long long ids_sum = 0, uniq_sum = 0;  // thread 0
-  uint32_t valid = 0;
-  for (int64_t s = blockIdx.x; s < S; s += gridDim.x) {
-    const int32_t *tr = transits_of(cp, initial, out, s);
-    for (int i = tid; i < cp.ntr; i += BM_THREADS) sh_tr[i] = tr[i];
-    for (int w = tid * 4; w < lay.words; w += BM_THREADS * 4) *reinterpret_cast<uint4 *>(bm + w) = make_uint4(0u, 0u, 0u, 0u);
-    __syncthreads();
-    // ---- pass 1: the union as a bitmap (and the LADIES row sums)
-    for (int i = warp; i < cp.ntr; i += BM_THREADS / 32) {  // short lists: a warp each
-      const int32_t t = sh_tr[i];
-      if (t < 0 || t >= cp.V) { if (LADIES && lane == 0) sh_rowsum[i] = 0.f; continue; }
-      const int32_t rs = __ldg(g.row_ptr + t), deg = __ldg(g.row_ptr + t + 1) - rs;
-      if (deg >= BM_BIG_LIST) continue;
-      double part = 0.0;
-      bm_stream<LADIES, 32>(g, bm, rs, deg, lane, part);
-      if (LADIES) {
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        if (lane == 0) sh_rowsum[i] = (float)part;
-      }
-    }
-    for (int i = 0; i < cp.ntr; i++) {  // long lists: the whole CTA
-      const int32_t t = sh_tr[i];
-      if (t < 0 || t >= cp.V) continue;
-      const int32_t rs = __ldg(g.row_ptr + t), deg = __ldg(g.row_ptr + t + 1) - rs;
-      if (tid == 0) ids_sum += (unsigned long long)deg;
-      if (deg < BM_BIG_LIST) continue;
-      double part = 0.0;
-      bm_stream<LADIES, BM_THREADS>(g, bm, rs, deg, tid, part);
-      if (LADIES) {
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        if (lane == 0) red[warp] = part;
-        __syncthreads();
-        if (tid == 0) {
-          double tot = 0.0;
-          for (int w = 0; w < BM_THREADS / 32; w++) tot += red[w];
-          sh_rowsum[i] = (float)tot;
-        }
-        __syncthreads();
-      }
-    }
-    __syncthreads();
-    // ---- candidates per group, ranks
-    for (int gi = tid; gi < lay.groups; gi += BM_THREADS) {
-      uint32_t c = 0;
-#pragma unroll
-      for (int k = 0; k < BM_GROUP_WORDS; k += 4) {
-        const uint4 q = *reinterpret_cast<const uint4 *>(bm + gi * BM_GROUP_WORDS + k);
-        c += __popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w);
-      }
-      gpref[gi] = c;
-    }
-    __syncthreads();
-    const uint32_t U = bm_scan_u32(gpref, lay.groups, red_u);
-    if (tid == 0) uniq_sum += U;
-    // ---- LADIES pass 2: the terms of every list entry, added to the candidate's accumulator
-    if (LADIES) {
-      for (uint32_t u = tid; u < U; u += BM_THREADS) acc[u] = 0.0;
-      __syncthreads();
-      for (int i = warp; i < cp.ntr; i += BM_THREADS / 32) {
-        const int32_t t = sh_tr[i];
-        if (t < 0 || t >= cp.V) continue;
-        const int32_t rs = __ldg(g.row_ptr + t), deg = __ldg(g.row_ptr + t + 1) - rs;
-        if (deg >= BM_BIG_LIST) continue;
-        bm_accumulate<32>(g, bm, gpref, acc, rs, deg, lane, sh_rowsum[i]);
-      }
-      for (int i = 0; i < cp.ntr; i++) {
-        const int32_t t = sh_tr[i];
-        if (t < 0 || t >= cp.V) continue;
-        const int32_t rs = __ldg(g.row_ptr + t), deg = __ldg(g.row_ptr + t + 1) - rs;
-        if (deg < BM_BIG_LIST) continue;
-        bm_accumulate<BM_THREADS>(g, bm, gpref, acc, rs, deg, tid, sh_rowsum[i]);
-      }
-      __syncthreads();
-    }
-    // ---- weight of every group, in candidate order; inclusive scan over the groups
-    for (int gi = tid; gi < lay.groups; gi += BM_THREADS) {
-      double sum = 0.0;
-      uint32_t r = gpref[gi];
-      for (int k = 0; k < BM_GROUP_WORDS; k++) {
-        uint32_t bits = bm[gi * BM_GROUP_WORDS + k];
-        while (bits) {
-          const int b = __ffs(bits) - 1;
-          bits &= bits - 1;
-          sum += (double)bm_weight<LADIES>(g, acc, (int32_t)(((gi * BM_GROUP_WORDS + k) << 5) + b), r);
-          r++;
-        }
-      }
-      gcdf[gi] = sum;
-    }
-    __syncthreads();
-    bm_scan_f64(gcdf, lay.groups, red);
-    const double total = gcdf[lay.groups - 1];
-    // ---- the layer's draws
-    for (int j = tid; j < cp.L; j += BM_THREADS) {
-      int32_t pick = cp.V;
-      float pr = 0.f;
-      if (U > 0 && total > 0.0) {
-        Rng rng(cp.seed, (uint32_t)(cp.first_sample + s), (uint32_t)cp.step, (uint32_t)j);
-        const double target = (double)rng.uniform() * total;
-        int lo = 0, hi = lay.groups - 1;  // first group whose prefix reaches the target
-        while (lo < hi) {
-          const int mid = lo + (hi - lo) / 2;
-          if (gcdf[mid] >= target) hi = mid; else lo = mid + 1;
-        }
-        double run = lo > 0 ? gcdf[lo - 1] : 0.0;
-        uint32_t r = gpref[lo];
-        int32_t last_v = cp.V;
-        float pw = 0.f;
-        bool found = false;
-        for (int gi = lo; gi < lay.groups && !found; gi++) {
-          for (int k = 0; k < BM_GROUP_WORDS && !found; k++) {
-            uint32_t bits = bm[gi * BM_GROUP_WORDS + k];
-            while (bits && !found) {
-              const int b = __ffs(bits) - 1;
-              bits &= bits - 1;
-              last_v = (int32_t)(((gi * BM_GROUP_WORDS + k) << 5) + b);
-              pw = bm_weight<LADIES>(g, acc, last_v, r);
-              run += (double)pw;
-              r++;
-              found = run >= target;
-            }
-          }
-        }
-        pick = last_v;  // not found: rounding left the target above the last prefix, the last candidate takes it
-        pr = (float)((double)pw / total);
-        valid++;
-      }
-      sh_layer[j] = pick;
-      out[s * cp.fs + (int64_t)cp.step * cp.L + j] = pick;
-      prob[s * cp.fs + (int64_t)cp.step * cp.L + j] = pr;
-    }
-    __syncthreads();
-    const int64_t a = (s * steps + cp.step) * (int64_t)cp.stride;
-    emit_adjacency(g, cp, sh_tr, sh_layer, adj_row + a, adj_col + a);
-    __syncthreads();
-  }
-  for (int o = 16; o > 0; o >>= 1) valid += __shfl_xor_sync(0xffffffffu, valid, o);
-  if (lane == 0 && valid) atomicAdd(&stats[0], (unsigned long long)valid);
-  if (tid == 0) {
-    if (ids_sum) atomicAdd(&stats[5], ids_sum);
-    if (uniq_sum) atomicAdd(&stats[6], uniq_sum);
-  }
-}
-
-// shared memory the layout may use; ND_COLLECTIVE_BITMAP_GLOBAL=1 puts the big part into global
-// scratch whatever the graph's size (the tests use it to cover that path on small graphs)
-static int bm_smem_budget(const nd_sampler *s) {
-  const char *e = getenv("ND_COLLECTIVE_BITMAP_GLOBAL");
-  return e && e[0] == '1' ? 0 : s->dev.smem_optin;
-}
-
-static BmLayout bm_layout(int32_t V, int ntr_max, int L, int smem_optin) {
-  BmLayout l;
-  l.words = (int)((((int64_t)V + 31) / 32 + BM_GROUP_WORDS - 1) / BM_GROUP_WORDS * BM_GROUP_WORDS);
-  l.groups = l.words / BM_GROUP_WORDS;
-  uint32_t big = 4u * (uint32_t)l.words;       // a multiple of 64
-  l.off_gcdf = big; big += 8u * (uint32_t)l.groups;
-  l.off_gpref = big; big += 4u * (uint32_t)(l.groups + 1);
-  big = (big + 255u) & ~255u;
-  const uint32_t small = 8u * 32u + 4u * 32u + 4u * (uint32_t)ntr_max + 4u * (uint32_t)L + 4u * (uint32_t)ntr_max;
-  const bool in_smem = (int64_t)big + small <= (int64_t)smem_optin;
-  uint32_t off = in_smem ? big : 0u;
-  l.off_red = off; off += 8u * 32u + 4u * 32u;
-  l.off_tr = off; off += 4u * (uint32_t)ntr_max;
-  l.off_layer = off; off += 4u * (uint32_t)L;
-  l.off_rowsum = off; off += 4u * (uint32_t)ntr_max;
-  l.bytes = off;
-  l.glob_bytes = in_smem ? 0u : big;
-  return l;
-}
-
 // clears the counters; stats[1] (live pairs) is known up front for these apps
 __global__ void coll_reset_kernel(unsigned long long *stats, unsigned long long pairs) {
   if (threadIdx.x < 8) stats[threadIdx.x] = threadIdx.x == 1 ? pairs : 0ull;
@@ -640,22 +400,12 @@ int nd_collective_alloc(nd_sampler *s) {
   ND_CUDA(cudaMalloc(&s->d_tmp, sizeof(int64_t) * (S1 + 1)));        // per-sample region offsets
   ND_CUDA(cudaMalloc(&s->d_nlive, sizeof(int32_t) * 4));
   if (p.app == ND_APP_FASTGCN_IS || p.app == ND_APP_LADIES_IS) {
-    // the union is built as a bitmap with a bit per vertex: in shared memory when it fits the CTA's
-    // opt-in shared memory, else in a per-CTA slice of global scratch; ND_COLLECTIVE_SORT=1 selects
+    // the union is built as a bitmap with a bit per vertex (nd_coll_bitmap.cu); ND_COLLECTIVE_SORT=1 selects
     // the sort pipeline instead (kept for the tests, which compare the two)
-    const BmLayout lay = bm_layout(s->g->V, B > L ? B : L, L, bm_smem_budget(s));
     const char *force = getenv("ND_COLLECTIVE_SORT");
-    const bool ladies = p.app == ND_APP_LADIES_IS;
     if (B <= 1024 && L <= 1024 && !(force && force[0] == '1')) {
       s->coll_bitmap = true;
-      s->coll_grid = (int)std::min<int64_t>(S1, (int64_t)s->dev.sms);
-      if (lay.glob_bytes) ND_CUDA(cudaMalloc(&s->d_bm, (size_t)lay.glob_bytes * (size_t)s->coll_grid));
-      if (ladies) {
-        ND_CUDA(cudaFuncSetAttribute(coll_bitmap_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.bytes));
-        ND_CUDA(cudaMalloc(&s->d_acc, sizeof(double) * (size_t)s->coll_grid * (size_t)s->g->V));
-      } else {
-        ND_CUDA(cudaFuncSetAttribute(coll_bitmap_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.bytes));
-      }
+      ND_TRY(nd_coll_bitmap_alloc(s));
     } else {
       ND_TRY(ensure_cand(s, (int64_t)1 << 22));
     }
@@ -679,35 +429,26 @@ int nd_collective_sample(nd_sampler *s, int mode) {
   cp.stride = (cp.B > cp.L ? cp.B : cp.L) * cp.L; cp.step = 0; cp.ntr = cp.B; cp.app = p.app;
   const bool ref_app = p.app == ND_APP_FASTGCN_REF || p.app == ND_APP_LADIES_REF;
   const unsigned long long pairs = (unsigned long long)(S * (cp.B + (int64_t)(p.steps - 1) * cp.L));
-  coll_reset_kernel<<<1, 32, 0, st>>>(s->d_stats, s->coll_bitmap && !ref_app ? pairs : 0ull);
-  nd_count_launches(1);
-  const int grid = (int)std::min<int64_t>(S, (int64_t)s->dev.sms * 8);
-  if (ref_app) {
+  if (s->coll_bitmap && !ref_app) {  // one launch, nothing comes back to the host: asynchronous like the walk and k-hop jobs
     nd_phase_begin(s, ND_PHASE_NEXT);
-    coll_ref_kernel<<<grid, CTHREADS, 0, st>>>(gv, cp, p.steps, S, s->d_initial, s->d_out, s->d_adj_row, s->d_adj_col, s->d_stats);
+    const int rc = nd_coll_bitmap_launch(s, cp, pairs);
+    nd_phase_end(s);
+    return rc;
+  }
+  if (ref_app) {
+    const RefLayout lay = ref_layout(p.steps, cp.B, cp.L);
+    if (lay.bytes > 48u * 1024u) ND_CUDA(cudaFuncSetAttribute(coll_ref_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.bytes));
+    const int per_sm = lay.bytes <= 24u * 1024u ? 8 : 1;
+    nd_phase_begin(s, ND_PHASE_NEXT);
+    coll_ref_kernel<<<(int)std::min<int64_t>(S, (int64_t)s->dev.sms * per_sm), CTHREADS, lay.bytes, st>>>(
+        gv, cp, lay, p.steps, S, s->d_initial, s->d_out, s->d_adj_row, s->d_adj_col, s->d_stats);
     nd_phase_end(s);
     nd_count_launches(1);
     ND_CUDA(cudaGetLastError());
     return ND_OK;
   }
-  if (s->coll_bitmap) {  // one launch per layer, nothing comes back to the host: asynchronous like the walk and k-hop jobs
-    const BmLayout lay = bm_layout(cp.V, cp.B > cp.L ? cp.B : cp.L, cp.L, bm_smem_budget(s));
-    for (int step = 0; step < p.steps; step++) {
-      cp.step = step;
-      cp.ntr = step == 0 ? cp.B : cp.L;
-      nd_phase_begin(s, ND_PHASE_NEXT);
-      if (p.app == ND_APP_LADIES_IS)
-        coll_bitmap_kernel<true><<<s->coll_grid, BM_THREADS, lay.bytes, st>>>(gv, cp, p.steps, S, lay, s->d_bm, s->d_initial, s->d_out, s->d_acc,
-                                                                             s->d_adj_row, s->d_adj_col, s->d_prob, s->d_stats);
-      else
-        coll_bitmap_kernel<false><<<s->coll_grid, BM_THREADS, lay.bytes, st>>>(gv, cp, p.steps, S, lay, s->d_bm, s->d_initial, s->d_out, nullptr,
-                                                                              s->d_adj_row, s->d_adj_col, s->d_prob, s->d_stats);
-      nd_phase_end(s);
-      nd_count_launches(1);
-    }
-    ND_CUDA(cudaGetLastError());
-    return ND_OK;
-  }
+  coll_reset_kernel<<<1, 32, 0, st>>>(s->d_stats, 0ull);
+  nd_count_launches(1);
   std::vector<int32_t> sizes((size_t)S);
   std::vector<int64_t> offs((size_t)S + 1);
   int64_t union_ids = 0;

@@ -72,6 +72,7 @@ struct nd_graph {
   float *w = nullptr;
   float *max_w = nullptr;
   void *block = nullptr;        // the one allocation the four arrays lie in, or null: an allocation each
+  size_t block_bytes = 0;
   // Derived layouts, built on the first sampler that needs them and shared by all samplers of the graph:
   mutable int2 *colw = nullptr;        // [E] (neighbour id, weight bits) records: one 8-byte gather per weighted try
   mutable int2 *vrec = nullptr;        // [V+1] (row start, max weight bits) per vertex: what a thread-per-walk kernel needs of a vertex in one sector
@@ -81,6 +82,10 @@ struct nd_graph {
   mutable uint8_t *wq = nullptr;       // [E] weights as whole 256ths of the row's maximum
   mutable int32_t *adjset = nullptr;   // node2vec membership: per-vertex hash sets of the neighbour ids, 8-slot buckets
   mutable uint32_t *adjsign = nullptr; // ... and the filter in front of them
+  mutable float *deg2 = nullptr;       // [V] deg * deg (FastGCN)
+  mutable float *term = nullptr;       // [E] (w / rowsum)^2 (LADIES)
+  mutable int32_t *hub_slot = nullptr; // [V] slot of the vertex's neighbourhood as a bitmap, -1: none
+  mutable uint32_t *hub_bits = nullptr;
 };
 
 struct NdGraphView {
@@ -220,7 +225,6 @@ struct nd_sampler {
   int64_t cand_cap = 0;
   bool coll_bitmap = false;       // importance sampling through the shared-memory bitmap kernel
   int coll_grid = 0;
-  double *d_acc = nullptr;        // LADIES: per-CTA accumulators of the candidates' weights
   unsigned char *d_bm = nullptr;  // per-CTA bitmap slices when a bit per vertex does not fit shared memory
 
   NdHostRows *hostrows = nullptr;

@@ -16,6 +16,7 @@
 #include <mutex>
 
 #include "nd_common.cuh"
+#include "nd_entries.cuh"
 #include "nd_nbrset.cuh"
 #include "nd_philox.cuh"
 #include "nd_walk_rows.cuh"
@@ -606,31 +607,6 @@ template <int APP, int LAYOUT>
 __global__ void __launch_bounds__(ROWS_THREADS, ROWS_CTAS) walk_next_count_kernel(const RowsArgs a) { walks<APP, LAYOUT>(a); }
 
 // ---------------------------------------------------------------- layouts, built by a graph's first sampler that reads them
-
-// source row of the CSR entry e, which lies in the rows [lo, hi)
-__device__ __forceinline__ int32_t row_of_entry(const int32_t *__restrict__ row_ptr, int32_t lo, int32_t hi, int64_t e) {
-  while (hi - lo > 1) {
-    const int32_t mid = lo + ((hi - lo) >> 1);
-    if ((int64_t)row_ptr[mid] <= e) lo = mid; else hi = mid;
-  }
-  return lo;
-}
-
-// f(entry, its row) for every entry.  A CTA takes BUILD_SPAN consecutive entries at a time: the rows of the
-// first and the last of them bound the search of all others.
-constexpr int BUILD_THREADS = 256, BUILD_SPAN = 2048;
-template <class F>
-__device__ __forceinline__ void for_entries(const int32_t *__restrict__ row_ptr, int32_t V, int64_t E, F f) {
-  __shared__ int32_t sh[2];
-  for (int64_t e0 = (int64_t)blockIdx.x * BUILD_SPAN; e0 < E; e0 += (int64_t)gridDim.x * BUILD_SPAN) {
-    const int64_t e1 = e0 + BUILD_SPAN < E ? e0 + BUILD_SPAN : E;
-    __syncthreads();
-    if (threadIdx.x < 2) sh[threadIdx.x] = row_of_entry(row_ptr, 0, V, threadIdx.x ? e1 - 1 : e0);
-    __syncthreads();
-    const int32_t lo = sh[0], hi = sh[1] + 1;
-    for (int64_t e = e0 + threadIdx.x; e < e1; e += BUILD_THREADS) f(e, row_of_entry(row_ptr, lo, hi, e));
-  }
-}
 
 __global__ void vrow_build_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int2 *__restrict__ vrow) {
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x)
