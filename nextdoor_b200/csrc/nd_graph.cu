@@ -257,7 +257,8 @@ struct BuildScratch {
   RecordFacts *facts;
   int32_t *d_n, *d_max_degree;
   int device = 0;
-  ~BuildScratch() { nd_pool_free(device, base); }
+  size_t bytes = 0;
+  ~BuildScratch() { nd_block_free(device, base, bytes); }
 };
 
 int build_scratch(BuildScratch *s, int device, int64_t n) {
@@ -265,7 +266,8 @@ int build_scratch(BuildScratch *s, int device, int64_t n) {
   const size_t words = ((size_t)(n > 0 ? n : 1) + 8 + 63) & ~(size_t)63;
   const NdRadixPlan pl = nd_radix_plan(32, n);
   const size_t radix = nd_radix_scratch_bytes(n);
-  ND_TRY(nd_pool_alloc(device, (void **)&s->base, 24 * words + radix + 256));
+  s->bytes = 24 * words + radix + 256;
+  ND_TRY(nd_block_alloc(device, (void **)&s->base, &s->bytes));
   for (int w = 0; w < 3; w++) { s->a[w] = (uint32_t *)s->base + w * words; s->b[w] = (uint32_t *)s->base + (3 + w) * words; }
   s->rec = (Rec12 *)s->b[0];
   unsigned char *p = s->base + 24 * words;
@@ -301,11 +303,12 @@ int build_from_soa(const NdDeviceInfo &dev, int64_t n, int32_t V, BuildScratch *
   }
   // one block: row offsets, ids and weights (32 bytes of padding for the 16-byte staging windows), maximum weights
   auto round = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  const size_t o_col = round(4 * ((size_t)V + 1)), o_w = o_col + round(4 * ((size_t)n + 8)), o_max = o_w + round(4 * ((size_t)n + 8)), all = o_max + round(4 * (size_t)V);
+  const size_t o_col = round(4 * ((size_t)V + 1)), o_w = o_col + round(4 * ((size_t)n + 8)), o_max = o_w + round(4 * ((size_t)n + 8));
+  size_t all = o_max + round(4 * (size_t)V);
   unsigned char *block = nullptr;
-  ND_TRY(nd_pool_alloc(dev.device, (void **)&block, all));
+  ND_TRY(nd_block_alloc(dev.device, (void **)&block, &all));
   nd_graph *g = new nd_graph();
-  g->device = dev.device; g->V = V; g->E = n; g->block = block;
+  g->device = dev.device; g->V = V; g->E = n; g->block = block; g->block_bytes = all;
   g->row_ptr = (int32_t *)block; g->col = (int32_t *)(block + o_col); g->w = (float *)(block + o_w); g->max_w = (float *)(block + o_max);
   auto build = [&]() -> int {
     ND_CUDA(cudaMemsetAsync(g->col + n, 0, sizeof(int32_t) * 8));
@@ -320,7 +323,7 @@ int build_from_soa(const NdDeviceInfo &dev, int64_t n, int32_t V, BuildScratch *
     return ND_OK;
   };
   const int rc = build();
-  if (rc != ND_OK) { nd_pool_free(dev.device, block); delete g; return rc; }
+  if (rc != ND_OK) { nd_block_free(dev.device, block, all); delete g; return rc; }
   nd_objects_add(1);
   *out = g;
   return ND_OK;
@@ -572,7 +575,7 @@ int nd_graph_device_ptrs(const nd_graph *g, const int32_t **row_ptr, const int32
 int nd_graph_destroy(nd_graph *g) {
   if (!g) return ND_OK;
   cudaSetDevice(g->device);
-  if (g->block) nd_pool_free(g->device, g->block);
+  if (g->block) nd_block_free(g->device, g->block, g->block_bytes);
   else { cudaFree(g->row_ptr); cudaFree(g->col); cudaFree(g->w); cudaFree(g->max_w); }
   cudaFree(g->colw); cudaFree(g->vrec); cudaFree(g->vrow); cudaFree(g->vrec4); cudaFree(g->erec); cudaFree(g->wq); cudaFree(g->adjset); cudaFree(g->adjsign);
   cudaFree(g->deg2); cudaFree(g->term); cudaFree(g->hub_slot); cudaFree(g->hub_bits);

@@ -271,59 +271,73 @@ int copy(int device, void *dst, const void *src, size_t bytes, bool up) {
 int nd_copy_to_host(int device, void *dst, const void *src, size_t bytes) { return copy(device, dst, src, bytes, false); }
 int nd_copy_to_device(int device, void *dst, const void *src, size_t bytes) { return copy(device, dst, src, bytes, true); }
 
-// ---------------------------------------------------------------- device memory pool
+// ---------------------------------------------------------------- device memory that is kept
 
 namespace {
-constexpr uint64_t POOL_KEEP = (uint64_t)1 << 30;
-std::mutex g_pools_mutex;
-std::vector<cudaMemPool_t> g_pools;   // by device, made at the first allocation
+constexpr size_t KEEP_BLOCK = (size_t)384 << 20, KEEP_ALL = (size_t)1 << 30;
+struct Block {
+  int device;
+  void *p;
+  size_t bytes;
+};
+std::mutex g_blocks_mutex;
+std::vector<Block> g_kept;   // free blocks, oldest first
+size_t g_kept_bytes = 0;
 
-int pool_of(int device, cudaMemPool_t *pool) {
-  std::lock_guard<std::mutex> lock(g_pools_mutex);
-  if ((size_t)device >= g_pools.size()) g_pools.resize((size_t)device + 1, nullptr);
-  if (!g_pools[(size_t)device]) {
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = device;
-    cudaMemPool_t p = nullptr;
-    ND_CUDA(cudaMemPoolCreate(&p, &props));
-    uint64_t keep = POOL_KEEP;
-    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-    g_pools[(size_t)device] = p;
-  }
-  *pool = g_pools[(size_t)device];
-  return ND_OK;
+void drop_oldest() {   // under the lock
+  cudaSetDevice(g_kept.front().device);
+  cudaFree(g_kept.front().p);
+  g_kept_bytes -= g_kept.front().bytes;
+  g_kept.erase(g_kept.begin());
 }
 }  // namespace
 
-int nd_pool_alloc(int device, void **p, size_t bytes) {
-  cudaMemPool_t pool = nullptr;
-  ND_TRY(pool_of(device, &pool));
-  ND_CUDA(cudaMallocFromPoolAsync(p, bytes, pool, nullptr));
+int nd_block_alloc(int device, void **p, size_t *bytes) {
+  {
+    std::lock_guard<std::mutex> lock(g_blocks_mutex);
+    size_t best = g_kept.size();
+    for (size_t k = 0; k < g_kept.size(); k++)
+      if (g_kept[k].device == device && g_kept[k].bytes >= *bytes && g_kept[k].bytes / 2 <= *bytes && (best == g_kept.size() || g_kept[k].bytes < g_kept[best].bytes))
+        best = k;
+    if (best < g_kept.size()) {
+      *p = g_kept[best].p;
+      *bytes = g_kept[best].bytes;
+      g_kept_bytes -= g_kept[best].bytes;
+      g_kept.erase(g_kept.begin() + (long)best);
+      return ND_OK;
+    }
+  }
+  if (cudaMalloc(p, *bytes) == cudaSuccess) return ND_OK;
+  cudaGetLastError();
+  {   // what is kept may be what is missing
+    std::lock_guard<std::mutex> lock(g_blocks_mutex);
+    while (!g_kept.empty()) drop_oldest();
+    cudaSetDevice(device);
+  }
+  ND_CUDA(cudaMalloc(p, *bytes));
   return ND_OK;
 }
 
-void nd_pool_free(int device, void *p) {
+void nd_block_free(int device, void *p, size_t bytes) {
   if (!p) return;
   cudaSetDevice(device);
-  cudaDeviceSynchronize();   // as cudaFree: no stream uses it any more
-  cudaFreeAsync(p, nullptr);
+  if (bytes > KEEP_BLOCK) { cudaFree(p); return; }
+  cudaDeviceSynchronize();   // as cudaFree does: no stream uses it any more
+  std::lock_guard<std::mutex> lock(g_blocks_mutex);
+  g_kept.push_back(Block{device, p, bytes});
+  g_kept_bytes += bytes;
+  while (g_kept_bytes > KEEP_ALL) drop_oldest();
+  cudaSetDevice(device);
 }
 
 void nd_objects_add(int n) {
   std::lock_guard<std::mutex> lock(g_objects_mutex);
   g_objects += n;
   if (g_objects > 0) return;
-  std::lock_guard<std::mutex> pools(g_pools_mutex);
+  std::lock_guard<std::mutex> blocks(g_blocks_mutex);
   int now = 0;
   cudaGetDevice(&now);
-  for (size_t d = 0; d < g_pools.size(); d++)
-    if (g_pools[d]) {
-      cudaSetDevice((int)d);
-      cudaStreamSynchronize(nullptr);
-      cudaMemPoolTrimTo(g_pools[d], 0);
-    }
+  while (!g_kept.empty()) drop_oldest();
   cudaSetDevice(now);
 }
 

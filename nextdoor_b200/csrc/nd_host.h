@@ -26,12 +26,13 @@ void nd_host_ranges(int64_t count, int threads, F fn) {
 int nd_copy_to_host(int device, void *dst, const void *src, size_t bytes);
 int nd_copy_to_device(int device, void *dst, const void *src, size_t bytes);
 
-// Device memory that is kept for the next allocation when it is freed, up to POOL_KEEP bytes per device while graphs
-// or samplers are alive (a cudaMalloc / cudaFree pair of a large block costs 0.5 to 30 ms, by the box).  Allocation
-// and release are ordered like work on the default stream; the release waits for the device.
-int nd_pool_alloc(int device, void **p, size_t bytes);
-void nd_pool_free(int device, void *p);
+// Device memory for building graphs.  Blocks of up to 384 MB are kept for the next build when they are freed, 1 GB of
+// them in all, while graphs or samplers are alive (a cudaMalloc / cudaFree pair costs 0.5 to 30 ms, by the box); a
+// failing allocation gives all of them back first.  `bytes`: in: at least, out: what the block has.  The release
+// waits for the device, as cudaFree does.
+int nd_block_alloc(int device, void **p, size_t *bytes);
+void nd_block_free(int device, void *p, size_t bytes);
 
-// Graphs and samplers alive: without any, the pool keeps nothing, and the staging memory of the
+// Graphs and samplers alive: without any, no block is kept, and the staging memory of the
 // copies is returned when the workers end.
 void nd_objects_add(int n);
