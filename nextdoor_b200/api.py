@@ -360,15 +360,14 @@ class PipelinedSampler:
         self._finish(k)                                   # this set's previous job still owns its staging buffers
         others = [j for j in self._pending if j != k]
         for j in others:                                  # the lengths of the job before have landed: its vertices
-            for _, _, smp in self.sets[j]:                # cross while this job is sampled
-                smp.host_update_fetch()
+            self._fetch(j)                                # cross while this job is sampled
         row_len = self._rows_of(out_host)
         for f, n, smp in self.parts:
             if initial_host is not None:
                 smp.set_initial(initial_host[f * self.isz:(f + n) * self.isz])
             smp.sample(mode, sync=False)
             smp.host_update_begin(out_host[f * self.fs:(f + n) * self.fs], row_len[f:f + n], self.copy_stream)
-        self._pending[k] = True
+        self._pending[k] = "begun"
         for j in others:                                  # ... and its rows are written while the device works on this one
             self._finish(j)
 
@@ -383,8 +382,16 @@ class PipelinedSampler:
         """The caller is going to write to `out_host` itself: the next job into it starts from a fresh fill."""
         self._row_len.pop((out_host.__array_interface__["data"][0], out_host.size), None)
 
+    def _fetch(self, k):
+        if self._pending.get(k) == "begun":
+            for _, _, smp in self.sets[k]:
+                smp.host_update_fetch()
+            self._pending[k] = "fetched"
+
     def _finish(self, k):
-        if self._pending.pop(k, None):
+        if k in self._pending:
+            self._fetch(k)                                # every chunk's vertices are on their way before the first rows are written
+            self._pending.pop(k)
             self.values_copied = sum(smp.host_update_finish() for _, _, smp in self.sets[k])
 
     def wait(self):

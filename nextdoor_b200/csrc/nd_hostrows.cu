@@ -28,6 +28,7 @@ struct NdHostRows {
   cudaStream_t cs = nullptr;
   int32_t *out = nullptr, *row_len = nullptr;
   int64_t total = 0;
+  std::vector<int64_t> part;    // sums of the lengths of the threads' row ranges
   bool dense = false;           // most slots are in use: the dense array is copied as it is
   int stage = 0;                // 0 idle, 1 begun, 2 fetched
   int threads = 1;
@@ -255,12 +256,13 @@ int nd_sampler_host_update_fetch(nd_sampler *s) {
   if (s->S == 0) { h->stage = 2; return ND_OK; }
   ND_CUDA(cudaSetDevice(s->g->device));
   ND_CUDA(cudaEventSynchronize(h->len_done));
-  std::vector<int64_t> part((size_t)h->threads, 0);
+  h->part.assign((size_t)h->threads + 1, 0);
+  std::vector<int64_t> &part = h->part;
   const int32_t *len = h->h_len;
   nd_host_ranges(s->S, h->threads, [&](int t, int64_t a, int64_t b) {
     int64_t sum = 0;
     for (int64_t i = a; i < b; i++) sum += len[i];
-    part[(size_t)t] = sum;
+    part[(size_t)t + 1] = sum;
   });
   for (int64_t v : part) h->total += v;
   h->dense = 2 * h->total > s->S * (int64_t)s->fs || !packable(s);
@@ -304,17 +306,14 @@ int nd_sampler_host_update_finish(nd_sampler *s, int64_t *values_copied) {
     });
     return ND_OK;
   }
-  // every thread needs the position of its first row in the packed array: the ranges' sums again
-  std::vector<int64_t> part((size_t)h->threads + 1, 0);
-  nd_host_ranges(s->S, h->threads, [&](int t, int64_t a, int64_t b) {
-    int64_t sum = 0;
-    for (int64_t i = a; i < b; i++) sum += len[i];
-    part[(size_t)t + 1] = sum;
-  });
+  // every thread needs the position of its first row in the packed array: the ranges' sums
+  std::vector<int64_t> &part = h->part;
   for (size_t t = 1; t < part.size(); t++) part[t] += part[t - 1];
   nd_host_ranges(s->S, h->threads, [&, out, row_len, len, vals](int t, int64_t a, int64_t b) {
     const int32_t *src = vals + part[(size_t)t];
+    constexpr int AHEAD = 24;   // rows lie apart and are not in any cache: ask for them before they are written
     for (int64_t i = a; i < b; i++) {
+      if (i + AHEAD < b && (len[i + AHEAD] | row_len[i + AHEAD])) __builtin_prefetch(out + (i + AHEAD) * steps, 1);
       const int32_t now = len[i], had = row_len[i];
       int32_t *row = out + i * steps;
       for (int k = 0; k < now; k++) row[k] = src[k];
