@@ -339,10 +339,10 @@ int nd_sampler_aux(nd_sampler *s, int32_t *adj_row, int32_t *adj_col, float *pro
   if (nd_is_collective(s->p.app)) {
     const int L = s->p.fanout[0], B = s->p.batch;
     const size_t n = (size_t)s->S * s->p.steps * (B > L ? B : L) * L;
-    const int dev = s->g->device;
-    if (adj_row) ND_TRY(nd_copy_to_host(dev, adj_row, s->d_adj_row, 4 * n));
-    if (adj_col) ND_TRY(nd_copy_to_host(dev, adj_col, s->d_adj_col, 4 * n));
-    if (prob && s->d_prob) ND_TRY(nd_copy_to_host(dev, prob, s->d_prob, 4 * (size_t)s->S * s->fs));
+    void *const dst[3] = {adj_row, adj_col, prob};
+    const void *const src[3] = {s->d_adj_row, s->d_adj_col, s->d_prob};
+    const size_t bytes[3] = {adj_row ? 4 * n : 0, adj_col ? 4 * n : 0, prob && s->d_prob ? 4 * (size_t)s->S * s->fs : 0};
+    ND_TRY(nd_copies_to_host(s->g->device, 3, dst, src, bytes));
   }
   if (hop_counts && s->d_hop_counts)
     ND_TRY(nd_copy_to_host(s->g->device, hop_counts, s->d_hop_counts, 4 * (size_t)s->S * s->p.steps));

@@ -4,9 +4,8 @@
 // Replaces Graph::load_from_edge_list_binary + csr_from_graph (src/graph.hpp:106-159,
 // src/csr.hpp:399-424: per-vertex std::vector, OpenMP std::sort, serial fill), transferCSRToGPUs
 // (src/nextdoor.cu:1893-1911) and create_csr_partitions (src/graph_partitioner.cuh:1-173).
-// The records are sorted by (src, dst, weight) with three stable LSD sorts of the in-house radix
-// sort (weight bits, then dst, then src), row offsets come from the boundaries of the sorted src
-// array, and the sorted dst / weight arrays become col / w in place.
+// The records are sorted by (src, dst, weight) with stable LSD sorts of the in-house radix sort (dst,
+// then src; weights inside runs of equal edges), row offsets come from the boundaries of the sorted src array.
 #include <fcntl.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -133,6 +132,72 @@ __global__ void rmat_kernel(int32_t V, int scale, int64_t M, uint64_t seed, uint
   }
 }
 
+// Records sorted by (src, dst) in their order of arrival: the weights of records with the same pair are brought into
+// order where they lie, by the thread that finds the first of them.  Almost all runs are of two or three; those longer
+// than RUN_THREAD (an R-MAT graph's hub pairs) go on a list for a CTA each, and runs longer than RUN_CTA set *too_long.
+constexpr int RUN_THREAD = 32, RUN_CTA = 4096;
+struct RunList {
+  int32_t too_long, count;
+};
+__global__ void sort_runs_kernel(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst, uint32_t *__restrict__ wk, int64_t n,
+                                 RunList *__restrict__ runs, uint32_t *__restrict__ list) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i + 1 < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t s = src[i], d = dst[i];
+    if (src[i + 1] != s || dst[i + 1] != d || (i > 0 && src[i - 1] == s && dst[i - 1] == d)) continue;
+    int m = 2;
+    while (m <= RUN_THREAD && i + m < n && src[i + m] == s && dst[i + m] == d) m++;
+    if (m > RUN_THREAD) { list[atomicAdd(&runs->count, 1)] = (uint32_t)i; continue; }
+    for (int k = 1; k < m; k++) {
+      const uint32_t x = wk[i + k];
+      int j = k;
+      for (; j > 0 && wk[i + j - 1] > x; j--) wk[i + j] = wk[i + j - 1];
+      wk[i + j] = x;
+    }
+  }
+}
+
+// a CTA per listed run: bitonic sort in shared memory (16 KB)
+__global__ void __launch_bounds__(256) sort_long_runs_kernel(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst, uint32_t *__restrict__ wk,
+                                                             int64_t n, RunList *__restrict__ runs, const uint32_t *__restrict__ list) {
+  __shared__ uint32_t key[RUN_CTA];
+  __shared__ int end;
+  const int count = runs->count;
+  for (int r = blockIdx.x; r < count; r += gridDim.x) {
+    const int64_t at = list[r];
+    const uint32_t s = src[at], d = dst[at];
+    __syncthreads();
+    if (threadIdx.x == 0) {   // past the last record of the run, which lie together: bisection over the window
+      int64_t lo = at, hi = n - at > RUN_CTA ? at + RUN_CTA + 1 : n;
+      while (hi - lo > 1) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (src[mid] == s && dst[mid] == d) lo = mid;
+        else hi = mid;
+      }
+      end = (int)(hi - at);
+    }
+    __syncthreads();
+    const int m = end;
+    if (m > RUN_CTA) {
+      if (threadIdx.x == 0) runs->too_long = 1;
+      continue;
+    }
+    int size = 64;
+    while (size < m) size *= 2;
+    for (int k = threadIdx.x; k < size; k += blockDim.x) key[k] = k < m ? wk[at + k] : 0xffffffffu;
+    for (int width = 2; width <= size; width *= 2)
+      for (int step = width / 2; step > 0; step /= 2) {
+        __syncthreads();
+        for (int k = threadIdx.x; k < size / 2; k += blockDim.x) {
+          const int x = (k / step) * 2 * step + k % step, y = x + step;
+          const uint32_t kx = key[x], ky = key[y];
+          if ((kx > ky) == ((x & width) == 0)) { key[x] = ky; key[y] = kx; }
+        }
+      }
+    __syncthreads();
+    for (int k = threadIdx.x; k < m; k += blockDim.x) wk[at + k] = key[k];
+  }
+}
+
 // The sorted records become the CSR: row_ptr (element i closes the rows (src[i-1], src[i]]), col, w.
 __global__ void csr_from_sorted_kernel(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst, const uint32_t *__restrict__ wk,
                                        int64_t n, int32_t V, int32_t *__restrict__ row_ptr, int32_t *__restrict__ col, float *__restrict__ w) {
@@ -256,6 +321,7 @@ struct BuildScratch {
   NdRadixScratch radix;
   RecordFacts *facts;
   int32_t *d_n, *d_max_degree;
+  RunList *runs;
   int device = 0;
   size_t bytes = 0;
   ~BuildScratch() { nd_block_free(device, base, bytes); }
@@ -274,6 +340,7 @@ int build_scratch(BuildScratch *s, int device, int64_t n) {
   s->facts = (RecordFacts *)p;
   s->d_n = (int32_t *)(p + 64);
   s->d_max_degree = (int32_t *)(p + 128);
+  s->runs = (RunList *)(p + 192);
   nd_radix_scratch_place(&s->radix, pl, p + 256);
   const RecordFacts none{-1, 0, 0xffffffffu, 0u};
   const int32_t n32 = (int32_t)n;
@@ -283,23 +350,38 @@ int build_scratch(BuildScratch *s, int device, int64_t n) {
   return ND_OK;
 }
 
-// records in bs->a (weights as keys) -> graph; key bits outside [lo_bit, hi_bit) are the same in all records
+// records in bs->a (weights as keys) -> graph; key bits outside [lo_bit, hi_bit) are the same in all records.  They are
+// sorted by dst, then src, and the few that share both by weight where they lie (10 passes over random edges with
+// random weights -> 6; 8.4M records on the host to a graph, copies included: 6.1 ms -> 4.9).  A graph that repeats one edge thousands of times goes on to the full sort.
 int build_from_soa(const NdDeviceInfo &dev, int64_t n, int32_t V, BuildScratch *bs, int lo_bit, int hi_bit, nd_graph **out) {
   ND_REQUIRE(n < ((int64_t)1 << 31), ND_ERR_RANGE, "%lld edges do not fit the int32 edge index of the CSR", (long long)n);
   const int vbits = nd_bit_length((uint32_t)(V > 1 ? V - 1 : 1));
-  const int key_word[3] = {2, 1, 0};
-  const int key_bits[3] = {hi_bit - lo_bit, vbits, vbits};
   uint32_t *cur[3] = {bs->a[0], bs->a[1], bs->a[2]}, *oth[3] = {bs->b[0], bs->b[1], bs->b[2]};
-  for (int k = 0; k < 3; k++) {
-    if (n < 2 || key_bits[k] <= 0) continue;
+  auto sort_by = [&](int word, int bits, int lo) -> int {
+    if (n < 2 || bits <= 0) return ND_OK;
     NdSortArrays arr;
     arr.nwords = 3;
     for (int w = 0; w < 3; w++) { arr.a[w] = cur[w]; arr.b[w] = oth[w]; }
     bool in_b = false;
-    NdRadixPlan pl = nd_radix_plan(key_bits[k], n);
-    if (k == 0) for (int p = 0; p < pl.passes; p++) pl.shift[p] += lo_bit;
-    ND_TRY(nd_radix_sort(dev, nullptr, &bs->radix, pl, arr, key_word[k], bs->d_n, nullptr, false, 0u, false, &in_b));
+    NdRadixPlan pl = nd_radix_plan(bits, n);
+    for (int p = 0; p < pl.passes; p++) pl.shift[p] += lo;
+    ND_TRY(nd_radix_sort(dev, nullptr, &bs->radix, pl, arr, word, bs->d_n, nullptr, false, 0u, false, &in_b));
     if (in_b) for (int w = 0; w < 3; w++) { uint32_t *t = cur[w]; cur[w] = oth[w]; oth[w] = t; }
+    return ND_OK;
+  };
+  ND_TRY(sort_by(1, vbits, 0));
+  ND_TRY(sort_by(0, vbits, 0));
+  if (hi_bit > lo_bit && n > 1) {
+    RunList runs;
+    sort_runs_kernel<<<grid_for(n, 256, dev.sms), 256>>>(cur[0], cur[1], cur[2], n, bs->runs, oth[0]);
+    sort_long_runs_kernel<<<dev.sms * 4, 256>>>(cur[0], cur[1], cur[2], n, bs->runs, oth[0]);
+    nd_count_launches(2);
+    ND_CUDA(cudaMemcpy(&runs, bs->runs, sizeof(runs), cudaMemcpyDeviceToHost));
+    if (runs.too_long) {
+      ND_TRY(sort_by(2, hi_bit - lo_bit, lo_bit));
+      ND_TRY(sort_by(1, vbits, 0));
+      ND_TRY(sort_by(0, vbits, 0));
+    }
   }
   // one block: row offsets, ids and weights (32 bytes of padding for the 16-byte staging windows), maximum weights
   auto round = [](size_t b) { return (b + 255) & ~(size_t)255; };
@@ -368,8 +450,10 @@ int nd_graph_from_csr(int device, int32_t V, int64_t E, const int32_t *row_ptr, 
   ND_CUDA(cudaMemset(g->w + E, 0, sizeof(float) * 8));
   ND_CUDA(cudaMemcpy(g->row_ptr, row_ptr, sizeof(int32_t) * ((size_t)V + 1), cudaMemcpyHostToDevice));
   if (E > 0) {
-    ND_TRY(nd_copy_to_device(device, g->col, col, sizeof(int32_t) * (size_t)E));
-    ND_TRY(nd_copy_to_device(device, g->w, w, sizeof(float) * (size_t)E));
+    void *const to[2] = {g->col, g->w};
+    const void *const from[2] = {col, w};
+    const size_t bytes[2] = {sizeof(int32_t) * (size_t)E, sizeof(float) * (size_t)E};
+    ND_TRY(nd_copies_to_device(device, 2, to, from, bytes));
   }
   if (max_w) {
     ND_CUDA(cudaMalloc(&g->max_w, sizeof(float) * (size_t)V));
@@ -424,8 +508,10 @@ int nd_graph_from_edges(int device, int64_t n, const int32_t *src, const int32_t
   ND_TRY(nd_device_info(device, &dev));
   BuildScratch bs;
   ND_TRY(build_scratch(&bs, device, n));
-  const void *from[3] = {src, dst, w};
-  for (int k = 0; k < 3; k++) ND_TRY(nd_copy_to_device(device, bs.a[k], from[k], 4 * (size_t)n));
+  void *const to[3] = {bs.a[0], bs.a[1], bs.a[2]};
+  const void *const from[3] = {src, dst, w};
+  const size_t bytes[3] = {4 * (size_t)n, 4 * (size_t)n, 4 * (size_t)n};
+  ND_TRY(nd_copies_to_device(device, 3, to, from, bytes));
   unpack_arrays_kernel<<<grid_for(n, 256, dev.sms), 256>>>(n, bs.a[0], bs.a[1], bs.a[2], bs.facts);
   nd_count_launches(1);
   return build_from_facts(dev, n, 0, &bs, out);
@@ -555,10 +641,11 @@ int nd_graph_info(const nd_graph *g, int32_t *V, int64_t *E, int32_t *max_degree
 int nd_graph_to_host(const nd_graph *g, int32_t *row_ptr, int32_t *col, float *w, float *max_w) {
   ND_REQUIRE(g, ND_ERR_ARG, "null graph");
   ND_CUDA(cudaSetDevice(g->device));
-  if (row_ptr) ND_TRY(nd_copy_to_host(g->device, row_ptr, g->row_ptr, sizeof(int32_t) * ((size_t)g->V + 1)));
-  if (col && g->E) ND_TRY(nd_copy_to_host(g->device, col, g->col, sizeof(int32_t) * (size_t)g->E));
-  if (w && g->E) ND_TRY(nd_copy_to_host(g->device, w, g->w, sizeof(float) * (size_t)g->E));
-  if (max_w) ND_TRY(nd_copy_to_host(g->device, max_w, g->max_w, sizeof(float) * (size_t)g->V));
+  void *const dst[4] = {row_ptr, col, w, max_w};
+  const void *const src[4] = {g->row_ptr, g->col, g->w, g->max_w};
+  const size_t bytes[4] = {row_ptr ? sizeof(int32_t) * ((size_t)g->V + 1) : 0, col ? sizeof(int32_t) * (size_t)g->E : 0,
+                           w ? sizeof(float) * (size_t)g->E : 0, max_w ? sizeof(float) * (size_t)g->V : 0};
+  ND_TRY(nd_copies_to_host(g->device, 4, dst, src, bytes));
   return ND_OK;
 }
 

@@ -133,6 +133,7 @@ namespace {
 
 constexpr size_t PIECE = (size_t)1 << 20;   // 1 MB: twenty microseconds on the wire
 constexpr int RING = 8;                    // pinned pieces
+constexpr size_t FRESH = (size_t)48 << 20;       // see staged()
 constexpr size_t STAGED_MIN = (size_t)2 << 20;   // below this the plain call is as fast
 
 struct Ring {
@@ -178,23 +179,37 @@ bool pageable(const void *p) {
   return at.type == cudaMemoryTypeUnregistered;
 }
 
+struct Segment {
+  unsigned char *host, *dev;
+  size_t bytes;
+};
+
 // Piece k of the copy uses slot k % RING.  The caller alone talks to the driver (threads that wait for
 // events get in each other's way): it enqueues the pieces in order and publishes how many
 // transfers are over.  The workers move pieces between the slots and the user's memory; the caller does so when
 // none of them has got on for a while, so the copy ends without them too.
-int staged(unsigned char *host, unsigned char *dev, size_t bytes, bool up) {
-  const size_t pieces = (bytes + PIECE - 1) / PIECE;
+int staged(const std::vector<Segment> &segments, size_t bytes, bool up) {
+  struct Piece { unsigned char *host, *dev; size_t size; };
+  std::vector<Piece> piece;
+  size_t most = PIECE / 8;   // small ones first, so that the wire and the workers are busy early
+  for (const Segment &g : segments)
+    for (size_t at = 0; at < g.bytes;) {
+      const size_t n = std::min(most, g.bytes - at);
+      piece.push_back(Piece{g.host + at, g.dev + at, n});
+      at += n;
+      if (most < PIECE && piece.size() % 4 == 0) most *= 2;
+    }
+  const size_t pieces = piece.size();
   std::vector<std::atomic<char>> moved(pieces);   // the host side of the piece is done
   std::atomic<size_t> over{0};                    // transfers that are complete
   std::atomic<size_t> next{0};                    // next piece to move
   std::atomic<bool> stop{false};
-  auto size = [&](size_t k) { return k + 1 < pieces ? PIECE : bytes - k * PIECE; };
   // up: the slot's last transfer is over; down: the piece's own is
   auto movable = [&](size_t k) { return up ? k < over.load(std::memory_order_acquire) + RING : k < over.load(std::memory_order_acquire); };
   auto move = [&](size_t k) {
     unsigned char *slot = g_ring.pinned + (k % RING) * PIECE;
-    if (up) memcpy(slot, host + k * PIECE, size(k));
-    else memcpy(host + k * PIECE, slot, size(k));
+    if (up) memcpy(slot, piece[k].host, piece[k].size);
+    else memcpy(piece[k].host, slot, piece[k].size);
     moved[k].store(1, std::memory_order_release);
   };
   std::atomic<int> helpers{0};                    // workers at it
@@ -217,8 +232,8 @@ int staged(unsigned char *host, unsigned char *dev, size_t bytes, bool up) {
     while (done < pieces) {
       if (sent < pieces && sent < done + RING && (up ? moved[sent].load(std::memory_order_acquire) != 0 : sent < RING || moved[sent - RING].load(std::memory_order_acquire) != 0)) {
         unsigned char *slot = g_ring.pinned + (sent % RING) * PIECE;
-        err = up ? cudaMemcpyAsync(dev + sent * PIECE, slot, size(sent), cudaMemcpyHostToDevice, g_ring.stream)
-                 : cudaMemcpyAsync(slot, dev + sent * PIECE, size(sent), cudaMemcpyDeviceToHost, g_ring.stream);
+        err = up ? cudaMemcpyAsync(piece[sent].dev, slot, piece[sent].size, cudaMemcpyHostToDevice, g_ring.stream)
+                 : cudaMemcpyAsync(slot, piece[sent].dev, piece[sent].size, cudaMemcpyDeviceToHost, g_ring.stream);
         if (err == cudaSuccess) err = cudaEventRecord(g_ring.done[sent % RING], g_ring.stream);
         if (err != cudaSuccess) return;
         sent++;
@@ -240,8 +255,10 @@ int staged(unsigned char *host, unsigned char *dev, size_t bytes, bool up) {
       if (k < pieces && movable(k) && next.compare_exchange_strong(k, k + 1)) move(k);
     }
   };
-  // five keep up with the wire (more help where the destination is fresh memory, 15 -> 20 GB/s, but take longer to wake)
-  const int movers = (int)std::min<size_t>(std::min<size_t>(pieces, 5), (size_t)std::max(1, nd_host_threads() - 1));
+  // Five keep up with the wire; a large destination is likely to be fresh memory, where more of them share the page
+  // faults (15 -> 25 GB/s), but take longer to wake.
+  const size_t want = !up && bytes >= FRESH ? 12 : 5;
+  const int movers = (int)std::min<size_t>(std::min<size_t>(pieces, want), (size_t)std::max(1, nd_host_threads() - 1));
   nd_host_run(movers, [&](int) { mover(); }, [&] {
     driver();
     stop.store(err != cudaSuccess);
@@ -253,23 +270,33 @@ int staged(unsigned char *host, unsigned char *dev, size_t bytes, bool up) {
   return ND_OK;
 }
 
-int copy(int device, void *dst, const void *src, size_t bytes, bool up) {
-  if (bytes == 0) return ND_OK;
+int copy(int device, int n, void *const *dst, const void *const *src, const size_t *bytes, bool up) {
   ND_CUDA(cudaSetDevice(device));
-  if (bytes >= STAGED_MIN && nd_host_threads() > 2 && pageable(up ? src : dst)) {
-    std::unique_lock<std::mutex> lock(g_ring.m, std::try_to_lock);
-    if (lock.owns_lock() && ring_ready(device))
-      return up ? staged((unsigned char *)const_cast<void *>(src), (unsigned char *)dst, bytes, true)
-                : staged((unsigned char *)dst, (unsigned char *)const_cast<void *>(src), bytes, false);
+  std::vector<Segment> segments;
+  size_t all = 0;
+  bool stage = nd_host_threads() > 2;
+  for (int k = 0; k < n; k++) {
+    if (!bytes[k]) continue;
+    unsigned char *d = (unsigned char *)dst[k], *s = (unsigned char *)const_cast<void *>(src[k]);
+    segments.push_back(up ? Segment{s, d, bytes[k]} : Segment{d, s, bytes[k]});
+    all += bytes[k];
   }
-  ND_CUDA(cudaMemcpy(dst, src, bytes, up ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost));
+  if (stage && all >= STAGED_MIN) {
+    for (const Segment &g : segments) stage = stage && pageable(g.host);
+    std::unique_lock<std::mutex> lock(g_ring.m, std::try_to_lock);
+    if (stage && lock.owns_lock() && ring_ready(device)) return staged(segments, all, up);
+  }
+  for (const Segment &g : segments)
+    ND_CUDA(cudaMemcpy(up ? g.dev : g.host, up ? g.host : g.dev, g.bytes, up ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost));
   return ND_OK;
 }
 
 }  // namespace
 
-int nd_copy_to_host(int device, void *dst, const void *src, size_t bytes) { return copy(device, dst, src, bytes, false); }
-int nd_copy_to_device(int device, void *dst, const void *src, size_t bytes) { return copy(device, dst, src, bytes, true); }
+int nd_copies_to_host(int device, int n, void *const *dst, const void *const *src, const size_t *bytes) { return copy(device, n, dst, src, bytes, false); }
+int nd_copies_to_device(int device, int n, void *const *dst, const void *const *src, const size_t *bytes) { return copy(device, n, dst, src, bytes, true); }
+int nd_copy_to_host(int device, void *dst, const void *src, size_t bytes) { return copy(device, 1, &dst, &src, &bytes, false); }
+int nd_copy_to_device(int device, void *dst, const void *src, size_t bytes) { return copy(device, 1, &dst, &src, &bytes, true); }
 
 // ---------------------------------------------------------------- device memory that is kept
 

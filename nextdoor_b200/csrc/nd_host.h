@@ -25,6 +25,8 @@ void nd_host_ranges(int64_t count, int threads, F fn) {
 // Blocking copies on a stream of their own: everything the copy depends on has to be complete.
 int nd_copy_to_host(int device, void *dst, const void *src, size_t bytes);
 int nd_copy_to_device(int device, void *dst, const void *src, size_t bytes);
+int nd_copies_to_host(int device, int n, void *const *dst, const void *const *src, const size_t *bytes);     // several as one
+int nd_copies_to_device(int device, int n, void *const *dst, const void *const *src, const size_t *bytes);
 
 // Device memory for building graphs.  Blocks of up to 384 MB are kept for the next build when they are freed, 1 GB of
 // them in all, while graphs or samplers are alive (a cudaMalloc / cudaFree pair costs 0.5 to 30 ms, by the box); a

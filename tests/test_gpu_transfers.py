@@ -66,3 +66,41 @@ def test_loader_sorts_by_all_bits_that_differ(nd, ndo, n, weights):
     exp_max = np.zeros(g.V, np.float32)
     np.maximum.at(exp_max, src, w)
     assert np.array_equal(max_w, exp_max)
+
+
+@pytest.mark.parametrize("repeats", [2, 31, 32, 33, 34, 4095, 4096, 4097, 9000])
+def test_loader_sorts_the_weights_of_repeated_edges(nd, repeats):
+    rng = np.random.default_rng(repeats)
+    pairs = np.stack([rng.integers(0, 40, 24), rng.integers(0, 40, 24)])
+    e = rng.permutation(np.concatenate([np.repeat(np.arange(23), rng.integers(1, 40, 23)), np.full(repeats, 23)]))
+    src, dst, w = pairs[0, e].astype(np.int32), pairs[1, e].astype(np.int32), (rng.random(len(e)) * 4 - 2).astype(np.float32)
+    row_ptr, col, got_w, _ = nd.Graph.from_edge_records(src, dst, w).to_host()
+    order = np.lexsort((w, dst, src))
+    assert np.array_equal(col, dst[order]) and np.array_equal(got_w, w[order])
+
+
+@pytest.mark.parametrize("S", [1, 31, 32, 255, 256, 257, 5000])
+@pytest.mark.parametrize("stop", [0.02, 0.6])
+def test_rows_packed_at_the_edges_of_a_chunk(nd, small_graph, S, stop):
+    import torch
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    V, steps = small_graph.V, 100
+    s = nd.Sampler(g, nd.app_params(2, steps=steps, seed=5, stop_prob=stop), num_samples=S)
+    full = torch.full((S, steps), V, dtype=torch.int32, device="cuda")
+    full_len = torch.zeros(S, dtype=torch.int32, device="cuda")
+    scratch = torch.empty(nd.rows_scratch_words(S), dtype=torch.int32, device="cuda")
+    host, host_len = np.full(S * steps, V, np.int32), np.zeros(S, np.int32)
+    rng = np.random.default_rng(S)
+    for _ in range(3):
+        s.set_initial(np.where(rng.random(S) < 0.2, -1, rng.integers(0, V, S)).astype(np.int32))
+        s.sample(1)
+        dense = s.final_samples()
+        len_ptr, vals_ptr = s.pack_rows()
+        assert s.pack_rows_total() == int((dense != V).sum())
+        nd.rows_unpack(0, None, S, steps, V, len_ptr, vals_ptr, full.data_ptr(), full_len.data_ptr(), scratch.data_ptr())
+        torch.cuda.synchronize()
+        assert np.array_equal(full.cpu().numpy(), dense)
+        s.host_update_begin(host, host_len)
+        s.host_update_fetch()
+        s.host_update_finish()
+        assert np.array_equal(host.reshape(S, steps), dense) and np.array_equal(host_len, (dense != V).sum(axis=1))
