@@ -28,7 +28,7 @@ struct NdHostRows {
   cudaStream_t cs = nullptr;
   int32_t *out = nullptr, *row_len = nullptr;
   int64_t total = 0;
-  std::vector<int64_t> part;    // sums of the lengths of the threads' row ranges
+  uint32_t *h_chunk = nullptr;  // pinned: d_chunk of the job being copied
   bool dense = false;           // most slots are in use: the dense array is copied as it is
   int stage = 0;                // 0 idle, 1 begun, 2 fetched
   int threads = 1;
@@ -36,21 +36,57 @@ struct NdHostRows {
 
 namespace {
 
-constexpr int PACK_THREADS = 256, PACK_PER_THREAD = 16, PACK_ROWS = PACK_THREADS * PACK_PER_THREAD;
+constexpr int PACK_ROWS = 256;   // rows of a chunk: one per thread of a CTA
 
-__global__ void __launch_bounds__(PACK_THREADS)
+// Where a warp's rows lie in the packed array.  A row is three or four vertices in a line of its own, so the kernels are
+// bound by how many of those lines are asked for at a time: a lane per row for the lengths, then a lane per vertex,
+// which finds its row by bisecting the warp's prefix sums, so that packed vertices are read and written coalesced
+// whatever the lengths (512k rows of PPR: 51 -> 12 us).
+struct WarpRows {
+  uint32_t len, inc;    // the lane's row: length, inclusive prefix in the warp
+  uint32_t total;       // of the warp
+  size_t pos;           // of the warp's first vertex
+
+  __device__ __forceinline__ WarpRows(const int32_t *__restrict__ lens, int64_t row, int64_t S, const uint32_t *__restrict__ chunk_base, uint32_t *wsum) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    len = row < S ? (uint32_t)lens[row] : 0u;
+    inc = len;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += u;
+    }
+    total = __shfl_sync(0xffffffffu, inc, 31);
+    if (lane == 0) wsum[warp] = total;
+    __syncthreads();
+    pos = chunk_base[blockIdx.x];
+    for (int w = 0; w < warp; w++) pos += wsum[w];
+  }
+  // fn(lane of the row, slot in the row, place in the warp's packed vertices)
+  template <typename F>
+  __device__ __forceinline__ void each(F fn) const {
+    for (uint32_t base = 0; base < total; base += 32) {
+      const uint32_t k = base + (threadIdx.x & 31);
+      int r = 0;
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1)
+        if (__shfl_sync(0xffffffffu, inc, r + step - 1) <= k) r += step;
+      const uint32_t first = __shfl_sync(0xffffffffu, inc - len, r);
+      if (k < total) fn(r, k - first, k);
+    }
+  }
+};
+
+__global__ void __launch_bounds__(PACK_ROWS)
 pack_sum_kernel(const int32_t *__restrict__ plen, int64_t S, uint32_t *__restrict__ chunk) {
-  __shared__ uint32_t wsum[PACK_THREADS / 32];
+  __shared__ uint32_t wsum[PACK_ROWS / 32];
   const int64_t first = (int64_t)blockIdx.x * PACK_ROWS;
-  uint32_t t = 0;
-  for (int r = threadIdx.x; r < PACK_ROWS; r += PACK_THREADS)
-    if (first + r < S) t += (uint32_t)plen[first + r];
+  uint32_t t = first + threadIdx.x < S ? (uint32_t)plen[first + threadIdx.x] : 0u;
   for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
   if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = t;
   __syncthreads();
   if (threadIdx.x == 0) {
     uint32_t a = 0;
-    for (int w = 0; w < PACK_THREADS / 32; w++) a += wsum[w];
+    for (int w = 0; w < PACK_ROWS / 32; w++) a += wsum[w];
     chunk[blockIdx.x] = a;
   }
 }
@@ -84,69 +120,27 @@ __global__ void __launch_bounds__(1024) pack_scan_kernel(uint32_t *__restrict__ 
 
 // the inverse of pack_rows_kernel on the receiving side: row r of `out` takes its len[r] vertices
 // from vals, the slots it held before beyond that (row_len[r]) go back to the invalid id
-__global__ void __launch_bounds__(PACK_THREADS)
+__global__ void __launch_bounds__(PACK_ROWS)
 unpack_rows_kernel(const int32_t *__restrict__ len, const int32_t *__restrict__ vals, const uint32_t *__restrict__ chunk_base,
                    int64_t S, int steps, int32_t invalid, int32_t *__restrict__ out, int32_t *__restrict__ row_len) {
-  __shared__ uint32_t wsum[PACK_THREADS / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t first = (int64_t)blockIdx.x * PACK_ROWS + (int64_t)threadIdx.x * PACK_PER_THREAD;
-  int32_t l[PACK_PER_THREAD];
-  uint32_t t = 0;
-#pragma unroll
-  for (int r = 0; r < PACK_PER_THREAD; r++) {
-    l[r] = first + r < S ? len[first + r] : 0;
-    t += (uint32_t)l[r];
-  }
-  uint32_t inc = t;
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += u;
-  }
-  if (lane == 31) wsum[warp] = inc;
-  __syncthreads();
-  size_t pos = (size_t)chunk_base[blockIdx.x] + inc - t;
-  for (int w = 0; w < warp; w++) pos += wsum[w];
-#pragma unroll
-  for (int r = 0; r < PACK_PER_THREAD; r++) {
-    if (first + r >= S) break;
-    int32_t *row = out + (first + r) * steps;
-    const int32_t had = row_len[first + r];
-    for (int k = 0; k < l[r]; k++) row[k] = vals[pos + k];
-    for (int k = l[r]; k < had; k++) row[k] = invalid;
-    if (had != l[r]) row_len[first + r] = l[r];
-    pos += (size_t)l[r];
-  }
+  __shared__ uint32_t wsum[PACK_ROWS / 32];
+  const int64_t mine = (int64_t)blockIdx.x * PACK_ROWS + threadIdx.x, first = mine - (threadIdx.x & 31);
+  const WarpRows rows(len, mine, S, chunk_base, wsum);
+  rows.each([&](int r, uint32_t slot, uint32_t k) { out[(first + r) * steps + slot] = vals[rows.pos + k]; });
+  if (mine >= S) return;
+  const int32_t had = row_len[mine];
+  for (int k = (int)rows.len; k < had; k++) out[mine * steps + k] = invalid;
+  if (had != (int)rows.len) row_len[mine] = (int32_t)rows.len;
 }
 
-// a thread owns PACK_PER_THREAD consecutive rows; their prefixes go to vals back to back
-__global__ void __launch_bounds__(PACK_THREADS)
+// the rows' prefixes to vals, back to back
+__global__ void __launch_bounds__(PACK_ROWS)
 pack_rows_kernel(const int32_t *__restrict__ plen, const int32_t *__restrict__ out, int64_t S, int steps,
                  const uint32_t *__restrict__ chunk_base, int32_t *__restrict__ vals) {
-  __shared__ uint32_t wsum[PACK_THREADS / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t first = (int64_t)blockIdx.x * PACK_ROWS + (int64_t)threadIdx.x * PACK_PER_THREAD;
-  int32_t l[PACK_PER_THREAD];
-  uint32_t t = 0;
-#pragma unroll
-  for (int r = 0; r < PACK_PER_THREAD; r++) {
-    l[r] = first + r < S ? plen[first + r] : 0;
-    t += (uint32_t)l[r];
-  }
-  uint32_t inc = t;
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += u;
-  }
-  if (lane == 31) wsum[warp] = inc;
-  __syncthreads();
-  size_t pos = (size_t)chunk_base[blockIdx.x] + inc - t;
-  for (int w = 0; w < warp; w++) pos += wsum[w];
-#pragma unroll
-  for (int r = 0; r < PACK_PER_THREAD; r++) {
-    const int32_t *row = out + (first + r) * steps;
-    for (int k = 0; k < l[r]; k++) vals[pos + k] = row[k];
-    pos += (size_t)l[r];
-  }
+  __shared__ uint32_t wsum[PACK_ROWS / 32];
+  const int64_t mine = (int64_t)blockIdx.x * PACK_ROWS + threadIdx.x, first = mine - (threadIdx.x & 31);
+  const WarpRows rows(plen, mine, S, chunk_base, wsum);
+  rows.each([&](int r, uint32_t slot, uint32_t k) { vals[rows.pos + k] = out[(first + r) * steps + slot]; });
 }
 
 // positions in the packed array are 32-bit
@@ -161,6 +155,7 @@ int hostrows_init(nd_sampler *s) {
   h->n_chunks = (int)((S1 + PACK_ROWS - 1) / PACK_ROWS);
   h->threads = nd_host_threads();
   cudaError_t e = cudaMallocHost(&h->h_len, sizeof(int32_t) * S1);
+  if (e == cudaSuccess) e = cudaMallocHost(&h->h_chunk, sizeof(uint32_t) * ((size_t)h->n_chunks + 1));
   if (e == cudaSuccess) e = cudaMallocHost(&h->h_total, sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMalloc(&h->d_chunk, sizeof(uint32_t) * ((size_t)h->n_chunks + 1));
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->packed, cudaEventDisableTiming);
@@ -180,9 +175,9 @@ int hostrows_init(nd_sampler *s) {
 int pack_enqueue(nd_sampler *s) {
   NdHostRows *h = s->hostrows;
   ND_TRY(nd_walk_ensure_tmp(s));
-  pack_sum_kernel<<<h->n_chunks, PACK_THREADS, 0, s->stream>>>(s->d_plen, s->S, h->d_chunk);
+  pack_sum_kernel<<<h->n_chunks, PACK_ROWS, 0, s->stream>>>(s->d_plen, s->S, h->d_chunk);
   pack_scan_kernel<<<1, 1024, 0, s->stream>>>(h->d_chunk, h->n_chunks);
-  pack_rows_kernel<<<h->n_chunks, PACK_THREADS, 0, s->stream>>>(s->d_plen, s->d_out, s->S, s->fs, h->d_chunk, s->d_tmp);
+  pack_rows_kernel<<<h->n_chunks, PACK_ROWS, 0, s->stream>>>(s->d_plen, s->d_out, s->S, s->fs, h->d_chunk, s->d_tmp);
   nd_count_launches(3);
   ND_CUDA(cudaGetLastError());
   return ND_OK;
@@ -197,6 +192,7 @@ void nd_hostrows_free(nd_sampler *s) {
   if (!h) return;
   if (h->h_len) cudaFreeHost(h->h_len);
   if (h->h_vals) cudaFreeHost(h->h_vals);
+  if (h->h_chunk) cudaFreeHost(h->h_chunk);
   cudaFree(h->d_chunk);
   if (h->packed) cudaEventDestroy(h->packed);
   if (h->len_done) cudaEventDestroy(h->len_done);
@@ -237,6 +233,8 @@ int nd_sampler_host_update_begin(nd_sampler *s, int32_t *out, int32_t *row_len, 
     ND_CUDA(cudaStreamWaitEvent(h->cs, h->packed, 0));
   }
   ND_CUDA(cudaMemcpyAsync(h->h_len, s->d_plen, sizeof(int32_t) * (size_t)s->S, cudaMemcpyDeviceToHost, h->cs));
+  if (packable(s))
+    ND_CUDA(cudaMemcpyAsync(h->h_chunk, h->d_chunk, sizeof(uint32_t) * ((size_t)h->n_chunks + 1), cudaMemcpyDeviceToHost, h->cs));
   ND_CUDA(cudaEventRecord(h->len_done, h->cs));
   if (h->cs != s->stream) {  // the next sampling of this sampler waits for the copies that read its buffers
     if (!s->copy_done) ND_CUDA(cudaEventCreateWithFlags(&s->copy_done, cudaEventDisableTiming));
@@ -256,15 +254,7 @@ int nd_sampler_host_update_fetch(nd_sampler *s) {
   if (s->S == 0) { h->stage = 2; return ND_OK; }
   ND_CUDA(cudaSetDevice(s->g->device));
   ND_CUDA(cudaEventSynchronize(h->len_done));
-  h->part.assign((size_t)h->threads + 1, 0);
-  std::vector<int64_t> &part = h->part;
-  const int32_t *len = h->h_len;
-  nd_host_ranges(s->S, h->threads, [&](int t, int64_t a, int64_t b) {
-    int64_t sum = 0;
-    for (int64_t i = a; i < b; i++) sum += len[i];
-    part[(size_t)t + 1] = sum;
-  });
-  for (int64_t v : part) h->total += v;
+  if (packable(s)) h->total = (int64_t)h->h_chunk[h->n_chunks];
   h->dense = 2 * h->total > s->S * (int64_t)s->fs || !packable(s);
   if (h->dense) {
     ND_CUDA(cudaMemcpyAsync(h->out, s->d_out, sizeof(int32_t) * (size_t)s->S * s->fs, cudaMemcpyDeviceToHost, h->cs));
@@ -306,11 +296,10 @@ int nd_sampler_host_update_finish(nd_sampler *s, int64_t *values_copied) {
     });
     return ND_OK;
   }
-  // every thread needs the position of its first row in the packed array: the ranges' sums
-  std::vector<int64_t> &part = h->part;
-  for (size_t t = 1; t < part.size(); t++) part[t] += part[t - 1];
-  nd_host_ranges(s->S, h->threads, [&, out, row_len, len, vals](int t, int64_t a, int64_t b) {
-    const int32_t *src = vals + part[(size_t)t];
+  const uint32_t *chunk = h->h_chunk;
+  nd_host_ranges(s->S, h->threads, [=](int, int64_t a, int64_t b) {
+    const int32_t *src = vals + chunk[a / PACK_ROWS];   // the position of the range's first row in the packed array
+    for (int64_t i = a - a % PACK_ROWS; i < a; i++) src += len[i];
     constexpr int AHEAD = 24;   // rows lie apart and are not in any cache: ask for them before they are written
     for (int64_t i = a; i < b; i++) {
       if (i + AHEAD < b && (len[i + AHEAD] | row_len[i + AHEAD])) __builtin_prefetch(out + (i + AHEAD) * steps, 1);
@@ -367,9 +356,9 @@ int nd_rows_unpack(int device, void *stream, int64_t n_rows, int steps, int32_t 
   ND_CUDA(cudaSetDevice(device));
   cudaStream_t st = (cudaStream_t)stream;
   const int n_chunks = (int)((n_rows + PACK_ROWS - 1) / PACK_ROWS);
-  pack_sum_kernel<<<n_chunks, PACK_THREADS, 0, st>>>(d_len, n_rows, d_scratch);
+  pack_sum_kernel<<<n_chunks, PACK_ROWS, 0, st>>>(d_len, n_rows, d_scratch);
   pack_scan_kernel<<<1, 1024, 0, st>>>(d_scratch, n_chunks);
-  unpack_rows_kernel<<<n_chunks, PACK_THREADS, 0, st>>>(d_len, d_vals, d_scratch, n_rows, steps, invalid, d_out, d_row_len);
+  unpack_rows_kernel<<<n_chunks, PACK_ROWS, 0, st>>>(d_len, d_vals, d_scratch, n_rows, steps, invalid, d_out, d_row_len);
   nd_count_launches(3);
   ND_CUDA(cudaGetLastError());
   return ND_OK;
