@@ -1,20 +1,22 @@
 // Importance-sampled layers (FastGCN, LADIES): a CTA per sample, all layers of all samples in one launch.
 //
 // The union of a sample's neighbour lists is a bitmap with a bit per vertex; the rank of a set bit is the
-// candidate's index in the sorted unique union, so nothing is sorted.  Candidate weights are summed per group of
-// 512 candidates in fp64 and scanned; a draw bisects the group sums and finds its candidate inside one group with
-// a warp.  Sums are fp64, so they agree with the sorted sequential order to ~1e-16 (FastGCN's integer weights sum
-// exactly).
+// candidate's index in the sorted unique union, so nothing is sorted.  Candidate weights are summed per group (FastGCN:
+// of 512 vertices, LADIES: of 512 candidates) in fp64 and scanned; a draw bisects the group sums and finds its candidate
+// inside one group with a warp.  Sums are fp64, so they agree with the sorted sequential order to ~1e-16 (FastGCN's
+// integer weights sum exactly).
 //
 // What bounds it, and what is done about it (2^20 vertices, 1024 batches of 64, 2 layers of 64: FastGCN
-// 4.8 -> 2.16 ms, LADIES 5.7 -> 2.44 ms):
+// 4.8 -> 1.13 ms, LADIES 5.7 -> 2.44 ms):
 //  * The second layer's transits are hubs (FastGCN draws them with the square of their degree), many of them the
 //    same one: repeated transits of a batch are taken once (LADIES with their multiplicity).
 //  * A hub's list (up to 140 K ids) costs a shared-memory test per id.  Vertices with at least V/64 neighbours
 //    have their neighbourhood as a bitmap, built once per graph: V/8 bytes that are ORed in registers, word by
 //    word, and stored to the union once; and an adjacency probe of such a transit is a bit test.
-//  * FastGCN's candidates are written out in order and their deg^2 fetched from an array of floats with many loads
-//    in flight: a thread that walks the bits of its words waits for every one (more than half of the time).
+//  * FastGCN's weights are summed without a list of candidates (writing that and fetching deg^2 one by one took more
+//    than half of the time): the degrees lie in vertex order as two planes of bytes, a lane takes eight vertices with one
+//    16-byte load, masks them with its byte of the bitmap and squares and sums them with dp4a.  Vertices with 2048
+//    neighbours or more, whose squares would overflow the 32-bit group sums, are a short list per graph.
 //  * LADIES' terms (w / rowsum)^2 depend on the edge alone: an array, built once per graph, instead of a pass over
 //    the weights and a division per entry and sample.  They are added up in shared memory, in tiles of
 //    consecutive candidates (lists are sorted, so a tile is a range of every list, all of them searched for at
@@ -22,6 +24,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
+#include <vector>
 
 #include "nd_collective.cuh"
 
@@ -30,8 +33,9 @@ namespace {
 using ndrng::Rng;
 
 constexpr int GROUP_WORDS = 16;   // words whose candidates are counted together
-constexpr int GROUP = 512;        // candidates whose weights are summed together
-constexpr int DENSE = 6;           // candidates of a bitmap word from which the warp writes them together
+constexpr int GROUP = 512;        // candidates (FastGCN: vertices, GROUP_WORDS words) whose weights are summed together
+constexpr int BIG_DEGREE = 2048;  // from here a vertex is on the list of big ones and its code is 0: 512 * 2047^2 < 2^31
+constexpr int FLIGHT = 4;         // groups a warp sums at a time
 constexpr int BIG_LIST = 4096;    // lists at least this long are streamed by the whole CTA
 constexpr int VEC = 4;            // 16-byte loads in flight per thread
 constexpr int CHUNK = 128;        // list entries a warp takes at a time (LADIES)
@@ -58,13 +62,14 @@ struct Args {
   unsigned char *gscratch;
   const int32_t *initial;
   int32_t *out;
-  float *wts_all;                          // [CTAs][V] the candidates' weights, in order
-  uint32_t *cand_all;                      // FastGCN: [CTAs][V] the candidates
+  float *wts_all;                          // LADIES: [CTAs][V] the candidates' weights, in order
   int32_t *pos_all;                        // LADIES: [CTAs][tiles + 1][transits] where the tiles begin in the lists
   int pos_stride;                          // ... entries per CTA
   int32_t *adj_row, *adj_col;
   float *prob;
-  const float *__restrict__ deg2;          // FastGCN: deg * deg
+  const uint4 *__restrict__ deg;           // FastGCN: the degrees of eight vertices, low bytes (x, y), high bytes (z, w)
+  const NdBigVertex *__restrict__ big;     // FastGCN: vertices with degrees from BIG_DEGREE, in order
+  int n_big;
   const float *__restrict__ term;          // LADIES: (w / rowsum)^2 per entry
   const int32_t *__restrict__ hub_slot;    // [V] slot of the vertex's bitmap, -1: none
   const uint32_t *__restrict__ hub_bits;   // [slots][words]
@@ -173,6 +178,17 @@ __device__ __forceinline__ int32_t lower_bound(const int32_t *__restrict__ col, 
   return e0;
 }
 
+// bits 0..3 -> 0xff in bytes 0..3
+__device__ __forceinline__ uint32_t byte_mask(uint32_t bits) { return (((bits & 15u) * 0x204081u) & 0x01010101u) * 255u; }
+
+// sum of deg^2 over the vertices of `bits` (eight vertices, degrees as in Args::deg)
+__device__ __forceinline__ uint32_t sum_squares(uint32_t bits, const uint4 &d) {
+  const uint32_t m0 = byte_mask(bits), m1 = byte_mask(bits >> 4);
+  const uint32_t l0 = d.x & m0, l1 = d.y & m1, h0 = d.z & m0, h1 = d.w & m1;
+  const uint32_t ll = __dp4a(l1, l1, __dp4a(l0, l0, 0u)), lh = __dp4a(l1, h1, __dp4a(l0, h0, 0u)), hh = __dp4a(h1, h1, __dp4a(h0, h0, 0u));
+  return ll + (lh << 9) + (hh << 16);
+}
+
 template <bool LADIES>
 __global__ void __launch_bounds__(1024, 1)
 coll_bitmap_kernel(const __grid_constant__ Args a) {
@@ -195,8 +211,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
   uint32_t *pre = reinterpret_cast<uint32_t *>(smem + lay.off_pre);
   double *tile = reinterpret_cast<double *>(smem + lay.off_tile);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
-  float *wts = a.wts_all + (size_t)blockIdx.x * (size_t)cp.V;
-  uint32_t *cand = LADIES ? nullptr : a.cand_all + (size_t)blockIdx.x * (size_t)cp.V;
+  float *wts = LADIES ? a.wts_all + (size_t)blockIdx.x * (size_t)cp.V : nullptr;
   int32_t *pos_tab = LADIES ? a.pos_all + (size_t)blockIdx.x * (size_t)a.pos_stride : nullptr;
   unsigned long long ids_sum = 0, uniq_sum = 0, draws = 0;   // thread 0
   for (int64_t s = blockIdx.x; s < a.S;) {
@@ -251,72 +266,66 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
       for (int i = 0; i < nu - nh; i++)             // long lists: the whole CTA
         if (rest[i].deg >= BIG_LIST) stream_list(a.g, bm, rest[i].rs, rest[i].deg, tid, blockDim.x);
       __syncthreads();
-      // ---- candidates per group (and per quad of words inside it): half a warp takes the 16 words of a group
-      for (int w0 = warp * 32; w0 < lay.words; w0 += warps * 32) {
-        const int w = w0 + lane;
-        const uint32_t bits = w < lay.words ? bm[w] : 0u;
-        const uint32_t c = __popc(bits);
-        uint32_t inc = c;
-        for (int o = 1; o < GROUP_WORDS; o <<= 1) {
-          const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o, GROUP_WORDS);
-          if ((lane & (GROUP_WORDS - 1)) >= o) inc += t;
-        }
-        if (w < lay.words) {
-          if ((lane & (GROUP_WORDS - 1)) == GROUP_WORDS - 1) gpref[w / GROUP_WORDS] = inc;
-          if ((lane & 3) == 0) qpre[w >> 2] = (uint16_t)(inc - c);
-        }
-      }
-      __syncthreads();
-      const uint32_t U = scan_u32(gpref, lay.groups, red_u);
-      if (tid == 0) uniq_sum += U;
-      const int groups = (int)((U + GROUP - 1) / GROUP);   // of candidates
+      uint32_t U;
+      int groups;
       if (!LADIES) {
-        // ---- the candidates in order, then the weight of every group
-        // (a word with few candidates by its lane -- neighbouring lanes write neighbouring places --, one with many
-        // by the warp: a lane each would write a sector each)
-        for (int w0 = warp * 32; w0 < lay.words; w0 += warps * 32) {
-          const int w = w0 + lane;
-          uint32_t bits = w < lay.words ? bm[w] : 0u;
-          uint32_t r = 0;
-          if (bits) {
-            const uint4 q = reinterpret_cast<const uint4 *>(bm)[w >> 2];
-            r = gpref[w / GROUP_WORDS] + qpre[w >> 2];
-            r += (w & 3) > 0 ? __popc(q.x) : 0;
-            r += (w & 3) > 1 ? __popc(q.y) : 0;
-            r += (w & 3) > 2 ? __popc(q.z) : 0;
+        // ---- the groups' weights, and the number of candidates
+        const uint8_t *bytes = reinterpret_cast<const uint8_t *>(bm);
+        uint32_t seen = 0;
+        groups = lay.groups;
+        for (int g0 = warp * FLIGHT; g0 < groups; g0 += warps * FLIGHT) {
+          uint32_t bits[2 * FLIGHT];
+          uint4 d[2 * FLIGHT];
+#pragma unroll
+          for (int k = 0; k < 2 * FLIGHT; k++) {
+            const int at = g0 * (GROUP / 8) + k * 32 + lane;
+            bits[k] = at < groups * (GROUP / 8) ? bytes[at] : 0u;
+            d[k] = bits[k] ? __ldg(a.deg + at) : make_uint4(0u, 0u, 0u, 0u);
           }
-          uint32_t dense = __ballot_sync(0xffffffffu, __popc(bits) >= DENSE);
-          const bool mine = !((dense >> lane) & 1u);
-          while (dense) {
-            const int l = __ffs(dense) - 1;
-            dense &= dense - 1;
-            const uint32_t b = __shfl_sync(0xffffffffu, bits, l), r1 = __shfl_sync(0xffffffffu, r, l);
-            if ((b >> lane) & 1u) cand[r1 + __popc(b & ((1u << lane) - 1u))] = (uint32_t)(((w0 + l) << 5) + lane);
+#pragma unroll
+          for (int k = 0; k < FLIGHT; k++) {
+            seen += __popc(bits[2 * k] | bits[2 * k + 1] << 8);
+            const uint32_t sum = __reduce_add_sync(0xffffffffu, sum_squares(bits[2 * k], d[2 * k]) + sum_squares(bits[2 * k + 1], d[2 * k + 1]));
+            if (lane == 0 && g0 + k < groups) gcdf[g0 + k] = (double)sum;
           }
-          if (mine)
-            while (bits) {
-              cand[r++] = (uint32_t)((w << 5) + __ffs(bits) - 1);
-              bits &= bits - 1;
-            }
         }
+        seen = __reduce_add_sync(0xffffffffu, seen);
+        if (lane == 0) red_u[warp] = seen;
         __syncthreads();
-        for (int gi = warp; gi < groups; gi += warps) {
-          float x[GROUP / 32];
-#pragma unroll
-          for (int k = 0; k < GROUP / 32; k++) {
-            const uint32_t r = (uint32_t)(gi * GROUP + k * 32 + lane);
-            x[k] = r < U ? __ldg(a.deg2 + __ldcg(cand + r)) : 0.f;
+        U = 0;
+        for (int w = 0; w < warps; w++) U += red_u[w];
+        for (int i0 = warp * 32; i0 < a.n_big; i0 += warps * 32) {   // the big ones; neighbours on the list mostly share a group
+          const NdBigVertex v = i0 + lane < a.n_big ? a.big[i0 + lane] : NdBigVertex{-1, 0.f};
+          const bool in = v.v >= 0 && ((bm[v.v >> 5] >> (v.v & 31)) & 1u);
+          double x = in ? (double)v.weight : 0.0;
+          int same;
+          __match_all_sync(0xffffffffu, v.v / GROUP, &same);
+          if (same) {
+            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+            if (lane == 0) atomicAdd(gcdf + v.v / GROUP, x);
+          } else if (in) {
+            atomicAdd(gcdf + v.v / GROUP, x);
           }
-#pragma unroll
-          for (int k = 0; k < GROUP / 32; k++)
-            if (gi * GROUP + k * 32 + lane < (int)U) wts[gi * GROUP + k * 32 + lane] = x[k];
-          double sum = 0.0;
-#pragma unroll
-          for (int k = 0; k < GROUP / 32; k++) sum += (double)x[k];
-          for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-          if (lane == 0) gcdf[gi] = sum;
         }
       } else {
+        // ---- candidates per group (and per quad of words inside it): half a warp takes the 16 words of a group
+        for (int w0 = warp * 32; w0 < lay.words; w0 += warps * 32) {
+          const int w = w0 + lane;
+          const uint32_t bits = w < lay.words ? bm[w] : 0u;
+          const uint32_t c = __popc(bits);
+          uint32_t inc = c;
+          for (int o = 1; o < GROUP_WORDS; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o, GROUP_WORDS);
+            if ((lane & (GROUP_WORDS - 1)) >= o) inc += t;
+          }
+          if (w < lay.words) {
+            if ((lane & (GROUP_WORDS - 1)) == GROUP_WORDS - 1) gpref[w / GROUP_WORDS] = inc;
+            if ((lane & 3) == 0) qpre[w >> 2] = (uint16_t)(inc - c);
+          }
+        }
+        __syncthreads();
+        U = scan_u32(gpref, lay.groups, red_u);
+        groups = (int)((U + GROUP - 1) / GROUP);   // of candidates
         // ---- the terms of every list entry, added up per candidate in tiles of consecutive candidates
         auto transit = [&](int i) -> const Transit & { return ut[i < nh ? i : cp.ntr - nu + i]; };
         int32_t *sh_pos = sh_mult;   // not needed any more
@@ -390,6 +399,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
         }
       }
       __syncthreads();
+      if (tid == 0) uniq_sum += U;
       scan_f64(gcdf, groups, red);
       const double total = groups > 0 ? gcdf[groups - 1] : 0.0;
       // ---- the layer's draws, a warp each
@@ -404,15 +414,35 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
             const int mid = lo + (hi - lo) / 2;
             if (gcdf[mid] >= target) hi = mid; else lo = mid + 1;
           }
+          // (a target of zero takes the first candidate of all, whatever its weight)
+          if (!LADIES && target <= 0.0) while (!__any_sync(0xffffffffu, bm[lo * GROUP_WORDS + (lane & (GROUP_WORDS - 1))])) lo++;
           const double before = lo > 0 ? gcdf[lo - 1] : 0.0;
-          // the group in four blocks of 128 candidates, a lane holding four of each: the first (block, lane) that
-          // reaches the target, then the first of its candidates that does
+          // the group in four blocks of 128 candidates (FastGCN: vertices), a lane holding four of each: the first (block,
+          // lane) that reaches the target, then the first of its candidates that does
           float x[4][4];
+          uint32_t there = 0;   // which of the lane's sixteen are candidates
 #pragma unroll
           for (int q = 0; q < 4; q++) {
             const uint32_t r = (uint32_t)(lo * GROUP + q * 128 + lane * 4);
+            if (LADIES) {
 #pragma unroll
-            for (int k = 0; k < 4; k++) x[q][k] = r + k < U ? __ldcg(wts + r + k) : 0.f;
+              for (int k = 0; k < 4; k++) {
+                x[q][k] = r + k < U ? __ldcg(wts + r + k) : 0.f;
+                there |= r + k < U ? 1u << (4 * q + k) : 0u;
+              }
+            } else {
+              const uint32_t bits = (bm[r >> 5] >> (r & 31)) & 15u;
+              const uint32_t *codes = reinterpret_cast<const uint32_t *>(a.deg + (r >> 3)) + ((r >> 2) & 1u);
+              const uint32_t low = bits ? __ldg(codes) : 0u, high = bits ? __ldg(codes + 2) : 0u;
+              there |= bits << (4 * q);
+#pragma unroll
+              for (int k = 0; k < 4; k++) {
+                int32_t d = (int32_t)((low >> (8 * k) & 255u) | (high >> (8 * k) & 255u) << 8);
+                if (((bits >> k) & 1u) == 0) d = 0;
+                else if (d == 0) d = __ldg(a.g.row_ptr + r + k + 1) - __ldg(a.g.row_ptr + r + k);
+                x[q][k] = __fmul_rn(__int2float_rn(d), __int2float_rn(d));
+              }
+            }
           }
           double at_block = before, lane_before = 0.0;
           bool found = false;
@@ -425,7 +455,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
               const double t = __shfl_up_sync(0xffffffffu, run, o);
               if (lane >= o) run += t;
             }
-            const bool some = (uint32_t)(lo * GROUP + q * 128 + lane * 4) < U;
+            const bool some = (there >> (4 * q)) & 15u;
             const uint32_t reach = __ballot_sync(0xffffffffu, some && at_block + run >= target), any = __ballot_sync(0xffffffffu, some);
             // (nobody reaches it, by rounding: the last candidates of the group)
             if (bq < 0 || !found) {
@@ -443,18 +473,19 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
           float wt = 0.f;
           double run = lane_before;
           bool hit = false;
+          const uint32_t its = __shfl_sync(0xffffffffu, there, bl) >> (4 * bq);
 #pragma unroll
           for (int k = 0; k < 4; k++) {
             const float own = bq == 0 ? x[0][k] : bq == 1 ? x[1][k] : bq == 2 ? x[2][k] : x[3][k];
             const float t = __shfl_sync(0xffffffffu, own, bl);
             run += (double)t;
-            if (!hit && first + k < U) {
+            if (!hit && ((its >> k) & 1u)) {
               rank = first + k;
               wt = t;
               hit = run >= target;
             }
           }
-          pick = LADIES ? vertex_of_rank(bm, gpref, lay.groups, rank) : (int32_t)__ldcg(cand + rank);
+          pick = LADIES ? vertex_of_rank(bm, gpref, lay.groups, rank) : (int32_t)rank;
           pr = (float)((double)wt / total);
         }
         if (lane == 0) {
@@ -488,10 +519,24 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
 
 // ---------------------------------------------------------------- arrays built once per graph
 
-__global__ void deg2_build_kernel(const int32_t *__restrict__ row_ptr, int32_t V, float *__restrict__ deg2) {
-  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x) {
-    const float d = __int2float_rn(row_ptr[v + 1] - row_ptr[v]);
-    deg2[v] = __fmul_rn(d, d);
+// a thread per eight vertices; the big ones go on the list (of `cap`), in any order
+__global__ void deg_build_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int64_t units, uint4 *__restrict__ deg, NdBigVertex *__restrict__ big,
+                                 int32_t *__restrict__ n_big, int cap) {
+  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < units; u += (int64_t)gridDim.x * blockDim.x) {
+    uint32_t low[2] = {0u, 0u}, high[2] = {0u, 0u};
+    for (int k = 0; k < 8; k++) {
+      const int64_t v = 8 * u + k;
+      if (v >= V) break;
+      const int32_t d = row_ptr[v + 1] - row_ptr[v];
+      if (d >= BIG_DEGREE) {
+        const int at = atomicAdd(n_big, 1);
+        if (at < cap) big[at] = NdBigVertex{(int32_t)v, __fmul_rn(__int2float_rn(d), __int2float_rn(d))};
+        continue;
+      }
+      low[k >> 2] |= (uint32_t)(d & 255) << (8 * (k & 3));
+      high[k >> 2] |= (uint32_t)(d >> 8) << (8 * (k & 3));
+    }
+    deg[u] = make_uint4(low[0], low[1], high[0], high[1]);
   }
 }
 
@@ -573,11 +618,24 @@ int ensure_layers(const nd_graph *g, int sms, bool ladies) {
     cudaFree(hubs);
     g->hub_slot = slot;
   }
-  if (!ladies && !g->deg2) {
-    float *d = nullptr;
-    ND_CUDA(cudaMalloc(&d, sizeof(float) * (size_t)g->V));
-    deg2_build_kernel<<<grid, 256>>>(g->row_ptr, g->V, d);
-    g->deg2 = d;
+  if (!ladies && !g->deg_codes) {
+    uint4 *deg = nullptr;
+    const int64_t units = 4 * (int64_t)words_of(g->V);
+    const int cap = (int)(g->E / BIG_DEGREE) + 1;
+    int32_t *count = nullptr, n = 0;
+    ND_CUDA(cudaMalloc(&deg, sizeof(uint4) * (size_t)std::max<int64_t>(units, 1)));
+    if (!g->big) ND_CUDA(cudaMalloc(&g->big, sizeof(NdBigVertex) * (size_t)cap));
+    ND_CUDA(cudaMalloc(&count, sizeof(int32_t)));
+    ND_CUDA(cudaMemset(count, 0, sizeof(int32_t)));
+    deg_build_kernel<<<grid, 256>>>(g->row_ptr, g->V, units, deg, g->big, count, cap);
+    ND_CUDA(cudaMemcpy(&n, count, sizeof(n), cudaMemcpyDeviceToHost));
+    cudaFree(count);
+    std::vector<NdBigVertex> big((size_t)n);
+    ND_CUDA(cudaMemcpy(big.data(), g->big, sizeof(NdBigVertex) * (size_t)n, cudaMemcpyDeviceToHost));
+    std::sort(big.begin(), big.end(), [](const NdBigVertex &x, const NdBigVertex &y) { return x.v < y.v; });
+    ND_CUDA(cudaMemcpy(g->big, big.data(), sizeof(NdBigVertex) * (size_t)n, cudaMemcpyHostToDevice));
+    g->n_big = n;
+    g->deg_codes = deg;
   }
   if (ladies && !g->term) {
     const size_t E = (size_t)(g->E > 0 ? g->E : 1);
@@ -618,8 +676,8 @@ Plan plan_of(const nd_sampler *s) {
   l.groups = l.words / GROUP_WORDS;
   uint32_t big = 4u * (uint32_t)l.words;       // a multiple of 64
   l.off_gcdf = big; big += 8u * (uint32_t)l.groups;
-  l.off_gpref = big; big += 4u * (uint32_t)(l.groups + 1);
-  l.off_qpre = big; big += 2u * (uint32_t)(l.words / 4);
+  l.off_gpref = big; big += ladies ? 4u * (uint32_t)(l.groups + 1) : 0u;
+  l.off_qpre = big; big += ladies ? 2u * (uint32_t)(l.words / 4) : 0u;
   big = (big + 255u) & ~255u;
   auto place = [&](uint32_t off) {
     l.off_red = off; off += 8u * 32u + 4u * 32u;
@@ -662,8 +720,7 @@ int nd_coll_bitmap_alloc(nd_sampler *s) {
   ND_TRY(ensure_layers(s->g, s->dev.sms, ladies));
   s->coll_grid = (int)std::min<int64_t>(s->S > 0 ? s->S : 1, (int64_t)s->dev.sms * p.per_sm);
   if (p.lay.glob_bytes) ND_CUDA(cudaMalloc(&s->d_bm, (size_t)p.lay.glob_bytes * (size_t)s->coll_grid));
-  ND_CUDA(cudaMalloc(&s->d_cand_w, sizeof(float) * (size_t)s->coll_grid * (size_t)s->g->V));
-  if (!ladies) ND_CUDA(cudaMalloc(&s->d_cand, sizeof(uint32_t) * (size_t)s->coll_grid * (size_t)s->g->V));
+  if (ladies) ND_CUDA(cudaMalloc(&s->d_cand_w, sizeof(float) * (size_t)s->coll_grid * (size_t)s->g->V));
   if (ladies) ND_CUDA(cudaMalloc(&s->d_runs, sizeof(int32_t) * (size_t)s->coll_grid * (size_t)pos_entries(s, p.lay)));
   ND_CUDA(cudaMalloc(&s->d_rows_acc, 16 * sizeof(unsigned long long)));
   ND_CUDA(cudaMemset(s->d_rows_acc, 0, 16 * sizeof(unsigned long long)));
@@ -674,9 +731,9 @@ int nd_coll_bitmap_launch(nd_sampler *s, const CollParams &cp, unsigned long lon
   const bool ladies = s->p.app == ND_APP_LADIES_IS;
   const Plan p = plan_of(s);
   const nd_graph *g = s->g;
-  const Args a{nd_view(g), cp, s->p.steps, s->S, p.lay, s->d_bm, s->d_initial, s->d_out, s->d_cand_w, (uint32_t *)s->d_cand,
+  const Args a{nd_view(g), cp, s->p.steps, s->S, p.lay, s->d_bm, s->d_initial, s->d_out, s->d_cand_w,
                s->d_runs, ladies ? pos_entries(s, p.lay) : 0, s->d_adj_row, s->d_adj_col, s->d_prob,
-               g->deg2, g->term, g->hub_slot, g->hub_bits, s->d_rows_acc, s->d_stats, pairs};
+               g->deg_codes, g->big, g->n_big, g->term, g->hub_slot, g->hub_bits, s->d_rows_acc, s->d_stats, pairs};
   if (ladies) {
     ND_CUDA(cudaFuncSetAttribute(coll_bitmap_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.lay.bytes));
     coll_bitmap_kernel<true><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);

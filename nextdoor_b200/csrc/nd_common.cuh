@@ -62,6 +62,11 @@ int nd_device_info(int device, NdDeviceInfo *info);
 // becomes 8 bytes of row offsets + 4 bytes of max weight), col[E] int32 sorted per row by
 // (neighbour, weight), w[E] fp32.
 
+struct NdBigVertex {
+  int32_t v;
+  float weight;   // deg * deg
+};
+
 struct nd_graph {
   int device = 0;
   int32_t V = 0;
@@ -82,7 +87,9 @@ struct nd_graph {
   mutable uint8_t *wq = nullptr;       // [E] weights as whole 256ths of the row's maximum
   mutable int32_t *adjset = nullptr;   // node2vec membership: per-vertex hash sets of the neighbour ids, 8-slot buckets
   mutable uint32_t *adjsign = nullptr; // ... and the filter in front of them
-  mutable float *deg2 = nullptr;       // [V] deg * deg (FastGCN)
+  mutable uint4 *deg_codes = nullptr;  // degrees of eight vertices each (FastGCN)
+  mutable NdBigVertex *big = nullptr;  // [n_big] vertices whose degrees the codes do not hold
+  mutable int n_big = 0;
   mutable float *term = nullptr;       // [E] (w / rowsum)^2 (LADIES)
   mutable int32_t *hub_slot = nullptr; // [V] slot of the vertex's neighbourhood as a bitmap, -1: none
   mutable uint32_t *hub_bits = nullptr;

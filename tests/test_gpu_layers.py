@@ -1,0 +1,30 @@
+"""Importance layers where the degrees do not fit the packed codes: vertices around the degrees at which the second byte
+and the list of big vertices begin, vertices without neighbours among the candidates, graphs that end inside a group."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("V", [6000, 6144, 20_001])
+@pytest.mark.parametrize("degrees", [(1, 2), (255, 256, 257), (2046, 2047), (2047, 2048, 2049, 5000)])
+@pytest.mark.parametrize("scratch", ["0", "1"])
+def test_fastgcn_weights_at_the_edges_of_the_codes(nd, ndo, monkeypatch, V, degrees, scratch):
+    monkeypatch.setenv("ND_COLLECTIVE_SORT", "0")
+    monkeypatch.setenv("ND_COLLECTIVE_BITMAP_GLOBAL", scratch)
+    rng = np.random.default_rng(V + degrees[0])
+    hubs = np.unique(np.concatenate([rng.integers(0, 40, 20), rng.integers(0, V, 40), [V - 1]]))
+    deg = np.where(rng.random(V) < 0.1, 0, rng.integers(1, 6, V))
+    deg[hubs] = rng.choice(degrees, len(hubs))
+    src = np.repeat(np.arange(V), deg).astype(np.int32)
+    dst = np.where(rng.random(len(src)) < 0.2, rng.choice(hubs, len(src)), rng.integers(0, V, len(src))).astype(np.int32)
+    hg = ndo.csr_from_records(src, dst, np.ones(len(src), np.float32), V=V)
+    g = nd.Graph.from_csr(hg.row_ptr, hg.col, hg.w, hg.max_w)
+    S, L = 60, 32
+    s = nd.Sampler(g, nd.app_params(8, steps=2, fanout=L, batch=24, seed=3), num_samples=S, first_sample=2)
+    s.sample()
+    exp = ndo.sample(hg, ndo.make_params(8, steps=2, fanout=L, batch=24, seed=3), S, first=2)
+    aux = s.aux()
+    assert np.array_equal(s.final_samples(), exp["out"])   # whole numbers: the sums are exact
+    assert np.array_equal(aux["prob"].reshape(-1), exp["prob"].reshape(-1))
+    assert np.array_equal(aux["adj_row"], exp["adj_row"]) and np.array_equal(aux["adj_col"], exp["adj_col"])
