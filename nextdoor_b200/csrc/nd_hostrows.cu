@@ -21,7 +21,7 @@ struct NdHostRows {
   int32_t *h_len = nullptr;     // pinned [S]: the rows' lengths of the job being copied
   int32_t *h_vals = nullptr;    // pinned: packed vertices
   size_t vals_cap = 0;
-  uint32_t *d_chunk = nullptr;  // per chunk of PACK_ROWS rows: sum of lengths, then exclusive prefix
+  uint32_t *d_chunk = nullptr;  // per chunk of PACK_CHUNK rows: sum of lengths, then exclusive prefix
   int n_chunks = 0;
   cudaEvent_t packed = nullptr, len_done = nullptr, vals_done = nullptr, total_done = nullptr;
   uint32_t *h_total = nullptr;  // pinned: number of packed vertices (nd_sampler_pack_rows)
@@ -36,7 +36,8 @@ struct NdHostRows {
 
 namespace {
 
-constexpr int PACK_ROWS = 256;   // rows of a chunk: one per thread of a CTA
+constexpr int PACK_CHUNK = 4096;   // rows whose lengths are summed together
+constexpr int PACK_ROWS = 256;     // rows of a CTA, one per thread
 
 // Where a warp's rows lie in the packed array.  A row is three or four vertices in a line of its own, so the kernels are
 // bound by how many of those lines are asked for at a time: a lane per row for the lengths, then a lane per vertex,
@@ -56,10 +57,15 @@ struct WarpRows {
       if (lane >= o) inc += u;
     }
     total = __shfl_sync(0xffffffffu, inc, 31);
-    if (lane == 0) wsum[warp] = total;
+    // the rows of the chunk before the CTA's: a few loads that neighbouring CTAs share
+    uint32_t before = 0;
+    for (int64_t r = (int64_t)(blockIdx.x / (PACK_CHUNK / PACK_ROWS)) * PACK_CHUNK + threadIdx.x; r < (int64_t)blockIdx.x * PACK_ROWS; r += PACK_ROWS)
+      before += (uint32_t)lens[r];
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) { wsum[warp] = total; wsum[PACK_ROWS / 32 + warp] = before; }
     __syncthreads();
-    pos = chunk_base[blockIdx.x];
-    for (int w = 0; w < warp; w++) pos += wsum[w];
+    pos = chunk_base[blockIdx.x / (PACK_CHUNK / PACK_ROWS)];
+    for (int w = 0; w < PACK_ROWS / 32; w++) pos += wsum[PACK_ROWS / 32 + w] + (w < warp ? wsum[w] : 0u);
   }
   // fn(lane of the row, slot in the row, place in the warp's packed vertices)
   template <typename F>
@@ -79,8 +85,10 @@ struct WarpRows {
 __global__ void __launch_bounds__(PACK_ROWS)
 pack_sum_kernel(const int32_t *__restrict__ plen, int64_t S, uint32_t *__restrict__ chunk) {
   __shared__ uint32_t wsum[PACK_ROWS / 32];
-  const int64_t first = (int64_t)blockIdx.x * PACK_ROWS;
-  uint32_t t = first + threadIdx.x < S ? (uint32_t)plen[first + threadIdx.x] : 0u;
+  const int64_t first = (int64_t)blockIdx.x * PACK_CHUNK;
+  uint32_t t = 0;
+#pragma unroll
+  for (int r = threadIdx.x; r < PACK_CHUNK; r += PACK_ROWS) t += first + r < S ? (uint32_t)plen[first + r] : 0u;
   for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
   if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = t;
   __syncthreads();
@@ -123,7 +131,7 @@ __global__ void __launch_bounds__(1024) pack_scan_kernel(uint32_t *__restrict__ 
 __global__ void __launch_bounds__(PACK_ROWS)
 unpack_rows_kernel(const int32_t *__restrict__ len, const int32_t *__restrict__ vals, const uint32_t *__restrict__ chunk_base,
                    int64_t S, int steps, int32_t invalid, int32_t *__restrict__ out, int32_t *__restrict__ row_len) {
-  __shared__ uint32_t wsum[PACK_ROWS / 32];
+  __shared__ uint32_t wsum[PACK_ROWS / 16];
   const int64_t mine = (int64_t)blockIdx.x * PACK_ROWS + threadIdx.x, first = mine - (threadIdx.x & 31);
   const WarpRows rows(len, mine, S, chunk_base, wsum);
   rows.each([&](int r, uint32_t slot, uint32_t k) { out[(first + r) * steps + slot] = vals[rows.pos + k]; });
@@ -137,7 +145,7 @@ unpack_rows_kernel(const int32_t *__restrict__ len, const int32_t *__restrict__ 
 __global__ void __launch_bounds__(PACK_ROWS)
 pack_rows_kernel(const int32_t *__restrict__ plen, const int32_t *__restrict__ out, int64_t S, int steps,
                  const uint32_t *__restrict__ chunk_base, int32_t *__restrict__ vals) {
-  __shared__ uint32_t wsum[PACK_ROWS / 32];
+  __shared__ uint32_t wsum[PACK_ROWS / 16];
   const int64_t mine = (int64_t)blockIdx.x * PACK_ROWS + threadIdx.x, first = mine - (threadIdx.x & 31);
   const WarpRows rows(plen, mine, S, chunk_base, wsum);
   rows.each([&](int r, uint32_t slot, uint32_t k) { vals[rows.pos + k] = out[(first + r) * steps + slot]; });
@@ -152,7 +160,7 @@ int hostrows_init(nd_sampler *s) {
   s->hostrows = new NdHostRows();   // a creation that fails half way is taken down again, so the next call starts over
   NdHostRows *h = s->hostrows;
   const size_t S1 = (size_t)(s->S > 0 ? s->S : 1);
-  h->n_chunks = (int)((S1 + PACK_ROWS - 1) / PACK_ROWS);
+  h->n_chunks = (int)((S1 + PACK_CHUNK - 1) / PACK_CHUNK);
   h->threads = nd_host_threads();
   cudaError_t e = cudaMallocHost(&h->h_len, sizeof(int32_t) * S1);
   if (e == cudaSuccess) e = cudaMallocHost(&h->h_chunk, sizeof(uint32_t) * ((size_t)h->n_chunks + 1));
@@ -177,7 +185,7 @@ int pack_enqueue(nd_sampler *s) {
   ND_TRY(nd_walk_ensure_tmp(s));
   pack_sum_kernel<<<h->n_chunks, PACK_ROWS, 0, s->stream>>>(s->d_plen, s->S, h->d_chunk);
   pack_scan_kernel<<<1, 1024, 0, s->stream>>>(h->d_chunk, h->n_chunks);
-  pack_rows_kernel<<<h->n_chunks, PACK_ROWS, 0, s->stream>>>(s->d_plen, s->d_out, s->S, s->fs, h->d_chunk, s->d_tmp);
+  pack_rows_kernel<<<(unsigned)((s->S + PACK_ROWS - 1) / PACK_ROWS), PACK_ROWS, 0, s->stream>>>(s->d_plen, s->d_out, s->S, s->fs, h->d_chunk, s->d_tmp);
   nd_count_launches(3);
   ND_CUDA(cudaGetLastError());
   return ND_OK;
@@ -298,8 +306,8 @@ int nd_sampler_host_update_finish(nd_sampler *s, int64_t *values_copied) {
   }
   const uint32_t *chunk = h->h_chunk;
   nd_host_ranges(s->S, h->threads, [=](int, int64_t a, int64_t b) {
-    const int32_t *src = vals + chunk[a / PACK_ROWS];   // the position of the range's first row in the packed array
-    for (int64_t i = a - a % PACK_ROWS; i < a; i++) src += len[i];
+    const int32_t *src = vals + chunk[a / PACK_CHUNK];   // the position of the range's first row in the packed array
+    for (int64_t i = a - a % PACK_CHUNK; i < a; i++) src += len[i];
     constexpr int AHEAD = 24;   // rows lie apart and are not in any cache: ask for them before they are written
     for (int64_t i = a; i < b; i++) {
       if (i + AHEAD < b && (len[i + AHEAD] | row_len[i + AHEAD])) __builtin_prefetch(out + (i + AHEAD) * steps, 1);
@@ -345,7 +353,7 @@ int nd_sampler_pack_rows_total(nd_sampler *s, int64_t *total) {
   return ND_OK;
 }
 
-int64_t nd_rows_scratch_words(int64_t n_rows) { return (n_rows + PACK_ROWS - 1) / PACK_ROWS + 1; }
+int64_t nd_rows_scratch_words(int64_t n_rows) { return (n_rows + PACK_CHUNK - 1) / PACK_CHUNK + 1; }
 
 int nd_rows_unpack(int device, void *stream, int64_t n_rows, int steps, int32_t invalid, const int32_t *d_len,
                    const int32_t *d_vals, int32_t *d_out, int32_t *d_row_len, uint32_t *d_scratch) {
@@ -355,10 +363,10 @@ int nd_rows_unpack(int device, void *stream, int64_t n_rows, int steps, int32_t 
   ND_REQUIRE(n_rows * (int64_t)steps < ((int64_t)1 << 32), ND_ERR_RANGE, "nd_rows_unpack: array too large for 32-bit positions");
   ND_CUDA(cudaSetDevice(device));
   cudaStream_t st = (cudaStream_t)stream;
-  const int n_chunks = (int)((n_rows + PACK_ROWS - 1) / PACK_ROWS);
+  const int n_chunks = (int)((n_rows + PACK_CHUNK - 1) / PACK_CHUNK);
   pack_sum_kernel<<<n_chunks, PACK_ROWS, 0, st>>>(d_len, n_rows, d_scratch);
   pack_scan_kernel<<<1, 1024, 0, st>>>(d_scratch, n_chunks);
-  unpack_rows_kernel<<<n_chunks, PACK_ROWS, 0, st>>>(d_len, d_vals, d_scratch, n_rows, steps, invalid, d_out, d_row_len);
+  unpack_rows_kernel<<<(unsigned)((n_rows + PACK_ROWS - 1) / PACK_ROWS), PACK_ROWS, 0, st>>>(d_len, d_vals, d_scratch, n_rows, steps, invalid, d_out, d_row_len);
   nd_count_launches(3);
   ND_CUDA(cudaGetLastError());
   return ND_OK;

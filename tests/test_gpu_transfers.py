@@ -79,7 +79,7 @@ def test_loader_sorts_the_weights_of_repeated_edges(nd, repeats):
     assert np.array_equal(col, dst[order]) and np.array_equal(got_w, w[order])
 
 
-@pytest.mark.parametrize("S", [1, 31, 32, 255, 256, 257, 5000])
+@pytest.mark.parametrize("S", [1, 31, 32, 255, 256, 257, 4095, 4097, 9000])
 @pytest.mark.parametrize("stop", [0.02, 0.6])
 def test_rows_packed_at_the_edges_of_a_chunk(nd, small_graph, S, stop):
     import torch
