@@ -27,6 +27,26 @@ def _ptr(a):
     return a.ctypes.data_as(C.c_void_p) if a is not None else None
 
 
+class _ResultMemory:
+    """Memory of a result array; it goes back to the library, which keeps some for the next result, with the last view."""
+
+    def __init__(self, count, dtype, device):
+        p = C.c_void_p()
+        check(lib.nd_result_alloc(device, count * np.dtype(dtype).itemsize, C.byref(p)))
+        self._free, self._p = lib.nd_result_free, p
+        self.__array_interface__ = {"version": 3, "shape": (count,), "typestr": np.dtype(dtype).str, "data": (p.value, False)}
+
+    def __del__(self):
+        if getattr(self, "_p", None):
+            self._free(self._p)
+
+
+def _result_array(count, dtype, device):
+    """np.empty for results; large ones in memory that is not faulted in again for every call."""
+    large = 2 << 20 <= count * np.dtype(dtype).itemsize <= 128 << 20
+    return np.asarray(_ResultMemory(count, dtype, device)) if large else np.empty(count, dtype)
+
+
 def app_params(app, steps=None, fanout=None, batch=64, p=2.0, q=0.5, stop_prob=0.01, seed=0,
                n2v_ref_compat=1) -> AppParams:
     """Defaults are the reference's compile-time constants: 100-step walks (randomWalks.cu:4),
@@ -118,10 +138,10 @@ class Graph:
         return cls(h, device)
 
     def to_host(self):
-        row_ptr = np.empty(self.V + 1, np.int32)
-        col = np.empty(self.E, np.int32)
-        w = np.empty(self.E, np.float32)
-        mw = np.empty(self.V, np.float32)
+        row_ptr = _result_array(self.V + 1, np.int32, self.device)
+        col = _result_array(self.E, np.int32, self.device)
+        w = _result_array(self.E, np.float32, self.device)
+        mw = _result_array(self.V, np.float32, self.device)
         check(lib.nd_graph_to_host(self._h, _ptr(row_ptr), _ptr(col), _ptr(w), _ptr(mw)))
         return row_ptr, col, w, mw
 
@@ -190,7 +210,7 @@ class Sampler:
 
     def final_samples(self, out=None):
         if out is None:
-            out = np.empty(self.S * self.fs, np.int32)
+            out = _result_array(self.S * self.fs, np.int32, self.graph.device)
         check(lib.nd_sampler_final_samples(self._h, _ptr(out)))
         return out.reshape(self.S, self.fs)
 
@@ -238,8 +258,8 @@ class Sampler:
         adj_row = adj_col = prob = hop = None
         if collective:
             n = self.S * self.params.steps * max(L, B) * L
-            adj_row = np.empty(n, np.int32)
-            adj_col = np.empty(n, np.int32)
+            adj_row = _result_array(n, np.int32, self.graph.device)
+            adj_col = _result_array(n, np.int32, self.graph.device)
             prob = np.zeros(self.S * self.fs, np.float32)
         if self.params.app == APP_KHOP_DISTINCT:
             hop = np.zeros(self.S * self.params.steps, np.int32)

@@ -227,6 +227,7 @@ struct nd_sampler {
   // collective
   int32_t *d_adj_row = nullptr, *d_adj_col = nullptr;
   float *d_prob = nullptr;
+  uint32_t *d_adj_bits = nullptr;      // the adjacency on its way to the host (made at the first use)
   int32_t *d_cand = nullptr;
   float *d_cand_w = nullptr;
   int64_t cand_cap = 0;

@@ -104,3 +104,34 @@ def test_rows_packed_at_the_edges_of_a_chunk(nd, small_graph, S, stop):
         s.host_update_fetch()
         s.host_update_finish()
         assert np.array_equal(host.reshape(S, steps), dense) and np.array_equal(host_len, (dense != V).sum(axis=1))
+
+
+@pytest.mark.parametrize("app", [6, 8, 9])
+@pytest.mark.parametrize("L,B,S", [(48, 50, 70), (7, 5, 2675), (1, 3, 43_691), (64, 64, 33)])
+def test_adjacency_crosses_as_bits(nd, ndo, small_graph, app, L, B, S):
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    s = nd.Sampler(g, nd.app_params(app, steps=2, fanout=L, batch=B, seed=6), num_samples=S)
+    s.sample()
+    exp = ndo.sample(small_graph, ndo.make_params(app, steps=2, fanout=L, batch=B, seed=6), S)
+    if np.array_equal(s.final_samples(), exp["out"]) or app == 6:   # (importance: a draw on an edge may fall to its neighbour)
+        aux = s.aux()
+        assert np.array_equal(aux["adj_row"], exp["adj_row"]) and np.array_equal(aux["adj_col"], exp["adj_col"])
+
+
+def test_results_own_their_memory(nd, small_graph):
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    s = nd.Sampler(g, nd.app_params(0, steps=10, seed=2), num_samples=300_000)
+    s.sample()
+    exp = np.zeros(3_000_000, np.int32)
+    s.final_samples(exp)
+    kept = [s.final_samples() for _ in range(3)]
+    for a in kept:
+        a[:] = -5
+    row = kept[1][7]                     # a view holds the whole
+    del kept[1]
+    for _ in range(5):                   # new memory, then lent again, then pinned
+        assert np.array_equal(s.final_samples().reshape(-1), exp)
+    assert (row == -5).all() and (kept[0] == -5).all() and (kept[1] == -5).all()
+    last = s.final_samples()
+    del s, g
+    assert np.array_equal(last.reshape(-1), exp)   # results outlive the sampler
