@@ -410,9 +410,15 @@ class PipelinedSampler:
 
     def _finish(self, k):
         if k in self._pending:
-            self._fetch(k)                                # every chunk's vertices are on their way before the first rows are written
-            self._pending.pop(k)
-            self.values_copied = sum(smp.host_update_finish() for _, _, smp in self.sets[k])
+            fetched = self._pending.pop(k) == "fetched"
+            parts = [smp for _, _, smp in self.sets[k]]
+            total = 0
+            for i, smp in enumerate(parts):               # a chunk's rows are written while the next one's vertices cross
+                if not fetched:
+                    for ahead in parts[i + 1 if i else 0:i + 2]:
+                        ahead.host_update_fetch()
+                total += smp.host_update_finish()
+            self.values_copied = total
 
     def wait(self):
         for k in list(self._pending):

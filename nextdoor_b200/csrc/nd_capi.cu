@@ -330,6 +330,7 @@ int nd_sampler_final_samples_async(nd_sampler *s, int32_t *out, void *copy_strea
   if (s->S > 0) ND_CUDA(cudaMemcpyAsync(out, s->d_out, sizeof(int32_t) * (size_t)s->S * s->fs, cudaMemcpyDeviceToHost, cs));
   if (cs != s->stream) {
     if (!s->copy_done) ND_CUDA(cudaEventCreateWithFlags(&s->copy_done, cudaEventDisableTiming));
+    if (s->copy_pending) ND_CUDA(cudaStreamWaitEvent(cs, s->copy_done, 0));   // the event stands for all copies of the job
     ND_CUDA(cudaEventRecord(s->copy_done, cs));
     s->copy_pending = true;
   }

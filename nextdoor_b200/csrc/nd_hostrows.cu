@@ -26,6 +26,7 @@ struct NdHostRows {
   cudaEvent_t packed = nullptr, len_done = nullptr, vals_done = nullptr, total_done = nullptr;
   uint32_t *h_total = nullptr;  // pinned: number of packed vertices (nd_sampler_pack_rows)
   cudaStream_t cs = nullptr;
+  cudaStream_t vs = nullptr;    // the vertices': on the caller's copy stream they would wait for the lengths of all chunks begun since
   int32_t *out = nullptr, *row_len = nullptr;
   int64_t total = 0;
   uint32_t *h_chunk = nullptr;  // pinned: d_chunk of the job being copied
@@ -166,6 +167,7 @@ int hostrows_init(nd_sampler *s) {
   if (e == cudaSuccess) e = cudaMallocHost(&h->h_chunk, sizeof(uint32_t) * ((size_t)h->n_chunks + 1));
   if (e == cudaSuccess) e = cudaMallocHost(&h->h_total, sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMalloc(&h->d_chunk, sizeof(uint32_t) * ((size_t)h->n_chunks + 1));
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->vs, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->packed, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->len_done, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->vals_done, cudaEventDisableTiming);
@@ -202,6 +204,7 @@ void nd_hostrows_free(nd_sampler *s) {
   if (h->h_vals) cudaFreeHost(h->h_vals);
   if (h->h_chunk) cudaFreeHost(h->h_chunk);
   cudaFree(h->d_chunk);
+  if (h->vs) cudaStreamDestroy(h->vs);
   if (h->packed) cudaEventDestroy(h->packed);
   if (h->len_done) cudaEventDestroy(h->len_done);
   if (h->vals_done) cudaEventDestroy(h->vals_done);
@@ -246,6 +249,7 @@ int nd_sampler_host_update_begin(nd_sampler *s, int32_t *out, int32_t *row_len, 
   ND_CUDA(cudaEventRecord(h->len_done, h->cs));
   if (h->cs != s->stream) {  // the next sampling of this sampler waits for the copies that read its buffers
     if (!s->copy_done) ND_CUDA(cudaEventCreateWithFlags(&s->copy_done, cudaEventDisableTiming));
+    if (s->copy_pending) ND_CUDA(cudaStreamWaitEvent(h->cs, s->copy_done, 0));
     ND_CUDA(cudaEventRecord(s->copy_done, h->cs));
     s->copy_pending = true;
   }
@@ -265,7 +269,7 @@ int nd_sampler_host_update_fetch(nd_sampler *s) {
   if (packable(s)) h->total = (int64_t)h->h_chunk[h->n_chunks];
   h->dense = 2 * h->total > s->S * (int64_t)s->fs || !packable(s);
   if (h->dense) {
-    ND_CUDA(cudaMemcpyAsync(h->out, s->d_out, sizeof(int32_t) * (size_t)s->S * s->fs, cudaMemcpyDeviceToHost, h->cs));
+    ND_CUDA(cudaMemcpyAsync(h->out, s->d_out, sizeof(int32_t) * (size_t)s->S * s->fs, cudaMemcpyDeviceToHost, h->vs));
   } else if (h->total > 0) {
     if ((size_t)h->total > h->vals_cap) {
       if (h->h_vals) ND_CUDA(cudaFreeHost(h->h_vals));
@@ -273,13 +277,13 @@ int nd_sampler_host_update_fetch(nd_sampler *s) {
       h->vals_cap = (size_t)h->total + (size_t)h->total / 4 + 4096;
       ND_CUDA(cudaMallocHost(&h->h_vals, sizeof(int32_t) * h->vals_cap));
     }
-    ND_CUDA(cudaMemcpyAsync(h->h_vals, s->d_tmp, sizeof(int32_t) * (size_t)h->total, cudaMemcpyDeviceToHost, h->cs));
+    ND_CUDA(cudaMemcpyAsync(h->h_vals, s->d_tmp, sizeof(int32_t) * (size_t)h->total, cudaMemcpyDeviceToHost, h->vs));
   }
-  ND_CUDA(cudaEventRecord(h->vals_done, h->cs));
-  if (h->cs != s->stream) {
-    ND_CUDA(cudaEventRecord(s->copy_done, h->cs));
-    s->copy_pending = true;
-  }
+  ND_CUDA(cudaEventRecord(h->vals_done, h->vs));
+  if (!s->copy_done) ND_CUDA(cudaEventCreateWithFlags(&s->copy_done, cudaEventDisableTiming));
+  if (s->copy_pending) ND_CUDA(cudaStreamWaitEvent(h->vs, s->copy_done, 0));   // the event stands for all copies of the job
+  ND_CUDA(cudaEventRecord(s->copy_done, h->vs));
+  s->copy_pending = true;
   h->stage = 2;
   return ND_OK;
 }
