@@ -208,11 +208,13 @@ radix_scatter_staged_kernel(NdSortArrays arr, int key_word, const int32_t *__res
     for (int i = threadIdx.x; i < WARPS * bins; i += THREADS) cnt[i] = 0;
     __syncthreads();
     const int wbase = tile * TILE + warp * (32 * IPT);
-    uint32_t k[IPT], rank[IPT], dig[IPT];
+    uint32_t k[IPT], rank[IPT], dig[IPT], word[NW][IPT];   // all words of the tile are asked for at once
 #pragma unroll
     for (int r = 0; r < IPT; r++) {
       const int i = wbase + r * 32 + lane;
       bool live = i < n;
+#pragma unroll
+      for (int w = 0; w < NW; w++) word[w][r] = live && w != key_word ? __ldcs(arr.a[w] + i) : 0u;
       if (live) {
         k[r] = keys[i];
         if (drop && k[r] == drop_key) live = false;
@@ -267,10 +269,9 @@ radix_scatter_staged_kernel(NdSortArrays arr, int key_word, const int32_t *__res
 #pragma unroll
     for (int r = 0; r < IPT; r++) {
       if (dig[r] != 0xffffffffu) {
-        const int i = wbase + r * 32 + lane;
         const uint32_t lp = lstart[dig[r]] + my[dig[r]] + rank[r];
 #pragma unroll
-        for (int w = 0; w < NW; w++) stage[w * TILE + lp] = (w == key_word) ? k[r] : arr.a[w][i];
+        for (int w = 0; w < NW; w++) stage[w * TILE + lp] = (w == key_word) ? k[r] : word[w][r];
       }
     }
     __syncthreads();
