@@ -137,15 +137,26 @@ coll_ref_kernel(NdGraphView g, CollParams cp, RefLayout lay, int steps, int64_t 
       }
       // the entries of the short lists; a thread's loads are independent
       constexpr int LOADS = 4;
-      for (uint32_t f0 = (uint32_t)tid; f0 < carry; f0 += CTHREADS * LOADS) {
+      for (uint32_t c0 = (uint32_t)warp * (32 * LOADS); c0 < carry; c0 += CTHREADS * LOADS) {
         int32_t v[LOADS];
         int at[LOADS];
+        // transits of the warp's first and last entry: last with pre <= f
+        const uint32_t c1 = min(c0 + 32 * LOADS, carry) - 1;
+        int from = 0, to = nt - 1;
+        for (int hi = to; from < hi;) {
+          const int mid = (from + hi + 1) >> 1;
+          if (pre[mid] <= c0) from = mid; else hi = mid - 1;
+        }
+        for (int lo = from; lo < to;) {
+          const int mid = (lo + to + 1) >> 1;
+          if (pre[mid] <= c1) lo = mid; else to = mid - 1;
+        }
 #pragma unroll
         for (int j = 0; j < LOADS; j++) {
-          const uint32_t f = f0 + (uint32_t)(j * CTHREADS);
+          const uint32_t f = c0 + (uint32_t)(j * 32 + lane);
           v[j] = -1; at[j] = 0;
           if (f < carry) {
-            int lo = 0, hi = nt - 1;   // last transit with pre <= f
+            int lo = from, hi = to;
             while (lo < hi) {
               const int mid = (lo + hi + 1) >> 1;
               if (pre[mid] <= f) lo = mid; else hi = mid - 1;
