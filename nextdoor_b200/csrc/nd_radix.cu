@@ -10,7 +10,10 @@
 // round trip; pairs carrying the drop key (dead walks) vanish in the first pass and the
 // surviving count is written next to the data.  The first hist can be fused into the kernel
 // that produces the keys (the next() kernels do that).
+#include <utility>
+
 #include "nd_common.cuh"
+
 
 namespace {
 
@@ -18,6 +21,21 @@ constexpr int THREADS = ND_RADIX_THREADS;
 constexpr int WARPS = THREADS / 32;
 constexpr int IPT = 8;                 // items per thread
 constexpr int TILE = THREADS * IPT;    // 2048 pairs per tile
+
+// CTAs of the scatter kernels per SM, by registers: left alone the compiler takes 122 and two CTAs fit (8.4M records of
+// three words, a pass: 140 us; three 101, four 88, six, with spills, 86)
+constexpr int SCATTER_CTAS = 4;
+
+// lanes with the same digit; a vote per bit (__match_any_sync takes longer: 88 -> 76 us a pass)
+__device__ __forceinline__ uint32_t peers_of(uint32_t digit, bool in, uint32_t mask) {
+  const uint32_t some = __ballot_sync(0xffffffffu, in);
+  uint32_t peers = in ? some : ~some;
+  for (uint32_t b = 1; b <= mask; b <<= 1) {
+    const uint32_t v = __ballot_sync(0xffffffffu, digit & b);
+    peers &= (digit & b) ? v : ~v;
+  }
+  return peers;
+}
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
   const int lane = threadIdx.x & 31;
@@ -109,8 +127,8 @@ radix_scan_kernel(const int32_t *__restrict__ d_n, int bins, uint32_t *__restric
 }
 
 template <int NW>
-__global__ void __launch_bounds__(THREADS)
-radix_scatter_kernel(NdSortArrays arr, int key_word, const int32_t *__restrict__ d_n, int shift, int bins,
+__global__ void __launch_bounds__(THREADS, SCATTER_CTAS)
+radix_scatter_kernel(const __grid_constant__ NdSortArrays arr, const int32_t *__restrict__ d_n, int shift, int bins,
                      bool drop, uint32_t drop_key, const uint32_t *__restrict__ tile_hist,
                      int64_t max_tiles, uint32_t *__restrict__ ghist_to_clear) {
   extern __shared__ uint32_t cnt[];  // [WARPS][bins]
@@ -120,29 +138,27 @@ radix_scatter_kernel(NdSortArrays arr, int key_word, const int32_t *__restrict__
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lt = (1u << lane) - 1u;
   uint32_t *my = cnt + warp * bins;
-  const uint32_t *__restrict__ keys = arr.a[key_word];
+  const uint32_t *__restrict__ keys = arr.a[0];
 
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     for (int i = threadIdx.x; i < WARPS * bins; i += THREADS) cnt[i] = 0;
     __syncthreads();
     const int wbase = tile * TILE + warp * (32 * IPT);
-    uint32_t k[IPT];
-    uint32_t rank[IPT];
-    uint32_t dig[IPT];
+    uint32_t k[IPT], rank[IPT];
+    uint32_t alive = 0;   // which of the lane's items there are
+    auto digit = [&](int r) { return (alive >> r) & 1u ? (k[r] >> shift) & mask : 0xffffffffu; };
 #pragma unroll
     for (int r = 0; r < IPT; r++) {
       const int i = wbase + r * 32 + lane;
       bool live = i < n;
-      if (live) {
-        k[r] = keys[i];
-        if (drop && k[r] == drop_key) live = false;
-      }
-      dig[r] = live ? ((k[r] >> shift) & mask) : 0xffffffffu;
+      k[r] = live ? keys[i] : 0u;
+      if (drop && k[r] == drop_key) live = false;
+      alive |= (live ? 1u : 0u) << r;
     }
 #pragma unroll
     for (int r = 0; r < IPT; r++) {
-      const uint32_t d = dig[r];
-      const uint32_t peers = __match_any_sync(0xffffffffu, d);
+      const uint32_t d = digit(r);
+      const uint32_t peers = peers_of(d, (alive >> r) & 1u, mask);
       const int leader = __ffs(peers) - 1;
       uint32_t old = 0;
       if (d != 0xffffffffu && lane == leader) {
@@ -167,11 +183,13 @@ radix_scatter_kernel(NdSortArrays arr, int key_word, const int32_t *__restrict__
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < IPT; r++) {
-      if (dig[r] != 0xffffffffu) {
+      const uint32_t d = digit(r);
+      if (d != 0xffffffffu) {
         const int i = wbase + r * 32 + lane;
-        const uint32_t pos = my[dig[r]] + rank[r];
+        const uint32_t pos = my[d] + rank[r];
+        arr.b[0][pos] = k[r];
 #pragma unroll
-        for (int w = 0; w < NW; w++) arr.b[w][pos] = (w == key_word) ? k[r] : arr.a[w][i];
+        for (int w = 1; w < NW; w++) arr.b[w][pos] = arr.a[w][i];
       }
     }
     __syncthreads();
@@ -186,8 +204,8 @@ radix_scatter_kernel(NdSortArrays arr, int key_word, const int32_t *__restrict__
 // radix_scatter_kernel.  Shared memory: [WARPS][bins] counters, [bins] tile-local starts, [bins]
 // global starts, [NW][TILE] staged words.
 template <int NW>
-__global__ void __launch_bounds__(THREADS)
-radix_scatter_staged_kernel(NdSortArrays arr, int key_word, const int32_t *__restrict__ d_n, int shift, int bins,
+__global__ void __launch_bounds__(THREADS, SCATTER_CTAS)
+radix_scatter_staged_kernel(const __grid_constant__ NdSortArrays arr, const int32_t *__restrict__ d_n, int shift, int bins,
                             bool drop, uint32_t drop_key, const uint32_t *__restrict__ tile_hist,
                             int64_t max_tiles, uint32_t *__restrict__ ghist_to_clear) {
   extern __shared__ uint32_t sm[];
@@ -202,29 +220,29 @@ radix_scatter_staged_kernel(NdSortArrays arr, int key_word, const int32_t *__res
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lt = (1u << lane) - 1u;
   uint32_t *my = cnt + warp * bins;
-  const uint32_t *__restrict__ keys = arr.a[key_word];
+  const uint32_t *__restrict__ keys = arr.a[0];
 
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     for (int i = threadIdx.x; i < WARPS * bins; i += THREADS) cnt[i] = 0;
     __syncthreads();
     const int wbase = tile * TILE + warp * (32 * IPT);
-    uint32_t k[IPT], rank[IPT], dig[IPT], word[NW][IPT];   // all words of the tile are asked for at once
+    uint32_t k[IPT], rank[IPT], word[NW][IPT];   // all words of the tile are asked for at once
+    uint32_t alive = 0;                          // which of the lane's items there are
+    auto digit = [&](int r) { return (alive >> r) & 1u ? (k[r] >> shift) & mask : 0xffffffffu; };
 #pragma unroll
     for (int r = 0; r < IPT; r++) {
       const int i = wbase + r * 32 + lane;
       bool live = i < n;
+      k[r] = live ? keys[i] : 0u;
 #pragma unroll
-      for (int w = 0; w < NW; w++) word[w][r] = live && w != key_word ? __ldcs(arr.a[w] + i) : 0u;
-      if (live) {
-        k[r] = keys[i];
-        if (drop && k[r] == drop_key) live = false;
-      }
-      dig[r] = live ? ((k[r] >> shift) & mask) : 0xffffffffu;
+      for (int w = 1; w < NW; w++) word[w][r] = live ? __ldcs(arr.a[w] + i) : 0u;
+      if (drop && k[r] == drop_key) live = false;
+      alive |= (live ? 1u : 0u) << r;
     }
 #pragma unroll
     for (int r = 0; r < IPT; r++) {
-      const uint32_t d = dig[r];
-      const uint32_t peers = __match_any_sync(0xffffffffu, d);
+      const uint32_t d = digit(r);
+      const uint32_t peers = peers_of(d, (alive >> r) & 1u, mask);
       const int leader = __ffs(peers) - 1;
       uint32_t old = 0;
       if (d != 0xffffffffu && lane == leader) {
@@ -268,15 +286,17 @@ radix_scatter_staged_kernel(NdSortArrays arr, int key_word, const int32_t *__res
     const uint32_t n_live = carry;
 #pragma unroll
     for (int r = 0; r < IPT; r++) {
-      if (dig[r] != 0xffffffffu) {
-        const uint32_t lp = lstart[dig[r]] + my[dig[r]] + rank[r];
+      const uint32_t d = digit(r);
+      if (d != 0xffffffffu) {
+        const uint32_t lp = lstart[d] + my[d] + rank[r];
+        stage[lp] = k[r];
 #pragma unroll
-        for (int w = 0; w < NW; w++) stage[w * TILE + lp] = (w == key_word) ? k[r] : word[w][r];
+        for (int w = 1; w < NW; w++) stage[w * TILE + lp] = word[w][r];
       }
     }
     __syncthreads();
     for (uint32_t j = threadIdx.x; j < n_live; j += THREADS) {
-      const uint32_t key = stage[key_word * TILE + j];
+      const uint32_t key = stage[j];
       const uint32_t d = (key >> shift) & mask;
       const uint32_t pos = gbase[d] + (j - lstart[d]);
 #pragma unroll
@@ -368,14 +388,16 @@ int nd_radix_sort(const NdDeviceInfo &dev, cudaStream_t st, NdRadixScratch *scr,
       radix_hist_kernel<<<grid, THREADS, 2 * bins * sizeof(uint32_t), st>>>(
           cur.a[key_word], n_ptr, pl.shift[p], bins, drop, drop_key, scr->tile_hist, pl.max_tiles, gh);
     }
+    std::swap(cur.a[0], cur.a[key_word]);   // the scatter kernels take the key first
+    std::swap(cur.b[0], cur.b[key_word]);
     radix_scan_kernel<<<bins, THREADS, 0, st>>>(n_ptr, bins, scr->tile_hist, pl.max_tiles, gh,
                                                   p == 0 ? d_n_out : nullptr);
     if (bins <= 256 && pl.max_n > ((int64_t)4 << 20)) {  // large maps: coalesced stores through a staged tile
       const size_t sms = sizeof(uint32_t) * ((size_t)WARPS * bins + 2 * (size_t)bins + (size_t)arr.nwords * TILE);
       switch (arr.nwords) {
-        case 1: radix_scatter_staged_kernel<1><<<grid, THREADS, sms, st>>>(cur, key_word, n_ptr, pl.shift[p], bins, drop, drop_key, scr->tile_hist, pl.max_tiles, gh); break;
-        case 2: radix_scatter_staged_kernel<2><<<grid, THREADS, sms, st>>>(cur, key_word, n_ptr, pl.shift[p], bins, drop, drop_key, scr->tile_hist, pl.max_tiles, gh); break;
-        default: radix_scatter_staged_kernel<3><<<grid, THREADS, sms, st>>>(cur, key_word, n_ptr, pl.shift[p], bins, drop, drop_key, scr->tile_hist, pl.max_tiles, gh); break;
+        case 1: radix_scatter_staged_kernel<1><<<(unsigned)tiles, THREADS, sms, st>>>(cur, n_ptr, pl.shift[p], bins, drop, drop_key, scr->tile_hist, pl.max_tiles, gh); break;
+        case 2: radix_scatter_staged_kernel<2><<<(unsigned)tiles, THREADS, sms, st>>>(cur, n_ptr, pl.shift[p], bins, drop, drop_key, scr->tile_hist, pl.max_tiles, gh); break;
+        default: radix_scatter_staged_kernel<3><<<(unsigned)tiles, THREADS, sms, st>>>(cur, n_ptr, pl.shift[p], bins, drop, drop_key, scr->tile_hist, pl.max_tiles, gh); break;
       }
       in_b = !in_b;
       nd_count_launches((p == 0 && first_hist_done) ? 2 : 3);
@@ -383,9 +405,9 @@ int nd_radix_sort(const NdDeviceInfo &dev, cudaStream_t st, NdRadixScratch *scr,
     }
     const size_t sm = (size_t)WARPS * bins * sizeof(uint32_t);
     switch (arr.nwords) {
-      case 1: radix_scatter_kernel<1><<<grid, THREADS, sm, st>>>(cur, key_word, n_ptr, pl.shift[p], bins, drop, drop_key, scr->tile_hist, pl.max_tiles, gh); break;
-      case 2: radix_scatter_kernel<2><<<grid, THREADS, sm, st>>>(cur, key_word, n_ptr, pl.shift[p], bins, drop, drop_key, scr->tile_hist, pl.max_tiles, gh); break;
-      default: radix_scatter_kernel<3><<<grid, THREADS, sm, st>>>(cur, key_word, n_ptr, pl.shift[p], bins, drop, drop_key, scr->tile_hist, pl.max_tiles, gh); break;
+      case 1: radix_scatter_kernel<1><<<grid, THREADS, sm, st>>>(cur, n_ptr, pl.shift[p], bins, drop, drop_key, scr->tile_hist, pl.max_tiles, gh); break;
+      case 2: radix_scatter_kernel<2><<<grid, THREADS, sm, st>>>(cur, n_ptr, pl.shift[p], bins, drop, drop_key, scr->tile_hist, pl.max_tiles, gh); break;
+      default: radix_scatter_kernel<3><<<grid, THREADS, sm, st>>>(cur, n_ptr, pl.shift[p], bins, drop, drop_key, scr->tile_hist, pl.max_tiles, gh); break;
     }
     in_b = !in_b;
     nd_count_launches((p == 0 && first_hist_done) ? 2 : 3);
