@@ -93,7 +93,7 @@ khop_rows_kernel(const __grid_constant__ KhopRows a) {
   int64_t s = (int64_t)blockIdx.x * warps + warp, s_end = s + 1;
   while (s < a.S) {
     {
-      int n_prev = 1, prefix_prev = 0, prefix = 0, n_last = 0;
+      int n_prev = 1, prefix_prev = 0, prefix = 0, n_last = 0, empty_from = a.steps;
       const uint32_t gs = (uint32_t)(a.first_sample + s);
       for (int k = 0; k < a.steps; k++) {
         const int f = a.fan[k], n = n_prev * f;
@@ -111,6 +111,12 @@ khop_rows_kernel(const __grid_constant__ KhopRows a) {
           }
           n_live += __popc(m);
           pairs += valid ? 1u : 0u;
+        }
+        // no hop has vertices from here on (half of the seeds of an R-MAT graph): the rest of the row is empty
+        if (n_live == 0) {
+          for (int i = prefix + lane; i < a.fs; i += 32) row[i] = a.V;
+          empty_from = k;
+          break;
         }
         // the last hop of a row whose hops are sorted anyway is gathered without its empty slots
         const bool dense = DISTINCT && k == a.steps - 1 && n <= SORT_MAX;
@@ -152,7 +158,11 @@ khop_rows_kernel(const __grid_constant__ KhopRows a) {
         __syncwarp();
         // phase two: the neighbours
         const int slots = dense ? m : n;
-        for (int c0 = lane; c0 < slots; c0 += 32 * GATHERS) {
+        if (slots <= 32) {   // (the unrolled loop costs its eight turns whatever the hop's length)
+          const int32_t e = lane < slots ? row[prefix + lane] : -1;
+          if (lane < slots) row[prefix + lane] = e >= 0 ? __ldg(a.col + e) : a.V;
+          edges += e >= 0 ? 1u : 0u;
+        } else for (int c0 = lane; c0 < slots; c0 += 32 * GATHERS) {
           int32_t v[GATHERS];
 #pragma unroll
           for (int j = 0; j < GATHERS; j++) {
@@ -176,7 +186,9 @@ khop_rows_kernel(const __grid_constant__ KhopRows a) {
         for (int k = 0; k < a.steps; k++) {
           n *= a.fan[k];
           int32_t *seg = row + off;
-          if (n <= SORT_MAX) {
+          if (k >= empty_from) {
+            if (n <= SORT_MAX && lane == 0) a.hop_counts[s * a.steps + k] = 0;
+          } else if (n <= SORT_MAX) {
             int m = k == a.steps - 1 ? n_last : 0;   // the vertices to the front, so that the network is no longer than they are
             if (m == 0 && k == a.steps - 1) for (int i = lane; i < n; i += 32) seg[i] = a.V;
             for (int i0 = 0; k < a.steps - 1 && i0 < n; i0 += 32) {
