@@ -7,10 +7,10 @@
 // integer weights sum exactly).
 //
 // What bounds it, and what is done about it (2^20 vertices, 1024 batches of 64, 2 layers of 64: FastGCN
-// 4.8 -> 1.13 ms, LADIES 5.7 -> 2.44 ms):
+// 4.8 -> 0.98 ms, LADIES 5.7 -> 2.44 ms):
 //  * The second layer's transits are hubs (FastGCN draws them with the square of their degree), many of them the
 //    same one: repeated transits of a batch are taken once (LADIES with their multiplicity).
-//  * A hub's list (up to 140 K ids) costs a shared-memory test per id.  Vertices with at least V/64 neighbours
+//  * A hub's list (up to 140 K ids) costs a shared-memory test per id.  Vertices with at least V/128 neighbours
 //    have their neighbourhood as a bitmap, built once per graph: V/8 bytes that are ORed in registers, word by
 //    word, and stored to the union once; and an adjacency probe of such a transit is a bit test.
 //  * FastGCN's weights are summed without a list of candidates (writing that and fetching deg^2 one by one took more
@@ -36,6 +36,7 @@ constexpr int GROUP_WORDS = 16;   // words whose candidates are counted together
 constexpr int GROUP = 512;        // candidates (FastGCN: vertices, GROUP_WORDS words) whose weights are summed together
 constexpr int BIG_DEGREE = 2048;  // from here a vertex is on the list of big ones and its code is 0: 512 * 2047^2 < 2^31
 constexpr int FLIGHT = 4;         // groups a warp sums at a time
+constexpr int HUB = 128, LADIES_HUB = 64;   // a vertex with at least V / HUB neighbours has a bitmap of them, and is ORed from V / LADIES_HUB on
 constexpr int BIG_LIST = 4096;    // lists at least this long are streamed by the whole CTA
 constexpr int VEC = 4;            // 16-byte loads in flight per thread
 constexpr int CHUNK = 128;        // list entries a warp takes at a time (LADIES)
@@ -241,7 +242,8 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
         const int32_t rs = __ldg(a.g.row_ptr + t), deg = __ldg(a.g.row_ptr + t + 1) - rs, slot = __ldg(a.hub_slot + t);
         ids += (unsigned long long)deg;
         if (sh_mult[i] > 0) {
-          ut[slot >= 0 ? atomicAdd(&sh_hubs, 1) : cp.ntr - 1 - atomicAdd(&sh_rest, 1)] = Transit{rs, deg, sh_mult[i], slot};
+          // (LADIES goes through the lists again, so that a hub's bitmap saves it less)
+          ut[slot >= 0 && (!LADIES || deg >= cp.V / LADIES_HUB) ? atomicAdd(&sh_hubs, 1) : cp.ntr - 1 - atomicAdd(&sh_rest, 1)] = Transit{rs, deg, sh_mult[i], slot};
         }
       }
       for (int o = 16; o > 0; o >>= 1) ids += __shfl_xor_sync(0xffffffffu, ids, o);
@@ -592,8 +594,10 @@ __global__ void hub_bits_kernel(const int32_t *__restrict__ row_ptr, const int32
 
 int words_of(int32_t V) { return (int)((((int64_t)V + 31) / 32 + GROUP_WORDS - 1) / GROUP_WORDS * GROUP_WORDS); }
 
-// A bitmap pays against the list it replaces from about V/64 neighbours: twice the list's bytes, but ORed a word at a
-// time.  At most HUBS of them (a graph can hold 64 E / V such vertices).
+// A bitmap pays against the list it replaces from about V/128 neighbours: four times the list's bytes, but ORed a word
+// at a time (FastGCN from V/64, V/128, V/192: 1.14, 0.98, 0.99 ms with 1024 batches on 2^20 vertices, 0.83, 0.59, 0.59 with 256 on
+// 2^21).
+// At most HUBS of them (a graph can hold 128 E / V such vertices).
 constexpr int HUBS = 1024;
 std::mutex g_layers_mutex;
 
@@ -605,7 +609,7 @@ int ensure_layers(const nd_graph *g, int sms, bool ladies) {
     ND_CUDA(cudaMalloc(&slot, sizeof(int32_t) * (size_t)g->V));
     ND_CUDA(cudaMalloc(&hubs, sizeof(int32_t) * (HUBS + 1)));
     ND_CUDA(cudaMemset(hubs + HUBS, 0, sizeof(int32_t)));
-    const int32_t least = std::max<int32_t>(g->V / 64, 256);
+    const int32_t least = std::max<int32_t>(g->V / HUB, 256);
     hub_slots_kernel<<<grid, 256>>>(g->row_ptr, g->V, least, HUBS, slot, hubs, hubs + HUBS);
     int32_t n = 0;
     ND_CUDA(cudaMemcpy(&n, hubs + HUBS, sizeof(n), cudaMemcpyDeviceToHost));
