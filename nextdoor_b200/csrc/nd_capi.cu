@@ -237,7 +237,7 @@ int nd_sampler_create(const nd_graph *g, const nd_app_params *p, int64_t num_sam
   const size_t S1 = (size_t)(num_samples > 0 ? num_samples : 1);
   auto fail = [&](int code) { free_sampler(s); return code; };
 #define ND_TRY_S(call) do { int c__ = (call); if (c__ != ND_OK) return fail(c__); } while (0)
-#define ND_CUDA_S(call) do { cudaError_t e__ = (call); if (e__ != cudaSuccess) { nd_set_error("%s failed: %s", #call, cudaGetErrorString(e__)); return fail(ND_ERR_CUDA); } } while (0)
+#define ND_CUDA_S(call) do { cudaError_t e__ = (call); if (e__ != cudaSuccess) { cudaGetLastError(); nd_set_error("%s failed: %s", #call, cudaGetErrorString(e__)); return fail(ND_ERR_CUDA); } } while (0)
   ND_CUDA_S(cudaMalloc(&s->d_initial, sizeof(int32_t) * S1 * s->isz));
   ND_CUDA_S(cudaMalloc(&s->d_out, sizeof(int32_t) * S1 * s->fs));
   ND_CUDA_S(cudaMalloc(&s->d_stats, sizeof(unsigned long long) * 8));
@@ -521,7 +521,7 @@ int nd_inverter_create(int device, int64_t max_pairs, int32_t invalid, nd_invert
   inv->invalid = invalid;
   int rc = nd_device_info(device, &inv->dev);
   if (rc == ND_OK) rc = nd_radix_scratch_alloc(&inv->scr, nd_bit_length((uint32_t)(invalid > 1 ? invalid - 1 : 1)), max_pairs);
-  if (rc == ND_OK && cudaMalloc(&inv->d_n, 2 * sizeof(int32_t)) != cudaSuccess) { nd_set_error("nd_inverter_create: cudaMalloc failed"); rc = ND_ERR_CUDA; }
+  if (rc == ND_OK && cudaMalloc(&inv->d_n, 2 * sizeof(int32_t)) != cudaSuccess) { cudaGetLastError(); nd_set_error("nd_inverter_create: cudaMalloc failed"); rc = ND_ERR_CUDA; }
   if (rc != ND_OK) { nd_radix_scratch_free(&inv->scr); cudaFree(inv->d_n); delete inv; return rc; }
   *out = inv;
   return ND_OK;

@@ -16,10 +16,12 @@
 void nd_set_error(const char *fmt, ...);
 void nd_count_launches(int n);  // bookkeeping behind nd_launch_count()
 
+// (a failed call also stays behind as the thread's last error, where the next call's check of its launches would find it)
 #define ND_CUDA(call)                                                                      \
   do {                                                                                     \
     cudaError_t e__ = (call);                                                              \
     if (e__ != cudaSuccess) {                                                              \
+      cudaGetLastError();                                                                  \
       nd_set_error("%s failed: %s (%s:%d)", #call, cudaGetErrorString(e__), __FILE__, __LINE__); \
       return ND_ERR_CUDA;                                                                  \
     }                                                                                      \
