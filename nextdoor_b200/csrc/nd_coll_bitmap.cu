@@ -601,61 +601,76 @@ int words_of(int32_t V) { return (int)((((int64_t)V + 31) / 32 + GROUP_WORDS - 1
 constexpr int HUBS = 1024;
 std::mutex g_layers_mutex;
 
+// bitmaps of the hubs' neighbourhoods
+int ensure_hubs(const nd_graph *g, int grid) {
+  if (g->hub_slot) return ND_OK;
+  NdDevMem<int32_t> slot, hubs;
+  NdDevMem<uint32_t> bits;
+  ND_TRY(slot.alloc((size_t)g->V));
+  ND_TRY(hubs.alloc(HUBS + 1));
+  ND_CUDA(cudaMemset(hubs.p + HUBS, 0, sizeof(int32_t)));
+  const int32_t least = std::max<int32_t>(g->V / HUB, 256);
+  hub_slots_kernel<<<grid, 256>>>(g->row_ptr, g->V, least, HUBS, slot.p, hubs.p, hubs.p + HUBS);
+  int32_t n = 0;
+  ND_CUDA(cudaMemcpy(&n, hubs.p + HUBS, sizeof(n), cudaMemcpyDeviceToHost));
+  n = std::min(n, HUBS);
+  const size_t words = (size_t)words_of(g->V) * (size_t)std::max(n, 1);
+  ND_TRY(bits.alloc(words));
+  ND_CUDA(cudaMemset(bits.p, 0, sizeof(uint32_t) * words));
+  if (n > 0) hub_bits_kernel<<<dim3((unsigned)n, 8), 256>>>(g->row_ptr, g->col, hubs.p, words_of(g->V), bits.p);
+  ND_CUDA(cudaDeviceSynchronize());
+  g->hub_bits = bits.release();
+  g->hub_slot = slot.release();
+  return ND_OK;
+}
+
+// FastGCN: the packed degrees and the list of big vertices
+int ensure_degrees(const nd_graph *g, int grid) {
+  if (g->deg_codes) return ND_OK;
+  const int64_t units = 4 * (int64_t)words_of(g->V);
+  const int cap = (int)(g->E / BIG_DEGREE) + 1;
+  NdDevMem<uint4> deg;
+  NdDevMem<NdBigVertex> big;
+  NdDevMem<int32_t> count;
+  int32_t n = 0;
+  ND_TRY(deg.alloc((size_t)std::max<int64_t>(units, 1)));
+  ND_TRY(big.alloc((size_t)cap));
+  ND_TRY(count.alloc(1));
+  ND_CUDA(cudaMemset(count.p, 0, sizeof(int32_t)));
+  deg_build_kernel<<<grid, 256>>>(g->row_ptr, g->V, units, deg.p, big.p, count.p, cap);
+  ND_CUDA(cudaMemcpy(&n, count.p, sizeof(n), cudaMemcpyDeviceToHost));
+  std::vector<NdBigVertex> list((size_t)n);
+  ND_CUDA(cudaMemcpy(list.data(), big.p, sizeof(NdBigVertex) * (size_t)n, cudaMemcpyDeviceToHost));
+  std::sort(list.begin(), list.end(), [](const NdBigVertex &x, const NdBigVertex &y) { return x.v < y.v; });
+  ND_CUDA(cudaMemcpy(big.p, list.data(), sizeof(NdBigVertex) * (size_t)n, cudaMemcpyHostToDevice));
+  g->n_big = n;
+  g->big = big.release();
+  g->deg_codes = deg.release();
+  return ND_OK;
+}
+
+// LADIES: the terms of the entries
+int ensure_terms(const nd_graph *g, int grid) {
+  if (g->term) return ND_OK;
+  NdDevMem<float> term;
+  NdDevMem<double> sum;
+  ND_TRY(term.alloc((size_t)(g->E > 0 ? g->E : 1)));
+  ND_TRY(sum.alloc((size_t)g->V));
+  ND_CUDA(cudaMemset(sum.p, 0, sizeof(double) * (size_t)g->V));
+  rowsum_build_kernel<<<grid, BUILD_THREADS>>>(g->row_ptr, g->w, g->V, g->E, sum.p);
+  term_build_kernel<<<grid, BUILD_THREADS>>>(g->row_ptr, g->w, sum.p, g->V, g->E, term.p);
+  ND_CUDA(cudaDeviceSynchronize());
+  g->term = term.release();
+  return ND_OK;
+}
+
+// What a graph's first sampler builds goes to the graph when all of it is there: a build that runs out of memory
+// leaves nothing behind.
 int ensure_layers(const nd_graph *g, int sms, bool ladies) {
   std::lock_guard<std::mutex> lock(g_layers_mutex);
   const int grid = sms * 16;
-  if (!g->hub_slot) {
-    int32_t *slot = nullptr, *hubs = nullptr;
-    ND_CUDA(cudaMalloc(&slot, sizeof(int32_t) * (size_t)g->V));
-    ND_CUDA(cudaMalloc(&hubs, sizeof(int32_t) * (HUBS + 1)));
-    ND_CUDA(cudaMemset(hubs + HUBS, 0, sizeof(int32_t)));
-    const int32_t least = std::max<int32_t>(g->V / HUB, 256);
-    hub_slots_kernel<<<grid, 256>>>(g->row_ptr, g->V, least, HUBS, slot, hubs, hubs + HUBS);
-    int32_t n = 0;
-    ND_CUDA(cudaMemcpy(&n, hubs + HUBS, sizeof(n), cudaMemcpyDeviceToHost));
-    n = std::min(n, HUBS);
-    const size_t words = (size_t)words_of(g->V) * (size_t)std::max(n, 1);
-    ND_CUDA(cudaMalloc(&g->hub_bits, sizeof(uint32_t) * words));
-    ND_CUDA(cudaMemset(g->hub_bits, 0, sizeof(uint32_t) * words));
-    if (n > 0) hub_bits_kernel<<<dim3((unsigned)n, 8), 256>>>(g->row_ptr, g->col, hubs, words_of(g->V), g->hub_bits);
-    ND_CUDA(cudaDeviceSynchronize());
-    cudaFree(hubs);
-    g->hub_slot = slot;
-  }
-  if (!ladies && !g->deg_codes) {
-    uint4 *deg = nullptr;
-    const int64_t units = 4 * (int64_t)words_of(g->V);
-    const int cap = (int)(g->E / BIG_DEGREE) + 1;
-    int32_t *count = nullptr, n = 0;
-    ND_CUDA(cudaMalloc(&deg, sizeof(uint4) * (size_t)std::max<int64_t>(units, 1)));
-    if (!g->big) ND_CUDA(cudaMalloc(&g->big, sizeof(NdBigVertex) * (size_t)cap));
-    ND_CUDA(cudaMalloc(&count, sizeof(int32_t)));
-    ND_CUDA(cudaMemset(count, 0, sizeof(int32_t)));
-    deg_build_kernel<<<grid, 256>>>(g->row_ptr, g->V, units, deg, g->big, count, cap);
-    ND_CUDA(cudaMemcpy(&n, count, sizeof(n), cudaMemcpyDeviceToHost));
-    cudaFree(count);
-    std::vector<NdBigVertex> big((size_t)n);
-    ND_CUDA(cudaMemcpy(big.data(), g->big, sizeof(NdBigVertex) * (size_t)n, cudaMemcpyDeviceToHost));
-    std::sort(big.begin(), big.end(), [](const NdBigVertex &x, const NdBigVertex &y) { return x.v < y.v; });
-    ND_CUDA(cudaMemcpy(g->big, big.data(), sizeof(NdBigVertex) * (size_t)n, cudaMemcpyHostToDevice));
-    g->n_big = n;
-    g->deg_codes = deg;
-  }
-  if (ladies && !g->term) {
-    const size_t E = (size_t)(g->E > 0 ? g->E : 1);
-    float *term = nullptr;
-    double *sum = nullptr;
-    ND_CUDA(cudaMalloc(&term, sizeof(float) * E));
-    ND_CUDA(cudaMalloc(&sum, sizeof(double) * (size_t)g->V));
-    ND_CUDA(cudaMemset(sum, 0, sizeof(double) * (size_t)g->V));
-    rowsum_build_kernel<<<grid, BUILD_THREADS>>>(g->row_ptr, g->w, g->V, g->E, sum);
-    term_build_kernel<<<grid, BUILD_THREADS>>>(g->row_ptr, g->w, sum, g->V, g->E, term);
-    ND_CUDA(cudaDeviceSynchronize());
-    cudaFree(sum);
-    g->term = term;
-  }
-  ND_CUDA(cudaGetLastError());
-  return ND_OK;
+  ND_TRY(ensure_hubs(g, grid));
+  return ladies ? ensure_terms(g, grid) : ensure_degrees(g, grid);
 }
 
 // shared memory the layout may use; ND_COLLECTIVE_BITMAP_GLOBAL=1 puts the big part into global

@@ -41,6 +41,21 @@ void nd_count_launches(int n);  // bookkeeping behind nd_launch_count()
     }                               \
   } while (0)
 
+// Device memory that is given back unless it is handed over: what a build that fails half way holds.
+template <class T>
+struct NdDevMem {
+  T *p = nullptr;
+  NdDevMem() = default;
+  NdDevMem(const NdDevMem &) = delete;
+  NdDevMem &operator=(const NdDevMem &) = delete;
+  ~NdDevMem() { if (p) cudaFree(p); }
+  int alloc(size_t n) {
+    ND_CUDA(cudaMalloc(&p, sizeof(T) * n));
+    return ND_OK;
+  }
+  T *release() { T *q = p; p = nullptr; return q; }
+};
+
 // bits of the device status word (a kernel ORs a bit in and carries on with bounded work)
 enum : int {
   ND_DEV_BAD_TRANSIT = 1,   // a transit id outside [0, V)

@@ -715,34 +715,85 @@ void launch(nd_sampler *s, RowsArgs &a, bool count) {
 }
 
 // The derived layouts of a graph are built by the first sampler that needs them; samplers of one
-// graph may be created from several host threads, so the builds are serialised.
+// graph may be created from several host threads, so the builds are serialised.  What belongs together goes to
+// the graph together, when all of it is there: a build that runs out of memory leaves nothing behind.
 std::mutex g_derived_mutex;
 
 template <class T>
 int make(T *&p, size_t n) {
-  T *q = nullptr;
-  ND_CUDA(cudaMalloc(&q, sizeof(T) * n));
-  p = q;
+  NdDevMem<T> m;
+  ND_TRY(m.alloc(n));
+  p = m.release();
   return ND_OK;
 }
 
 // (neighbour id, weight) records and per-vertex (row start, maximum weight) records
 int ensure_colw(const nd_graph *g, int sms) {
   if (g->colw || g->E == 0) return ND_OK;
-  int2 *cw = nullptr;
-  ND_TRY(make(cw, (size_t)g->E));
-  if (!g->vrec && make(g->vrec, (size_t)g->V + 1) != ND_OK) { cudaFree(cw); return ND_ERR_CUDA; }
-  colw_build_kernel<<<sms * 16, 256>>>(g->col, g->w, g->E, cw);
-  vrec_build_kernel<<<sms * 16, 256>>>(g->row_ptr, g->max_w, g->V, g->vrec);
+  NdDevMem<int2> colw, vrec;
+  ND_TRY(colw.alloc((size_t)g->E));
+  ND_TRY(vrec.alloc((size_t)g->V + 1));
+  colw_build_kernel<<<sms * 16, 256>>>(g->col, g->w, g->E, colw.p);
+  vrec_build_kernel<<<sms * 16, 256>>>(g->row_ptr, g->max_w, g->V, vrec.p);
   ND_CUDA(cudaDeviceSynchronize());
-  g->colw = cw;
+  g->colw = colw.release();
+  g->vrec = vrec.release();
   return ND_OK;
 }
 
 int ensure_vrow(const nd_graph *g, int sms) {
   if (g->vrow) return ND_OK;
-  ND_TRY(make(g->vrow, (size_t)g->V));
-  vrow_build_kernel<<<sms * 16, 256>>>(g->row_ptr, g->V, g->vrow);
+  NdDevMem<int2> vrow;
+  ND_TRY(vrow.alloc((size_t)g->V));
+  vrow_build_kernel<<<sms * 16, 256>>>(g->row_ptr, g->V, vrow.p);
+  ND_CUDA(cudaGetLastError());
+  g->vrow = vrow.release();
+  return ND_OK;
+}
+
+// per-vertex records with the maximum weight, and the weights as bytes
+int ensure_wq(const nd_graph *g, int sms) {
+  if (g->wq) return ND_OK;
+  NdDevMem<int4> vrec4;
+  NdDevMem<uint8_t> wq;
+  ND_TRY(vrec4.alloc((size_t)g->V));
+  ND_TRY(wq.alloc((size_t)(g->E > 0 ? g->E : 1)));
+  vrec4_build_kernel<<<sms * 16, 256>>>(g->row_ptr, g->max_w, g->V, vrec4.p);
+  wq_build_kernel<<<sms * 16, BUILD_THREADS>>>(g->row_ptr, g->max_w, g->w, g->V, g->E, wq.p);
+  ND_CUDA(cudaGetLastError());
+  g->vrec4 = vrec4.release();
+  g->wq = wq.release();
+  return ND_OK;
+}
+
+int ensure_erec(const nd_graph *g, int sms) {
+  if (g->erec) return ND_OK;
+  NdDevMem<int4> erec;
+  ND_TRY(erec.alloc((size_t)(g->E > 0 ? g->E : 1)));
+  erec_build_kernel<<<sms * 16, 256>>>(g->col, g->row_ptr, g->E, erec.p);
+  ND_CUDA(cudaGetLastError());
+  g->erec = erec.release();
+  return ND_OK;
+}
+
+// the neighbour sets (8 bytes per CSR entry) and the filter in front of them (one byte); `d_status` / `h_status`: the
+// status word the build reports to
+int ensure_adjset(const nd_graph *g, int sms, int *d_status, const int *h_status) {
+  if (g->adjset) return ND_OK;
+  const size_t words = (size_t)(g->E > 0 ? g->E : 1) / 4 + 2, slots = 8 * words;
+  NdDevMem<uint32_t> sign;
+  NdDevMem<int32_t> set;
+  ND_TRY(sign.alloc(words));
+  ND_TRY(set.alloc(slots));
+  ND_CUDA(cudaMemset(sign.p, 0, 4 * words));
+  ND_CUDA(cudaMemset(set.p, 0xff, sizeof(int32_t) * slots));
+  adjsign_build_kernel<<<sms * 16, BUILD_THREADS>>>(g->row_ptr, g->col, g->V, g->E, sign.p);
+  adjset_build_kernel<<<sms * 16, BUILD_THREADS>>>(g->row_ptr, g->col, g->V, g->E, set.p, d_status);
+  ND_CUDA(cudaDeviceSynchronize());
+  const int st = *(const volatile int *)h_status;
+  ND_REQUIRE(st == 0, ND_ERR_DEVICE, "neighbour-set construction failed (status %d)", st);
+  g->adjsign = sign.release();
+  g->adjset = set.release();
   return ND_OK;
 }
 
@@ -760,45 +811,16 @@ int nd_graph_ensure_colw(const nd_graph *g, int sms) {
 
 int nd_walk_rows_alloc(nd_sampler *s) {
   const nd_graph *g = s->g;
-  const size_t E = (size_t)(g->E > 0 ? g->E : 1);
-  const int grid = s->dev.sms * 16;
-  const int app = s->p.app;
-  if (s->S > (int64_t)s->dev.sms * ROWS_CTAS * ROWS_THREADS) ND_TRY(make(s->d_list, (size_t)s->S));
+  const int sms = s->dev.sms, app = s->p.app;
+  if (s->S > (int64_t)sms * ROWS_CTAS * ROWS_THREADS) ND_TRY(make(s->d_list, (size_t)s->S));
   const size_t acc = 16 + ((size_t)s->p.steps + 1) / 2;
   ND_TRY(make(s->d_rows_acc, acc));
   ND_CUDA(cudaMemset(s->d_rows_acc, 0, 8 * acc));
   std::lock_guard<std::mutex> lock(g_derived_mutex);
-  if (app == ND_APP_DEEPWALK || app == ND_APP_PPR) {
-    if (!alt_layout(s)) return ensure_colw(g, s->dev.sms);
-    if (!g->wq) {
-      ND_TRY(make(g->vrec4, (size_t)g->V));
-      vrec4_build_kernel<<<grid, 256>>>(g->row_ptr, g->max_w, g->V, g->vrec4);
-      ND_TRY(make(g->wq, E));
-      wq_build_kernel<<<grid, BUILD_THREADS>>>(g->row_ptr, g->max_w, g->w, g->V, g->E, g->wq);
-    }
-    ND_CUDA(cudaGetLastError());
-    return ND_OK;
-  }
-  ND_TRY(ensure_vrow(g, s->dev.sms));
-  if (app == ND_APP_UNIFORM_WALK && alt_layout(s) && !g->erec) {
-    ND_TRY(make(g->erec, E));
-    erec_build_kernel<<<grid, 256>>>(g->col, g->row_ptr, g->E, g->erec);
-  }
-  if (app == ND_APP_NODE2VEC && !g->adjset) {   // 8 bytes per CSR entry, and one of filter
-    const size_t words = E / 4 + 2, slots = 8 * words;
-    ND_TRY(make(g->adjsign, words));
-    ND_CUDA(cudaMemset(g->adjsign, 0, 4 * words));
-    adjsign_build_kernel<<<grid, BUILD_THREADS>>>(g->row_ptr, g->col, g->V, g->E, g->adjsign);
-    int32_t *set = nullptr;
-    ND_TRY(make(set, slots));
-    ND_CUDA(cudaMemset(set, 0xff, sizeof(int32_t) * slots));
-    adjset_build_kernel<<<grid, BUILD_THREADS>>>(g->row_ptr, g->col, g->V, g->E, set, s->d_status);
-    ND_CUDA(cudaDeviceSynchronize());
-    const int st = *(volatile int *)s->h_status;
-    if (st) { cudaFree(set); ND_REQUIRE(false, ND_ERR_DEVICE, "neighbour-set construction failed (status %d)", st); }
-    g->adjset = set;
-  }
-  ND_CUDA(cudaGetLastError());
+  if (app == ND_APP_DEEPWALK || app == ND_APP_PPR) return alt_layout(s) ? ensure_wq(g, sms) : ensure_colw(g, sms);
+  ND_TRY(ensure_vrow(g, sms));
+  if (app == ND_APP_UNIFORM_WALK && alt_layout(s)) ND_TRY(ensure_erec(g, sms));
+  if (app == ND_APP_NODE2VEC) ND_TRY(ensure_adjset(g, sms, s->d_status, s->h_status));
   return ND_OK;
 }
 

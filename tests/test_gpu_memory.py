@@ -1,6 +1,14 @@
-"""Calls that fail for want of device memory: what they leave behind."""
+"""Calls that fail for want of device memory: what they leave behind.  The cases that fill the GPU's memory are
+processes of their own."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+MB = 1 << 20
 
 
 @pytest.mark.gpu
@@ -17,3 +25,76 @@ def test_a_failed_call_does_not_fail_the_next(nd, small_graph, app):
         s = nd.Sampler(g, pr, num_samples=50)
         s.sample()
         assert np.array_equal(s.final_samples(), expected)
+
+
+class Filled:
+    """All but about `left` bytes of the device's memory, allocated and never touched."""
+
+    def __init__(self, left):
+        import torch
+        torch.cuda.synchronize()
+        self.torch, self.held, chunk = torch, [], 1 << 40
+        while chunk >= 2 * MB:
+            n = min(chunk, torch.cuda.mem_get_info()[0] - left) // (2 * MB) * (2 * MB)
+            if n <= 0:
+                break
+            try:
+                self.held.append(torch.empty(n, dtype=torch.uint8, device="cuda"))
+            except torch.OutOfMemoryError:
+                chunk = n // 2
+
+    def free(self):
+        self.held.clear()
+        self.torch.cuda.empty_cache()
+
+
+def free_bytes():
+    import torch
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def samples(nd, graph, app):
+    s = nd.Sampler(graph, nd.app_params(app, steps=4 if app < 4 else 2, fanout=8, batch=8, seed=4), num_samples=500)
+    s.sample(1)
+    return s.final_samples().copy()
+
+
+# Memory that runs out in the middle of what a graph's first sampler builds: the call fails, nothing it has allocated
+# stays behind, and the same call succeeds when there is room again.  What it builds, in MB: DeepWalk 16 + 32, node2vec
+# 8 + 32 + 256, FastGCN 4 + 30 + 2, LADIES 4 + 30 + 128 + 8; the limits end in the middle of each.
+def first_samplers(app):
+    from nextdoor_b200 import api as nd
+    tiny = nd.Graph.rmat(1000, 4000, seed=1)
+    samples(nd, tiny, app)                       # the kernels are loaded
+    expected = samples(nd, nd.Graph.rmat(1 << 20, 1 << 24, seed=0), app)
+    graph, failed = nd.Graph.rmat(1 << 20, 1 << 24, seed=0), 0
+    for left in (14, 22, 30, 44, 60, 90, 150, 200, 290):
+        fill = Filled(left * MB)
+        room = []
+        for _ in range(4):
+            try:
+                got = samples(nd, graph, app)
+            except nd.NdError as e:
+                assert "memory" in str(e), e
+                room.append(free_bytes())
+                failed += 1
+            else:
+                fill.free()
+                assert np.array_equal(got, expected) and failed >= 4, failed
+                return
+        assert min(room[1:]) >= room[0], [x / MB for x in room]     # a second failure takes nothing more
+        fill.free()
+    assert np.array_equal(samples(nd, graph, app), expected) and failed >= 4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", [f"first_samplers({app})" for app in (1, 3, 8, 9)])
+def test_nothing_stays_behind(case):
+    r = subprocess.run([sys.executable, os.path.abspath(__file__), case], capture_output=True, text=True, timeout=300, cwd=ROOT)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+
+
+if __name__ == "__main__":
+    sys.path.insert(0, ROOT)
+    eval(sys.argv[1])
