@@ -423,14 +423,21 @@ int nd_graph_finish(nd_graph *g, cudaStream_t st) {
     if (g->E > 0)
       max_weight_kernel<<<grid_for(g->E, 256, dev.sms), 256, 0, st>>>(g->row_ptr, nullptr, g->w, g->V, g->E, (int32_t *)g->max_w);
   }
-  int32_t *d_m = nullptr;
-  ND_CUDA(cudaMalloc(&d_m, sizeof(int32_t)));
-  ND_CUDA(cudaMemsetAsync(d_m, 0, sizeof(int32_t), st));
-  max_degree_kernel<<<grid_for(g->V, 256, dev.sms), 256, 0, st>>>(g->row_ptr, g->V, d_m);
-  ND_CUDA(cudaMemcpyAsync(&g->max_degree, d_m, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+  NdDevMem<int32_t> m;
+  ND_TRY(m.alloc(1));
+  ND_CUDA(cudaMemsetAsync(m.p, 0, sizeof(int32_t), st));
+  max_degree_kernel<<<grid_for(g->V, 256, dev.sms), 256, 0, st>>>(g->row_ptr, g->V, m.p);
+  ND_CUDA(cudaMemcpyAsync(&g->max_degree, m.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   ND_CUDA(cudaStreamSynchronize(st));
-  cudaFree(d_m);
   return ND_OK;
+}
+
+static void free_graph(nd_graph *g) {
+  if (g->block) nd_block_free(g->device, g->block, g->block_bytes);
+  else { cudaFree(g->row_ptr); cudaFree(g->col); cudaFree(g->w); cudaFree(g->max_w); }
+  cudaFree(g->colw); cudaFree(g->vrec); cudaFree(g->vrow); cudaFree(g->vrec4); cudaFree(g->erec); cudaFree(g->wq); cudaFree(g->adjset); cudaFree(g->adjsign);
+  cudaFree(g->deg_codes); cudaFree(g->big); cudaFree(g->term); cudaFree(g->hub_slot); cudaFree(g->hub_bits);
+  delete g;
 }
 
 extern "C" {
@@ -443,24 +450,28 @@ int nd_graph_from_csr(int device, int32_t V, int64_t E, const int32_t *row_ptr, 
   ND_CUDA(cudaSetDevice(device));
   nd_graph *g = new nd_graph();
   g->device = device; g->V = V; g->E = E;
-  ND_CUDA(cudaMalloc(&g->row_ptr, sizeof(int32_t) * ((size_t)V + 1)));
-  // 32 bytes of padding: staging copies read whole 16-byte windows around a list
-  ND_CUDA(cudaMalloc(&g->col, sizeof(int32_t) * ((size_t)E + 8)));
-  ND_CUDA(cudaMalloc(&g->w, sizeof(float) * ((size_t)E + 8)));
-  ND_CUDA(cudaMemset(g->col + E, 0, sizeof(int32_t) * 8));
-  ND_CUDA(cudaMemset(g->w + E, 0, sizeof(float) * 8));
-  ND_CUDA(cudaMemcpy(g->row_ptr, row_ptr, sizeof(int32_t) * ((size_t)V + 1), cudaMemcpyHostToDevice));
-  if (E > 0) {
-    void *const to[2] = {g->col, g->w};
-    const void *const from[2] = {col, w};
-    const size_t bytes[2] = {sizeof(int32_t) * (size_t)E, sizeof(float) * (size_t)E};
-    ND_TRY(nd_copies_to_device(device, 2, to, from, bytes));
-  }
-  if (max_w) {
-    ND_CUDA(cudaMalloc(&g->max_w, sizeof(float) * (size_t)V));
-    ND_CUDA(cudaMemcpy(g->max_w, max_w, sizeof(float) * (size_t)V, cudaMemcpyHostToDevice));
-  }
-  ND_TRY(nd_graph_finish(g, nullptr));
+  auto build = [&]() -> int {
+    ND_CUDA(cudaMalloc(&g->row_ptr, sizeof(int32_t) * ((size_t)V + 1)));
+    // 32 bytes of padding: staging copies read whole 16-byte windows around a list
+    ND_CUDA(cudaMalloc(&g->col, sizeof(int32_t) * ((size_t)E + 8)));
+    ND_CUDA(cudaMalloc(&g->w, sizeof(float) * ((size_t)E + 8)));
+    ND_CUDA(cudaMemset(g->col + E, 0, sizeof(int32_t) * 8));
+    ND_CUDA(cudaMemset(g->w + E, 0, sizeof(float) * 8));
+    ND_CUDA(cudaMemcpy(g->row_ptr, row_ptr, sizeof(int32_t) * ((size_t)V + 1), cudaMemcpyHostToDevice));
+    if (E > 0) {
+      void *const to[2] = {g->col, g->w};
+      const void *const from[2] = {col, w};
+      const size_t bytes[2] = {sizeof(int32_t) * (size_t)E, sizeof(float) * (size_t)E};
+      ND_TRY(nd_copies_to_device(device, 2, to, from, bytes));
+    }
+    if (max_w) {
+      ND_CUDA(cudaMalloc(&g->max_w, sizeof(float) * (size_t)V));
+      ND_CUDA(cudaMemcpy(g->max_w, max_w, sizeof(float) * (size_t)V, cudaMemcpyHostToDevice));
+    }
+    return nd_graph_finish(g, nullptr);
+  };
+  const int rc = build();
+  if (rc != ND_OK) { free_graph(g); return rc; }
   nd_objects_add(1);
   *out = g;
   return ND_OK;
@@ -663,11 +674,7 @@ int nd_graph_device_ptrs(const nd_graph *g, const int32_t **row_ptr, const int32
 int nd_graph_destroy(nd_graph *g) {
   if (!g) return ND_OK;
   cudaSetDevice(g->device);
-  if (g->block) nd_block_free(g->device, g->block, g->block_bytes);
-  else { cudaFree(g->row_ptr); cudaFree(g->col); cudaFree(g->w); cudaFree(g->max_w); }
-  cudaFree(g->colw); cudaFree(g->vrec); cudaFree(g->vrow); cudaFree(g->vrec4); cudaFree(g->erec); cudaFree(g->wq); cudaFree(g->adjset); cudaFree(g->adjsign);
-  cudaFree(g->deg_codes); cudaFree(g->big); cudaFree(g->term); cudaFree(g->hub_slot); cudaFree(g->hub_bits);
-  delete g;
+  free_graph(g);
   nd_objects_add(-1);
   return ND_OK;
 }
@@ -677,19 +684,20 @@ int nd_graph_partition(const nd_graph *g, int64_t budget_bytes, int32_t max_part
   ND_REQUIRE(g && first_v && last_v && first_e && last_e && n_parts && max_parts >= 1, ND_ERR_ARG, "nd_graph_partition: bad argument");
   ND_REQUIRE(budget_bytes >= 20, ND_ERR_ARG, "partition budget of %lld bytes cannot hold one vertex and one edge", (long long)budget_bytes);
   ND_CUDA(cudaSetDevice(g->device));
-  int32_t *d_fv, *d_lv, *d_n;
-  long long *d_fe, *d_le;
-  ND_CUDA(cudaMalloc(&d_fv, 4 * (size_t)max_parts)); ND_CUDA(cudaMalloc(&d_lv, 4 * (size_t)max_parts));
-  ND_CUDA(cudaMalloc(&d_fe, 8 * (size_t)max_parts)); ND_CUDA(cudaMalloc(&d_le, 8 * (size_t)max_parts));
-  ND_CUDA(cudaMalloc(&d_n, 4));
-  partition_kernel<<<1, 32>>>(g->row_ptr, g->V, budget_bytes, max_parts, d_fv, d_lv, d_fe, d_le, d_n);
-  ND_CUDA(cudaMemcpy(n_parts, d_n, 4, cudaMemcpyDeviceToHost));
+  NdDevMem<int32_t> fv, lv, parts;
+  NdDevMem<long long> fe, le;
+  ND_TRY(fv.alloc((size_t)max_parts));
+  ND_TRY(lv.alloc((size_t)max_parts));
+  ND_TRY(fe.alloc((size_t)max_parts));
+  ND_TRY(le.alloc((size_t)max_parts));
+  ND_TRY(parts.alloc(1));
+  partition_kernel<<<1, 32>>>(g->row_ptr, g->V, budget_bytes, max_parts, fv.p, lv.p, fe.p, le.p, parts.p);
+  ND_CUDA(cudaMemcpy(n_parts, parts.p, 4, cudaMemcpyDeviceToHost));
   const size_t k = (size_t)*n_parts;
-  ND_CUDA(cudaMemcpy(first_v, d_fv, 4 * k, cudaMemcpyDeviceToHost));
-  ND_CUDA(cudaMemcpy(last_v, d_lv, 4 * k, cudaMemcpyDeviceToHost));
-  ND_CUDA(cudaMemcpy(first_e, d_fe, 8 * k, cudaMemcpyDeviceToHost));
-  ND_CUDA(cudaMemcpy(last_e, d_le, 8 * k, cudaMemcpyDeviceToHost));
-  cudaFree(d_fv); cudaFree(d_lv); cudaFree(d_fe); cudaFree(d_le); cudaFree(d_n);
+  ND_CUDA(cudaMemcpy(first_v, fv.p, 4 * k, cudaMemcpyDeviceToHost));
+  ND_CUDA(cudaMemcpy(last_v, lv.p, 4 * k, cudaMemcpyDeviceToHost));
+  ND_CUDA(cudaMemcpy(first_e, fe.p, 8 * k, cudaMemcpyDeviceToHost));
+  ND_CUDA(cudaMemcpy(last_e, le.p, 8 * k, cudaMemcpyDeviceToHost));
   return ND_OK;
 }
 

@@ -88,8 +88,39 @@ def first_samplers(app):
     assert np.array_equal(samples(nd, graph, app), expected) and failed >= 4
 
 
+# ids and weights of 64 MB each, row offsets and maxima of 4; the partitioner's arrays of 4, 4, 8 and 8 MB
+def graphs_and_partitions(what):
+    from nextdoor_b200 import api as nd
+    row_ptr, col, w, max_w = nd.Graph.rmat(1 << 20, 1 << 23, seed=0).to_host()
+    graph = nd.Graph.from_csr(row_ptr, col, w, max_w) if what == "partition" else None
+
+    def call():
+        if graph:
+            graph.partition(1 << 20, max_parts=1 << 20)
+        else:
+            nd.Graph.from_csr(row_ptr, col, w, max_w).free()
+
+    call()
+    failed = 0
+    for left in (4, 7, 10, 14, 20, 40, 80, 120, 160):
+        fill = Filled(left * MB)
+        room = []
+        for _ in range(4):
+            try:
+                call()
+            except nd.NdError as e:
+                assert "memory" in str(e), e
+                failed += 1
+            room.append(free_bytes())
+        assert min(room[1:]) >= room[0], [x / MB for x in room]
+        fill.free()
+    call()
+    assert failed >= 4
+
+
 @pytest.mark.gpu
-@pytest.mark.parametrize("case", [f"first_samplers({app})" for app in (1, 3, 8, 9)])
+@pytest.mark.parametrize("case", [f"first_samplers({app})" for app in (1, 3, 8, 9)]
+                         + [f"graphs_and_partitions('{what}')" for what in ("csr", "partition")])
 def test_nothing_stays_behind(case):
     r = subprocess.run([sys.executable, os.path.abspath(__file__), case], capture_output=True, text=True, timeout=300, cwd=ROOT)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
