@@ -238,9 +238,9 @@ int nd_sampler_create(const nd_graph *g, const nd_app_params *p, int64_t num_sam
   auto fail = [&](int code) { free_sampler(s); return code; };
 #define ND_TRY_S(call) do { int c__ = (call); if (c__ != ND_OK) return fail(c__); } while (0)
 #define ND_CUDA_S(call) do { cudaError_t e__ = (call); if (e__ != cudaSuccess) { cudaGetLastError(); nd_set_error("%s failed: %s", #call, cudaGetErrorString(e__)); return fail(ND_ERR_CUDA); } } while (0)
-  ND_CUDA_S(cudaMalloc(&s->d_initial, sizeof(int32_t) * S1 * s->isz));
-  ND_CUDA_S(cudaMalloc(&s->d_out, sizeof(int32_t) * S1 * s->fs));
-  ND_CUDA_S(cudaMalloc(&s->d_stats, sizeof(unsigned long long) * 8));
+  ND_CUDA_S(nd_malloc(&s->d_initial, sizeof(int32_t) * S1 * s->isz));
+  ND_CUDA_S(nd_malloc(&s->d_out, sizeof(int32_t) * S1 * s->fs));
+  ND_CUDA_S(nd_malloc(&s->d_stats, sizeof(unsigned long long) * 8));
   ND_TRY_S(status_word_get(&s->h_status, &s->d_status));
   ND_CUDA_S(cudaMemset(s->d_stats, 0, sizeof(unsigned long long) * 8));
   if (nd_is_walk(p->app)) ND_TRY_S(nd_walk_alloc(s));
@@ -359,7 +359,7 @@ int nd_sampler_aux(nd_sampler *s, int32_t *adj_row, int32_t *adj_col, float *pro
     bool done = false;
     if (adj_row && adj_col && n >= ADJ_BITS_MIN) {
       ND_CUDA(cudaSetDevice(s->g->device));
-      if (!s->d_adj_bits) ND_CUDA(cudaMalloc(&s->d_adj_bits, 4 * ((n + 31) / 32)));
+      if (!s->d_adj_bits) ND_CUDA(nd_malloc(&s->d_adj_bits, 4 * ((n + 31) / 32)));
       adj_bits_kernel<<<s->dev.sms * 8, 256, 0, s->stream>>>(s->d_adj_row, (int64_t)n, s->d_adj_bits);
       nd_count_launches(1);
       ND_CUDA(cudaStreamSynchronize(s->stream));
@@ -477,7 +477,7 @@ int nd_invert_map(int device, int64_t n, int32_t *keys_in, int32_t *vals_in, int
   NdRadixScratch scr;
   ND_TRY(nd_radix_scratch_alloc(&scr, nd_bit_length((uint32_t)(invalid > 1 ? invalid - 1 : 1)), n));
   int32_t *d_n = nullptr;
-  ND_CUDA(cudaMalloc(&d_n, 2 * sizeof(int32_t)));
+  ND_CUDA(nd_malloc(&d_n, 2 * sizeof(int32_t)));
   const int32_t n32 = (int32_t)n;
   ND_CUDA(cudaMemcpy(d_n, &n32, sizeof(int32_t), cudaMemcpyHostToDevice));
   NdSortArrays arr;
@@ -521,7 +521,7 @@ int nd_inverter_create(int device, int64_t max_pairs, int32_t invalid, nd_invert
   inv->invalid = invalid;
   int rc = nd_device_info(device, &inv->dev);
   if (rc == ND_OK) rc = nd_radix_scratch_alloc(&inv->scr, nd_bit_length((uint32_t)(invalid > 1 ? invalid - 1 : 1)), max_pairs);
-  if (rc == ND_OK && cudaMalloc(&inv->d_n, 2 * sizeof(int32_t)) != cudaSuccess) { cudaGetLastError(); nd_set_error("nd_inverter_create: cudaMalloc failed"); rc = ND_ERR_CUDA; }
+  if (rc == ND_OK && nd_malloc(&inv->d_n, 2 * sizeof(int32_t)) != cudaSuccess) { cudaGetLastError(); nd_set_error("nd_inverter_create: cudaMalloc failed"); rc = ND_ERR_CUDA; }
   if (rc != ND_OK) { nd_radix_scratch_free(&inv->scr); cudaFree(inv->d_n); delete inv; return rc; }
   *out = inv;
   return ND_OK;

@@ -738,10 +738,10 @@ int nd_coll_bitmap_alloc(nd_sampler *s) {
   const Plan p = plan_of(s);
   ND_TRY(ensure_layers(s->g, s->dev.sms, ladies));
   s->coll_grid = (int)std::min<int64_t>(s->S > 0 ? s->S : 1, (int64_t)s->dev.sms * p.per_sm);
-  if (p.lay.glob_bytes) ND_CUDA(cudaMalloc(&s->d_bm, (size_t)p.lay.glob_bytes * (size_t)s->coll_grid));
-  if (ladies) ND_CUDA(cudaMalloc(&s->d_cand_w, sizeof(float) * (size_t)s->coll_grid * (size_t)s->g->V));
-  if (ladies) ND_CUDA(cudaMalloc(&s->d_runs, sizeof(int32_t) * (size_t)s->coll_grid * (size_t)pos_entries(s, p.lay)));
-  ND_CUDA(cudaMalloc(&s->d_rows_acc, 16 * sizeof(unsigned long long)));
+  if (p.lay.glob_bytes) ND_CUDA(nd_malloc(&s->d_bm, (size_t)p.lay.glob_bytes * (size_t)s->coll_grid));
+  if (ladies) ND_CUDA(nd_malloc(&s->d_cand_w, sizeof(float) * (size_t)s->coll_grid * (size_t)s->g->V));
+  if (ladies) ND_CUDA(nd_malloc(&s->d_runs, sizeof(int32_t) * (size_t)s->coll_grid * (size_t)pos_entries(s, p.lay)));
+  ND_CUDA(nd_malloc(&s->d_rows_acc, 16 * sizeof(unsigned long long)));
   ND_CUDA(cudaMemset(s->d_rows_acc, 0, 16 * sizeof(unsigned long long)));
   return ND_OK;
 }

@@ -391,8 +391,8 @@ static int ensure_cand(nd_sampler *s, int64_t need) {
   cudaFree(s->d_cand); cudaFree(s->d_cand_w);
   nd_radix_scratch_free(&s->radix);
   s->d_cand = nullptr; s->d_cand_w = nullptr; s->cand_cap = 0;
-  ND_CUDA(cudaMalloc(&s->d_cand, sizeof(uint32_t) * 6 * (size_t)cap));
-  ND_CUDA(cudaMalloc(&s->d_cand_w, (sizeof(float) + sizeof(double)) * (size_t)cap));  // cdf (fp64) first, then weights
+  ND_CUDA(nd_malloc(&s->d_cand, sizeof(uint32_t) * 6 * (size_t)cap));
+  ND_CUDA(nd_malloc(&s->d_cand_w, (sizeof(float) + sizeof(double)) * (size_t)cap));  // cdf (fp64) first, then weights
   ND_TRY(nd_radix_scratch_alloc(&s->radix, 32, cap));
   s->cand_cap = cap;
   return ND_OK;
@@ -403,13 +403,13 @@ int nd_collective_alloc(nd_sampler *s) {
   const int L = p.fanout[0], B = p.batch;
   const size_t S1 = (size_t)(s->S > 0 ? s->S : 1);
   const size_t adj = S1 * p.steps * (size_t)(B > L ? B : L) * L;
-  ND_CUDA(cudaMalloc(&s->d_adj_row, sizeof(int32_t) * adj));
-  ND_CUDA(cudaMalloc(&s->d_adj_col, sizeof(int32_t) * adj));
-  ND_CUDA(cudaMalloc(&s->d_prob, sizeof(float) * S1 * s->fs));
+  ND_CUDA(nd_malloc(&s->d_adj_row, sizeof(int32_t) * adj));
+  ND_CUDA(nd_malloc(&s->d_adj_col, sizeof(int32_t) * adj));
+  ND_CUDA(nd_malloc(&s->d_prob, sizeof(float) * S1 * s->fs));
   ND_CUDA(cudaMemset(s->d_prob, 0, sizeof(float) * S1 * s->fs));
-  ND_CUDA(cudaMalloc(&s->d_len, sizeof(int32_t) * (S1 + 1)));        // per-sample sizes of the layer
-  ND_CUDA(cudaMalloc(&s->d_tmp, sizeof(int64_t) * (S1 + 1)));        // per-sample region offsets
-  ND_CUDA(cudaMalloc(&s->d_nlive, sizeof(int32_t) * 4));
+  ND_CUDA(nd_malloc(&s->d_len, sizeof(int32_t) * (S1 + 1)));        // per-sample sizes of the layer
+  ND_CUDA(nd_malloc(&s->d_tmp, sizeof(int64_t) * (S1 + 1)));        // per-sample region offsets
+  ND_CUDA(nd_malloc(&s->d_nlive, sizeof(int32_t) * 4));
   if (p.app == ND_APP_FASTGCN_IS || p.app == ND_APP_LADIES_IS) {
     // the union is built as a bitmap with a bit per vertex (nd_coll_bitmap.cu); ND_COLLECTIVE_SORT=1 selects
     // the sort pipeline instead (kept for the tests, which compare the two)

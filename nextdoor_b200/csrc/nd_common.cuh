@@ -41,6 +41,16 @@ void nd_count_launches(int n);  // bookkeeping behind nd_launch_count()
     }                               \
   } while (0)
 
+// cudaMalloc for everything of the library: what it keeps of freed blocks (nd_host.h) goes back before this fails.
+cudaError_t nd_malloc_bytes(void **p, size_t bytes);
+template <class T>
+cudaError_t nd_malloc(T **p, size_t bytes) {
+  void *q = nullptr;
+  const cudaError_t e = nd_malloc_bytes(&q, bytes);
+  if (e == cudaSuccess) *p = (T *)q;
+  return e;
+}
+
 // Device memory that is given back unless it is handed over: what a build that fails half way holds.
 template <class T>
 struct NdDevMem {
@@ -50,7 +60,7 @@ struct NdDevMem {
   NdDevMem &operator=(const NdDevMem &) = delete;
   ~NdDevMem() { if (p) cudaFree(p); }
   int alloc(size_t n) {
-    ND_CUDA(cudaMalloc(&p, sizeof(T) * n));
+    ND_CUDA(nd_malloc(&p, sizeof(T) * n));
     return ND_OK;
   }
   T *release() { T *q = p; p = nullptr; return q; }

@@ -418,7 +418,7 @@ int nd_graph_finish(nd_graph *g, cudaStream_t st) {
   NdDeviceInfo dev;
   ND_TRY(nd_device_info(g->device, &dev));
   if (!g->max_w) {
-    ND_CUDA(cudaMalloc(&g->max_w, sizeof(float) * (size_t)(g->V > 0 ? g->V : 1)));
+    ND_CUDA(nd_malloc(&g->max_w, sizeof(float) * (size_t)(g->V > 0 ? g->V : 1)));
     ND_CUDA(cudaMemsetAsync(g->max_w, 0, sizeof(float) * (size_t)g->V, st));
     if (g->E > 0)
       max_weight_kernel<<<grid_for(g->E, 256, dev.sms), 256, 0, st>>>(g->row_ptr, nullptr, g->w, g->V, g->E, (int32_t *)g->max_w);
@@ -451,10 +451,10 @@ int nd_graph_from_csr(int device, int32_t V, int64_t E, const int32_t *row_ptr, 
   nd_graph *g = new nd_graph();
   g->device = device; g->V = V; g->E = E;
   auto build = [&]() -> int {
-    ND_CUDA(cudaMalloc(&g->row_ptr, sizeof(int32_t) * ((size_t)V + 1)));
+    ND_CUDA(nd_malloc(&g->row_ptr, sizeof(int32_t) * ((size_t)V + 1)));
     // 32 bytes of padding: staging copies read whole 16-byte windows around a list
-    ND_CUDA(cudaMalloc(&g->col, sizeof(int32_t) * ((size_t)E + 8)));
-    ND_CUDA(cudaMalloc(&g->w, sizeof(float) * ((size_t)E + 8)));
+    ND_CUDA(nd_malloc(&g->col, sizeof(int32_t) * ((size_t)E + 8)));
+    ND_CUDA(nd_malloc(&g->w, sizeof(float) * ((size_t)E + 8)));
     ND_CUDA(cudaMemset(g->col + E, 0, sizeof(int32_t) * 8));
     ND_CUDA(cudaMemset(g->w + E, 0, sizeof(float) * 8));
     ND_CUDA(cudaMemcpy(g->row_ptr, row_ptr, sizeof(int32_t) * ((size_t)V + 1), cudaMemcpyHostToDevice));
@@ -465,7 +465,7 @@ int nd_graph_from_csr(int device, int32_t V, int64_t E, const int32_t *row_ptr, 
       ND_TRY(nd_copies_to_device(device, 2, to, from, bytes));
     }
     if (max_w) {
-      ND_CUDA(cudaMalloc(&g->max_w, sizeof(float) * (size_t)V));
+      ND_CUDA(nd_malloc(&g->max_w, sizeof(float) * (size_t)V));
       ND_CUDA(cudaMemcpy(g->max_w, max_w, sizeof(float) * (size_t)V, cudaMemcpyHostToDevice));
     }
     return nd_graph_finish(g, nullptr);

@@ -357,6 +357,21 @@ void drop_oldest() {   // under the lock
 }
 }  // namespace
 
+cudaError_t nd_malloc_bytes(void **p, size_t bytes) {
+  const cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  {   // what is kept may be what is missing
+    std::lock_guard<std::mutex> lock(g_blocks_mutex);
+    if (g_kept.empty()) return e;
+    int now = 0;
+    cudaGetDevice(&now);
+    while (!g_kept.empty()) drop_oldest();
+    cudaSetDevice(now);
+  }
+  return cudaMalloc(p, bytes);
+}
+
 int nd_block_alloc(int device, void **p, size_t *bytes) {
   {
     std::lock_guard<std::mutex> lock(g_blocks_mutex);
@@ -372,14 +387,7 @@ int nd_block_alloc(int device, void **p, size_t *bytes) {
       return ND_OK;
     }
   }
-  if (cudaMalloc(p, *bytes) == cudaSuccess) return ND_OK;
-  cudaGetLastError();
-  {   // what is kept may be what is missing
-    std::lock_guard<std::mutex> lock(g_blocks_mutex);
-    while (!g_kept.empty()) drop_oldest();
-    cudaSetDevice(device);
-  }
-  ND_CUDA(cudaMalloc(p, *bytes));
+  ND_CUDA(nd_malloc_bytes(p, *bytes));
   return ND_OK;
 }
 

@@ -166,7 +166,7 @@ int hostrows_init(nd_sampler *s) {
   cudaError_t e = cudaMallocHost(&h->h_len, sizeof(int32_t) * S1);
   if (e == cudaSuccess) e = cudaMallocHost(&h->h_chunk, sizeof(uint32_t) * ((size_t)h->n_chunks + 1));
   if (e == cudaSuccess) e = cudaMallocHost(&h->h_total, sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMalloc(&h->d_chunk, sizeof(uint32_t) * ((size_t)h->n_chunks + 1));
+  if (e == cudaSuccess) e = nd_malloc(&h->d_chunk, sizeof(uint32_t) * ((size_t)h->n_chunks + 1));
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->vs, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->packed, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->len_done, cudaEventDisableTiming);

@@ -404,10 +404,10 @@ int nd_khop_alloc(nd_sampler *s) {
   const int64_t S = s->S;
   s->map_cap = S * cap;
   ND_REQUIRE(s->map_cap * 32 < ((int64_t)1 << 31), ND_ERR_RANGE, "%lld (transit, sample) pairs per step do not fit int32 pair ids", (long long)s->map_cap);
-  ND_CUDA(cudaMalloc(&s->d_nlive, sizeof(int32_t) * (size_t)(2 * p.steps + 4)));
+  ND_CUDA(nd_malloc(&s->d_nlive, sizeof(int32_t) * (size_t)(2 * p.steps + 4)));
   s->d_init_n = s->d_nlive;
   s->map_stale = true;
-  if (p.app == ND_APP_KHOP_DISTINCT) ND_CUDA(cudaMalloc(&s->d_hop_counts, sizeof(int32_t) * (size_t)(S > 0 ? S : 1) * p.steps));
+  if (p.app == ND_APP_KHOP_DISTINCT) ND_CUDA(nd_malloc(&s->d_hop_counts, sizeof(int32_t) * (size_t)(S > 0 ? S : 1) * p.steps));
   return nd_khop_rows_alloc(s);
 }
 
@@ -418,16 +418,16 @@ static int tp_alloc(nd_sampler *s) {
   const int64_t S = s->S;
   const size_t mc = (size_t)(s->map_cap > 0 ? s->map_cap : 1);
   for (int i = 0; i < 2; i++) {
-    if (!s->d_map_key[i]) ND_CUDA(cudaMalloc(&s->d_map_key[i], sizeof(int32_t) * mc));
-    if (!s->d_map_val[i]) ND_CUDA(cudaMalloc(&s->d_map_val[i], sizeof(int32_t) * mc));
+    if (!s->d_map_key[i]) ND_CUDA(nd_malloc(&s->d_map_key[i], sizeof(int32_t) * mc));
+    if (!s->d_map_val[i]) ND_CUDA(nd_malloc(&s->d_map_val[i], sizeof(int32_t) * mc));
   }
-  if (!s->d_init_key) ND_CUDA(cudaMalloc(&s->d_init_key, sizeof(int32_t) * (size_t)(S > 0 ? S : 1)));
-  if (!s->d_init_val) ND_CUDA(cudaMalloc(&s->d_init_val, sizeof(int32_t) * (size_t)(S > 0 ? S : 1)));
+  if (!s->d_init_key) ND_CUDA(nd_malloc(&s->d_init_key, sizeof(int32_t) * (size_t)(S > 0 ? S : 1)));
+  if (!s->d_init_val) ND_CUDA(nd_malloc(&s->d_init_val, sizeof(int32_t) * (size_t)(S > 0 ? S : 1)));
   // work items of the block / grid bins: a staged run has >= 1 pair and is cut every 128+ pairs
   s->runs_cap = s->map_cap / 2 + s->map_cap / 128 + 1024;
-  if (!s->d_runs) ND_CUDA(cudaMalloc(&s->d_runs, sizeof(int2) * (size_t)s->runs_cap));
-  if (!s->d_bin_counts) ND_CUDA(cudaMalloc(&s->d_bin_counts, sizeof(int32_t) * 4 * (size_t)p.steps));
-  if (!s->d_state) ND_CUDA(cudaMalloc(&s->d_state, (size_t)s->g->V + 16));  // per-transit bin flags (kernelTypeForTransit, src/nextdoor.cu:2309)
+  if (!s->d_runs) ND_CUDA(nd_malloc(&s->d_runs, sizeof(int2) * (size_t)s->runs_cap));
+  if (!s->d_bin_counts) ND_CUDA(nd_malloc(&s->d_bin_counts, sizeof(int32_t) * 4 * (size_t)p.steps));
+  if (!s->d_state) ND_CUDA(nd_malloc(&s->d_state, (size_t)s->g->V + 16));  // per-transit bin flags (kernelTypeForTransit, src/nextdoor.cu:2309)
   const int key_bits = nd_bit_length((uint32_t)(s->g->V > 1 ? s->g->V - 1 : 1));
   if (!s->radix.tile_hist) ND_TRY(nd_radix_scratch_alloc(&s->radix, key_bits, s->map_cap > S ? s->map_cap : S));
   // host-known sizes of the unsorted child maps, kept on the device for the sort

@@ -250,7 +250,7 @@ bool nd_khop_rows_fits(const nd_sampler *s) { return s->fs <= ROW_MAX; }
 
 int nd_khop_rows_alloc(nd_sampler *s) {
   ND_TRY(nd_graph_ensure_vrow(s->g, s->dev.sms));
-  ND_CUDA(cudaMalloc(&s->d_rows_acc, 16 * sizeof(unsigned long long)));
+  ND_CUDA(nd_malloc(&s->d_rows_acc, 16 * sizeof(unsigned long long)));
   ND_CUDA(cudaMemset(s->d_rows_acc, 0, 16 * sizeof(unsigned long long)));
   return ND_OK;
 }

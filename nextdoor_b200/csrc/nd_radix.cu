@@ -356,7 +356,7 @@ void nd_radix_scratch_place(NdRadixScratch *s, const NdRadixPlan &plan, void *at
 
 int nd_radix_scratch_alloc(NdRadixScratch *s, int key_bits, int64_t max_n) {
   void *p = nullptr;
-  ND_CUDA(cudaMalloc(&p, nd_radix_scratch_bytes(max_n)));
+  ND_CUDA(nd_malloc(&p, nd_radix_scratch_bytes(max_n)));
   nd_radix_scratch_place(s, nd_radix_plan(key_bits, max_n), p);
   ND_CUDA(cudaMemset(s->ghist, 0, sizeof(uint32_t) * 8 * s->cap_bins));
   return ND_OK;

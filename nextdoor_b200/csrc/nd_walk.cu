@@ -1136,7 +1136,7 @@ int nd_walk_step_launch(const nd_graph *g, const nd_app_params *p, int step, int
 }
 
 int nd_walk_ensure_tmp(nd_sampler *s) {
-  if (!s->d_tmp) ND_CUDA(cudaMalloc(&s->d_tmp, sizeof(int32_t) * (size_t)(s->S > 0 ? s->S : 1) * s->p.steps));
+  if (!s->d_tmp) ND_CUDA(nd_malloc(&s->d_tmp, sizeof(int32_t) * (size_t)(s->S > 0 ? s->S : 1) * s->p.steps));
   return ND_OK;
 }
 
@@ -1145,10 +1145,10 @@ int nd_walk_alloc(nd_sampler *s) {
   const int steps = s->p.steps;
   ND_REQUIRE(steps >= 1 && steps <= 4096, ND_ERR_ARG, "walk length %d out of range [1,4096]", steps);
   // the result array starts out all-invalid with no slot in use (every kernel that writes rows keeps it that way)
-  ND_CUDA(cudaMalloc(&s->d_plen, sizeof(int32_t) * (size_t)(S > 0 ? S : 1)));
+  ND_CUDA(nd_malloc(&s->d_plen, sizeof(int32_t) * (size_t)(S > 0 ? S : 1)));
   ND_CUDA(cudaMemset(s->d_plen, 0, sizeof(int32_t) * (size_t)(S > 0 ? S : 1)));
   if (S > 0) walk_fill_kernel<<<s->dev.sms * 8, 256>>>(s->d_out, S * steps / 4, S * steps, s->g->V);
-  ND_CUDA(cudaMalloc(&s->d_nlive, sizeof(int32_t) * (size_t)(steps + 5)));  // live pairs per step, a spare slot, the tail launch's work counter, walks that can start, pairs of the initial map
+  ND_CUDA(nd_malloc(&s->d_nlive, sizeof(int32_t) * (size_t)(steps + 5)));  // live pairs per step, a spare slot, the tail launch's work counter, walks that can start, pairs of the initial map
   s->d_init_n = s->d_nlive + steps + 4;
   s->map_stale = true;
   return nd_walk_rows_alloc(s);
@@ -1160,15 +1160,15 @@ static int tp_alloc(nd_sampler *s) {
   const size_t S1 = (size_t)(S > 0 ? S : 1);
   ND_TRY(nd_walk_ensure_tmp(s));
   if (s->p.app == ND_APP_DEEPWALK || s->p.app == ND_APP_PPR) ND_TRY(nd_graph_ensure_colw(s->g, s->dev.sms));
-  if (!s->d_len) ND_CUDA(cudaMalloc(&s->d_len, sizeof(int32_t) * S1));
-  if (s->p.app == ND_APP_NODE2VEC && !s->d_state) ND_CUDA(cudaMalloc(&s->d_state, sizeof(int32_t) * S1));
+  if (!s->d_len) ND_CUDA(nd_malloc(&s->d_len, sizeof(int32_t) * S1));
+  if (s->p.app == ND_APP_NODE2VEC && !s->d_state) ND_CUDA(nd_malloc(&s->d_state, sizeof(int32_t) * S1));
   s->map_cap = S;
   for (int i = 0; i < 2; i++) {
-    if (!s->d_map_key[i]) ND_CUDA(cudaMalloc(&s->d_map_key[i], sizeof(int32_t) * S1));
-    if (!s->d_map_val[i]) ND_CUDA(cudaMalloc(&s->d_map_val[i], sizeof(int32_t) * S1));
+    if (!s->d_map_key[i]) ND_CUDA(nd_malloc(&s->d_map_key[i], sizeof(int32_t) * S1));
+    if (!s->d_map_val[i]) ND_CUDA(nd_malloc(&s->d_map_val[i], sizeof(int32_t) * S1));
   }
-  if (!s->d_init_key) ND_CUDA(cudaMalloc(&s->d_init_key, sizeof(int32_t) * S1));
-  if (!s->d_init_val) ND_CUDA(cudaMalloc(&s->d_init_val, sizeof(int32_t) * S1));
+  if (!s->d_init_key) ND_CUDA(nd_malloc(&s->d_init_key, sizeof(int32_t) * S1));
+  if (!s->d_init_val) ND_CUDA(nd_malloc(&s->d_init_val, sizeof(int32_t) * S1));
   const int key_bits = nd_bit_length((uint32_t)(s->g->V > 1 ? s->g->V - 1 : 1));
   if (!s->radix.tile_hist) ND_TRY(nd_radix_scratch_alloc(&s->radix, key_bits, S));
   return ND_OK;
@@ -1179,14 +1179,14 @@ static int loop_alloc(nd_sampler *s) {
   if (s->loop_ready) return ND_OK;
   const size_t V = (size_t)s->g->V, S1 = (size_t)(s->S > 0 ? s->S : 1);
   const size_t bins = (V + CNT_SUPER - 1) / CNT_SUPER;
-  if (!s->d_cnt) ND_CUDA(cudaMalloc(&s->d_cnt, sizeof(uint32_t) * bins * CNT_SUPER));   // padded to whole bins
-  if (!s->d_offs) ND_CUDA(cudaMalloc(&s->d_offs, sizeof(uint32_t) * bins * CNT_SUPER));
-  if (!s->d_bsum) ND_CUDA(cudaMalloc(&s->d_bsum, sizeof(uint32_t) * bins));
-  if (!s->d_rank) ND_CUDA(cudaMalloc(&s->d_rank, sizeof(int32_t) * S1));
+  if (!s->d_cnt) ND_CUDA(nd_malloc(&s->d_cnt, sizeof(uint32_t) * bins * CNT_SUPER));   // padded to whole bins
+  if (!s->d_offs) ND_CUDA(nd_malloc(&s->d_offs, sizeof(uint32_t) * bins * CNT_SUPER));
+  if (!s->d_bsum) ND_CUDA(nd_malloc(&s->d_bsum, sizeof(uint32_t) * bins));
+  if (!s->d_rank) ND_CUDA(nd_malloc(&s->d_rank, sizeof(int32_t) * S1));
   ND_CUDA(cudaMemset(s->d_cnt, 0, sizeof(uint32_t) * bins * CNT_SUPER));
   ND_CUDA(cudaMemset(s->d_bsum, 0, sizeof(uint32_t) * bins));
-  for (int i = 0; i < 2; i++) if (!s->d_srec[i]) ND_CUDA(cudaMalloc(&s->d_srec[i], sizeof(int2) * S1));
-  if (!s->d_init_rec) ND_CUDA(cudaMalloc(&s->d_init_rec, sizeof(int2) * S1));
+  for (int i = 0; i < 2; i++) if (!s->d_srec[i]) ND_CUDA(nd_malloc(&s->d_srec[i], sizeof(int2) * S1));
+  if (!s->d_init_rec) ND_CUDA(nd_malloc(&s->d_init_rec, sizeof(int2) * S1));
   if (s->p.app == ND_APP_PPR && s->p.stop_prob > 0.f && !s->h_active) {  // the tail launch runs beside the result update
     ND_CUDA(cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking));
     ND_CUDA(cudaEventCreateWithFlags(&s->side_fork, cudaEventDisableTiming));

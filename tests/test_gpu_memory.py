@@ -65,9 +65,7 @@ def samples(nd, graph, app):
 # 8 + 32 + 256, FastGCN 4 + 30 + 2, LADIES 4 + 30 + 128 + 8; the limits end in the middle of each.
 def first_samplers(app):
     from nextdoor_b200 import api as nd
-    tiny = nd.Graph.rmat(1000, 4000, seed=1)
-    samples(nd, tiny, app)                       # the kernels are loaded
-    expected = samples(nd, nd.Graph.rmat(1 << 20, 1 << 24, seed=0), app)
+    expected = samples(nd, nd.Graph.rmat(1 << 20, 1 << 24, seed=0), app)   # (and nothing is alive after it: no block is kept)
     graph, failed = nd.Graph.rmat(1 << 20, 1 << 24, seed=0), 0
     for left in (14, 22, 30, 44, 60, 90, 150, 200, 290):
         fill = Filled(left * MB)
@@ -83,7 +81,7 @@ def first_samplers(app):
                 fill.free()
                 assert np.array_equal(got, expected) and failed >= 4, failed
                 return
-        assert min(room[1:]) >= room[0], [x / MB for x in room]     # a second failure takes nothing more
+        assert min(room[1:]) > room[0] - MB, [x / MB for x in room]     # a second failure takes no more (the least array is 4 MB; small ones share pages)
         fill.free()
     assert np.array_equal(samples(nd, graph, app), expected) and failed >= 4
 
@@ -112,15 +110,32 @@ def graphs_and_partitions(what):
                 assert "memory" in str(e), e
                 failed += 1
             room.append(free_bytes())
-        assert min(room[1:]) >= room[0], [x / MB for x in room]
+        assert min(room[1:]) > room[0] - MB, [x / MB for x in room]
         fill.free()
     call()
     assert failed >= 4
 
 
+# a freed graph's block of 140 MB is kept for the next build, and a sampler needs the room
+def kept_blocks():
+    from nextdoor_b200 import api as nd
+    small = nd.Graph.rmat(1000, 4000, seed=1)
+    uniform = nd.app_params(0, steps=100, seed=4)
+    s = nd.Sampler(small, uniform, num_samples=1000)
+    s.sample()
+    expected = s.final_samples().copy()
+    nd.Graph.rmat(1 << 20, 1 << 23, seed=0).free()
+    fill = Filled(20 * MB)
+    assert free_bytes() < 24 * MB
+    s = nd.Sampler(small, uniform, num_samples=300_000)          # 120 MB
+    s.sample()
+    assert np.array_equal(s.final_samples()[:1000], expected)
+    fill.free()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("case", [f"first_samplers({app})" for app in (1, 3, 8, 9)]
-                         + [f"graphs_and_partitions('{what}')" for what in ("csr", "partition")])
+                         + [f"graphs_and_partitions('{what}')" for what in ("csr", "partition")] + ["kept_blocks()"])
 def test_nothing_stays_behind(case):
     r = subprocess.run([sys.executable, os.path.abspath(__file__), case], capture_output=True, text=True, timeout=300, cwd=ROOT)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
