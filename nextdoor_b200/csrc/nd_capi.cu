@@ -359,7 +359,9 @@ int nd_sampler_aux(nd_sampler *s, int32_t *adj_row, int32_t *adj_col, float *pro
     bool done = false;
     if (adj_row && adj_col && n >= ADJ_BITS_MIN) {
       ND_CUDA(cudaSetDevice(s->g->device));
-      if (!s->d_adj_bits) ND_CUDA(nd_malloc(&s->d_adj_bits, 4 * ((n + 31) / 32)));
+      if (!s->d_adj_bits && nd_malloc(&s->d_adj_bits, 4 * ((n + 31) / 32)) != cudaSuccess) cudaGetLastError();   // the plain copies need none
+    }
+    if (adj_row && adj_col && n >= ADJ_BITS_MIN && s->d_adj_bits) {
       adj_bits_kernel<<<s->dev.sms * 8, 256, 0, s->stream>>>(s->d_adj_row, (int64_t)n, s->d_adj_bits);
       nd_count_launches(1);
       ND_CUDA(cudaStreamSynchronize(s->stream));

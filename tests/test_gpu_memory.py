@@ -133,9 +133,24 @@ def kept_blocks():
     fill.free()
 
 
+# the adjacency of 102 M entries crosses as 13 MB of bits, which do not fit: it is copied as it is
+def adjacency():
+    from nextdoor_b200 import api as nd
+    graph = nd.Graph.rmat(20_000, 80_000, seed=1)
+    s, t = (nd.Sampler(graph, nd.app_params(6, steps=5, seed=2), num_samples=5000) for _ in range(2))
+    s.sample()
+    t.sample()
+    expected = t.aux()
+    fill = Filled(6 * MB)
+    got = s.aux()
+    fill.free()
+    assert (got["adj_row"] >= 0).any()
+    assert np.array_equal(got["adj_row"], expected["adj_row"]) and np.array_equal(got["adj_col"], expected["adj_col"])
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("case", [f"first_samplers({app})" for app in (1, 3, 8, 9)]
-                         + [f"graphs_and_partitions('{what}')" for what in ("csr", "partition")] + ["kept_blocks()"])
+                         + [f"graphs_and_partitions('{what}')" for what in ("csr", "partition")] + ["kept_blocks()", "adjacency()"])
 def test_nothing_stays_behind(case):
     r = subprocess.run([sys.executable, os.path.abspath(__file__), case], capture_output=True, text=True, timeout=300, cwd=ROOT)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
