@@ -673,8 +673,8 @@ int ensure_layers(const nd_graph *g, int sms, bool ladies) {
   return ladies ? ensure_terms(g, grid) : ensure_degrees(g, grid);
 }
 
-// shared memory the layout may use; ND_COLLECTIVE_BITMAP_GLOBAL=1 puts the big part into global
-// scratch whatever the graph's size (the tests use it to cover that path on small graphs)
+// ND_COLLECTIVE_BITMAP_GLOBAL=1 puts the big part into global scratch whatever the graph's size (the tests use it to
+// cover that path on small graphs).  Asked once per sampler: its buffers are sized by the answer.
 bool force_global() {
   const char *e = getenv("ND_COLLECTIVE_BITMAP_GLOBAL");
   return e && e[0] == '1';
@@ -711,7 +711,7 @@ Plan plan_of(const nd_sampler *s) {
   const uint32_t optin = (uint32_t)s->dev.smem_optin - 64u, half = optin / 2u - 1024u;
   const uint32_t need = place(big) + tile_least;
   Plan p;
-  const bool global = force_global() || need > optin;
+  const bool global = s->coll_global || need > optin;
   const uint32_t base = place(global ? 0u : big);
   const bool two = !global && need <= half;
   const uint32_t room = (two ? half : optin) - base;
@@ -735,6 +735,7 @@ int pos_entries(const nd_sampler *s, const Layout &lay) {
 
 int nd_coll_bitmap_alloc(nd_sampler *s) {
   const bool ladies = s->p.app == ND_APP_LADIES_IS;
+  s->coll_global = force_global();
   const Plan p = plan_of(s);
   ND_TRY(ensure_layers(s->g, s->dev.sms, ladies));
   s->coll_grid = (int)std::min<int64_t>(s->S > 0 ? s->S : 1, (int64_t)s->dev.sms * p.per_sm);

@@ -259,6 +259,7 @@ struct nd_sampler {
   float *d_cand_w = nullptr;
   int64_t cand_cap = 0;
   bool coll_bitmap = false;       // importance sampling through the shared-memory bitmap kernel
+  bool coll_global = false;       // ... whose bitmaps are put into global scratch whatever the graph's size
   int coll_grid = 0;
   unsigned char *d_bm = nullptr;  // per-CTA bitmap slices when a bit per vertex does not fit shared memory
 

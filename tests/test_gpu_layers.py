@@ -28,3 +28,18 @@ def test_fastgcn_weights_at_the_edges_of_the_codes(nd, ndo, monkeypatch, V, degr
     assert np.array_equal(s.final_samples(), exp["out"])   # whole numbers: the sums are exact
     assert np.array_equal(aux["prob"].reshape(-1), exp["prob"].reshape(-1))
     assert np.array_equal(aux["adj_row"], exp["adj_row"]) and np.array_equal(aux["adj_col"], exp["adj_col"])
+
+
+@pytest.mark.parametrize("app", [8, 9])
+@pytest.mark.parametrize("created,sampled", [("0", "1"), ("1", "0")])
+def test_a_sampler_keeps_the_layout_it_was_created_with(nd, monkeypatch, small_graph, app, created, sampled):
+    """The switch that moves the bitmaps to global scratch is asked when the buffers are sized, not again by a job."""
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    out = []
+    for at_creation in (created, sampled):
+        monkeypatch.setenv("ND_COLLECTIVE_BITMAP_GLOBAL", at_creation)
+        s = nd.Sampler(g, nd.app_params(app, steps=2, fanout=32, batch=24, seed=3), num_samples=400)
+        monkeypatch.setenv("ND_COLLECTIVE_BITMAP_GLOBAL", sampled)
+        s.sample()
+        out.append(s.final_samples())
+    assert np.array_equal(out[0], out[1])
