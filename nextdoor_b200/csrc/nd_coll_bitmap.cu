@@ -708,7 +708,7 @@ Plan plan_of(const nd_sampler *s) {
     return (off + 15u) & ~15u;
   };
   const uint32_t tile_least = ladies ? 8u * 4096u : 0u, tile_most = ladies ? 8u * 16384u : 0u;   // whole groups
-  const uint32_t optin = (uint32_t)s->dev.smem_optin - 64u, half = optin / 2u - 1024u;
+  const uint32_t optin = (uint32_t)(s->dev.smem_optin - ND_SMEM_STATIC), half = optin / 2u - 1024u;
   const uint32_t need = place(big) + tile_least;
   Plan p;
   const bool global = s->coll_global || need > optin;
@@ -738,6 +738,7 @@ int nd_coll_bitmap_alloc(nd_sampler *s) {
   s->coll_global = force_global();
   const Plan p = plan_of(s);
   ND_TRY(ensure_layers(s->g, s->dev.sms, ladies));
+  ND_CUDA(ladies ? nd_smem_most(coll_bitmap_kernel<true>, s->dev) : nd_smem_most(coll_bitmap_kernel<false>, s->dev));
   s->coll_grid = (int)std::min<int64_t>(s->S > 0 ? s->S : 1, (int64_t)s->dev.sms * p.per_sm);
   if (p.lay.glob_bytes) ND_CUDA(nd_malloc(&s->d_bm, (size_t)p.lay.glob_bytes * (size_t)s->coll_grid));
   if (ladies) ND_CUDA(nd_malloc(&s->d_cand_w, sizeof(float) * (size_t)s->coll_grid * (size_t)s->g->V));
@@ -754,13 +755,8 @@ int nd_coll_bitmap_launch(nd_sampler *s, const CollParams &cp, unsigned long lon
   const Args a{nd_view(g), cp, s->p.steps, s->S, p.lay, s->d_bm, s->d_initial, s->d_out, s->d_cand_w,
                s->d_runs, ladies ? pos_entries(s, p.lay) : 0, s->d_adj_row, s->d_adj_col, s->d_prob,
                g->deg_codes, g->big, g->n_big, g->term, g->hub_slot, g->hub_bits, s->d_rows_acc, s->d_stats, pairs};
-  if (ladies) {
-    ND_CUDA(cudaFuncSetAttribute(coll_bitmap_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.lay.bytes));
-    coll_bitmap_kernel<true><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
-  } else {
-    ND_CUDA(cudaFuncSetAttribute(coll_bitmap_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.lay.bytes));
-    coll_bitmap_kernel<false><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
-  }
+  if (ladies) coll_bitmap_kernel<true><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
+  else coll_bitmap_kernel<false><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
   nd_count_launches(1);
   ND_CUDA(cudaGetLastError());
   return ND_OK;

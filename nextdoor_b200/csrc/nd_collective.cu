@@ -410,6 +410,7 @@ int nd_collective_alloc(nd_sampler *s) {
   ND_CUDA(nd_malloc(&s->d_len, sizeof(int32_t) * (S1 + 1)));        // per-sample sizes of the layer
   ND_CUDA(nd_malloc(&s->d_tmp, sizeof(int64_t) * (S1 + 1)));        // per-sample region offsets
   ND_CUDA(nd_malloc(&s->d_nlive, sizeof(int32_t) * 4));
+  ND_CUDA(nd_smem_most(coll_ref_kernel, s->dev));
   if (p.app == ND_APP_FASTGCN_IS || p.app == ND_APP_LADIES_IS) {
     // the union is built as a bitmap with a bit per vertex (nd_coll_bitmap.cu); ND_COLLECTIVE_SORT=1 selects
     // the sort pipeline instead (kept for the tests, which compare the two)
@@ -448,7 +449,6 @@ int nd_collective_sample(nd_sampler *s, int mode) {
   }
   if (ref_app) {
     const RefLayout lay = ref_layout(p.steps, cp.B, cp.L);
-    if (lay.bytes > 48u * 1024u) ND_CUDA(cudaFuncSetAttribute(coll_ref_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lay.bytes));
     const int per_sm = lay.bytes <= 24u * 1024u ? 8 : 1;
     nd_phase_begin(s, ND_PHASE_NEXT);
     coll_ref_kernel<<<(int)std::min<int64_t>(S, (int64_t)s->dev.sms * per_sm), CTHREADS, lay.bytes, st>>>(

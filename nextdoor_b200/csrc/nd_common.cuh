@@ -83,6 +83,14 @@ struct NdDeviceInfo {
 };
 int nd_device_info(int device, NdDeviceInfo *info);
 
+// What a launch may take of dynamic shared memory.  The limit belongs to the kernel, not to the launch: threads that set
+// it to the size of their own launches take each other's away, so it is always set to the most there is.
+static constexpr int ND_SMEM_STATIC = 64;   // left for the kernel's own arrays
+template <class K>
+cudaError_t nd_smem_most(K kernel, const NdDeviceInfo &dev) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin - ND_SMEM_STATIC);
+}
+
 // ---------------------------------------------------------------- graph replica (SoA in HBM)
 //
 // row_ptr[V+1] int32 exclusive ends (the reference's 16-byte AoS vertex record, src/csr.hpp:49-79,

@@ -250,6 +250,7 @@ bool nd_khop_rows_fits(const nd_sampler *s) { return s->fs <= ROW_MAX; }
 
 int nd_khop_rows_alloc(nd_sampler *s) {
   ND_TRY(nd_graph_ensure_vrow(s->g, s->dev.sms));
+  ND_CUDA(s->p.app == ND_APP_KHOP_DISTINCT ? nd_smem_most(khop_rows_kernel<true>, s->dev) : nd_smem_most(khop_rows_kernel<false>, s->dev));
   ND_CUDA(nd_malloc(&s->d_rows_acc, 16 * sizeof(unsigned long long)));
   ND_CUDA(cudaMemset(s->d_rows_acc, 0, 16 * sizeof(unsigned long long)));
   return ND_OK;
@@ -276,10 +277,6 @@ int nd_khop_rows_launch(nd_sampler *s) {
   const int64_t groups = (s->S + warps - 1) / warps, cap = (int64_t)s->dev.sms * khop_ctas(distinct) * 8 / warps;
   const int grid = (int)(groups < cap ? groups : cap);
   a.batch = s->S > (int64_t)grid * warps * 16 ? 4 : 1;   // one by one where four would leave warps idle at the end
-  if (smem > 48 * 1024) {
-    if (distinct) ND_CUDA(cudaFuncSetAttribute(khop_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    else ND_CUDA(cudaFuncSetAttribute(khop_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  }
   if (distinct) khop_rows_kernel<true><<<grid, warps * 32, smem, s->stream>>>(a);
   else khop_rows_kernel<false><<<grid, warps * 32, smem, s->stream>>>(a);
   nd_count_launches(1);

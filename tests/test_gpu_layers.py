@@ -43,3 +43,32 @@ def test_a_sampler_keeps_the_layout_it_was_created_with(nd, monkeypatch, small_g
         s.sample()
         out.append(s.final_samples())
     assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("app,sizes", [(8, [(16, 16), (600, 600)]), (9, [(16, 16), (600, 600)]), (7, [(600, 600), (1000, 1000)]), (4, [(16, 15, 13), (15, 15, 17)])])
+def test_threads_with_different_shared_memory(nd, small_graph, app, sizes):
+    """The limit of a kernel's dynamic shared memory is the kernel's: a thread that launches with little must not lower
+    it under another's launch."""
+    import threading
+    wide = nd.Graph.rmat(300_000, 600_000, seed=1)
+    graphs = [nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w), wide]
+    samplers = []
+    for g, size in zip(graphs, sizes):
+        pr = nd.app_params(app, fanout=list(size), seed=3) if app == 4 else nd.app_params(app, steps=1, fanout=size[0], batch=size[1], seed=3)
+        samplers.append(nd.Sampler(g, pr, num_samples=2))
+    errors = []
+
+    def work(s):
+        try:
+            for _ in range(1500):
+                s.sample(sync=False)
+            s.sync()
+        except nd.NdError as e:
+            errors.append(str(e))
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in samplers]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
