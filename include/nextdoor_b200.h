@@ -105,6 +105,9 @@ int nd_graph_to_host(const nd_graph *g, int32_t *row_ptr, int32_t *col, float *w
 /* device addresses of the replica (GPUCSRPartition, src/csr.hpp:387-393) */
 int nd_graph_device_ptrs(const nd_graph *g, const int32_t **row_ptr, const int32_t **col,
                          const float **w, const float **max_w);
+/* device address of the slots [V] of the neighbourhoods that importance layers keep as bitmaps (-1: none); null before
+ * the graph's first sampler of such layers */
+int nd_graph_hub_slots(const nd_graph *g, const int32_t **slot);
 int nd_graph_destroy(nd_graph *g);
 /* create_csr_partitions (src/graph_partitioner.cuh:1-173): contiguous vertex ranges under a byte
  * budget (16 B per vertex record, 4 B per edge); boundaries are found on the device. */

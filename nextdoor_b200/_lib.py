@@ -62,6 +62,7 @@ _SIGS = {
     "nd_graph_info": (C.c_int, [VP, C.POINTER(C.c_int32), C.POINTER(C.c_int64), C.POINTER(C.c_int32), C.POINTER(C.c_int)]),
     "nd_graph_to_host": (C.c_int, [VP, VP, VP, VP, VP]),
     "nd_graph_device_ptrs": (C.c_int, [VP, C.POINTER(VP), C.POINTER(VP), C.POINTER(VP), C.POINTER(VP)]),
+    "nd_graph_hub_slots": (C.c_int, [VP, C.POINTER(VP)]),
     "nd_graph_destroy": (C.c_int, [VP]),
     "nd_graph_partition": (C.c_int, [VP, C.c_int64, C.c_int32, VP, VP, VP, VP, C.POINTER(C.c_int32)]),
     "nd_final_sample_size": (C.c_int, [C.POINTER(AppParams)]),

@@ -569,11 +569,22 @@ term_build_kernel(const int32_t *__restrict__ row_ptr, const float *__restrict__
   });
 }
 
-__global__ void hub_slots_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int32_t least, int cap, int32_t *__restrict__ slot,
+// Vertices in the order in which they get a bitmap: more neighbours first, of equally many the lower id; no two the same.
+__host__ __device__ __forceinline__ uint64_t hub_rank(int32_t deg, uint32_t v) { return (uint64_t)(uint32_t)deg << 32 | (0xffffffffu - v); }
+
+__global__ void __launch_bounds__(256) hub_count_kernel(const int32_t *__restrict__ row_ptr, int32_t V, uint64_t least, int32_t *__restrict__ count) {
+  int32_t n = 0;
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x)
+    n += hub_rank(row_ptr[v + 1] - row_ptr[v], (uint32_t)v) >= least ? 1 : 0;
+  n = __reduce_add_sync(0xffffffffu, n);
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd(count, n);
+}
+
+__global__ void hub_slots_kernel(const int32_t *__restrict__ row_ptr, int32_t V, uint64_t least, int cap, int32_t *__restrict__ slot,
                                  int32_t *__restrict__ hubs, int32_t *__restrict__ count) {
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x) {
     int32_t at = -1;
-    if (row_ptr[v + 1] - row_ptr[v] >= least) {
+    if (hub_rank(row_ptr[v + 1] - row_ptr[v], (uint32_t)v) >= least) {
       at = atomicAdd(count, 1);
       if (at < cap) hubs[at] = (int32_t)v; else at = -1;
     }
@@ -597,7 +608,9 @@ int words_of(int32_t V) { return (int)((((int64_t)V + 31) / 32 + GROUP_WORDS - 1
 // A bitmap pays against the list it replaces from about V/128 neighbours: four times the list's bytes, but ORed a word
 // at a time (FastGCN from V/64, V/128, V/192: 1.14, 0.98, 0.99 ms with 1024 batches on 2^20 vertices, 0.83, 0.59, 0.59 with 256 on
 // 2^21).
-// At most HUBS of them (a graph can hold 128 E / V such vertices).
+// At most HUBS of them, those with the most neighbours: a graph can hold 128 E / V such vertices.  (1024 batches on 233 K
+// vertices and 114 M entries: FastGCN 4.1 ms with the 1024 that came first, 0.79 with the largest; LADIES, which goes
+// through the lists again, 22.6 and 21.7.  Finding the rank adds 1.2 ms to the first sampler of such a graph.)
 constexpr int HUBS = 1024;
 std::mutex g_layers_mutex;
 
@@ -608,12 +621,26 @@ int ensure_hubs(const nd_graph *g, int grid) {
   NdDevMem<uint32_t> bits;
   ND_TRY(slot.alloc((size_t)g->V));
   ND_TRY(hubs.alloc(HUBS + 1));
-  ND_CUDA(cudaMemset(hubs.p + HUBS, 0, sizeof(int32_t)));
-  const int32_t least = std::max<int32_t>(g->V / HUB, 256);
-  hub_slots_kernel<<<grid, 256>>>(g->row_ptr, g->V, least, HUBS, slot.p, hubs.p, hubs.p + HUBS);
+  int32_t *const count = hubs.p + HUBS;
   int32_t n = 0;
-  ND_CUDA(cudaMemcpy(&n, hubs.p + HUBS, sizeof(n), cudaMemcpyDeviceToHost));
-  n = std::min(n, HUBS);
+  auto slots = [&](uint64_t least) -> int {
+    ND_CUDA(cudaMemset(count, 0, sizeof(int32_t)));
+    hub_slots_kernel<<<grid, 256>>>(g->row_ptr, g->V, least, HUBS, slot.p, hubs.p, count);
+    ND_CUDA(cudaMemcpy(&n, count, sizeof(n), cudaMemcpyDeviceToHost));
+    return ND_OK;
+  };
+  uint64_t least = (uint64_t)std::max<int32_t>(g->V / HUB, 256) << 32;
+  ND_TRY(slots(least));
+  if (n > HUBS) {   // the rank that HUBS vertices reach, by bisection: at most 63 passes over the row offsets
+    for (uint64_t lo = least, hi = (uint64_t)1 << 63; n != HUBS;) {
+      least = lo + (hi - lo) / 2;
+      ND_CUDA(cudaMemset(count, 0, sizeof(int32_t)));
+      hub_count_kernel<<<grid, 256>>>(g->row_ptr, g->V, least, count);
+      ND_CUDA(cudaMemcpy(&n, count, sizeof(n), cudaMemcpyDeviceToHost));
+      if (n > HUBS) lo = least; else hi = least;
+    }
+    ND_TRY(slots(least));
+  }
   const size_t words = (size_t)words_of(g->V) * (size_t)std::max(n, 1);
   ND_TRY(bits.alloc(words));
   ND_CUDA(cudaMemset(bits.p, 0, sizeof(uint32_t) * words));
@@ -732,6 +759,13 @@ int pos_entries(const nd_sampler *s, const Layout &lay) {
 }
 
 }  // namespace
+
+extern "C" int nd_graph_hub_slots(const nd_graph *g, const int32_t **slot) {
+  ND_REQUIRE(g && slot, ND_ERR_ARG, "nd_graph_hub_slots: null argument");
+  std::lock_guard<std::mutex> lock(g_layers_mutex);
+  *slot = g->hub_slot;
+  return ND_OK;
+}
 
 int nd_coll_bitmap_alloc(nd_sampler *s) {
   const bool ladies = s->p.app == ND_APP_LADIES_IS;

@@ -72,3 +72,34 @@ def test_threads_with_different_shared_memory(nd, small_graph, app, sizes):
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+@pytest.mark.parametrize("kind,hubs", [("apart", 1023), ("apart", 1025), ("apart", 2500), ("equal", 1500), ("few ties", 1500)])
+@pytest.mark.parametrize("app", [8, 9])
+def test_bitmaps_go_to_the_vertices_with_the_most_neighbours(nd, ndo, app, kind, hubs):
+    """1024 neighbourhoods are kept as bitmaps; of more vertices with enough neighbours the largest have one, of equal
+    ones those with the lowest ids."""
+    import ctypes as C
+    import torch
+    V = 8000                                       # 256 neighbours and more
+    rng = np.random.default_rng(hubs)
+    ids = rng.permutation(V)[:hubs]
+    deg = np.zeros(V, np.int64)
+    deg[rng.integers(0, V, 2000)] = rng.integers(1, 250, 2000)
+    deg[ids] = {"apart": 256 + np.arange(hubs) // 2, "equal": np.full(hubs, 300), "few ties": 256 + rng.integers(0, 4, hubs)}[kind]
+    src = np.repeat(np.arange(V), deg).astype(np.int32)
+    dst = np.concatenate([(v + 1 + np.arange(d) * 13) % V for v, d in enumerate(deg) if d]).astype(np.int32)
+    hg = ndo.csr_from_records(src, dst, np.ones(len(src), np.float32), V=V)
+    g = nd.Graph.from_csr(hg.row_ptr, hg.col, hg.w, hg.max_w)
+    s = nd.Sampler(g, nd.app_params(app, steps=2, fanout=32, batch=24, seed=3), num_samples=80)
+    p = C.c_void_p()
+    nd.check(nd.lib.nd_graph_hub_slots(g._h, C.byref(p)))
+    shape = {"shape": (V,), "typestr": "<i4", "data": (p.value, False), "version": 3}
+    slot = torch.as_tensor(type("Slots", (), {"__cuda_array_interface__": shape})(), device="cuda").cpu().numpy()
+    order = np.lexsort((np.arange(V), -deg))
+    with_bitmap = order[:1024][deg[order[:1024]] >= 256]
+    assert np.array_equal(np.flatnonzero(slot >= 0), np.sort(with_bitmap))
+    assert np.array_equal(np.sort(slot[slot >= 0]), np.arange(len(with_bitmap)))
+    s.sample()
+    exp = ndo.sample(hg, ndo.make_params(app, steps=2, fanout=32, batch=24, seed=3), 80)
+    assert np.array_equal(s.final_samples(), exp["out"])
