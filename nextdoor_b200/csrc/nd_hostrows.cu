@@ -274,8 +274,10 @@ int nd_sampler_host_update_fetch(nd_sampler *s) {
     if ((size_t)h->total > h->vals_cap) {
       if (h->h_vals) ND_CUDA(cudaFreeHost(h->h_vals));
       h->h_vals = nullptr;
-      h->vals_cap = (size_t)h->total + (size_t)h->total / 4 + 4096;
-      ND_CUDA(cudaMallocHost(&h->h_vals, sizeof(int32_t) * h->vals_cap));
+      h->vals_cap = 0;
+      const size_t cap = (size_t)h->total + (size_t)h->total / 4 + 4096;
+      ND_CUDA(cudaMallocHost(&h->h_vals, sizeof(int32_t) * cap));
+      h->vals_cap = cap;
     }
     ND_CUDA(cudaMemcpyAsync(h->h_vals, s->d_tmp, sizeof(int32_t) * (size_t)h->total, cudaMemcpyDeviceToHost, h->vs));
   }

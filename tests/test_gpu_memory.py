@@ -148,9 +148,39 @@ def adjacency():
     assert np.array_equal(got["adj_row"], expected["adj_row"]) and np.array_equal(got["adj_col"], expected["adj_col"])
 
 
+# pinned memory for the rows of a job (16 MB and more) that the process may not have: the update fails, the next one works
+def pinned_rows():
+    import resource
+    from nextdoor_b200 import api as nd
+    graph = nd.Graph.rmat(1 << 18, 1 << 21, seed=1)
+    S, steps = 1 << 20, 50
+    s = nd.Sampler(graph, nd.app_params(2, steps=steps, seed=2, stop_prob=0.1), num_samples=S)
+    out, row_len = np.full(S * steps, graph.V, np.int32), np.zeros(S, np.int32)
+    seeds = (np.arange(S) % graph.V).astype(np.int32)
+
+    def update(initial):
+        s.set_initial(initial)
+        s.sample(1)
+        s.host_update_begin(out, row_len)
+        s.host_update_fetch()
+        s.host_update_finish()
+
+    update(np.full(S, -1, np.int32))             # no rows: everything but their memory is there
+    old = resource.getrlimit(resource.RLIMIT_AS)
+    pages = int(open("/proc/self/statm").read().split()[0])
+    resource.setrlimit(resource.RLIMIT_AS, (pages * resource.getpagesize() + 8 * MB, old[1]))
+    try:
+        with pytest.raises(nd.NdError, match="memory"):
+            update(seeds)
+    finally:
+        resource.setrlimit(resource.RLIMIT_AS, old)
+    update(seeds)
+    assert np.array_equal(out.reshape(S, steps), s.final_samples())
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("case", [f"first_samplers({app})" for app in (1, 3, 8, 9)]
-                         + [f"graphs_and_partitions('{what}')" for what in ("csr", "partition")] + ["kept_blocks()", "adjacency()"])
+                         + [f"graphs_and_partitions('{what}')" for what in ("csr", "partition")] + ["kept_blocks()", "adjacency()", "pinned_rows()"])
 def test_nothing_stays_behind(case):
     r = subprocess.run([sys.executable, os.path.abspath(__file__), case], capture_output=True, text=True, timeout=300, cwd=ROOT)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
