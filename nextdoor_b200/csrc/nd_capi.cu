@@ -459,7 +459,7 @@ int nd_sampler_next_kernel(const nd_sampler *s, int mode, char *name, int n) {
 
 int nd_sampler_destroy(nd_sampler *s) {
   if (!s) return ND_OK;
-  cudaSetDevice(s->g->device);
+  cudaSetDevice(s->dev.device);   // (not the graph's: garbage collection may have destroyed the graph first)
   cudaStreamSynchronize(s->stream);
   free_sampler(s);
   nd_objects_add(-1);

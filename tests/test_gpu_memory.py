@@ -27,6 +27,25 @@ def test_a_failed_call_does_not_fail_the_next(nd, small_graph, app):
         assert np.array_equal(s.final_samples(), expected)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("app", [0, 4, 9])
+def test_a_graph_destroyed_before_its_sampler(nd, small_graph, app):
+    """As garbage collection does it with a cycle that holds both."""
+    def make():
+        g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+        s = nd.Sampler(g, nd.app_params(app, seed=1), num_samples=50)
+        s.sample()
+        return g, s
+
+    pairs = [make() for _ in range(4)]
+    expected = pairs[0][1].final_samples().copy()
+    for g, _ in pairs:
+        g.free()
+    for _, s in pairs:
+        s.free()
+    assert np.array_equal(make()[1].final_samples(), expected)
+
+
 class Filled:
     """All but about `left` bytes of the device's memory, allocated and never touched."""
 
