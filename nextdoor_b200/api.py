@@ -382,11 +382,15 @@ class PipelinedSampler:
         for j in others:                                  # the lengths of the job before have landed: its vertices
             self._fetch(j)                                # cross while this job is sampled
         row_len = self._rows_of(out_host)
-        for f, n, smp in self.parts:
-            if initial_host is not None:
-                smp.set_initial(initial_host[f * self.isz:(f + n) * self.isz])
-            smp.sample(mode, sync=False)
-            smp.host_update_begin(out_host[f * self.fs:(f + n) * self.fs], row_len[f:f + n], self.copy_stream)
+        try:
+            for f, n, smp in self.parts:
+                if initial_host is not None:
+                    smp.set_initial(initial_host[f * self.isz:(f + n) * self.isz])
+                smp.sample(mode, sync=False)
+                smp.host_update_begin(out_host[f * self.fs:(f + n) * self.fs], row_len[f:f + n], self.copy_stream)
+        except Exception:
+            self._end_updates(k)
+            raise
         self._pending[k] = "begun"
         for j in others:                                  # ... and its rows are written while the device works on this one
             self._finish(j)
@@ -404,8 +408,13 @@ class PipelinedSampler:
 
     def _fetch(self, k):
         if self._pending.get(k) == "begun":
-            for _, _, smp in self.sets[k]:
-                smp.host_update_fetch()
+            try:
+                for _, _, smp in self.sets[k]:
+                    smp.host_update_fetch()
+            except Exception:
+                del self._pending[k]
+                self._end_updates(k)
+                raise
             self._pending[k] = "fetched"
 
     def _finish(self, k):
@@ -413,12 +422,24 @@ class PipelinedSampler:
             fetched = self._pending.pop(k) == "fetched"
             parts = [smp for _, _, smp in self.sets[k]]
             total = 0
-            for i, smp in enumerate(parts):               # a chunk's rows are written while the next one's vertices cross
-                if not fetched:
-                    for ahead in parts[i + 1 if i else 0:i + 2]:
-                        ahead.host_update_fetch()
-                total += smp.host_update_finish()
+            try:
+                for i, smp in enumerate(parts):           # a chunk's rows are written while the next one's vertices cross
+                    if not fetched:
+                        for ahead in parts[i + 1 if i else 0:i + 2]:
+                            ahead.host_update_fetch()
+                    total += smp.host_update_finish()
+            except Exception:
+                self._end_updates(k)
+                raise
             self.values_copied = total
+
+    def _end_updates(self, k):
+        """After an error: no chunk of set k is left with an update that is begun and not finished."""
+        for _, _, smp in self.sets[k]:
+            try:
+                smp.host_update_finish()
+            except NdError:                               # it had none, or it is the one that fails
+                pass
 
     def wait(self):
         for k in list(self._pending):

@@ -106,6 +106,43 @@ def test_rows_packed_at_the_edges_of_a_chunk(nd, small_graph, S, stop):
         assert np.array_equal(host.reshape(S, steps), dense) and np.array_equal(host_len, (dense != V).sum(axis=1))
 
 
+@pytest.mark.parametrize("call", ["host_update_begin", "host_update_fetch", "host_update_finish"])
+@pytest.mark.parametrize("depth", [1, 2])
+def test_a_pipeline_goes_on_after_an_error(nd, small_graph, monkeypatch, call, depth):
+    import torch
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    S, steps = 9001, 30
+    streams = torch.cuda.Stream(), torch.cuda.Stream()
+    params = nd.app_params(2, steps=steps, seed=5, stop_prob=0.2)
+    pipe = nd.PipelinedSampler(g, params, S, chunks=3, depth=depth, sparse_rows=True, stream=streams[0].cuda_stream,
+                               copy_stream=streams[1].cuda_stream)
+    seeds = [np.random.default_rng(k).integers(0, g.V, S).astype(np.int32) for k in range(2)]
+    outs = [np.zeros(S * steps, np.int32) for _ in range(2)]
+    pipe.run(seeds[0], outs[0])
+
+    def failing(smp):
+        def fails(*args):
+            if call == "host_update_finish":      # the update is over all the same
+                type(smp).host_update_finish(smp)
+            raise nd.NdError(2, "no")
+        return fails
+
+    with monkeypatch.context() as m:
+        for parts in pipe.sets:
+            m.setattr(parts[1][2], call, failing(parts[1][2]))
+        with pytest.raises(nd.NdError):
+            for k in (0, 1):
+                pipe.run_async(seeds[1 - k], outs[k])
+            pipe.wait()
+    for k in (0, 1, 1):
+        pipe.run_async(seeds[k], outs[k])
+    pipe.wait()
+    for k in (0, 1):
+        s = nd.Sampler(g, params, num_samples=S, initial=seeds[k])
+        s.sample()
+        assert np.array_equal(outs[k].reshape(S, steps), s.final_samples())
+
+
 @pytest.mark.parametrize("app", [6, 8, 9])
 @pytest.mark.parametrize("L,B,S", [(48, 50, 70), (7, 5, 2675), (1, 3, 43_691), (64, 64, 33)])
 def test_adjacency_crosses_as_bits(nd, ndo, small_graph, app, L, B, S):
