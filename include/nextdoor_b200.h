@@ -213,7 +213,9 @@ int nd_sampler_phase_ms(nd_sampler *s, float *ms, int32_t *launches, int n);
 /* Name of the next() kernel (for walks: with the app) that nd_sampler_sample(s, mode) launches: the
  * reference picks its kernels by kernelType and the load-balancing flag (src/nextdoor.cu:2400-2928),
  * this library also by app, graph size and its environment switches, so a measurement can label
- * itself with what ran.  `name` receives at most n bytes including the terminator. */
+ * itself with what ran.  `name` receives at most n bytes including the terminator.  The sample-parallel
+ * mode of walks is reported as walk_sp_kernel: the kernel of the load-balanced mode, walk_next_count_kernel,
+ * without the count of live walks. */
 int nd_sampler_next_kernel(const nd_sampler *s, int mode, char *name, int n);
 /* freeDeviceData (src/nextdoor.cu:2088-2115) */
 int nd_sampler_destroy(nd_sampler *s);

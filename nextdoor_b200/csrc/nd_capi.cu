@@ -442,7 +442,7 @@ int nd_sampler_next_kernel(const nd_sampler *s, int mode, char *name, int n) {
   const int app = s->p.app;
   if (nd_is_walk(app)) {
     const char *k = mode == ND_MODE_TRANSIT_PARALLEL ? "walk_next_tp_kernel"
-                    : mode == ND_MODE_SAMPLE_PARALLEL ? "walk_sp_kernel"
+                    : mode == ND_MODE_SAMPLE_PARALLEL ? "walk_sp_kernel"   // (walk_next_count_kernel, not counting)
                     : nd_walk_step_loop(s) ? "walk_next_ticket_kernel" : "walk_next_count_kernel";
     snprintf(name, (size_t)n, "%s<%s>", k, walk_app[app]);
   } else if (nd_is_khop(app)) {

@@ -598,11 +598,7 @@ __device__ __forceinline__ void walks(const RowsArgs &a) {
   else weighted_walks<APP, LAYOUT>(a);
 }
 
-// the sample-parallel mode
-template <int APP, int LAYOUT>
-__global__ void __launch_bounds__(ROWS_THREADS, ROWS_CTAS) walk_sp_kernel(const RowsArgs a) { walks<APP, LAYOUT>(a); }
-
-// the load-balanced mode: the same walks, and the walks that are alive at every step are counted
+// Both modes; the load-balanced one also counts the walks that are alive at every step (RowsArgs::ended).
 template <int APP, int LAYOUT>
 __global__ void __launch_bounds__(ROWS_THREADS, ROWS_CTAS) walk_next_count_kernel(const RowsArgs a) { walks<APP, LAYOUT>(a); }
 
@@ -709,8 +705,7 @@ void launch(nd_sampler *s, RowsArgs &a, bool count) {
   } else {
     a.list = nullptr;
   }
-  if (count) walk_next_count_kernel<APP, LAYOUT><<<grid, ROWS_THREADS, smem, s->stream>>>(a);
-  else walk_sp_kernel<APP, LAYOUT><<<grid, ROWS_THREADS, smem, s->stream>>>(a);
+  walk_next_count_kernel<APP, LAYOUT><<<grid, ROWS_THREADS, smem, s->stream>>>(a);
   nd_count_launches(1);
 }
 
