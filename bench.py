@@ -17,8 +17,9 @@ c2) gives the roofline of the transit-parallel next() kernel the target is state
 (`c2_next_roofline`), and on one GPU the reference's own GPU build is timed on the same c2 graph
 (`reference_gpu`) when its binaries are present.
 
-Prints ONE JSON line (rank 0).  --impl reference times the reference's own next() bodies on the
-host cores (oracle/_ref, else the oracle port) on a bounded sample of the same workload.
+Prints ONE JSON line (rank 0).  --impl reference prints why the reference cannot be run here; the same
+workload on the host cores (the reference's own next() bodies of oracle/_ref where they exist for it,
+else the oracle port, on a bounded sample) is `cpu_baseline`.
 """
 from __future__ import annotations
 
@@ -331,55 +332,16 @@ def partitioned_bench(a, wl, nd, torch, rank, world, local, seed):
         dist.destroy_process_group()
 
 
-def reference_arm(a, wl, seed):
-    """--impl reference: the reference's next() bodies (oracle/_ref) or the oracle port on all host
-    threads, each step a bounded prefix of the workload's samples."""
-    from oracle import ndo
-    V, M = wl["V"], wl["M"]
-    t0 = time.perf_counter()
-    hg = host_graph_cached(ndo, V, M, seed)   # same generator definition as the device one
-    t_graph = time.perf_counter() - t0
-    vals = []
-    for i in range(a.warmup + a.steps):
-        cb = cpu_baseline(hg, wl, seed, budget_s=6.0)
-        if i >= a.warmup:
-            vals.append(cb)
-    v = float(np.mean([c["value"] for c in vals]))
-    cb = dict(vals[-1], value=v)
-    print(json.dumps({
-        "impl": "reference", "metric": "sampled edges/sec", "value": v, "unit": "sampled edges/s", "n_gpus": a.gpus,
-        "steps": a.steps, "warmup": a.warmup, "ms_per_step": 1e3 * float(np.mean([c["seconds"] for c in vals])),
-        "higher_is_better": True, "scaling": "strong",
-        "vs_baseline": None, "dtype": "int32", "data": "synthetic",
-        "config": {"workload": f"{a.workload}: {wl['desc']}", "host_graph_build_s": round(t_graph, 2)},
-        "cpu_baseline": cb, "e2e": {"value": v, "unit": "sampled edges/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}))
-
-
-def host_graph_cached(ndo, V, M, seed):
-    """The oracle's R-MAT graph on the host.  Building the 2^24-vertex graph takes minutes on the
-    host cores and the driver runs this arm once per GPU count, so the arrays are kept in the
-    system's temporary directory between runs of one box."""
-    import tempfile
-    if M < (1 << 26):
-        return ndo.rmat_graph(V, M, seed)
-    d = os.path.join(tempfile.gettempdir(), f"nd_b200_rmat_{V}_{M}_{seed}")
-    names = ("row_ptr", "col", "w", "max_w")
-    try:
-        if os.path.exists(os.path.join(d, "done")):
-            arrs = [np.load(os.path.join(d, n + ".npy")) for n in names]
-            if arrs[0].shape[0] == V + 1 and arrs[1].shape[0] == int(arrs[0][-1]):
-                return ndo.HostGraph(*arrs)
-    except Exception:
-        pass
-    hg = ndo.rmat_graph(V, M, seed)
-    try:
-        os.makedirs(d, exist_ok=True)
-        for n in names:
-            np.save(os.path.join(d, n + ".npy"), getattr(hg, n))
-        open(os.path.join(d, "done"), "w").close()
-    except Exception:
-        pass
-    return hg
+def reference_arm(wl):
+    """--impl reference.  The reference draws on GPUs only: it has no CPU sampler, its GPU programs are built from its
+    source tree, and it has no package to install.  What this repository has in its place (the oracle on the host
+    cores) is its own code and is reported as `cpu_baseline` of the main line, not as the reference."""
+    why = "the reference has no CPU sampler and no installable package, and its GPU programs are not built here"
+    if wl["app"] == 2 and abs(wl.get("stop_prob", 0.01) - 0.01) > 1e-9:
+        why += f"; its PPR stops with a fixed probability of 0.01 (randomWalks.cu:105), not this workload's {wl['stop_prob']}"
+    elif wl["app"] in (5, 8, 9):
+        why += "; it does not implement this workload's application"
+    print(json.dumps({"impl": "reference", "unavailable": why}))
 
 
 def next_kernel_name(nd, smp, mode):
@@ -533,7 +495,7 @@ def main():
 
     if a.impl == "reference":
         if rank == 0:
-            reference_arm(a, wl, seed)
+            reference_arm(wl)
         return
 
     import torch
