@@ -150,9 +150,14 @@ def test_adjacency_crosses_as_bits(nd, ndo, small_graph, app, L, B, S):
     s = nd.Sampler(g, nd.app_params(app, steps=2, fanout=L, batch=B, seed=6), num_samples=S)
     s.sample()
     exp = ndo.sample(small_graph, ndo.make_params(app, steps=2, fanout=L, batch=B, seed=6), S)
-    if np.array_equal(s.final_samples(), exp["out"]) or app == 6:   # (importance: a draw on an edge may fall to its neighbour)
-        aux = s.aux()
-        assert np.array_equal(aux["adj_row"], exp["adj_row"]) and np.array_equal(aux["adj_col"], exp["adj_col"])
+    same = (s.final_samples() == exp["out"]).all(axis=1)
+    # LADIES: a draw on the edge of an interval may fall to its neighbour.  The sums agree to 1e-16 and a draw has 32
+    # bits, so of S * 2 * L draws (at most 87,382) less than one in a thousand runs of this test has even one
+    assert (~same).sum() <= (1 if app == 9 else 0)
+    aux = s.aux()
+    for k in ("adj_row", "adj_col"):
+        assert np.array_equal(aux[k].reshape(S, -1)[same], exp[k].reshape(S, -1)[same])
+    assert (aux["adj_row"] >= 0).sum() > 0
 
 
 def test_results_own_their_memory(nd, small_graph):
