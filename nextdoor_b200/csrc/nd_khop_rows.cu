@@ -24,7 +24,9 @@ constexpr int ROW_MAX = 4096;        // longest row that is kept in shared memor
 
 // CTAs of 256 per SM (registers): measured 4 / 5 / 6 / 8 on 262,144 seeds, 25 x 10, 2^21 vertices: with
 // replacement 0.403 / 0.396 / 0.428 / 0.526 ms, without 0.548 / 0.524 / 0.500 / 0.498
-__host__ __device__ constexpr int khop_ctas(bool distinct) { return distinct ? 6 : 5; }
+constexpr int CTAS = 5;
+constexpr int CTAS_DISTINCT = 6;
+__host__ __device__ constexpr int khop_ctas(bool distinct) { return distinct ? CTAS_DISTINCT : CTAS; }
 
 struct KhopRows {
   uint64_t seed;

@@ -1,4 +1,5 @@
 import os
+import re
 import sys
 
 import numpy as np
@@ -11,6 +12,18 @@ if ROOT not in sys.path:
 
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (run on the B200 box)")
+
+
+def kernel_constant(source, name):
+    """The value of an integer constant of a kernel file: tests at the edge of a launch's size read it where it is set."""
+    text = open(os.path.join(ROOT, "nextdoor_b200", "csrc", source)).read()
+    return int(re.search(rf"constexpr int {name} = (\d+);", text).group(1))
+
+
+def sm_count():
+    """148 on a B200; the tests' parameters are collected where there is no GPU, too."""
+    import torch
+    return torch.cuda.get_device_properties(0).multi_processor_count if torch.cuda.is_available() else 148
 
 
 @pytest.fixture(scope="session")

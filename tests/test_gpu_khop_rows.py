@@ -3,8 +3,11 @@ beyond what a warp sorts in registers, rows too long for shared memory, fewer an
 import numpy as np
 import pytest
 
+from conftest import kernel_constant, sm_count
+
 pytestmark = pytest.mark.gpu
-WARPS = 148 * 40                 # resident warps of one B200 (with replacement)
+# resident warps of the GPU, by app
+WARPS = {app: sm_count() * 8 * kernel_constant("nd_khop_rows.cu", name) for app, name in ((4, "CTAS"), (5, "CTAS_DISTINCT"))}
 
 
 def _compare(nd, ndo, hg, app, fanout, S, seed=3, modes=(1, 2)):
@@ -29,9 +32,9 @@ def test_fanouts(nd, ndo, small_graph, app, fanout):
 
 
 @pytest.mark.parametrize("app", [4, 5])
-@pytest.mark.parametrize("S", [1, 4, 5, WARPS - 1, WARPS + 1, 17 * WARPS])
-def test_sample_counts(nd, ndo, small_graph, app, S):
-    _compare(nd, ndo, small_graph, app, [3, 2], S)
+@pytest.mark.parametrize("warps,more", [(0, 1), (0, 4), (0, 5), (1, -1), (1, 1), (16, 1), (17, 0)])
+def test_sample_counts(nd, ndo, small_graph, app, warps, more):
+    _compare(nd, ndo, small_graph, app, [3, 2], warps * WARPS[app] + more)
 
 
 def test_rows_beyond_shared_memory(nd, ndo, small_graph):

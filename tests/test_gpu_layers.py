@@ -45,7 +45,7 @@ def test_a_sampler_keeps_the_layout_it_was_created_with(nd, monkeypatch, small_g
     assert np.array_equal(out[0], out[1])
 
 
-@pytest.mark.parametrize("app,sizes", [(8, [(16, 16), (600, 600)]), (9, [(16, 16), (600, 600)]), (7, [(600, 600), (1000, 1000)]), (4, [(16, 15, 13), (15, 15, 17)])])
+@pytest.mark.parametrize("app,sizes", [(8, [(16, 16), (600, 600)]), (9, [(16, 16), (600, 600)]), (7, [(560, 560), (640, 640)]), (4, [(16, 15, 13), (15, 15, 17)])])
 def test_threads_with_different_shared_memory(nd, small_graph, app, sizes):
     """The limit of a kernel's dynamic shared memory is the kernel's: a thread that launches with little must not lower
     it under another's launch."""
@@ -60,7 +60,7 @@ def test_threads_with_different_shared_memory(nd, small_graph, app, sizes):
 
     def work(s):
         try:
-            for _ in range(1500):
+            for _ in range(300 if app == 7 else 1500):
                 s.sample(sync=False)
             s.sync()
         except nd.NdError as e:

@@ -4,8 +4,11 @@ decides nothing, rows that shrink and grow between passes."""
 import numpy as np
 import pytest
 
+from conftest import kernel_constant, sm_count
+
 pytestmark = pytest.mark.gpu
-LANES = 148 * 12 * 128          # resident lanes of one B200
+# resident lanes of the GPU
+LANES = sm_count() * kernel_constant("nd_walk_rows.cu", "ROWS_CTAS") * kernel_constant("nd_walk_rows.cu", "ROWS_THREADS")
 
 
 def _graph(nd, hg):
