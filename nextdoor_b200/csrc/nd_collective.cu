@@ -56,7 +56,8 @@ static RefLayout ref_layout(int steps, int B, int L) {
   RefLayout r;
   const int ntr = B > L ? B : L;
   r.flag_words = (L + 31) / 32;
-  for (r.per_pass = steps;; r.per_pass--) {
+  // (a layer's filter is a kilobyte: no more than 24 of them fit, and the sums below stay in 32 bits)
+  for (r.per_pass = std::min(steps, 24);; r.per_pass--) {
     const uint32_t k = (uint32_t)r.per_pass, nt = k * (uint32_t)ntr;
     uint32_t off = 0;
     r.off_ids = off; off += 4u * (k + 1u) * (uint32_t)L;   // the layer before the pass too: its transits

@@ -103,3 +103,15 @@ def test_bitmaps_go_to_the_vertices_with_the_most_neighbours(nd, ndo, app, kind,
     s.sample()
     exp = ndo.sample(hg, ndo.make_params(app, steps=2, fanout=32, batch=24, seed=3), 80)
     assert np.array_equal(s.final_samples(), exp["out"])
+
+
+@pytest.mark.parametrize("steps", [23, 24, 25, 4_098_254])
+def test_reference_layers_of_many_steps(nd, ndo, small_graph, steps):
+    """The bytes of the last one's layers, all in one pass, are 2904 beyond 2^32."""
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    s = nd.Sampler(g, nd.app_params(6, steps=steps, fanout=1, batch=1, seed=3), num_samples=1)
+    s.sample()
+    exp = ndo.sample(small_graph, ndo.make_params(6, steps=steps, fanout=1, batch=1, seed=3), 1)
+    aux = s.aux()
+    assert np.array_equal(s.final_samples(), exp["out"])
+    assert np.array_equal(aux["adj_row"], exp["adj_row"]) and np.array_equal(aux["adj_col"], exp["adj_col"])
