@@ -7,10 +7,13 @@
 // integer weights sum exactly).
 //
 // What bounds it, and what is done about it (2^20 vertices, 1024 batches of 64, 2 layers of 64: FastGCN
-// 4.8 -> 0.98 ms, LADIES 5.7 -> 2.44 ms):
+// 4.8 -> 0.98 ms, LADIES 5.7 -> 2.44 ms).  One CTA fills an SM, and neither memory nor issue slots are full: FastGCN issues
+// in 58 % of the cycles (612 M warp instructions; 5.6 GB out of the L2 at 24 % of its rate), LADIES in 46 % (1.09 G
+// instructions for 131 M list entries, the distinct ones of 313 M); the warps wait for barriers between the phases, for
+// shared memory and for loads:
 //  * The second layer's transits are hubs (FastGCN draws them with the square of their degree), many of them the
 //    same one: repeated transits of a batch are taken once (LADIES with their multiplicity).
-//  * A hub's list (up to 140 K ids) costs a shared-memory test per id.  Vertices with at least V/128 neighbours
+//  * A hub's list (up to 140 K ids; FastGCN's second layer has 28 distinct hubs a sample) costs a shared-memory test per id.  Vertices with at least V/128 neighbours
 //    have their neighbourhood as a bitmap, built once per graph: V/8 bytes that are ORed in registers, word by
 //    word, and stored to the union once; and an adjacency probe of such a transit is a bit test.
 //  * FastGCN's weights are summed without a list of candidates (writing that and fetching deg^2 one by one took more
@@ -42,9 +45,10 @@ constexpr int VEC = 4;            // 16-byte loads in flight per thread
 constexpr int CHUNK = 128;        // list entries a warp takes at a time (LADIES)
 constexpr int CHUNK_LOADS = CHUNK / 32;
 
-// The bitmap, the counts of groups and quads of words and the CDF make the "big" part (V/8 + 5V/128 bytes); it lives in shared memory when the whole layout fits the CTA's opt-in shared memory (graphs up
-// to about 1.2 M vertices) and otherwise in a per-CTA slice of a global scratch array (glob_bytes > 0), where the
-// same code runs on L2-resident words.  The rest is always in shared memory.
+// The bitmap, the counts of groups and quads of words and the CDF make the "big" part (V/8 + 5V/128 bytes).  It lives in
+// shared memory when the whole layout fits the CTA's opt-in shared memory (graphs up to about 1.2 M vertices) and
+// otherwise in a per-CTA slice of a global scratch array (glob_bytes > 0), where the same code runs on L2-resident
+// words.  The rest is always in shared memory.
 struct Layout {
   int words, groups;
   uint32_t off_gcdf, off_gpref, off_qpre;              // inside the big part (the bitmap is at 0)
@@ -606,8 +610,8 @@ __global__ void hub_bits_kernel(const int32_t *__restrict__ row_ptr, const int32
 int words_of(int32_t V) { return (int)((((int64_t)V + 31) / 32 + GROUP_WORDS - 1) / GROUP_WORDS * GROUP_WORDS); }
 
 // A bitmap pays against the list it replaces from about V/128 neighbours: four times the list's bytes, but ORed a word
-// at a time (FastGCN from V/64, V/128, V/192: 1.14, 0.98, 0.99 ms with 1024 batches on 2^20 vertices, 0.83, 0.59, 0.59 with 256 on
-// 2^21).
+// at a time (FastGCN from V/64, V/128, V/192: 1.14, 0.98, 0.99 ms with 1024 batches on 2^20 vertices, 0.83, 0.59, 0.59
+// with 256 on 2^21).
 // At most HUBS of them, those with the most neighbours: a graph can hold 128 E / V such vertices.  (1024 batches on 233 K
 // vertices and 114 M entries: FastGCN 4.1 ms with the 1024 that came first, 0.79 with the largest; LADIES, which goes
 // through the lists again, 22.6 and 21.7.  Finding the rank adds 1.2 ms to the first sampler of such a graph.)

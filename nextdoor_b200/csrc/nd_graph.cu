@@ -352,8 +352,10 @@ int build_scratch(BuildScratch *s, int device, int64_t n) {
 }
 
 // records in bs->a (weights as keys) -> graph; key bits outside [lo_bit, hi_bit) are the same in all records.  They are
-// sorted by dst, then src, and the few that share both by weight where they lie (10 passes over random edges with
-// random weights -> 6; 8.4M records on the host to a graph, copies included: 6.1 ms -> 4.9; 3.7 with the scatter of nd_radix.cu).  A graph that repeats one edge thousands of times goes on to the full sort.
+// sorted by dst, then src, and the few that share both by weight where they lie: 6 passes instead of 10 over random edges
+// with random weights (8.4M records on the host to a graph, copies included: 6.1 ms -> 4.9; 4.0 since the scatter of
+// nd_radix.cu, of it 0.89 on the device: the passes 0.11 each).  A graph that repeats one edge thousands of times goes
+// on to the full sort.
 int build_from_soa(const NdDeviceInfo &dev, int64_t n, int32_t V, BuildScratch *bs, int lo_bit, int hi_bit, nd_graph **out) {
   ND_REQUIRE(n < ((int64_t)1 << 31), ND_ERR_RANGE, "%lld edges do not fit the int32 edge index of the CSR", (long long)n);
   const int vbits = nd_bit_length((uint32_t)(V > 1 ? V - 1 : 1));

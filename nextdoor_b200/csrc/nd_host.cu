@@ -4,7 +4,8 @@
 // thread copies to or from its own pinned buffer, and faults in a fresh destination page by page); PCIe moves
 // 53-55.  Here the pieces of a large copy go through a ring of pinned buffers that several workers fill or empty
 // at once: 31-36 GB/s up and into memory that is there, 15-20 into fresh pages (pieces of 512 KB 27, of 1 MB 31;
-// non-temporal stores and a second stream gain nothing).  One copy at a time uses the ring; a second one, and small ones, take the plain call.
+// non-temporal stores and a second stream gain nothing).  One copy at a time uses the ring; a second one, and small
+// ones, take the plain call.
 #include "nd_host.h"
 
 #include <stdlib.h>
@@ -256,8 +257,8 @@ int staged(const std::vector<Segment> &segments, size_t bytes, bool up) {
       if (k < pieces && movable(k) && next.compare_exchange_strong(k, k + 1)) move(k);
     }
   };
-  // Four keep up with the wire (100 MB up: 2.8 ms; 3.3 with three or eight, 3.3 with pieces of 1 MB); a large destination is likely to be fresh memory, where more of them share the page
-  // faults (15 -> 25 GB/s), but take longer to wake.
+  // Four keep up with the wire (100 MB up: 2.8 ms; 3.3 with three or eight, 3.3 with pieces of 1 MB).  A large destination
+  // is likely to be fresh memory, where more of them share the page faults (15 -> 25 GB/s), but take longer to wake.
   const size_t want = !up && bytes >= FRESH ? 12 : 4;
   const int movers = (int)std::min<size_t>(std::min<size_t>(pieces, want), (size_t)std::max(1, nd_host_threads() - 1));
   nd_host_run(movers, [&](int) { mover(); }, [&] {

@@ -34,8 +34,8 @@ int nd_adjacency_to_host(int device, const uint32_t *bits, int64_t entries, int 
 
 // Device memory for building graphs.  Blocks of up to 384 MB are kept for the next build when they are freed, 1 GB of
 // them in all, while graphs or samplers are alive (a cudaMalloc / cudaFree pair costs 0.5 to 30 ms, by the box); an
-// allocation of the library that would fail gives all of them back first.  `bytes`: in: at least, out: what the block has.  The release
-// waits for the device, as cudaFree does.
+// allocation of the library that would fail gives all of them back first.  `bytes`: in: at least, out: what the block
+// has.  The release waits for the device, as cudaFree does.
 int nd_block_alloc(int device, void **p, size_t *bytes);
 void nd_block_free(int device, void *p, size_t bytes);
 

@@ -8,9 +8,10 @@
 // (src/apps/khop/khop.cu:10-23); ND_APP_KHOP_DISTINCT without replacement, every hop sorted and made unique at
 // the end (src/distinct.cuh:1-111).  A warp writes its row at the end.
 // What bounds it: with replacement, gathers of 4 bytes from the adjacency array at the rate of random DRAM
-// reads (262,144 seeds, 25 x 10, 2^21 vertices: 0.89 ms transit-parallel -> 0.36); without, the instructions
-// of the draws and of the sort (1.15 -> 0.49 ms); a mini-batch of 1024, the chain seed -> row -> neighbours ->
-// rows -> neighbours (74 -> 12 us with the seeds' copy).
+// reads (262,144 seeds, 25 x 10, 2^21 vertices: 0.89 ms transit-parallel -> 0.36); without (1.15 -> 0.49 ms), the
+// instructions: 341 M of a warp, 0.29 ms at one per cycle and scheduler, and of the 18 cycles from one to the next 5.5 are
+// spent waiting for the next instruction to be fetched, 2.6 for memory and 2.5 for shared memory (DRAM 34 %); a mini-batch
+// of 1024, the chain seed -> row -> neighbours -> rows -> neighbours (74 -> 12 us with the seeds' copy).
 #include "nd_common.cuh"
 #include "nd_khop_rows.cuh"
 #include "nd_philox.cuh"

@@ -6,13 +6,15 @@
 // 5.2 -> 1.6 ms, node2vec 7.6 -> 2.3 ms, PPR on 2^24 vertices 5.4 -> 2.5 ms).
 //
 // What bounds it.  Large graphs: the rate of random DRAM reads.  A walker picks every CSR entry with the same
-// probability, the entry arrays do not fit the L2, and a gather of 4 or 8 bytes costs a 64-byte DRAM read; the
-// kernels run at 4.1-5.0 TB/s of such reads (58-66 % of the pins; streaming copies reach 6.5).  So what
+// probability, the entry arrays do not fit the L2, and a gather of 4 or 8 bytes costs a 64-byte DRAM read; on 2^20
+// vertices the kernels move 5.2 (node2vec), 5.0 (DeepWalk) and 4.8 TB/s (uniform walk), 59-63 % of the pins, PPR on 2^22
+// vertices 4.0 (49 %); a streaming copy reaches 6.5.  So what
 // counts is the number of gathers that miss, hence: one try per round for the weighted apps (no speculation),
 // the weights as one byte per entry where that array has a chance to stay in the L2, the first stop draw of
 // a step made before the vertex is fetched, a filter in front of node2vec's sets, rows written once, in
-// 32-byte sectors.  Small graphs: the chain of dependent L2 reads of a walk, two per step, one where the
-// entries carry the neighbour's row.
+// 32-byte sectors.  Small graphs: the chain of a walk, two dependent L2 reads per step, one where the entries carry the
+// neighbour's row, and the instructions between them (57 K vertices: a step is 0.5 us, 121 instructions of a warp at 8.2
+// cycles each, 45 % of them waiting for the read).
 #include <mutex>
 
 #include "nd_common.cuh"
