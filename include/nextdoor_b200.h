@@ -79,7 +79,8 @@ int64_t nd_launch_count(void);
 
 /* transferCSRToGPUs / copyPartitionToGPU (src/nextdoor.cu:1893-1911, src/utils.hpp:378-395):
  * upload a host CSR.  row_ptr has V+1 entries with exclusive ends; max_w may be NULL (computed
- * on the device as Vertex::max_weight does, src/graph.hpp:71-80). */
+ * on the device as Vertex::max_weight does, src/graph.hpp:71-80).  The ids of a row may come in any order; the adjacency
+ * entries of the layer apps, which are found by bisection as in src/csr.hpp:343-359, need them ascending. */
 int nd_graph_from_csr(int device, int32_t V, int64_t E, const int32_t *row_ptr, const int32_t *col,
                       const float *w, const float *max_w, nd_graph **out);
 /* Graph::load_from_edge_list_binary + csr_from_graph (src/graph.hpp:106-159, src/csr.hpp:399-424),

@@ -23,7 +23,8 @@
 //  * LADIES' terms (w / rowsum)^2 depend on the edge alone: an array, built once per graph, instead of a pass over
 //    the weights and a division per entry and sample.  They are added up in shared memory, in tiles of
 //    consecutive candidates (lists are sorted, so a tile is a range of every list, all of them searched for at
-//    once), not with atomics on global memory.
+//    once), not with atomics on global memory.  CSR arrays of a caller may hold rows in any order: those lists are gone
+//    through whole for every tile.
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
@@ -70,6 +71,7 @@ struct Args {
   float *wts_all;                          // LADIES: [CTAs][V] the candidates' weights, in order
   int32_t *pos_all;                        // LADIES: [CTAs][tiles + 1][transits] where the tiles begin in the lists
   int pos_stride;                          // ... entries per CTA
+  int sorted;                              // LADIES: the lists ascend, so that a tile is a range of each
   int32_t *adj_row, *adj_col;
   float *prob;
   const uint4 *__restrict__ deg;           // FastGCN: the degrees of eight vertices, low bytes (x, y), high bytes (z, w)
@@ -336,7 +338,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
         auto transit = [&](int i) -> const Transit & { return ut[i < nh ? i : cp.ntr - nu + i]; };
         int32_t *sh_pos = sh_mult;   // not needed any more
         const int tiles = (int)((U + lay.tile - 1) / lay.tile);
-        for (int q = tid; q < (tiles + 1) * nu; q += blockDim.x) {   // where every tile begins in every list
+        for (int q = tid; a.sorted && q < (tiles + 1) * nu; q += blockDim.x) {   // where every tile begins in every list
           const int k = q / nu, i = q - k * nu;
           const Transit t = transit(i);
           int32_t e = t.rs;
@@ -350,9 +352,10 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
           __syncthreads();
           for (uint32_t r = tid; r < n; r += blockDim.x) tile[r] = 0.0;
           for (int i = tid; i < nu; i += blockDim.x) {
-            const int32_t at = __ldcg(pos + i);
+            // (lists in another order are gone through whole for every tile)
+            const int32_t at = a.sorted ? __ldcg(pos + i) : transit(i).rs;
             sh_pos[i] = at;
-            pre[i] = (uint32_t)(__ldcg(pos + nu + i) - at);
+            pre[i] = a.sorted ? (uint32_t)(__ldcg(pos + nu + i) - at) : (uint32_t)transit(i).deg;
           }
           __syncthreads();
           const uint32_t total = scan_u32(pre, nu, red_u);
@@ -388,7 +391,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
                 r += in_quad > 2 ? __popc(q.z) : 0;
                 const uint32_t own = in_quad == 0 ? q.x : in_quad == 1 ? q.y : in_quad == 2 ? q.z : q.w;
                 r += __popc(own & ((1u << (v[j] & 31)) - 1u));
-                atomicAdd(tile + (r - r0), (double)x[j] * (double)m[j]);
+                if (r - r0 < n) atomicAdd(tile + (r - r0), (double)x[j] * (double)m[j]);
               }
           }
           __syncthreads();
@@ -565,6 +568,13 @@ rowsum_build_kernel(const int32_t *__restrict__ row_ptr, const float *__restrict
 }
 
 __global__ void __launch_bounds__(BUILD_THREADS)
+unsorted_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col, int32_t V, int64_t E, int *__restrict__ unsorted) {
+  for_entries(row_ptr, V, E, [&](int64_t e, int32_t v) {
+    if (e + 1 < (int64_t)row_ptr[v + 1] && col[e] > col[e + 1]) *unsorted = 1;
+  });
+}
+
+__global__ void __launch_bounds__(BUILD_THREADS)
 term_build_kernel(const int32_t *__restrict__ row_ptr, const float *__restrict__ w, const double *__restrict__ sum, int32_t V, int64_t E,
                   float *__restrict__ term) {
   for_entries(row_ptr, V, E, [&](int64_t e, int32_t v) {
@@ -680,9 +690,18 @@ int ensure_degrees(const nd_graph *g, int grid) {
   return ND_OK;
 }
 
-// LADIES: the terms of the entries
+// LADIES: the terms of the entries, and whether the rows ascend
 int ensure_terms(const nd_graph *g, int grid) {
   if (g->term) return ND_OK;
+  if (g->rows_sorted < 0) {
+    NdDevMem<int> flag;
+    int unsorted = 0;
+    ND_TRY(flag.alloc(1));
+    ND_CUDA(cudaMemset(flag.p, 0, sizeof(int)));
+    unsorted_kernel<<<grid, BUILD_THREADS>>>(g->row_ptr, g->col, g->V, g->E, flag.p);
+    ND_CUDA(cudaMemcpy(&unsorted, flag.p, sizeof(int), cudaMemcpyDeviceToHost));
+    g->rows_sorted = unsorted ? 0 : 1;
+  }
   NdDevMem<float> term;
   NdDevMem<double> sum;
   ND_TRY(term.alloc((size_t)(g->E > 0 ? g->E : 1)));
@@ -791,7 +810,7 @@ int nd_coll_bitmap_launch(nd_sampler *s, const CollParams &cp, unsigned long lon
   const Plan p = plan_of(s);
   const nd_graph *g = s->g;
   const Args a{nd_view(g), cp, s->p.steps, s->S, p.lay, s->d_bm, s->d_initial, s->d_out, s->d_cand_w,
-               s->d_runs, ladies ? pos_entries(s, p.lay) : 0, s->d_adj_row, s->d_adj_col, s->d_prob,
+               s->d_runs, ladies ? pos_entries(s, p.lay) : 0, g->rows_sorted, s->d_adj_row, s->d_adj_col, s->d_prob,
                g->deg_codes, g->big, g->n_big, g->term, g->hub_slot, g->hub_bits, s->d_rows_acc, s->d_stats, pairs};
   if (ladies) coll_bitmap_kernel<true><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
   else coll_bitmap_kernel<false><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);

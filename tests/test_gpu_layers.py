@@ -115,3 +115,24 @@ def test_reference_layers_of_many_steps(nd, ndo, small_graph, steps):
     aux = s.aux()
     assert np.array_equal(s.final_samples(), exp["out"])
     assert np.array_equal(aux["adj_row"], exp["adj_row"]) and np.array_equal(aux["adj_col"], exp["adj_col"])
+
+
+@pytest.mark.parametrize("V,M,B,L", [(2000, 12_000, 24, 32), (60_000, 3_000_000, 500, 64)])
+@pytest.mark.parametrize("scratch", ["0", "1"])
+@pytest.mark.parametrize("app", [8, 9])
+def test_rows_in_any_order(nd, monkeypatch, app, scratch, V, M, B, L):
+    """CSR arrays of a caller whose rows do not ascend have the layers of the same graph with rows that do."""
+    monkeypatch.setenv("ND_COLLECTIVE_BITMAP_GLOBAL", scratch)
+    row_ptr, col, w, max_w = nd.Graph.rmat(V, M, seed=1).to_host()
+    rng = np.random.default_rng(V)
+    order = np.lexsort((rng.random(len(col)), np.repeat(np.arange(V), np.diff(row_ptr))))
+    init = rng.integers(0, V, 40 * B).astype(np.int32)
+    out = []
+    for c, x in ((col, w), (col[order], w[order])):
+        s = nd.Sampler(nd.Graph.from_csr(row_ptr, c, x, max_w), nd.app_params(app, steps=2, fanout=L, batch=B, seed=3), num_samples=40, initial=init)
+        s.sample()
+        out.append((s.final_samples(), s.aux()["prob"], s.stats()["union_unique"]))
+    assert V < 16_384 or out[0][2] / 80 > 16_384        # more candidates than an accumulator tile holds
+    # the row sums are added up in another order, to 1e-16: less than one draw in 10^9 can fall to its neighbour for it
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][2] == out[1][2]
+    assert np.allclose(out[0][1], out[1][1], rtol=1e-6, atol=0)
