@@ -151,8 +151,9 @@ def test_adjacency_crosses_as_bits(nd, ndo, small_graph, app, L, B, S):
     s.sample()
     exp = ndo.sample(small_graph, ndo.make_params(app, steps=2, fanout=L, batch=B, seed=6), S)
     same = (s.final_samples() == exp["out"]).all(axis=1)
-    # LADIES: a draw on the edge of an interval may fall to its neighbour.  The sums agree to 1e-16 and a draw has 32
-    # bits, so of S * 2 * L draws (at most 87,382) less than one in a thousand runs of this test has even one
+    # LADIES: a draw on the edge of an interval may fall to its neighbour.  The oracle adds a candidate's terms up in 32
+    # bits, each sum off by up to 6e-8 of itself, so that the edges lie about 1e-6 of the whole apart in all: of the
+    # S * 2 * L draws (at most 87,382) 0.1 is expected to differ
     assert (~same).sum() <= (1 if app == 9 else 0)
     aux = s.aux()
     for k in ("adj_row", "adj_col"):
