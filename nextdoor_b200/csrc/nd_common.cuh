@@ -118,9 +118,9 @@ struct nd_graph {
   mutable int2 *colw = nullptr;        // [E] (neighbour id, weight bits) records: one 8-byte gather per weighted try
   mutable int2 *vrec = nullptr;        // [V+1] (row start, max weight bits) per vertex: what a thread-per-walk kernel needs of a vertex in one sector
   mutable int2 *vrow = nullptr;        // [V] (row start, degree): one load per vertex
-  mutable int4 *vrec4 = nullptr;       // [V] (row start, degree, max weight bits, 0)
   mutable int4 *erec = nullptr;        // [E] (neighbour id, its row start, its degree, 0)
-  mutable uint8_t *wq = nullptr;       // [E] weights as whole 256ths of the row's maximum
+  mutable uint32_t *pack = nullptr;    // [E] neighbour id << 8 | weight as whole 256ths of the row's maximum
+  mutable int odd_max = -1;            // some row's maximum weight rules `pack` out (-1: not asked yet)
   mutable int32_t *adjset = nullptr;   // node2vec membership: per-vertex hash sets of the neighbour ids, 8-slot buckets
   mutable uint32_t *adjsign = nullptr; // ... and the filter in front of them
   mutable uint4 *deg_codes = nullptr;  // degrees of eight vertices each (FastGCN)

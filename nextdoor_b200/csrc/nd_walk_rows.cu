@@ -3,15 +3,15 @@
 // organisation of a job gives the same samples, and on B200 a lane that keeps its walk in registers beats a
 // step-by-step pass over a transit-sorted map at every number of walks (measured, transit-parallel loop with
 // counting inversion -> this file: uniform walk on 57 K vertices 1.10 -> 0.07 ms, DeepWalk on 2^20 vertices
-// 5.2 -> 1.6 ms, node2vec 7.6 -> 2.3 ms, PPR on 2^24 vertices 5.4 -> 2.5 ms).
+// 5.2 -> 1.4 ms, node2vec 7.6 -> 2.3 ms, PPR on 2^24 vertices 5.4 -> 2.5 ms).
 //
 // What bounds it.  Large graphs: the rate of random DRAM reads.  A walker picks every CSR entry with the same
-// probability, the entry arrays do not fit the L2, and a gather of 4 or 8 bytes costs a 64-byte DRAM read; on 2^20
-// vertices the kernels move 5.2 (node2vec), 5.0 (DeepWalk) and 4.8 TB/s (uniform walk), 59-63 % of the pins, PPR on 2^22
-// vertices 4.0 (49 %); a streaming copy reaches 6.5.  So what
-// counts is the number of gathers that miss, hence: one try per round for the weighted apps (no speculation),
-// the weights as one byte per entry where that array has a chance to stay in the L2, the first stop draw of
-// a step made before the vertex is fetched, a filter in front of node2vec's sets, rows written once, in
+// probability, and a gather that misses the L2 reads a whole line of 128 bytes (11.1 GB for 91 M gathers of 4 bytes from
+// 2 GB); the GPU serves 40-45 G of those a second, and as many of 64 bytes (the loads' L2::64B): not the bytes are the
+// bound.  Independent gathers run at 285 G/s from up to 75 MB, 195 from 90, 139 from 110, 117 from 134, 88 from
+// 200, 55 from 400, 40 from 2 GB and more.  So what counts is the number of gathers, and the size of what they go to,
+// hence: one try per round for the weighted apps (no speculation), the id and its weight in one word, the first stop draw
+// of a step made before the vertex is fetched, a filter in front of node2vec's sets, rows written once, in
 // 32-byte sectors.  Small graphs: the chain of a walk, two dependent L2 reads per step, one where the entries carry the
 // neighbour's row, and the instructions between them (57 K vertices: a step is 0.5 us, 121 instructions of a warp at 8.2
 // cycles each, 45 % of them waiting for the read).
@@ -39,11 +39,10 @@ struct RowsArgs {
   const float *__restrict__ w;
   const float *__restrict__ max_w;
   const int2 *__restrict__ vrow;     // [V] (row start, degree)
-  const int4 *__restrict__ vrec4;    // [V] (row start, degree, max weight bits, 0)
   const int4 *__restrict__ erec;     // [E] (neighbour, its row start, its degree, 0)
   const int2 *__restrict__ colw;     // [E] (neighbour, weight bits)
   const int2 *__restrict__ vrec;     // [V+1] (row start, max weight bits)
-  const uint8_t *__restrict__ wq;    // [E] weights as 256ths of the row's maximum, rounded down
+  const uint32_t *__restrict__ pack; // [E] neighbour << 8 | weight as 256ths of the row's maximum, rounded down
   const int32_t *__restrict__ adjset;
   const uint32_t *__restrict__ adjsign;
   uint64_t seed;
@@ -67,21 +66,18 @@ struct RowsArgs {
 template <int APP>
 __host__ __device__ constexpr bool weighted() { return APP == ND_APP_DEEPWALK || APP == ND_APP_PPR; }
 
-// Layouts.  ALT: uniform walk: entries that carry the neighbour's row; weighted walks: one byte per weight.
+// Layouts of the entries.  ALT: uniform walk: they carry the neighbour's row; weighted walks: id and weight in a word.
 enum : int { LAYOUT_PLAIN = 0, LAYOUT_ALT = 1 };
 
-// ---- loads.  The small per-vertex and per-entry arrays ask to stay in the L2; a weighted walk's neighbour
-// ids bypass the L1, which then serves the bytes and vertex records of the hubs (DeepWalk 1.80 -> 1.63 ms;
-// the uniform walk and node2vec are slower that way: 0.94 -> 1.21, 2.32 -> 2.50 ms).
+// ---- loads.  The small per-vertex and per-entry arrays ask to stay in the L2; the (id, weight) records, an array far
+// larger than the L2, bypass the L1.
 struct Hot {
   uint64_t pol;
   __device__ __forceinline__ Hot() { asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol)); }
   __device__ __forceinline__ int32_t ld(const int32_t *p) const { int32_t v; asm("ld.global.nc.L2::cache_hint.s32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol)); return v; }
-  __device__ __forceinline__ uint32_t ld(const uint8_t *p) const { uint32_t v; asm("ld.global.nc.L2::cache_hint.u8 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol)); return v; }
   __device__ __forceinline__ int2 ld(const int2 *p) const { int2 v; asm("ld.global.nc.L2::cache_hint.v2.s32 {%0, %1}, [%2], %3;" : "=r"(v.x), "=r"(v.y) : "l"(p), "l"(pol)); return v; }
   __device__ __forceinline__ int4 ld(const int4 *p) const { int4 v; asm("ld.global.nc.L2::cache_hint.v4.s32 {%0, %1, %2, %3}, [%4], %5;" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(pol)); return v; }
 };
-__device__ __forceinline__ int32_t ld_once(const int32_t *p) { int32_t v; asm("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(v) : "l"(p)); return v; }
 __device__ __forceinline__ int2 ld_once(const int2 *p) { int2 v; asm("ld.global.nc.L1::no_allocate.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p)); return v; }
 
 // ---- rows of the result
@@ -203,7 +199,7 @@ __device__ __forceinline__ int32_t draw_index(uint32_t u, int32_t n) { return nd
 // walks of a lane follow from its place, the next ones are handed out to its warp 64 at a time.  A job whose
 // walks all have a lane takes them in order, without the pass that makes the list.
 constexpr int START_PER_THREAD = 4;
-template <int APP>
+template <int APP, int LAYOUT>
 __global__ void __launch_bounds__(256) walk_start_kernel(const RowsArgs a) {
   __shared__ uint32_t sh_n, sh_dead;
   __shared__ unsigned long long sh_base;
@@ -231,7 +227,7 @@ __global__ void __launch_bounds__(256) walk_start_kernel(const RowsArgs a) {
       draw_block(a, (uint32_t)s, 0, 0u, o);
       active = !(ndrng::u32_to_uniform(o[0]) < a.stop_prob);
     }
-    e[j] = make_int4((int)(uint32_t)s, rs, active ? deg : 0, weighted<APP>() ? (active ? __float_as_int(__ldg(a.max_w + t[j])) : 0) : t[j]);
+    e[j] = make_int4((int)(uint32_t)s, rs, active ? deg : 0, weighted<APP>() && LAYOUT == LAYOUT_PLAIN ? (active ? __float_as_int(__ldg(a.max_w + t[j])) : 0) : t[j]);
     if (!active) {
       for (int k = 0; k < had[j]; k++) a.out[s * a.steps + k] = a.V;
       if (had[j]) a.plen[s] = 0;
@@ -260,8 +256,7 @@ __global__ void __launch_bounds__(256) walk_start_kernel(const RowsArgs a) {
 // (row start, degree, max weight bits or vertex) of a vertex
 template <int APP, int LAYOUT>
 __device__ __forceinline__ int4 vertex_of(const RowsArgs &a, const Hot &hot, int32_t v) {
-  if (weighted<APP>()) {
-    if (LAYOUT == LAYOUT_ALT) return hot.ld(a.vrec4 + v);
+  if (weighted<APP>() && LAYOUT == LAYOUT_PLAIN) {
     const int2 r = hot.ld(a.vrec + v), n = hot.ld(a.vrec + v + 1);
     return make_int4(r.x, n.x - r.x, r.y, 0);
   }
@@ -279,11 +274,24 @@ __device__ __forceinline__ int4 walk_of(const RowsArgs &a, const Hot &hot, int64
   return make_int4((int)(uint32_t)i, v.x, v.y, v.z);
 }
 
+// Walks that run their full length (EQUAL) take equal rounds: with w rounds of lanes every round takes n / w walks, or the
+// last one would run a fraction of the lanes for as long as the others; and a warp gets 32 at a time.
+template <bool EQUAL>
 struct Taker {
+  static constexpr int GRANT = EQUAL ? 32 : 64;
   int64_t n, lanes, cur, end;
   __device__ __forceinline__ explicit Taker(const RowsArgs &a)
-      : n(a.list ? (int64_t)a.acc[9] : a.S), lanes((int64_t)gridDim.x * ROWS_THREADS), cur(0), end(0) {}
-  __device__ __forceinline__ int64_t first() const { return (int64_t)blockIdx.x * ROWS_THREADS + threadIdx.x; }
+      : n(a.list ? (int64_t)a.acc[9] : a.S), lanes((int64_t)gridDim.x * ROWS_THREADS), cur(0), end(0) {
+    if (EQUAL && n > lanes) {
+      const int64_t rounds = (n + lanes - 1) / lanes;
+      lanes = ((n + rounds - 1) / rounds + 31) / 32 * 32;
+    }
+  }
+  // the lane's first walk (n or more: none)
+  __device__ __forceinline__ int64_t first() const {
+    const int64_t i = (int64_t)blockIdx.x * ROWS_THREADS + threadIdx.x;
+    return i < lanes ? i : n;
+  }
   // the next walk of every lane that wants one (n or more: none left); the whole warp calls it
   __device__ __forceinline__ int64_t next(const RowsArgs &a, unsigned want) {
     const int lane = threadIdx.x & 31;
@@ -295,12 +303,12 @@ struct Taker {
     } else {
       unsigned long long nb = (unsigned long long)n;
       if (n > lanes) {
-        if (lane == 0) nb = (unsigned long long)lanes + atomicAdd(&a.acc[8], 64ull);
+        if (lane == 0) nb = (unsigned long long)lanes + atomicAdd(&a.acc[8], (unsigned long long)GRANT);
         nb = __shfl_sync(0xffffffffu, nb, 0);
       }
       if (my >= avail) i = (int64_t)nb + (my - avail);
       cur = (int64_t)nb + (need - avail);
-      end = (int64_t)nb + 64;
+      end = (int64_t)nb + GRANT;
     }
     return i;
   }
@@ -309,8 +317,7 @@ struct Taker {
 // ---------------------------------------------------------------- uniform walk (example/uniformRandWalk.cu:27-37)
 //
 // The lanes of a warp go in step.  The draw of the next step does not depend on the vertex: it is made while
-// the gather is in flight, so that a step is its dependent reads and little else.  Equal waves: with w waves
-// of lanes every wave takes n / w walks, or the last one would run a fraction of the lanes for as long.
+// the gather is in flight, so that a step is its dependent reads and little else.  Equal rounds, as in Taker.
 template <int LAYOUT>
 __device__ __forceinline__ void uniform_walks(const RowsArgs &a) {
   constexpr bool FAT = LAYOUT == LAYOUT_ALT;
@@ -318,12 +325,12 @@ __device__ __forceinline__ void uniform_walks(const RowsArgs &a) {
   __shared__ unsigned int sums[2];
   Rows<PIECE> rows(a, sums);
   const Hot hot;
-  const Taker take(a);
-  const int64_t waves = (take.n + take.lanes - 1) / take.lanes, per = waves ? (take.n + waves - 1) / waves : 0;
-  for (int64_t wave = 0; wave < waves; wave++) {
-    const int64_t w0 = wave * per, wn = take.n - w0 < per ? take.n - w0 : per;
-    if (take.first() >= wn) continue;
-    const int4 e = walk_of<ND_APP_UNIFORM_WALK, LAYOUT>(a, hot, w0 + take.first());
+  const int64_t all = a.list ? (int64_t)a.acc[9] : a.S, lanes = (int64_t)gridDim.x * ROWS_THREADS, me = (int64_t)blockIdx.x * ROWS_THREADS + threadIdx.x;
+  const int64_t rounds = (all + lanes - 1) / lanes, per = rounds ? (all + rounds - 1) / rounds : 0;
+  for (int64_t round = 0; round < rounds; round++) {
+    const int64_t w0 = round * per, wn = all - w0 < per ? all - w0 : per;
+    if (me >= wn) continue;
+    const int4 e = walk_of<ND_APP_UNIFORM_WALK, LAYOUT>(a, hot, w0 + me);
     const uint32_t s = (uint32_t)e.x;
     int32_t rs = e.y, deg = e.z;
     uint32_t u[4];
@@ -359,19 +366,21 @@ __device__ __forceinline__ void uniform_walks(const RowsArgs &a) {
 // step: PPR's stop draw, then two per try; a block of four is made once and kept (k0..k2).
 // PPR makes the stop draw of a step before it fetches the vertex, which a walk that stops never needs.
 //
-// Weights.  PLAIN: (id, weight) records, one gather per try.  ALT: the row's weights as whole 256ths of its
-// maximum, rounded down (a byte per entry): b/256 <= w/max < (b+1)/256 decides all but one try in 256 --
-// those read the weight -- and the id is gathered once per step.  Same decisions, as b * (max/256) and
-// (b+1) * (max/256), rounded as the kernel rounds them, were compared with w when b was chosen.  ALT moves
-// fewer DRAM reads while the bytes have a chance to stay in the L2 (WQ_ENTRIES): DeepWalk on 33.5 M entries
-// 1.99 -> 1.63 ms, but a byte array that is itself read from DRAM is one more read per step.
+// Weights.  PLAIN: (id, weight) records.  ALT: the id and the weight as whole 256ths of the row's maximum, rounded down, in
+// one word: b/256 <= w/max < (b+1)/256 decides all but one try in 256 without the weight or the maximum -- u <= b/256
+// accepts and u >= (b+1)/256 rejects, and both follow for u * max against w because b * (max/256) and
+// (b+1) * (max/256), rounded as the kernel rounds u * max, were compared with w when b was chosen.  One gather per try
+// where there were a byte per try, then the id: DeepWalk on 2^20 vertices 1.57 -> 1.40 ms, on 600 K 0.93 -> 0.61, on 40 K
+// 0.20 -> 0.15; PPR on 2^21 0.46 -> 0.38.  The words go through the L1 like any other load: ld.global.nc with
+// L1::no_allocate leaves them the first to go in the L2 as well, three of four tries on 134 MB of them then miss instead of
+// two of five (DeepWalk 1.93 ms), and only arrays far larger than the L2 (PLAIN) lose nothing by it.
 template <int APP, int LAYOUT>
 __device__ __forceinline__ void weighted_walks(const RowsArgs &a) {
   constexpr bool PPR = APP == ND_APP_PPR;
   __shared__ unsigned int sums[2];
   Rows<piece<APP>()> rows(a, sums);
   const Hot hot;
-  Taker take(a);
+  Taker<!PPR> take(a);
   uint32_t s = 0, k0 = 0, k1 = 0, k2 = 0, tries = 0;
   // cur: the vertex the walk has moved to, its record not fetched yet; -1: (rs, deg, mw) are those of the walk's vertex
   int32_t rs = 0, deg = 0, mw = 0, cur = -1;
@@ -413,20 +422,18 @@ __device__ __forceinline__ void weighted_walks(const RowsArgs &a) {
       }
     }
     if (deg <= 0 || over) continue;   // no walk, a vertex without neighbours, or a walk just taken: it starts in the next trip
-    const float max_w = __int_as_float(mw);
     const int32_t x = draw_index(dx, deg);
-    const float y = __fmul_rn(ndrng::u32_to_uniform(dy), max_w);
+    const float u = ndrng::u32_to_uniform(dy);
     int32_t nbr = AGAIN;
     if (LAYOUT == LAYOUT_ALT) {
-      const uint32_t b = hot.ld(a.wq + rs + x);
-      const float unit = __fmul_rn(max_w, 0.00390625f);
-      const float lo = __fmul_rn(__uint2float_rn(b), unit), hi = __fmul_rn(__uint2float_rn(b + 1u), unit);
-      bool accept = deg == 1 || (b > 0u && y <= lo);
-      if (!accept && !(b < 255u && y > hi)) accept = !(y > __ldg(a.w + rs + x));
-      if (accept) nbr = ld_once(a.col + rs + x);
+      const uint32_t r = __ldg(a.pack + rs + x), b = r & 255u;
+      bool accept = deg == 1 || u <= (float)b * 0.00390625f;
+      if (!accept && (b == 255u || u < (float)(b + 1u) * 0.00390625f))
+        accept = !(__fmul_rn(u, __ldg(a.max_w + mw)) > __ldg(a.w + rs + x));
+      if (accept) nbr = (int32_t)(r >> 8);
     } else {
       const int2 r = ld_once(a.colw + rs + x);
-      if (deg == 1 || !(y > __int_as_float(r.y))) nbr = r.x;
+      if (deg == 1 || !(__fmul_rn(u, __int_as_float(mw)) > __int_as_float(r.y))) nbr = r.x;
     }
     tries += deg > 1 ? 1u : 0u;
     if (nbr == AGAIN && ++t > RETRY_CAP) {
@@ -494,7 +501,7 @@ __device__ __forceinline__ void n2v_walks(const RowsArgs &a) {
   Rows<piece<APP>()> rows(a, sums);
   const Hot hot;
   const N2vConsts c(a.p, a.q);
-  Taker take(a);
+  Taker<true> take(a);
   uint32_t s = 0, tries = 0, words = 0;
   int32_t rs = 0, deg = 0, cur = 0, prev = 0, ts = 0, tn = 0;   // [ts, ts + tn): the row of the previous vertex
   int step = -1, round = 0;
@@ -621,11 +628,6 @@ __global__ void vrec_build_kernel(const int32_t *__restrict__ row_ptr, const flo
     vrec[v] = make_int2(row_ptr[v], v < V ? __float_as_int(max_w[v]) : 0);
 }
 
-__global__ void vrec4_build_kernel(const int32_t *__restrict__ row_ptr, const float *__restrict__ max_w, int32_t V, int4 *__restrict__ vrec) {
-  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x)
-    vrec[v] = make_int4(row_ptr[v], row_ptr[v + 1] - row_ptr[v], __float_as_int(max_w[v]), 0);
-}
-
 __global__ void erec_build_kernel(const int32_t *__restrict__ col, const int32_t *__restrict__ row_ptr, int64_t E, int4 *__restrict__ erec) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
     const int32_t v = col[e], rs = row_ptr[v];
@@ -633,9 +635,16 @@ __global__ void erec_build_kernel(const int32_t *__restrict__ col, const int32_t
   }
 }
 
+// A row whose maximum is negative, not a number or so small that its 256th is not exact: the comparisons that the packed
+// weights replace do not follow from one another there.
+__global__ void odd_max_kernel(const int32_t *__restrict__ row_ptr, const float *__restrict__ max_w, int32_t V, int *__restrict__ odd) {
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x)
+    if (row_ptr[v + 1] - row_ptr[v] > 1 && !(max_w[v] == 0.f || max_w[v] >= 7.8886090522101181e-31f)) *odd = 1;   // 2^-100
+}
+
 __global__ void __launch_bounds__(BUILD_THREADS)
-wq_build_kernel(const int32_t *__restrict__ row_ptr, const float *__restrict__ max_w, const float *__restrict__ w, int32_t V, int64_t E,
-                uint8_t *__restrict__ wq) {
+pack_build_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col, const float *__restrict__ max_w, const float *__restrict__ w,
+                  int32_t V, int64_t E, uint32_t *__restrict__ pack) {
   for_entries(row_ptr, V, E, [&](int64_t e, int32_t v) {
     const float x = w[e], unit = __fmul_rn(max_w[v], 0.00390625f);
     int b = 255;   // a weight that is not a number accepts every draw: decided by comparing with it
@@ -645,7 +654,7 @@ wq_build_kernel(const int32_t *__restrict__ row_ptr, const float *__restrict__ m
       while (b > 0 && !(__fmul_rn((float)b, unit) <= x)) b--;
       while (b < 255 && __fmul_rn((float)(b + 1), unit) <= x) b++;
     }
-    wq[e] = (uint8_t)b;
+    pack[e] = (uint32_t)col[e] << 8 | (uint32_t)b;
   });
 }
 
@@ -687,12 +696,14 @@ adjset_build_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restri
 // Entries that carry the neighbour's row (16 bytes each) shorten a step to one dependent read; they pay while
 // the array stays in a die's half of the L2 with room to spare: 32 MB.
 constexpr int64_t ERECS = (int64_t)1 << 21;
-// The byte array of the weights: see weighted_walks.
-constexpr int64_t WQ_ENTRIES = (int64_t)1 << 26;
+// Ids that leave a byte of a word to the weight.
+constexpr int32_t PACK_V = 1 << 24;
 
-bool alt_layout(const nd_sampler *s) {
-  if (s->p.app == ND_APP_UNIFORM_WALK) return s->g->E <= ERECS;
-  return (s->p.app == ND_APP_DEEPWALK || s->p.app == ND_APP_PPR) && s->g->E <= WQ_ENTRIES;
+int layout_of(const nd_sampler *s) {
+  const nd_graph *g = s->g;
+  if (s->p.app == ND_APP_DEEPWALK || s->p.app == ND_APP_PPR) return g->pack ? LAYOUT_ALT : LAYOUT_PLAIN;
+  if (s->p.app == ND_APP_UNIFORM_WALK && g->E <= ERECS) return LAYOUT_ALT;
+  return LAYOUT_PLAIN;
 }
 
 template <int APP, int LAYOUT>
@@ -702,13 +713,20 @@ void launch(nd_sampler *s, RowsArgs &a, bool count) {
   const int smem = 4 * piece<APP>() * ROWS_THREADS + (count ? 4 * a.steps : 0);
   if (ctas > cap) {   // more walks than lanes: start from the list
     constexpr int per_cta = 256 * START_PER_THREAD;
-    walk_start_kernel<APP><<<(int)((s->S + per_cta - 1) / per_cta), 256, 0, s->stream>>>(a);
+    walk_start_kernel<APP, LAYOUT><<<(int)((s->S + per_cta - 1) / per_cta), 256, 0, s->stream>>>(a);
     nd_count_launches(1);
   } else {
     a.list = nullptr;
   }
   walk_next_count_kernel<APP, LAYOUT><<<grid, ROWS_THREADS, smem, s->stream>>>(a);
   nd_count_launches(1);
+}
+
+template <int APP>
+void launch_as(nd_sampler *s, RowsArgs &a, bool count) {
+  const int layout = layout_of(s);
+  if (APP != ND_APP_NODE2VEC && layout == LAYOUT_ALT) return launch<APP, APP != ND_APP_NODE2VEC ? LAYOUT_ALT : LAYOUT_PLAIN>(s, a, count);
+  launch<APP, LAYOUT_PLAIN>(s, a, count);
 }
 
 // The derived layouts of a graph are built by the first sampler that needs them; samplers of one
@@ -748,18 +766,24 @@ int ensure_vrow(const nd_graph *g, int sms) {
   return ND_OK;
 }
 
-// per-vertex records with the maximum weight, and the weights as bytes
-int ensure_wq(const nd_graph *g, int sms) {
-  if (g->wq) return ND_OK;
-  NdDevMem<int4> vrec4;
-  NdDevMem<uint8_t> wq;
-  ND_TRY(vrec4.alloc((size_t)g->V));
-  ND_TRY(wq.alloc((size_t)(g->E > 0 ? g->E : 1)));
-  vrec4_build_kernel<<<sms * 16, 256>>>(g->row_ptr, g->max_w, g->V, vrec4.p);
-  wq_build_kernel<<<sms * 16, BUILD_THREADS>>>(g->row_ptr, g->max_w, g->w, g->V, g->E, wq.p);
+// ids and weights in one word, or the records of ensure_colw where they do not fit one
+int ensure_weighted(const nd_graph *g, int sms) {
+  if (g->pack) return ND_OK;
+  if (g->V > PACK_V || g->odd_max == 1) return ensure_colw(g, sms);
+  ND_TRY(ensure_vrow(g, sms));
+  NdDevMem<int> flag;
+  int odd = 0;
+  ND_TRY(flag.alloc(1));
+  ND_CUDA(cudaMemset(flag.p, 0, sizeof(int)));
+  odd_max_kernel<<<sms * 16, 256>>>(g->row_ptr, g->max_w, g->V, flag.p);
+  ND_CUDA(cudaMemcpy(&odd, flag.p, sizeof(int), cudaMemcpyDeviceToHost));
+  g->odd_max = odd;
+  if (odd) return ensure_colw(g, sms);
+  NdDevMem<uint32_t> pack;
+  ND_TRY(pack.alloc((size_t)(g->E > 0 ? g->E : 1)));
+  pack_build_kernel<<<sms * 16, BUILD_THREADS>>>(g->row_ptr, g->col, g->max_w, g->w, g->V, g->E, pack.p);
   ND_CUDA(cudaGetLastError());
-  g->vrec4 = vrec4.release();
-  g->wq = wq.release();
+  g->pack = pack.release();
   return ND_OK;
 }
 
@@ -814,9 +838,9 @@ int nd_walk_rows_alloc(nd_sampler *s) {
   ND_TRY(make(s->d_rows_acc, acc));
   ND_CUDA(cudaMemset(s->d_rows_acc, 0, 8 * acc));
   std::lock_guard<std::mutex> lock(g_derived_mutex);
-  if (app == ND_APP_DEEPWALK || app == ND_APP_PPR) return alt_layout(s) ? ensure_wq(g, sms) : ensure_colw(g, sms);
+  if (app == ND_APP_DEEPWALK || app == ND_APP_PPR) return ensure_weighted(g, sms);
   ND_TRY(ensure_vrow(g, sms));
-  if (app == ND_APP_UNIFORM_WALK && alt_layout(s)) ND_TRY(ensure_erec(g, sms));
+  if (app == ND_APP_UNIFORM_WALK && layout_of(s) == LAYOUT_ALT) ND_TRY(ensure_erec(g, sms));
   if (app == ND_APP_NODE2VEC) ND_TRY(ensure_adjset(g, sms, s->d_status, s->h_status));
   return ND_OK;
 }
@@ -824,15 +848,14 @@ int nd_walk_rows_alloc(nd_sampler *s) {
 int nd_walk_rows_launch(nd_sampler *s, bool count) {
   const nd_graph *g = s->g;
   uint32_t *ended = count ? reinterpret_cast<uint32_t *>(s->d_rows_acc + 16) : nullptr;
-  RowsArgs a{g->V, g->row_ptr, g->col, g->w, g->max_w, g->vrow, g->vrec4, g->erec, g->colw, g->vrec, g->wq, g->adjset, g->adjsign,
+  RowsArgs a{g->V, g->row_ptr, g->col, g->w, g->max_w, g->vrow, g->erec, g->colw, g->vrec, g->pack, g->adjset, g->adjsign,
              s->p.seed, s->p.p, s->p.q, s->p.stop_prob, s->p.n2v_ref_compat, s->p.steps, s->first, s->S, s->d_initial, s->d_out,
              s->d_plen, s->d_list, s->d_rows_acc, ended, s->d_stats, (uint32_t *)s->d_nlive, s->d_status};
-  const bool alt = alt_layout(s);
   switch (s->p.app) {
-    case ND_APP_UNIFORM_WALK: if (alt) launch<ND_APP_UNIFORM_WALK, LAYOUT_ALT>(s, a, count); else launch<ND_APP_UNIFORM_WALK, LAYOUT_PLAIN>(s, a, count); break;
-    case ND_APP_DEEPWALK: if (alt) launch<ND_APP_DEEPWALK, LAYOUT_ALT>(s, a, count); else launch<ND_APP_DEEPWALK, LAYOUT_PLAIN>(s, a, count); break;
-    case ND_APP_PPR: if (alt) launch<ND_APP_PPR, LAYOUT_ALT>(s, a, count); else launch<ND_APP_PPR, LAYOUT_PLAIN>(s, a, count); break;
-    default: launch<ND_APP_NODE2VEC, LAYOUT_PLAIN>(s, a, count); break;
+    case ND_APP_UNIFORM_WALK: launch_as<ND_APP_UNIFORM_WALK>(s, a, count); break;
+    case ND_APP_DEEPWALK: launch_as<ND_APP_DEEPWALK>(s, a, count); break;
+    case ND_APP_PPR: launch_as<ND_APP_PPR>(s, a, count); break;
+    default: launch_as<ND_APP_NODE2VEC>(s, a, count); break;
   }
   ND_CUDA(cudaGetLastError());
   return ND_OK;

@@ -65,3 +65,54 @@ def test_weights_at_the_edges_of_their_byte_code(nd, ndo, small_graph, kind):
     exp = ndo.sample(hg, ndo.make_params(1, steps=12, seed=11), 4000)
     assert np.array_equal(s.final_samples(), exp["out"])
     assert s.stats()["weight_tries"] == exp["counters"]["weight_tries"]
+
+
+@pytest.mark.parametrize("app", [1, 2])
+@pytest.mark.parametrize("kind", ["nan", "negative", "least", "below", "infinite"])
+def test_maxima_that_rule_packed_weights_in_or_out(nd, ndo, small_graph, app, kind):
+    """A caller's maxima: the packed weights decide by them, or the records do where they cannot."""
+    rng = np.random.default_rng(2)
+    n = small_graph.E
+    w = (rng.random(n) + 0.25).astype(np.float32)
+    odd = {"nan": np.nan, "negative": -1.0, "least": 2.0 ** -100, "below": 2.0 ** -101, "infinite": np.inf}[kind]
+    mw = np.where(rng.random(small_graph.V) < 0.2, odd, small_graph.max_w).astype(np.float32)
+    if kind == "infinite":   # a finite weight under an infinite maximum is never accepted
+        w[rng.random(n) < 0.5] = np.inf
+        src = np.repeat(np.arange(small_graph.V, dtype=np.int32), small_graph.degree())
+        mw = np.zeros(small_graph.V, np.float32)
+        np.maximum.at(mw, src, w)
+    hg = ndo.HostGraph(small_graph.row_ptr, small_graph.col, w, mw)
+    s = nd.Sampler(_graph(nd, hg), nd.app_params(app, steps=9, seed=4, stop_prob=0.1), num_samples=3000)
+    s.sample(1)
+    exp = ndo.sample(hg, ndo.make_params(app, steps=9, seed=4, stop_prob=0.1), 3000)
+    assert np.array_equal(s.final_samples(), exp["out"])
+    assert s.stats()["weight_tries"] == exp["counters"]["weight_tries"]
+
+
+@pytest.mark.parametrize("V", [1 << 24, (1 << 24) + 1])
+def test_ids_up_to_and_beyond_the_packed_width(nd, ndo, V):
+    rng = np.random.default_rng(3)
+    ids = np.unique(np.concatenate([rng.integers(0, V, 300), [0, V - 1, V - 2]])).astype(np.int32)
+    src = np.concatenate([rng.choice(ids, 4000), [V - 1]]).astype(np.int32)
+    dst = np.concatenate([rng.choice(ids, 4000), [V - 2]]).astype(np.int32)
+    hg = ndo.csr_from_records(src, dst, (rng.random(len(src)) + 0.1).astype(np.float32), V=V)
+    init = rng.choice(ids, 1000).astype(np.int32)
+    for app in (1, 2):
+        s = nd.Sampler(_graph(nd, hg), nd.app_params(app, steps=9, seed=4, stop_prob=0.1), num_samples=1000, initial=init)
+        s.sample(1)
+        exp = ndo.sample(hg, ndo.make_params(app, steps=9, seed=4, stop_prob=0.1), 1000, initial=init)
+        assert np.array_equal(s.final_samples(), exp["out"]), app
+
+
+@pytest.mark.parametrize("app", [1, 3])
+@pytest.mark.parametrize("S", [2 * LANES, 2 * LANES + 33, 3 * LANES - 1])
+def test_rounds_of_walks(nd, ndo, small_graph, app, S):
+    rng = np.random.default_rng(S)
+    able = np.flatnonzero(small_graph.degree() > 0)
+    init = rng.choice(able, S).astype(np.int32)   # every walk can start: the list is as long as the job
+    s = nd.Sampler(_graph(nd, small_graph), nd.app_params(app, steps=3, seed=3), num_samples=S, initial=init)
+    exp = ndo.sample(small_graph, ndo.make_params(app, steps=3, seed=3), S, initial=init)
+    for _ in range(2):
+        s.sample(1)
+        assert np.array_equal(s.final_samples(), exp["out"])
+        assert s.stats()["live_pairs"] == exp["counters"]["live_pairs"]
