@@ -43,6 +43,7 @@ struct RowsArgs {
   const int2 *__restrict__ colw;     // [E] (neighbour, weight bits)
   const int2 *__restrict__ vrec;     // [V+1] (row start, max weight bits)
   const uint32_t *__restrict__ pack; // [E] neighbour << 8 | weight as 256ths of the row's maximum, rounded down
+  const uint2 *__restrict__ col3;    // [E/3] three neighbours of 21 bits each
   const int32_t *__restrict__ adjset;
   const uint32_t *__restrict__ adjsign;
   uint64_t seed;
@@ -67,7 +68,8 @@ template <int APP>
 __host__ __device__ constexpr bool weighted() { return APP == ND_APP_DEEPWALK || APP == ND_APP_PPR; }
 
 // Layouts of the entries.  ALT: uniform walk: they carry the neighbour's row; weighted walks: id and weight in a word.
-enum : int { LAYOUT_PLAIN = 0, LAYOUT_ALT = 1 };
+// DENSE (uniform walk, node2vec): three ids of 21 bits in 8 bytes.
+enum : int { LAYOUT_PLAIN = 0, LAYOUT_ALT = 1, LAYOUT_DENSE = 2 };
 
 // ---- loads.  The small per-vertex and per-entry arrays ask to stay in the L2; the (id, weight) records, an array far
 // larger than the L2, bypass the L1.
@@ -79,6 +81,25 @@ struct Hot {
   __device__ __forceinline__ int4 ld(const int4 *p) const { int4 v; asm("ld.global.nc.L2::cache_hint.v4.s32 {%0, %1, %2, %3}, [%4], %5;" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(pol)); return v; }
 };
 __device__ __forceinline__ int2 ld_once(const int2 *p) { int2 v; asm("ld.global.nc.L1::no_allocate.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p)); return v; }
+
+// ---- ids without their unused bits
+//
+// Between 64 MB and a few times the L2, a smaller array is fewer misses: three ids of 21 bits in 8 bytes, 2.67 bytes an
+// entry (2^20 vertices, 33.5 M entries, 134 -> 89 MB: uniform walk 0.91 -> 0.78 ms, node2vec 2.26 -> 2.14; 2^21
+// vertices, 50 M entries: 1.57 -> 1.37, 3.88 -> 3.61; 600 K, 14.4 M: 0.34 -> 0.32, 0.98 -> 1.00; 300 K, 7.2 M, inside the
+// L2 either way: 0.17 -> 0.18, 0.21 -> 0.22).
+constexpr int DENSE_IDS = 3, DENSE_ID_BITS = 21;
+constexpr int32_t DENSE_V = 1 << DENSE_ID_BITS;
+constexpr int64_t DENSE_ENTRIES = (int64_t)1 << 24;
+
+// neighbour of entry e
+template <int LAYOUT>
+__device__ __forceinline__ int32_t id_of(const RowsArgs &a, int32_t e) {
+  if (LAYOUT != LAYOUT_DENSE) return __ldg(a.col + e);
+  const uint32_t group = (uint32_t)e / DENSE_IDS, off = ((uint32_t)e - DENSE_IDS * group) * DENSE_ID_BITS;
+  const uint2 q = __ldg(a.col3 + group);
+  return (int32_t)((uint32_t)(((unsigned long long)q.y << 32 | q.x) >> off) & ((1u << DENSE_ID_BITS) - 1u));
+}
 
 // ---- rows of the result
 //
@@ -345,7 +366,7 @@ __device__ __forceinline__ void uniform_walks(const RowsArgs &a) {
         draw_block(a, s, step + 1, 0u, u);
         v = f.x; r = make_int2(f.y, f.z);
       } else {
-        v = __ldg(a.col + rs + x);
+        v = id_of<LAYOUT>(a, rs + x);
         draw_block(a, s, step + 1, 0u, u);
         if (step + 1 < a.steps) r = hot.ld(a.vrow + v);
       }
@@ -494,6 +515,7 @@ __device__ __forceinline__ bool member_exact(const RowsArgs &a, int32_t ts, int3
 // membership accepts it (one try per round: 2.32 -> 2.6 ms).  A membership test asks the filter first: a word
 // of 8 bits per neighbour answers about 95 % of the tests that fail (88 % of all), the rest read the set
 // (without the filter 2.9 ms).
+template <int LAYOUT>
 __device__ __forceinline__ void n2v_walks(const RowsArgs &a) {
   constexpr int APP = ND_APP_NODE2VEC;
   constexpr int TRIES = 2;
@@ -529,7 +551,7 @@ __device__ __forceinline__ void n2v_walks(const RowsArgs &a) {
       for (int j = TRIES - 1; j >= 0; j--) if (y[j] < c.sure) n_try = j + 1;
       if (simple) n_try = 1;
 #pragma unroll
-      for (int j = 0; j < TRIES; j++) v[j] = j < n_try ? __ldg(a.col + rs + x[j]) : -1;
+      for (int j = 0; j < TRIES; j++) v[j] = j < n_try ? id_of<LAYOUT>(a, rs + x[j]) : -1;
       const uint32_t w0 = (uint32_t)ts >> 2, n_words = ((uint32_t)(ts + tn) >> 2) - w0;
       bool is_ret[TRIES], need[TRIES];
       uint32_t h[TRIES], word[TRIES];
@@ -603,7 +625,7 @@ __device__ __forceinline__ void n2v_walks(const RowsArgs &a) {
 template <int APP, int LAYOUT>
 __device__ __forceinline__ void walks(const RowsArgs &a) {
   if (APP == ND_APP_UNIFORM_WALK) uniform_walks<LAYOUT>(a);
-  else if (APP == ND_APP_NODE2VEC) n2v_walks(a);
+  else if (APP == ND_APP_NODE2VEC) n2v_walks<LAYOUT>(a);
   else weighted_walks<APP, LAYOUT>(a);
 }
 
@@ -658,6 +680,16 @@ pack_build_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restrict
   });
 }
 
+__global__ void col3_build_kernel(const int32_t *__restrict__ col, int64_t E, uint2 *__restrict__ col3) {
+  const int64_t n = (E + DENSE_IDS - 1) / DENSE_IDS;
+  for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < n; g += (int64_t)gridDim.x * blockDim.x) {
+    unsigned long long q = 0;
+    for (int k = 0; k < DENSE_IDS; k++)
+      if (DENSE_IDS * g + k < E) q |= (unsigned long long)(uint32_t)col[DENSE_IDS * g + k] << (k * DENSE_ID_BITS);
+    col3[g] = make_uint2((uint32_t)q, (uint32_t)(q >> 32));
+  }
+}
+
 __global__ void __launch_bounds__(BUILD_THREADS)
 adjsign_build_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col, int32_t V, int64_t E, uint32_t *__restrict__ sign) {
   for_entries(row_ptr, V, E, [&](int64_t e, int32_t t) {
@@ -698,12 +730,11 @@ adjset_build_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restri
 constexpr int64_t ERECS = (int64_t)1 << 21;
 // Ids that leave a byte of a word to the weight.
 constexpr int32_t PACK_V = 1 << 24;
-
 int layout_of(const nd_sampler *s) {
   const nd_graph *g = s->g;
   if (s->p.app == ND_APP_DEEPWALK || s->p.app == ND_APP_PPR) return g->pack ? LAYOUT_ALT : LAYOUT_PLAIN;
   if (s->p.app == ND_APP_UNIFORM_WALK && g->E <= ERECS) return LAYOUT_ALT;
-  return LAYOUT_PLAIN;
+  return g->V <= DENSE_V && g->E >= DENSE_ENTRIES ? LAYOUT_DENSE : LAYOUT_PLAIN;
 }
 
 template <int APP, int LAYOUT>
@@ -726,6 +757,7 @@ template <int APP>
 void launch_as(nd_sampler *s, RowsArgs &a, bool count) {
   const int layout = layout_of(s);
   if (APP != ND_APP_NODE2VEC && layout == LAYOUT_ALT) return launch<APP, APP != ND_APP_NODE2VEC ? LAYOUT_ALT : LAYOUT_PLAIN>(s, a, count);
+  if (!weighted<APP>() && layout == LAYOUT_DENSE) return launch<APP, !weighted<APP>() ? LAYOUT_DENSE : LAYOUT_PLAIN>(s, a, count);
   launch<APP, LAYOUT_PLAIN>(s, a, count);
 }
 
@@ -787,6 +819,16 @@ int ensure_weighted(const nd_graph *g, int sms) {
   return ND_OK;
 }
 
+int ensure_col3(const nd_graph *g, int sms) {
+  if (g->col3) return ND_OK;
+  NdDevMem<uint2> col3;
+  ND_TRY(col3.alloc((size_t)(g->E / DENSE_IDS + 1)));
+  col3_build_kernel<<<sms * 16, 256>>>(g->col, g->E, col3.p);
+  ND_CUDA(cudaGetLastError());
+  g->col3 = col3.release();
+  return ND_OK;
+}
+
 int ensure_erec(const nd_graph *g, int sms) {
   if (g->erec) return ND_OK;
   NdDevMem<int4> erec;
@@ -841,6 +883,7 @@ int nd_walk_rows_alloc(nd_sampler *s) {
   if (app == ND_APP_DEEPWALK || app == ND_APP_PPR) return ensure_weighted(g, sms);
   ND_TRY(ensure_vrow(g, sms));
   if (app == ND_APP_UNIFORM_WALK && layout_of(s) == LAYOUT_ALT) ND_TRY(ensure_erec(g, sms));
+  if (layout_of(s) == LAYOUT_DENSE) ND_TRY(ensure_col3(g, sms));
   if (app == ND_APP_NODE2VEC) ND_TRY(ensure_adjset(g, sms, s->d_status, s->h_status));
   return ND_OK;
 }
@@ -848,7 +891,7 @@ int nd_walk_rows_alloc(nd_sampler *s) {
 int nd_walk_rows_launch(nd_sampler *s, bool count) {
   const nd_graph *g = s->g;
   uint32_t *ended = count ? reinterpret_cast<uint32_t *>(s->d_rows_acc + 16) : nullptr;
-  RowsArgs a{g->V, g->row_ptr, g->col, g->w, g->max_w, g->vrow, g->erec, g->colw, g->vrec, g->pack, g->adjset, g->adjsign,
+  RowsArgs a{g->V, g->row_ptr, g->col, g->w, g->max_w, g->vrow, g->erec, g->colw, g->vrec, g->pack, g->col3, g->adjset, g->adjsign,
              s->p.seed, s->p.p, s->p.q, s->p.stop_prob, s->p.n2v_ref_compat, s->p.steps, s->first, s->S, s->d_initial, s->d_out,
              s->d_plen, s->d_list, s->d_rows_acc, ended, s->d_stats, (uint32_t *)s->d_nlive, s->d_status};
   switch (s->p.app) {

@@ -116,3 +116,18 @@ def test_rounds_of_walks(nd, ndo, small_graph, app, S):
         s.sample(1)
         assert np.array_equal(s.final_samples(), exp["out"])
         assert s.stats()["live_pairs"] == exp["counters"]["live_pairs"]
+
+
+@pytest.mark.parametrize("app", [0, 3])
+@pytest.mark.parametrize("V,M", [(1 << 21, (1 << 23) - 1), (1 << 21, 1 << 23), (1 << 21, (1 << 23) + 1), (1 << 21, (1 << 23) + 2), ((1 << 21) + 1, 1 << 23),
+                                 (3000, 1 << 23)])
+def test_ids_of_21_bits(nd, app, V, M):
+    """Against the exact-sort mode, which reads the plain ids."""
+    g = nd.Graph.rmat(V, M, seed=3)
+    init = np.random.default_rng(M).integers(0, V, 20000).astype(np.int32)
+    s = nd.Sampler(g, nd.app_params(app, steps=15, seed=5), num_samples=len(init), initial=init)
+    s.sample(0)
+    exp = s.final_samples().copy()
+    for mode in (1, 2):
+        s.sample(mode)
+        assert np.array_equal(s.final_samples(), exp), mode
