@@ -157,7 +157,7 @@ int nd_sampler_final_samples_async(nd_sampler *s, int32_t *out, void *copy_strea
  *   fetch:  waits for the lengths, then enqueues the copy of the packed vertices (or of the dense array when
  *           more than half of its slots are in use); optional -- finish calls it when the caller did not.
  *   finish: waits for that copy and writes the rows with host threads (ND_HOST_THREADS, default: the hardware
- *           threads, at most 32); `values_copied` (may be NULL) receives the number of vertex slots that crossed.
+ *           threads, at most 32), a share of them by the GPU where it can reach both arrays; `values_copied` (may be NULL) receives the number of vertex slots that crossed.
  * One update at a time per sampler; the sampler's next sample() waits on the device for the copies. */
 int nd_sampler_host_update_begin(nd_sampler *s, int32_t *out, int32_t *row_len, void *copy_stream);
 int nd_sampler_host_update_fetch(nd_sampler *s);
@@ -169,6 +169,10 @@ int nd_host_fill_int32(int32_t *dst, int64_t n, int32_t value);
  * nor copies through a staging buffer. */
 int nd_result_alloc(int device, int64_t bytes, void **p);
 int nd_result_free(void *p);
+/* Pinned host memory, zero.  Row lengths in it, beside a pinned `out`, let the GPU write a share of the rows of an
+ * update itself (in finish; a sample() between fetch and finish then waits until that share is on the host). */
+int nd_pinned_alloc(int device, int64_t bytes, void **p);
+int nd_pinned_free(void *p);
 /* The same packing between GPUs (no counterpart in the reference, which concatenates dense per-device arrays on the
  * host, src/nextdoor.cu:3211-3237).  nd_sampler_pack_rows enqueues the packing on the sampler's stream and returns
  * the device addresses of the row lengths [num_samples] and of the packed vertices (valid until the sampler's next

@@ -80,6 +80,8 @@ _SIGS = {
     "nd_sampler_host_update_finish": (C.c_int, [VP, C.POINTER(C.c_int64)]),
     "nd_result_alloc": (C.c_int, [C.c_int, C.c_int64, VP]),
     "nd_result_free": (C.c_int, [VP]),
+    "nd_pinned_alloc": (C.c_int, [C.c_int, C.c_int64, VP]),
+    "nd_pinned_free": (C.c_int, [VP]),
     "nd_host_fill_int32": (C.c_int, [VP, C.c_int64, C.c_int32]),
     "nd_sampler_pack_rows": (C.c_int, [VP, C.POINTER(VP), C.POINTER(VP)]),
     "nd_sampler_pack_rows_total": (C.c_int, [VP, C.POINTER(C.c_int64)]),

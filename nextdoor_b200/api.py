@@ -41,6 +41,20 @@ class _ResultMemory:
             self._free(self._p)
 
 
+class _PinnedMemory:
+    """Pinned memory of an array that the GPU reads and writes, zero to begin with."""
+
+    def __init__(self, count, dtype, device):
+        p = C.c_void_p()
+        check(lib.nd_pinned_alloc(device, count * np.dtype(dtype).itemsize, C.byref(p)))
+        self._free, self._p = lib.nd_pinned_free, p
+        self.__array_interface__ = {"version": 3, "shape": (count,), "typestr": np.dtype(dtype).str, "data": (p.value, False)}
+
+    def __del__(self):
+        if getattr(self, "_p", None):
+            self._free(self._p)
+
+
 def _result_array(count, dtype, device):
     """np.empty for results; large ones in memory that is not faulted in again for every call."""
     large = 2 << 20 <= count * np.dtype(dtype).itemsize <= 128 << 20
@@ -399,7 +413,10 @@ class PipelinedSampler:
         key = (out_host.__array_interface__["data"][0], out_host.size)
         if key not in self._row_len:
             host_fill(out_host, self.invalid)
-            self._row_len[key] = np.zeros(self.S, np.int32)
+            try:
+                self._row_len[key] = np.asarray(_PinnedMemory(max(self.S, 1), np.int32, self.device))[:self.S]
+            except NdError:                               # no memory to pin: the host threads write all rows
+                self._row_len[key] = np.zeros(self.S, np.int32)
         return self._row_len[key]
 
     def forget(self, out_host):
@@ -424,8 +441,8 @@ class PipelinedSampler:
             total = 0
             try:
                 for i, smp in enumerate(parts):           # a chunk's rows are written while the next one's vertices cross
-                    if not fetched:
-                        for ahead in parts[i + 1 if i else 0:i + 2]:
+                    if not fetched:                       # (the first one's while the second is sampled)
+                        for ahead in parts[:1] if i == 0 else parts[1:3] if i == 1 else parts[i + 1:i + 2]:
                             ahead.host_update_fetch()
                     total += smp.host_update_finish()
             except Exception:

@@ -286,6 +286,7 @@ int nd_sampler_sample(nd_sampler *s, int mode) {
   }
   s->sampled = true;
   if (s->S == 0) return ND_OK;
+  ND_TRY(nd_hostrows_keep(s));
   if (s->copy_pending) {  // a result copy on another stream still reads the buffers this job overwrites
     ND_CUDA(cudaStreamWaitEvent(s->stream, s->copy_done, 0));
     s->copy_pending = false;

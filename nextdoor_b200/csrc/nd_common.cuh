@@ -279,6 +279,7 @@ struct nd_sampler {
   int64_t host_stats[8] = {0};
 };
 void nd_hostrows_free(nd_sampler *s);
+int nd_hostrows_keep(nd_sampler *s);
 
 // phase timing helpers (no-ops unless profiling is on)
 void nd_phase_begin(nd_sampler *s, int phase);

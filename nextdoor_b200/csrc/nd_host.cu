@@ -482,6 +482,21 @@ extern "C" int nd_result_free(void *p) {
   return ND_OK;
 }
 
+extern "C" int nd_pinned_alloc(int device, int64_t bytes, void **p) {
+  ND_REQUIRE(p && bytes > 0, ND_ERR_ARG, "nd_pinned_alloc: bad argument");
+  ND_CUDA(cudaSetDevice(device));
+  void *q = nullptr;
+  ND_CUDA(cudaHostAlloc(&q, (size_t)bytes, cudaHostAllocPortable));
+  memset(q, 0, (size_t)bytes);
+  *p = q;
+  return ND_OK;
+}
+
+extern "C" int nd_pinned_free(void *p) {
+  if (p) ND_CUDA(cudaFreeHost(p));
+  return ND_OK;
+}
+
 void nd_objects_add(int n) {
   std::lock_guard<std::mutex> lock(g_objects_mutex);
   g_objects += n;

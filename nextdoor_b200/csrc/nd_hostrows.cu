@@ -12,7 +12,13 @@
 // previous update of that array.  Three calls, so that the caller can overlap them with the next
 // job's sampling: begin (enqueue) -> fetch (lengths have landed: enqueue the vertices) -> finish
 // (vertices have landed: write the rows).
-#include <vector>
+//
+// Where the GPU can reach the caller's array and lengths (pinned memory) it writes a share of the rows itself, while the
+// host threads write the others: the threads are bound by a cache line of the array or two per row, the GPU by the wire,
+// and neither takes the other's time (2^21 rows of PPR: 2.3 ms by 16 threads, 2.2 by the GPU).
+#include <algorithm>
+
+#include <cuda.h>
 
 #include "nd_common.cuh"
 #include "nd_host.h"
@@ -32,6 +38,9 @@ struct NdHostRows {
   uint32_t *h_chunk = nullptr;  // pinned: d_chunk of the job being copied
   bool dense = false;           // most slots are in use: the dense array is copied as it is
   int stage = 0;                // 0 idle, 1 begun, 2 fetched
+  int64_t direct = 0;           // rows from the front that the GPU writes
+  int32_t *dev_out = nullptr, *dev_row_len = nullptr;   // ... where it finds the caller's arrays
+  cudaStream_t ds = nullptr;    // ... and the stream it does it on
   int threads = 1;
 };
 
@@ -49,7 +58,9 @@ struct WarpRows {
   uint32_t total;       // of the warp
   size_t pos;           // of the warp's first vertex
 
-  __device__ __forceinline__ WarpRows(const int32_t *__restrict__ lens, int64_t row, int64_t S, const uint32_t *__restrict__ chunk_base, uint32_t *wsum) {
+  // `block`: the CTA's place among those of all rows; the packed array begins with the rows of chunk `chunk0`
+  __device__ __forceinline__ WarpRows(const int32_t *__restrict__ lens, int64_t row, int64_t S, const uint32_t *__restrict__ chunk_base, uint32_t *wsum,
+                                      uint32_t block, uint32_t chunk0) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     len = row < S ? (uint32_t)lens[row] : 0u;
     inc = len;
@@ -60,12 +71,12 @@ struct WarpRows {
     total = __shfl_sync(0xffffffffu, inc, 31);
     // the rows of the chunk before the CTA's: a few loads that neighbouring CTAs share
     uint32_t before = 0;
-    for (int64_t r = (int64_t)(blockIdx.x / (PACK_CHUNK / PACK_ROWS)) * PACK_CHUNK + threadIdx.x; r < (int64_t)blockIdx.x * PACK_ROWS; r += PACK_ROWS)
+    for (int64_t r = (int64_t)(block / (PACK_CHUNK / PACK_ROWS)) * PACK_CHUNK + threadIdx.x; r < (int64_t)block * PACK_ROWS; r += PACK_ROWS)
       before += (uint32_t)lens[r];
     before = __reduce_add_sync(0xffffffffu, before);
     if (lane == 0) { wsum[warp] = total; wsum[PACK_ROWS / 32 + warp] = before; }
     __syncthreads();
-    pos = chunk_base[blockIdx.x / (PACK_CHUNK / PACK_ROWS)];
+    pos = chunk_base[block / (PACK_CHUNK / PACK_ROWS)] - chunk_base[chunk0];
     for (int w = 0; w < PACK_ROWS / 32; w++) pos += wsum[PACK_ROWS / 32 + w] + (w < warp ? wsum[w] : 0u);
   }
   // fn(lane of the row, slot in the row, place in the warp's packed vertices)
@@ -134,7 +145,7 @@ unpack_rows_kernel(const int32_t *__restrict__ len, const int32_t *__restrict__ 
                    int64_t S, int steps, int32_t invalid, int32_t *__restrict__ out, int32_t *__restrict__ row_len) {
   __shared__ uint32_t wsum[PACK_ROWS / 16];
   const int64_t mine = (int64_t)blockIdx.x * PACK_ROWS + threadIdx.x, first = mine - (threadIdx.x & 31);
-  const WarpRows rows(len, mine, S, chunk_base, wsum);
+  const WarpRows rows(len, mine, S, chunk_base, wsum, blockIdx.x, 0u);
   rows.each([&](int r, uint32_t slot, uint32_t k) { out[(first + r) * steps + slot] = vals[rows.pos + k]; });
   if (mine >= S) return;
   const int32_t had = row_len[mine];
@@ -142,14 +153,82 @@ unpack_rows_kernel(const int32_t *__restrict__ len, const int32_t *__restrict__ 
   if (had != (int)rows.len) row_len[mine] = (int32_t)rows.len;
 }
 
-// the rows' prefixes to vals, back to back
+// the prefixes of the rows from chunk `chunk0` on to vals, back to back
 __global__ void __launch_bounds__(PACK_ROWS)
 pack_rows_kernel(const int32_t *__restrict__ plen, const int32_t *__restrict__ out, int64_t S, int steps,
-                 const uint32_t *__restrict__ chunk_base, int32_t *__restrict__ vals) {
+                 const uint32_t *__restrict__ chunk_base, uint32_t chunk0, int32_t *__restrict__ vals) {
   __shared__ uint32_t wsum[PACK_ROWS / 16];
-  const int64_t mine = (int64_t)blockIdx.x * PACK_ROWS + threadIdx.x, first = mine - (threadIdx.x & 31);
-  const WarpRows rows(plen, mine, S, chunk_base, wsum);
+  const uint32_t block = blockIdx.x + chunk0 * (PACK_CHUNK / PACK_ROWS);
+  const int64_t mine = (int64_t)block * PACK_ROWS + threadIdx.x, first = mine - (threadIdx.x & 31);
+  const WarpRows rows(plen, mine, S, chunk_base, wsum, block, chunk0);
   rows.each([&](int r, uint32_t slot, uint32_t k) { vals[rows.pos + k] = out[(first + r) * steps + slot]; });
+}
+
+// The first `n` rows of the sampler's array into the caller's: the 64-byte lines of every row that hold a slot a walk fills
+// now or filled at the array's previous update, whole, as the sampler's array holds the invalid id behind a row's
+// vertices too.  Bound by the wire: 1.1 M rows of 2^21 are 1.8 M lines, 2.2 ms at 52 GB/s; the vertices alone
+// are 1.5 M writes of 4 to 32 bytes and take 2.9, their 32-byte sectors 2.4.  Two lanes to a line; 128 threads of 32
+// registers find room beside the kernel that samples the next chunk.
+constexpr int DIRECT_THREADS = 128;
+__global__ void __launch_bounds__(DIRECT_THREADS, 16)
+direct_rows_kernel(const int32_t *__restrict__ plen, const int32_t *__restrict__ from, int64_t n, int steps, int32_t *out, int32_t *row_len) {
+  const int lane = threadIdx.x & 31;
+  const int64_t shift = (int64_t)((uintptr_t)out / 4 % 16);   // the array begins that many slots into a line
+  for (int64_t first = (int64_t)blockIdx.x * DIRECT_THREADS + threadIdx.x - lane; first < n; first += (int64_t)gridDim.x * DIRECT_THREADS) {
+    const int64_t mine = first + lane;
+    const int32_t now = mine < n ? plen[mine] : 0, had = mine < n ? row_len[mine] : 0, len = now > had ? now : had;
+    if (__any_sync(0xffffffffu, now != had) && mine < n) row_len[mine] = now;
+    const int64_t line0 = (mine * steps + shift) / 16;
+    const uint32_t lines = len > 0 ? (uint32_t)((mine * steps + len - 1 + shift) / 16 - line0) + 1u : 0u;
+    uint32_t inc = lines;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += u;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
+    for (uint32_t base = 0; base < total; base += 16) {
+      const uint32_t k = base + lane / 2;
+      int r = 0;
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1)
+        if (__shfl_sync(0xffffffffu, inc, r + step - 1) <= k) r += step;
+      const int64_t line = __shfl_sync(0xffffffffu, line0 - (int64_t)(inc - lines), r & 31) + k;
+      if (k >= total) continue;
+      const int64_t at = line * 16 + lane % 2 * 8 - shift;   // eight slots
+      if (at >= 0 && at + 8 <= n * steps) {
+        int32_t v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) v[j] = from[at + j];
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(out + at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]),
+                     "r"(v[5]), "r"(v[6]), "r"(v[7])
+                     : "memory");
+      } else {
+        for (int j = 0; j < 8; j++)
+          if (at + j >= 0 && at + j < n * steps) out[at + j] = from[at + j];
+      }
+    }
+  }
+}
+
+// Where the GPU finds `bytes` of host memory at `p`: inside one pinned allocation or registration, or null.
+void *reachable(const void *p, size_t bytes) {
+  static const auto range = []() -> CUresult (*)(unsigned int, CUpointer_attribute *, void **, CUdeviceptr) {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess) f = nullptr;
+    cudaGetLastError();
+    return (CUresult(*)(unsigned int, CUpointer_attribute *, void **, CUdeviceptr))f;
+  }();
+  cudaPointerAttributes at;
+  if (!range || cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  if (at.type != cudaMemoryTypeHost || !at.devicePointer || at.devicePointer != p) return nullptr;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  CUpointer_attribute what[2] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void *into[2] = {&start, &size};
+  if (range(2, what, into, (CUdeviceptr)p) != CUDA_SUCCESS) return nullptr;
+  const uintptr_t a = (uintptr_t)p, s0 = (uintptr_t)start;
+  return a >= s0 && a - s0 <= size && bytes <= size - (a - s0) ? at.devicePointer : nullptr;
 }
 
 // positions in the packed array are 32-bit
@@ -181,21 +260,68 @@ int hostrows_init(nd_sampler *s) {
   return ND_OK;
 }
 
-// the rows' prefixes packed into the staging array of the walk (free between two passes), on the sampler's stream
-int pack_enqueue(nd_sampler *s) {
+// The rows that the GPU writes itself, whole chunks from the front: as fast as 16 host threads (above).  The host's memory
+// serves both, so that they are not twice as fast together: jobs of 2^21 rows 3.2 -> 2.4 ms with half of them, 2.8 with
+// a third and with all, 2.7 with three quarters.
+int64_t direct_rows(nd_sampler *s, int32_t *out, int32_t *row_len) {
+  NdHostRows *h = s->hostrows;
+  if (s->S < 4 * PACK_CHUNK || (uintptr_t)out % 4 || (uintptr_t)row_len % 4) return 0;
+  h->dev_out = (int32_t *)reachable(out, sizeof(int32_t) * (size_t)s->S * s->fs);
+  h->dev_row_len = (int32_t *)reachable(row_len, sizeof(int32_t) * (size_t)s->S);
+  if (!h->dev_out || !h->dev_row_len) return 0;
+  if (!h->ds && cudaStreamCreateWithFlags(&h->ds, cudaStreamNonBlocking) != cudaSuccess) { cudaGetLastError(); h->ds = nullptr; return 0; }
+  return s->S * 16 / (16 + h->threads) / PACK_CHUNK * PACK_CHUNK;
+}
+
+// the prefixes of the rows from `first` on (a chunk's) packed into the staging array of the walk (free between two
+// passes), on the sampler's stream
+int pack_enqueue(nd_sampler *s, int64_t first) {
   NdHostRows *h = s->hostrows;
   ND_TRY(nd_walk_ensure_tmp(s));
   pack_sum_kernel<<<h->n_chunks, PACK_ROWS, 0, s->stream>>>(s->d_plen, s->S, h->d_chunk);
   pack_scan_kernel<<<1, 1024, 0, s->stream>>>(h->d_chunk, h->n_chunks);
-  pack_rows_kernel<<<(unsigned)((s->S + PACK_ROWS - 1) / PACK_ROWS), PACK_ROWS, 0, s->stream>>>(s->d_plen, s->d_out, s->S, s->fs, h->d_chunk, s->d_tmp);
+  pack_rows_kernel<<<(unsigned)((s->S - first + PACK_ROWS - 1) / PACK_ROWS), PACK_ROWS, 0, s->stream>>>(s->d_plen, s->d_out, s->S, s->fs, h->d_chunk,
+                                                                                                       (uint32_t)(first / PACK_CHUNK), s->d_tmp);
   nd_count_launches(3);
   ND_CUDA(cudaGetLastError());
   return ND_OK;
 }
 
+// the packed vertices to the host, once the chunks' sums are there
+int fetch_vals(nd_sampler *s, cudaStream_t st) {
+  NdHostRows *h = s->hostrows;
+  const size_t n = (size_t)h->total - h->h_chunk[h->direct / PACK_CHUNK];
+  if (n > h->vals_cap) {
+    if (h->h_vals) ND_CUDA(cudaFreeHost(h->h_vals));
+    h->h_vals = nullptr;
+    h->vals_cap = 0;
+    const size_t cap = n + n / 4 + 4096;
+    ND_CUDA(cudaMallocHost(&h->h_vals, sizeof(int32_t) * cap));
+    h->vals_cap = cap;
+  }
+  if (n > 0) ND_CUDA(cudaMemcpyAsync(h->h_vals, s->d_tmp, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
+  return ND_OK;
+}
+
 }  // namespace
 
-void nd_hostrows_free(nd_sampler *s);
+// The sampler's array is about to change while the GPU has rows of it left to write: these go to the host threads, too.
+int nd_hostrows_keep(nd_sampler *s) {
+  NdHostRows *h = s->hostrows;
+  if (!h || h->stage == 0 || h->direct == 0) return ND_OK;
+  const int stage = h->stage;
+  h->stage = 0;   // an error below abandons the update
+  ND_CUDA(cudaEventSynchronize(h->len_done));
+  if (stage == 2) ND_CUDA(cudaEventSynchronize(h->vals_done));
+  h->direct = 0;
+  h->total = (int64_t)h->h_chunk[h->n_chunks];
+  ND_TRY(pack_enqueue(s, 0));
+  ND_CUDA(cudaMemcpyAsync(h->h_len, s->d_plen, sizeof(int32_t) * (size_t)s->S, cudaMemcpyDeviceToHost, s->stream));
+  if (stage == 2) ND_TRY(fetch_vals(s, s->stream));
+  ND_CUDA(cudaStreamSynchronize(s->stream));
+  h->stage = stage;
+  return ND_OK;
+}
 
 void nd_hostrows_free(nd_sampler *s) {
   NdHostRows *h = s->hostrows;
@@ -205,6 +331,7 @@ void nd_hostrows_free(nd_sampler *s) {
   if (h->h_chunk) cudaFreeHost(h->h_chunk);
   cudaFree(h->d_chunk);
   if (h->vs) cudaStreamDestroy(h->vs);
+  if (h->ds) cudaStreamDestroy(h->ds);
   if (h->packed) cudaEventDestroy(h->packed);
   if (h->len_done) cudaEventDestroy(h->len_done);
   if (h->vals_done) cudaEventDestroy(h->vals_done);
@@ -238,12 +365,13 @@ int nd_sampler_host_update_begin(nd_sampler *s, int32_t *out, int32_t *row_len, 
   h->cs = copy_stream ? (cudaStream_t)copy_stream : s->stream;
   if (s->S == 0) { h->stage = 1; return ND_OK; }
   // (an error below leaves stage 0: nothing was begun as far as the caller is concerned)
-  if (packable(s)) ND_TRY(pack_enqueue(s));   // (larger arrays take the dense copy in fetch)
+  h->direct = packable(s) ? direct_rows(s, out, row_len) : 0;
+  if (packable(s)) ND_TRY(pack_enqueue(s, h->direct));   // (larger arrays take the dense copy in fetch)
   if (h->cs != s->stream) {
     ND_CUDA(cudaEventRecord(h->packed, s->stream));
     ND_CUDA(cudaStreamWaitEvent(h->cs, h->packed, 0));
   }
-  ND_CUDA(cudaMemcpyAsync(h->h_len, s->d_plen, sizeof(int32_t) * (size_t)s->S, cudaMemcpyDeviceToHost, h->cs));
+  ND_CUDA(cudaMemcpyAsync(h->h_len + h->direct, s->d_plen + h->direct, sizeof(int32_t) * (size_t)(s->S - h->direct), cudaMemcpyDeviceToHost, h->cs));
   if (packable(s))
     ND_CUDA(cudaMemcpyAsync(h->h_chunk, h->d_chunk, sizeof(uint32_t) * ((size_t)h->n_chunks + 1), cudaMemcpyDeviceToHost, h->cs));
   ND_CUDA(cudaEventRecord(h->len_done, h->cs));
@@ -270,16 +398,10 @@ int nd_sampler_host_update_fetch(nd_sampler *s) {
   h->dense = 2 * h->total > s->S * (int64_t)s->fs || !packable(s);
   if (h->dense) {
     ND_CUDA(cudaMemcpyAsync(h->out, s->d_out, sizeof(int32_t) * (size_t)s->S * s->fs, cudaMemcpyDeviceToHost, h->vs));
+    if (h->direct) ND_CUDA(cudaMemcpyAsync(h->h_len, s->d_plen, sizeof(int32_t) * (size_t)h->direct, cudaMemcpyDeviceToHost, h->vs));
+    h->direct = 0;
   } else if (h->total > 0) {
-    if ((size_t)h->total > h->vals_cap) {
-      if (h->h_vals) ND_CUDA(cudaFreeHost(h->h_vals));
-      h->h_vals = nullptr;
-      h->vals_cap = 0;
-      const size_t cap = (size_t)h->total + (size_t)h->total / 4 + 4096;
-      ND_CUDA(cudaMallocHost(&h->h_vals, sizeof(int32_t) * cap));
-      h->vals_cap = cap;
-    }
-    ND_CUDA(cudaMemcpyAsync(h->h_vals, s->d_tmp, sizeof(int32_t) * (size_t)h->total, cudaMemcpyDeviceToHost, h->vs));
+    ND_TRY(fetch_vals(s, h->vs));
   }
   ND_CUDA(cudaEventRecord(h->vals_done, h->vs));
   if (!s->copy_done) ND_CUDA(cudaEventCreateWithFlags(&s->copy_done, cudaEventDisableTiming));
@@ -311,8 +433,17 @@ int nd_sampler_host_update_finish(nd_sampler *s, int64_t *values_copied) {
     return ND_OK;
   }
   const uint32_t *chunk = h->h_chunk;
-  nd_host_ranges(s->S, h->threads, [=](int, int64_t a, int64_t b) {
-    const int32_t *src = vals + chunk[a / PACK_CHUNK];   // the position of the range's first row in the packed array
+  const int64_t direct = h->direct;
+  const cudaStream_t ds = h->ds;
+  if (direct) {
+    const int grid = (int)std::min<int64_t>((direct + DIRECT_THREADS - 1) / DIRECT_THREADS, (int64_t)s->dev.sms * 4);
+    direct_rows_kernel<<<grid, DIRECT_THREADS, 0, ds>>>(s->d_plen, s->d_out, direct, steps, h->dev_out, h->dev_row_len);
+    nd_count_launches(1);
+    ND_CUDA(cudaGetLastError());
+  }
+  nd_host_ranges(s->S - direct, h->threads, [=](int, int64_t a, int64_t b) {
+    a += direct; b += direct;
+    const int32_t *src = vals + (chunk[a / PACK_CHUNK] - chunk[direct / PACK_CHUNK]);   // the position of the range's first row in the packed array
     for (int64_t i = a - a % PACK_CHUNK; i < a; i++) src += len[i];
     constexpr int AHEAD = 24;   // rows lie apart and are not in any cache: ask for them before they are written
     for (int64_t i = a; i < b; i++) {
@@ -325,6 +456,7 @@ int nd_sampler_host_update_finish(nd_sampler *s, int64_t *values_copied) {
       if (now != had) row_len[i] = now;
     }
   });
+  if (direct) ND_CUDA(cudaStreamSynchronize(ds));
   return ND_OK;
 }
 
@@ -344,7 +476,7 @@ int nd_sampler_pack_rows(nd_sampler *s, const int32_t **d_row_len, const int32_t
   *d_vals = s->d_tmp;
   *h->h_total = 0;
   if (s->S > 0) {
-    ND_TRY(pack_enqueue(s));
+    ND_TRY(pack_enqueue(s, 0));
     ND_CUDA(cudaMemcpyAsync(h->h_total, h->d_chunk + h->n_chunks, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
   }
   ND_CUDA(cudaEventRecord(h->total_done, s->stream));

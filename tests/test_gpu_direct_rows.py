@@ -1,0 +1,60 @@
+"""Rows of a caller's pinned array that the GPU writes itself: lines that begin anywhere, shares at whole chunks of rows, rows
+that shrink and grow, arrays that turn dense, and a job that starts before the last one's rows are written."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _pinned(n, offset, fill):
+    return torch.full((n + offset,), fill, dtype=torch.int32).pin_memory().numpy()[offset:]
+
+
+@pytest.mark.parametrize("S,steps,offset", [(1 << 14, 7, 0), ((1 << 14) + 1, 100, 1), (20479, 16, 3), (40961, 101, 13), (65536, 5, 5)])
+def test_rows_in_pinned_memory(nd, small_graph, S, steps, offset):
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    rng = np.random.default_rng(S)
+    out = _pinned(S * steps + 16, offset, g.V)
+    out[S * steps:] = -7                                  # behind the array
+    row_len = _pinned(S, 0, 0)
+    samplers = [nd.Sampler(g, nd.app_params(2, steps=steps, seed=k, stop_prob=p), num_samples=S) for k, p in ((1, 0.3), (2, 0.05), (3, 0.0005))]
+    for job in range(7):
+        s = samplers[(0, 1, 0, 2, 0, 1, 1)[job]]
+        s.set_initial(rng.integers(-1, g.V, S).astype(np.int32))
+        s.sample(1)
+        exp = s.final_samples()
+        s.host_update_begin(out[:S * steps], row_len)
+        if job == 4:                                      # the next job of the sampler begins before the rows are written
+            s.set_initial(rng.integers(0, g.V, S).astype(np.int32))
+            s.sample(1)
+        if job >= 5:
+            s.host_update_fetch()
+        if job == 5:
+            s.set_initial(rng.integers(0, g.V, S).astype(np.int32))
+            s.sample(1)
+        assert s.host_update_finish() >= (exp != g.V).sum()
+        assert np.array_equal(out[:S * steps].reshape(S, steps), exp), job
+        assert np.array_equal(row_len, (exp != g.V).sum(axis=1)), job
+        assert (out[S * steps:S * steps + 16] == -7).all()
+
+
+@pytest.mark.parametrize("depth", [1, 2])
+def test_pipeline_into_pinned_arrays(nd, small_graph, depth):
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    S, rng = 70001, np.random.default_rng(depth)
+    pr = nd.app_params(2, steps=40, seed=9, stop_prob=0.15)
+    outs = [_pinned(S * 40, k, 0) for k in range(2)]
+    streams = torch.cuda.Stream(), torch.cuda.Stream()
+    pipe = nd.PipelinedSampler(g, pr, S, chunks=3, depth=depth, stream=streams[0].cuda_stream, copy_stream=streams[1].cuda_stream, sparse_rows=True)
+    whole = nd.Sampler(g, pr, num_samples=S)
+    seeds = [rng.integers(0, g.V, S).astype(np.int32) for _ in range(6)]
+    for k, init in enumerate(seeds):                      # back to back, the arrays in turn and the same one twice
+        pipe.run_async(init, outs[(0, 1, 1, 0, 1, 0)[k]])
+        if k in (1, 3):
+            pipe.wait()
+    pipe.wait()
+    for out, k in ((outs[0], 5), (outs[1], 4)):
+        whole.set_initial(seeds[k])
+        whole.sample(1)
+        assert np.array_equal(out.reshape(S, 40), whole.final_samples()), k
