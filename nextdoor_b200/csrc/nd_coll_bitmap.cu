@@ -1,16 +1,16 @@
 // Importance-sampled layers (FastGCN, LADIES): a CTA per sample, all layers of all samples in one launch.
 //
 // The union of a sample's neighbour lists is a bitmap with a bit per vertex; the rank of a set bit is the
-// candidate's index in the sorted unique union, so nothing is sorted.  Candidate weights are summed per group (FastGCN:
-// of 512 vertices, LADIES: of 512 candidates) in fp64 and scanned; a draw bisects the group sums and finds its candidate
+// candidate's place in the sorted unique union, so nothing is sorted.  Candidate weights are summed per group (FastGCN:
+// of 512 vertices, LADIES: of 128) in fp64 and scanned; a draw bisects the group sums and finds its candidate
 // inside one group with a warp.  Sums are fp64, so they agree with the sorted sequential order to ~1e-16 (FastGCN's
 // integer weights sum exactly).
 //
 // What bounds it, and what is done about it (2^20 vertices, 1024 batches of 64, 2 layers of 64: FastGCN
-// 4.8 -> 0.98 ms, LADIES 5.7 -> 2.44 ms).  One CTA fills an SM, and neither memory nor issue slots are full: FastGCN issues
-// in 58 % of the cycles (612 M warp instructions; 5.6 GB out of the L2 at 24 % of its rate), LADIES in 46 % (1.09 G
-// instructions for 131 M list entries, the distinct ones of 313 M); the warps wait for barriers between the phases, for
-// shared memory and for loads:
+// 4.8 -> 0.98 ms, LADIES 5.7 -> 1.07 ms).  One CTA fills an SM, and neither memory nor issue slots are full: FastGCN issues
+// in 58 % of the cycles (612 M warp instructions; 5.6 GB out of the L2 at 24 % of its rate), LADIES in 57 % (610 M
+// instructions for 131 M list entries, the distinct ones of 313 M), its shared memory is busy in half of them; the warps
+// wait for barriers between the phases, for shared memory and for loads:
 //  * The second layer's transits are hubs (FastGCN draws them with the square of their degree), many of them the
 //    same one: repeated transits of a batch are taken once (LADIES with their multiplicity).
 //  * A hub's list (up to 140 K ids; FastGCN's second layer has 28 distinct hubs a sample) costs a shared-memory test per id.  Vertices with at least V/128 neighbours
@@ -21,10 +21,16 @@
 //    16-byte load, masks them with its byte of the bitmap and squares and sums them with dp4a.  Vertices with 2048
 //    neighbours or more, whose squares would overflow the 32-bit group sums, are a short list per graph.
 //  * LADIES' terms (w / rowsum)^2 depend on the edge alone: an array, built once per graph, instead of a pass over
-//    the weights and a division per entry and sample.  They are added up in shared memory, in tiles of
-//    consecutive candidates (lists are sorted, so a tile is a range of every list, all of them searched for at
-//    once), not with atomics on global memory.  CSR arrays of a caller may hold rows in any order: those lists are gone
-//    through whole for every tile.
+//    the weights and a division per entry and sample.  One pass over the lists sets the union's bits and adds the terms
+//    up per group; then the groups that the draws fall into get an accumulator per vertex, where the union was,
+//    and a second pass adds up the terms of their candidates alone (131 K entries, 37 of 8192 groups, 9 % of the entries).
+//    No order of the lists is asked for.  (Until then the candidates' weights were added up by rank, in tiles of shared
+//    memory: the rank of every entry, a double added per entry, a few barriers per tile; 1024 batches on 2^20 vertices 2.50
+//    -> 1.07 ms, 256 on 2^21 1.37 -> 0.64, 700 batches of 100 and 3 layers of 100 on 100 K 1.52 -> 0.88.)  A thread
+//    takes eight entries, 32 bytes of ids and of terms; what neighbouring entries add to one group is added up in
+//    registers and across the lanes first, as a 64-bit add in shared memory costs 18 cycles a warp.  Groups of 128: with
+//    larger ones the second pass adds more, with smaller ones the first (64: 1.08, 256: 1.05 ms, but 0.29 instead of 0.25
+//    with 300 batches on 500 K).
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
@@ -36,25 +42,28 @@ namespace {
 
 using ndrng::Rng;
 
-constexpr int GROUP_WORDS = 16;   // words whose candidates are counted together
-constexpr int GROUP = 512;        // candidates (FastGCN: vertices, GROUP_WORDS words) whose weights are summed together
+constexpr int GROUP_WORDS = 16;   // words of a FastGCN group; bitmaps are whole ones
+constexpr int GROUP = 512;        // FastGCN: vertices (GROUP_WORDS words) whose weights are summed together
+constexpr int LADIES_GROUP_BITS = 7;   // LADIES: 2^7 vertices, more where the sums of the groups would not fit shared memory
 constexpr int BIG_DEGREE = 2048;  // from here a vertex is on the list of big ones and its code is 0: 512 * 2047^2 < 2^31
 constexpr int FLIGHT = 4;         // groups a warp sums at a time
 constexpr int HUB = 128, LADIES_HUB = 64;   // a vertex with at least V / HUB neighbours has a bitmap of them, and is ORed from V / LADIES_HUB on
 constexpr int BIG_LIST = 4096;    // lists at least this long are streamed by the whole CTA
 constexpr int VEC = 4;            // 16-byte loads in flight per thread
-constexpr int CHUNK = 128;        // list entries a warp takes at a time (LADIES)
-constexpr int CHUNK_LOADS = CHUNK / 32;
+constexpr int OCT = 8;            // list entries a thread takes at a time: 32 aligned bytes (LADIES)
 
-// The bitmap, the counts of groups and quads of words and the CDF make the "big" part (V/8 + 5V/128 bytes).  It lives in
-// shared memory when the whole layout fits the CTA's opt-in shared memory (graphs up to about 1.2 M vertices) and
-// otherwise in a per-CTA slice of a global scratch array (glob_bytes > 0), where the same code runs on L2-resident
-// words.  The rest is always in shared memory.
+// The bitmap and FastGCN's CDF make the "big" part (V/8 + V/64 bytes).  It lives in shared memory when the whole layout
+// fits the CTA's opt-in shared memory (graphs up to about 1.2 M vertices) and otherwise in a per-CTA slice of a global
+// scratch array (glob_bytes > 0), where the same code runs on L2-resident words.  The rest is always in shared memory.
 struct Layout {
   int words, groups;
-  uint32_t off_gcdf, off_gpref, off_qpre;              // inside the big part (the bitmap is at 0)
-  uint32_t off_red, off_tr, off_layer, off_ut, off_mult, off_pre, off_tile;   // inside shared memory
-  uint32_t tile;                                       // accumulators in shared memory (LADIES)
+  int group_bits;                                      // LADIES: vertices of a group, as a power of two
+  int slots;                                           // LADIES: groups with accumulators at a time
+  uint32_t off_gcdf;                                   // FastGCN: inside the big part (the bitmap is at 0); LADIES: inside shared memory, unless sums_far
+  bool sums_far;
+  uint32_t off_red, off_tr, off_layer, off_ut, off_mult, off_pre;   // inside shared memory
+  uint32_t off_draw, off_there, off_acc;                // LADIES: the same; the accumulators may be where the bitmap is
+  uint32_t off_slot;                                   // LADIES: with the groups' sums
   uint32_t bytes;                                      // dynamic shared memory of the launch
   uint32_t glob_bytes;                                 // per-CTA slice of the global scratch, 0 = big part in shared memory
 };
@@ -68,10 +77,6 @@ struct Args {
   unsigned char *gscratch;
   const int32_t *initial;
   int32_t *out;
-  float *wts_all;                          // LADIES: [CTAs][V] the candidates' weights, in order
-  int32_t *pos_all;                        // LADIES: [CTAs][tiles + 1][transits] where the tiles begin in the lists
-  int pos_stride;                          // ... entries per CTA
-  int sorted;                              // LADIES: the lists ascend, so that a tile is a range of each
   int32_t *adj_row, *adj_col;
   float *prob;
   const uint4 *__restrict__ deg;           // FastGCN: the degrees of eight vertices, low bytes (x, y), high bytes (z, w)
@@ -87,6 +92,8 @@ struct Args {
 
 // a transit of the batch: row start, degree, how often it occurs, bitmap slot
 struct Transit { int32_t rs, deg, mult, slot; };
+
+constexpr uint32_t NO_SLOT = 255u;
 
 __device__ __forceinline__ void mark(uint32_t *bm, int32_t v) {
   const uint32_t bit = 1u << (v & 31);
@@ -140,49 +147,178 @@ __device__ __forceinline__ uint32_t scan_u32(uint32_t *a, int n, uint32_t *red) 
   return total;
 }
 
+// (a warp takes whole rows of 32, so that neighbouring lanes read neighbouring words)
 __device__ __forceinline__ void scan_f64(double *a, int n, double *red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int per = (n + blockDim.x - 1) / blockDim.x;
-  const int b = min((int)threadIdx.x * per, n), e = min(b + per, n);
-  double sum = 0.0;
-  for (int i = b; i < e; i++) sum += a[i];
-  double inc = sum;
-  for (int o = 1; o < 32; o <<= 1) {
-    const double t = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += t;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int per = ((n + 31) / 32 + warps - 1) / warps * 32, b = warp * per;
+  double carry = 0.0;
+  for (int i0 = b; i0 < b + per && i0 < n; i0 += 32) {
+    const int i = i0 + lane;
+    double run = i < n ? a[i] : 0.0;
+    for (int o = 1; o < 32; o <<= 1) {
+      const double t = __shfl_up_sync(0xffffffffu, run, o);
+      if (lane >= o) run += t;
+    }
+    run += carry;
+    if (i < n) a[i] = run;
+    carry = __shfl_sync(0xffffffffu, run, 31);
   }
-  if (lane == 31) red[warp] = inc;
+  if (lane == 0) red[warp] = carry;
   __syncthreads();
-  double base = inc - sum;
+  double base = 0.0;
   for (int w = 0; w < warp; w++) base += red[w];
-  for (int i = b; i < e; i++) { base += a[i]; a[i] = base; }
+  for (int i = b + lane; i < b + per && i < n; i += 32) a[i] += base;
   __syncthreads();
 }
 
-// vertex of rank r (r < number of candidates)
-__device__ __forceinline__ int32_t vertex_of_rank(const uint32_t *bm, const uint32_t *gpref, int groups, uint32_t r) {
-  int lo = 0, hi = groups - 1;   // last group with gpref <= r
-  while (lo < hi) {
+// eight consecutive words at an address that is a multiple of 32
+__device__ __forceinline__ void load8(const int32_t *p, int32_t (&v)[OCT]) {
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "l"(p));
+}
+
+// Octs: the aligned groups of eight entries that a list touches.
+__device__ __forceinline__ uint32_t octs_of(int32_t rs, int32_t deg) { return deg > 0 ? (((uint32_t)rs + (uint32_t)deg + OCT - 1u) / OCT) - (uint32_t)rs / OCT : 0u; }
+
+// the list of oct o of all: the last with pre <= o
+__device__ __forceinline__ int list_of_oct(const uint32_t *pre, int nu, uint32_t o) {
+  int lo = 0;
+  for (int hi = nu - 1; lo < hi;) {
     const int mid = (lo + hi + 1) >> 1;
-    if (gpref[mid] <= r) lo = mid; else hi = mid - 1;
+    if (pre[mid] <= o) lo = mid; else hi = mid - 1;
   }
-  uint32_t left = r - gpref[lo];
-  for (int w = lo * GROUP_WORDS;; w++) {
-    uint32_t bits = bm[w];
-    const uint32_t c = __popc(bits);
-    if (left >= c) { left -= c; continue; }
-    while (left--) bits &= bits - 1;
-    return (w << 5) + __ffs(bits) - 1;
+  return lo;
+}
+
+// the entries of an oct that belong to the list, as bits
+__device__ __forceinline__ uint32_t oct_mask(int64_t e, const Transit &t) {
+  const int64_t lo = (int64_t)t.rs - e, hi = (int64_t)t.rs + t.deg - e;
+  return (hi >= OCT ? 0xffu : (1u << (int)hi) - 1u) & (lo <= 0 ? 0xffu : 0xffu << (int)lo);
+}
+
+// LADIES: the terms of the lists' entries into the sums of their groups, the entries of lists without a bitmap into the
+// union.  A lane takes an oct and adds up what follows in one group; what the last entries of a lane's and the first of the
+// next one's share is passed on, so that neighbouring entries of a long list cost one atomic and the lanes' atomics do not
+// meet.
+__device__ __forceinline__ void add_terms(const NdGraphView &g, const float *__restrict__ term, const Transit *ut, int ntr, int nh, int nu,
+                                          const uint32_t *pre, uint32_t total, uint32_t *bm, double *sums, int group_bits) {
+  const int lane = threadIdx.x & 31;
+  int i = 0;
+  for (uint32_t o0 = threadIdx.x - lane; o0 < total; o0 += blockDim.x) {
+    const uint32_t o = o0 + lane;
+    int first = -1, at = -1;    // the groups of the lane's first and last entries
+    double sum = 0.0, sum_first = 0.0;
+    double mult = 0.0;
+    bool several = false;
+    if (o < total) {
+      if (i + 1 < nu && pre[i + 1] <= o) i = list_of_oct(pre, nu, o);
+      const Transit t = ut[i < nh ? i : ntr - nu + i];
+      const int64_t e = ((int64_t)((uint32_t)t.rs / OCT) + (int64_t)(o - pre[i])) * OCT;
+      int32_t v[OCT], x[OCT];
+      load8(g.col + e, v);
+      load8(reinterpret_cast<const int32_t *>(term) + e, x);
+      const uint32_t in = oct_mask(e, t);
+      mult = (double)t.mult;
+      if (i >= nh) {
+        uint32_t word[OCT];
+#pragma unroll
+        for (int j = 0; j < OCT; j++) word[j] = (in >> j) & 1u ? bm[(uint32_t)v[j] >> 5] : ~0u;
+#pragma unroll
+        for (int j = 0; j < OCT; j++)
+          if (!((word[j] >> (v[j] & 31)) & 1u)) atomicOr(bm + ((uint32_t)v[j] >> 5), 1u << (v[j] & 31));
+      }
+#pragma unroll
+      for (int j = 0; j < OCT; j++) {
+        if (!((in >> j) & 1u)) continue;
+        const int group = v[j] >> group_bits;
+        if (group != at) {
+          if (at < 0) first = group;
+          else if (!several) { sum_first = sum; several = true; }
+          else atomicAdd(sums + at, sum * mult);
+          at = group;
+          sum = 0.0;
+        }
+        sum += (double)__int_as_float(x[j]);
+      }
+    }
+    const int at_before = __shfl_up_sync(0xffffffffu, at, 1), i_before = __shfl_up_sync(0xffffffffu, i, 1);
+    const bool joins = lane > 0 && first >= 0 && first == at_before && i == i_before;
+    const uint32_t joined = __ballot_sync(0xffffffffu, joins);
+    double before = 0.0;
+    if (joined) {
+      const uint32_t heads = __ballot_sync(0xffffffffu, several || !joins);
+      const int head = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+      for (int step = 1; step < 32; step <<= 1) {
+        const double t = __shfl_up_sync(0xffffffffu, sum, step);
+        if (lane - step >= head) sum += t;
+      }
+      before = __shfl_up_sync(0xffffffffu, sum, 1);
+    }
+    if (several) atomicAdd(sums + first, (joins ? sum_first + before : sum_first) * mult);
+    if (at >= 0 && !((joined >> 1 >> lane) & 1u)) atomicAdd(sums + at, sum * mult);
   }
 }
 
-// first entry of the sorted list [e0, e1) that is at least v
-__device__ __forceinline__ int32_t lower_bound(const int32_t *__restrict__ col, int32_t e0, int32_t e1, int32_t v) {
-  while (e0 < e1) {
-    const int32_t m = e0 + ((e1 - e0) >> 1);
-    if (__ldg(col + m) < v) e0 = m + 1; else e1 = m;
+// LADIES: the weights of the candidates of the groups that slot[] gives an accumulator for each vertex (NO_SLOT: none)
+__device__ __forceinline__ void add_candidates(const NdGraphView &g, const float *__restrict__ term, const Transit *ut, int ntr, int nh, int nu,
+                                               const uint32_t *pre, uint32_t total, const uint8_t *slot, double *acc, int group_bits) {
+  int i = 0;
+  for (uint32_t o = threadIdx.x; o < total; o += blockDim.x) {
+    if (i + 1 < nu && pre[i + 1] <= o) i = list_of_oct(pre, nu, o);
+    const Transit t = ut[i < nh ? i : ntr - nu + i];
+    const int64_t e = ((int64_t)((uint32_t)t.rs / OCT) + (int64_t)(o - pre[i])) * OCT;
+    int32_t v[OCT], x[OCT];
+    load8(g.col + e, v);
+    load8(reinterpret_cast<const int32_t *>(term) + e, x);
+    const uint32_t in = oct_mask(e, t);
+    uint32_t k[OCT];
+#pragma unroll
+    for (int j = 0; j < OCT; j++) k[j] = (in >> j) & 1u ? slot[v[j] >> group_bits] : NO_SLOT;
+#pragma unroll
+    for (int j = 0; j < OCT; j++)
+      if (k[j] != NO_SLOT) atomicAdd(acc + ((size_t)k[j] << group_bits) + (v[j] & ((1 << group_bits) - 1)), (double)__int_as_float(x[j]) * (double)t.mult);
   }
-  return e0;
+}
+
+// LADIES: the draw's candidate in its group, by a warp: the first whose running sum reaches the target, or by rounding the
+// last there is.  Blocks of 128 candidates, a lane holding four.
+__device__ __forceinline__ void pick_in_group(const double *acc, const uint32_t *there, int n, double before, double target, int &pick, double &wt) {
+  const int lane = threadIdx.x & 31;
+  double at_block = before, run = before;
+  int first = 0;
+  uint32_t its = 0;
+  bool found = false;
+  for (int q = 0; q < n && !found; q += 128) {
+    const int r = q + lane * 4;
+    const uint32_t bits = (there[r >> 5] >> (r & 31)) & 15u;
+    const double *x = acc + r;
+    const double mine = (x[0] + x[1]) + (x[2] + x[3]);
+    double upto = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+      const double t = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += t;
+    }
+    const uint32_t reach = __ballot_sync(0xffffffffu, bits && at_block + upto >= target), any = __ballot_sync(0xffffffffu, bits != 0u);
+    if (any) {
+      found = reach != 0u;
+      const int l = found ? __ffs(reach) - 1 : 31 - __clz(any);
+      first = q + l * 4;
+      its = __shfl_sync(0xffffffffu, bits, l);
+      run = at_block + __shfl_sync(0xffffffffu, upto - mine, l);
+    }
+    at_block += __shfl_sync(0xffffffffu, upto, 31);
+  }
+  bool hit = false;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const double t = acc[first + k];
+    run += t;
+    if (!hit && ((its >> k) & 1u)) {
+      pick = first + k;
+      wt = t;
+      hit = run >= target;
+    }
+  }
 }
 
 // bits 0..3 -> 0xff in bytes 0..3
@@ -196,7 +332,8 @@ __device__ __forceinline__ uint32_t sum_squares(uint32_t bits, const uint4 &d) {
   return ll + (lh << 9) + (hh << 16);
 }
 
-template <bool LADIES>
+// SUMS_FAR: LADIES' group sums are in the big part.
+template <bool LADIES, bool SUMS_FAR>
 __global__ void __launch_bounds__(1024, 1)
 coll_bitmap_kernel(const __grid_constant__ Args a) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -206,9 +343,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
   CollParams cp = a.cp;
   unsigned char *big = lay.glob_bytes ? a.gscratch + (size_t)blockIdx.x * lay.glob_bytes : smem;
   uint32_t *bm = reinterpret_cast<uint32_t *>(big);
-  double *gcdf = reinterpret_cast<double *>(big + lay.off_gcdf);
-  uint32_t *gpref = reinterpret_cast<uint32_t *>(big + lay.off_gpref);
-  uint16_t *qpre = reinterpret_cast<uint16_t *>(big + lay.off_qpre);
+  double *gcdf = reinterpret_cast<double *>((LADIES && !SUMS_FAR ? smem : big) + lay.off_gcdf);
   double *red = reinterpret_cast<double *>(smem + lay.off_red);   // 32 doubles, 32 words
   uint32_t *red_u = reinterpret_cast<uint32_t *>(red + 32);
   int32_t *sh_tr = reinterpret_cast<int32_t *>(smem + lay.off_tr);
@@ -216,10 +351,13 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
   Transit *ut = reinterpret_cast<Transit *>(smem + lay.off_ut);
   int32_t *sh_mult = reinterpret_cast<int32_t *>(smem + lay.off_mult);   // how often a transit occurs; 0: an earlier one is the same
   uint32_t *pre = reinterpret_cast<uint32_t *>(smem + lay.off_pre);
-  double *tile = reinterpret_cast<double *>(smem + lay.off_tile);
+  double *acc = reinterpret_cast<double *>(smem + lay.off_acc);          // LADIES from here on
+  uint32_t *there = reinterpret_cast<uint32_t *>(smem + lay.off_there);
+  double *sh_target = reinterpret_cast<double *>(smem + lay.off_draw);   // of a draw: the point of the CDF, its group, the first draw of the group
+  int32_t *sh_group = reinterpret_cast<int32_t *>(sh_target + cp.L), *sh_first = sh_group + cp.L;
+  uint32_t *sh_firsts = reinterpret_cast<uint32_t *>(sh_first + cp.L);   // draws that are the first of their group, as bits
+  uint8_t *slot = (LADIES && !SUMS_FAR ? smem : big) + lay.off_slot;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
-  float *wts = LADIES ? a.wts_all + (size_t)blockIdx.x * (size_t)cp.V : nullptr;
-  int32_t *pos_tab = LADIES ? a.pos_all + (size_t)blockIdx.x * (size_t)a.pos_stride : nullptr;
   unsigned long long ids_sum = 0, uniq_sum = 0, draws = 0;   // thread 0
   for (int64_t s = blockIdx.x; s < a.S;) {
     for (int step = 0; step < a.steps; step++) {
@@ -248,7 +386,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
         const int32_t rs = __ldg(a.g.row_ptr + t), deg = __ldg(a.g.row_ptr + t + 1) - rs, slot = __ldg(a.hub_slot + t);
         ids += (unsigned long long)deg;
         if (sh_mult[i] > 0) {
-          // (LADIES goes through the lists again, so that a hub's bitmap saves it less)
+          // (LADIES goes through the lists for their terms, so that a hub's bitmap saves it less)
           ut[slot >= 0 && (!LADIES || deg >= cp.V / LADIES_HUB) ? atomicAdd(&sh_hubs, 1) : cp.ntr - 1 - atomicAdd(&sh_rest, 1)] = Transit{rs, deg, sh_mult[i], slot};
         }
       }
@@ -267,20 +405,18 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
         }
         reinterpret_cast<uint4 *>(bm)[w4] = u;
       }
-      __syncthreads();
-      const Transit *rest = ut + cp.ntr - (nu - nh);
-      for (int i = warp; i < nu - nh; i += warps)   // short lists: a warp each
-        if (rest[i].deg < BIG_LIST) stream_list(a.g, bm, rest[i].rs, rest[i].deg, lane, 32);
-      for (int i = 0; i < nu - nh; i++)             // long lists: the whole CTA
-        if (rest[i].deg >= BIG_LIST) stream_list(a.g, bm, rest[i].rs, rest[i].deg, tid, blockDim.x);
-      __syncthreads();
-      uint32_t U;
-      int groups;
+      const int groups = lay.groups;
+      uint32_t seen = 0, octs = 0;
       if (!LADIES) {
+        __syncthreads();
+        const Transit *rest = ut + cp.ntr - (nu - nh);
+        for (int i = warp; i < nu - nh; i += warps)   // short lists: a warp each
+          if (rest[i].deg < BIG_LIST) stream_list(a.g, bm, rest[i].rs, rest[i].deg, lane, 32);
+        for (int i = 0; i < nu - nh; i++)             // long lists: the whole CTA
+          if (rest[i].deg >= BIG_LIST) stream_list(a.g, bm, rest[i].rs, rest[i].deg, tid, blockDim.x);
+        __syncthreads();
         // ---- the groups' weights, and the number of candidates
         const uint8_t *bytes = reinterpret_cast<const uint8_t *>(bm);
-        uint32_t seen = 0;
-        groups = lay.groups;
         for (int g0 = warp * FLIGHT; g0 < groups; g0 += warps * FLIGHT) {
           uint32_t bits[2 * FLIGHT];
           uint4 d[2 * FLIGHT];
@@ -297,11 +433,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
             if (lane == 0 && g0 + k < groups) gcdf[g0 + k] = (double)sum;
           }
         }
-        seen = __reduce_add_sync(0xffffffffu, seen);
-        if (lane == 0) red_u[warp] = seen;
         __syncthreads();
-        U = 0;
-        for (int w = 0; w < warps; w++) U += red_u[w];
         for (int i0 = warp * 32; i0 < a.n_big; i0 += warps * 32) {   // the big ones; neighbours on the list mostly share a group
           const NdBigVertex v = i0 + lane < a.n_big ? a.big[i0 + lane] : NdBigVertex{-1, 0.f};
           const bool in = v.v >= 0 && ((bm[v.v >> 5] >> (v.v & 31)) & 1u);
@@ -316,103 +448,104 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
           }
         }
       } else {
-        // ---- candidates per group (and per quad of words inside it): half a warp takes the 16 words of a group
-        for (int w0 = warp * 32; w0 < lay.words; w0 += warps * 32) {
-          const int w = w0 + lane;
-          const uint32_t bits = w < lay.words ? bm[w] : 0u;
-          const uint32_t c = __popc(bits);
-          uint32_t inc = c;
-          for (int o = 1; o < GROUP_WORDS; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o, GROUP_WORDS);
-            if ((lane & (GROUP_WORDS - 1)) >= o) inc += t;
-          }
-          if (w < lay.words) {
-            if ((lane & (GROUP_WORDS - 1)) == GROUP_WORDS - 1) gpref[w / GROUP_WORDS] = inc;
-            if ((lane & 3) == 0) qpre[w >> 2] = (uint16_t)(inc - c);
-          }
+        // ---- the groups' weights and the rest of the union, then the number of candidates
+        for (int k = tid; k < groups; k += blockDim.x) gcdf[k] = 0.0;
+        for (int i = tid; i < nu; i += blockDim.x) {
+          const Transit &t = ut[i < nh ? i : cp.ntr - nu + i];
+          pre[i] = octs_of(t.rs, t.deg);
         }
         __syncthreads();
-        U = scan_u32(gpref, lay.groups, red_u);
-        groups = (int)((U + GROUP - 1) / GROUP);   // of candidates
-        // ---- the terms of every list entry, added up per candidate in tiles of consecutive candidates
-        auto transit = [&](int i) -> const Transit & { return ut[i < nh ? i : cp.ntr - nu + i]; };
-        int32_t *sh_pos = sh_mult;   // not needed any more
-        const int tiles = (int)((U + lay.tile - 1) / lay.tile);
-        for (int q = tid; a.sorted && q < (tiles + 1) * nu; q += blockDim.x) {   // where every tile begins in every list
-          const int k = q / nu, i = q - k * nu;
-          const Transit t = transit(i);
-          int32_t e = t.rs;
-          if (k == tiles) e = t.rs + t.deg;
-          else if (k > 0) e = lower_bound(a.g.col, t.rs, t.rs + t.deg, vertex_of_rank(bm, gpref, lay.groups, (uint32_t)k * lay.tile));
-          pos_tab[q] = e;
-        }
-        for (int k = 0; k < tiles; k++) {
-          const uint32_t r0 = (uint32_t)k * lay.tile, n = min(lay.tile, U - r0);
-          const int32_t *pos = pos_tab + k * nu;
-          __syncthreads();
-          for (uint32_t r = tid; r < n; r += blockDim.x) tile[r] = 0.0;
-          for (int i = tid; i < nu; i += blockDim.x) {
-            // (lists in another order are gone through whole for every tile)
-            const int32_t at = a.sorted ? __ldcg(pos + i) : transit(i).rs;
-            sh_pos[i] = at;
-            pre[i] = a.sorted ? (uint32_t)(__ldcg(pos + nu + i) - at) : (uint32_t)transit(i).deg;
-          }
-          __syncthreads();
-          const uint32_t total = scan_u32(pre, nu, red_u);
-          for (uint32_t c0 = (uint32_t)warp * CHUNK; c0 < total; c0 += (uint32_t)warps * CHUNK) {
-            int lo = 0, hi = nu - 1;   // transit of the chunk's first entry: the last with pre <= c0
-            while (lo < hi) {
-              const int mid = (lo + hi + 1) >> 1;
-              if (pre[mid] <= c0) lo = mid; else hi = mid - 1;
-            }
-            int32_t v[CHUNK_LOADS];
-            float x[CHUNK_LOADS];
-            int m[CHUNK_LOADS];
-#pragma unroll
-            for (int j = 0; j < CHUNK_LOADS; j++) {
-              const uint32_t f = c0 + (uint32_t)(j * 32 + lane);
-              v[j] = -1; x[j] = 0.f; m[j] = 0;
-              if (f < total) {
-                while (lo + 1 < nu && pre[lo + 1] <= f) lo++;
-                const int32_t e = sh_pos[lo] + (int32_t)(f - pre[lo]);
-                v[j] = __ldg(a.g.col + e);
-                x[j] = __ldg(a.term + e);
-                m[j] = transit(lo).mult;
-              }
-            }
-#pragma unroll
-            for (int j = 0; j < CHUNK_LOADS; j++)
-              if (v[j] >= 0) {
-                const uint32_t word = (uint32_t)v[j] >> 5, quad = word >> 2, in_quad = word & 3u;
-                const uint4 q = *reinterpret_cast<const uint4 *>(bm + 4 * quad);
-                uint32_t r = gpref[word / GROUP_WORDS] + qpre[quad];
-                r += in_quad > 0 ? __popc(q.x) : 0;
-                r += in_quad > 1 ? __popc(q.y) : 0;
-                r += in_quad > 2 ? __popc(q.z) : 0;
-                const uint32_t own = in_quad == 0 ? q.x : in_quad == 1 ? q.y : in_quad == 2 ? q.z : q.w;
-                r += __popc(own & ((1u << (v[j] & 31)) - 1u));
-                if (r - r0 < n) atomicAdd(tile + (r - r0), (double)x[j] * (double)m[j]);
-              }
-          }
-          __syncthreads();
-          for (uint32_t g0 = (uint32_t)warp * GROUP; g0 < n; g0 += (uint32_t)warps * GROUP) {   // weights out, and the groups' sums
-            double sum = 0.0;
-            for (uint32_t r = g0 + lane; r < g0 + GROUP && r < n; r += 32) {
-              const float x = (float)tile[r];
-              wts[r0 + r] = x;
-              sum += (double)x;
-            }
-            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            if (lane == 0) gcdf[(r0 + g0) / GROUP] = sum;
-          }
+        octs = scan_u32(pre, nu, red_u);
+        add_terms(a.g, a.term, ut, cp.ntr, nh, nu, pre, octs, bm, gcdf, lay.group_bits);
+        __syncthreads();
+        for (int w4 = tid; w4 < lay.words / 4; w4 += blockDim.x) {
+          const uint4 u = reinterpret_cast<const uint4 *>(bm)[w4];
+          seen += __popc(u.x) + __popc(u.y) + __popc(u.z) + __popc(u.w);
         }
       }
+      seen = __reduce_add_sync(0xffffffffu, seen);
+      if (lane == 0) red_u[warp] = seen;
       __syncthreads();
+      uint32_t U = 0;
+      for (int w = 0; w < warps; w++) U += red_u[w];
       if (tid == 0) uniq_sum += U;
       scan_f64(gcdf, groups, red);
       const double total = groups > 0 ? gcdf[groups - 1] : 0.0;
-      // ---- the layer's draws, a warp each
-      for (int j = warp; j < cp.L; j += warps) {
+      // ---- the layer's draws
+      if (LADIES) {
+        const bool any = U > 0 && total > 0.0;
+        const int n = 1 << lay.group_bits;
+        for (int j = tid; j < cp.L; j += blockDim.x) {
+          if (!any) {
+            sh_layer[j] = cp.V;
+            a.out[s * cp.fs + (int64_t)cp.step * cp.L + j] = cp.V;
+            a.prob[s * cp.fs + (int64_t)cp.step * cp.L + j] = 0.f;
+            continue;
+          }
+          Rng rng(cp.seed, (uint32_t)(cp.first_sample + s), (uint32_t)cp.step, (uint32_t)j);
+          const double target = (double)rng.uniform() * total;
+          int lo = 0, hi = groups - 1;  // first group whose prefix reaches the target (rounding: the last one takes what is above all)
+          while (lo < hi) {
+            const int mid = lo + (hi - lo) / 2;
+            if (gcdf[mid] >= target) hi = mid; else lo = mid + 1;
+          }
+          sh_target[j] = target;
+          sh_group[j] = lo;
+        }
+        if (any) {
+          // the groups drawn from, each once, in the order of their first draws
+          __syncthreads();
+          for (int j0 = tid - lane; j0 < cp.L; j0 += blockDim.x) {
+            const int j = j0 + lane, group = j < cp.L ? sh_group[j] : -1;
+            int first = j;
+#pragma unroll 8
+            for (int k = 0; k < j0 + 32 && k < cp.L; k++) first = sh_group[k] == group && k < first ? k : first;
+            if (j < cp.L) sh_first[j] = first;
+            const uint32_t firsts = __ballot_sync(0xffffffffu, j < cp.L && first == j);
+            if (lane == 0) sh_firsts[j0 / 32] = firsts;
+          }
+          __syncthreads();
+          auto slot_of = [&](int j) {
+            const int first = sh_first[j];
+            int before = __popc(sh_firsts[first / 32] & ((1u << (first & 31)) - 1u));
+            for (int k = 0; k < first / 32; k++) before += __popc(sh_firsts[k]);
+            return before;
+          };
+          int drawn = 0;
+          for (int k = 0; k < (cp.L + 31) / 32; k++) drawn += __popc(sh_firsts[k]);
+          for (int q = tid; q < cp.L * (n / 32); q += blockDim.x) {   // the accumulators may lie where the union is
+            const int j = q / (n / 32), w = q % (n / 32);
+            if (sh_first[j] == j) there[slot_of(j) * (n / 32) + w] = bm[(size_t)sh_group[j] * (n / 32) + w];
+          }
+          for (int s0 = 0; s0 < drawn; s0 += lay.slots) {
+            const int here = min(drawn - s0, lay.slots);
+            __syncthreads();
+            for (int k = tid; k < here * n; k += blockDim.x) acc[k] = 0.0;
+            for (int k = tid; k < groups; k += blockDim.x) slot[k] = (uint8_t)NO_SLOT;
+            __syncthreads();
+            for (int j = tid; j < cp.L; j += blockDim.x) {
+              const int k = sh_first[j] == j ? slot_of(j) - s0 : -1;
+              if (k >= 0 && k < here) slot[sh_group[j]] = (uint8_t)k;
+            }
+            __syncthreads();
+            add_candidates(a.g, a.term, ut, cp.ntr, nh, nu, pre, octs, slot, acc, lay.group_bits);
+            __syncthreads();
+            for (int j = warp; j < cp.L; j += warps) {
+              const int k = slot_of(j) - s0, group = sh_group[j];
+              if (k < 0 || k >= here) continue;
+              int pick = 0;
+              double wt = 0.0;
+              pick_in_group(acc + (size_t)k * n, there + (s0 + k) * (n / 32), n, group > 0 ? gcdf[group - 1] : 0.0, sh_target[j], pick, wt);
+              if (lane == 0) {
+                sh_layer[j] = group * n + pick;
+                a.out[s * cp.fs + (int64_t)cp.step * cp.L + j] = group * n + pick;
+                a.prob[s * cp.fs + (int64_t)cp.step * cp.L + j] = (float)(wt / total);
+              }
+            }
+          }
+        }
+      }
+      for (int j = LADIES ? cp.L : warp; j < cp.L; j += warps) {   // FastGCN: a warp each
         int32_t pick = cp.V;
         float pr = 0.f;
         if (U > 0 && total > 0.0) {
@@ -424,22 +557,16 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
             if (gcdf[mid] >= target) hi = mid; else lo = mid + 1;
           }
           // (a target of zero takes the first candidate of all, whatever its weight)
-          if (!LADIES && target <= 0.0) while (!__any_sync(0xffffffffu, bm[lo * GROUP_WORDS + (lane & (GROUP_WORDS - 1))])) lo++;
+          if (target <= 0.0) while (!__any_sync(0xffffffffu, bm[lo * GROUP_WORDS + (lane & (GROUP_WORDS - 1))])) lo++;
           const double before = lo > 0 ? gcdf[lo - 1] : 0.0;
-          // the group in four blocks of 128 candidates (FastGCN: vertices), a lane holding four of each: the first (block,
+          // the group in four blocks of 128 vertices, a lane holding four of each: the first (block,
           // lane) that reaches the target, then the first of its candidates that does
           float x[4][4];
           uint32_t there = 0;   // which of the lane's sixteen are candidates
 #pragma unroll
           for (int q = 0; q < 4; q++) {
             const uint32_t r = (uint32_t)(lo * GROUP + q * 128 + lane * 4);
-            if (LADIES) {
-#pragma unroll
-              for (int k = 0; k < 4; k++) {
-                x[q][k] = r + k < U ? __ldcg(wts + r + k) : 0.f;
-                there |= r + k < U ? 1u << (4 * q + k) : 0u;
-              }
-            } else {
+            {
               const uint32_t bits = (bm[r >> 5] >> (r & 31)) & 15u;
               const uint32_t *codes = reinterpret_cast<const uint32_t *>(a.deg + (r >> 3)) + ((r >> 2) & 1u);
               const uint32_t low = bits ? __ldg(codes) : 0u, high = bits ? __ldg(codes + 2) : 0u;
@@ -494,7 +621,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
               hit = run >= target;
             }
           }
-          pick = LADIES ? vertex_of_rank(bm, gpref, lay.groups, rank) : (int32_t)rank;
+          pick = (int32_t)rank;
           pr = (float)((double)wt / total);
         }
         if (lane == 0) {
@@ -564,13 +691,6 @@ rowsum_build_kernel(const int32_t *__restrict__ row_ptr, const float *__restrict
         atomicAdd(sum + v, x);
       }
     }
-  });
-}
-
-__global__ void __launch_bounds__(BUILD_THREADS)
-unsorted_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col, int32_t V, int64_t E, int *__restrict__ unsorted) {
-  for_entries(row_ptr, V, E, [&](int64_t e, int32_t v) {
-    if (e + 1 < (int64_t)row_ptr[v + 1] && col[e] > col[e + 1]) *unsorted = 1;
   });
 }
 
@@ -690,21 +810,12 @@ int ensure_degrees(const nd_graph *g, int grid) {
   return ND_OK;
 }
 
-// LADIES: the terms of the entries, and whether the rows ascend
+// LADIES: the terms of the entries
 int ensure_terms(const nd_graph *g, int grid) {
   if (g->term) return ND_OK;
-  if (g->rows_sorted < 0) {
-    NdDevMem<int> flag;
-    int unsorted = 0;
-    ND_TRY(flag.alloc(1));
-    ND_CUDA(cudaMemset(flag.p, 0, sizeof(int)));
-    unsorted_kernel<<<grid, BUILD_THREADS>>>(g->row_ptr, g->col, g->V, g->E, flag.p);
-    ND_CUDA(cudaMemcpy(&unsorted, flag.p, sizeof(int), cudaMemcpyDeviceToHost));
-    g->rows_sorted = unsorted ? 0 : 1;
-  }
   NdDevMem<float> term;
   NdDevMem<double> sum;
-  ND_TRY(term.alloc((size_t)(g->E > 0 ? g->E : 1)));
+  ND_TRY(term.alloc((size_t)g->E + OCT));
   ND_TRY(sum.alloc((size_t)g->V));
   ND_CUDA(cudaMemset(sum.p, 0, sizeof(double) * (size_t)g->V));
   rowsum_build_kernel<<<grid, BUILD_THREADS>>>(g->row_ptr, g->w, g->V, g->E, sum.p);
@@ -740,45 +851,59 @@ Plan plan_of(const nd_sampler *s) {
   const int32_t V = s->g->V;
   const int L = s->p.fanout[0], B = s->p.batch, ntr = B > L ? B : L;
   const bool ladies = s->p.app == ND_APP_LADIES_IS;
+  const uint32_t optin = (uint32_t)(s->dev.smem_optin - ND_SMEM_STATIC), half = optin / 2u - 1024u;
   Layout l;
   l.words = words_of(V);
-  l.groups = l.words / GROUP_WORDS;
-  uint32_t big = 4u * (uint32_t)l.words;       // a multiple of 64
-  l.off_gcdf = big; big += 8u * (uint32_t)l.groups;
-  l.off_gpref = big; big += ladies ? 4u * (uint32_t)(l.groups + 1) : 0u;
-  l.off_qpre = big; big += ladies ? 2u * (uint32_t)(l.words / 4) : 0u;
-  big = (big + 255u) & ~255u;
-  auto place = [&](uint32_t off) {
+  l.sums_far = false;
+  // The layout with `group_bits`, the big part in shared memory or not; its bytes without accumulators of their own.
+  auto place = [&](int group_bits, bool global) {
+    l.group_bits = group_bits;
+    l.groups = ladies ? (int)(((int64_t)l.words * 32 + (1 << group_bits) - 1) >> group_bits) : l.words / GROUP_WORDS;
+    const uint32_t sums = 8u * (uint32_t)l.groups, slots = ladies ? ((uint32_t)l.groups + 15u) & ~15u : 0u;
+    uint32_t big = 4u * (uint32_t)l.words;       // a multiple of 64
+    if (!ladies || l.sums_far) { l.off_gcdf = big; l.off_slot = big + sums; big += sums + slots; }
+    big = (big + 255u) & ~255u;
+    l.glob_bytes = global ? big : 0u;
+    uint32_t off = global ? 0u : big;
+    if (ladies && !l.sums_far) { l.off_gcdf = off; l.off_slot = off + sums; off += sums + slots; }
+    l.off_draw = off; off += ladies ? (16u * (uint32_t)L + 4u * (((uint32_t)L + 31u) / 32u) + 7u) & ~7u : 0u;
     l.off_red = off; off += 8u * 32u + 4u * 32u;
     l.off_ut = off; off += (uint32_t)sizeof(Transit) * (uint32_t)ntr;
     l.off_tr = off; off += 4u * (uint32_t)ntr;
     l.off_layer = off; off += 4u * (uint32_t)L;
     l.off_mult = off; off += 4u * (uint32_t)ntr;
     l.off_pre = off; off += ladies ? 4u * (uint32_t)ntr : 0u;
+    l.off_there = off; off += ladies ? (uint32_t)L << (group_bits - 3) : 0u;
     return (off + 15u) & ~15u;
   };
-  const uint32_t tile_least = ladies ? 8u * 4096u : 0u, tile_most = ladies ? 8u * 16384u : 0u;   // whole groups
-  const uint32_t optin = (uint32_t)(s->dev.smem_optin - ND_SMEM_STATIC), half = optin / 2u - 1024u;
-  const uint32_t need = place(big) + tile_least;
+  // Accumulators of a group that is drawn from: in the bitmap's place where that holds SLOTS of them or one for every
+  // draw, else in what is left of `room`.
+  constexpr uint32_t SLOTS = 16;
+  auto fits = [&](int bits, bool global, uint32_t room) {
+    const uint32_t used = place(bits, global), slot = 8u << bits, wanted = std::min<uint32_t>((uint32_t)L, NO_SLOT);
+    l.bytes = used;
+    if (!ladies) return used <= room;
+    const uint32_t over = global ? 0u : 4u * (uint32_t)l.words / slot, beside = used < room ? (room - used) / slot : 0u;
+    l.off_acc = over >= std::min(wanted, std::max(SLOTS, beside)) ? 0u : used;
+    l.slots = (int)std::min(wanted, l.off_acc ? beside : over);
+    if (l.off_acc) l.bytes += slot * (uint32_t)l.slots;
+    return used <= room && (uint32_t)l.slots >= std::min(wanted, SLOTS);
+  };
+  bool two = false, placed = false;
+  const int most = ladies ? LADIES_GROUP_BITS + 2 : LADIES_GROUP_BITS;
+  for (int bits = LADIES_GROUP_BITS; bits <= most && !placed && !s->coll_global; bits++) placed = two = fits(bits, false, half);
+  for (int bits = LADIES_GROUP_BITS; bits <= most && !placed && !s->coll_global; bits++) placed = fits(bits, false, optin);
+  for (int bits = LADIES_GROUP_BITS; !placed && bits <= LADIES_GROUP_BITS + 5; bits++) placed = fits(bits, true, optin);
+  if (!placed) {   // (LADIES from about 12 M vertices on, or thousands of transits)
+    l.sums_far = true;
+    fits(LADIES_GROUP_BITS, true, optin);
+    if (ladies && l.slots < 1) { l.slots = 1; l.bytes += 8u << LADIES_GROUP_BITS; }
+  }
   Plan p;
-  const bool global = s->coll_global || need > optin;
-  const uint32_t base = place(global ? 0u : big);
-  const bool two = !global && need <= half;
-  const uint32_t room = (two ? half : optin) - base;
-  l.off_tile = base;
-  l.tile = std::min(room, tile_most) / (8u * GROUP) * GROUP;
-  l.bytes = base + 8u * l.tile;
-  l.glob_bytes = global ? big : 0u;
-  p.lay = l;
   p.threads = two ? 512 : 1024;
   p.per_sm = two ? 2 : 1;
+  p.lay = l;
   return p;
-}
-
-// LADIES: where the tiles begin in the transits' lists
-int pos_entries(const nd_sampler *s, const Layout &lay) {
-  const int L = s->p.fanout[0], B = s->p.batch;
-  return (int)((s->g->V + lay.tile - 1) / lay.tile + 1) * (B > L ? B : L);
 }
 
 }  // namespace
@@ -795,11 +920,10 @@ int nd_coll_bitmap_alloc(nd_sampler *s) {
   s->coll_global = force_global();
   const Plan p = plan_of(s);
   ND_TRY(ensure_layers(s->g, s->dev.sms, ladies));
-  ND_CUDA(ladies ? nd_smem_most(coll_bitmap_kernel<true>, s->dev) : nd_smem_most(coll_bitmap_kernel<false>, s->dev));
+  ND_CUDA(ladies ? (p.lay.sums_far ? nd_smem_most(coll_bitmap_kernel<true, true>, s->dev) : nd_smem_most(coll_bitmap_kernel<true, false>, s->dev))
+                 : nd_smem_most(coll_bitmap_kernel<false, false>, s->dev));
   s->coll_grid = (int)std::min<int64_t>(s->S > 0 ? s->S : 1, (int64_t)s->dev.sms * p.per_sm);
   if (p.lay.glob_bytes) ND_CUDA(nd_malloc(&s->d_bm, (size_t)p.lay.glob_bytes * (size_t)s->coll_grid));
-  if (ladies) ND_CUDA(nd_malloc(&s->d_cand_w, sizeof(float) * (size_t)s->coll_grid * (size_t)s->g->V));
-  if (ladies) ND_CUDA(nd_malloc(&s->d_runs, sizeof(int32_t) * (size_t)s->coll_grid * (size_t)pos_entries(s, p.lay)));
   ND_CUDA(nd_malloc(&s->d_rows_acc, 16 * sizeof(unsigned long long)));
   ND_CUDA(cudaMemset(s->d_rows_acc, 0, 16 * sizeof(unsigned long long)));
   return ND_OK;
@@ -809,11 +933,11 @@ int nd_coll_bitmap_launch(nd_sampler *s, const CollParams &cp, unsigned long lon
   const bool ladies = s->p.app == ND_APP_LADIES_IS;
   const Plan p = plan_of(s);
   const nd_graph *g = s->g;
-  const Args a{nd_view(g), cp, s->p.steps, s->S, p.lay, s->d_bm, s->d_initial, s->d_out, s->d_cand_w,
-               s->d_runs, ladies ? pos_entries(s, p.lay) : 0, g->rows_sorted, s->d_adj_row, s->d_adj_col, s->d_prob,
+  const Args a{nd_view(g), cp, s->p.steps, s->S, p.lay, s->d_bm, s->d_initial, s->d_out, s->d_adj_row, s->d_adj_col, s->d_prob,
                g->deg_codes, g->big, g->n_big, g->term, g->hub_slot, g->hub_bits, s->d_rows_acc, s->d_stats, pairs};
-  if (ladies) coll_bitmap_kernel<true><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
-  else coll_bitmap_kernel<false><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
+  if (ladies && p.lay.sums_far) coll_bitmap_kernel<true, true><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
+  else if (ladies) coll_bitmap_kernel<true, false><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
+  else coll_bitmap_kernel<false, false><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
   nd_count_launches(1);
   ND_CUDA(cudaGetLastError());
   return ND_OK;

@@ -28,23 +28,55 @@ __device__ __forceinline__ bool has_edge_logn(const NdGraphView &g, int32_t src,
 }
 
 // adjacency entries of one layer of one sample: (row,col) = (i,j) where transit i -- vertex j is an edge.  A transit
-// with a bitmap of its neighbours (hub_slot, null: none have one) is asked by a bit test.
+// with a bitmap of its neighbours (hub_slot, null: none have one) is asked by a bit test, the others' lists are bisected, a
+// few entries at a time side by side: every step of a search waits for the one before.
 __device__ __forceinline__ void emit_adjacency(const NdGraphView &g, const CollParams &cp, const int32_t *tr,
                                                const int32_t *layer, int32_t *arow, int32_t *acol, const int32_t *hub_slot = nullptr,
                                                const uint32_t *hub_bits = nullptr, int words = 0) {
-  for (int e = threadIdx.x; e < cp.stride; e += blockDim.x) {
-    const int i = e / cp.L, j = e - i * cp.L;
-    int32_t ri = -1, cj = -1;
-    if (i < cp.ntr) {
-      const int32_t t = tr[i], v = layer[j];
-      if (t >= 0 && t < cp.V && v >= 0 && v < cp.V) {
-        const int32_t slot = hub_slot ? __ldg(hub_slot + t) : -1;
-        const bool edge = slot >= 0 ? (__ldg(hub_bits + (size_t)slot * words + ((uint32_t)v >> 5)) >> (v & 31)) & 1u : has_edge_logn(g, t, v);
-        if (edge) { ri = i; cj = j; }
+  constexpr int SIDE = 4;
+  for (int e0 = threadIdx.x; e0 < cp.stride; e0 += SIDE * blockDim.x) {
+    int32_t v[SIDE], l[SIDE], r[SIDE];   // searched for in [l, r)
+    bool edge[SIDE];
+#pragma unroll
+    for (int k = 0; k < SIDE; k++) {
+      const int e = e0 + k * (int)blockDim.x, i = e / cp.L, j = e - i * cp.L;
+      l[k] = r[k] = 0; v[k] = -1; edge[k] = false;
+      if (e >= cp.stride || i >= cp.ntr) continue;
+      const int32_t t = tr[i];
+      v[k] = layer[j];
+      if (t < 0 || t >= cp.V || v[k] < 0 || v[k] >= cp.V) continue;
+      const int32_t slot = hub_slot ? __ldg(hub_slot + t) : -1;
+      if (slot >= 0) {
+        edge[k] = (__ldg(hub_bits + (size_t)slot * words + ((uint32_t)v[k] >> 5)) >> (v[k] & 31)) & 1u;
+      } else {
+        l[k] = __ldg(g.row_ptr + t);
+        r[k] = __ldg(g.row_ptr + t + 1);
       }
     }
-    arow[e] = ri;
-    acol[e] = cj;
+    for (bool more = true; more;) {
+      more = false;
+      int32_t m[SIDE], c[SIDE];
+#pragma unroll
+      for (int k = 0; k < SIDE; k++) {
+        m[k] = l[k] + (r[k] - l[k]) / 2;
+        c[k] = l[k] < r[k] ? __ldg(g.col + m[k]) : 0;
+      }
+#pragma unroll
+      for (int k = 0; k < SIDE; k++) {
+        if (l[k] >= r[k]) continue;
+        if (c[k] == v[k]) { edge[k] = true; l[k] = r[k]; }
+        else if (c[k] < v[k]) l[k] = m[k] + 1;
+        else r[k] = m[k];
+        more |= l[k] < r[k];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < SIDE; k++) {
+      const int e = e0 + k * (int)blockDim.x, i = e / cp.L;
+      if (e >= cp.stride) continue;
+      arow[e] = edge[k] ? i : -1;
+      acol[e] = edge[k] ? e - i * cp.L : -1;
+    }
   }
 }
 

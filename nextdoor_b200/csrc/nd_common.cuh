@@ -113,7 +113,6 @@ struct nd_graph {
   float *max_w = nullptr;
   void *block = nullptr;        // the one allocation the four arrays lie in, or null: an allocation each
   size_t block_bytes = 0;
-  mutable int rows_sorted = -1; // the rows' ids ascend (the library's own builds: 1; CSR arrays of a caller: -1, not asked yet)
   // Derived layouts, built on the first sampler that needs them and shared by all samplers of the graph:
   mutable int2 *colw = nullptr;        // [E] (neighbour id, weight bits) records: one 8-byte gather per weighted try
   mutable int2 *vrec = nullptr;        // [V+1] (row start, max weight bits) per vertex: what a thread-per-walk kernel needs of a vertex in one sector

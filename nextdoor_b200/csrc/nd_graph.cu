@@ -393,7 +393,7 @@ int build_from_soa(const NdDeviceInfo &dev, int64_t n, int32_t V, BuildScratch *
   unsigned char *block = nullptr;
   ND_TRY(nd_block_alloc(dev.device, (void **)&block, &all));
   nd_graph *g = new nd_graph();
-  g->device = dev.device; g->V = V; g->E = n; g->block = block; g->block_bytes = all; g->rows_sorted = 1;
+  g->device = dev.device; g->V = V; g->E = n; g->block = block; g->block_bytes = all;
   g->row_ptr = (int32_t *)block; g->col = (int32_t *)(block + o_col); g->w = (float *)(block + o_w); g->max_w = (float *)(block + o_max);
   auto build = [&]() -> int {
     ND_CUDA(cudaMemsetAsync(g->col + n, 0, sizeof(int32_t) * 8));

@@ -136,3 +136,57 @@ def test_rows_in_any_order(nd, monkeypatch, app, scratch, V, M, B, L):
     # the row sums are added up in another order, to 1e-16: less than one draw in 10^9 can fall to its neighbour for it
     assert np.array_equal(out[0][0], out[1][0]) and out[0][2] == out[1][2]
     assert np.allclose(out[0][1], out[1][1], rtol=1e-6, atol=0)
+
+
+def _ladies(nd, ndo, hg, S, B, L, init):
+    """Against 64-bit sums of the 32-bit terms.  2^18 terms added up in any order differ by 2^18 * 2^-53 of the total at
+    most: a draw may fall to another candidate only that near to the end of one."""
+    V, steps = hg.V, 2
+    s = nd.Sampler(nd.Graph.from_csr(hg.row_ptr, hg.col, hg.w, hg.max_w), nd.app_params(9, steps=steps, fanout=L, batch=B, seed=3), num_samples=S, initial=init)
+    s.sample()
+    got, aux = s.final_samples().reshape(S, steps, L), s.aux()
+    prob, seen = aux["prob"].reshape(S, steps, L), 0
+    for smp in range(S):
+        for step in range(steps):
+            transits = init.reshape(S, B)[smp] if step == 0 else got[smp, step - 1]
+            transits = transits[transits < V]
+            rows = [slice(hg.row_ptr[t], hg.row_ptr[t + 1]) for t in transits]
+            ids = np.concatenate([hg.col[r] for r in rows] or [np.zeros(0, np.int32)])
+            share = np.concatenate([hg.w[r] / np.float32(hg.w[r].astype(np.float64).sum()) for r in rows] or [np.zeros(0, np.float32)])
+            cand, at = np.unique(ids, return_inverse=True)
+            seen += len(cand)
+            if len(cand) == 0:
+                assert (got[smp, step] == V).all()
+                continue
+            cdf = np.cumsum(np.bincount(at, (share * share).astype(np.float64)))
+            u = np.array([ndo.lib().ndo_uniform(3, smp, step, j, 0) for j in range(L)], np.float32)
+            target = u.astype(np.float64) * cdf[-1]
+            k = np.minimum(np.searchsorted(cdf, target), len(cand) - 1)
+            mine = np.searchsorted(cand, got[smp, step])
+            assert np.array_equal(cand[mine], got[smp, step])
+            bound = 2.0 ** -35 * cdf[-1]
+            ok = (mine == k) | ((mine == k + 1) & (cdf[k] - target <= bound)) | ((mine == k - 1) & (target - cdf[k - 1] <= bound))
+            assert ok.all()
+            assert np.allclose(prob[smp, step], np.diff(cdf, prepend=0.0)[mine] / cdf[-1], rtol=1e-6, atol=2.0 ** -35)
+    assert s.stats()["union_unique"] == seen
+    assert ndo.check_adjacency(hg, ndo.make_params(9, steps=steps, fanout=L, batch=B, seed=3), S, init, s.final_samples(), aux["adj_row"], aux["adj_col"]) == 0
+
+
+@pytest.mark.parametrize("V,B,L", [(129, 3, 1), (200_000, 100, 300), (200_000, 40, 31), (1_100_000, 64, 33), (1_300_000, 64, 64)])
+def test_ladies_groups_and_accumulators(nd, ndo, V, B, L):
+    """More groups drawn from than have accumulators at a time, groups that end behind the last vertex, lists that begin and end
+    anywhere in an oct, the bitmap's place with and without room for them."""
+    hg = ndo.rmat_graph(V, max(8 * V, 600) if V < 500_000 else 3 * V, seed=2)
+    init = np.random.default_rng(V + L).integers(0, V, 20 * B).astype(np.int32)
+    _ladies(nd, ndo, hg, 20, B, L, init)
+
+
+@pytest.mark.parametrize("V", [3_000_000, 9_000_000, 20_000_000])
+def test_ladies_of_many_vertices(nd, ndo, V):
+    """Larger groups, then their sums in global scratch."""
+    rng = np.random.default_rng(V)
+    ids = rng.integers(0, V, 3000)
+    src = np.concatenate([rng.choice(ids, 60_000), [V - 1]]).astype(np.int32)
+    dst = np.concatenate([rng.choice(ids, 60_000), [ids[0]]]).astype(np.int32)
+    hg = ndo.csr_from_records(src, dst, (rng.random(len(src)) + 0.1).astype(np.float32), V=V)
+    _ladies(nd, ndo, hg, 6, 32, 64, rng.choice(ids, 6 * 32).astype(np.int32))
