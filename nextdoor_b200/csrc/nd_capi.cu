@@ -127,7 +127,7 @@ void free_sampler(nd_sampler *s) {
   for (int i = 0; i < 2; i++) { cudaFree(s->d_map_key[i]); cudaFree(s->d_map_val[i]); }
   cudaFree(s->d_init_key); cudaFree(s->d_init_val); cudaFree(s->d_nlive); cudaFree(s->d_stats); status_word_put(s->h_status);
   cudaFree(s->d_runs); cudaFree(s->d_bin_counts); cudaFree(s->d_hop_counts);
-  cudaFree(s->d_adj_row); cudaFree(s->d_adj_bits); cudaFree(s->d_adj_col); cudaFree(s->d_prob); cudaFree(s->d_cand); cudaFree(s->d_cand_w); cudaFree(s->d_bm);
+  cudaFree(s->d_adj); cudaFree(s->d_prob); cudaFree(s->d_cand); cudaFree(s->d_cand_w); cudaFree(s->d_bm);
   cudaFree(s->d_cnt); cudaFree(s->d_offs); cudaFree(s->d_bsum); cudaFree(s->d_rank);
   for (int i = 0; i < 2; i++) cudaFree(s->d_srec[i]);
   cudaFree(s->d_init_rec); cudaFree(s->d_list); cudaFree(s->d_rows_acc);
@@ -169,18 +169,6 @@ int check_params(const nd_app_params *p) {
 }  // namespace
 
 namespace {
-
-constexpr size_t ADJ_BITS_MIN = (size_t)1 << 18;   // entries (2 MB in two arrays): below this the plain copies are as fast
-
-// bit e: entry e of the adjacency is an edge; a word per warp (reads at the memory's rate)
-__global__ void __launch_bounds__(256) adj_bits_kernel(const int32_t *__restrict__ row, int64_t n, uint32_t *__restrict__ bits) {
-  const int64_t words = (n + 31) / 32;
-  for (int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; w < words; w += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-    const int64_t e = 32 * w + (threadIdx.x & 31);
-    const uint32_t b = __ballot_sync(0xffffffffu, e < n && __ldcs(row + e) >= 0);
-    if ((threadIdx.x & 31) == 0) bits[w] = b;
-  }
-}
 
 }  // namespace
 
@@ -356,23 +344,8 @@ int nd_sampler_aux(nd_sampler *s, int32_t *adj_row, int32_t *adj_col, float *pro
   ND_TRY(nd_sampler_sync(s));
   if (nd_is_collective(s->p.app)) {
     const int L = s->p.fanout[0], B = s->p.batch;
-    const size_t n = (size_t)s->S * s->p.steps * (B > L ? B : L) * L;
-    bool done = false;
-    if (adj_row && adj_col && n >= ADJ_BITS_MIN) {
-      ND_CUDA(cudaSetDevice(s->g->device));
-      if (!s->d_adj_bits && nd_malloc(&s->d_adj_bits, 4 * ((n + 31) / 32)) != cudaSuccess) cudaGetLastError();   // the plain copies need none
-    }
-    if (adj_row && adj_col && n >= ADJ_BITS_MIN && s->d_adj_bits) {
-      adj_bits_kernel<<<s->dev.sms * 8, 256, 0, s->stream>>>(s->d_adj_row, (int64_t)n, s->d_adj_bits);
-      nd_count_launches(1);
-      ND_CUDA(cudaStreamSynchronize(s->stream));
-      ND_TRY(nd_adjacency_to_host(s->g->device, s->d_adj_bits, (int64_t)n, (B > L ? B : L) * L, L, adj_row, adj_col, &done));
-    }
-    void *const dst[3] = {adj_row, adj_col, prob};
-    const void *const src[3] = {s->d_adj_row, s->d_adj_col, s->d_prob};
-    const size_t adj = done ? 0 : 4 * n;
-    const size_t bytes[3] = {adj_row ? adj : 0, adj_col ? adj : 0, prob && s->d_prob ? 4 * (size_t)s->S * s->fs : 0};
-    ND_TRY(nd_copies_to_host(s->g->device, 3, dst, src, bytes));
+    ND_TRY(nd_adjacency_to_host(s->g->device, s->d_adj, s->S * s->p.steps, (B > L ? B : L) * L, L, adj_row, adj_col));
+    if (prob && s->d_prob) ND_TRY(nd_copy_to_host(s->g->device, prob, s->d_prob, 4 * (size_t)s->S * s->fs));
   }
   if (hop_counts && s->d_hop_counts)
     ND_TRY(nd_copy_to_host(s->g->device, hop_counts, s->d_hop_counts, 4 * (size_t)s->S * s->p.steps));

@@ -77,7 +77,7 @@ struct Args {
   unsigned char *gscratch;
   const int32_t *initial;
   int32_t *out;
-  int32_t *adj_row, *adj_col;
+  uint32_t *adj;
   float *prob;
   const uint4 *__restrict__ deg;           // FastGCN: the degrees of eight vertices, low bytes (x, y), high bytes (z, w)
   const NdBigVertex *__restrict__ big;     // FastGCN: vertices with degrees from BIG_DEGREE, in order
@@ -632,8 +632,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
       }
       if (tid == 0) { if (U > 0 && total > 0.0) draws += (unsigned long long)cp.L; }
       __syncthreads();
-      const int64_t at = (s * a.steps + cp.step) * (int64_t)cp.stride;
-      emit_adjacency(a.g, cp, sh_tr, sh_layer, a.adj_row + at, a.adj_col + at, a.hub_slot, a.hub_bits, lay.words);
+      emit_adjacency(a.g, cp, sh_tr, sh_layer, a.adj + (s * a.steps + cp.step) * (int64_t)adj_words(cp.stride), a.hub_slot, a.hub_bits, lay.words);
       __syncthreads();
     }
     if (tid == 0) sh_sample = a.S > gridDim.x ? (long long)gridDim.x + (long long)atomicAdd(&a.acc[8], 1ull) : (long long)a.S;
@@ -933,7 +932,7 @@ int nd_coll_bitmap_launch(nd_sampler *s, const CollParams &cp, unsigned long lon
   const bool ladies = s->p.app == ND_APP_LADIES_IS;
   const Plan p = plan_of(s);
   const nd_graph *g = s->g;
-  const Args a{nd_view(g), cp, s->p.steps, s->S, p.lay, s->d_bm, s->d_initial, s->d_out, s->d_adj_row, s->d_adj_col, s->d_prob,
+  const Args a{nd_view(g), cp, s->p.steps, s->S, p.lay, s->d_bm, s->d_initial, s->d_out, s->d_adj, s->d_prob,
                g->deg_codes, g->big, g->n_big, g->term, g->hub_slot, g->hub_bits, s->d_rows_acc, s->d_stats, pairs};
   if (ladies && p.lay.sums_far) coll_bitmap_kernel<true, true><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
   else if (ladies) coll_bitmap_kernel<true, false><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);

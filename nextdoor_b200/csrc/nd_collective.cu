@@ -41,8 +41,8 @@ constexpr int CTHREADS = 256;
 // CTA, every entry asks a filter of the layer's ids in shared memory, and the few that pass look for the id.
 // A list longer than PROBE_RATIO times the layer is bisected for every id instead.  (One bisection per
 // (transit, slot) pair, 205 M of them for 10,000 samples of 5 x 64 x 64 on 57 K vertices: 1.04 ms, now 0.57.)
-// What is left: 1.6 GB of adjacency entries, in 16-byte stores (36 % of the DRAM's rate over the launch), and 377 M warp
-// instructions, issued in 68 % of the cycles, with barriers between drawing, probing and writing.
+// The flags of the edges that were found are the adjacency as it is kept: a bit per entry (the two arrays of the
+// reference's form, 1.6 GB for those samples, took 0.1 ms of 0.54).
 constexpr int FILTER_WORDS = 256;   // 8192 bits per layer
 constexpr int PROBE_RATIO = 8;
 
@@ -75,7 +75,7 @@ static RefLayout ref_layout(int steps, int B, int L) {
 
 __global__ void __launch_bounds__(CTHREADS)
 coll_ref_kernel(NdGraphView g, CollParams cp, RefLayout lay, int steps, int64_t S, const int32_t *__restrict__ initial, int32_t *__restrict__ out,
-                int32_t *__restrict__ adj_row, int32_t *__restrict__ adj_col, unsigned long long *__restrict__ stats) {
+                uint32_t *__restrict__ adj, unsigned long long *__restrict__ stats) {
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ uint32_t red[CTHREADS / 32];
   int32_t *ids = reinterpret_cast<int32_t *>(sm + lay.off_ids);
@@ -189,27 +189,23 @@ coll_ref_kernel(NdGraphView g, CollParams cp, RefLayout lay, int steps, int64_t 
         if (lo < rs[i] + deg_of[i] && __ldg(g.col + lo) == id) atomicOr(flags + i * lay.flag_words + (j >> 5), 1u << (j & 31));
       }
       __syncthreads();
-      // adjacency entries: (row, col) = (i, j) where transit i -- vertex j is an edge
-      for (int k = 0; k < kn; k++) {
+      // the layers' adjacency: the flags are the bits where a transit's are whole words
+      const int words = adj_words(cp.stride);
+      for (int q = tid; q < kn * words; q += CTHREADS) {
+        const int k = q / words, w = q - k * words;
         const int first = k == 0 ? 0 : n0 + (k - 1) * L, n = k == 0 ? n0 : L;
-        const int64_t a = (s * steps + k0 + k) * (int64_t)cp.stride;
-        auto set = [&](int i, int j) { return i < n && ((flags[(first + i) * lay.flag_words + (j >> 5)] >> (j & 31)) & 1u); };
-        if ((L & 3) == 0) {
-          int4 *ar = reinterpret_cast<int4 *>(adj_row + a), *ac = reinterpret_cast<int4 *>(adj_col + a);
-          for (int q = tid; q < cp.stride / 4; q += CTHREADS) {
-            const int i = 4 * q / L, j = 4 * q - i * L;
-            const uint32_t b = i < n ? (flags[(first + i) * lay.flag_words + (j >> 5)] >> (j & 31)) & 15u : 0u;
-            __stcs(ar + q, make_int4(b & 1u ? i : -1, b & 2u ? i : -1, b & 4u ? i : -1, b & 8u ? i : -1));
-            __stcs(ac + q, make_int4(b & 1u ? j : -1, b & 2u ? j + 1 : -1, b & 4u ? j + 2 : -1, b & 8u ? j + 3 : -1));
-          }
+        uint32_t bits = 0u;
+        if ((L & 31) == 0) {
+          if (w / lay.flag_words < n) bits = flags[first * lay.flag_words + w];
         } else {
-          for (int e = tid; e < cp.stride; e += CTHREADS) {
-            const int i = e / L, j = e - i * L;
-            const bool b = set(i, j);
-            adj_row[a + e] = b ? i : -1;
-            adj_col[a + e] = b ? j : -1;
+          for (int e = 32 * w; e < 32 * w + 32;) {   // up to the end of the word, of the transit's flags' word or of its row
+            const int i = e / L, j = e - i * L, len = min(min(32 * w + 32 - e, L - j), 32 - (j & 31));
+            if (i >= n) break;
+            bits |= (flags[(first + i) * lay.flag_words + (j >> 5)] >> (j & 31) & (0xffffffffu >> (32 - len))) << (e & 31);
+            e += len;
           }
         }
+        __stcs(adj + (s * steps + k0) * (int64_t)words + q, bits);
       }
     }
   }
@@ -316,8 +312,8 @@ coll_weigh_kernel(NdGraphView g, int app, int64_t n, const uint32_t *__restrict_
 __global__ void __launch_bounds__(CTHREADS)
 coll_sample_kernel(NdGraphView g, CollParams cp, int steps, int64_t s0, int64_t s1, const int32_t *__restrict__ initial,
                    int32_t *out, const int64_t *__restrict__ offs, const uint32_t *__restrict__ c_id,
-                   const float *__restrict__ wt, double *__restrict__ cdf, int32_t *__restrict__ adj_row,
-                   int32_t *__restrict__ adj_col, float *__restrict__ prob, unsigned long long *__restrict__ stats) {
+                   const float *__restrict__ wt, double *__restrict__ cdf, uint32_t *__restrict__ adj,
+                   float *__restrict__ prob, unsigned long long *__restrict__ stats) {
   __shared__ double warp_tot[CTHREADS / 32];
   __shared__ double carry_sh;
   __shared__ int32_t sh_tr[1024];
@@ -370,8 +366,7 @@ coll_sample_kernel(NdGraphView g, CollParams cp, int steps, int64_t s0, int64_t 
       prob[s * cp.fs + (int64_t)cp.step * cp.L + j] = pr;
     }
     __syncthreads();
-    const int64_t a = (s * steps + cp.step) * (int64_t)cp.stride;
-    emit_adjacency(g, cp, sh_tr, sh_layer, adj_row + a, adj_col + a);
+    emit_adjacency(g, cp, sh_tr, sh_layer, adj + (s * steps + cp.step) * (int64_t)adj_words(cp.stride));
     for (int o = 16; o > 0; o >>= 1) valid += __shfl_xor_sync(0xffffffffu, valid, o);
     if (lane == 0 && valid) atomicAdd(&stats[0], (unsigned long long)valid);
     __syncthreads();
@@ -404,9 +399,7 @@ int nd_collective_alloc(nd_sampler *s) {
   const nd_app_params &p = s->p;
   const int L = p.fanout[0], B = p.batch;
   const size_t S1 = (size_t)(s->S > 0 ? s->S : 1);
-  const size_t adj = S1 * p.steps * (size_t)(B > L ? B : L) * L;
-  ND_CUDA(nd_malloc(&s->d_adj_row, sizeof(int32_t) * adj));
-  ND_CUDA(nd_malloc(&s->d_adj_col, sizeof(int32_t) * adj));
+  ND_CUDA(nd_malloc(&s->d_adj, sizeof(uint32_t) * S1 * p.steps * (size_t)adj_words((B > L ? B : L) * L)));
   ND_CUDA(nd_malloc(&s->d_prob, sizeof(float) * S1 * s->fs));
   ND_CUDA(cudaMemset(s->d_prob, 0, sizeof(float) * S1 * s->fs));
   ND_CUDA(nd_malloc(&s->d_len, sizeof(int32_t) * (S1 + 1)));        // per-sample sizes of the layer
@@ -454,7 +447,7 @@ int nd_collective_sample(nd_sampler *s, int mode) {
     const int per_sm = lay.bytes <= 24u * 1024u ? 8 : 1;
     nd_phase_begin(s, ND_PHASE_NEXT);
     coll_ref_kernel<<<(int)std::min<int64_t>(S, (int64_t)s->dev.sms * per_sm), CTHREADS, lay.bytes, st>>>(
-        gv, cp, lay, p.steps, S, s->d_initial, s->d_out, s->d_adj_row, s->d_adj_col, s->d_stats);
+        gv, cp, lay, p.steps, S, s->d_initial, s->d_out, s->d_adj, s->d_stats);
     nd_phase_end(s);
     nd_count_launches(1);
     ND_CUDA(cudaGetLastError());
@@ -517,14 +510,14 @@ int nd_collective_sample(nd_sampler *s, int mode) {
         nd_phase_end(s);
         nd_phase_begin(s, ND_PHASE_NEXT);
         coll_sample_kernel<<<cgrid, CTHREADS, 0, st>>>(gv, cp, p.steps, s0, s1, s->d_initial, s->d_out, d_offs, cur[0], wt, cdf,
-                                                     s->d_adj_row, s->d_adj_col, s->d_prob, s->d_stats);
+                                                     s->d_adj, s->d_prob, s->d_stats);
         nd_count_launches(1);
         nd_phase_end(s);
         // the next chunk reuses the buffers and the host copy of its size
         ND_CUDA(cudaStreamSynchronize(st));
       } else {
         coll_sample_kernel<<<cgrid, CTHREADS, 0, st>>>(gv, cp, p.steps, s0, s1, s->d_initial, s->d_out, d_offs, c_a[0], wt, cdf,
-                                                     s->d_adj_row, s->d_adj_col, s->d_prob, s->d_stats);
+                                                     s->d_adj, s->d_prob, s->d_stats);
         nd_count_launches(1);
       }
       s0 = s1;

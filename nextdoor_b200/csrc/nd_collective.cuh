@@ -27,14 +27,19 @@ __device__ __forceinline__ bool has_edge_logn(const NdGraphView &g, int32_t src,
   return false;
 }
 
-// adjacency entries of one layer of one sample: (row,col) = (i,j) where transit i -- vertex j is an edge.  A transit
+// The adjacency of a layer of a sample is a bit per entry (entry i * L + j: transit i -- vertex j is an edge) in whole
+// words; nd_sampler_aux hands it out as (row, col) = (i, j) or (-1, -1).
+__host__ __device__ inline int adj_words(int stride) { return (stride + 31) / 32; }
+
+// the adjacency of one layer of one sample, by the whole CTA (whole warps).  A transit
 // with a bitmap of its neighbours (hub_slot, null: none have one) is asked by a bit test, the others' lists are bisected, a
 // few entries at a time side by side: every step of a search waits for the one before.
 __device__ __forceinline__ void emit_adjacency(const NdGraphView &g, const CollParams &cp, const int32_t *tr,
-                                               const int32_t *layer, int32_t *arow, int32_t *acol, const int32_t *hub_slot = nullptr,
+                                               const int32_t *layer, uint32_t *adj, const int32_t *hub_slot = nullptr,
                                                const uint32_t *hub_bits = nullptr, int words = 0) {
   constexpr int SIDE = 4;
-  for (int e0 = threadIdx.x; e0 < cp.stride; e0 += SIDE * blockDim.x) {
+  const int lane = threadIdx.x & 31;
+  for (int e0 = threadIdx.x; e0 - lane < cp.stride; e0 += SIDE * blockDim.x) {
     int32_t v[SIDE], l[SIDE], r[SIDE];   // searched for in [l, r)
     bool edge[SIDE];
 #pragma unroll
@@ -72,10 +77,9 @@ __device__ __forceinline__ void emit_adjacency(const NdGraphView &g, const CollP
     }
 #pragma unroll
     for (int k = 0; k < SIDE; k++) {
-      const int e = e0 + k * (int)blockDim.x, i = e / cp.L;
-      if (e >= cp.stride) continue;
-      arow[e] = edge[k] ? i : -1;
-      acol[e] = edge[k] ? e - i * cp.L : -1;
+      const int e = e0 + k * (int)blockDim.x;
+      const uint32_t word = __ballot_sync(0xffffffffu, edge[k]);
+      if (lane == 0 && e < cp.stride) adj[e / 32] = word;
     }
   }
 }

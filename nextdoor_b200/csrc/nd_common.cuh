@@ -261,9 +261,8 @@ struct nd_sampler {
   int32_t *d_bin_counts = nullptr;
   int32_t *d_hop_counts = nullptr;
   // collective
-  int32_t *d_adj_row = nullptr, *d_adj_col = nullptr;
   float *d_prob = nullptr;
-  uint32_t *d_adj_bits = nullptr;      // the adjacency on its way to the host (made at the first use)
+  uint32_t *d_adj = nullptr;           // the layers' adjacency, a bit per entry
   int32_t *d_cand = nullptr;
   float *d_cand_w = nullptr;
   int64_t cand_cap = 0;

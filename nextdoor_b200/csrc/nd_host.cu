@@ -18,7 +18,9 @@
 #include <chrono>
 #include <condition_variable>
 #include <deque>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -298,37 +300,56 @@ int copy(int device, int n, void *const *dst, const void *const *src, const size
 
 }  // namespace
 
-// Results that are mostly one value cross as a bit per entry: 1/64 of the bytes of an adjacency's two arrays, which the
-// workers write here (67 MB: 2.6 ms copied into memory that is there, 0.9 written).
-int nd_adjacency_to_host(int device, const uint32_t *bits, int64_t entries, int stride, int L, int32_t *row, int32_t *col, bool *done) {
-  *done = false;
+// Adjacencies are a bit per entry on the device and on the way, 1/64 of the bytes of the two arrays that the workers write
+// here (67 MB: 2.6 ms copied into memory that is there, 0.9 written).
+constexpr int64_t SMALL_ADJACENCY = 1 << 13;   // words (2 MB in two arrays) that the caller's thread writes by itself
+int nd_adjacency_to_host(int device, const uint32_t *bits, int64_t layers, int stride, int L, int32_t *row, int32_t *col) {
+  if (layers <= 0 || !(row || col)) return ND_OK;
   ND_CUDA(cudaSetDevice(device));
-  std::unique_lock<std::mutex> lock(g_ring.m, std::try_to_lock);
-  if (nd_host_threads() <= 2 || !lock.owns_lock() || !ring_ready(device)) return ND_OK;
-  const int64_t words = (entries + 31) / 32, most = (int64_t)(PIECE * RING / 4);
-  for (int64_t w0 = 0; w0 < words; w0 += most) {
-    const int64_t n = std::min(most, words - w0);
-    ND_CUDA(cudaMemcpyAsync(g_ring.pinned, bits + w0, 4 * (size_t)n, cudaMemcpyDeviceToHost, g_ring.stream));
-    ND_CUDA(cudaStreamSynchronize(g_ring.stream));
-    const uint32_t *in = (const uint32_t *)g_ring.pinned;
-    nd_host_ranges(n, nd_host_threads(), [=](int, int64_t a, int64_t b) {
+  const int per = (stride + 31) / 32;
+  const int64_t words = layers * per;
+  auto expand = [&](const uint32_t *in, int64_t w0, int64_t n) {
+    nd_host_ranges(n, n < SMALL_ADJACENCY ? 1 : nd_host_threads(), [=](int, int64_t a, int64_t b) {
       for (int64_t w = a; w < b; w++) {
-        const int64_t e0 = 32 * (w0 + w);
-        const size_t len = (size_t)std::min<int64_t>(32, entries - e0);
-        int32_t *r = row + e0, *c = col + e0;
-        if (len == 32) { memset(r, 0xff, 128); memset(c, 0xff, 128); }
-        else { memset(r, 0xff, 4 * len); memset(c, 0xff, 4 * len); }
-        const int64_t at = e0 % stride;
+        const int64_t layer = (w0 + w) / per;
+        const int at = (int)((w0 + w) - layer * per) * 32;
+        const int64_t e0 = layer * stride + at;
+        const size_t len = (size_t)std::min(32, stride - at);
+        if (len == 32) {
+          if (row) memset(row + e0, 0xff, 128);
+          if (col) memset(col + e0, 0xff, 128);
+        } else {
+          if (row) memset(row + e0, 0xff, 4 * len);
+          if (col) memset(col + e0, 0xff, 4 * len);
+        }
         for (uint32_t left = in[w]; left; left &= left - 1) {
-          const int k = __builtin_ctz(left);
-          const int p = (int)((at + k) % stride);   // in the layer of a sample: transit p / L, vertex p % L
-          r[k] = p / L;
-          c[k] = p % L;
+          const int k = __builtin_ctz(left);   // in the layer: transit (at + k) / L, vertex (at + k) % L
+          if (row) row[e0 + k] = (at + k) / L;
+          if (col) col[e0 + k] = (at + k) % L;
         }
       }
     });
+  };
+  std::unique_lock<std::mutex> lock(g_ring.m, std::defer_lock);
+  if (words >= SMALL_ADJACENCY && lock.try_lock() && ring_ready(device)) {
+    const int64_t most = (int64_t)(PIECE * RING / 4);
+    for (int64_t w0 = 0; w0 < words; w0 += most) {
+      const int64_t n = std::min(most, words - w0);
+      ND_CUDA(cudaMemcpyAsync(g_ring.pinned, bits + w0, 4 * (size_t)n, cudaMemcpyDeviceToHost, g_ring.stream));
+      ND_CUDA(cudaStreamSynchronize(g_ring.stream));
+      expand((const uint32_t *)g_ring.pinned, w0, n);
+    }
+    return ND_OK;
   }
-  *done = true;
+  if (lock.owns_lock()) lock.unlock();
+  const int64_t most = std::min<int64_t>(words, 1 << 20);
+  const std::unique_ptr<uint32_t[]> in(new (std::nothrow) uint32_t[(size_t)most]);
+  ND_REQUIRE(in, ND_ERR_RANGE, "no memory for the adjacency's bits");
+  for (int64_t w0 = 0; w0 < words; w0 += most) {
+    const int64_t n = std::min(most, words - w0);
+    ND_TRY(nd_copy_to_host(device, in.get(), bits + w0, 4 * (size_t)n));
+    expand(in.get(), w0, n);
+  }
   return ND_OK;
 }
 

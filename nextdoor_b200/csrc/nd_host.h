@@ -28,9 +28,9 @@ int nd_copy_to_device(int device, void *dst, const void *src, size_t bytes);
 int nd_copies_to_host(int device, int n, void *const *dst, const void *const *src, const size_t *bytes);     // several as one
 int nd_copies_to_device(int device, int n, void *const *dst, const void *const *src, const size_t *bytes);
 
-// Adjacency entries (row, col) = (i, j) or (-1, -1), entry i * L + j of a block of `stride`, from a bit each.  *done:
-// false where the ring cannot be had; nothing is written then.
-int nd_adjacency_to_host(int device, const uint32_t *bits, int64_t entries, int stride, int L, int32_t *row, int32_t *col, bool *done);
+// Adjacency entries (row, col) = (i, j) or (-1, -1), entry i * L + j of a layer of `stride`, from a bit each, a layer in whole
+// words; row or col may be null.
+int nd_adjacency_to_host(int device, const uint32_t *bits, int64_t layers, int stride, int L, int32_t *row, int32_t *col);
 
 // Device memory for building graphs.  Blocks of up to 384 MB are kept for the next build when they are freed, 1 GB of
 // them in all, while graphs or samplers are alive (a cudaMalloc / cudaFree pair costs 0.5 to 30 ms, by the box); an

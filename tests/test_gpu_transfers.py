@@ -161,6 +161,19 @@ def test_adjacency_crosses_as_bits(nd, ndo, small_graph, app, L, B, S):
     assert (aux["adj_row"] >= 0).sum() > 0
 
 
+@pytest.mark.parametrize("L,B,S", [(33, 20, 3), (33, 20, 300), (64, 64, 100)])
+def test_one_array_of_an_adjacency(nd, small_graph, L, B, S):
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    s = nd.Sampler(g, nd.app_params(6, steps=3, fanout=L, batch=B, seed=6), num_samples=S)
+    s.sample()
+    both = s.aux()
+    for k in ("adj_row", "adj_col"):
+        one = np.full(both[k].size + 1, 7, np.int32)
+        ptr = one.ctypes.data
+        nd.check(nd.lib.nd_sampler_aux(s._h, ptr if k == "adj_row" else None, ptr if k == "adj_col" else None, None, None))
+        assert np.array_equal(one[:-1], both[k].reshape(-1)) and one[-1] == 7
+
+
 def test_results_own_their_memory(nd, small_graph):
     g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
     s = nd.Sampler(g, nd.app_params(0, steps=10, seed=2), num_samples=300_000)
