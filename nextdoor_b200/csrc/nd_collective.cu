@@ -51,12 +51,14 @@ struct RefLayout {
   uint32_t off_ids, off_tr, off_rs, off_deg, off_pre, off_filter, off_flags;    // bytes
   uint32_t bytes;
   int flag_words;                                                      // per transit
+  uint32_t inv_L;                                                      // 2^32 / L, rounded up (L > 1): x / L is the high half of x * inv_L below 2^16
 };
 
 static RefLayout ref_layout(int steps, int B, int L) {
   RefLayout r;
   const int ntr = B > L ? B : L;
   r.flag_words = (L + 31) / 32;
+  r.inv_L = L > 1 ? (uint32_t)((((uint64_t)1 << 32) + (uint32_t)L - 1) / (uint32_t)L) : 0u;
   // (a layer's filter is a kilobyte: no more than 24 of them fit, and the sums below stay in 32 bits)
   for (r.per_pass = std::min(steps, 24);; r.per_pass--) {
     const uint32_t k = (uint32_t)r.per_pass, nt = k * (uint32_t)ntr;
@@ -169,12 +171,18 @@ coll_ref_kernel(NdGraphView g, CollParams cp, RefLayout lay, int steps, int64_t 
         }
 #pragma unroll
         for (int j = 0; j < LOADS; j++) {
-          if (v[j] < 0) continue;
-          const int k = at[j] < n0 ? 0 : 1 + (at[j] - n0) / L;
-          if (!((filter[k * FILTER_WORDS + (((uint32_t)v[j] >> 5) & (FILTER_WORDS - 1))] >> (v[j] & 31)) & 1u)) continue;
-          const int32_t *layer = ids + L + k * L;
-          for (int q = 0; q < L; q++)
-            if (layer[q] == v[j]) atomicOr(flags + at[j] * lay.flag_words + (q >> 5), 1u << (q & 31));
+          const int x = at[j] - n0, k = x < 0 ? 0 : 1 + (L > 1 ? (int)__umulhi((uint32_t)x, lay.inv_L) : x);
+          const bool may = v[j] >= 0 && ((filter[k * FILTER_WORDS + (((uint32_t)v[j] >> 5) & (FILTER_WORDS - 1))] >> (v[j] & 31)) & 1u);
+          for (uint32_t left = __ballot_sync(0xffffffffu, may); left; left &= left - 1) {   // the warp looks for each of them
+            const int src = __ffs(left) - 1;
+            const int32_t id = __shfl_sync(0xffffffffu, v[j], src);
+            const int i = __shfl_sync(0xffffffffu, at[j], src), layer = __shfl_sync(0xffffffffu, k, src);
+            for (int w = 0; w < lay.flag_words; w++) {
+              const int q = 32 * w + lane;
+              const uint32_t found = __ballot_sync(0xffffffffu, q < L && ids[L + layer * L + q] == id);
+              if (found && lane == 0) atomicOr(flags + i * lay.flag_words + w, found);
+            }
+          }
         }
       }
       const int nheavy = heavy;
