@@ -75,6 +75,15 @@ static RefLayout ref_layout(int steps, int B, int L) {
   }
 }
 
+// the last i of [lo, hi] with pre[i] <= f, lo if there is none
+__device__ __forceinline__ int last_at_most(const uint32_t *pre, int lo, int hi, uint32_t f) {
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (pre[mid] <= f) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
 __global__ void __launch_bounds__(CTHREADS)
 coll_ref_kernel(NdGraphView g, CollParams cp, RefLayout lay, int steps, int64_t S, const int32_t *__restrict__ initial, int32_t *__restrict__ out,
                 uint32_t *__restrict__ adj, unsigned long long *__restrict__ stats) {
@@ -139,36 +148,33 @@ coll_ref_kernel(NdGraphView g, CollParams cp, RefLayout lay, int steps, int64_t 
         carry += all;
         __syncthreads();
       }
-      // the entries of the short lists; a thread's loads are independent
+      // the entries of the short lists: a warp takes a run of them, a lane four neighbouring ones at a time
       constexpr int LOADS = 4;
-      for (uint32_t c0 = (uint32_t)warp * (32 * LOADS); c0 < carry; c0 += CTHREADS * LOADS) {
+      const uint32_t chunks = (carry + 32 * LOADS - 1) / (32 * LOADS), each = (chunks + CTHREADS / 32 - 1) / (CTHREADS / 32) * (32 * LOADS);
+      const uint32_t run_end = min(((uint32_t)warp + 1u) * each, carry);
+      int from = 0;   // transit of the chunk's first entry: the last with pre <= c0
+      if (warp * each < run_end) from = last_at_most(pre, 0, nt - 1, warp * each);
+      for (uint32_t c0 = warp * each; c0 < run_end; c0 += 32 * LOADS) {
         int32_t v[LOADS];
         int at[LOADS];
-        // transits of the warp's first and last entry: last with pre <= f
-        const uint32_t c1 = min(c0 + 32 * LOADS, carry) - 1;
-        int from = 0, to = nt - 1;
-        for (int hi = to; from < hi;) {
-          const int mid = (from + hi + 1) >> 1;
-          if (pre[mid] <= c0) from = mid; else hi = mid - 1;
-        }
-        for (int lo = from; lo < to;) {
-          const int mid = (lo + to + 1) >> 1;
-          if (pre[mid] <= c1) lo = mid; else to = mid - 1;
-        }
+        const uint32_t c1 = min(c0 + 32 * LOADS, run_end) - 1;
+        int to;   // transit of its last entry: seldom 32 further on
+        const uint32_t within = __ballot_sync(0xffffffffu, from + 1 + lane < nt && pre[from + 1 + lane] <= c1);
+        if (within == 0xffffffffu) to = last_at_most(pre, from + 32, nt - 1, c1);
+        else to = from + __popc(within);
+        const uint32_t f0 = c0 + (uint32_t)(LOADS * lane);
+        int lo = f0 <= c1 ? last_at_most(pre, from, to, f0) : to;
 #pragma unroll
         for (int j = 0; j < LOADS; j++) {
-          const uint32_t f = c0 + (uint32_t)(j * 32 + lane);
-          v[j] = -1; at[j] = 0;
-          if (f < carry) {
-            int lo = from, hi = to;
-            while (lo < hi) {
-              const int mid = (lo + hi + 1) >> 1;
-              if (pre[mid] <= f) lo = mid; else hi = mid - 1;
-            }
-            at[j] = lo;
+          const uint32_t f = f0 + j;
+          v[j] = -1;
+          if (f <= c1) {
+            while (lo < to && pre[lo + 1] <= f) lo++;
             v[j] = __ldg(g.col + rs[lo] + (int32_t)(f - pre[lo]));
           }
+          at[j] = lo;
         }
+        from = to;
 #pragma unroll
         for (int j = 0; j < LOADS; j++) {
           const int x = at[j] - n0, k = x < 0 ? 0 : 1 + (L > 1 ? (int)__umulhi((uint32_t)x, lay.inv_L) : x);
