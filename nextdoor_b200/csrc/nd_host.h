@@ -22,6 +22,9 @@ void nd_host_ranges(int64_t count, int threads, F fn) {
   nd_host_run(threads, [&](int t) { fn(t, count * t / threads, count * (t + 1) / threads); });
 }
 
+// `n` words, written past the caches.
+void nd_fill_past_caches(int32_t *to, int64_t n, int32_t value);
+
 // Blocking copies on a stream of their own: everything the copy depends on has to be complete.
 int nd_copy_to_host(int device, void *dst, const void *src, size_t bytes);
 int nd_copy_to_device(int device, void *dst, const void *src, size_t bytes);

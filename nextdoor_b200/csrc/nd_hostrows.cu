@@ -347,7 +347,7 @@ int nd_host_fill_int32(int32_t *dst, int64_t n, int32_t value) {
   ND_REQUIRE(dst || n == 0, ND_ERR_ARG, "nd_host_fill_int32: null destination");
   ND_REQUIRE(n >= 0, ND_ERR_ARG, "nd_host_fill_int32: negative length");
   nd_host_ranges(n, nd_host_threads(), [=](int, int64_t a, int64_t b) {
-    for (int64_t i = a; i < b; i++) dst[i] = value;
+    nd_fill_past_caches(dst + a, b - a, value);
   });
   return ND_OK;
 }

@@ -92,3 +92,13 @@ def test_header_is_plain_c_and_cxx():
         exe = shutil.which(cc) or os.path.join("/usr/bin", cc)
         r = subprocess.run([exe, std, "-fsyntax-only", "-Wall", "-x", lang, hdr], capture_output=True, text=True)
         assert r.returncode == 0, r.stderr
+
+
+@pytest.mark.parametrize("offset", range(5))
+@pytest.mark.parametrize("n", [0, 1, 3, 4, 67, 100_003])
+def test_host_fill_of_any_words(offset, n):
+    import numpy as np
+    from nextdoor_b200 import api
+    a = np.full(n + 16, -5, np.int32)
+    api.host_fill(a[offset:offset + n], 7)
+    assert (a[offset:offset + n] == 7).all() and (a[:offset] == -5).all() and (a[offset + n:] == -5).all()
