@@ -7,8 +7,8 @@
 // integer weights sum exactly).
 //
 // What bounds it, and what is done about it (2^20 vertices, 1024 batches of 64, 2 layers of 64: FastGCN
-// 4.8 -> 0.98 ms, LADIES 5.7 -> 1.07 ms).  One CTA fills an SM, and neither memory nor issue slots are full: FastGCN issues
-// in 58 % of the cycles (612 M warp instructions; 5.6 GB out of the L2 at 24 % of its rate), LADIES in 57 % (610 M
+// 4.8 -> 0.89 ms, LADIES 5.7 -> 1.07 ms).  One CTA fills an SM, and neither memory nor issue slots are full: FastGCN issued
+// in 58 % of the cycles at 0.98 ms (5.6 GB out of the L2 at 24 % of its rate), LADIES in 57 % (610 M
 // instructions for 131 M list entries, the distinct ones of 313 M), its shared memory is busy in half of them; the warps
 // wait for barriers between the phases, for shared memory and for loads:
 //  * The second layer's transits are hubs (FastGCN draws them with the square of their degree), many of them the
@@ -19,7 +19,10 @@
 //  * FastGCN's weights are summed without a list of candidates (writing that and fetching deg^2 one by one took more
 //    than half of the time): the degrees lie in vertex order as two planes of bytes, a lane takes eight vertices with one
 //    16-byte load, masks them with its byte of the bitmap and squares and sums them with dp4a.  Vertices with 2048
-//    neighbours or more, whose squares would overflow the 32-bit group sums, are a short list per graph.
+//    neighbours or more, whose squares would overflow the 32-bit group sums, are a short list per graph.  Groups without a
+//    candidate, most of a first layer's, are passed over; the list's weights are added up per group across the lanes; a
+//    draw asks for all row offsets of its group at once (0.98 -> 0.89 ms; the squares as three planes of bytes: 1.01, the
+//    third costs more than the products save).
 //  * LADIES' terms (w / rowsum)^2 depend on the edge alone: an array, built once per graph, instead of a pass over
 //    the weights and a division per entry and sample.  One pass over the lists sets the union's bits and adds the terms
 //    up per group; then the groups that the draws fall into get an accumulator per vertex, where the union was,
@@ -46,7 +49,7 @@ constexpr int GROUP_WORDS = 16;   // words of a FastGCN group; bitmaps are whole
 constexpr int GROUP = 512;        // FastGCN: vertices (GROUP_WORDS words) whose weights are summed together
 constexpr int LADIES_GROUP_BITS = 7;   // LADIES: 2^7 vertices, more where the sums of the groups would not fit shared memory
 constexpr int BIG_DEGREE = 2048;  // from here a vertex is on the list of big ones and its code is 0: 512 * 2047^2 < 2^31
-constexpr int FLIGHT = 4;         // groups a warp sums at a time
+constexpr int FLIGHT = 3;         // groups a warp sums at a time
 constexpr int HUB = 128, LADIES_HUB = 64;   // a vertex with at least V / HUB neighbours has a bitmap of them, and is ORed from V / LADIES_HUB on
 constexpr int BIG_LIST = 4096;    // lists at least this long are streamed by the whole CTA
 constexpr int VEC = 4;            // 16-byte loads in flight per thread
@@ -324,13 +327,19 @@ __device__ __forceinline__ void pick_in_group(const double *acc, const uint32_t 
 // bits 0..3 -> 0xff in bytes 0..3
 __device__ __forceinline__ uint32_t byte_mask(uint32_t bits) { return (((bits & 15u) * 0x204081u) & 0x01010101u) * 255u; }
 
-// sum of deg^2 over the vertices of `bits` (eight vertices, degrees as in Args::deg)
-__device__ __forceinline__ uint32_t sum_squares(uint32_t bits, const uint4 &d) {
-  const uint32_t m0 = byte_mask(bits), m1 = byte_mask(bits >> 4);
-  const uint32_t l0 = d.x & m0, l1 = d.y & m1, h0 = d.z & m0, h1 = d.w & m1;
-  const uint32_t ll = __dp4a(l1, l1, __dp4a(l0, l0, 0u)), lh = __dp4a(l1, h1, __dp4a(l0, h0, 0u)), hh = __dp4a(h1, h1, __dp4a(h0, h0, 0u));
-  return ll + (lh << 9) + (hh << 16);
-}
+// The sum of deg^2 over the vertices of `bits` (eight vertices, degrees as in Args::deg), in products of low, low and high, and
+// high bytes.
+struct Squares {
+  uint32_t ll = 0u, lh = 0u, hh = 0u;
+  __device__ __forceinline__ void add(uint32_t bits, const uint4 &d) {
+    const uint32_t m0 = byte_mask(bits), m1 = byte_mask(bits >> 4);
+    const uint32_t l0 = d.x & m0, l1 = d.y & m1;
+    ll = __dp4a(l1, d.y, __dp4a(l0, d.x, ll));
+    lh = __dp4a(l1, d.w, __dp4a(l0, d.z, lh));
+    hh = __dp4a(d.w & m1, d.w, __dp4a(d.z & m0, d.z, hh));
+  }
+  __device__ __forceinline__ uint32_t sum() const { return ll + (lh << 9) + (hh << 16); }
+};
 
 // SUMS_FAR: LADIES' group sums are in the big part.
 template <bool LADIES, bool SUMS_FAR>
@@ -418,18 +427,27 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
         // ---- the groups' weights, and the number of candidates
         const uint8_t *bytes = reinterpret_cast<const uint8_t *>(bm);
         for (int g0 = warp * FLIGHT; g0 < groups; g0 += warps * FLIGHT) {
-          uint32_t bits[2 * FLIGHT];
+          uint32_t bits[2 * FLIGHT], some = 0u;
           uint4 d[2 * FLIGHT];
 #pragma unroll
           for (int k = 0; k < 2 * FLIGHT; k++) {
             const int at = g0 * (GROUP / 8) + k * 32 + lane;
             bits[k] = at < groups * (GROUP / 8) ? bytes[at] : 0u;
-            d[k] = bits[k] ? __ldg(a.deg + at) : make_uint4(0u, 0u, 0u, 0u);
+            some |= bits[k];
           }
+          if (!__any_sync(0xffffffffu, some)) {   // (a first layer's thousand candidates leave most groups empty)
+            if (lane < FLIGHT && g0 + lane < groups) gcdf[g0 + lane] = 0.0;
+            continue;
+          }
+#pragma unroll
+          for (int k = 0; k < 2 * FLIGHT; k++) d[k] = bits[k] ? __ldg(a.deg + g0 * (GROUP / 8) + k * 32 + lane) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
           for (int k = 0; k < FLIGHT; k++) {
             seen += __popc(bits[2 * k] | bits[2 * k + 1] << 8);
-            const uint32_t sum = __reduce_add_sync(0xffffffffu, sum_squares(bits[2 * k], d[2 * k]) + sum_squares(bits[2 * k + 1], d[2 * k + 1]));
+            Squares sq;
+            sq.add(bits[2 * k], d[2 * k]);
+            sq.add(bits[2 * k + 1], d[2 * k + 1]);
+            const uint32_t sum = __reduce_add_sync(0xffffffffu, sq.sum());
             if (lane == 0 && g0 + k < groups) gcdf[g0 + k] = (double)sum;
           }
         }
@@ -437,15 +455,16 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
         for (int i0 = warp * 32; i0 < a.n_big; i0 += warps * 32) {   // the big ones; neighbours on the list mostly share a group
           const NdBigVertex v = i0 + lane < a.n_big ? a.big[i0 + lane] : NdBigVertex{-1, 0.f};
           const bool in = v.v >= 0 && ((bm[v.v >> 5] >> (v.v & 31)) & 1u);
+          // (in order, so that what falls into one group is added up across the lanes first)
           double x = in ? (double)v.weight : 0.0;
-          int same;
-          __match_all_sync(0xffffffffu, v.v / GROUP, &same);
-          if (same) {
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-            if (lane == 0) atomicAdd(gcdf + v.v / GROUP, x);
-          } else if (in) {
-            atomicAdd(gcdf + v.v / GROUP, x);
+          const int group = v.v >= 0 ? v.v / GROUP : -1, group_before = __shfl_up_sync(0xffffffffu, group, 1);
+          const uint32_t heads = __ballot_sync(0xffffffffu, lane == 0 || group != group_before);
+          const int head = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+          for (int o = 1; o < 32; o <<= 1) {
+            const double t = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane - o >= head) x += t;
           }
+          if (x > 0.0 && (lane == 31 || (heads >> (lane + 1)) & 1u)) atomicAdd(gcdf + group, x);
         }
       } else {
         // ---- the groups' weights and the rest of the union, then the number of candidates
@@ -563,28 +582,27 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
           // lane) that reaches the target, then the first of its candidates that does
           float x[4][4];
           uint32_t there = 0;   // which of the lane's sixteen are candidates
+          int32_t at[4][5];
 #pragma unroll
-          for (int q = 0; q < 4; q++) {
-            const uint32_t r = (uint32_t)(lo * GROUP + q * 128 + lane * 4);
-            {
-              const uint32_t bits = (bm[r >> 5] >> (r & 31)) & 15u;
-              const uint32_t *codes = reinterpret_cast<const uint32_t *>(a.deg + (r >> 3)) + ((r >> 2) & 1u);
-              const uint32_t low = bits ? __ldg(codes) : 0u, high = bits ? __ldg(codes + 2) : 0u;
-              there |= bits << (4 * q);
+          for (int q = 0; q < 4; q++) {   // the degrees from the row offsets, all of them asked for at once
+            const int64_t r = (int64_t)lo * GROUP + q * 128 + lane * 4;
+            there |= ((bm[r >> 5] >> (r & 31)) & 15u) << (4 * q);
 #pragma unroll
-              for (int k = 0; k < 4; k++) {
-                int32_t d = (int32_t)((low >> (8 * k) & 255u) | (high >> (8 * k) & 255u) << 8);
-                if (((bits >> k) & 1u) == 0) d = 0;
-                else if (d == 0) d = __ldg(a.g.row_ptr + r + k + 1) - __ldg(a.g.row_ptr + r + k);
-                x[q][k] = __fmul_rn(__int2float_rn(d), __int2float_rn(d));
-              }
-            }
+            for (int k = 0; k < 5; k++) at[q][k] = __ldg(a.g.row_ptr + (r + k < cp.V ? r + k : (int64_t)cp.V));
           }
+#pragma unroll
+          for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+              const float d = (there >> (4 * q + k)) & 1u ? __int2float_rn(at[q][k + 1] - at[q][k]) : 0.f;
+              x[q][k] = __fmul_rn(d, d);
+            }
           double at_block = before, lane_before = 0.0;
           bool found = false;
           int bq = -1, bl = 0;
 #pragma unroll
           for (int q = 0; q < 4; q++) {
+            if (found) break;
             const double mine = ((double)x[q][0] + (double)x[q][1]) + ((double)x[q][2] + (double)x[q][3]);
             double run = mine;
             for (int o = 1; o < 32; o <<= 1) {
@@ -594,13 +612,11 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
             const bool some = (there >> (4 * q)) & 15u;
             const uint32_t reach = __ballot_sync(0xffffffffu, some && at_block + run >= target), any = __ballot_sync(0xffffffffu, some);
             // (nobody reaches it, by rounding: the last candidates of the group)
-            if (bq < 0 || !found) {
-              if (reach || any) {
-                bq = q;
-                bl = reach ? __ffs(reach) - 1 : 31 - __clz(any);
-                lane_before = at_block + __shfl_sync(0xffffffffu, run - mine, bl);
-                found = reach != 0u;
-              }
+            if (any) {
+              bq = q;
+              bl = reach ? __ffs(reach) - 1 : 31 - __clz(any);
+              lane_before = at_block + __shfl_sync(0xffffffffu, run - mine, bl);
+              found = reach != 0u;
             }
             at_block += __shfl_sync(0xffffffffu, run, 31);
           }
