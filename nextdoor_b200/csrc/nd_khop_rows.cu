@@ -30,7 +30,7 @@ constexpr int CTAS_DISTINCT = 6;
 __host__ __device__ constexpr int khop_ctas(bool distinct) { return distinct ? CTAS_DISTINCT : CTAS; }
 
 struct KhopRows {
-  uint64_t seed;
+  ndrng::RoundKeys keys;
   int64_t first_sample, S;
   int32_t V, fs;
   int steps;
@@ -45,6 +45,13 @@ struct KhopRows {
   unsigned long long *__restrict__ acc;    // counters of the running job: [0] edges, [1] pairs, [8] samples handed out, [10] CTAs that are done; zero between jobs
   unsigned long long *__restrict__ stats;  // published by the last CTA
 };
+
+// the first draw of a slot, below n
+__device__ __forceinline__ int32_t draw(const KhopRows &a, uint32_t sample, int hop, int slot, int32_t n) {
+  uint32_t o[4];
+  ndrng::philox4x32_10(sample, (uint32_t)hop, (uint32_t)slot, 0u, a.keys, o);
+  return ndrng::rand_int_from(ndrng::u32_to_uniform(o[0]), n);
+}
 
 // Entry (relative to the list) that slot j of a parent with `deg` > f neighbours picks without replacement:
 // Floyd, slot after slot -- a candidate that is taken is replaced by m_j = deg - f + j.  Slot j's candidate is
@@ -130,8 +137,7 @@ khop_rows_kernel(const __grid_constant__ KhopRows a) {
         if (!DISTINCT) {
           for (int c = lane; c < n_live * f; c += 32) {
             const int l = c / f, slot = live_p[l] * f + (c - l * f);
-            ndrng::Rng rng(a.seed, gs, (uint32_t)k, (uint32_t)slot);
-            row[prefix + slot] = live_rs[l] + rng.rand_int(live_deg[l]);
+            row[prefix + slot] = live_rs[l] + draw(a, gs, k, slot, live_deg[l]);
           }
         } else {
           const int per = 32 / f, sub = lane / f, j = lane - sub * f, base = sub * f;
@@ -143,8 +149,7 @@ khop_rows_kernel(const __grid_constant__ KhopRows a) {
             const int slot = on ? live_p[l] * f + j : 0;
             int32_t idx = deg <= f ? (j < deg ? j : -1) : 0;
             if (deg > f) {
-              ndrng::Rng rng(a.seed, gs, (uint32_t)k, (uint32_t)slot);
-              idx = rng.rand_int(deg - f + j + 1);
+              idx = draw(a, gs, k, slot, deg - f + j + 1);
             }
             const int32_t pick = floyd(deg > f ? idx : -1 - lane, deg, f, j, base, group, deg > f);
             if (deg > f) idx = pick;
@@ -263,7 +268,7 @@ int nd_khop_rows_launch(nd_sampler *s) {
   const nd_app_params &p = s->p;
   const bool distinct = p.app == ND_APP_KHOP_DISTINCT;
   KhopRows a;
-  a.seed = p.seed; a.first_sample = s->first; a.S = s->S; a.V = s->g->V; a.fs = s->fs; a.steps = p.steps;
+  a.keys = ndrng::RoundKeys(p.seed); a.first_sample = s->first; a.S = s->S; a.V = s->g->V; a.fs = s->fs; a.steps = p.steps;
   int n = 1;
   a.parents_max = 1;
   for (int k = 0; k < p.steps; k++) {

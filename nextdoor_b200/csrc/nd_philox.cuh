@@ -34,6 +34,31 @@ __host__ __device__ __forceinline__ void philox4x32_10(uint32_t c0, uint32_t c1,
   out[0] = c0; out[1] = c1; out[2] = c2; out[3] = c3;
 }
 
+// The keys of the ten rounds, from the run seed, as part of a kernel's parameters: there they are operands of the rounds'
+// exclusive-ors, where keys made on the way are two more instructions a round.
+struct RoundKeys {
+  uint32_t k[20];
+  __host__ explicit RoundKeys(uint64_t seed) {
+    for (uint32_t r = 0; r < 10; r++) {
+      k[2 * r] = (uint32_t)seed + r * 0x9E3779B9u;
+      k[2 * r + 1] = (uint32_t)(seed >> 32) + r * 0xBB67AE85u;
+    }
+  }
+  RoundKeys() = default;
+};
+
+__device__ __forceinline__ void philox4x32_10(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, const RoundKeys &keys, uint32_t out[4]) {
+#pragma unroll
+  for (int r = 0; r < 10; r++) {
+    const uint32_t hi0 = __umulhi(0xD2511F53u, c0), lo0 = 0xD2511F53u * c0;
+    const uint32_t hi1 = __umulhi(0xCD9E8D57u, c2), lo1 = 0xCD9E8D57u * c2;
+    c0 = hi1 ^ c1 ^ keys.k[2 * r];
+    c2 = hi0 ^ c3 ^ keys.k[2 * r + 1];
+    c1 = lo1; c3 = lo0;
+  }
+  out[0] = c0; out[1] = c1; out[2] = c2; out[3] = c3;
+}
+
 __device__ __forceinline__ float u32_to_uniform(uint32_t x) {
   // one exact power-of-two scaling and one rounded add: identical to the host oracle
   return __fadd_rn(__fmul_rn(__uint2float_rn(x), 2.3283064365386963e-10f), 1.1641532182693481e-10f);

@@ -46,7 +46,7 @@ struct RowsArgs {
   const uint2 *__restrict__ col3;    // [E/3] three neighbours of 21 bits each
   const int32_t *__restrict__ adjset;
   const uint32_t *__restrict__ adjsign;
-  uint64_t seed;
+  ndrng::RoundKeys keys;
   float p, q, stop_prob;
   int n2v_compat, steps;
   int64_t first_sample, S;
@@ -209,7 +209,7 @@ struct Rows {
 };
 
 __device__ __forceinline__ void draw_block(const RowsArgs &a, uint32_t s, int step, uint32_t block, uint32_t (&o)[4]) {
-  ndrng::philox4x32_10((uint32_t)(a.first_sample + s), (uint32_t)step, 0u, block, (uint32_t)a.seed, (uint32_t)(a.seed >> 32), o);
+  ndrng::philox4x32_10((uint32_t)(a.first_sample + s), (uint32_t)step, 0u, block, a.keys, o);
 }
 __device__ __forceinline__ int32_t draw_index(uint32_t u, int32_t n) { return ndrng::rand_int_from(ndrng::u32_to_uniform(u), n); }
 
@@ -221,7 +221,7 @@ __device__ __forceinline__ int32_t draw_index(uint32_t u, int32_t n) { return nd
 // walks all have a lane takes them in order, without the pass that makes the list.
 constexpr int START_PER_THREAD = 4;
 template <int APP, int LAYOUT>
-__global__ void __launch_bounds__(256) walk_start_kernel(const RowsArgs a) {
+__global__ void __launch_bounds__(256) walk_start_kernel(const __grid_constant__ RowsArgs a) {
   __shared__ uint32_t sh_n, sh_dead;
   __shared__ unsigned long long sh_base;
   if (threadIdx.x == 0) { sh_n = 0u; sh_dead = 0u; }
@@ -631,7 +631,7 @@ __device__ __forceinline__ void walks(const RowsArgs &a) {
 
 // Both modes; the load-balanced one also counts the walks that are alive at every step (RowsArgs::ended).
 template <int APP, int LAYOUT>
-__global__ void __launch_bounds__(ROWS_THREADS, ROWS_CTAS) walk_next_count_kernel(const RowsArgs a) { walks<APP, LAYOUT>(a); }
+__global__ void __launch_bounds__(ROWS_THREADS, ROWS_CTAS) walk_next_count_kernel(const __grid_constant__ RowsArgs a) { walks<APP, LAYOUT>(a); }
 
 // ---------------------------------------------------------------- layouts, built by a graph's first sampler that reads them
 
@@ -892,7 +892,7 @@ int nd_walk_rows_launch(nd_sampler *s, bool count) {
   const nd_graph *g = s->g;
   uint32_t *ended = count ? reinterpret_cast<uint32_t *>(s->d_rows_acc + 16) : nullptr;
   RowsArgs a{g->V, g->row_ptr, g->col, g->w, g->max_w, g->vrow, g->erec, g->colw, g->vrec, g->pack, g->col3, g->adjset, g->adjsign,
-             s->p.seed, s->p.p, s->p.q, s->p.stop_prob, s->p.n2v_ref_compat, s->p.steps, s->first, s->S, s->d_initial, s->d_out,
+             ndrng::RoundKeys(s->p.seed), s->p.p, s->p.q, s->p.stop_prob, s->p.n2v_ref_compat, s->p.steps, s->first, s->S, s->d_initial, s->d_out,
              s->d_plen, s->d_list, s->d_rows_acc, ended, s->d_stats, (uint32_t *)s->d_nlive, s->d_status};
   switch (s->p.app) {
     case ND_APP_UNIFORM_WALK: launch_as<ND_APP_UNIFORM_WALK>(s, a, count); break;
