@@ -92,6 +92,32 @@ __global__ void unpack_arrays_kernel(int64_t n, const uint32_t *__restrict__ src
   facts_out(facts, m, bad, ka, ko);
 }
 
+// Records whose weights are still on the way: what their ids say, and their places in the order of arrival.
+__global__ void id_facts_kernel(int64_t n, const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst, uint32_t *__restrict__ place,
+                                RecordFacts *__restrict__ facts) {
+  int32_t m = -1;
+  bool bad = false;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t s = (int32_t)src[i], d = (int32_t)dst[i];
+    place[i] = (uint32_t)i;
+    bad |= s < 0 || d < 0;
+    m = max(m, max(s, d));
+  }
+  facts_out(facts, m, bad, 0xffffffffu, 0u);
+}
+
+// ... and the weights' keys once these are there and the places sorted
+__global__ void place_weights_kernel(int64_t n, const uint32_t *__restrict__ place, const float *__restrict__ w, uint32_t *__restrict__ wk,
+                                     RecordFacts *__restrict__ facts) {
+  uint32_t ka = 0xffffffffu, ko = 0u;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t k = float_to_key(__ldg(w + place[i]));
+    wk[i] = k;
+    ka &= k; ko |= k;
+  }
+  facts_out(facts, -1, false, ka, ko);
+}
+
 // R-MAT (a,b,c,d) = (.57,.19,.19,.05).  Undirected edge e, attempt t: Philox counter
 // (e_lo, e_hi, t, level/4), key = seed ^ "RMAT"; level l consumes draw l with integer quadrant
 // thresholds; an attempt with an endpoint >= V or src == dst is retried; the weight is draw
@@ -141,7 +167,8 @@ struct RunList {
   int32_t too_long, count;
 };
 __global__ void sort_runs_kernel(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst, uint32_t *__restrict__ wk, int64_t n,
-                                 RunList *__restrict__ runs, uint32_t *__restrict__ list) {
+                                 RunList *__restrict__ runs, uint32_t *__restrict__ list, const RecordFacts *__restrict__ facts) {
+  if (facts->key_and == facts->key_or) return;   // all weights are the same
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i + 1 < n; i += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t s = src[i], d = dst[i], s1 = src[i + 1], d1 = dst[i + 1];   // (loads that do not wait for one another)
     if (s1 != s || d1 != d || (i > 0 && src[i - 1] == s && dst[i - 1] == d)) continue;
@@ -199,32 +226,29 @@ __global__ void __launch_bounds__(256) sort_long_runs_kernel(const uint32_t *__r
   }
 }
 
-// The sorted records become the CSR: row_ptr (element i closes the rows (src[i-1], src[i]]), col, w.
-__global__ void csr_from_sorted_kernel(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst, const uint32_t *__restrict__ wk,
-                                       int64_t n, int32_t V, int32_t *__restrict__ row_ptr, int32_t *__restrict__ col, float *__restrict__ w) {
+// The sorted records become the CSR: row_ptr (element i closes the rows (src[i-1], src[i]]) and col.
+__global__ void csr_from_sorted_kernel(const uint32_t *__restrict__ src, const uint32_t *__restrict__ dst, int64_t n, int32_t V,
+                                       int32_t *__restrict__ row_ptr, int32_t *__restrict__ col) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t lo = i == 0 ? 0 : (int64_t)src[i - 1] + 1;
     const int64_t hi = i == n ? V : (int64_t)src[i];
     for (int64_t v = lo; v <= hi; v++) row_ptr[v] = (int32_t)i;
-    if (i < n) {
-      col[i] = (int32_t)dst[i];
-      w[i] = key_to_float(wk[i]);
-    }
+    if (i < n) col[i] = (int32_t)dst[i];
   }
 }
 
 // Vertex::max_weight (src/graph.hpp:71-80) starts from 0, so only positive weights can raise it
 // and their bit patterns order like ints.  Thread per edge; the owner row comes from the sorted
 // src array when the CSR was just built here, else from a bisection of row_ptr; a warp whose 32
-// edges share one row reduces first and issues a single atomic.
-__global__ void max_weight_kernel(const int32_t *__restrict__ row_ptr, const uint32_t *__restrict__ src,
-                                  const float *__restrict__ w, int32_t V, int64_t E,
-                                  int32_t *__restrict__ max_w_bits) {
+// edges share one row reduces first and issues a single atomic.  With wk, the sorted weights' keys, it makes the weights, too.
+__global__ void max_weight_kernel(const int32_t *__restrict__ row_ptr, const uint32_t *__restrict__ src, const uint32_t *__restrict__ wk,
+                                  float *__restrict__ w, int32_t V, int64_t E, int32_t *__restrict__ max_w_bits) {
   for (int64_t base = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~31ll; base < E;
        base += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = base + (threadIdx.x & 31);
     const bool in = i < E;
-    const float x = in ? w[i] : 0.f;
+    const float x = !in ? 0.f : wk ? key_to_float(wk[i]) : w[i];
+    if (in && wk) w[i] = x;
     int32_t v = -1;
     if (in) {
       if (src) {
@@ -356,11 +380,26 @@ int build_scratch(BuildScratch *s, int device, int64_t n) {
 // with random weights (8.4M records on the host to a graph, copies included: 6.1 ms -> 4.9; 4.0 since the scatter of
 // nd_radix.cu, of it 0.89 on the device: the passes 0.11 each).  A graph that repeats one edge thousands of times goes
 // on to the full sort.
-int build_from_soa(const NdDeviceInfo &dev, int64_t n, int32_t V, BuildScratch *bs, int lo_bit, int hi_bit, nd_graph **out) {
-  ND_REQUIRE(n < ((int64_t)1 << 31), ND_ERR_RANGE, "%lld edges do not fit the int32 edge index of the CSR", (long long)n);
-  const int vbits = nd_bit_length((uint32_t)(V > 1 ? V - 1 : 1));
-  uint32_t *cur[3] = {bs->a[0], bs->a[1], bs->a[2]}, *oth[3] = {bs->b[0], bs->b[1], bs->b[2]};
-  auto sort_by = [&](int word, int bits, int lo) -> int {
+struct Build {
+  const NdDeviceInfo &dev;
+  const int64_t n;
+  const int32_t V;
+  BuildScratch *bs;
+  const int vbits;
+  uint32_t *cur[3], *oth[3];
+  nd_graph *g = nullptr;
+
+  Build(const NdDeviceInfo &dev_, int64_t n_, int32_t V_, BuildScratch *bs_)
+      : dev(dev_), n(n_), V(V_), bs(bs_), vbits(nd_bit_length((uint32_t)(V_ > 1 ? V_ - 1 : 1))) {
+    for (int w = 0; w < 3; w++) { cur[w] = bs->a[w]; oth[w] = bs->b[w]; }
+  }
+  ~Build() {   // a build that fails gives the graph's memory back
+    if (!g) return;
+    nd_block_free(dev.device, g->block, g->block_bytes);
+    delete g;
+  }
+
+  int sort_by(int word, int bits, int lo) {
     if (n < 2 || bits <= 0) return ND_OK;
     NdSortArrays arr;
     arr.nwords = 3;
@@ -371,47 +410,66 @@ int build_from_soa(const NdDeviceInfo &dev, int64_t n, int32_t V, BuildScratch *
     ND_TRY(nd_radix_sort(dev, nullptr, &bs->radix, pl, arr, word, bs->d_n, nullptr, false, 0u, false, &in_b));
     if (in_b) for (int w = 0; w < 3; w++) { uint32_t *t = cur[w]; cur[w] = oth[w]; oth[w] = t; }
     return ND_OK;
-  };
-  ND_TRY(sort_by(1, vbits, 0));
-  ND_TRY(sort_by(0, vbits, 0));
-  if (hi_bit > lo_bit && n > 1) {
+  }
+  int sort_by_ids() {
+    ND_TRY(sort_by(1, vbits, 0));
+    return sort_by(0, vbits, 0);
+  }
+
+  // cur[2] (weight keys) of records that share both ids, brought into order
+  int sort_weights(int lo_bit, int hi_bit) {
+    if (hi_bit <= lo_bit || n <= 1) return ND_OK;
     RunList runs;
-    sort_runs_kernel<<<grid_for(n, 256, dev.sms), 256>>>(cur[0], cur[1], cur[2], n, bs->runs, oth[0]);
+    sort_runs_kernel<<<grid_for(n, 256, dev.sms), 256>>>(cur[0], cur[1], cur[2], n, bs->runs, oth[0], bs->facts);
     sort_long_runs_kernel<<<dev.sms * 4, 256>>>(cur[0], cur[1], cur[2], n, bs->runs, oth[0]);
     nd_count_launches(2);
     ND_CUDA(cudaMemcpy(&runs, bs->runs, sizeof(runs), cudaMemcpyDeviceToHost));
-    if (runs.too_long) {
-      ND_TRY(sort_by(2, hi_bit - lo_bit, lo_bit));
-      ND_TRY(sort_by(1, vbits, 0));
-      ND_TRY(sort_by(0, vbits, 0));
-    }
+    if (!runs.too_long) return ND_OK;
+    ND_TRY(sort_by(2, hi_bit - lo_bit, lo_bit));
+    return sort_by_ids();
   }
-  // one block: row offsets, ids and weights (32 bytes of padding for the 16-byte staging windows), maximum weights
-  auto round = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  const size_t o_col = round(4 * ((size_t)V + 1)), o_w = o_col + round(4 * ((size_t)n + 8)), o_max = o_w + round(4 * ((size_t)n + 8));
-  size_t all = o_max + round(4 * (size_t)V);
-  unsigned char *block = nullptr;
-  ND_TRY(nd_block_alloc(dev.device, (void **)&block, &all));
-  nd_graph *g = new nd_graph();
-  g->device = dev.device; g->V = V; g->E = n; g->block = block; g->block_bytes = all;
-  g->row_ptr = (int32_t *)block; g->col = (int32_t *)(block + o_col); g->w = (float *)(block + o_w); g->max_w = (float *)(block + o_max);
-  auto build = [&]() -> int {
+
+  // the graph's arrays, from the sorted ids
+  int csr() {
+    // one block: row offsets, ids and weights (32 bytes of padding for the 16-byte staging windows), maximum weights
+    auto round = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t o_col = round(4 * ((size_t)V + 1)), o_w = o_col + round(4 * ((size_t)n + 8)), o_max = o_w + round(4 * ((size_t)n + 8));
+    size_t all = o_max + round(4 * (size_t)V);
+    unsigned char *block = nullptr;
+    ND_TRY(nd_block_alloc(dev.device, (void **)&block, &all));
+    g = new nd_graph();
+    g->device = dev.device; g->V = V; g->E = n; g->block = block; g->block_bytes = all;
+    g->row_ptr = (int32_t *)block; g->col = (int32_t *)(block + o_col); g->w = (float *)(block + o_w); g->max_w = (float *)(block + o_max);
     ND_CUDA(cudaMemsetAsync(g->col + n, 0, sizeof(int32_t) * 8));
     ND_CUDA(cudaMemsetAsync(g->w + n, 0, sizeof(float) * 8));
     ND_CUDA(cudaMemsetAsync(g->max_w, 0, sizeof(float) * (size_t)V));
-    csr_from_sorted_kernel<<<grid_for(n + 1, 256, dev.sms), 256>>>(cur[0], cur[1], cur[2], n, V, g->row_ptr, g->col, g->w);
-    if (n > 0) max_weight_kernel<<<grid_for(n, 256, dev.sms), 256>>>(g->row_ptr, cur[0], g->w, V, n, (int32_t *)g->max_w);
+    csr_from_sorted_kernel<<<grid_for(n + 1, 256, dev.sms), 256>>>(cur[0], cur[1], n, V, g->row_ptr, g->col);
     max_degree_kernel<<<grid_for(V, 256, dev.sms), 256>>>(g->row_ptr, V, bs->d_max_degree);
-    nd_count_launches(3);
+    nd_count_launches(2);
+    ND_CUDA(cudaGetLastError());
+    return ND_OK;
+  }
+
+  // ... and the weights, from their sorted keys
+  int finish(nd_graph **out) {
+    if (n > 0) max_weight_kernel<<<grid_for(n, 256, dev.sms), 256>>>(g->row_ptr, cur[0], cur[2], g->w, V, n, (int32_t *)g->max_w);
+    nd_count_launches(1);
     ND_CUDA(cudaGetLastError());
     ND_CUDA(cudaMemcpy(&g->max_degree, bs->d_max_degree, sizeof(int32_t), cudaMemcpyDeviceToHost));
+    nd_objects_add(1);
+    *out = g;
+    g = nullptr;
     return ND_OK;
-  };
-  const int rc = build();
-  if (rc != ND_OK) { nd_block_free(dev.device, block, all); delete g; return rc; }
-  nd_objects_add(1);
-  *out = g;
-  return ND_OK;
+  }
+};
+
+int build_from_soa(const NdDeviceInfo &dev, int64_t n, int32_t V, BuildScratch *bs, int lo_bit, int hi_bit, nd_graph **out) {
+  ND_REQUIRE(n < ((int64_t)1 << 31), ND_ERR_RANGE, "%lld edges do not fit the int32 edge index of the CSR", (long long)n);
+  Build b(dev, n, V, bs);
+  ND_TRY(b.sort_by_ids());
+  ND_TRY(b.sort_weights(lo_bit, hi_bit));
+  ND_TRY(b.csr());
+  return b.finish(out);
 }
 
 }  // namespace
@@ -423,7 +481,7 @@ int nd_graph_finish(nd_graph *g, cudaStream_t st) {
     ND_CUDA(nd_malloc(&g->max_w, sizeof(float) * (size_t)(g->V > 0 ? g->V : 1)));
     ND_CUDA(cudaMemsetAsync(g->max_w, 0, sizeof(float) * (size_t)g->V, st));
     if (g->E > 0)
-      max_weight_kernel<<<grid_for(g->E, 256, dev.sms), 256, 0, st>>>(g->row_ptr, nullptr, g->w, g->V, g->E, (int32_t *)g->max_w);
+      max_weight_kernel<<<grid_for(g->E, 256, dev.sms), 256, 0, st>>>(g->row_ptr, nullptr, nullptr, g->w, g->V, g->E, (int32_t *)g->max_w);
   }
   NdDevMem<int32_t> m;
   ND_TRY(m.alloc(1));
@@ -485,15 +543,22 @@ int nd_graph_from_edge_records(int device, int64_t n, const void *records, nd_gr
   return from_edge_records_min_v(device, n, records, 0, out);
 }
 
-// the facts of the unpacked records decide the rest of the build; min_v: lower bound of the vertex count (the
-// adjacency-list format numbers vertices by line, including lines without edges)
+// the vertex count that the ids ask for; min_v: its lower bound (the adjacency-list format numbers vertices by line,
+// including lines without edges)
+static int vertices_of(const RecordFacts &f, int32_t min_v, int32_t *V) {
+  ND_REQUIRE(f.bad == 0 && f.max_id != 0x7fffffff, ND_ERR_RANGE, "edge records hold a negative or out-of-range vertex id");
+  *V = f.max_id + 1 > 0 ? f.max_id + 1 : 1;  // vertex count = max id + 1 (src/graph.hpp:131-142)
+  if (*V < min_v) *V = min_v;
+  return ND_OK;
+}
+
+// the facts of the unpacked records decide the rest of the build
 static int build_from_facts(const NdDeviceInfo &dev, int64_t n, int32_t min_v, BuildScratch *bs, nd_graph **out) {
   RecordFacts f;
+  int32_t V;
   ND_CUDA(cudaGetLastError());
   ND_CUDA(cudaMemcpy(&f, bs->facts, sizeof(f), cudaMemcpyDeviceToHost));
-  ND_REQUIRE(f.bad == 0 && f.max_id != 0x7fffffff, ND_ERR_RANGE, "edge records hold a negative or out-of-range vertex id");
-  int32_t V = f.max_id + 1 > 0 ? f.max_id + 1 : 1;  // vertex count = max id + 1 (src/graph.hpp:131-142)
-  if (V < min_v) V = min_v;
+  ND_TRY(vertices_of(f, min_v, &V));
   const uint32_t differ = f.key_and ^ f.key_or;
   int lo = 0, hi = nd_bit_length(differ);
   while (lo < hi && !((differ >> lo) & 1u)) lo++;
@@ -514,6 +579,11 @@ static int from_edge_records_min_v(int device, int64_t n, const void *records, i
   return build_from_facts(dev, n, min_v, &bs, out);
 }
 
+// From this many records on the ids are sorted, with their places as the third word, while the weights are on the wire
+// (8.4 M records 3.07 -> 2.63 ms, 4.2 M 1.76 -> 1.47, 2.1 M 1.03 -> 0.95; 1 M 0.64 -> 0.60 to 0.69, 260 K 0.35 -> 0.42: the
+// ids' facts are waited for in between).
+static constexpr int64_t WEIGHTS_LATER = (int64_t)1 << 21;
+
 int nd_graph_from_edges(int device, int64_t n, const int32_t *src, const int32_t *dst, const float *w, nd_graph **out) {
   ND_REQUIRE(out && ((src && dst && w) || n == 0) && n >= 0, ND_ERR_ARG, "nd_graph_from_edges: bad argument");
   ND_REQUIRE(n < ((int64_t)1 << 31), ND_ERR_RANGE, "%lld edges do not fit the int32 edge index of the CSR", (long long)n);
@@ -525,10 +595,34 @@ int nd_graph_from_edges(int device, int64_t n, const int32_t *src, const int32_t
   void *const to[3] = {bs.a[0], bs.a[1], bs.a[2]};
   const void *const from[3] = {src, dst, w};
   const size_t bytes[3] = {4 * (size_t)n, 4 * (size_t)n, 4 * (size_t)n};
-  ND_TRY(nd_copies_to_device(device, 3, to, from, bytes));
-  unpack_arrays_kernel<<<grid_for(n, 256, dev.sms), 256>>>(n, bs.a[0], bs.a[1], bs.a[2], bs.facts);
+  if (n < WEIGHTS_LATER) {
+    ND_TRY(nd_copies_to_device(device, 3, to, from, bytes));
+    unpack_arrays_kernel<<<grid_for(n, 256, dev.sms), 256>>>(n, bs.a[0], bs.a[1], bs.a[2], bs.facts);
+    nd_count_launches(1);
+    return build_from_facts(dev, n, 0, &bs, out);
+  }
+  // (the weights' arrival does not touch what the sorts work on: a block of its own)
+  BuildScratch weights;
+  weights.device = device;
+  weights.bytes = 4 * (size_t)n;
+  ND_TRY(nd_block_alloc(device, (void **)&weights.base, &weights.bytes));
+  ND_TRY(nd_copies_to_device(device, 2, to, from, bytes));
+  id_facts_kernel<<<grid_for(n, 256, dev.sms), 256>>>(n, bs.a[0], bs.a[1], bs.a[2], bs.facts);
   nd_count_launches(1);
-  return build_from_facts(dev, n, 0, &bs, out);
+  RecordFacts f;
+  int32_t V;
+  ND_CUDA(cudaGetLastError());
+  ND_CUDA(cudaMemcpy(&f, bs.facts, sizeof(f), cudaMemcpyDeviceToHost));
+  ND_TRY(vertices_of(f, 0, &V));
+  Build b(dev, n, V, &bs);
+  ND_TRY(b.sort_by_ids());
+  ND_TRY(b.csr());
+  ND_TRY(nd_copy_to_device(device, weights.base, w, bytes[2]));
+  place_weights_kernel<<<grid_for(n, 256, dev.sms), 256>>>(n, b.cur[2], (const float *)weights.base, b.oth[2], bs.facts);
+  std::swap(b.cur[2], b.oth[2]);
+  nd_count_launches(1);
+  ND_TRY(b.sort_weights(0, 32));
+  return b.finish(out);
 }
 
 int nd_graph_load_edge_list_binary(int device, const char *path, nd_graph **out) {

@@ -191,3 +191,29 @@ def test_results_own_their_memory(nd, small_graph):
     last = s.final_samples()
     del s, g
     assert np.array_equal(last.reshape(-1), exp)   # results outlive the sampler
+
+
+@pytest.mark.parametrize("n,V,weights,repeats", [((1 << 21) - 1, 50_000, "random", 0), (1 << 21, 50_000, "random", 3000), ((1 << 21) + 33, 1 << 20, "same", 0),
+                                                 ((1 << 21) + 33, 3000, "signs", 9000)])
+def test_loader_of_ids_before_weights(nd, n, V, weights, repeats):
+    """Sizes from which on the ids are sorted while the weights are on their way: the same CSR, whatever repeats."""
+    rng = np.random.default_rng(n + V)
+    src, dst = rng.integers(0, V, n).astype(np.int32), (V * rng.random(n) ** 4).astype(np.int32)
+    src[:repeats], dst[:repeats] = 7, 11
+    w = {"random": rng.random(n) * 4 + 1, "same": np.full(n, 2.5), "signs": rng.choice([-2.0, -1.0, 1.0, 2.0], n)}[weights].astype(np.float32)
+    at = rng.permutation(n)
+    src, dst, w = src[at], dst[at], w[at]
+    g = nd.Graph.from_edge_records(src, dst, w)
+    row_ptr, col, got_w, max_w = g.to_host()
+    order = np.lexsort((w, dst, src))
+    assert g.V == max(src.max(), dst.max()) + 1 and g.max_degree == np.bincount(src).max()
+    assert np.array_equal(col, dst[order]) and np.array_equal(got_w, w[order])
+    assert np.array_equal(np.diff(row_ptr), np.bincount(src, minlength=g.V))
+    exp_max = np.zeros(g.V, np.float32)
+    np.maximum.at(exp_max, src, w)
+    assert np.array_equal(max_w, exp_max)
+    dst[n // 2] = -3
+    with pytest.raises(nd.NdError):
+        nd.Graph.from_edge_records(src, dst, w)
+    dst[n // 2] = 3
+    assert nd.Graph.from_edge_records(src, dst, w).E == n
