@@ -69,7 +69,8 @@ __host__ __device__ constexpr bool weighted() { return APP == ND_APP_DEEPWALK ||
 
 // Layouts of the entries.  ALT: uniform walk: they carry the neighbour's row; weighted walks: id and weight in a word.
 // DENSE (uniform walk, node2vec): three ids of 21 bits in 8 bytes.
-enum : int { LAYOUT_PLAIN = 0, LAYOUT_ALT = 1, LAYOUT_DENSE = 2 };
+// FAR: weighted walks as ALT, node2vec as PLAIN, rows from the offsets.
+enum : int { LAYOUT_PLAIN = 0, LAYOUT_ALT = 1, LAYOUT_DENSE = 2, LAYOUT_FAR = 3 };
 
 // ---- loads.  The small per-vertex and per-entry arrays ask to stay in the L2; the (id, weight) records, an array far
 // larger than the L2, bypass the L1.
@@ -274,6 +275,18 @@ __global__ void __launch_bounds__(256) walk_start_kernel(const __grid_constant__
     if (e[j].z > 0) a.list[sh_base + at[j]] = e[j];
 }
 
+// Row start and degree of a vertex.  Two row offsets lie in one sector seven times out of eight and take half of the room
+// of a record of both, which is one load: FAR, from FAR_V vertices on, where the records do not fit the L2 beside what
+// else a walk reads (PPR on 2^24 vertices 2.47 -> 2.38 ms, node2vec on 2^22 15.4 -> 15.0, DeepWalk on 2^22 the same;
+// DeepWalk on 2^20 1.41 with the records, 1.52 with the offsets; uniform walk on 2^22 3.26 and 3.35: keeps the records).
+constexpr int32_t FAR_V = 1 << 22;
+template <int LAYOUT>
+__device__ __forceinline__ int2 row_of(const RowsArgs &a, const Hot &hot, int32_t v) {
+  if (LAYOUT != LAYOUT_FAR) return hot.ld(a.vrow + v);
+  const int32_t at = hot.ld(a.row_ptr + v), end = hot.ld(a.row_ptr + v + 1);
+  return make_int2(at, end - at);
+}
+
 // (row start, degree, max weight bits or vertex) of a vertex
 template <int APP, int LAYOUT>
 __device__ __forceinline__ int4 vertex_of(const RowsArgs &a, const Hot &hot, int32_t v) {
@@ -281,7 +294,7 @@ __device__ __forceinline__ int4 vertex_of(const RowsArgs &a, const Hot &hot, int
     const int2 r = hot.ld(a.vrec + v), n = hot.ld(a.vrec + v + 1);
     return make_int4(r.x, n.x - r.x, r.y, 0);
   }
-  const int2 r = hot.ld(a.vrow + v);
+  const int2 r = row_of<LAYOUT>(a, hot, v);
   return make_int4(r.x, r.y, v, 0);
 }
 
@@ -368,7 +381,7 @@ __device__ __forceinline__ void uniform_walks(const RowsArgs &a) {
       } else {
         v = id_of<LAYOUT>(a, rs + x);
         draw_block(a, s, step + 1, 0u, u);
-        if (step + 1 < a.steps) r = hot.ld(a.vrow + v);
+        if (step + 1 < a.steps) r = row_of<LAYOUT>(a, hot, v);
       }
       rows.put(a, s, step, v);
       rs = r.x;
@@ -446,7 +459,7 @@ __device__ __forceinline__ void weighted_walks(const RowsArgs &a) {
     const int32_t x = draw_index(dx, deg);
     const float u = ndrng::u32_to_uniform(dy);
     int32_t nbr = AGAIN;
-    if (LAYOUT == LAYOUT_ALT) {
+    if (LAYOUT != LAYOUT_PLAIN) {
       const uint32_t r = __ldg(a.pack + rs + x), b = r & 255u;
       bool accept = deg == 1 || u <= (float)b * 0.00390625f;
       if (!accept && (b == 255u || u < (float)(b + 1u) * 0.00390625f))
@@ -528,7 +541,7 @@ __device__ __forceinline__ void n2v_walks(const RowsArgs &a) {
   int32_t rs = 0, deg = 0, cur = 0, prev = 0, ts = 0, tn = 0;   // [ts, ts + tn): the row of the previous vertex
   int step = -1, round = 0;
   if (take.first() < take.n) {
-    const int4 e = walk_of<APP, LAYOUT_PLAIN>(a, hot, take.first());
+    const int4 e = walk_of<APP, LAYOUT>(a, hot, take.first());
     s = (uint32_t)e.x; rs = e.y; deg = e.z; cur = e.w; step = 0;
   }
   while (__any_sync(0xffffffffu, step >= 0)) {
@@ -594,12 +607,12 @@ __device__ __forceinline__ void n2v_walks(const RowsArgs &a) {
     const bool moved = nbr >= 0, over = over0 || (moved && step + 1 == a.steps);
     int4 next = make_int4(0, 0, 0, 0);   // the new vertex, or the next walk (w: there is one)
     uint32_t s_next = 0;
-    if (moved && !over) next = vertex_of<APP, LAYOUT_PLAIN>(a, hot, nbr);
+    if (moved && !over) next = vertex_of<APP, LAYOUT>(a, hot, nbr);
     const unsigned want = __ballot_sync(0xffffffffu, over);
     if (want) {
       const int64_t i = take.next(a, want);
       if (over && i < take.n) {
-        const int4 e = walk_of<APP, LAYOUT_PLAIN>(a, hot, i);
+        const int4 e = walk_of<APP, LAYOUT>(a, hot, i);
         next = make_int4(e.y, e.z, e.w, 1);
         s_next = (uint32_t)e.x;
       }
@@ -732,7 +745,8 @@ constexpr int64_t ERECS = (int64_t)1 << 21;
 constexpr int32_t PACK_V = 1 << 24;
 int layout_of(const nd_sampler *s) {
   const nd_graph *g = s->g;
-  if (s->p.app == ND_APP_DEEPWALK || s->p.app == ND_APP_PPR) return g->pack ? LAYOUT_ALT : LAYOUT_PLAIN;
+  if (s->p.app == ND_APP_DEEPWALK || s->p.app == ND_APP_PPR) return !g->pack ? LAYOUT_PLAIN : g->V >= FAR_V ? LAYOUT_FAR : LAYOUT_ALT;
+  if (s->p.app == ND_APP_NODE2VEC && g->V >= FAR_V) return LAYOUT_FAR;
   if (s->p.app == ND_APP_UNIFORM_WALK && g->E <= ERECS) return LAYOUT_ALT;
   return g->V <= DENSE_V && g->E >= DENSE_ENTRIES ? LAYOUT_DENSE : LAYOUT_PLAIN;
 }
@@ -758,6 +772,7 @@ void launch_as(nd_sampler *s, RowsArgs &a, bool count) {
   const int layout = layout_of(s);
   if (APP != ND_APP_NODE2VEC && layout == LAYOUT_ALT) return launch<APP, APP != ND_APP_NODE2VEC ? LAYOUT_ALT : LAYOUT_PLAIN>(s, a, count);
   if (!weighted<APP>() && layout == LAYOUT_DENSE) return launch<APP, !weighted<APP>() ? LAYOUT_DENSE : LAYOUT_PLAIN>(s, a, count);
+  if (APP != ND_APP_UNIFORM_WALK && layout == LAYOUT_FAR) return launch<APP, APP != ND_APP_UNIFORM_WALK ? LAYOUT_FAR : LAYOUT_PLAIN>(s, a, count);
   launch<APP, LAYOUT_PLAIN>(s, a, count);
 }
 
@@ -802,7 +817,7 @@ int ensure_vrow(const nd_graph *g, int sms) {
 int ensure_weighted(const nd_graph *g, int sms) {
   if (g->pack) return ND_OK;
   if (g->V > PACK_V || g->odd_max == 1) return ensure_colw(g, sms);
-  ND_TRY(ensure_vrow(g, sms));
+  if (g->V < FAR_V) ND_TRY(ensure_vrow(g, sms));
   NdDevMem<int> flag;
   int odd = 0;
   ND_TRY(flag.alloc(1));
@@ -881,7 +896,7 @@ int nd_walk_rows_alloc(nd_sampler *s) {
   ND_CUDA(cudaMemset(s->d_rows_acc, 0, 8 * acc));
   std::lock_guard<std::mutex> lock(g_derived_mutex);
   if (app == ND_APP_DEEPWALK || app == ND_APP_PPR) return ensure_weighted(g, sms);
-  ND_TRY(ensure_vrow(g, sms));
+  if (layout_of(s) != LAYOUT_FAR) ND_TRY(ensure_vrow(g, sms));
   if (app == ND_APP_UNIFORM_WALK && layout_of(s) == LAYOUT_ALT) ND_TRY(ensure_erec(g, sms));
   if (layout_of(s) == LAYOUT_DENSE) ND_TRY(ensure_col3(g, sms));
   if (app == ND_APP_NODE2VEC) ND_TRY(ensure_adjset(g, sms, s->d_status, s->h_status));
