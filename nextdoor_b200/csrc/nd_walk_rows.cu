@@ -39,7 +39,7 @@ struct RowsArgs {
   const float *__restrict__ w;
   const float *__restrict__ max_w;
   const int2 *__restrict__ vrow;     // [V] (row start, degree)
-  const int4 *__restrict__ erec;     // [E] (neighbour, its row start, its degree, 0)
+  const int4 *__restrict__ erec;     // [E] (neighbour, its row start, its degree, weight as 256ths of the row's maximum, rounded down)
   const int2 *__restrict__ colw;     // [E] (neighbour, weight bits)
   const int2 *__restrict__ vrec;     // [V+1] (row start, max weight bits)
   const uint32_t *__restrict__ pack; // [E] neighbour << 8 | weight as 256ths of the row's maximum, rounded down
@@ -67,10 +67,10 @@ struct RowsArgs {
 template <int APP>
 __host__ __device__ constexpr bool weighted() { return APP == ND_APP_DEEPWALK || APP == ND_APP_PPR; }
 
-// Layouts of the entries.  ALT: uniform walk: they carry the neighbour's row; weighted walks: id and weight in a word.
-// DENSE (uniform walk, node2vec): three ids of 21 bits in 8 bytes.
-// FAR: weighted walks as ALT, node2vec as PLAIN, rows from the offsets.
-enum : int { LAYOUT_PLAIN = 0, LAYOUT_ALT = 1, LAYOUT_DENSE = 2, LAYOUT_FAR = 3 };
+// Layouts of the entries.  ALT (weighted walks): id and weight in a word.  FAT (uniform, weighted walks): they carry the
+// neighbour's row, and the weight.  DENSE (uniform walk, node2vec): three ids of 21 bits in 8 bytes.  FAR: weighted walks as
+// ALT, node2vec as PLAIN, rows from the offsets.
+enum : int { LAYOUT_PLAIN = 0, LAYOUT_ALT = 1, LAYOUT_DENSE = 2, LAYOUT_FAR = 3, LAYOUT_FAT = 4 };
 
 // ---- loads.  The small per-vertex and per-entry arrays ask to stay in the L2; the (id, weight) records, an array far
 // larger than the L2, bypass the L1.
@@ -354,7 +354,7 @@ struct Taker {
 // the gather is in flight, so that a step is its dependent reads and little else.  Equal rounds, as in Taker.
 template <int LAYOUT>
 __device__ __forceinline__ void uniform_walks(const RowsArgs &a) {
-  constexpr bool FAT = LAYOUT == LAYOUT_ALT;
+  constexpr bool FAT = LAYOUT == LAYOUT_FAT;
   constexpr int PIECE = piece<ND_APP_UNIFORM_WALK>();
   __shared__ unsigned int sums[2];
   Rows<PIECE> rows(a, sums);
@@ -459,12 +459,20 @@ __device__ __forceinline__ void weighted_walks(const RowsArgs &a) {
     const int32_t x = draw_index(dx, deg);
     const float u = ndrng::u32_to_uniform(dy);
     int32_t nbr = AGAIN;
+    int2 row = make_int2(0, 0);   // FAT: the neighbour's
     if (LAYOUT != LAYOUT_PLAIN) {
-      const uint32_t r = __ldg(a.pack + rs + x), b = r & 255u;
+      uint32_t id, b;
+      if (LAYOUT == LAYOUT_FAT) {
+        const int4 r = hot.ld(a.erec + rs + x);
+        id = (uint32_t)r.x; b = (uint32_t)r.w; row = make_int2(r.y, r.z);
+      } else {
+        const uint32_t r = __ldg(a.pack + rs + x);
+        id = r >> 8; b = r & 255u;
+      }
       bool accept = deg == 1 || u <= (float)b * 0.00390625f;
       if (!accept && (b == 255u || u < (float)(b + 1u) * 0.00390625f))
         accept = !(__fmul_rn(u, __ldg(a.max_w + mw)) > __ldg(a.w + rs + x));
-      if (accept) nbr = (int32_t)(r >> 8);
+      if (accept) nbr = (int32_t)id;
     } else {
       const int2 r = ld_once(a.colw + rs + x);
       if (deg == 1 || !(__fmul_rn(u, __int_as_float(mw)) > __int_as_float(r.y))) nbr = r.x;
@@ -473,12 +481,13 @@ __device__ __forceinline__ void weighted_walks(const RowsArgs &a) {
     if (nbr == AGAIN && ++t > RETRY_CAP) {
       atomicOr(a.status, ND_DEV_RETRY_LIMIT);
       nbr = __ldg(a.col + rs);
+      if (LAYOUT == LAYOUT_FAT) row = row_of<LAYOUT>(a, hot, nbr);
     }
     if (nbr >= 0) {
       rows.put(a, s, step, nbr);
       step++;
       t = 0;
-      cur = nbr;
+      if (LAYOUT == LAYOUT_FAT) { rs = row.x; deg = row.y; mw = nbr; } else { cur = nbr; }
     }
   }
   rows.out(a, tries, 2, 0u);
@@ -663,13 +672,6 @@ __global__ void vrec_build_kernel(const int32_t *__restrict__ row_ptr, const flo
     vrec[v] = make_int2(row_ptr[v], v < V ? __float_as_int(max_w[v]) : 0);
 }
 
-__global__ void erec_build_kernel(const int32_t *__restrict__ col, const int32_t *__restrict__ row_ptr, int64_t E, int4 *__restrict__ erec) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E; e += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t v = col[e], rs = row_ptr[v];
-    erec[e] = make_int4(v, rs, row_ptr[v + 1] - rs, 0);
-  }
-}
-
 // A row whose maximum is negative, not a number or so small that its 256th is not exact: the comparisons that the packed
 // weights replace do not follow from one another there.
 __global__ void odd_max_kernel(const int32_t *__restrict__ row_ptr, const float *__restrict__ max_w, int32_t V, int *__restrict__ odd) {
@@ -677,19 +679,31 @@ __global__ void odd_max_kernel(const int32_t *__restrict__ row_ptr, const float 
     if (row_ptr[v + 1] - row_ptr[v] > 1 && !(max_w[v] == 0.f || max_w[v] >= 7.8886090522101181e-31f)) *odd = 1;   // 2^-100
 }
 
+// a weight as 256ths of its row's maximum, rounded down
+__device__ __forceinline__ uint32_t weight_code(float w, float max_w) {
+  const float unit = __fmul_rn(max_w, 0.00390625f);
+  int b = 255;   // a weight that is not a number accepts every draw: decided by comparing with it
+  if (w == w) {
+    const float r = __fdiv_rn(w, unit);
+    b = r > 0.f ? (r < 255.f ? (int)r : 255) : 0;
+    while (b > 0 && !(__fmul_rn((float)b, unit) <= w)) b--;
+    while (b < 255 && __fmul_rn((float)(b + 1), unit) <= w) b++;
+  }
+  return (uint32_t)b;
+}
+
 __global__ void __launch_bounds__(BUILD_THREADS)
 pack_build_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col, const float *__restrict__ max_w, const float *__restrict__ w,
                   int32_t V, int64_t E, uint32_t *__restrict__ pack) {
+  for_entries(row_ptr, V, E, [&](int64_t e, int32_t v) { pack[e] = (uint32_t)col[e] << 8 | weight_code(w[e], max_w[v]); });
+}
+
+__global__ void __launch_bounds__(BUILD_THREADS)
+erec_build_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col, const float *__restrict__ max_w, const float *__restrict__ w,
+                  int32_t V, int64_t E, int4 *__restrict__ erec) {
   for_entries(row_ptr, V, E, [&](int64_t e, int32_t v) {
-    const float x = w[e], unit = __fmul_rn(max_w[v], 0.00390625f);
-    int b = 255;   // a weight that is not a number accepts every draw: decided by comparing with it
-    if (x == x) {
-      const float r = __fdiv_rn(x, unit);
-      b = r > 0.f ? (r < 255.f ? (int)r : 255) : 0;
-      while (b > 0 && !(__fmul_rn((float)b, unit) <= x)) b--;
-      while (b < 255 && __fmul_rn((float)(b + 1), unit) <= x) b++;
-    }
-    pack[e] = (uint32_t)col[e] << 8 | (uint32_t)b;
+    const int32_t to = col[e], rs = row_ptr[to];
+    erec[e] = make_int4(to, rs, row_ptr[to + 1] - rs, (int)weight_code(w[e], max_w[v]));
   });
 }
 
@@ -738,16 +752,19 @@ adjset_build_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restri
   });
 }
 
-// Entries that carry the neighbour's row (16 bytes each) shorten a step to one dependent read; they pay while
-// the array stays in a die's half of the L2 with room to spare: 32 MB.
-constexpr int64_t ERECS = (int64_t)1 << 21;
+// Entries that carry the neighbour's row (16 bytes each) shorten a step by a dependent read; they pay while the array, here
+// 64 MB, stays in the L2 (130 K vertices, 2.8 M entries, without and with: uniform walk 95 -> 83 us, PPR 115 -> 106, DeepWalk
+// 203 -> 198; 60 K, 1.2 M: PPR 117 -> 104; 200 K, 4.8 M: 131 -> 120, 142 -> 132, 293 -> 291; 300 K, 7.2 M: uniform walk
+// 171 -> 197, DeepWalk 329 -> 350).  node2vec fetches two candidates a round and waits for the filter anyway: 298 -> 326.
+constexpr int64_t ERECS = (int64_t)1 << 22;
 // Ids that leave a byte of a word to the weight.
 constexpr int32_t PACK_V = 1 << 24;
 int layout_of(const nd_sampler *s) {
   const nd_graph *g = s->g;
-  if (s->p.app == ND_APP_DEEPWALK || s->p.app == ND_APP_PPR) return !g->pack ? LAYOUT_PLAIN : g->V >= FAR_V ? LAYOUT_FAR : LAYOUT_ALT;
+  const bool weighted = s->p.app == ND_APP_DEEPWALK || s->p.app == ND_APP_PPR;
+  if (s->p.app != ND_APP_NODE2VEC && g->erec && (!weighted || g->odd_max == 0)) return LAYOUT_FAT;
+  if (weighted) return !g->pack ? LAYOUT_PLAIN : g->V >= FAR_V ? LAYOUT_FAR : LAYOUT_ALT;
   if (s->p.app == ND_APP_NODE2VEC && g->V >= FAR_V) return LAYOUT_FAR;
-  if (s->p.app == ND_APP_UNIFORM_WALK && g->E <= ERECS) return LAYOUT_ALT;
   return g->V <= DENSE_V && g->E >= DENSE_ENTRIES ? LAYOUT_DENSE : LAYOUT_PLAIN;
 }
 
@@ -769,11 +786,14 @@ void launch(nd_sampler *s, RowsArgs &a, bool count) {
 
 template <int APP>
 void launch_as(nd_sampler *s, RowsArgs &a, bool count) {
-  const int layout = layout_of(s);
-  if (APP != ND_APP_NODE2VEC && layout == LAYOUT_ALT) return launch<APP, APP != ND_APP_NODE2VEC ? LAYOUT_ALT : LAYOUT_PLAIN>(s, a, count);
-  if (!weighted<APP>() && layout == LAYOUT_DENSE) return launch<APP, !weighted<APP>() ? LAYOUT_DENSE : LAYOUT_PLAIN>(s, a, count);
-  if (APP != ND_APP_UNIFORM_WALK && layout == LAYOUT_FAR) return launch<APP, APP != ND_APP_UNIFORM_WALK ? LAYOUT_FAR : LAYOUT_PLAIN>(s, a, count);
-  launch<APP, LAYOUT_PLAIN>(s, a, count);
+  constexpr bool w = weighted<APP>(), n2v = APP == ND_APP_NODE2VEC;
+  switch (layout_of(s)) {   // (the others are not layouts of the app)
+    case LAYOUT_FAT: return launch<APP, n2v ? LAYOUT_PLAIN : LAYOUT_FAT>(s, a, count);
+    case LAYOUT_ALT: return launch<APP, w ? LAYOUT_ALT : LAYOUT_PLAIN>(s, a, count);
+    case LAYOUT_DENSE: return launch<APP, w ? LAYOUT_PLAIN : LAYOUT_DENSE>(s, a, count);
+    case LAYOUT_FAR: return launch<APP, w || n2v ? LAYOUT_FAR : LAYOUT_PLAIN>(s, a, count);
+    default: return launch<APP, LAYOUT_PLAIN>(s, a, count);
+  }
 }
 
 // The derived layouts of a graph are built by the first sampler that needs them; samplers of one
@@ -813,19 +833,32 @@ int ensure_vrow(const nd_graph *g, int sms) {
   return ND_OK;
 }
 
-// ids and weights in one word, or the records of ensure_colw where they do not fit one
+int ensure_erec(const nd_graph *g, int sms) {
+  if (g->erec) return ND_OK;
+  NdDevMem<int4> erec;
+  ND_TRY(erec.alloc((size_t)(g->E > 0 ? g->E : 1)));
+  erec_build_kernel<<<sms * 16, BUILD_THREADS>>>(g->row_ptr, g->col, g->max_w, g->w, g->V, g->E, erec.p);
+  ND_CUDA(cudaGetLastError());
+  g->erec = erec.release();
+  return ND_OK;
+}
+
+// entries with rows, ids and weights in one word, or the records of ensure_colw where neither holds the weights
 int ensure_weighted(const nd_graph *g, int sms) {
+  if (g->odd_max < 0) {
+    NdDevMem<int> flag;
+    int odd = 0;
+    ND_TRY(flag.alloc(1));
+    ND_CUDA(cudaMemset(flag.p, 0, sizeof(int)));
+    odd_max_kernel<<<sms * 16, 256>>>(g->row_ptr, g->max_w, g->V, flag.p);
+    ND_CUDA(cudaMemcpy(&odd, flag.p, sizeof(int), cudaMemcpyDeviceToHost));
+    g->odd_max = odd;
+  }
+  const bool fat = g->E <= ERECS;
+  if (g->odd_max == 1 || (!fat && g->V > PACK_V)) return ensure_colw(g, sms);
+  if (fat || g->V < FAR_V) ND_TRY(ensure_vrow(g, sms));
+  if (fat) return ensure_erec(g, sms);
   if (g->pack) return ND_OK;
-  if (g->V > PACK_V || g->odd_max == 1) return ensure_colw(g, sms);
-  if (g->V < FAR_V) ND_TRY(ensure_vrow(g, sms));
-  NdDevMem<int> flag;
-  int odd = 0;
-  ND_TRY(flag.alloc(1));
-  ND_CUDA(cudaMemset(flag.p, 0, sizeof(int)));
-  odd_max_kernel<<<sms * 16, 256>>>(g->row_ptr, g->max_w, g->V, flag.p);
-  ND_CUDA(cudaMemcpy(&odd, flag.p, sizeof(int), cudaMemcpyDeviceToHost));
-  g->odd_max = odd;
-  if (odd) return ensure_colw(g, sms);
   NdDevMem<uint32_t> pack;
   ND_TRY(pack.alloc((size_t)(g->E > 0 ? g->E : 1)));
   pack_build_kernel<<<sms * 16, BUILD_THREADS>>>(g->row_ptr, g->col, g->max_w, g->w, g->V, g->E, pack.p);
@@ -841,16 +874,6 @@ int ensure_col3(const nd_graph *g, int sms) {
   col3_build_kernel<<<sms * 16, 256>>>(g->col, g->E, col3.p);
   ND_CUDA(cudaGetLastError());
   g->col3 = col3.release();
-  return ND_OK;
-}
-
-int ensure_erec(const nd_graph *g, int sms) {
-  if (g->erec) return ND_OK;
-  NdDevMem<int4> erec;
-  ND_TRY(erec.alloc((size_t)(g->E > 0 ? g->E : 1)));
-  erec_build_kernel<<<sms * 16, 256>>>(g->col, g->row_ptr, g->E, erec.p);
-  ND_CUDA(cudaGetLastError());
-  g->erec = erec.release();
   return ND_OK;
 }
 
@@ -896,8 +919,8 @@ int nd_walk_rows_alloc(nd_sampler *s) {
   ND_CUDA(cudaMemset(s->d_rows_acc, 0, 8 * acc));
   std::lock_guard<std::mutex> lock(g_derived_mutex);
   if (app == ND_APP_DEEPWALK || app == ND_APP_PPR) return ensure_weighted(g, sms);
+  if (app == ND_APP_UNIFORM_WALK && g->E <= ERECS) ND_TRY(ensure_erec(g, sms));
   if (layout_of(s) != LAYOUT_FAR) ND_TRY(ensure_vrow(g, sms));
-  if (app == ND_APP_UNIFORM_WALK && layout_of(s) == LAYOUT_ALT) ND_TRY(ensure_erec(g, sms));
   if (layout_of(s) == LAYOUT_DENSE) ND_TRY(ensure_col3(g, sms));
   if (app == ND_APP_NODE2VEC) ND_TRY(ensure_adjset(g, sms, s->d_status, s->h_status));
   return ND_OK;

@@ -131,3 +131,18 @@ def test_ids_of_21_bits(nd, app, V, M):
     for mode in (1, 2):
         s.sample(mode)
         assert np.array_equal(s.final_samples(), exp), mode
+
+
+@pytest.mark.parametrize("app", [0, 1, 2, 3])
+@pytest.mark.parametrize("V,M", [(60_000, (1 << 21) - 3), (60_000, 1 << 21), (60_000, (1 << 21) + 1), ((1 << 22) - 1, 1 << 21), (1 << 22, (1 << 21) + 1)])
+def test_entries_with_and_without_rows(nd, app, V, M):
+    """Around 2^22 entries and 2^22 vertices, against the exact-sort mode, which reads the plain arrays."""
+    g = nd.Graph.rmat(V, M, seed=3)
+    init = np.random.default_rng(M).integers(0, V, 20000).astype(np.int32)
+    s = nd.Sampler(g, nd.app_params(app, steps=15, seed=5, stop_prob=0.05), num_samples=len(init), initial=init)
+    s.sample(0)
+    exp = s.final_samples().copy()
+    tries = s.stats()["weight_tries"]
+    for mode in (1, 2):
+        s.sample(mode)
+        assert np.array_equal(s.final_samples(), exp) and s.stats()["weight_tries"] == tries, mode
