@@ -7,9 +7,9 @@
 // integer weights sum exactly).
 //
 // What bounds it, and what is done about it (2^20 vertices, 1024 batches of 64, 2 layers of 64: FastGCN
-// 4.8 -> 0.89 ms, LADIES 5.7 -> 1.07 ms).  One CTA fills an SM, and neither memory nor issue slots are full: FastGCN issued
-// in 58 % of the cycles at 0.98 ms (5.6 GB out of the L2 at 24 % of its rate), LADIES in 57 % (610 M
-// instructions for 131 M list entries, the distinct ones of 313 M), its shared memory is busy in half of them; the warps
+// 4.8 -> 0.89 ms, LADIES 5.7 -> 0.80 ms).  One CTA fills an SM, and neither memory nor issue slots are full: FastGCN issued
+// in 58 % of the cycles at 0.98 ms (5.6 GB out of the L2 at 24 % of its rate), LADIES in 57 % at 1.07 (610 M
+// instructions for 131 M list entries, the distinct ones of 313 M), its shared memory busy in half of them; the warps
 // wait for barriers between the phases, for shared memory and for loads:
 //  * The second layer's transits are hubs (FastGCN draws them with the square of their degree), many of them the
 //    same one: repeated transits of a batch are taken once (LADIES with their multiplicity).
@@ -27,13 +27,17 @@
 //    the weights and a division per entry and sample.  One pass over the lists sets the union's bits and adds the terms
 //    up per group; then the groups that the draws fall into get an accumulator per vertex, where the union was,
 //    and a second pass adds up the terms of their candidates alone (131 K entries, 37 of 8192 groups, 9 % of the entries).
-//    No order of the lists is asked for.  (Until then the candidates' weights were added up by rank, in tiles of shared
-//    memory: the rank of every entry, a double added per entry, a few barriers per tile; 1024 batches on 2^20 vertices 2.50
-//    -> 1.07 ms, 256 on 2^21 1.37 -> 0.64, 700 batches of 100 and 3 layers of 100 on 100 K 1.52 -> 0.88.)  A thread
-//    takes eight entries, 32 bytes of ids and of terms; what neighbouring entries add to one group is added up in
-//    registers and across the lanes first, as a 64-bit add in shared memory costs 18 cycles a warp.  Groups of 128: with
-//    larger ones the second pass adds more, with smaller ones the first (64: 1.08, 256: 1.05 ms, but 0.29 instead of 0.25
-//    with 300 batches on 500 K).
+//    (Until then the candidates' weights were added up by rank, in tiles of shared memory: the rank of every entry, a
+//    double added per entry, a few barriers per tile; 1024 batches on 2^20 vertices 2.50 -> 1.07 ms, 256 on 2^21 1.37 ->
+//    0.64, 700 batches of 100 and 3 layers of 100 on 100 K 1.52 -> 0.88.)  A thread takes eight entries, 32 bytes of ids and
+//    of terms; what neighbouring entries add to one group is added up in registers and across the lanes first, as a 64-bit
+//    add in shared memory costs 18 cycles a warp.  Groups of 128: with larger ones the second pass adds more, with smaller
+//    ones the first (64: 1.08, 256: 1.05 ms, but 0.29 instead of 0.25 with 300 batches on 500 K).
+//  * Hubs hold two thirds of the entries of a second layer (2.7 of 27 lists).  Both passes leave them out: their sums per
+//    group are a table per graph, 64 KB a hub, and a group's candidates are a range of the hub's neighbours, each kept
+//    once with the sum of its terms (graphs repeat edges between hubs hundreds of times: the plain range, with all its adds
+//    to one candidate, took longer than the pass it replaced).  1.07 -> 0.80, 0.64 -> 0.51, 0.88 -> 0.72, 0.25 -> 0.19 ms.
+//    Where the tables would be larger than HUB_TABLES, or a hub's list does not ascend, hubs are lists like the others.
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
@@ -50,7 +54,7 @@ constexpr int GROUP = 512;        // FastGCN: vertices (GROUP_WORDS words) whose
 constexpr int LADIES_GROUP_BITS = 7;   // LADIES: 2^7 vertices, more where the sums of the groups would not fit shared memory
 constexpr int BIG_DEGREE = 2048;  // from here a vertex is on the list of big ones and its code is 0: 512 * 2047^2 < 2^31
 constexpr int FLIGHT = 3;         // groups a warp sums at a time
-constexpr int HUB = 128, LADIES_HUB = 64;   // a vertex with at least V / HUB neighbours has a bitmap of them, and is ORed from V / LADIES_HUB on
+constexpr int HUB = 128;          // a vertex with at least V / HUB neighbours has a bitmap of them
 constexpr int BIG_LIST = 4096;    // lists at least this long are streamed by the whole CTA
 constexpr int VEC = 4;            // 16-byte loads in flight per thread
 constexpr int OCT = 8;            // list entries a thread takes at a time: 32 aligned bytes (LADIES)
@@ -88,6 +92,10 @@ struct Args {
   const float *__restrict__ term;          // LADIES: (w / rowsum)^2 per entry
   const int32_t *__restrict__ hub_slot;    // [V] slot of the vertex's bitmap, -1: none
   const uint32_t *__restrict__ hub_bits;   // [slots][words]
+  const double *__restrict__ hub_sums;     // LADIES: [slots][groups] the terms of a hub's list per group, or null
+  const int32_t *__restrict__ hub_starts;  // ... [slots][groups + 1] where each group of it begins in
+  const int32_t *__restrict__ hub_ids;     // ... the hubs' neighbours, each once
+  const double *__restrict__ hub_terms;    // ... and the sums of their terms
   unsigned long long *acc;                 // counters of the running job: [0] draws, [5] ids, [6] candidates, [8] next sample, [10] CTAs done; zero between jobs
   unsigned long long *stats;               // published by the last CTA
   unsigned long long pairs;
@@ -199,8 +207,8 @@ __device__ __forceinline__ uint32_t oct_mask(int64_t e, const Transit &t) {
   return (hi >= OCT ? 0xffu : (1u << (int)hi) - 1u) & (lo <= 0 ? 0xffu : 0xffu << (int)lo);
 }
 
-// LADIES: the terms of the lists' entries into the sums of their groups, the entries of lists without a bitmap into the
-// union.  A lane takes an oct and adds up what follows in one group; what the last entries of a lane's and the first of the
+// LADIES: the terms of the entries of lists without tables into the sums of their groups, and the entries into the
+// union (hubs have no octs).  A lane takes an oct and adds up what follows in one group; what the last entries of a lane's and the first of the
 // next one's share is passed on, so that neighbouring entries of a long list cost one atomic and the lanes' atomics do not
 // meet.
 __device__ __forceinline__ void add_terms(const NdGraphView &g, const float *__restrict__ term, const Transit *ut, int ntr, int nh, int nu,
@@ -222,7 +230,7 @@ __device__ __forceinline__ void add_terms(const NdGraphView &g, const float *__r
       load8(reinterpret_cast<const int32_t *>(term) + e, x);
       const uint32_t in = oct_mask(e, t);
       mult = (double)t.mult;
-      if (i >= nh) {
+      {
         uint32_t word[OCT];
 #pragma unroll
         for (int j = 0; j < OCT; j++) word[j] = (in >> j) & 1u ? bm[(uint32_t)v[j] >> 5] : ~0u;
@@ -395,8 +403,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
         const int32_t rs = __ldg(a.g.row_ptr + t), deg = __ldg(a.g.row_ptr + t + 1) - rs, slot = __ldg(a.hub_slot + t);
         ids += (unsigned long long)deg;
         if (sh_mult[i] > 0) {
-          // (LADIES goes through the lists for their terms, so that a hub's bitmap saves it less)
-          ut[slot >= 0 && (!LADIES || deg >= cp.V / LADIES_HUB) ? atomicAdd(&sh_hubs, 1) : cp.ntr - 1 - atomicAdd(&sh_rest, 1)] = Transit{rs, deg, sh_mult[i], slot};
+          ut[slot >= 0 && (!LADIES || a.hub_sums) ? atomicAdd(&sh_hubs, 1) : cp.ntr - 1 - atomicAdd(&sh_rest, 1)] = Transit{rs, deg, sh_mult[i], slot};
         }
       }
       for (int o = 16; o > 0; o >>= 1) ids += __shfl_xor_sync(0xffffffffu, ids, o);
@@ -468,10 +475,15 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
         }
       } else {
         // ---- the groups' weights and the rest of the union, then the number of candidates
-        for (int k = tid; k < groups; k += blockDim.x) gcdf[k] = 0.0;
+        for (int k = tid; k < groups; k += blockDim.x) {
+          double sum = 0.0;
+#pragma unroll 4
+          for (int i = 0; i < nh; i++) sum += __ldg(a.hub_sums + (size_t)ut[i].slot * groups + k) * (double)ut[i].mult;
+          gcdf[k] = sum;
+        }
         for (int i = tid; i < nu; i += blockDim.x) {
           const Transit &t = ut[i < nh ? i : cp.ntr - nu + i];
-          pre[i] = octs_of(t.rs, t.deg);
+          pre[i] = i < nh ? 0u : octs_of(t.rs, t.deg);
         }
         __syncthreads();
         octs = scan_u32(pre, nu, red_u);
@@ -544,10 +556,21 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
             __syncthreads();
             for (int j = tid; j < cp.L; j += blockDim.x) {
               const int k = sh_first[j] == j ? slot_of(j) - s0 : -1;
-              if (k >= 0 && k < here) slot[sh_group[j]] = (uint8_t)k;
+              if (k >= 0 && k < here) {
+                slot[sh_group[j]] = (uint8_t)k;
+                sh_mult[k] = sh_group[j];   // (not needed any more: the groups of the slots)
+              }
             }
             __syncthreads();
             add_candidates(a.g, a.term, ut, cp.ntr, nh, nu, pre, octs, slot, acc, lay.group_bits);
+            for (int q = warp; q < here * nh; q += warps) {   // hubs: a warp goes to a group of one
+              const int k = q / nh;
+              const Transit t = ut[q - k * nh];
+              const int32_t *at = a.hub_starts + (size_t)t.slot * (groups + 1) + sh_mult[k];
+              const int32_t end = __ldg(at + 1);
+              for (int32_t e = __ldg(at) + lane; e < end; e += 32)
+                atomicAdd(acc + ((size_t)k << lay.group_bits) + (__ldg(a.hub_ids + e) & (n - 1)), __ldg(a.hub_terms + e) * (double)t.mult);
+            }
             __syncthreads();
             for (int j = warp; j < cp.L; j += warps) {
               const int k = slot_of(j) - s0, group = sh_group[j];
@@ -741,6 +764,57 @@ __global__ void hub_slots_kernel(const int32_t *__restrict__ row_ptr, int32_t V,
   }
 }
 
+// LADIES: a hub's neighbours, each once, and the sums of their terms, a CTA per hub (graphs repeat edges between hubs hundreds
+// of times); hub i's go to ids[offs[i]] and on, their number to count[i].  *odd: a list does not ascend.
+__global__ void __launch_bounds__(256) hub_unique_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col, const float *__restrict__ term,
+                                                         const int32_t *__restrict__ hubs, const int32_t *__restrict__ offs, int32_t *__restrict__ ids,
+                                                         double *__restrict__ terms, int32_t *__restrict__ count, int *__restrict__ odd) {
+  __shared__ int32_t heads_of[8];
+  const int32_t v = hubs[blockIdx.x], rs = row_ptr[v], end = row_ptr[v + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int32_t at = offs[blockIdx.x];
+  for (int32_t e0 = rs; e0 < end; e0 += 256) {
+    const int32_t e = e0 + (int32_t)threadIdx.x;
+    const int32_t c = e < end ? col[e] : 0, before = e < end && e > rs ? col[e - 1] : -1;
+    if (e < end && before > c) *odd = 1;
+    const bool head = e < end && c != before;
+    const uint32_t heads = __ballot_sync(0xffffffffu, head);
+    __syncthreads();
+    if (lane == 0) heads_of[warp] = __popc(heads);
+    __syncthreads();
+    int32_t to = at + __popc(heads & ((1u << lane) - 1u));
+    for (int w = 0; w < 8; w++) {
+      if (w < warp) to += heads_of[w];
+      at += heads_of[w];
+    }
+    if (head) {
+      double sum = 0.0;
+      for (int32_t x = e; x < end && col[x] == c; x++) sum += (double)term[x];
+      ids[to] = c;
+      terms[to] = sum;
+    }
+  }
+  if (threadIdx.x == 0) count[blockIdx.x] = at - offs[blockIdx.x];
+}
+
+// ... and its groups: where each begins there, and its sum
+__global__ void __launch_bounds__(256) hub_table_kernel(const int32_t *__restrict__ ids, const double *__restrict__ terms, const int32_t *__restrict__ offs,
+                                                        const int32_t *__restrict__ count, int groups, int group_bits, double *__restrict__ sums,
+                                                        int32_t *__restrict__ starts) {
+  const int32_t first = offs[blockIdx.x], end = first + count[blockIdx.x];
+  for (int k = threadIdx.x; k <= groups; k += blockDim.x) {
+    int32_t lo = first, hi = end;   // first neighbour of group k or a later one
+    while (lo < hi) {
+      const int32_t mid = lo + ((hi - lo) >> 1);
+      if ((int64_t)ids[mid] < (int64_t)k << group_bits) lo = mid + 1; else hi = mid;
+    }
+    starts[(size_t)blockIdx.x * (groups + 1) + k] = lo;
+    double sum = 0.0;
+    for (; k < groups && lo < end && ids[lo] >> group_bits == k; lo++) sum += terms[lo];
+    if (k < groups) sums[(size_t)blockIdx.x * groups + k] = sum;
+  }
+}
+
 // a CTA row per hub, `gridDim.y` CTAs share its list
 __global__ void hub_bits_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col, const int32_t *__restrict__ hubs, int words,
                                 uint32_t *__restrict__ bits) {
@@ -795,6 +869,8 @@ int ensure_hubs(const nd_graph *g, int grid) {
   ND_CUDA(cudaMemset(bits.p, 0, sizeof(uint32_t) * words));
   if (n > 0) hub_bits_kernel<<<dim3((unsigned)n, 8), 256>>>(g->row_ptr, g->col, hubs.p, words_of(g->V), bits.p);
   ND_CUDA(cudaDeviceSynchronize());
+  g->n_hubs = n;
+  g->hubs = hubs.release();
   g->hub_bits = bits.release();
   g->hub_slot = slot.release();
   return ND_OK;
@@ -840,13 +916,62 @@ int ensure_terms(const nd_graph *g, int grid) {
   return ND_OK;
 }
 
+// LADIES: the hubs' neighbours and groups of 2^bits vertices, unless they would take more than HUB_TABLES bytes or a list
+// does not ascend
+constexpr size_t HUB_TABLES = (size_t)256 << 20;
+int ensure_hub_tables(const nd_graph *g, const Layout &lay) {
+  NdHubTable &t = g->hub_tables[lay.group_bits - LADIES_GROUP_BITS];
+  const size_t n = (size_t)g->n_hubs, groups = (size_t)lay.groups;
+  if (t.sums || n == 0 || g->hub_lists == 0 || n * (12 * groups + 4) > HUB_TABLES) return ND_OK;
+  if (g->hub_lists < 0) {
+    std::vector<int32_t> hubs(n), offs(n + 1);
+    ND_CUDA(cudaMemcpy(hubs.data(), g->hubs, sizeof(int32_t) * n, cudaMemcpyDeviceToHost));
+    int64_t all = 0;
+    for (size_t i = 0; i < n; i++) {
+      int32_t row[2];
+      ND_CUDA(cudaMemcpy(row, g->row_ptr + hubs[i], sizeof(row), cudaMemcpyDeviceToHost));
+      offs[i] = (int32_t)all;
+      all += row[1] - row[0];
+    }
+    if (12 * (size_t)all > HUB_TABLES) { g->hub_lists = 0; return ND_OK; }
+    NdDevMem<int32_t> ids, d_offs;
+    NdDevMem<double> terms;
+    NdDevMem<int> flag;
+    int odd = 0;
+    ND_TRY(ids.alloc((size_t)all));
+    ND_TRY(terms.alloc((size_t)all));
+    ND_TRY(d_offs.alloc(2 * n));
+    ND_TRY(flag.alloc(1));
+    ND_CUDA(cudaMemset(flag.p, 0, sizeof(int)));
+    ND_CUDA(cudaMemcpy(d_offs.p, offs.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice));
+    hub_unique_kernel<<<(unsigned)n, 256>>>(g->row_ptr, g->col, g->term, g->hubs, d_offs.p, ids.p, terms.p, d_offs.p + n, flag.p);
+    ND_CUDA(cudaMemcpy(&odd, flag.p, sizeof(int), cudaMemcpyDeviceToHost));
+    g->hub_lists = odd ? 0 : 1;
+    if (odd) return ND_OK;
+    g->hub_ids = ids.release();
+    g->hub_terms = terms.release();
+    g->hub_offs = d_offs.release();
+  }
+  NdDevMem<double> sums;
+  NdDevMem<int32_t> starts;
+  ND_TRY(sums.alloc(n * groups));
+  ND_TRY(starts.alloc(n * (groups + 1)));
+  hub_table_kernel<<<(unsigned)n, 256>>>(g->hub_ids, g->hub_terms, g->hub_offs, g->hub_offs + n, lay.groups, lay.group_bits, sums.p, starts.p);
+  ND_CUDA(cudaDeviceSynchronize());
+  t.starts = starts.release();
+  t.sums = sums.release();
+  return ND_OK;
+}
+
 // What a graph's first sampler builds goes to the graph when all of it is there: a build that runs out of memory
 // leaves nothing behind.
-int ensure_layers(const nd_graph *g, int sms, bool ladies) {
+int ensure_layers(const nd_graph *g, int sms, bool ladies, const Layout &lay) {
   std::lock_guard<std::mutex> lock(g_layers_mutex);
   const int grid = sms * 16;
   ND_TRY(ensure_hubs(g, grid));
-  return ladies ? ensure_terms(g, grid) : ensure_degrees(g, grid);
+  if (!ladies) return ensure_degrees(g, grid);
+  ND_TRY(ensure_terms(g, grid));
+  return lay.sums_far ? ND_OK : ensure_hub_tables(g, lay);
 }
 
 // ND_COLLECTIVE_BITMAP_GLOBAL=1 puts the big part into global scratch whatever the graph's size (the tests use it to
@@ -934,7 +1059,7 @@ int nd_coll_bitmap_alloc(nd_sampler *s) {
   const bool ladies = s->p.app == ND_APP_LADIES_IS;
   s->coll_global = force_global();
   const Plan p = plan_of(s);
-  ND_TRY(ensure_layers(s->g, s->dev.sms, ladies));
+  ND_TRY(ensure_layers(s->g, s->dev.sms, ladies, p.lay));
   ND_CUDA(ladies ? (p.lay.sums_far ? nd_smem_most(coll_bitmap_kernel<true, true>, s->dev) : nd_smem_most(coll_bitmap_kernel<true, false>, s->dev))
                  : nd_smem_most(coll_bitmap_kernel<false, false>, s->dev));
   s->coll_grid = (int)std::min<int64_t>(s->S > 0 ? s->S : 1, (int64_t)s->dev.sms * p.per_sm);
@@ -948,8 +1073,9 @@ int nd_coll_bitmap_launch(nd_sampler *s, const CollParams &cp, unsigned long lon
   const bool ladies = s->p.app == ND_APP_LADIES_IS;
   const Plan p = plan_of(s);
   const nd_graph *g = s->g;
+  const NdHubTable table = ladies && !p.lay.sums_far ? g->hub_tables[p.lay.group_bits - LADIES_GROUP_BITS] : NdHubTable{};
   const Args a{nd_view(g), cp, s->p.steps, s->S, p.lay, s->d_bm, s->d_initial, s->d_out, s->d_adj, s->d_prob,
-               g->deg_codes, g->big, g->n_big, g->term, g->hub_slot, g->hub_bits, s->d_rows_acc, s->d_stats, pairs};
+               g->deg_codes, g->big, g->n_big, g->term, g->hub_slot, g->hub_bits, table.sums, table.starts, g->hub_ids, g->hub_terms, s->d_rows_acc, s->d_stats, pairs};
   if (ladies && p.lay.sums_far) coll_bitmap_kernel<true, true><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
   else if (ladies) coll_bitmap_kernel<true, false><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
   else coll_bitmap_kernel<false, false><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);

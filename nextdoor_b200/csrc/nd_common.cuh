@@ -102,6 +102,12 @@ struct NdBigVertex {
   float weight;   // deg * deg
 };
 
+// The terms of the hubs' neighbours per group of vertices, and where the groups begin among them (LADIES).
+struct NdHubTable {
+  double *sums = nullptr;
+  int32_t *starts = nullptr;
+};
+
 struct nd_graph {
   int device = 0;
   int32_t V = 0;
@@ -129,6 +135,13 @@ struct nd_graph {
   mutable float *term = nullptr;       // [E] (w / rowsum)^2 (LADIES)
   mutable int32_t *hub_slot = nullptr; // [V] slot of the vertex's neighbourhood as a bitmap, -1: none
   mutable uint32_t *hub_bits = nullptr;
+  mutable int32_t *hubs = nullptr;     // [n_hubs] the vertices by their slots
+  mutable int n_hubs = 0;
+  mutable int hub_lists = -1;          // LADIES: the next three are there (0: they cannot be, -1: not asked yet)
+  mutable int32_t *hub_ids = nullptr;  // the hubs' neighbours, each once, hub after hub
+  mutable double *hub_terms = nullptr; // the sums of their terms
+  mutable int32_t *hub_offs = nullptr; // [2 n_hubs] where the hubs begin, how many there are
+  mutable NdHubTable hub_tables[6];    // ... by the size of its groups
 };
 
 struct NdGraphView {

@@ -138,7 +138,7 @@ def test_rows_in_any_order(nd, monkeypatch, app, scratch, V, M, B, L):
     assert np.allclose(out[0][1], out[1][1], rtol=1e-6, atol=0)
 
 
-def _ladies(nd, ndo, hg, S, B, L, init):
+def _ladies(nd, ndo, hg, S, B, L, init, adjacency=True):
     """Against 64-bit sums of the 32-bit terms.  2^18 terms added up in any order differ by 2^18 * 2^-53 of the total at
     most: a draw may fall to another candidate only that near to the end of one."""
     V, steps = hg.V, 2
@@ -169,7 +169,8 @@ def _ladies(nd, ndo, hg, S, B, L, init):
             assert ok.all()
             assert np.allclose(prob[smp, step], np.diff(cdf, prepend=0.0)[mine] / cdf[-1], rtol=1e-6, atol=2.0 ** -35)
     assert s.stats()["union_unique"] == seen
-    assert ndo.check_adjacency(hg, ndo.make_params(9, steps=steps, fanout=L, batch=B, seed=3), S, init, s.final_samples(), aux["adj_row"], aux["adj_col"]) == 0
+    if adjacency:   # (whose probes ask for lists that ascend)
+        assert ndo.check_adjacency(hg, ndo.make_params(9, steps=steps, fanout=L, batch=B, seed=3), S, init, s.final_samples(), aux["adj_row"], aux["adj_col"]) == 0
 
 
 @pytest.mark.parametrize("V,B,L", [(129, 3, 1), (200_000, 100, 300), (200_000, 40, 31), (1_100_000, 64, 33), (1_300_000, 64, 64)])
@@ -190,3 +191,25 @@ def test_ladies_of_many_vertices(nd, ndo, V):
     dst = np.concatenate([rng.choice(ids, 60_000), [ids[0]]]).astype(np.int32)
     hg = ndo.csr_from_records(src, dst, (rng.random(len(src)) + 0.1).astype(np.float32), V=V)
     _ladies(nd, ndo, hg, 6, 32, 64, rng.choice(ids, 6 * 32).astype(np.int32))
+
+
+@pytest.mark.parametrize("order", ["ascending", "hub's list"])
+@pytest.mark.parametrize("repeats", [1, 40])
+def test_ladies_hubs_by_tables(nd, ndo, order, repeats):
+    """Hubs whose neighbours occur once and many times, whose lists end inside a group, and one whose list is in another order."""
+    V, rng = 40_000, np.random.default_rng(repeats)
+    hubs = np.array([0, 5, 127, 128, 20_000, V - 1])
+    deg = rng.integers(0, 9, V)
+    deg[hubs] = [300, 312, 313, 5000, 9001, 30_000]     # V / 128 = 312: one of them is none
+    src = np.repeat(np.arange(V), deg).astype(np.int32)
+    dst = (V * rng.random(len(src)) ** 2).astype(np.int32)
+    often = np.isin(src, hubs) & (rng.random(len(src)) < 0.5)
+    dst[often] = dst[often] // repeats * repeats        # on average `repeats` times the same neighbour
+    toward = ~np.isin(src, hubs) & (rng.random(len(src)) < 0.3)
+    dst[toward] = rng.choice(hubs, toward.sum())
+    hg = ndo.csr_from_records(src, dst, (rng.random(len(src)) + 0.1).astype(np.float32), V=V)
+    if order != "ascending":
+        a, b = hg.row_ptr[20_000], hg.row_ptr[20_001]
+        hg.col[a:b], hg.w[a:b] = hg.col[a:b][::-1].copy(), hg.w[a:b][::-1].copy()
+    init = np.where(rng.random(30 * 24) < 0.2, rng.choice(hubs, 30 * 24), rng.integers(0, V, 30 * 24)).astype(np.int32)
+    _ladies(nd, ndo, hg, 30, 24, 48, init, adjacency=order == "ascending")
