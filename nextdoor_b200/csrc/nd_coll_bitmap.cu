@@ -68,7 +68,7 @@ struct Layout {
   int slots;                                           // LADIES: groups with accumulators at a time
   uint32_t off_gcdf;                                   // FastGCN: inside the big part (the bitmap is at 0); LADIES: inside shared memory, unless sums_far
   bool sums_far;
-  uint32_t off_red, off_tr, off_layer, off_ut, off_mult, off_pre;   // inside shared memory
+  uint32_t off_red, off_tr, off_layer, off_ut, off_mult, off_same, off_pre;   // inside shared memory
   uint32_t off_draw, off_there, off_acc;                // LADIES: the same; the accumulators may be where the bitmap is
   uint32_t off_slot;                                   // LADIES: with the groups' sums
   uint32_t bytes;                                      // dynamic shared memory of the launch
@@ -366,13 +366,15 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
   int32_t *sh_tr = reinterpret_cast<int32_t *>(smem + lay.off_tr);
   int32_t *sh_layer = reinterpret_cast<int32_t *>(smem + lay.off_layer);
   Transit *ut = reinterpret_cast<Transit *>(smem + lay.off_ut);
-  int32_t *sh_mult = reinterpret_cast<int32_t *>(smem + lay.off_mult);   // how often a transit occurs; 0: an earlier one is the same
+  int32_t *sh_mult = reinterpret_cast<int32_t *>(smem + lay.off_mult);   // how often a transit occurs (the first of a kind counts); then its place in ut, -1: not a vertex
+  int32_t *sh_same = reinterpret_cast<int32_t *>(smem + lay.off_same);   // the first transit that is the same
   uint32_t *pre = reinterpret_cast<uint32_t *>(smem + lay.off_pre);
   double *acc = reinterpret_cast<double *>(smem + lay.off_acc);          // LADIES from here on
   uint32_t *there = reinterpret_cast<uint32_t *>(smem + lay.off_there);
   double *sh_target = reinterpret_cast<double *>(smem + lay.off_draw);   // of a draw: the point of the CDF, its group, the first draw of the group
   int32_t *sh_group = reinterpret_cast<int32_t *>(sh_target + cp.L), *sh_first = sh_group + cp.L;
-  uint32_t *sh_firsts = reinterpret_cast<uint32_t *>(sh_first + cp.L);   // draws that are the first of their group, as bits
+  int32_t *sh_slot_group = sh_first + cp.L;
+  uint32_t *sh_firsts = reinterpret_cast<uint32_t *>(sh_slot_group + cp.L);   // draws that are the first of their group, as bits
   uint8_t *slot = (LADIES && !SUMS_FAR ? smem : big) + lay.off_slot;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
   unsigned long long ids_sum = 0, uniq_sum = 0, draws = 0;   // thread 0
@@ -388,23 +390,30 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
       }
       __syncthreads();
       // ---- the batch's transits, each once: the hubs from the front of the list, the others from its end
-      for (int q = tid; q < cp.ntr * cp.ntr; q += blockDim.x) {
-        const int i = q / cp.ntr, j = q - i * cp.ntr;
-        if (j > i && sh_tr[i] == sh_tr[j]) {   // the first of a kind counts the others, which are struck out (negative)
-          atomicAdd(sh_mult + i, 1);
-          atomicOr(sh_mult + j, (int)0x80000000);
-        }
+      for (int j = tid; j < cp.ntr; j += blockDim.x) {
+        const int32_t t = sh_tr[j];
+        int first = j;
+#pragma unroll 8
+        for (int k = 0; k < j; k++) first = sh_tr[k] == t && k < first ? k : first;
+        sh_same[j] = first;
+        if (first != j) atomicAdd(sh_mult + first, 1);
       }
       __syncthreads();
       unsigned long long ids = 0;
       for (int i = tid; i < cp.ntr; i += blockDim.x) {
         const int32_t t = sh_tr[i];
-        if (t < 0 || t >= cp.V) continue;
-        const int32_t rs = __ldg(a.g.row_ptr + t), deg = __ldg(a.g.row_ptr + t + 1) - rs, slot = __ldg(a.hub_slot + t);
-        ids += (unsigned long long)deg;
-        if (sh_mult[i] > 0) {
-          ut[slot >= 0 && (!LADIES || a.hub_sums) ? atomicAdd(&sh_hubs, 1) : cp.ntr - 1 - atomicAdd(&sh_rest, 1)] = Transit{rs, deg, sh_mult[i], slot};
+        const bool valid = t >= 0 && t < cp.V, first = sh_same[i] == i;
+        int place = -1;
+        if (valid) {
+          const int32_t rs = __ldg(a.g.row_ptr + t), deg = __ldg(a.g.row_ptr + t + 1) - rs;
+          ids += (unsigned long long)deg;
+          if (first) {
+            const int32_t slot = __ldg(a.hub_slot + t);
+            place = slot >= 0 && (!LADIES || a.hub_sums) ? atomicAdd(&sh_hubs, 1) : cp.ntr - 1 - atomicAdd(&sh_rest, 1);
+            ut[place] = Transit{rs, deg, sh_mult[i], slot};
+          }
         }
+        if (first) sh_mult[i] = place;
       }
       for (int o = 16; o > 0; o >>= 1) ids += __shfl_xor_sync(0xffffffffu, ids, o);
       if (lane == 0) reinterpret_cast<unsigned long long *>(red)[warp] = ids;
@@ -558,7 +567,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
               const int k = sh_first[j] == j ? slot_of(j) - s0 : -1;
               if (k >= 0 && k < here) {
                 slot[sh_group[j]] = (uint8_t)k;
-                sh_mult[k] = sh_group[j];   // (not needed any more: the groups of the slots)
+                sh_slot_group[k] = sh_group[j];
               }
             }
             __syncthreads();
@@ -566,7 +575,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
             for (int q = warp; q < here * nh; q += warps) {   // hubs: a warp goes to a group of one
               const int k = q / nh;
               const Transit t = ut[q - k * nh];
-              const int32_t *at = a.hub_starts + (size_t)t.slot * (groups + 1) + sh_mult[k];
+              const int32_t *at = a.hub_starts + (size_t)t.slot * (groups + 1) + sh_slot_group[k];
               const int32_t end = __ldg(at + 1);
               for (int32_t e = __ldg(at) + lane; e < end; e += 32)
                 atomicAdd(acc + ((size_t)k << lay.group_bits) + (__ldg(a.hub_ids + e) & (n - 1)), __ldg(a.hub_terms + e) * (double)t.mult);
@@ -671,7 +680,33 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
       }
       if (tid == 0) { if (U > 0 && total > 0.0) draws += (unsigned long long)cp.L; }
       __syncthreads();
-      emit_adjacency(a.g, cp, sh_tr, sh_layer, a.adj + (s * a.steps + cp.step) * (int64_t)adj_words(cp.stride), a.hub_slot, a.hub_bits, lay.words);
+      uint32_t *adj = a.adj + (s * a.steps + cp.step) * (int64_t)adj_words(cp.stride);
+      if (nu < cp.ntr && (int64_t)nu * cp.L <= (int64_t)lay.words * 32) {
+        // repeated transits have the same entries: each list is asked once, where the union was, and the answers copied
+        probe_pairs(a.g.col, a.hub_bits, lay.words, nu * cp.L, bm, [&](int e, PairList &list, int32_t &v) {
+          const int d = e / cp.L;
+          const Transit &t = ut[d < nh ? d : cp.ntr - 1 - (d - nh)];
+          list = PairList{t.rs, t.deg, t.slot};
+          v = sh_layer[e - d * cp.L];
+          return v >= 0 && v < cp.V;
+        });
+        __syncthreads();
+        for (int e0 = tid - lane; e0 < cp.stride; e0 += blockDim.x) {
+          const int e = e0 + lane, i = e / cp.L;
+          bool edge = false;
+          if (e < cp.stride && i < cp.ntr) {
+            const int place = sh_mult[sh_same[i]];
+            if (place >= 0) {
+              const int at = (place < nh ? place : nh + (cp.ntr - 1 - place)) * cp.L + (e - i * cp.L);
+              edge = (bm[at >> 5] >> (at & 31)) & 1u;
+            }
+          }
+          const uint32_t word = __ballot_sync(0xffffffffu, edge);
+          if (lane == 0) adj[e0 / 32] = word;
+        }
+      } else {
+        emit_adjacency(a.g, cp, sh_tr, sh_layer, adj, a.hub_slot, a.hub_bits, lay.words);
+      }
       __syncthreads();
     }
     if (tid == 0) sh_sample = a.S > gridDim.x ? (long long)gridDim.x + (long long)atomicAdd(&a.acc[8], 1ull) : (long long)a.S;
@@ -1006,12 +1041,13 @@ Plan plan_of(const nd_sampler *s) {
     l.glob_bytes = global ? big : 0u;
     uint32_t off = global ? 0u : big;
     if (ladies && !l.sums_far) { l.off_gcdf = off; l.off_slot = off + sums; off += sums + slots; }
-    l.off_draw = off; off += ladies ? (16u * (uint32_t)L + 4u * (((uint32_t)L + 31u) / 32u) + 7u) & ~7u : 0u;
+    l.off_draw = off; off += ladies ? (20u * (uint32_t)L + 4u * (((uint32_t)L + 31u) / 32u) + 7u) & ~7u : 0u;
     l.off_red = off; off += 8u * 32u + 4u * 32u;
     l.off_ut = off; off += (uint32_t)sizeof(Transit) * (uint32_t)ntr;
     l.off_tr = off; off += 4u * (uint32_t)ntr;
     l.off_layer = off; off += 4u * (uint32_t)L;
     l.off_mult = off; off += 4u * (uint32_t)ntr;
+    l.off_same = off; off += 4u * (uint32_t)ntr;
     l.off_pre = off; off += ladies ? 4u * (uint32_t)ntr : 0u;
     l.off_there = off; off += ladies ? (uint32_t)L << (group_bits - 3) : 0u;
     return (off + 15u) & ~15u;
