@@ -799,41 +799,51 @@ __global__ void hub_slots_kernel(const int32_t *__restrict__ row_ptr, int32_t V,
   }
 }
 
+__global__ void hub_degrees_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ hubs, int n, int32_t *__restrict__ deg) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) deg[i] = row_ptr[hubs[i] + 1] - row_ptr[hubs[i]];
+}
+
 // LADIES: a hub's neighbours, each once, and the sums of their terms, a CTA per hub (graphs repeat edges between hubs hundreds
-// of times); hub i's go to ids[offs[i]] and on, their number to count[i].  *odd: a list does not ascend.
-__global__ void __launch_bounds__(256) hub_unique_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col, const float *__restrict__ term,
-                                                         const int32_t *__restrict__ hubs, const int32_t *__restrict__ offs, int32_t *__restrict__ ids,
-                                                         double *__restrict__ terms, int32_t *__restrict__ count, int *__restrict__ odd) {
-  __shared__ int32_t heads_of[8];
+// of times: what a warp has of one neighbour is added up first); hub i's go to ids[offs[i]] and on, terms zero before,
+// their number to count[i].  *odd: a list does not ascend.
+constexpr int HUB_THREADS = 1024;
+__global__ void __launch_bounds__(HUB_THREADS) hub_unique_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col,
+                                                                 const float *__restrict__ term, const int32_t *__restrict__ hubs,
+                                                                 const int32_t *__restrict__ offs, int32_t *__restrict__ ids, double *__restrict__ terms,
+                                                                 int32_t *__restrict__ count, int *__restrict__ odd) {
+  __shared__ int32_t heads_of[HUB_THREADS / 32];
   const int32_t v = hubs[blockIdx.x], rs = row_ptr[v], end = row_ptr[v + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int32_t at = offs[blockIdx.x];
-  for (int32_t e0 = rs; e0 < end; e0 += 256) {
+  for (int32_t e0 = rs; e0 < end; e0 += HUB_THREADS) {
     const int32_t e = e0 + (int32_t)threadIdx.x;
     const int32_t c = e < end ? col[e] : 0, before = e < end && e > rs ? col[e - 1] : -1;
     if (e < end && before > c) *odd = 1;
-    const bool head = e < end && c != before;
-    const uint32_t heads = __ballot_sync(0xffffffffu, head);
+    const uint32_t heads = __ballot_sync(0xffffffffu, e < end && c != before);
     __syncthreads();
     if (lane == 0) heads_of[warp] = __popc(heads);
     __syncthreads();
-    int32_t to = at + __popc(heads & ((1u << lane) - 1u));
-    for (int w = 0; w < 8; w++) {
+    int32_t to = at + __popc(heads & (0xffffffffu >> (31 - lane))) - 1;   // the neighbour's place: of the last head up to here
+    for (int w = 0; w < HUB_THREADS / 32; w++) {
       if (w < warp) to += heads_of[w];
       at += heads_of[w];
     }
-    if (head) {
-      double sum = 0.0;
-      for (int32_t x = e; x < end && col[x] == c; x++) sum += (double)term[x];
-      ids[to] = c;
-      terms[to] = sum;
+    double sum = e < end ? (double)term[e] : 0.0;
+    const int head = 31 - __clz((heads | 1u) & (0xffffffffu >> (31 - lane)));
+    for (int step = 1; step < 32; step <<= 1) {
+      const double t = __shfl_up_sync(0xffffffffu, sum, step);
+      if (lane - step >= head) sum += t;
     }
+    if (e >= end) continue;
+    if ((heads >> lane) & 1u) ids[to] = c;
+    if (lane == 31 || e + 1 == end || ((heads >> (lane + 1)) & 1u)) atomicAdd(terms + to, sum);
   }
   if (threadIdx.x == 0) count[blockIdx.x] = at - offs[blockIdx.x];
 }
 
 // ... and its groups: where each begins there, and its sum
-__global__ void __launch_bounds__(256) hub_table_kernel(const int32_t *__restrict__ ids, const double *__restrict__ terms, const int32_t *__restrict__ offs,
+__global__ void __launch_bounds__(HUB_THREADS) hub_table_kernel(const int32_t *__restrict__ ids, const double *__restrict__ terms, const int32_t *__restrict__ offs,
                                                         const int32_t *__restrict__ count, int groups, int group_bits, double *__restrict__ sums,
                                                         int32_t *__restrict__ starts) {
   const int32_t first = offs[blockIdx.x], end = first + count[blockIdx.x];
@@ -959,27 +969,28 @@ int ensure_hub_tables(const nd_graph *g, const Layout &lay) {
   const size_t n = (size_t)g->n_hubs, groups = (size_t)lay.groups;
   if (t.sums || n == 0 || g->hub_lists == 0 || n * (12 * groups + 4) > HUB_TABLES) return ND_OK;
   if (g->hub_lists < 0) {
-    std::vector<int32_t> hubs(n), offs(n + 1);
-    ND_CUDA(cudaMemcpy(hubs.data(), g->hubs, sizeof(int32_t) * n, cudaMemcpyDeviceToHost));
+    NdDevMem<int32_t> ids, d_offs;
+    ND_TRY(d_offs.alloc(2 * n));
+    std::vector<int32_t> offs(n);
+    hub_degrees_kernel<<<(unsigned)(n + 255) / 256, 256>>>(g->row_ptr, g->hubs, (int)n, d_offs.p);
+    ND_CUDA(cudaMemcpy(offs.data(), d_offs.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost));
     int64_t all = 0;
     for (size_t i = 0; i < n; i++) {
-      int32_t row[2];
-      ND_CUDA(cudaMemcpy(row, g->row_ptr + hubs[i], sizeof(row), cudaMemcpyDeviceToHost));
+      const int32_t deg = offs[i];
       offs[i] = (int32_t)all;
-      all += row[1] - row[0];
+      all += deg;
     }
     if (12 * (size_t)all > HUB_TABLES) { g->hub_lists = 0; return ND_OK; }
-    NdDevMem<int32_t> ids, d_offs;
     NdDevMem<double> terms;
     NdDevMem<int> flag;
     int odd = 0;
     ND_TRY(ids.alloc((size_t)all));
     ND_TRY(terms.alloc((size_t)all));
-    ND_TRY(d_offs.alloc(2 * n));
     ND_TRY(flag.alloc(1));
     ND_CUDA(cudaMemset(flag.p, 0, sizeof(int)));
     ND_CUDA(cudaMemcpy(d_offs.p, offs.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice));
-    hub_unique_kernel<<<(unsigned)n, 256>>>(g->row_ptr, g->col, g->term, g->hubs, d_offs.p, ids.p, terms.p, d_offs.p + n, flag.p);
+    ND_CUDA(cudaMemset(terms.p, 0, sizeof(double) * (size_t)all));
+    hub_unique_kernel<<<(unsigned)n, HUB_THREADS>>>(g->row_ptr, g->col, g->term, g->hubs, d_offs.p, ids.p, terms.p, d_offs.p + n, flag.p);
     ND_CUDA(cudaMemcpy(&odd, flag.p, sizeof(int), cudaMemcpyDeviceToHost));
     g->hub_lists = odd ? 0 : 1;
     if (odd) return ND_OK;
@@ -991,7 +1002,7 @@ int ensure_hub_tables(const nd_graph *g, const Layout &lay) {
   NdDevMem<int32_t> starts;
   ND_TRY(sums.alloc(n * groups));
   ND_TRY(starts.alloc(n * (groups + 1)));
-  hub_table_kernel<<<(unsigned)n, 256>>>(g->hub_ids, g->hub_terms, g->hub_offs, g->hub_offs + n, lay.groups, lay.group_bits, sums.p, starts.p);
+  hub_table_kernel<<<(unsigned)n, HUB_THREADS>>>(g->hub_ids, g->hub_terms, g->hub_offs, g->hub_offs + n, lay.groups, lay.group_bits, sums.p, starts.p);
   ND_CUDA(cudaDeviceSynchronize());
   t.starts = starts.release();
   t.sums = sums.release();
