@@ -961,8 +961,8 @@ int ensure_terms(const nd_graph *g, int grid) {
   return ND_OK;
 }
 
-// LADIES: the hubs' neighbours and groups of 2^bits vertices, unless they would take more than HUB_TABLES bytes or a list
-// does not ascend
+// LADIES: the hubs' neighbours and groups of 2^bits vertices, unless they would take more than HUB_TABLES bytes, the
+// device has no room for them or a list does not ascend
 constexpr size_t HUB_TABLES = (size_t)256 << 20;
 int ensure_hub_tables(const nd_graph *g, const Layout &lay) {
   NdHubTable &t = g->hub_tables[lay.group_bits - LADIES_GROUP_BITS];
@@ -970,7 +970,7 @@ int ensure_hub_tables(const nd_graph *g, const Layout &lay) {
   if (t.sums || n == 0 || g->hub_lists == 0 || n * (12 * groups + 4) > HUB_TABLES) return ND_OK;
   if (g->hub_lists < 0) {
     NdDevMem<int32_t> ids, d_offs;
-    ND_TRY(d_offs.alloc(2 * n));
+    if (d_offs.alloc(2 * n) != ND_OK) return ND_OK;
     std::vector<int32_t> offs(n);
     hub_degrees_kernel<<<(unsigned)(n + 255) / 256, 256>>>(g->row_ptr, g->hubs, (int)n, d_offs.p);
     ND_CUDA(cudaMemcpy(offs.data(), d_offs.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost));
@@ -984,9 +984,7 @@ int ensure_hub_tables(const nd_graph *g, const Layout &lay) {
     NdDevMem<double> terms;
     NdDevMem<int> flag;
     int odd = 0;
-    ND_TRY(ids.alloc((size_t)all));
-    ND_TRY(terms.alloc((size_t)all));
-    ND_TRY(flag.alloc(1));
+    if (ids.alloc((size_t)all) != ND_OK || terms.alloc((size_t)all) != ND_OK || flag.alloc(1) != ND_OK) return ND_OK;
     ND_CUDA(cudaMemset(flag.p, 0, sizeof(int)));
     ND_CUDA(cudaMemcpy(d_offs.p, offs.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice));
     ND_CUDA(cudaMemset(terms.p, 0, sizeof(double) * (size_t)all));
@@ -1000,8 +998,7 @@ int ensure_hub_tables(const nd_graph *g, const Layout &lay) {
   }
   NdDevMem<double> sums;
   NdDevMem<int32_t> starts;
-  ND_TRY(sums.alloc(n * groups));
-  ND_TRY(starts.alloc(n * (groups + 1)));
+  if (sums.alloc(n * groups) != ND_OK || starts.alloc(n * (groups + 1)) != ND_OK) return ND_OK;
   hub_table_kernel<<<(unsigned)n, HUB_THREADS>>>(g->hub_ids, g->hub_terms, g->hub_offs, g->hub_offs + n, lay.groups, lay.group_bits, sums.p, starts.p);
   ND_CUDA(cudaDeviceSynchronize());
   t.starts = starts.release();
@@ -1011,13 +1008,16 @@ int ensure_hub_tables(const nd_graph *g, const Layout &lay) {
 
 // What a graph's first sampler builds goes to the graph when all of it is there: a build that runs out of memory
 // leaves nothing behind.
-int ensure_layers(const nd_graph *g, int sms, bool ladies, const Layout &lay) {
+int ensure_layers(const nd_graph *g, int sms, bool ladies, const Layout &lay, NdHubTable *table) {
   std::lock_guard<std::mutex> lock(g_layers_mutex);
   const int grid = sms * 16;
   ND_TRY(ensure_hubs(g, grid));
   if (!ladies) return ensure_degrees(g, grid);
   ND_TRY(ensure_terms(g, grid));
-  return lay.sums_far ? ND_OK : ensure_hub_tables(g, lay);
+  if (lay.sums_far) return ND_OK;
+  ND_TRY(ensure_hub_tables(g, lay));
+  *table = g->hub_tables[lay.group_bits - LADIES_GROUP_BITS];
+  return ND_OK;
 }
 
 // ND_COLLECTIVE_BITMAP_GLOBAL=1 puts the big part into global scratch whatever the graph's size (the tests use it to
@@ -1106,23 +1106,21 @@ int nd_coll_bitmap_alloc(nd_sampler *s) {
   const bool ladies = s->p.app == ND_APP_LADIES_IS;
   s->coll_global = force_global();
   const Plan p = plan_of(s);
-  ND_TRY(ensure_layers(s->g, s->dev.sms, ladies, p.lay));
   ND_CUDA(ladies ? (p.lay.sums_far ? nd_smem_most(coll_bitmap_kernel<true, true>, s->dev) : nd_smem_most(coll_bitmap_kernel<true, false>, s->dev))
                  : nd_smem_most(coll_bitmap_kernel<false, false>, s->dev));
   s->coll_grid = (int)std::min<int64_t>(s->S > 0 ? s->S : 1, (int64_t)s->dev.sms * p.per_sm);
   if (p.lay.glob_bytes) ND_CUDA(nd_malloc(&s->d_bm, (size_t)p.lay.glob_bytes * (size_t)s->coll_grid));
   ND_CUDA(nd_malloc(&s->d_rows_acc, 16 * sizeof(unsigned long long)));
   ND_CUDA(cudaMemset(s->d_rows_acc, 0, 16 * sizeof(unsigned long long)));
-  return ND_OK;
+  return ensure_layers(s->g, s->dev.sms, ladies, p.lay, &s->hub_table);   // last: what is optional there leaves the sampler its room
 }
 
 int nd_coll_bitmap_launch(nd_sampler *s, const CollParams &cp, unsigned long long pairs) {
   const bool ladies = s->p.app == ND_APP_LADIES_IS;
   const Plan p = plan_of(s);
   const nd_graph *g = s->g;
-  const NdHubTable table = ladies && !p.lay.sums_far ? g->hub_tables[p.lay.group_bits - LADIES_GROUP_BITS] : NdHubTable{};
   const Args a{nd_view(g), cp, s->p.steps, s->S, p.lay, s->d_bm, s->d_initial, s->d_out, s->d_adj, s->d_prob,
-               g->deg_codes, g->big, g->n_big, g->term, g->hub_slot, g->hub_bits, table.sums, table.starts, g->hub_ids, g->hub_terms, s->d_rows_acc, s->d_stats, pairs};
+               g->deg_codes, g->big, g->n_big, g->term, g->hub_slot, g->hub_bits, s->hub_table.sums, s->hub_table.starts, g->hub_ids, g->hub_terms, s->d_rows_acc, s->d_stats, pairs};
   if (ladies && p.lay.sums_far) coll_bitmap_kernel<true, true><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
   else if (ladies) coll_bitmap_kernel<true, false><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
   else coll_bitmap_kernel<false, false><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);

@@ -248,6 +248,7 @@ struct nd_sampler {
   void *d_init_rec = nullptr;
   bool loop_ready = false;
   // a lane per walk (nd_walk_rows.cu): walks that can start, counters of the running job
+  int layout = 0;                 // what its kernels read of the graph (nd_walk_rows.cu)
   int4 *d_list = nullptr;
   unsigned long long *d_rows_acc = nullptr;
   bool live_is_ended = false;     // d_nlive holds walks by the number of their vertices (see nd_sampler_live_pairs)
@@ -282,6 +283,7 @@ struct nd_sampler {
   bool coll_bitmap = false;       // importance sampling through the shared-memory bitmap kernel
   bool coll_global = false;       // ... whose bitmaps are put into global scratch whatever the graph's size
   int coll_grid = 0;
+  NdHubTable hub_table;           // LADIES: of the graph's tables, the one that its kernel reads; null: none
   unsigned char *d_bm = nullptr;  // per-CTA bitmap slices when a bit per vertex does not fit shared memory
 
   NdHostRows *hostrows = nullptr;

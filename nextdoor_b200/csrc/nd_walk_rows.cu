@@ -3,7 +3,7 @@
 // organisation of a job gives the same samples, and on B200 a lane that keeps its walk in registers beats a
 // step-by-step pass over a transit-sorted map at every number of walks (measured, transit-parallel loop with
 // counting inversion -> this file: uniform walk on 57 K vertices 1.10 -> 0.07 ms, DeepWalk on 2^20 vertices
-// 5.2 -> 1.4 ms, node2vec 7.6 -> 2.3 ms, PPR on 2^24 vertices 5.4 -> 2.5 ms).
+// 5.2 -> 1.4 ms, node2vec 7.6 -> 2.1 ms, PPR on 2^24 vertices 5.4 -> 2.4 ms).
 //
 // What bounds it.  Large graphs: the rate of random DRAM reads.  A walker picks every CSR entry with the same
 // probability, and a gather that misses the L2 reads a whole line of 128 bytes (11.1 GB for 91 M gathers of 4 bytes from
@@ -759,14 +759,6 @@ adjset_build_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restri
 constexpr int64_t ERECS = (int64_t)1 << 22;
 // Ids that leave a byte of a word to the weight.
 constexpr int32_t PACK_V = 1 << 24;
-int layout_of(const nd_sampler *s) {
-  const nd_graph *g = s->g;
-  const bool weighted = s->p.app == ND_APP_DEEPWALK || s->p.app == ND_APP_PPR;
-  if (s->p.app != ND_APP_NODE2VEC && g->erec && (!weighted || g->odd_max == 0)) return LAYOUT_FAT;
-  if (weighted) return !g->pack ? LAYOUT_PLAIN : g->V >= FAR_V ? LAYOUT_FAR : LAYOUT_ALT;
-  if (s->p.app == ND_APP_NODE2VEC && g->V >= FAR_V) return LAYOUT_FAR;
-  return g->V <= DENSE_V && g->E >= DENSE_ENTRIES ? LAYOUT_DENSE : LAYOUT_PLAIN;
-}
 
 template <int APP, int LAYOUT>
 void launch(nd_sampler *s, RowsArgs &a, bool count) {
@@ -787,7 +779,7 @@ void launch(nd_sampler *s, RowsArgs &a, bool count) {
 template <int APP>
 void launch_as(nd_sampler *s, RowsArgs &a, bool count) {
   constexpr bool w = weighted<APP>(), n2v = APP == ND_APP_NODE2VEC;
-  switch (layout_of(s)) {   // (the others are not layouts of the app)
+  switch (s->layout) {   // (the others are not layouts of the app)
     case LAYOUT_FAT: return launch<APP, n2v ? LAYOUT_PLAIN : LAYOUT_FAT>(s, a, count);
     case LAYOUT_ALT: return launch<APP, w ? LAYOUT_ALT : LAYOUT_PLAIN>(s, a, count);
     case LAYOUT_DENSE: return launch<APP, w ? LAYOUT_PLAIN : LAYOUT_DENSE>(s, a, count);
@@ -797,8 +789,9 @@ void launch_as(nd_sampler *s, RowsArgs &a, bool count) {
 }
 
 // The derived layouts of a graph are built by the first sampler that needs them; samplers of one
-// graph may be created from several host threads, so the builds are serialised.  What belongs together goes to
-// the graph together, when all of it is there: a build that runs out of memory leaves nothing behind.
+// graph may be created from several host threads, so the builds are serialised, and a sampler keeps the layout that it
+// found room for: another's may come to the graph later.  What belongs together goes to the graph together, when all of
+// it is there: a build that runs out of memory leaves nothing behind.
 std::mutex g_derived_mutex;
 
 template <class T>
@@ -833,18 +826,21 @@ int ensure_vrow(const nd_graph *g, int sms) {
   return ND_OK;
 }
 
-int ensure_erec(const nd_graph *g, int sms) {
+// `there`: there was room for it
+int ensure_erec(const nd_graph *g, int sms, bool *there) {
+  *there = g->erec != nullptr;
   if (g->erec) return ND_OK;
   NdDevMem<int4> erec;
-  ND_TRY(erec.alloc((size_t)(g->E > 0 ? g->E : 1)));
+  if (erec.alloc((size_t)(g->E > 0 ? g->E : 1)) != ND_OK) return ND_OK;
   erec_build_kernel<<<sms * 16, BUILD_THREADS>>>(g->row_ptr, g->col, g->max_w, g->w, g->V, g->E, erec.p);
   ND_CUDA(cudaGetLastError());
   g->erec = erec.release();
+  *there = true;
   return ND_OK;
 }
 
 // entries with rows, ids and weights in one word, or the records of ensure_colw where neither holds the weights
-int ensure_weighted(const nd_graph *g, int sms) {
+int ensure_weighted(const nd_graph *g, int sms, int *layout) {
   if (g->odd_max < 0) {
     NdDevMem<int> flag;
     int odd = 0;
@@ -854,11 +850,14 @@ int ensure_weighted(const nd_graph *g, int sms) {
     ND_CUDA(cudaMemcpy(&odd, flag.p, sizeof(int), cudaMemcpyDeviceToHost));
     g->odd_max = odd;
   }
-  const bool fat = g->E <= ERECS;
-  if (g->odd_max == 1 || (!fat && g->V > PACK_V)) return ensure_colw(g, sms);
+  *layout = LAYOUT_PLAIN;
+  if (g->odd_max == 1) return ensure_colw(g, sms);
+  bool fat = g->E <= ERECS;
+  if (fat) ND_TRY(ensure_erec(g, sms, &fat));
+  if (!fat && g->V > PACK_V) return ensure_colw(g, sms);
   if (fat || g->V < FAR_V) ND_TRY(ensure_vrow(g, sms));
-  if (fat) return ensure_erec(g, sms);
-  if (g->pack) return ND_OK;
+  *layout = fat ? LAYOUT_FAT : g->V >= FAR_V ? LAYOUT_FAR : LAYOUT_ALT;
+  if (fat || g->pack) return ND_OK;
   NdDevMem<uint32_t> pack;
   ND_TRY(pack.alloc((size_t)(g->E > 0 ? g->E : 1)));
   pack_build_kernel<<<sms * 16, BUILD_THREADS>>>(g->row_ptr, g->col, g->max_w, g->w, g->V, g->E, pack.p);
@@ -867,13 +866,15 @@ int ensure_weighted(const nd_graph *g, int sms) {
   return ND_OK;
 }
 
-int ensure_col3(const nd_graph *g, int sms) {
+int ensure_col3(const nd_graph *g, int sms, bool *there) {
+  *there = g->col3 != nullptr;
   if (g->col3) return ND_OK;
   NdDevMem<uint2> col3;
-  ND_TRY(col3.alloc((size_t)(g->E / DENSE_IDS + 1)));
+  if (col3.alloc((size_t)(g->E / DENSE_IDS + 1)) != ND_OK) return ND_OK;
   col3_build_kernel<<<sms * 16, 256>>>(g->col, g->E, col3.p);
   ND_CUDA(cudaGetLastError());
   g->col3 = col3.release();
+  *there = true;
   return ND_OK;
 }
 
@@ -918,11 +919,14 @@ int nd_walk_rows_alloc(nd_sampler *s) {
   ND_TRY(make(s->d_rows_acc, acc));
   ND_CUDA(cudaMemset(s->d_rows_acc, 0, 8 * acc));
   std::lock_guard<std::mutex> lock(g_derived_mutex);
-  if (app == ND_APP_DEEPWALK || app == ND_APP_PPR) return ensure_weighted(g, sms);
-  if (app == ND_APP_UNIFORM_WALK && g->E <= ERECS) ND_TRY(ensure_erec(g, sms));
-  if (layout_of(s) != LAYOUT_FAR) ND_TRY(ensure_vrow(g, sms));
-  if (layout_of(s) == LAYOUT_DENSE) ND_TRY(ensure_col3(g, sms));
-  if (app == ND_APP_NODE2VEC) ND_TRY(ensure_adjset(g, sms, s->d_status, s->h_status));
+  if (app == ND_APP_DEEPWALK || app == ND_APP_PPR) return ensure_weighted(g, sms, &s->layout);
+  const bool n2v = app == ND_APP_NODE2VEC, far = n2v && g->V >= FAR_V;
+  if (!far) ND_TRY(ensure_vrow(g, sms));
+  if (n2v) ND_TRY(ensure_adjset(g, sms, s->d_status, s->h_status));
+  bool fat = !n2v && g->E <= ERECS, dense = !far && g->V <= DENSE_V && g->E >= DENSE_ENTRIES;
+  if (fat) ND_TRY(ensure_erec(g, sms, &fat));
+  if (dense) ND_TRY(ensure_col3(g, sms, &dense));
+  s->layout = far ? LAYOUT_FAR : fat ? LAYOUT_FAT : dense ? LAYOUT_DENSE : LAYOUT_PLAIN;
   return ND_OK;
 }
 
