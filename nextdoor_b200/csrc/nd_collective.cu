@@ -3,7 +3,7 @@
 //
 // ND_APP_FASTGCN_REF / ND_APP_LADIES_REF follow the reference's shipped next()
 // (src/apps/fastgcn/fastgcnSampling.cu:23-47, src/apps/ladies/ladiessampling.cu:23-47): a vertex
-// drawn uniformly from the whole graph, then one has_edge_logn probe (src/csr.hpp:343-359) per
+// drawn uniformly from the whole graph, then one probe of the list (src/csr.hpp:343-359) per
 // transit to fill the layer's adjacency (row, col) entries.
 //
 // ND_APP_FASTGCN_IS / ND_APP_LADIES_IS are the importance samplers the reference does not have:

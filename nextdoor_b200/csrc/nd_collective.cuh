@@ -16,17 +16,6 @@ __device__ __forceinline__ const int32_t *transits_of(const CollParams &cp, cons
   return cp.step == 0 ? initial + s * cp.B : out + s * cp.fs + (int64_t)(cp.step - 1) * cp.L;
 }
 
-__device__ __forceinline__ bool has_edge_logn(const NdGraphView &g, int32_t src, int32_t dst) {
-  int32_t l = __ldg(g.row_ptr + src), r = __ldg(g.row_ptr + src + 1) - 1;
-  while (l <= r) {
-    const int32_t m = l + (r - l) / 2;
-    const int32_t e = __ldg(g.col + m);
-    if (e == dst) return true;
-    if (e < dst) l = m + 1; else r = m - 1;
-  }
-  return false;
-}
-
 // The adjacency of a layer of a sample is a bit per entry (entry i * L + j: transit i -- vertex j is an edge) in whole
 // words; nd_sampler_aux hands it out as (row, col) = (i, j) or (-1, -1).
 __host__ __device__ inline int adj_words(int stride) { return (stride + 31) / 32; }

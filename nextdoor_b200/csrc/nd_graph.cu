@@ -377,8 +377,8 @@ int build_scratch(BuildScratch *s, int device, int64_t n) {
 
 // records in bs->a (weights as keys) -> graph; key bits outside [lo_bit, hi_bit) are the same in all records.  They are
 // sorted by dst, then src, and the few that share both by weight where they lie: 6 passes instead of 10 over random edges
-// with random weights (8.4M records on the host to a graph, copies included: 6.1 ms -> 4.9; 4.0 since the scatter of
-// nd_radix.cu, of it 0.89 on the device: the passes 0.11 each).  A graph that repeats one edge thousands of times goes
+// with random weights (8.4M records on the host to a graph, copies included: 6.1 ms -> 4.9; 2.8 since the scatter of
+// nd_radix.cu, 0.11 a pass, and with the ids sorted while the weights are on the wire).  A graph that repeats one edge thousands of times goes
 // on to the full sort.
 struct Build {
   const NdDeviceInfo &dev;
