@@ -274,6 +274,11 @@ int nd_sampler_sample(nd_sampler *s, int mode) {
   }
   s->sampled = true;
   if (s->S == 0) return ND_OK;
+  if (nd_is_walk(s->p.app) && !s->in_graph) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s->stream, &st) != cudaSuccess) cudaGetLastError();
+    s->in_graph = st != cudaStreamCaptureStatusNone;
+  }
   ND_TRY(nd_hostrows_keep(s));
   if (s->copy_pending) {  // a result copy on another stream still reads the buffers this job overwrites
     ND_CUDA(cudaStreamWaitEvent(s->stream, s->copy_done, 0));

@@ -251,6 +251,7 @@ struct nd_sampler {
   int layout = 0;                 // what its kernels read of the graph (nd_walk_rows.cu)
   int4 *d_list = nullptr;
   unsigned long long *d_rows_acc = nullptr;
+  bool in_graph = false;          // walks: a caller has captured a job, whose replays the sampler does not see
   bool live_is_ended = false;     // d_nlive holds walks by the number of their vertices (see nd_sampler_live_pairs)
   bool map_stale = false;         // the initial map does not belong to the seeds (walks: sorted by the first job that needs it)
   int32_t *d_init_n = nullptr;    // pairs of the initial map (inside d_nlive)

@@ -260,15 +260,20 @@ int hostrows_init(nd_sampler *s) {
   return ND_OK;
 }
 
+bool find_rows(nd_sampler *s) {
+  NdHostRows *h = s->hostrows;
+  h->dev_out = (int32_t *)reachable(h->out, sizeof(int32_t) * (size_t)s->S * s->fs);
+  h->dev_row_len = (int32_t *)reachable(h->row_len, sizeof(int32_t) * (size_t)s->S);
+  return h->dev_out && h->dev_row_len;
+}
+
 // The rows that the GPU writes itself, whole chunks from the front: as fast as 16 host threads (above).  The host's memory
 // serves both, so that they are not twice as fast together: jobs of 2^21 rows 3.2 -> 2.4 ms with half of them, 2.8 with
 // a third and with all, 2.7 with three quarters.
 int64_t direct_rows(nd_sampler *s, int32_t *out, int32_t *row_len) {
   NdHostRows *h = s->hostrows;
-  if (s->S < 4 * PACK_CHUNK || (uintptr_t)out % 4 || (uintptr_t)row_len % 4) return 0;
-  h->dev_out = (int32_t *)reachable(out, sizeof(int32_t) * (size_t)s->S * s->fs);
-  h->dev_row_len = (int32_t *)reachable(row_len, sizeof(int32_t) * (size_t)s->S);
-  if (!h->dev_out || !h->dev_row_len) return 0;
+  if (s->S < 4 * PACK_CHUNK || s->in_graph || (uintptr_t)out % 4 || (uintptr_t)row_len % 4) return 0;
+  if (!find_rows(s)) return 0;
   if (!h->ds && cudaStreamCreateWithFlags(&h->ds, cudaStreamNonBlocking) != cudaSuccess) { cudaGetLastError(); h->ds = nullptr; return 0; }
   return s->S * 16 / (16 + h->threads) / PACK_CHUNK * PACK_CHUNK;
 }
@@ -305,7 +310,8 @@ int fetch_vals(nd_sampler *s, cudaStream_t st) {
 
 }  // namespace
 
-// The sampler's array is about to change while the GPU has rows of it left to write: these go to the host threads, too.
+// The sampler's array is about to change while the GPU has rows of it left to write, or the GPU no longer reaches the
+// array: these rows go to the host threads, too.
 int nd_hostrows_keep(nd_sampler *s) {
   NdHostRows *h = s->hostrows;
   if (!h || h->stage == 0 || h->direct == 0) return ND_OK;
@@ -416,6 +422,7 @@ int nd_sampler_host_update_finish(nd_sampler *s, int64_t *values_copied) {
   ND_REQUIRE(s && s->hostrows && s->hostrows->stage >= 1, ND_ERR_STATE, "nd_sampler_host_update_finish without a begun update");
   NdHostRows *h = s->hostrows;
   if (h->stage == 1) ND_TRY(nd_sampler_host_update_fetch(s));
+  if (h->direct && !find_rows(s)) ND_TRY(nd_hostrows_keep(s));   // (unregistered since the update was begun)
   ND_REQUIRE(h->stage == 2, ND_ERR_STATE, "nd_sampler_host_update_finish: the update was abandoned after an error");
   h->stage = 0;
   if (values_copied) *values_copied = h->dense ? s->S * (int64_t)s->fs : h->total;

@@ -58,3 +58,44 @@ def test_pipeline_into_pinned_arrays(nd, small_graph, depth):
         whole.set_initial(seeds[k])
         whole.sample(1)
         assert np.array_equal(out.reshape(S, 40), whole.final_samples()), k
+
+
+@pytest.mark.parametrize("step", ["unregistered", "replayed"])
+def test_rows_that_the_gpu_may_no_longer_write(nd, small_graph, step):
+    """Between the begin and the finish of an update the array stops being pinned, or a captured job runs again."""
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    S, steps, rng = 1 << 14, 40, np.random.default_rng(3)
+    s = nd.Sampler(g, nd.app_params(2, steps=steps, seed=5, stop_prob=0.2), num_samples=S)
+    rt, page, stream = torch.cuda.cudart(), 4096, torch.cuda.Stream()
+    own = np.full(S * steps + 1024, g.V, np.int32)
+    out = own[(-own.ctypes.data % page) // 4:][:S * steps]
+    row_len = _pinned(S, 0, 0)
+    assert int(rt.cudaHostRegister(out.ctypes.data, out.nbytes, 0)) == 0
+    s.set_stream(stream.cuda_stream)
+    first, second = (rng.integers(0, g.V, S).astype(np.int32) for _ in range(2))
+    graph = torch.cuda.CUDAGraph()
+    if step == "replayed":
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+            s.sample(1, sync=False)
+        s.set_initial(first)
+        with torch.cuda.stream(stream):
+            graph.replay()
+    else:
+        s.set_initial(first)
+        s.sample(1, sync=False)
+    expected = s.final_samples().copy()
+    s.host_update_begin(out, row_len)
+    if step == "replayed":
+        s.set_initial(second)
+        with torch.cuda.stream(stream):
+            graph.replay()
+        s.sync()
+        assert not np.array_equal(s.final_samples(), expected)
+    else:
+        stream.synchronize()
+        assert int(rt.cudaHostUnregister(out.ctypes.data)) == 0
+    s.host_update_finish()
+    if step == "replayed":
+        assert int(rt.cudaHostUnregister(out.ctypes.data)) == 0
+    assert np.array_equal(out.reshape(S, steps), expected)
+    assert np.array_equal(row_len, (expected != g.V).sum(axis=1))
