@@ -773,7 +773,7 @@ def main():
                 "h2d_bytes_per_step": int(4 * S_total * smp.isz),
                 "d2h_bytes_per_step": int(4 * (S_total + e2e_values)) if e2e_sparse else int(S_total * fs * 4),
                 "host_result": ("the caller's dense [samples, finalSampleSize] host array, kept from step to step: row lengths and the rows' "
-                                "valid prefixes cross PCIe, host threads rewrite the slots that changed (nd_sampler_host_update_*)"
+                                "valid prefixes cross PCIe, host threads and the GPU rewrite the slots that changed (nd_sampler_host_update_*)"
                                 if e2e_sparse else "the dense [samples, finalSampleSize] array copied every step"),
                 "dense_result_bytes": int(S_total * fs * 4),
                 "dense_copy": None if not ms_e2e_dense else {
