@@ -158,19 +158,25 @@ __device__ __forceinline__ uint32_t scan_u32(uint32_t *a, int n, uint32_t *red) 
   return total;
 }
 
-// (a warp takes whole rows of 32, so that neighbouring lanes read neighbouring words)
+// (a warp takes whole rows of 32, so that neighbouring lanes read neighbouring words.  The adds that lead to two
+// neighbouring sums come in different orders, so the sums may differ by a rounding where nothing lies between them: an
+// element of zero takes over the sum before it, and the first sum to reach a target is never one of those.)
 __device__ __forceinline__ void scan_f64(double *a, int n, double *red) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int per = ((n + 31) / 32 + warps - 1) / warps * 32, b = warp * per;
   double carry = 0.0;
   for (int i0 = b; i0 < b + per && i0 < n; i0 += 32) {
     const int i = i0 + lane;
-    double run = i < n ? a[i] : 0.0;
+    const double own = i < n ? a[i] : 0.0;
+    double run = own;
     for (int o = 1; o < 32; o <<= 1) {
       const double t = __shfl_up_sync(0xffffffffu, run, o);
       if (lane >= o) run += t;
     }
     run += carry;
+    const uint32_t upto = __ballot_sync(0xffffffffu, own != 0.0) & (0xffffffffu >> (31 - lane));
+    const double last = __shfl_sync(0xffffffffu, run, upto ? 31 - __clz(upto) : 0);
+    run = upto ? last : carry;
     if (i < n) a[i] = run;
     carry = __shfl_sync(0xffffffffu, run, 31);
   }

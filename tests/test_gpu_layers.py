@@ -193,6 +193,39 @@ def test_ladies_of_many_vertices(nd, ndo, V):
     _ladies(nd, ndo, hg, 6, 32, 64, rng.choice(ids, 6 * 32).astype(np.int32))
 
 
+# draw 44 of this sample is 0xffffffd3 with seed 0: the one in 2^25 that the uniform number 1.0 comes from
+TOP_SAMPLE, TOP_SLOT = 571_925, 44
+
+
+def _top_layer(nd, ndo, V, ids, w, L=64):
+    """The layer of a batch that is vertex 0 alone, whose neighbours are `ids`."""
+    assert ndo.lib().ndo_uniform(0, TOP_SAMPLE, 0, TOP_SLOT, 0) == 1.0
+    src, order = np.zeros(len(ids), np.int32), np.argsort(ids, kind="stable")
+    hg = ndo.csr_from_records(src, ids[order].astype(np.int32), w[order].astype(np.float32), V=V)
+    s = nd.Sampler(nd.Graph.from_csr(hg.row_ptr, hg.col, hg.w, hg.max_w), nd.app_params(9, steps=1, fanout=L, batch=1, seed=0), num_samples=1,
+                   first_sample=TOP_SAMPLE, initial=np.zeros(1, np.int32))
+    s.sample()
+    return s.final_samples()[0], s.aux()["prob"]
+
+
+@pytest.mark.parametrize("V", [3600, 70_000, 200_000, 1_300_000])
+@pytest.mark.parametrize("scratch", ["0", "1"])
+def test_ladies_draws_end_where_there_are_candidates(nd, ndo, monkeypatch, V, scratch):
+    """Weights over eight decades, with which the sums of the groups are not exact, one neighbour in a group, and most groups
+    without any, those behind the last one among them."""
+    monkeypatch.setenv("ND_COLLECTIVE_BITMAP_GLOBAL", scratch)
+    for seed in range(5, 25):
+        rng = np.random.default_rng(seed)
+        n = 22 if V == 3600 else int(rng.integers(20, 300))
+        ids = 128 * rng.permutation(V // 128 - 2)[:n]
+        w = 10 ** rng.uniform(-8, 0, n)
+        if V == 3600:
+            ids = np.sort(ids)
+        layer, prob = _top_layer(nd, ndo, V, ids, w)
+        assert np.isin(layer, ids).all(), (seed, layer[~np.isin(layer, ids)])
+        assert (prob > 0).all(), seed
+
+
 @pytest.mark.parametrize("order", ["ascending", "hub's list"])
 @pytest.mark.parametrize("repeats", [1, 40])
 def test_ladies_hubs_by_tables(nd, ndo, order, repeats):
