@@ -69,7 +69,7 @@ struct Layout {
   uint32_t off_gcdf;                                   // FastGCN: inside the big part (the bitmap is at 0); LADIES: inside shared memory, unless sums_far
   bool sums_far;
   uint32_t off_red, off_tr, off_layer, off_ut, off_mult, off_same, off_pre;   // inside shared memory
-  uint32_t off_draw, off_there, off_acc;                // LADIES: the same; the accumulators may be where the bitmap is
+  uint32_t off_draw, off_acc;                           // LADIES: the same; the accumulators may be where the bitmap is
   uint32_t off_slot;                                   // LADIES: with the groups' sums
   uint32_t bytes;                                      // dynamic shared memory of the launch
   uint32_t glob_bytes;                                 // per-CTA slice of the global scratch, 0 = big part in shared memory
@@ -298,16 +298,16 @@ __device__ __forceinline__ void add_candidates(const NdGraphView &g, const float
 }
 
 // LADIES: the draw's candidate in its group, by a warp: the first whose running sum reaches the target, or by rounding the
-// last there is.  Blocks of 128 candidates, a lane holding four.
-__device__ __forceinline__ void pick_in_group(const double *acc, const uint32_t *there, int n, double before, double target, int &pick, double &wt) {
+// last there is.  Blocks of 128 candidates, a lane holding four.  One with a weight of zero is none (its running sum is
+// the one before it, which another order of the adds may leave a rounding below the target); a group that is drawn from
+// has one that is not.
+__device__ __forceinline__ void pick_in_group(const double *acc, int n, double before, double target, int &pick, double &wt) {
   const int lane = threadIdx.x & 31;
   double at_block = before, run = before;
   int first = 0;
-  uint32_t its = 0;
   bool found = false;
   for (int q = 0; q < n && !found; q += 128) {
     const int r = q + lane * 4;
-    const uint32_t bits = (there[r >> 5] >> (r & 31)) & 15u;
     const double *x = acc + r;
     const double mine = (x[0] + x[1]) + (x[2] + x[3]);
     double upto = mine;
@@ -315,12 +315,11 @@ __device__ __forceinline__ void pick_in_group(const double *acc, const uint32_t 
       const double t = __shfl_up_sync(0xffffffffu, upto, o);
       if (lane >= o) upto += t;
     }
-    const uint32_t reach = __ballot_sync(0xffffffffu, bits && at_block + upto >= target), any = __ballot_sync(0xffffffffu, bits != 0u);
+    const uint32_t reach = __ballot_sync(0xffffffffu, mine > 0.0 && at_block + upto >= target), any = __ballot_sync(0xffffffffu, mine > 0.0);
     if (any) {
       found = reach != 0u;
       const int l = found ? __ffs(reach) - 1 : 31 - __clz(any);
       first = q + l * 4;
-      its = __shfl_sync(0xffffffffu, bits, l);
       run = at_block + __shfl_sync(0xffffffffu, upto - mine, l);
     }
     at_block += __shfl_sync(0xffffffffu, upto, 31);
@@ -330,7 +329,7 @@ __device__ __forceinline__ void pick_in_group(const double *acc, const uint32_t 
   for (int k = 0; k < 4; k++) {
     const double t = acc[first + k];
     run += t;
-    if (!hit && ((its >> k) & 1u)) {
+    if (!hit && t > 0.0) {
       pick = first + k;
       wt = t;
       hit = run >= target;
@@ -376,7 +375,6 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
   int32_t *sh_same = reinterpret_cast<int32_t *>(smem + lay.off_same);   // the first transit that is the same
   uint32_t *pre = reinterpret_cast<uint32_t *>(smem + lay.off_pre);
   double *acc = reinterpret_cast<double *>(smem + lay.off_acc);          // LADIES from here on
-  uint32_t *there = reinterpret_cast<uint32_t *>(smem + lay.off_there);
   double *sh_target = reinterpret_cast<double *>(smem + lay.off_draw);   // of a draw: the point of the CDF, its group, the first draw of the group
   int32_t *sh_group = reinterpret_cast<int32_t *>(sh_target + cp.L), *sh_first = sh_group + cp.L;
   int32_t *sh_slot_group = sh_first + cp.L;
@@ -559,10 +557,6 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
           };
           int drawn = 0;
           for (int k = 0; k < (cp.L + 31) / 32; k++) drawn += __popc(sh_firsts[k]);
-          for (int q = tid; q < cp.L * (n / 32); q += blockDim.x) {   // the accumulators may lie where the union is
-            const int j = q / (n / 32), w = q % (n / 32);
-            if (sh_first[j] == j) there[slot_of(j) * (n / 32) + w] = bm[(size_t)sh_group[j] * (n / 32) + w];
-          }
           for (int s0 = 0; s0 < drawn; s0 += lay.slots) {
             const int here = min(drawn - s0, lay.slots);
             __syncthreads();
@@ -592,7 +586,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
               if (k < 0 || k >= here) continue;
               int pick = 0;
               double wt = 0.0;
-              pick_in_group(acc + (size_t)k * n, there + (s0 + k) * (n / 32), n, group > 0 ? gcdf[group - 1] : 0.0, sh_target[j], pick, wt);
+              pick_in_group(acc + (size_t)k * n, n, group > 0 ? gcdf[group - 1] : 0.0, sh_target[j], pick, wt);
               if (lane == 0) {
                 sh_layer[j] = group * n + pick;
                 a.out[s * cp.fs + (int64_t)cp.step * cp.L + j] = group * n + pick;
@@ -1066,7 +1060,6 @@ Plan plan_of(const nd_sampler *s) {
     l.off_mult = off; off += 4u * (uint32_t)ntr;
     l.off_same = off; off += 4u * (uint32_t)ntr;
     l.off_pre = off; off += ladies ? 4u * (uint32_t)ntr : 0u;
-    l.off_there = off; off += ladies ? (uint32_t)L << (group_bits - 3) : 0u;
     return (off + 15u) & ~15u;
   };
   // Accumulators of a group that is drawn from: in the bitmap's place where that holds SLOTS of them or one for every

@@ -226,6 +226,19 @@ def test_ladies_draws_end_where_there_are_candidates(nd, ndo, monkeypatch, V, sc
         assert (prob > 0).all(), seed
 
 
+@pytest.mark.parametrize("V", [3600, 200_000])
+def test_ladies_draws_no_neighbour_of_weight_zero(nd, ndo, V):
+    """Groups of a dozen candidates with weights over eight decades, between and behind them neighbours that cannot be drawn."""
+    for seed in range(60):
+        rng = np.random.default_rng(seed)
+        ids = np.sort((128 * rng.permutation(V // 128 - 2)[:8, None] + rng.permutation(60)[:12]).reshape(-1))
+        w = 10 ** rng.uniform(-8, 0, len(ids))
+        nothing = np.setdiff1d(np.concatenate([ids + 1, ids + 40]), ids)
+        layer, prob = _top_layer(nd, ndo, V, np.concatenate([ids, nothing]), np.concatenate([w, np.zeros(len(nothing))]))
+        assert np.isin(layer, ids).all(), (seed, layer[~np.isin(layer, ids)])
+        assert (prob > 0).all(), seed
+
+
 @pytest.mark.parametrize("order", ["ascending", "hub's list"])
 @pytest.mark.parametrize("repeats", [1, 40])
 def test_ladies_hubs_by_tables(nd, ndo, order, repeats):
