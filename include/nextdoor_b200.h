@@ -158,7 +158,9 @@ int nd_sampler_final_samples_async(nd_sampler *s, int32_t *out, void *copy_strea
  *           more than half of its slots are in use); optional -- finish calls it when the caller did not.
  *   finish: waits for that copy and writes the rows with host threads (ND_HOST_THREADS, default: the hardware
  *           threads, at most 32), a share of them by the GPU where it can reach both arrays; `values_copied` (may be NULL) receives the number of vertex slots that crossed.
- * One update at a time per sampler; the sampler's next sample() waits on the device for the copies. */
+ * One update at a time per sampler.  The sampler's next sample() may come at any point after begin: it returns at once and
+ * waits on the device for the copies (one in a mode that writes the staging array of the packed rows, the transit-parallel
+ * modes or ND_WALK_* switches, first sends the packed rows to the host where they are not on their way, and waits for it). */
 int nd_sampler_host_update_begin(nd_sampler *s, int32_t *out, int32_t *row_len, void *copy_stream);
 int nd_sampler_host_update_fetch(nd_sampler *s);
 int nd_sampler_host_update_finish(nd_sampler *s, int64_t *values_copied);

@@ -279,7 +279,7 @@ int nd_sampler_sample(nd_sampler *s, int mode) {
     if (cudaStreamIsCapturing(s->stream, &st) != cudaSuccess) cudaGetLastError();
     s->in_graph = st != cudaStreamCaptureStatusNone;
   }
-  ND_TRY(nd_hostrows_keep(s));
+  ND_TRY(nd_hostrows_next_job(s, nd_is_walk(s->p.app) && !nd_walk_lane_per_walk(s, mode)));
   if (s->copy_pending) {  // a result copy on another stream still reads the buffers this job overwrites
     ND_CUDA(cudaStreamWaitEvent(s->stream, s->copy_done, 0));
     s->copy_pending = false;

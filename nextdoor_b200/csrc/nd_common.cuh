@@ -293,7 +293,7 @@ struct nd_sampler {
   int64_t host_stats[8] = {0};
 };
 void nd_hostrows_free(nd_sampler *s);
-int nd_hostrows_keep(nd_sampler *s);
+int nd_hostrows_next_job(nd_sampler *s, bool staging);
 
 // phase timing helpers (no-ops unless profiling is on)
 void nd_phase_begin(nd_sampler *s, int phase);
@@ -312,6 +312,7 @@ int nd_walk_step_status_read(cudaStream_t st, int *status);
 int nd_walk_alloc(nd_sampler *s);
 int nd_walk_ensure_tmp(nd_sampler *s);   // d_tmp
 bool nd_walk_step_loop(const nd_sampler *s);   // the load-balanced mode takes the step loop over sorted maps (its switches are set)
+bool nd_walk_lane_per_walk(const nd_sampler *s, int mode);   // a job in this mode leaves d_tmp and the transit maps alone
 int nd_walk_sample(nd_sampler *s, int mode);
 int nd_khop_alloc(nd_sampler *s);
 int nd_khop_sample(nd_sampler *s, int mode);

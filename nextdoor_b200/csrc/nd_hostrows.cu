@@ -16,6 +16,10 @@
 // Where the GPU can reach the caller's array and lengths (pinned memory) it writes a share of the rows itself, while the
 // host threads write the others: the threads are bound by a cache line of the array or two per row, the GPU by the wire,
 // and neither takes the other's time (2^21 rows of PPR: 2.3 ms by 16 threads, 2.2 by the GPU).
+//
+// An update lives on what begin has packed: from then on the sampler's result may change, and its next job neither
+// waits for the host nor is waited for.  (Except where the job writes the staging array that the packed rows lie in, as the
+// transit-parallel modes do: nd_hostrows_next_job.)
 #include <algorithm>
 
 #include <cuda.h>
@@ -36,9 +40,12 @@ struct NdHostRows {
   int32_t *out = nullptr, *row_len = nullptr;
   int64_t total = 0;
   uint32_t *h_chunk = nullptr;  // pinned: d_chunk of the job being copied
+  bool moved = false;           // the sampler's result may be another job's by now
+  bool ahead = false;           // fetched by the sampler's next job, the caller's fetch is still to come
   bool dense = false;           // most slots are in use: the dense array is copied as it is
   int stage = 0;                // 0 idle, 1 begun, 2 fetched
   int64_t direct = 0;           // rows from the front that the GPU writes
+  uint32_t *d_pos = nullptr;    // ... [direct + 1]: where each of them begins in the packed array
   int32_t *dev_out = nullptr, *dev_row_len = nullptr;   // ... where it finds the caller's arrays
   cudaStream_t ds = nullptr;    // ... and the stream it does it on
   int threads = 1;
@@ -58,9 +65,7 @@ struct WarpRows {
   uint32_t total;       // of the warp
   size_t pos;           // of the warp's first vertex
 
-  // `block`: the CTA's place among those of all rows; the packed array begins with the rows of chunk `chunk0`
-  __device__ __forceinline__ WarpRows(const int32_t *__restrict__ lens, int64_t row, int64_t S, const uint32_t *__restrict__ chunk_base, uint32_t *wsum,
-                                      uint32_t block, uint32_t chunk0) {
+  __device__ __forceinline__ WarpRows(const int32_t *__restrict__ lens, int64_t row, int64_t S, const uint32_t *__restrict__ chunk_base, uint32_t *wsum) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     len = row < S ? (uint32_t)lens[row] : 0u;
     inc = len;
@@ -71,12 +76,12 @@ struct WarpRows {
     total = __shfl_sync(0xffffffffu, inc, 31);
     // the rows of the chunk before the CTA's: a few loads that neighbouring CTAs share
     uint32_t before = 0;
-    for (int64_t r = (int64_t)(block / (PACK_CHUNK / PACK_ROWS)) * PACK_CHUNK + threadIdx.x; r < (int64_t)block * PACK_ROWS; r += PACK_ROWS)
+    for (int64_t r = (int64_t)(blockIdx.x / (PACK_CHUNK / PACK_ROWS)) * PACK_CHUNK + threadIdx.x; r < (int64_t)blockIdx.x * PACK_ROWS; r += PACK_ROWS)
       before += (uint32_t)lens[r];
     before = __reduce_add_sync(0xffffffffu, before);
     if (lane == 0) { wsum[warp] = total; wsum[PACK_ROWS / 32 + warp] = before; }
     __syncthreads();
-    pos = chunk_base[block / (PACK_CHUNK / PACK_ROWS)] - chunk_base[chunk0];
+    pos = chunk_base[blockIdx.x / (PACK_CHUNK / PACK_ROWS)];
     for (int w = 0; w < PACK_ROWS / 32; w++) pos += wsum[PACK_ROWS / 32 + w] + (w < warp ? wsum[w] : 0u);
   }
   // fn(lane of the row, slot in the row, place in the warp's packed vertices)
@@ -145,7 +150,7 @@ unpack_rows_kernel(const int32_t *__restrict__ len, const int32_t *__restrict__ 
                    int64_t S, int steps, int32_t invalid, int32_t *__restrict__ out, int32_t *__restrict__ row_len) {
   __shared__ uint32_t wsum[PACK_ROWS / 16];
   const int64_t mine = (int64_t)blockIdx.x * PACK_ROWS + threadIdx.x, first = mine - (threadIdx.x & 31);
-  const WarpRows rows(len, mine, S, chunk_base, wsum, blockIdx.x, 0u);
+  const WarpRows rows(len, mine, S, chunk_base, wsum);
   rows.each([&](int r, uint32_t slot, uint32_t k) { out[(first + r) * steps + slot] = vals[rows.pos + k]; });
   if (mine >= S) return;
   const int32_t had = row_len[mine];
@@ -153,33 +158,36 @@ unpack_rows_kernel(const int32_t *__restrict__ len, const int32_t *__restrict__ 
   if (had != (int)rows.len) row_len[mine] = (int32_t)rows.len;
 }
 
-// the prefixes of the rows from chunk `chunk0` on to vals, back to back
+// the prefixes of the rows to vals, back to back, and where the first `placed` rows and the one behind them begin there
 __global__ void __launch_bounds__(PACK_ROWS)
 pack_rows_kernel(const int32_t *__restrict__ plen, const int32_t *__restrict__ out, int64_t S, int steps,
-                 const uint32_t *__restrict__ chunk_base, uint32_t chunk0, int32_t *__restrict__ vals) {
+                 const uint32_t *__restrict__ chunk_base, int64_t placed, uint32_t *__restrict__ place, int32_t *__restrict__ vals) {
   __shared__ uint32_t wsum[PACK_ROWS / 16];
-  const uint32_t block = blockIdx.x + chunk0 * (PACK_CHUNK / PACK_ROWS);
-  const int64_t mine = (int64_t)block * PACK_ROWS + threadIdx.x, first = mine - (threadIdx.x & 31);
-  const WarpRows rows(plen, mine, S, chunk_base, wsum, block, chunk0);
+  const int64_t mine = (int64_t)blockIdx.x * PACK_ROWS + threadIdx.x, first = mine - (threadIdx.x & 31);
+  const WarpRows rows(plen, mine, S, chunk_base, wsum);
+  if (placed > 0 && mine <= placed) place[mine] = (uint32_t)rows.pos + rows.inc - rows.len;
   rows.each([&](int r, uint32_t slot, uint32_t k) { vals[rows.pos + k] = out[(first + r) * steps + slot]; });
 }
 
-// The first `n` rows of the sampler's array into the caller's: the 64-byte lines of every row that hold a slot a walk fills
-// now or filled at the array's previous update, whole, as the sampler's array holds the invalid id behind a row's
-// vertices too.  Bound by the wire: 1.1 M rows of 2^21 are 1.8 M lines, 2.2 ms at 52 GB/s; the vertices alone
-// are 1.5 M writes of 4 to 32 bytes and take 2.9, their 32-byte sectors 2.4.  Two lanes to a line; 128 threads of 32
-// registers find room beside the kernel that samples the next chunk.
+// The first `n` rows of the packed array into the caller's: the 64-byte lines of every row that hold a slot a walk fills
+// now or filled at the array's previous update, whole (what lies behind a row's vertices is the invalid id, in the
+// neighbouring rows of a line as well).  Bound by the wire: 1.1 M rows of 2^21 are 1.8 M lines, 2.2 ms at 52 GB/s; the
+// vertices alone are 1.5 M writes of 4 to 32 bytes and take 2.9, their 32-byte sectors 2.4.  Two lanes to a line; 128
+// threads of 32 registers find room beside the kernel that samples the next chunk.
 constexpr int DIRECT_THREADS = 128;
 __global__ void __launch_bounds__(DIRECT_THREADS, 16)
-direct_rows_kernel(const int32_t *__restrict__ plen, const int32_t *__restrict__ from, int64_t n, int steps, int32_t *out, int32_t *row_len) {
+direct_rows_kernel(const uint32_t *__restrict__ pos, const int32_t *__restrict__ vals, uint32_t n, uint32_t steps, int32_t invalid, int32_t *out,
+                   int32_t *row_len) {
   const int lane = threadIdx.x & 31;
-  const int64_t shift = (int64_t)((uintptr_t)out / 4 % 16);   // the array begins that many slots into a line
-  for (int64_t first = (int64_t)blockIdx.x * DIRECT_THREADS + threadIdx.x - lane; first < n; first += (int64_t)gridDim.x * DIRECT_THREADS) {
-    const int64_t mine = first + lane;
-    const int32_t now = mine < n ? plen[mine] : 0, had = mine < n ? row_len[mine] : 0, len = now > had ? now : had;
+  // places are counted from the line that the array begins in (32-bit: n * steps is at most 16/17 of 2^32, see direct_rows)
+  const uint32_t begin = (uint32_t)((uintptr_t)out / 4 % 16), end = begin + n * steps;
+  for (uint32_t first = blockIdx.x * DIRECT_THREADS + threadIdx.x - lane; first < n; first += gridDim.x * DIRECT_THREADS) {
+    const uint32_t mine = first + lane;
+    const int32_t now = mine < n ? (int32_t)(pos[mine + 1] - pos[mine]) : 0, had = mine < n ? row_len[mine] : 0;
+    const uint32_t len = min((uint32_t)max(now, had), steps);
     if (__any_sync(0xffffffffu, now != had) && mine < n) row_len[mine] = now;
-    const int64_t line0 = (mine * steps + shift) / 16;
-    const uint32_t lines = len > 0 ? (uint32_t)((mine * steps + len - 1 + shift) / 16 - line0) + 1u : 0u;
+    const uint32_t line0 = (begin + mine * steps) / 16;
+    const uint32_t lines = len > 0 ? (begin + mine * steps + len - 1) / 16 - line0 + 1u : 0u;
     uint32_t inc = lines;
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
@@ -192,19 +200,32 @@ direct_rows_kernel(const int32_t *__restrict__ plen, const int32_t *__restrict__
 #pragma unroll
       for (int step = 16; step > 0; step >>= 1)
         if (__shfl_sync(0xffffffffu, inc, r + step - 1) <= k) r += step;
-      const int64_t line = __shfl_sync(0xffffffffu, line0 - (int64_t)(inc - lines), r & 31) + k;
-      if (k >= total) continue;
-      const int64_t at = line * 16 + lane % 2 * 8 - shift;   // eight slots
-      if (at >= 0 && at + 8 <= n * steps) {
-        int32_t v[8];
+      const uint32_t line = __shfl_sync(0xffffffffu, line0 - (inc - lines), r & 31) + k;
+      const uint32_t at = line * 16 + lane % 2 * 8;   // eight places, of rows that may begin and end anywhere in them
+      if (k >= total || at >= end || at + 8 <= begin) continue;
+      const uint32_t slot0 = at > begin ? at - begin : 0u;
+      uint32_t row = slot0 / steps, slot = slot0 - row * steps, p = pos[row], behind = pos[row + 1];
+      int32_t v[8];
 #pragma unroll
-        for (int j = 0; j < 8; j++) v[j] = from[at + j];
-        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(out + at), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]),
+      for (int j = 0; j < 8; j++) {
+        v[j] = invalid;
+        if (at + j < begin || at + j >= end) continue;
+        if (slot < behind - p) v[j] = vals[p + slot];
+        if (++slot == steps) {
+          slot = 0u;
+          p = behind;
+          if (++row < n) behind = pos[row + 1];
+        }
+      }
+      int32_t *const to = out - begin + at;
+      if (at >= begin && at + 8 <= end) {
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(to), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]),
                      "r"(v[5]), "r"(v[6]), "r"(v[7])
                      : "memory");
       } else {
+#pragma unroll
         for (int j = 0; j < 8; j++)
-          if (at + j >= 0 && at + j < n * steps) out[at + j] = from[at + j];
+          if (at + j >= begin && at + j < end) to[j] = v[j];
       }
     }
   }
@@ -269,24 +290,26 @@ bool find_rows(nd_sampler *s) {
 
 // The rows that the GPU writes itself, whole chunks from the front: as fast as 16 host threads (above).  The host's memory
 // serves both, so that they are not twice as fast together: jobs of 2^21 rows 3.2 -> 2.4 ms with half of them, 2.8 with
-// a third and with all, 2.7 with three quarters.
+// a third and with all, 2.7 with three quarters.  None where a caller has captured a job, whose replays may come at any time.
 int64_t direct_rows(nd_sampler *s, int32_t *out, int32_t *row_len) {
   NdHostRows *h = s->hostrows;
   if (s->S < 4 * PACK_CHUNK || s->in_graph || (uintptr_t)out % 4 || (uintptr_t)row_len % 4) return 0;
   if (!find_rows(s)) return 0;
+  const int64_t n = s->S * 16 / (16 + h->threads) / PACK_CHUNK * PACK_CHUNK;
+  if (n == 0) return 0;
   if (!h->ds && cudaStreamCreateWithFlags(&h->ds, cudaStreamNonBlocking) != cudaSuccess) { cudaGetLastError(); h->ds = nullptr; return 0; }
-  return s->S * 16 / (16 + h->threads) / PACK_CHUNK * PACK_CHUNK;
+  if (!h->d_pos && nd_malloc(&h->d_pos, sizeof(uint32_t) * ((size_t)n + 1)) != cudaSuccess) { cudaGetLastError(); h->d_pos = nullptr; return 0; }
+  return n;
 }
 
-// the prefixes of the rows from `first` on (a chunk's) packed into the staging array of the walk (free between two
-// passes), on the sampler's stream
-int pack_enqueue(nd_sampler *s, int64_t first) {
+// the prefixes of the rows packed into the staging array of the walk (free between two passes), on the sampler's stream
+int pack_enqueue(nd_sampler *s, int64_t placed) {
   NdHostRows *h = s->hostrows;
   ND_TRY(nd_walk_ensure_tmp(s));
   pack_sum_kernel<<<h->n_chunks, PACK_ROWS, 0, s->stream>>>(s->d_plen, s->S, h->d_chunk);
   pack_scan_kernel<<<1, 1024, 0, s->stream>>>(h->d_chunk, h->n_chunks);
-  pack_rows_kernel<<<(unsigned)((s->S - first + PACK_ROWS - 1) / PACK_ROWS), PACK_ROWS, 0, s->stream>>>(s->d_plen, s->d_out, s->S, s->fs, h->d_chunk,
-                                                                                                       (uint32_t)(first / PACK_CHUNK), s->d_tmp);
+  pack_rows_kernel<<<(unsigned)((s->S + PACK_ROWS - 1) / PACK_ROWS), PACK_ROWS, 0, s->stream>>>(s->d_plen, s->d_out, s->S, s->fs, h->d_chunk, placed, h->d_pos,
+                                                                                               s->d_tmp);
   nd_count_launches(3);
   ND_CUDA(cudaGetLastError());
   return ND_OK;
@@ -295,7 +318,7 @@ int pack_enqueue(nd_sampler *s, int64_t first) {
 // the packed vertices to the host, once the chunks' sums are there
 int fetch_vals(nd_sampler *s, cudaStream_t st) {
   NdHostRows *h = s->hostrows;
-  const size_t n = (size_t)h->total - h->h_chunk[h->direct / PACK_CHUNK];
+  const size_t first = h->h_chunk[h->direct / PACK_CHUNK], n = (size_t)h->total - first;
   if (n > h->vals_cap) {
     if (h->h_vals) ND_CUDA(cudaFreeHost(h->h_vals));
     h->h_vals = nullptr;
@@ -304,28 +327,47 @@ int fetch_vals(nd_sampler *s, cudaStream_t st) {
     ND_CUDA(cudaMallocHost(&h->h_vals, sizeof(int32_t) * cap));
     h->vals_cap = cap;
   }
-  if (n > 0) ND_CUDA(cudaMemcpyAsync(h->h_vals, s->d_tmp, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
+  if (n > 0) ND_CUDA(cudaMemcpyAsync(h->h_vals, s->d_tmp + first, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st));
+  return ND_OK;
+}
+
+// The rows of a fetched update that the GPU was to write go to the host threads, too.
+int rows_to_host(nd_sampler *s) {
+  NdHostRows *h = s->hostrows;
+  const int64_t n = h->direct;
+  const bool ahead = h->ahead;
+  h->stage = 0;   // an error below abandons the update
+  h->ahead = false;
+  ND_CUDA(cudaEventSynchronize(h->vals_done));
+  h->direct = 0;
+  ND_TRY(fetch_vals(s, h->vs));
+  ND_CUDA(cudaMemcpyAsync(h->h_len, h->d_pos, sizeof(uint32_t) * (size_t)n, cudaMemcpyDeviceToHost, h->vs));
+  ND_CUDA(cudaStreamSynchronize(h->vs));
+  uint32_t end = h->h_chunk[n / PACK_CHUNK];
+  for (int64_t i = n - 1; i >= 0; i--) {
+    const uint32_t pos = (uint32_t)h->h_len[i];
+    h->h_len[i] = (int32_t)(end - pos);
+    end = pos;
+  }
+  h->stage = 2;
+  h->ahead = ahead;
   return ND_OK;
 }
 
 }  // namespace
 
-// The sampler's array is about to change while the GPU has rows of it left to write, or the GPU no longer reaches the
-// array: these rows go to the host threads, too.
-int nd_hostrows_keep(nd_sampler *s) {
+// The sampler's next job is about to be enqueued.  An update in between only has to know, unless the job writes the array
+// that the packed rows lie in (`staging`) or there are none (a result too large for them): then what is not on its way
+// to the host yet is sent there first.
+int nd_hostrows_next_job(nd_sampler *s, bool staging) {
   NdHostRows *h = s->hostrows;
-  if (!h || h->stage == 0 || h->direct == 0) return ND_OK;
-  const int stage = h->stage;
-  h->stage = 0;   // an error below abandons the update
-  ND_CUDA(cudaEventSynchronize(h->len_done));
-  if (stage == 2) ND_CUDA(cudaEventSynchronize(h->vals_done));
-  h->direct = 0;
-  h->total = (int64_t)h->h_chunk[h->n_chunks];
-  ND_TRY(pack_enqueue(s, 0));
-  ND_CUDA(cudaMemcpyAsync(h->h_len, s->d_plen, sizeof(int32_t) * (size_t)s->S, cudaMemcpyDeviceToHost, s->stream));
-  if (stage == 2) ND_TRY(fetch_vals(s, s->stream));
-  ND_CUDA(cudaStreamSynchronize(s->stream));
-  h->stage = stage;
+  if (!h || h->stage == 0) return ND_OK;
+  if (h->stage == 1 && (staging || !packable(s))) {
+    ND_TRY(nd_sampler_host_update_fetch(s));
+    h->ahead = true;
+  }
+  if (staging && h->direct) ND_TRY(rows_to_host(s));
+  h->moved = true;
   return ND_OK;
 }
 
@@ -336,6 +378,7 @@ void nd_hostrows_free(nd_sampler *s) {
   if (h->h_vals) cudaFreeHost(h->h_vals);
   if (h->h_chunk) cudaFreeHost(h->h_chunk);
   cudaFree(h->d_chunk);
+  cudaFree(h->d_pos);
   if (h->vs) cudaStreamDestroy(h->vs);
   if (h->ds) cudaStreamDestroy(h->ds);
   if (h->packed) cudaEventDestroy(h->packed);
@@ -371,6 +414,7 @@ int nd_sampler_host_update_begin(nd_sampler *s, int32_t *out, int32_t *row_len, 
   h->cs = copy_stream ? (cudaStream_t)copy_stream : s->stream;
   if (s->S == 0) { h->stage = 1; return ND_OK; }
   // (an error below leaves stage 0: nothing was begun as far as the caller is concerned)
+  h->moved = s->in_graph;
   h->direct = packable(s) ? direct_rows(s, out, row_len) : 0;
   if (packable(s)) ND_TRY(pack_enqueue(s, h->direct));   // (larger arrays take the dense copy in fetch)
   if (h->cs != s->stream) {
@@ -392,8 +436,9 @@ int nd_sampler_host_update_begin(nd_sampler *s, int32_t *out, int32_t *row_len, 
 }
 
 int nd_sampler_host_update_fetch(nd_sampler *s) {
-  ND_REQUIRE(s && s->hostrows && s->hostrows->stage == 1, ND_ERR_STATE, "nd_sampler_host_update_fetch without a begun update");
+  ND_REQUIRE(s && s->hostrows && (s->hostrows->stage == 1 || s->hostrows->ahead), ND_ERR_STATE, "nd_sampler_host_update_fetch without a begun update");
   NdHostRows *h = s->hostrows;
+  if (h->ahead) { h->ahead = false; return ND_OK; }
   h->stage = 0;   // an error below abandons the update; stage 2 is set once the copy is enqueued
   h->total = 0;
   h->dense = false;
@@ -401,7 +446,7 @@ int nd_sampler_host_update_fetch(nd_sampler *s) {
   ND_CUDA(cudaSetDevice(s->g->device));
   ND_CUDA(cudaEventSynchronize(h->len_done));
   if (packable(s)) h->total = (int64_t)h->h_chunk[h->n_chunks];
-  h->dense = 2 * h->total > s->S * (int64_t)s->fs || !packable(s);
+  h->dense = (2 * h->total > s->S * (int64_t)s->fs && !h->moved) || !packable(s);
   if (h->dense) {
     ND_CUDA(cudaMemcpyAsync(h->out, s->d_out, sizeof(int32_t) * (size_t)s->S * s->fs, cudaMemcpyDeviceToHost, h->vs));
     if (h->direct) ND_CUDA(cudaMemcpyAsync(h->h_len, s->d_plen, sizeof(int32_t) * (size_t)h->direct, cudaMemcpyDeviceToHost, h->vs));
@@ -422,9 +467,10 @@ int nd_sampler_host_update_finish(nd_sampler *s, int64_t *values_copied) {
   ND_REQUIRE(s && s->hostrows && s->hostrows->stage >= 1, ND_ERR_STATE, "nd_sampler_host_update_finish without a begun update");
   NdHostRows *h = s->hostrows;
   if (h->stage == 1) ND_TRY(nd_sampler_host_update_fetch(s));
-  if (h->direct && !find_rows(s)) ND_TRY(nd_hostrows_keep(s));   // (unregistered since the update was begun)
+  if (h->direct && !find_rows(s)) ND_TRY(rows_to_host(s));   // (unregistered since the update was begun)
   ND_REQUIRE(h->stage == 2, ND_ERR_STATE, "nd_sampler_host_update_finish: the update was abandoned after an error");
   h->stage = 0;
+  h->ahead = false;
   if (values_copied) *values_copied = h->dense ? s->S * (int64_t)s->fs : h->total;
   if (s->S == 0) return ND_OK;
   ND_CUDA(cudaSetDevice(s->g->device));
@@ -444,7 +490,7 @@ int nd_sampler_host_update_finish(nd_sampler *s, int64_t *values_copied) {
   const cudaStream_t ds = h->ds;
   if (direct) {
     const int grid = (int)std::min<int64_t>((direct + DIRECT_THREADS - 1) / DIRECT_THREADS, (int64_t)s->dev.sms * 4);
-    direct_rows_kernel<<<grid, DIRECT_THREADS, 0, ds>>>(s->d_plen, s->d_out, direct, steps, h->dev_out, h->dev_row_len);
+    direct_rows_kernel<<<grid, DIRECT_THREADS, 0, ds>>>(h->d_pos, s->d_tmp, (uint32_t)direct, (uint32_t)steps, invalid, h->dev_out, h->dev_row_len);
     nd_count_launches(1);
     ND_CUDA(cudaGetLastError());
   }

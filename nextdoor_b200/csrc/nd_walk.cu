@@ -1033,6 +1033,10 @@ bool step_loop(const nd_sampler *s) {
 
 bool nd_walk_step_loop(const nd_sampler *s) { return step_loop(s); }
 
+bool nd_walk_lane_per_walk(const nd_sampler *s, int mode) {
+  return mode == ND_MODE_SAMPLE_PARALLEL || (mode == ND_MODE_TRANSIT_PARALLEL_LB && !step_loop(s));
+}
+
 namespace {
 __device__ int g_step_status;                       // device status word of nd_walk_step
 
@@ -1381,9 +1385,9 @@ static int walk_enqueue(nd_sampler *s, int mode) {
 }
 
 int nd_walk_sample(nd_sampler *s, int mode) {
-  const bool loop = mode == ND_MODE_TRANSIT_PARALLEL_LB && step_loop(s);
-  s->live_is_ended = mode == ND_MODE_TRANSIT_PARALLEL_LB && !loop;
-  if (mode == ND_MODE_SAMPLE_PARALLEL || s->live_is_ended) {   // a lane per walk: one or two launches, nothing to capture
+  const bool rows = nd_walk_lane_per_walk(s, mode), loop = mode == ND_MODE_TRANSIT_PARALLEL_LB && !rows;
+  s->live_is_ended = mode == ND_MODE_TRANSIT_PARALLEL_LB && rows;
+  if (rows) {   // a lane per walk: one or two launches, nothing to capture
     nd_phase_begin(s, ND_PHASE_NEXT);
     const int rc = nd_walk_rows_launch(s, mode == ND_MODE_TRANSIT_PARALLEL_LB);
     nd_phase_end(s);

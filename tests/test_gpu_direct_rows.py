@@ -99,3 +99,87 @@ def test_rows_that_the_gpu_may_no_longer_write(nd, small_graph, step):
         assert int(rt.cudaHostUnregister(out.ctypes.data)) == 0
     assert np.array_equal(out.reshape(S, steps), expected)
     assert np.array_equal(row_len, (expected != g.V).sum(axis=1))
+
+
+def _update(nd, g, S, steps, stop, pinned, app=2):
+    s = nd.Sampler(g, nd.app_params(app, steps=steps, seed=5, stop_prob=stop), num_samples=S)
+    out, row_len = (_pinned(S * steps, 0, g.V), _pinned(S, 0, 0)) if pinned else (np.full(S * steps, g.V, np.int32), np.zeros(S, np.int32))
+    return s, out, row_len
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("stop,mode,then", [(0.2, 1, 1), (0.2, 2, 0), (0.2, 0, 0), (0.0005, 1, 1), (0.0005, 1, 2), (0.0005, 0, 0)])
+@pytest.mark.parametrize("between", ["begin and fetch", "fetch and finish"])
+def test_the_next_job_at_any_time(nd, small_graph, pinned, stop, mode, then, between):
+    """... in a mode that writes the array that the packed rows lie in, and with rows that are mostly full."""
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    S, steps, rng = 20_000, 40, np.random.default_rng(3)
+    s, out, row_len = _update(nd, g, S, steps, stop, pinned)
+    for _ in range(3):
+        s.set_initial(rng.integers(0, g.V, S).astype(np.int32))
+        s.sample(mode)
+        expected = s.final_samples().copy()
+        s.host_update_begin(out, row_len)
+        if between == "fetch and finish":
+            s.host_update_fetch()
+        s.set_initial(rng.integers(0, g.V, S).astype(np.int32))
+        s.sample(then, sync=False)
+        if between == "begin and fetch":
+            s.host_update_fetch()
+        s.sync()
+        s.host_update_finish()
+        assert np.array_equal(out.reshape(S, steps), expected)
+        assert np.array_equal(row_len, (expected != g.V).sum(axis=1))
+
+
+@pytest.mark.parametrize("copy_stream", [False, True])
+def test_the_next_job_does_not_wait_on_the_host(nd, small_graph, copy_stream):
+    import time
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    S, steps, rng = 1 << 15, 40, np.random.default_rng(3)
+    s, out, row_len = _update(nd, g, S, steps, 0.2, True)
+    streams = torch.cuda.Stream(), torch.cuda.Stream()
+    s.set_stream(streams[0].cuda_stream)
+    seeds = [torch.from_numpy(rng.integers(0, g.V, S).astype(np.int32)).pin_memory().numpy() for _ in range(2)]
+    for job in range(2):                                  # the second: everything is loaded and allocated
+        s.set_initial(seeds[0])
+        s.sample(1)
+        expected = s.final_samples().copy()
+        with torch.cuda.stream(streams[0]):
+            torch.cuda._sleep(500_000_000)                # a quarter of a second
+        start = time.perf_counter()
+        s.host_update_begin(out, row_len, streams[1].cuda_stream if copy_stream else None)
+        s.set_initial(seeds[1])
+        s.sample(1, sync=False)
+        took = time.perf_counter() - start
+        assert not streams[0].query() and (job == 0 or took < 0.1), took
+        s.host_update_fetch()
+        s.host_update_finish()
+        s.sync()
+        assert np.array_equal(out.reshape(S, steps), expected)
+
+
+def test_a_job_is_captured_while_an_update_is_open(nd, small_graph):
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    S, steps, rng = 1 << 15, 40, np.random.default_rng(3)
+    s, out, row_len = _update(nd, g, S, steps, 0.2, True)
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    s.set_stream(stream.cuda_stream)
+    first, second = (rng.integers(0, g.V, S).astype(np.int32) for _ in range(2))
+    s.set_initial(first)
+    s.sample(1)
+    expected = s.final_samples().copy()
+    s.host_update_begin(out, row_len)
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+        s.sample(1, sync=False)
+    s.set_initial(second)
+    with torch.cuda.stream(stream):
+        graph.replay()
+    s.sync()
+    replayed = s.final_samples().copy()
+    assert not np.array_equal(replayed, expected)
+    s.host_update_finish()
+    assert np.array_equal(out.reshape(S, steps), expected)
+    s.host_update_begin(out, row_len)
+    s.host_update_finish()
+    assert np.array_equal(out.reshape(S, steps), replayed)
