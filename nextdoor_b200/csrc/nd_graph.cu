@@ -602,11 +602,6 @@ int nd_graph_from_edges(int device, int64_t n, const int32_t *src, const int32_t
     nd_count_launches(1);
     return build_from_facts(dev, n, 0, &bs, out);
   }
-  // (the weights' arrival does not touch what the sorts work on: a block of its own)
-  BuildScratch weights;
-  weights.device = device;
-  weights.bytes = 4 * (size_t)n;
-  ND_TRY(nd_block_alloc(device, (void **)&weights.base, &weights.bytes));
   ND_TRY(nd_copies_to_device(device, 2, to, from, bytes));
   id_facts_kernel<<<grid_for(n, 256, dev.sms), 256>>>(n, bs.a[0], bs.a[1], bs.a[2], bs.facts);
   nd_count_launches(1);
@@ -618,8 +613,9 @@ int nd_graph_from_edges(int device, int64_t n, const int32_t *src, const int32_t
   Build b(dev, n, V, &bs);
   ND_TRY(b.sort_by_ids());
   ND_TRY(b.csr());
-  ND_TRY(nd_copy_to_device(device, weights.base, w, bytes[2]));
-  place_weights_kernel<<<grid_for(n, 256, dev.sms), 256>>>(n, b.cur[2], (const float *)weights.base, b.oth[2], bs.facts);
+  // they arrive in the graph's own array, which the sorts do not touch, and go from there to the sorted places as keys
+  ND_TRY(nd_copy_to_device(device, b.g->w, w, bytes[2]));
+  place_weights_kernel<<<grid_for(n, 256, dev.sms), 256>>>(n, b.cur[2], b.g->w, b.oth[2], bs.facts);
   std::swap(b.cur[2], b.oth[2]);
   nd_count_launches(1);
   ND_TRY(b.sort_weights(0, 32));

@@ -197,6 +197,29 @@ def pinned_rows():
     assert np.array_equal(out.reshape(S, steps), s.final_samples())
 
 
+# a load needs no more memory where its ids are sorted while the weights are on the wire, from 2^21 records on
+def loads():
+    from nextdoor_b200 import api as nd
+    rng, n, V = np.random.default_rng(1), 1 << 21, 1 << 18
+    src, dst, w = rng.integers(0, V, n).astype(np.int32), rng.integers(0, V, n).astype(np.int32), rng.random(n).astype(np.float32)
+    src[0] = V - 1
+    need = []
+    for k in (n - 1, n):
+        lo, hi = 0, 256
+        while hi - lo > 1:
+            mid = (lo + hi) // 2
+            fill = Filled(mid * MB)
+            try:
+                nd.Graph.from_edge_records(src[:k], dst[:k], w[:k]).free()
+                hi = mid
+            except nd.NdError as e:
+                assert "memory" in str(e), e
+                lo = mid
+            fill.free()
+        need.append(hi)
+    assert 60 < need[0] < 256 and need[1] <= need[0] + 4, need    # MB: three words a record twice, the graph; memory comes in pages of 2
+
+
 # What a first sampler builds only to be faster (the last of it: entries of 64 MB, ids of 48, tables of the hubs) and finds no
 # room for, it does without
 def without_the_last(app, vertices, edges, spare):
@@ -229,7 +252,7 @@ def test_a_sampler_without_room_for_what_is_optional(app, vertices, edges, spare
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("case", [f"first_samplers({app})" for app in (1, 3, 8, 9)]
-                         + [f"graphs_and_partitions('{what}')" for what in ("csr", "partition")] + ["kept_blocks()", "adjacency()", "pinned_rows()"])
+                         + [f"graphs_and_partitions('{what}')" for what in ("csr", "partition")] + ["kept_blocks()", "adjacency()", "pinned_rows()", "loads()"])
 def test_nothing_stays_behind(case):
     r = subprocess.run([sys.executable, os.path.abspath(__file__), case], capture_output=True, text=True, timeout=300, cwd=ROOT)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
