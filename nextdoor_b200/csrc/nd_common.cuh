@@ -125,8 +125,9 @@ struct nd_graph {
   mutable int2 *vrow = nullptr;        // [V] (row start, degree): one load per vertex
   mutable int4 *erec = nullptr;        // [E] (neighbour id, its row start, its degree, 0)
   mutable uint32_t *pack = nullptr;    // [E] neighbour id << 8 | weight as whole 256ths of the row's maximum
+  mutable uint8_t *codes = nullptr;    // [E] ... the weights alone, where there is no room for both
   mutable uint2 *col3 = nullptr;       // [E/3] three neighbour ids of 21 bits to 8 bytes
-  mutable int odd_max = -1;            // some row's maximum weight rules `pack` out (-1: not asked yet)
+  mutable int odd_max = -1;            // some row's maximum weight rules `pack` and `codes` out (-1: not asked yet)
   mutable int32_t *adjset = nullptr;   // node2vec membership: per-vertex hash sets of the neighbour ids, 8-slot buckets
   mutable uint32_t *adjsign = nullptr; // ... and the filter in front of them
   mutable uint4 *deg_codes = nullptr;  // degrees of eight vertices each (FastGCN)

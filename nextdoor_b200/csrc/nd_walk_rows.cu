@@ -43,6 +43,7 @@ struct RowsArgs {
   const int2 *__restrict__ colw;     // [E] (neighbour, weight bits)
   const int2 *__restrict__ vrec;     // [V+1] (row start, max weight bits)
   const uint32_t *__restrict__ pack; // [E] neighbour << 8 | weight as 256ths of the row's maximum, rounded down
+  const uint8_t *__restrict__ codes; // [E] the weights of `pack` alone
   const uint2 *__restrict__ col3;    // [E/3] three neighbours of 21 bits each
   const int32_t *__restrict__ adjset;
   const uint32_t *__restrict__ adjsign;
@@ -69,8 +70,9 @@ __host__ __device__ constexpr bool weighted() { return APP == ND_APP_DEEPWALK ||
 
 // Layouts of the entries.  ALT (weighted walks): id and weight in a word.  FAT (uniform, weighted walks): they carry the
 // neighbour's row, and the weight.  DENSE (uniform walk, node2vec): three ids of 21 bits in 8 bytes.  FAR: weighted walks as
-// ALT, node2vec as PLAIN, rows from the offsets.
-enum : int { LAYOUT_PLAIN = 0, LAYOUT_ALT = 1, LAYOUT_DENSE = 2, LAYOUT_FAR = 3, LAYOUT_FAT = 4 };
+// ALT, node2vec as PLAIN, rows from the offsets.  CODES (weighted walks): a byte of weight beside the ids, rows from the
+// offsets: what needs the least memory.
+enum : int { LAYOUT_PLAIN = 0, LAYOUT_ALT = 1, LAYOUT_DENSE = 2, LAYOUT_FAR = 3, LAYOUT_FAT = 4, LAYOUT_CODES = 5 };
 
 // ---- loads.  The small per-vertex and per-entry arrays ask to stay in the L2; the (id, weight) records, an array far
 // larger than the L2, bypass the L1.
@@ -282,7 +284,7 @@ __global__ void __launch_bounds__(256) walk_start_kernel(const __grid_constant__
 constexpr int32_t FAR_V = 1 << 22;
 template <int LAYOUT>
 __device__ __forceinline__ int2 row_of(const RowsArgs &a, const Hot &hot, int32_t v) {
-  if (LAYOUT != LAYOUT_FAR) return hot.ld(a.vrow + v);
+  if (LAYOUT != LAYOUT_FAR && LAYOUT != LAYOUT_CODES) return hot.ld(a.vrow + v);
   const int32_t at = hot.ld(a.row_ptr + v), end = hot.ld(a.row_ptr + v + 1);
   return make_int2(at, end - at);
 }
@@ -465,6 +467,8 @@ __device__ __forceinline__ void weighted_walks(const RowsArgs &a) {
       if (LAYOUT == LAYOUT_FAT) {
         const int4 r = hot.ld(a.erec + rs + x);
         id = (uint32_t)r.x; b = (uint32_t)r.w; row = make_int2(r.y, r.z);
+      } else if (LAYOUT == LAYOUT_CODES) {
+        id = 0u; b = __ldg(a.codes + rs + x);
       } else {
         const uint32_t r = __ldg(a.pack + rs + x);
         id = r >> 8; b = r & 255u;
@@ -472,7 +476,7 @@ __device__ __forceinline__ void weighted_walks(const RowsArgs &a) {
       bool accept = deg == 1 || u <= (float)b * 0.00390625f;
       if (!accept && (b == 255u || u < (float)(b + 1u) * 0.00390625f))
         accept = !(__fmul_rn(u, __ldg(a.max_w + mw)) > __ldg(a.w + rs + x));
-      if (accept) nbr = (int32_t)id;
+      if (accept) nbr = LAYOUT == LAYOUT_CODES ? __ldg(a.col + rs + x) : (int32_t)id;
     } else {
       const int2 r = ld_once(a.colw + rs + x);
       if (deg == 1 || !(__fmul_rn(u, __int_as_float(mw)) > __int_as_float(r.y))) nbr = r.x;
@@ -699,6 +703,12 @@ pack_build_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restrict
 }
 
 __global__ void __launch_bounds__(BUILD_THREADS)
+codes_build_kernel(const int32_t *__restrict__ row_ptr, const float *__restrict__ max_w, const float *__restrict__ w, int32_t V, int64_t E,
+                   uint8_t *__restrict__ codes) {
+  for_entries(row_ptr, V, E, [&](int64_t e, int32_t v) { codes[e] = (uint8_t)weight_code(w[e], max_w[v]); });
+}
+
+__global__ void __launch_bounds__(BUILD_THREADS)
 erec_build_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ col, const float *__restrict__ max_w, const float *__restrict__ w,
                   int32_t V, int64_t E, int4 *__restrict__ erec) {
   for_entries(row_ptr, V, E, [&](int64_t e, int32_t v) {
@@ -783,6 +793,7 @@ void launch_as(nd_sampler *s, RowsArgs &a, bool count) {
     case LAYOUT_FAT: return launch<APP, n2v ? LAYOUT_PLAIN : LAYOUT_FAT>(s, a, count);
     case LAYOUT_ALT: return launch<APP, w ? LAYOUT_ALT : LAYOUT_PLAIN>(s, a, count);
     case LAYOUT_DENSE: return launch<APP, w ? LAYOUT_PLAIN : LAYOUT_DENSE>(s, a, count);
+    case LAYOUT_CODES: return launch<APP, w ? LAYOUT_CODES : LAYOUT_PLAIN>(s, a, count);
     case LAYOUT_FAR: return launch<APP, w || n2v ? LAYOUT_FAR : LAYOUT_PLAIN>(s, a, count);
     default: return launch<APP, LAYOUT_PLAIN>(s, a, count);
   }
@@ -839,7 +850,30 @@ int ensure_erec(const nd_graph *g, int sms, bool *there) {
   return ND_OK;
 }
 
-// entries with rows, ids and weights in one word, or the records of ensure_colw where neither holds the weights
+int ensure_pack(const nd_graph *g, int sms, bool *there) {
+  *there = g->pack != nullptr;
+  if (g->pack) return ND_OK;
+  NdDevMem<uint32_t> pack;
+  if (pack.alloc((size_t)(g->E > 0 ? g->E : 1)) != ND_OK) return ND_OK;
+  pack_build_kernel<<<sms * 16, BUILD_THREADS>>>(g->row_ptr, g->col, g->max_w, g->w, g->V, g->E, pack.p);
+  ND_CUDA(cudaGetLastError());
+  g->pack = pack.release();
+  *there = true;
+  return ND_OK;
+}
+
+int ensure_codes(const nd_graph *g, int sms) {
+  if (g->codes) return ND_OK;
+  NdDevMem<uint8_t> codes;
+  ND_TRY(codes.alloc((size_t)(g->E > 0 ? g->E : 1)));
+  codes_build_kernel<<<sms * 16, BUILD_THREADS>>>(g->row_ptr, g->max_w, g->w, g->V, g->E, codes.p);
+  ND_CUDA(cudaGetLastError());
+  g->codes = codes.release();
+  return ND_OK;
+}
+
+// Entries with rows, ids and weights in one word, or the records of ensure_colw where a word does not hold the ids; a byte of
+// weight per entry where there is no room for those.  Rows whose weights are no codes have the records.
 int ensure_weighted(const nd_graph *g, int sms, int *layout) {
   if (g->odd_max < 0) {
     NdDevMem<int> flag;
@@ -852,18 +886,16 @@ int ensure_weighted(const nd_graph *g, int sms, int *layout) {
   }
   *layout = LAYOUT_PLAIN;
   if (g->odd_max == 1) return ensure_colw(g, sms);
-  bool fat = g->E <= ERECS;
-  if (fat) ND_TRY(ensure_erec(g, sms, &fat));
-  if (!fat && g->V > PACK_V) return ensure_colw(g, sms);
-  if (fat || g->V < FAR_V) ND_TRY(ensure_vrow(g, sms));
-  *layout = fat ? LAYOUT_FAT : g->V >= FAR_V ? LAYOUT_FAR : LAYOUT_ALT;
-  if (fat || g->pack) return ND_OK;
-  NdDevMem<uint32_t> pack;
-  ND_TRY(pack.alloc((size_t)(g->E > 0 ? g->E : 1)));
-  pack_build_kernel<<<sms * 16, BUILD_THREADS>>>(g->row_ptr, g->col, g->max_w, g->w, g->V, g->E, pack.p);
-  ND_CUDA(cudaGetLastError());
-  g->pack = pack.release();
-  return ND_OK;
+  const bool near = g->V < FAR_V;
+  bool there = false;
+  const bool rows = (near || g->E <= ERECS) && ensure_vrow(g, sms) == ND_OK;
+  if (rows && g->E <= ERECS) ND_TRY(ensure_erec(g, sms, &there));
+  if (there) { *layout = LAYOUT_FAT; return ND_OK; }
+  if (g->V <= PACK_V) ND_TRY(ensure_pack(g, sms, &there));
+  if (there) { *layout = rows && near ? LAYOUT_ALT : LAYOUT_FAR; return ND_OK; }
+  if (g->V > PACK_V && ensure_colw(g, sms) == ND_OK) return ND_OK;
+  *layout = LAYOUT_CODES;
+  return ensure_codes(g, sms);
 }
 
 int ensure_col3(const nd_graph *g, int sms, bool *there) {
@@ -933,7 +965,7 @@ int nd_walk_rows_alloc(nd_sampler *s) {
 int nd_walk_rows_launch(nd_sampler *s, bool count) {
   const nd_graph *g = s->g;
   uint32_t *ended = count ? reinterpret_cast<uint32_t *>(s->d_rows_acc + 16) : nullptr;
-  RowsArgs a{g->V, g->row_ptr, g->col, g->w, g->max_w, g->vrow, g->erec, g->colw, g->vrec, g->pack, g->col3, g->adjset, g->adjsign,
+  RowsArgs a{g->V, g->row_ptr, g->col, g->w, g->max_w, g->vrow, g->erec, g->colw, g->vrec, g->pack, g->codes, g->col3, g->adjset, g->adjsign,
              ndrng::RoundKeys(s->p.seed), s->p.p, s->p.q, s->p.stop_prob, s->p.n2v_ref_compat, s->p.steps, s->first, s->S, s->d_initial, s->d_out,
              s->d_plen, s->d_list, s->d_rows_acc, ended, s->d_stats, (uint32_t *)s->d_nlive, s->d_status};
   switch (s->p.app) {
