@@ -354,7 +354,8 @@ class PipelinedSampler:
         self.sets, self._job = [], 0
         # Walk jobs move only the rows' valid prefixes to the host (nd_sampler_host_update_*): the
         # per-row lengths of every host array this object has filled, by the array's address, and
-        # the jobs whose rows are still to be written (at most one per sampler set).
+        # the jobs whose rows are still to be written (at most one per sampler set): how far each is,
+        # and the array and lengths it is going to write, which stay alive with it.
         self.sparse_rows = sparse_rows and params.app <= APP_NODE2VEC
         self.invalid = graph.V
         self._row_len, self._pending = {}, {}
@@ -405,12 +406,16 @@ class PipelinedSampler:
         except Exception:
             self._end_updates(k)
             raise
-        self._pending[k] = "begun"
+        self._pending[k] = ["begun", out_host, row_len]
         for j in others:                                  # ... and its rows are written while the device works on this one
             self._finish(j)
 
+    @staticmethod
+    def _key(out_host):
+        return out_host.__array_interface__["data"][0], out_host.size
+
     def _rows_of(self, out_host):
-        key = (out_host.__array_interface__["data"][0], out_host.size)
+        key = self._key(out_host)
         if key not in self._row_len:
             host_fill(out_host, self.invalid)
             try:
@@ -420,11 +425,17 @@ class PipelinedSampler:
         return self._row_len[key]
 
     def forget(self, out_host):
-        """The caller is going to write to `out_host` itself: the next job into it starts from a fresh fill."""
-        self._row_len.pop((out_host.__array_interface__["data"][0], out_host.size), None)
+        """The caller is going to write to `out_host` itself: the next job into it starts from a fresh fill.  A job
+        whose rows are still to be written there is finished first."""
+        key = self._key(out_host)
+        try:
+            for k in [k for k, job in self._pending.items() if self._key(job[1]) == key]:
+                self._finish(k)
+        finally:
+            self._row_len.pop(key, None)
 
     def _fetch(self, k):
-        if self._pending.get(k) == "begun":
+        if k in self._pending and self._pending[k][0] == "begun":
             try:
                 for _, _, smp in self.sets[k]:
                     smp.host_update_fetch()
@@ -432,11 +443,12 @@ class PipelinedSampler:
                 del self._pending[k]
                 self._end_updates(k)
                 raise
-            self._pending[k] = "fetched"
+            self._pending[k][0] = "fetched"
 
     def _finish(self, k):
         if k in self._pending:
-            fetched = self._pending.pop(k) == "fetched"
+            job = self._pending.pop(k)                     # (held until the rows are written)
+            fetched = job[0] == "fetched"
             parts = [smp for _, _, smp in self.sets[k]]
             total = 0
             try:

@@ -60,6 +60,31 @@ def test_pipeline_into_pinned_arrays(nd, small_graph, depth):
         assert np.array_equal(out.reshape(S, 40), whole.final_samples()), k
 
 
+@pytest.mark.parametrize("depth", [1, 2])
+@pytest.mark.parametrize("pinned", [False, True])
+def test_an_array_is_forgotten_while_its_rows_are_to_be_written(nd, small_graph, depth, pinned):
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    S, steps, rng = 70_001, 40, np.random.default_rng(depth)
+    pr = nd.app_params(2, steps=steps, seed=9, stop_prob=0.15)
+    outs = [_pinned(S * steps, 0, 0) if pinned else np.zeros(S * steps, np.int32) for _ in range(2)]
+    pipe = nd.PipelinedSampler(g, pr, S, chunks=3, depth=depth, sparse_rows=True)
+    whole = nd.Sampler(g, pr, num_samples=S)
+    for job in range(6):
+        out, init = outs[job % 2], rng.integers(0, g.V, S).astype(np.int32)
+        whole.set_initial(init)
+        whole.sample(1)
+        pipe.run_async(init, out)
+        if job in (1, 2, 4):
+            pipe.forget(out)                              # the rows are there, and what the caller writes stays
+            assert np.array_equal(out.reshape(S, steps), whole.final_samples())
+            out[:] = -3
+            pipe.wait()
+            assert (out == -3).all()
+        else:
+            pipe.wait()
+            assert np.array_equal(out.reshape(S, steps), whole.final_samples())
+
+
 @pytest.mark.parametrize("step", ["unregistered", "replayed"])
 def test_rows_that_the_gpu_may_no_longer_write(nd, small_graph, step):
     """Between the begin and the finish of an update the array stops being pinned, or a captured job runs again."""
