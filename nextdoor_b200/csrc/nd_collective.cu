@@ -371,6 +371,8 @@ coll_sample_kernel(NdGraphView g, CollParams cp, int steps, int64_t s0, int64_t 
           const int64_t mid = lo + (hi - lo) / 2;
           if (cdf[base + mid] >= target) hi = mid; else lo = mid + 1;
         }
+        // (by rounding one behind a candidate, of weight zero or the candidate's id again)
+        while (lo > 0 && !(wt[base + lo] > 0.f)) lo--;
         pick = (int32_t)c_id[base + lo];
         pr = (float)((double)wt[base + lo] / total);
         valid++;

@@ -227,9 +227,11 @@ def test_ladies_draws_end_where_there_are_candidates(nd, ndo, monkeypatch, V, sc
 
 
 @pytest.mark.parametrize("V", [3600, 200_000])
-def test_ladies_draws_no_neighbour_of_weight_zero(nd, ndo, V):
+@pytest.mark.parametrize("sort", ["0", "1"])
+def test_ladies_draws_no_neighbour_of_weight_zero(nd, ndo, monkeypatch, V, sort):
     """Groups of a dozen candidates with weights over eight decades, between and behind them neighbours that cannot be drawn."""
-    for seed in range(60):
+    monkeypatch.setenv("ND_COLLECTIVE_SORT", sort)
+    for seed in range(190):
         rng = np.random.default_rng(seed)
         ids = np.sort((128 * rng.permutation(V // 128 - 2)[:8, None] + rng.permutation(60)[:12]).reshape(-1))
         w = 10 ** rng.uniform(-8, 0, len(ids))
