@@ -168,10 +168,6 @@ int check_params(const nd_app_params *p) {
 
 }  // namespace
 
-namespace {
-
-}  // namespace
-
 extern "C" {
 
 const char *nd_last_error(void) { return g_err; }

@@ -40,7 +40,7 @@ constexpr int CTHREADS = 256;
 // first and all their (transit, layer) pairs are probed together: the transits' lists are flattened over the
 // CTA, every entry asks a filter of the layer's ids in shared memory, and the few that pass look for the id.
 // A list longer than PROBE_RATIO times the layer is bisected for every id instead.  (One bisection per
-// (transit, slot) pair, 205 M of them for 10,000 samples of 5 x 64 x 64 on 57 K vertices: 1.04 ms, now 0.57.)
+// (transit, slot) pair, 205 M of them for 10,000 samples of 5 x 64 x 64 on 57 K vertices: 1.04 ms, the kernel now 0.24.)
 // The flags of the edges that were found are the adjacency as it is kept: a bit per entry (the two arrays of the
 // reference's form, 1.6 GB for those samples, took 0.1 ms of 0.54).
 constexpr int FILTER_WORDS = 256;   // 8192 bits per layer

@@ -123,7 +123,7 @@ struct nd_graph {
   mutable int2 *colw = nullptr;        // [E] (neighbour id, weight bits) records: one 8-byte gather per weighted try
   mutable int2 *vrec = nullptr;        // [V+1] (row start, max weight bits) per vertex: what a thread-per-walk kernel needs of a vertex in one sector
   mutable int2 *vrow = nullptr;        // [V] (row start, degree): one load per vertex
-  mutable int4 *erec = nullptr;        // [E] (neighbour id, its row start, its degree, 0)
+  mutable int4 *erec = nullptr;        // [E] (neighbour id, its row start, its degree, weight as in `pack`)
   mutable uint32_t *pack = nullptr;    // [E] neighbour id << 8 | weight as whole 256ths of the row's maximum
   mutable uint8_t *codes = nullptr;    // [E] ... the weights alone, where there is no room for both
   mutable uint2 *col3 = nullptr;       // [E/3] three neighbour ids of 21 bits to 8 bytes

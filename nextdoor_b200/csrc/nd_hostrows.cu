@@ -289,8 +289,10 @@ bool find_rows(nd_sampler *s) {
 }
 
 // The rows that the GPU writes itself, whole chunks from the front: as fast as 16 host threads (above).  The host's memory
-// serves both, so that they are not twice as fast together: jobs of 2^21 rows 3.2 -> 2.4 ms with half of them, 2.8 with
-// a third and with all, 2.7 with three quarters.  None where a caller has captured a job, whose replays may come at any time.
+// serves both, so that they are not twice as fast together.  Jobs of 2^21 rows on a host of 16 hardware threads, no share, a
+// third, half, two thirds, four fifths: by 4 threads 9.1, 6.1, 4.6, 3.2, 2.6 ms; by 8 5.0, 3.9, 3.1, 2.5, 2.7; by 16 3.5, 2.5,
+// 2.4, 2.6, 2.8; by 32, two to a hardware thread, 4.0, 2.8, 2.4, 2.5, 2.8.  (Threads that the host does not have, or that
+// other processes use, count all the same: ND_HOST_THREADS says how many there are.)  None where a caller has captured a job, whose replays may come at any time.
 int64_t direct_rows(nd_sampler *s, int32_t *out, int32_t *row_len) {
   NdHostRows *h = s->hostrows;
   if (s->S < 4 * PACK_CHUNK || s->in_graph || (uintptr_t)out % 4 || (uintptr_t)row_len % 4) return 0;

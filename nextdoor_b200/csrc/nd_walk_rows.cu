@@ -13,7 +13,7 @@
 // hence: one try per round for the weighted apps (no speculation), the id and its weight in one word, the first stop draw
 // of a step made before the vertex is fetched, a filter in front of node2vec's sets, rows written once, in
 // 32-byte sectors.  Small graphs: the chain of a walk, two dependent L2 reads per step, one where the entries carry the
-// neighbour's row, and the instructions between them (57 K vertices: a step is 0.5 us, 121 instructions of a warp at 8.2
+// neighbour's row, and the instructions between them (57 K vertices: a step is 0.5 us, 111 instructions of a warp at 8.9
 // cycles each, 45 % of them waiting for the read).
 #include <mutex>
 
@@ -311,7 +311,10 @@ __device__ __forceinline__ int4 walk_of(const RowsArgs &a, const Hot &hot, int64
 }
 
 // Walks that run their full length (EQUAL) take equal rounds: with w rounds of lanes every round takes n / w walks, or the
-// last one would run a fraction of the lanes for as long as the others; and a warp gets 32 at a time.
+// last one would run a fraction of the lanes for as long as the others; and a warp gets 32 at a time.  (Without and with,
+// one walk per vertex: node2vec on 400 K vertices 1.20 -> 0.95 ms, 600 K 1.34 -> 1.21, 2^20 2.08 -> 2.11, 1.5 M 3.15 -> 2.87,
+// 2^21 4.89 -> 4.59; DeepWalk 0.68 -> 0.60, 0.80 -> 0.74, 1.37 -> 1.40, 2.02 -> 1.91, 3.13 -> 2.96: what it gives is the part of
+// a round that the last one lacks, and 2^20 with few of them empty lacks little.)
 template <bool EQUAL>
 struct Taker {
   static constexpr int GRANT = EQUAL ? 32 : 64;
@@ -765,7 +768,7 @@ adjset_build_kernel(const int32_t *__restrict__ row_ptr, const int32_t *__restri
 // Entries that carry the neighbour's row (16 bytes each) shorten a step by a dependent read; they pay while the array, here
 // 64 MB, stays in the L2 (130 K vertices, 2.8 M entries, without and with: uniform walk 95 -> 83 us, PPR 115 -> 106, DeepWalk
 // 203 -> 198; 60 K, 1.2 M: PPR 117 -> 104; 200 K, 4.8 M: 131 -> 120, 142 -> 132, 293 -> 291; 300 K, 7.2 M: uniform walk
-// 171 -> 197, DeepWalk 329 -> 350).  node2vec fetches two candidates a round and waits for the filter anyway: 298 -> 326.
+// 171 -> 197, DeepWalk 329 -> 350).  Built by the first sampler of a graph: 0.4 ms at 2.8 M entries.  node2vec fetches two candidates a round and waits for the filter anyway: 298 -> 326.
 constexpr int64_t ERECS = (int64_t)1 << 22;
 // Ids that leave a byte of a word to the weight.
 constexpr int32_t PACK_V = 1 << 24;

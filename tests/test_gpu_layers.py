@@ -161,13 +161,13 @@ def _ladies(nd, ndo, hg, S, B, L, init, adjacency=True):
             cdf = np.cumsum(np.bincount(at, (share * share).astype(np.float64)))
             u = np.array([ndo.lib().ndo_uniform(3, smp, step, j, 0) for j in range(L)], np.float32)
             target = u.astype(np.float64) * cdf[-1]
-            k = np.minimum(np.searchsorted(cdf, target), len(cand) - 1)
-            mine = np.searchsorted(cand, got[smp, step])
+            mine = np.minimum(np.searchsorted(cand, got[smp, step]), len(cand) - 1)
             assert np.array_equal(cand[mine], got[smp, step])
             bound = 2.0 ** -35 * cdf[-1]
-            ok = (mine == k) | ((mine == k + 1) & (cdf[k] - target <= bound)) | ((mine == k - 1) & (target - cdf[k - 1] <= bound))
-            assert ok.all()
-            assert np.allclose(prob[smp, step], np.diff(cdf, prepend=0.0)[mine] / cdf[-1], rtol=1e-6, atol=2.0 ** -35)
+            before = np.concatenate([[0.0], cdf])[mine]
+            assert (cdf[mine] >= target - bound).all() and (before <= target + bound).all()
+            assert (prob[smp, step] > 0).all()
+            assert np.allclose(prob[smp, step], (cdf[mine] - before) / cdf[-1], rtol=1e-6, atol=2.0 ** -35)
     assert s.stats()["union_unique"] == seen
     if adjacency:   # (whose probes ask for lists that ascend)
         assert ndo.check_adjacency(hg, ndo.make_params(9, steps=steps, fanout=L, batch=B, seed=3), S, init, s.final_samples(), aux["adj_row"], aux["adj_col"]) == 0
@@ -241,10 +241,11 @@ def test_ladies_draws_no_neighbour_of_weight_zero(nd, ndo, monkeypatch, V, sort)
         assert (prob > 0).all(), seed
 
 
-@pytest.mark.parametrize("order", ["ascending", "hub's list"])
+@pytest.mark.parametrize("order,decades", [("ascending", 0), ("ascending", 8), ("hub's list", 0)])
 @pytest.mark.parametrize("repeats", [1, 40])
-def test_ladies_hubs_by_tables(nd, ndo, order, repeats):
-    """Hubs whose neighbours occur once and many times, whose lists end inside a group, and one whose list is in another order."""
+def test_ladies_hubs_by_tables(nd, ndo, order, decades, repeats):
+    """Hubs whose neighbours occur once and many times, whose lists end inside a group, and one whose list is in another order;
+    weights of one size and over eight decades."""
     V, rng = 40_000, np.random.default_rng(repeats)
     hubs = np.array([0, 5, 127, 128, 20_000, V - 1])
     deg = rng.integers(0, 9, V)
@@ -255,7 +256,8 @@ def test_ladies_hubs_by_tables(nd, ndo, order, repeats):
     dst[often] = dst[often] // repeats * repeats        # on average `repeats` times the same neighbour
     toward = ~np.isin(src, hubs) & (rng.random(len(src)) < 0.3)
     dst[toward] = rng.choice(hubs, toward.sum())
-    hg = ndo.csr_from_records(src, dst, (rng.random(len(src)) + 0.1).astype(np.float32), V=V)
+    w = 10 ** rng.uniform(-decades, 0, len(src)) if decades else rng.random(len(src)) + 0.1
+    hg = ndo.csr_from_records(src, dst, w.astype(np.float32), V=V)
     if order != "ascending":
         a, b = hg.row_ptr[20_000], hg.row_ptr[20_001]
         hg.col[a:b], hg.w[a:b] = hg.col[a:b][::-1].copy(), hg.w[a:b][::-1].copy()
