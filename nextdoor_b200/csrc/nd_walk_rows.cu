@@ -42,8 +42,7 @@ struct RowsArgs {
   const int4 *__restrict__ erec;     // [E] (neighbour, its row start, its degree, weight as 256ths of the row's maximum, rounded down)
   const int2 *__restrict__ colw;     // [E] (neighbour, weight bits)
   const int2 *__restrict__ vrec;     // [V+1] (row start, max weight bits)
-  const uint32_t *__restrict__ pack; // [E] neighbour << 8 | weight as 256ths of the row's maximum, rounded down
-  const uint8_t *__restrict__ codes; // [E] the weights of `pack` alone
+  const uint32_t *__restrict__ pack; // [E] neighbour << 8 | weight as 256ths of the row's maximum, rounded down (CODES: a byte each, the weight)
   const uint2 *__restrict__ col3;    // [E/3] three neighbours of 21 bits each
   const int32_t *__restrict__ adjset;
   const uint32_t *__restrict__ adjsign;
@@ -471,7 +470,7 @@ __device__ __forceinline__ void weighted_walks(const RowsArgs &a) {
         const int4 r = hot.ld(a.erec + rs + x);
         id = (uint32_t)r.x; b = (uint32_t)r.w; row = make_int2(r.y, r.z);
       } else if (LAYOUT == LAYOUT_CODES) {
-        id = 0u; b = __ldg(a.codes + rs + x);
+        id = 0u; b = __ldg(reinterpret_cast<const uint8_t *>(a.pack) + rs + x);
       } else {
         const uint32_t r = __ldg(a.pack + rs + x);
         id = r >> 8; b = r & 255u;
@@ -968,7 +967,8 @@ int nd_walk_rows_alloc(nd_sampler *s) {
 int nd_walk_rows_launch(nd_sampler *s, bool count) {
   const nd_graph *g = s->g;
   uint32_t *ended = count ? reinterpret_cast<uint32_t *>(s->d_rows_acc + 16) : nullptr;
-  RowsArgs a{g->V, g->row_ptr, g->col, g->w, g->max_w, g->vrow, g->erec, g->colw, g->vrec, g->pack, g->codes, g->col3, g->adjset, g->adjsign,
+  RowsArgs a{g->V, g->row_ptr, g->col, g->w, g->max_w, g->vrow, g->erec, g->colw, g->vrec,
+             s->layout == LAYOUT_CODES ? reinterpret_cast<const uint32_t *>(g->codes) : g->pack, g->col3, g->adjset, g->adjsign,
              ndrng::RoundKeys(s->p.seed), s->p.p, s->p.q, s->p.stop_prob, s->p.n2v_ref_compat, s->p.steps, s->first, s->S, s->d_initial, s->d_out,
              s->d_plen, s->d_list, s->d_rows_acc, ended, s->d_stats, (uint32_t *)s->d_nlive, s->d_status};
   switch (s->p.app) {
