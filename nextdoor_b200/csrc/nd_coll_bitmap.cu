@@ -7,8 +7,8 @@
 // integer weights sum exactly).
 //
 // What bounds it, and what is done about it (2^20 vertices, 1024 batches of 64, 2 layers of 64: FastGCN
-// 4.8 -> 0.89 ms, LADIES 5.7 -> 0.80 ms).  One CTA fills an SM, and neither memory nor issue slots are full: FastGCN issued
-// in 58 % of the cycles at 0.98 ms (5.6 GB out of the L2 at 24 % of its rate), LADIES in 57 % at 1.07 (610 M
+// 4.8 -> 0.74 ms, LADIES 5.7 -> 0.80 ms).  One CTA fills an SM, and neither memory nor issue slots are full: FastGCN issued
+// in 58 % of the cycles at 0.89 ms (5.5 GB out of the L2 at 18 % of its rate), LADIES in 57 % at 1.07 (610 M
 // instructions for 131 M list entries, the distinct ones of 313 M), its shared memory busy in half of them; the warps
 // wait for barriers between the phases, for shared memory and for loads:
 //  * The second layer's transits are hubs (FastGCN draws them with the square of their degree), many of them the
@@ -17,12 +17,16 @@
 //    have their neighbourhood as a bitmap, built once per graph: V/8 bytes that are ORed in registers, word by
 //    word, and stored to the union once; and an adjacency probe of such a transit is a bit test.
 //  * FastGCN's weights are summed without a list of candidates (writing that and fetching deg^2 one by one took more
-//    than half of the time): the degrees lie in vertex order as two planes of bytes, a lane takes eight vertices with one
-//    16-byte load, masks them with its byte of the bitmap and squares and sums them with dp4a.  Vertices with 2048
-//    neighbours or more, whose squares would overflow the 32-bit group sums, are a short list per graph.  Groups without a
-//    candidate, most of a first layer's, are passed over; the list's weights are added up per group across the lanes; a
-//    draw asks for all row offsets of its group at once (0.98 -> 0.89 ms; the squares as three planes of bytes: 1.01, the
-//    third costs more than the products save).
+//    than half of the time).  The degrees lie in vertex order, a byte each: a lane takes sixteen vertices with one load, masks
+//    them with its half word of the bitmap and squares and sums them with dp4a.  That is bound by the products (four cycles
+//    each): the two bytes that hold degrees up to 2047 take three times as many, so that from 256 on, where few vertices have
+//    as many, they are a list (20 K of 2^20, 65 against 160 thousand cycles an SM); where they are not few the codes have a
+//    second byte, for the groups that need it.  Groups without a candidate are passed over, and the lists beside the hubs',
+//    where they are short (a first layer's: 2 K entries), are weighed entry by entry as they come into the union, an eight of
+//    entries to a thread, instead of looking through 2^20 vertices for them (390 -> 100 thousand cycles an SM with the lists
+//    a warp each before; V / FEW: 64 0.755, 16 0.79 ms).  Groups' sums are two 32-bit words until they are scanned: a 64-bit
+//    add in shared memory is a loop.  0.89 -> 0.74 ms, 256 batches on 2^21 0.56 -> 0.46, 700 of 100 on 100 K 0.50 -> 0.46.
+//  * A draw of FastGCN asks for all row offsets of its group at once (0.98 -> 0.89 ms).
 //  * LADIES' terms (w / rowsum)^2 depend on the edge alone: an array, built once per graph, instead of a pass over
 //    the weights and a division per entry and sample.  One pass over the lists sets the union's bits and adds the terms
 //    up per group; then the groups that the draws fall into get an accumulator per vertex, where the union was,
@@ -52,11 +56,12 @@ using ndrng::Rng;
 constexpr int GROUP_WORDS = 16;   // words of a FastGCN group; bitmaps are whole ones
 constexpr int GROUP = 512;        // FastGCN: vertices (GROUP_WORDS words) whose weights are summed together
 constexpr int LADIES_GROUP_BITS = 7;   // LADIES: 2^7 vertices, more where the sums of the groups would not fit shared memory
-constexpr int BIG_DEGREE = 2048;  // from here a vertex is on the list of big ones and its code is 0: 512 * 2047^2 < 2^31
-constexpr int FLIGHT = 3;         // groups a warp sums at a time
+constexpr int RUN = 4;            // listed vertices a thread takes at a time
+constexpr int BIG_DEGREE = 2048;  // from here a vertex is listed and its code is 0: 512 * 2047^2 < 2^31
+constexpr int LISTED = 32;        // degrees are codes of a byte where fewer than V / LISTED vertices do not fit one
+constexpr int FLIGHT = 6;         // groups a warp sums at a time (2^20 vertices 3: 0.74, 4: 0.73, 6: 0.73 ms; 2^21 0.49, 0.48, 0.46)
 constexpr int HUB = 128;          // a vertex with at least V / HUB neighbours has a bitmap of them
-constexpr int BIG_LIST = 4096;    // lists at least this long are streamed by the whole CTA
-constexpr int VEC = 4;            // 16-byte loads in flight per thread
+constexpr int FEW = 64;           // lists with fewer than V / FEW entries in all are weighed entry by entry
 constexpr int OCT = 8;            // list entries a thread takes at a time: 32 aligned bytes (LADIES)
 
 // The bitmap and FastGCN's CDF make the "big" part (V/8 + V/64 bytes).  It lives in shared memory when the whole layout
@@ -75,6 +80,15 @@ struct Layout {
   uint32_t glob_bytes;                                 // per-CTA slice of the global scratch, 0 = big part in shared memory
 };
 
+// The degrees in vertex order, FastGCN.  Codes: the low bytes of sixteen vertices' each, then the high ones; a listed
+// vertex's is zero.
+struct Degrees {
+  const uint4 *__restrict__ codes;
+  const uint32_t *__restrict__ wide;        // a bit per group: it has high bytes that are not zero; null: none has
+  const int2 *__restrict__ listed;          // [n_listed] (vertex, degree) in order, read in whole runs
+  int n_listed;
+};
+
 struct Args {
   NdGraphView g;
   CollParams cp;
@@ -86,9 +100,9 @@ struct Args {
   int32_t *out;
   uint32_t *adj;
   float *prob;
-  const uint4 *__restrict__ deg;           // FastGCN: the degrees of eight vertices, low bytes (x, y), high bytes (z, w)
-  const NdBigVertex *__restrict__ big;     // FastGCN: vertices with degrees from BIG_DEGREE, in order
-  int n_big;
+  Degrees deg;                             // FastGCN
+  const NdBigVertex *__restrict__ huge;    // ... vertices with at least HUGE_DEGREE neighbours
+  int n_huge;
   const float *__restrict__ term;          // LADIES: (w / rowsum)^2 per entry
   const int32_t *__restrict__ hub_slot;    // [V] slot of the vertex's bitmap, -1: none
   const uint32_t *__restrict__ hub_bits;   // [slots][words]
@@ -105,33 +119,6 @@ struct Args {
 struct Transit { int32_t rs, deg, mult, slot; };
 
 constexpr uint32_t NO_SLOT = 255u;
-
-__device__ __forceinline__ void mark(uint32_t *bm, int32_t v) {
-  const uint32_t bit = 1u << (v & 31);
-  uint32_t *wp = bm + ((uint32_t)v >> 5);
-  if (!(*(volatile uint32_t *)wp & bit)) atomicOr(wp, bit);  // lists overlap: most bits are set already
-}
-
-// Streams one neighbour list with `stride` cooperating threads and sets the neighbours' bits.  The body of the list is
-// read as 16-byte vectors (the arrays are 256-byte aligned, so entry rs + head is 16-byte aligned for
-// head = (4 - rs % 4) % 4), VEC vectors in flight per thread; head and tail entries one by one.
-__device__ __forceinline__ void stream_list(const NdGraphView &g, uint32_t *bm, int32_t rs, int32_t deg, int me, int stride) {
-  const int32_t *__restrict__ col = g.col + rs;
-  int head = (4 - (rs & 3)) & 3;
-  if (head > deg) head = deg;
-  if (me < head) mark(bm, __ldg(col + me));
-  const int n4 = (deg - head) >> 2;
-  const int4 *__restrict__ col4 = reinterpret_cast<const int4 *>(col + head);
-  for (int e0 = me; e0 < n4; e0 += stride * VEC) {
-    int4 v[VEC];
-#pragma unroll
-    for (int k = 0; k < VEC; k++) v[k] = e0 + k * stride < n4 ? __ldg(col4 + e0 + k * stride) : make_int4(-1, -1, -1, -1);
-#pragma unroll
-    for (int k = 0; k < VEC; k++)
-      if (v[k].x >= 0) { mark(bm, v[k].x); mark(bm, v[k].y); mark(bm, v[k].z); mark(bm, v[k].w); }
-  }
-  for (int e = head + (n4 << 2) + me; e < deg; e += stride) mark(bm, __ldg(col + e));
-}
 
 // exclusive (uint32) or inclusive (double) scan of an array by the whole CTA: every thread owns a contiguous
 // chunk, the chunk totals are scanned through warp shuffles
@@ -211,6 +198,80 @@ __device__ __forceinline__ int list_of_oct(const uint32_t *pre, int nu, uint32_t
 __device__ __forceinline__ uint32_t oct_mask(int64_t e, const Transit &t) {
   const int64_t lo = (int64_t)t.rs - e, hi = (int64_t)t.rs + t.deg - e;
   return (hi >= OCT ? 0xffu : (1u << (int)hi) - 1u) & (lo <= 0 ? 0xffu : 0xffu << (int)lo);
+}
+
+__device__ __forceinline__ float square(int32_t deg) {
+  const float d = __int2float_rn(deg);
+  return __fmul_rn(d, d);
+}
+
+// ... as a whole number, which it is
+__device__ __forceinline__ unsigned long long weight_of(int32_t deg) { return deg <= 4096 ? (unsigned long long)((uint32_t)deg * (uint32_t)deg) : (unsigned long long)square(deg); }
+
+// FastGCN: a group's sum is two words while it is added up (64-bit adds in shared memory are loops): low SUM_BITS bits of the
+// weights below, the rest above.  A group's 512 weights fit them up to HUGE_DEGREE neighbours.
+constexpr int SUM_BITS = 22, HUGE_DEGREE = 1 << 22;
+struct Sum {
+  uint32_t low = 0, high = 0;
+  __device__ __forceinline__ void add(int32_t deg) {
+    if (deg < BIG_DEGREE) {
+      low += (uint32_t)(deg * deg);
+    } else if (deg < HUGE_DEGREE) {
+      const unsigned long long w = weight_of(deg);
+      low += (uint32_t)w & ((1u << SUM_BITS) - 1u);
+      high += (uint32_t)(w >> SUM_BITS);
+    }
+  }
+  __device__ __forceinline__ void to(uint2 *sums, int group) const {
+    if (low) atomicAdd(&sums[group].x, low);
+    if (high) atomicAdd(&sums[group].y, high);
+  }
+  static __device__ __forceinline__ double value(const uint2 &s) { return (double)s.x + (double)(1 << SUM_BITS) * (double)s.y; }
+};
+
+// FastGCN: the entries of the lists without bitmaps into the union; with WEIGHTS what they add to it goes to the groups' sums
+// and is counted (the number the thread has added).
+template <bool WEIGHTS>
+__device__ __forceinline__ uint32_t add_lists(const NdGraphView &g, const Transit *rest, int n, const uint32_t *pre, uint32_t total, uint32_t *bm, uint2 *sums) {
+  uint32_t added = 0;
+  int i = 0;
+  for (uint32_t o = threadIdx.x; o < total; o += blockDim.x) {
+    if (i + 1 < n && pre[i + 1] <= o) i = list_of_oct(pre, n, o);
+    const Transit t = rest[i];
+    const int64_t e = ((int64_t)((uint32_t)t.rs / OCT) + (int64_t)(o - pre[i])) * OCT;
+    int32_t v[OCT];
+    load8(g.col + e, v);
+    uint32_t fresh = oct_mask(e, t);
+    {
+      uint32_t word[OCT];
+#pragma unroll
+      for (int j = 0; j < OCT; j++) word[j] = (fresh >> j) & 1u ? bm[(uint32_t)v[j] >> 5] : ~0u;
+#pragma unroll
+      for (int j = 0; j < OCT; j++) {   // (most ids of a hub's neighbours are there already)
+        const uint32_t bit = 1u << (v[j] & 31);
+        if ((word[j] & bit) || (atomicOr(bm + ((uint32_t)v[j] >> 5), bit) & bit)) fresh &= ~(1u << j);
+      }
+    }
+    if (!WEIGHTS || !fresh) continue;
+    added += __popc(fresh);
+    int32_t deg[OCT];
+#pragma unroll
+    for (int j = 0; j < OCT; j++) deg[j] = (fresh >> j) & 1u ? __ldg(g.row_ptr + v[j] + 1) - __ldg(g.row_ptr + v[j]) : 0;
+    int at = -1;
+    Sum sum;
+#pragma unroll
+    for (int j = 0; j < OCT; j++) {
+      if (!((fresh >> j) & 1u)) continue;
+      if (v[j] / GROUP != at) {
+        if (at >= 0) sum.to(sums, at);
+        at = v[j] / GROUP;
+        sum = Sum();
+      }
+      sum.add(deg[j]);
+    }
+    sum.to(sums, at);
+  }
+  return added;
 }
 
 // LADIES: the terms of the entries of lists without tables into the sums of their groups, and the entries into the
@@ -297,6 +358,16 @@ __device__ __forceinline__ void add_candidates(const NdGraphView &g, const float
   }
 }
 
+// first group whose prefix reaches the target (rounding: the last one takes what is above all)
+__device__ __forceinline__ int first_reaching(const double *cdf, int n, double target) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = lo + (hi - lo) / 2;
+    if (cdf[mid] >= target) hi = mid; else lo = mid + 1;
+  }
+  return lo;
+}
+
 // LADIES: the draw's candidate in its group, by a warp: the first whose running sum reaches the target, or by rounding the
 // last there is.  Blocks of 128 candidates, a lane holding four.  One with a weight of zero is none (its running sum is
 // the one before it, which another order of the adds may leave a rounding below the target); a group that is drawn from
@@ -337,22 +408,87 @@ __device__ __forceinline__ void pick_in_group(const double *acc, int n, double b
   }
 }
 
-// bits 0..3 -> 0xff in bytes 0..3
-__device__ __forceinline__ uint32_t byte_mask(uint32_t bits) { return (((bits & 15u) * 0x204081u) & 0x01010101u) * 255u; }
+// bits 0..3 (no others) -> 0xff in bytes 0..3
+__device__ __forceinline__ uint32_t byte_mask(uint32_t bits) {
+  uint32_t m;
+  asm("prmt.b32 %0, %1, 0, 0xba98;" : "=r"(m) : "r"(bits * 0x10204080u));   // each to the top of its byte, which is filled with it
+  return m;
+}
 
-// The sum of deg^2 over the vertices of `bits` (eight vertices, degrees as in Args::deg), in products of low, low and high, and
-// high bytes.
-struct Squares {
-  uint32_t ll = 0u, lh = 0u, hh = 0u;
-  __device__ __forceinline__ void add(uint32_t bits, const uint4 &d) {
-    const uint32_t m0 = byte_mask(bits), m1 = byte_mask(bits >> 4);
-    const uint32_t l0 = d.x & m0, l1 = d.y & m1;
-    ll = __dp4a(l1, d.y, __dp4a(l0, d.x, ll));
-    lh = __dp4a(l1, d.w, __dp4a(l0, d.z, lh));
-    hh = __dp4a(d.w & m1, d.w, __dp4a(d.z & m0, d.z, hh));
+// The sum of deg^2 over the vertices of `bits` (sixteen, low and high bytes of their degrees as in Args::deg), in products of
+// low, low and high, and high bytes.
+template <bool WIDE>
+__device__ __forceinline__ uint32_t squares(uint32_t bits, const uint4 &low, const uint4 &high) {
+  const uint32_t m0 = byte_mask(bits & 15u), m1 = byte_mask((bits >> 4) & 15u), m2 = byte_mask((bits >> 8) & 15u), m3 = byte_mask(bits >> 12);
+  const uint32_t l0 = low.x & m0, l1 = low.y & m1, l2 = low.z & m2, l3 = low.w & m3;
+  const uint32_t ll = __dp4a(l3, l3, __dp4a(l2, l2, __dp4a(l1, l1, __dp4a(l0, l0, 0u))));
+  if (!WIDE) return ll;
+  const uint32_t lh = __dp4a(l3, high.w, __dp4a(l2, high.z, __dp4a(l1, high.y, __dp4a(l0, high.x, 0u))));
+  const uint32_t hh = __dp4a(high.w & m3, high.w, __dp4a(high.z & m2, high.z, __dp4a(high.y & m1, high.y, __dp4a(high.x & m0, high.x, 0u))));
+  return ll + (lh << 9) + (hh << 16);
+}
+
+// FastGCN: the groups' weights, without HUGE_DEGREE ones; the candidates the thread has seen.  A warp takes FLIGHT groups at a
+// time: a lane sixteen vertices' codes, then the group's listed vertices side by side.  WIDE: the codes have high bytes.
+template <bool WIDE>
+__device__ __forceinline__ uint32_t sum_groups(const uint32_t *bm, const Degrees &d, int words, int groups, uint2 *sums) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const uint16_t *half = reinterpret_cast<const uint16_t *>(bm);
+  const uint4 *__restrict__ high_bytes = d.codes + (int64_t)words * 2;
+  uint32_t seen = 0;
+  for (int g0 = warp * FLIGHT; g0 < groups; g0 += warps * FLIGHT) {
+    uint32_t bits[FLIGHT], some = 0u;
+    bool wide[FLIGHT];
+    uint4 lo[FLIGHT], hi[FLIGHT];
+#pragma unroll
+    for (int k = 0; k < FLIGHT; k++) {
+      bits[k] = g0 + k < groups ? half[(g0 + k) * 32 + lane] : 0u;
+      wide[k] = WIDE && g0 + k < groups && ((__ldg(d.wide + (g0 + k) / 32) >> ((g0 + k) & 31)) & 1u);
+      some |= bits[k];
+    }
+    if (!__any_sync(0xffffffffu, some)) continue;   // (a first layer's thousand candidates leave most groups empty)
+#pragma unroll
+    for (int k = 0; k < FLIGHT; k++) {
+      const int unit = (g0 + k) * 32 + lane;
+      lo[k] = bits[k] ? __ldg(d.codes + unit) : make_uint4(0u, 0u, 0u, 0u);
+      if (WIDE) hi[k] = wide[k] && bits[k] ? __ldg(high_bytes + unit) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int k = 0; k < FLIGHT; k++) {
+      seen += __popc(bits[k]);
+      const uint32_t low = __reduce_add_sync(0xffffffffu, squares<WIDE>(bits[k], lo[k], hi[k]));
+      if (lane == 0 && low) atomicAdd(&sums[g0 + k].x, low);
+    }
   }
-  __device__ __forceinline__ uint32_t sum() const { return ll + (lh << 9) + (hh << 16); }
-};
+  return seen;
+}
+
+// ... and over the listed vertices; neighbours on the list mostly share a group
+__device__ __forceinline__ void sum_listed(const uint32_t *bm, const Degrees &d, uint2 *sums) {
+  for (int i0 = threadIdx.x * RUN; i0 < d.n_listed; i0 += blockDim.x * RUN) {
+    int32_t v[RUN], deg[RUN];
+    uint32_t word[RUN];
+#pragma unroll
+    for (int k = 0; k < RUN; k += 2) {
+      const int4 two = __ldg(reinterpret_cast<const int4 *>(d.listed + i0 + k));
+      v[k] = two.x; deg[k] = two.y; v[k + 1] = two.z; deg[k + 1] = two.w;
+    }
+#pragma unroll
+    for (int k = 0; k < RUN; k++) word[k] = i0 + k < d.n_listed ? bm[v[k] >> 5] : 0u;
+    int at = v[0] / GROUP;
+    Sum sum;
+#pragma unroll
+    for (int k = 0; k < RUN; k++) {
+      if (v[k] / GROUP != at) {
+        sum.to(sums, at);
+        at = v[k] / GROUP;
+        sum = Sum();
+      }
+      if ((word[k] >> (v[k] & 31)) & 1u) sum.add(deg[k]);
+    }
+    sum.to(sums, at);
+  }
+}
 
 // SUMS_FAR: LADIES' group sums are in the big part.
 template <bool LADIES, bool SUMS_FAR>
@@ -366,6 +502,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
   unsigned char *big = lay.glob_bytes ? a.gscratch + (size_t)blockIdx.x * lay.glob_bytes : smem;
   uint32_t *bm = reinterpret_cast<uint32_t *>(big);
   double *gcdf = reinterpret_cast<double *>((LADIES && !SUMS_FAR ? smem : big) + lay.off_gcdf);
+  uint2 *gsum = reinterpret_cast<uint2 *>(gcdf);                         // FastGCN: its weights while they are added up
   double *red = reinterpret_cast<double *>(smem + lay.off_red);   // 32 doubles, 32 words
   uint32_t *red_u = reinterpret_cast<uint32_t *>(red + 32);
   int32_t *sh_tr = reinterpret_cast<int32_t *>(smem + lay.off_tr);
@@ -374,8 +511,8 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
   int32_t *sh_mult = reinterpret_cast<int32_t *>(smem + lay.off_mult);   // how often a transit occurs (the first of a kind counts); then its place in ut, -1: not a vertex
   int32_t *sh_same = reinterpret_cast<int32_t *>(smem + lay.off_same);   // the first transit that is the same
   uint32_t *pre = reinterpret_cast<uint32_t *>(smem + lay.off_pre);
+  double *sh_target = reinterpret_cast<double *>(smem + lay.off_draw);   // of a draw: the point of the CDF, its group, LADIES: the first draw of the group
   double *acc = reinterpret_cast<double *>(smem + lay.off_acc);          // LADIES from here on
-  double *sh_target = reinterpret_cast<double *>(smem + lay.off_draw);   // of a draw: the point of the CDF, its group, the first draw of the group
   int32_t *sh_group = reinterpret_cast<int32_t *>(sh_target + cp.L), *sh_first = sh_group + cp.L;
   int32_t *sh_slot_group = sh_first + cp.L;
   uint32_t *sh_firsts = reinterpret_cast<uint32_t *>(sh_slot_group + cp.L);   // draws that are the first of their group, as bits
@@ -437,54 +574,24 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
       const int groups = lay.groups;
       uint32_t seen = 0, octs = 0;
       if (!LADIES) {
-        __syncthreads();
         const Transit *rest = ut + cp.ntr - (nu - nh);
-        for (int i = warp; i < nu - nh; i += warps)   // short lists: a warp each
-          if (rest[i].deg < BIG_LIST) stream_list(a.g, bm, rest[i].rs, rest[i].deg, lane, 32);
-        for (int i = 0; i < nu - nh; i++)             // long lists: the whole CTA
-          if (rest[i].deg >= BIG_LIST) stream_list(a.g, bm, rest[i].rs, rest[i].deg, tid, blockDim.x);
+        for (int i = tid; i < nu - nh; i += blockDim.x) pre[i] = octs_of(rest[i].rs, rest[i].deg);
+        for (int k = tid; k < groups; k += blockDim.x) gsum[k] = make_uint2(0u, 0u);
         __syncthreads();
-        // ---- the groups' weights, and the number of candidates
-        const uint8_t *bytes = reinterpret_cast<const uint8_t *>(bm);
-        for (int g0 = warp * FLIGHT; g0 < groups; g0 += warps * FLIGHT) {
-          uint32_t bits[2 * FLIGHT], some = 0u;
-          uint4 d[2 * FLIGHT];
-#pragma unroll
-          for (int k = 0; k < 2 * FLIGHT; k++) {
-            const int at = g0 * (GROUP / 8) + k * 32 + lane;
-            bits[k] = at < groups * (GROUP / 8) ? bytes[at] : 0u;
-            some |= bits[k];
-          }
-          if (!__any_sync(0xffffffffu, some)) {   // (a first layer's thousand candidates leave most groups empty)
-            if (lane < FLIGHT && g0 + lane < groups) gcdf[g0 + lane] = 0.0;
-            continue;
-          }
-#pragma unroll
-          for (int k = 0; k < 2 * FLIGHT; k++) d[k] = bits[k] ? __ldg(a.deg + g0 * (GROUP / 8) + k * 32 + lane) : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-          for (int k = 0; k < FLIGHT; k++) {
-            seen += __popc(bits[2 * k] | bits[2 * k + 1] << 8);
-            Squares sq;
-            sq.add(bits[2 * k], d[2 * k]);
-            sq.add(bits[2 * k + 1], d[2 * k + 1]);
-            const uint32_t sum = __reduce_add_sync(0xffffffffu, sq.sum());
-            if (lane == 0 && g0 + k < groups) gcdf[g0 + k] = (double)sum;
-          }
+        octs = scan_u32(pre, nu - nh, red_u);
+        // Few entries beside the hubs': what they add is weighed one by one, else the whole union is gone through.
+        const bool few = (int64_t)octs * OCT * FEW <= cp.V;
+        if (!few) {
+          add_lists<false>(a.g, rest, nu - nh, pre, octs, bm, gsum);
+          __syncthreads();
         }
-        __syncthreads();
-        for (int i0 = warp * 32; i0 < a.n_big; i0 += warps * 32) {   // the big ones; neighbours on the list mostly share a group
-          const NdBigVertex v = i0 + lane < a.n_big ? a.big[i0 + lane] : NdBigVertex{-1, 0.f};
-          const bool in = v.v >= 0 && ((bm[v.v >> 5] >> (v.v & 31)) & 1u);
-          // (in order, so that what falls into one group is added up across the lanes first)
-          double x = in ? (double)v.weight : 0.0;
-          const int group = v.v >= 0 ? v.v / GROUP : -1, group_before = __shfl_up_sync(0xffffffffu, group, 1);
-          const uint32_t heads = __ballot_sync(0xffffffffu, lane == 0 || group != group_before);
-          const int head = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
-          for (int o = 1; o < 32; o <<= 1) {
-            const double t = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane - o >= head) x += t;
-          }
-          if (x > 0.0 && (lane == 31 || (heads >> (lane + 1)) & 1u)) atomicAdd(gcdf + group, x);
+        if (!few || nh > 0) {
+          seen += a.deg.wide ? sum_groups<true>(bm, a.deg, lay.words, groups, gsum) : sum_groups<false>(bm, a.deg, lay.words, groups, gsum);
+          sum_listed(bm, a.deg, gsum);
+        }
+        if (few) {
+          if (nh > 0) __syncthreads();
+          seen += add_lists<true>(a.g, rest, nu - nh, pre, octs, bm, gsum);
         }
       } else {
         // ---- the groups' weights and the rest of the union, then the number of candidates
@@ -513,6 +620,17 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
       uint32_t U = 0;
       for (int w = 0; w < warps; w++) U += red_u[w];
       if (tid == 0) uniq_sum += U;
+      if (!LADIES) {
+        for (int k = tid; k < groups; k += blockDim.x) gcdf[k] = Sum::value(gsum[k]);   // (in its place)
+        __syncthreads();
+        if (a.n_huge) {
+          for (int i = tid; i < a.n_huge; i += blockDim.x) {
+            const NdBigVertex v = a.huge[i];
+            if ((bm[v.v >> 5] >> (v.v & 31)) & 1u) atomicAdd(gcdf + v.v / GROUP, (double)v.weight);
+          }
+          __syncthreads();
+        }
+      }
       scan_f64(gcdf, groups, red);
       const double total = groups > 0 ? gcdf[groups - 1] : 0.0;
       // ---- the layer's draws
@@ -528,13 +646,8 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
           }
           Rng rng(cp.seed, (uint32_t)(cp.first_sample + s), (uint32_t)cp.step, (uint32_t)j);
           const double target = (double)rng.uniform() * total;
-          int lo = 0, hi = groups - 1;  // first group whose prefix reaches the target (rounding: the last one takes what is above all)
-          while (lo < hi) {
-            const int mid = lo + (hi - lo) / 2;
-            if (gcdf[mid] >= target) hi = mid; else lo = mid + 1;
-          }
           sh_target[j] = target;
-          sh_group[j] = lo;
+          sh_group[j] = first_reaching(gcdf, groups, target);
         }
         if (any) {
           // the groups drawn from, each once, in the order of their first draws
@@ -728,24 +841,70 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
 
 // ---------------------------------------------------------------- arrays built once per graph
 
-// a thread per eight vertices; the big ones go on the list (of `cap`), in any order
-__global__ void deg_build_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int64_t units, uint4 *__restrict__ deg, NdBigVertex *__restrict__ big,
-                                 int32_t *__restrict__ n_big, int cap) {
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < units; u += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t low[2] = {0u, 0u}, high[2] = {0u, 0u};
-    for (int k = 0; k < 8; k++) {
-      const int64_t v = 8 * u + k;
-      if (v >= V) break;
-      const int32_t d = row_ptr[v + 1] - row_ptr[v];
-      if (d >= BIG_DEGREE) {
-        const int at = atomicAdd(n_big, 1);
-        if (at < cap) big[at] = NdBigVertex{(int32_t)v, __fmul_rn(__int2float_rn(d), __int2float_rn(d))};
-        continue;
-      }
+// vertices with at least 256, BIG_DEGREE, HUGE_DEGREE neighbours
+__global__ void __launch_bounds__(256) deg_count_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int32_t *__restrict__ count) {
+  int32_t n[3] = {0, 0, 0};
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t d = row_ptr[v + 1] - row_ptr[v];
+    n[0] += d >= 256 ? 1 : 0; n[1] += d >= BIG_DEGREE ? 1 : 0; n[2] += d >= HUGE_DEGREE ? 1 : 0;
+  }
+  for (int k = 0; k < 3; k++) {
+    n[k] = __reduce_add_sync(0xffffffffu, n[k]);
+    if ((threadIdx.x & 31) == 0 && n[k]) atomicAdd(count + k, n[k]);
+  }
+}
+
+// A warp per group, a lane per sixteen vertices: codes, flags, and how many of the group's vertices have `least` neighbours or
+// more; then those onto their list, and the ones for `huge` onto theirs, in any order.
+__global__ void __launch_bounds__(256)
+deg_build_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int64_t units, int32_t least, uint4 *__restrict__ deg, uint32_t *__restrict__ wide,
+                 int32_t *__restrict__ count) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < units; u += (int64_t)gridDim.x * blockDim.x) {   // (whole warps)
+    uint32_t low[4] = {0u, 0u, 0u, 0u}, high[4] = {0u, 0u, 0u, 0u};
+    int listed = 0;
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+      const int64_t v = 16 * u + k;
+      const int32_t d = v < V ? row_ptr[v + 1] - row_ptr[v] : 0;
+      if (d >= least) { listed += d < HUGE_DEGREE ? 1 : 0; continue; }
       low[k >> 2] |= (uint32_t)(d & 255) << (8 * (k & 3));
       high[k >> 2] |= (uint32_t)(d >> 8) << (8 * (k & 3));
     }
-    deg[u] = make_uint4(low[0], low[1], high[0], high[1]);
+    deg[u] = make_uint4(low[0], low[1], low[2], low[3]);
+    deg[units + u] = make_uint4(high[0], high[1], high[2], high[3]);
+    const int64_t group = 16 * u / GROUP;
+    if (__any_sync(0xffffffffu, (high[0] | high[1] | high[2] | high[3]) != 0u) && lane == 0) atomicOr(wide + group / 32, 1u << (group & 31));
+    listed = __reduce_add_sync(0xffffffffu, listed);
+    if (lane == 0) count[group] = listed;
+  }
+}
+
+__global__ void __launch_bounds__(256)
+deg_list_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int64_t units, int32_t least, const int32_t *__restrict__ listed_at, int2 *__restrict__ listed,
+                NdBigVertex *__restrict__ huge, int32_t *__restrict__ n_huge) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < units; u += (int64_t)gridDim.x * blockDim.x) {
+    int32_t d[16];
+    int mine = 0;
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+      const int64_t v = 16 * u + k;
+      d[k] = v < V ? row_ptr[v + 1] - row_ptr[v] : 0;
+      mine += d[k] >= least && d[k] < HUGE_DEGREE ? 1 : 0;
+    }
+    int upto = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += t;
+    }
+    int32_t at = listed_at[16 * u / GROUP] + upto - mine;
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+      if (d[k] < least) continue;
+      if (d[k] < HUGE_DEGREE) listed[at++] = make_int2((int32_t)(16 * u + k), d[k]);
+      else huge[atomicAdd(n_huge, 1)] = NdBigVertex{(int32_t)(16 * u + k), square(d[k])};
+    }
   }
 }
 
@@ -921,27 +1080,47 @@ int ensure_hubs(const nd_graph *g, int grid) {
   return ND_OK;
 }
 
-// FastGCN: the packed degrees and the list of big vertices
+// FastGCN: the packed degrees and the vertices whose degrees they do not hold, listed: from 256 on where those are few, else
+// from BIG_DEGREE on.
 int ensure_degrees(const nd_graph *g, int grid) {
   if (g->deg_codes) return ND_OK;
-  const int64_t units = 4 * (int64_t)words_of(g->V);
-  const int cap = (int)(g->E / BIG_DEGREE) + 1;
+  const int64_t units = 2 * (int64_t)words_of(g->V);
+  const size_t groups = (size_t)units / (GROUP / 16), flags = (groups + 31) / 32 + 1;
   NdDevMem<uint4> deg;
-  NdDevMem<NdBigVertex> big;
-  NdDevMem<int32_t> count;
-  int32_t n = 0;
-  ND_TRY(deg.alloc((size_t)std::max<int64_t>(units, 1)));
-  ND_TRY(big.alloc((size_t)cap));
-  ND_TRY(count.alloc(1));
-  ND_CUDA(cudaMemset(count.p, 0, sizeof(int32_t)));
-  deg_build_kernel<<<grid, 256>>>(g->row_ptr, g->V, units, deg.p, big.p, count.p, cap);
-  ND_CUDA(cudaMemcpy(&n, count.p, sizeof(n), cudaMemcpyDeviceToHost));
-  std::vector<NdBigVertex> list((size_t)n);
-  ND_CUDA(cudaMemcpy(list.data(), big.p, sizeof(NdBigVertex) * (size_t)n, cudaMemcpyDeviceToHost));
-  std::sort(list.begin(), list.end(), [](const NdBigVertex &x, const NdBigVertex &y) { return x.v < y.v; });
-  ND_CUDA(cudaMemcpy(big.p, list.data(), sizeof(NdBigVertex) * (size_t)n, cudaMemcpyHostToDevice));
-  g->n_big = n;
-  g->big = big.release();
+  NdDevMem<int32_t> at;
+  NdDevMem<int2> listed;
+  NdDevMem<NdBigVertex> huge;
+  int32_t n[3] = {0, 0, 0};   // vertices with at least 256, BIG_DEGREE, HUGE_DEGREE neighbours
+  ND_TRY(deg.alloc((size_t)(2 * units) + (flags + 3) / 4));
+  ND_TRY(at.alloc(groups + 5));
+  int32_t *const count = at.p + groups + 1;   // of n, then of the huge ones listed
+  ND_CUDA(cudaMemset(at.p, 0, sizeof(int32_t) * (groups + 5)));
+  ND_CUDA(cudaMemset(deg.p + 2 * units, 0, sizeof(uint32_t) * flags));
+  deg_count_kernel<<<grid, 256>>>(g->row_ptr, g->V, count);
+  ND_CUDA(cudaMemcpy(n, count, sizeof(n), cudaMemcpyDeviceToHost));
+  const bool few = (int64_t)n[0] * LISTED <= g->V;
+  const int32_t least = few ? 256 : BIG_DEGREE;
+  const size_t n_listed = (size_t)(n[few ? 0 : 1] - n[2]), room = n_listed + RUN;
+  ND_TRY(listed.alloc(room));
+  ND_CUDA(cudaMemset(listed.p, 0, sizeof(int2) * room));
+  ND_TRY(huge.alloc((size_t)n[2] + 1));
+  deg_build_kernel<<<grid, 256>>>(g->row_ptr, g->V, units, least, deg.p, reinterpret_cast<uint32_t *>(deg.p + 2 * units), at.p);
+  std::vector<int32_t> starts(groups + 1);
+  ND_CUDA(cudaMemcpy(starts.data(), at.p, sizeof(int32_t) * groups, cudaMemcpyDeviceToHost));
+  int32_t all = 0;
+  for (int32_t &s : starts) {
+    const int32_t own = s;
+    s = all;
+    all += own;
+  }
+  ND_CUDA(cudaMemcpy(at.p, starts.data(), sizeof(int32_t) * (groups + 1), cudaMemcpyHostToDevice));
+  deg_list_kernel<<<grid, 256>>>(g->row_ptr, g->V, units, least, at.p, listed.p, huge.p, count + 3);
+  ND_CUDA(cudaDeviceSynchronize());
+  g->n_huge = n[2];
+  g->deg_wide = !few;
+  g->huge = huge.release();
+  g->listed = listed.release();
+  g->n_listed = (int)n_listed;
   g->deg_codes = deg.release();
   return ND_OK;
 }
@@ -1052,14 +1231,14 @@ Plan plan_of(const nd_sampler *s) {
     l.glob_bytes = global ? big : 0u;
     uint32_t off = global ? 0u : big;
     if (ladies && !l.sums_far) { l.off_gcdf = off; l.off_slot = off + sums; off += sums + slots; }
-    l.off_draw = off; off += ladies ? (20u * (uint32_t)L + 4u * (((uint32_t)L + 31u) / 32u) + 7u) & ~7u : 0u;
+    l.off_draw = off; off += ((ladies ? 20u * (uint32_t)L + 4u * (((uint32_t)L + 31u) / 32u) : 12u * (uint32_t)L) + 7u) & ~7u;
     l.off_red = off; off += 8u * 32u + 4u * 32u;
     l.off_ut = off; off += (uint32_t)sizeof(Transit) * (uint32_t)ntr;
     l.off_tr = off; off += 4u * (uint32_t)ntr;
     l.off_layer = off; off += 4u * (uint32_t)L;
     l.off_mult = off; off += 4u * (uint32_t)ntr;
     l.off_same = off; off += 4u * (uint32_t)ntr;
-    l.off_pre = off; off += ladies ? 4u * (uint32_t)ntr : 0u;
+    l.off_pre = off; off += 4u * (uint32_t)ntr;
     return (off + 15u) & ~15u;
   };
   // Accumulators of a group that is drawn from: in the bitmap's place where that holds SLOTS of them or one for every
@@ -1119,7 +1298,8 @@ int nd_coll_bitmap_launch(nd_sampler *s, const CollParams &cp, unsigned long lon
   const Plan p = plan_of(s);
   const nd_graph *g = s->g;
   const Args a{nd_view(g), cp, s->p.steps, s->S, p.lay, s->d_bm, s->d_initial, s->d_out, s->d_adj, s->d_prob,
-               g->deg_codes, g->big, g->n_big, g->term, g->hub_slot, g->hub_bits, s->hub_table.sums, s->hub_table.starts, g->hub_ids, g->hub_terms, s->d_rows_acc, s->d_stats, pairs};
+               Degrees{g->deg_codes, g->deg_wide ? reinterpret_cast<const uint32_t *>(g->deg_codes + 4 * (int64_t)p.lay.words) : nullptr, g->listed, g->n_listed},
+               g->huge, g->n_huge, g->term, g->hub_slot, g->hub_bits, s->hub_table.sums, s->hub_table.starts, g->hub_ids, g->hub_terms, s->d_rows_acc, s->d_stats, pairs};
   if (ladies && p.lay.sums_far) coll_bitmap_kernel<true, true><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
   else if (ladies) coll_bitmap_kernel<true, false><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
   else coll_bitmap_kernel<false, false><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);

@@ -263,3 +263,33 @@ def test_ladies_hubs_by_tables(nd, ndo, order, decades, repeats):
         hg.col[a:b], hg.w[a:b] = hg.col[a:b][::-1].copy(), hg.w[a:b][::-1].copy()
     init = np.where(rng.random(30 * 24) < 0.2, rng.choice(hubs, 30 * 24), rng.integers(0, V, 30 * 24)).astype(np.int32)
     _ladies(nd, ndo, hg, 30, 24, 48, init, adjacency=order == "ascending")
+
+
+@pytest.mark.parametrize("V,share,largest,batch", [(20_001, 0.05, 300, 24), (6144, 0.2, 2047, 24), (20_001, 0.02, 300, 24), (70_000, 0.0, 5000, 4),
+                                                   (70_000, 0.001, 9000, 300), (6000, 0.0, 1 << 22, 24), (50_000, 0.0, (1 << 22) + 9, 6)])
+@pytest.mark.parametrize("scratch", ["0", "1"])
+def test_fastgcn_weights_of_listed_vertices(nd, ndo, monkeypatch, V, share, largest, batch, scratch):
+    """A byte per degree or two, by the share of the vertices that do not fit one; few and many entries beside the hubs';
+    squares that are not whole in 24 bits, and weights that the sums of the groups do not hold (from 2^22 neighbours)."""
+    monkeypatch.setenv("ND_COLLECTIVE_BITMAP_GLOBAL", scratch)
+    rng = np.random.default_rng(V + largest)
+    deg = np.where(rng.random(V) < 0.1, 0, rng.integers(1, 6, V))
+    many = rng.random(V) < share
+    deg[many] = rng.integers(256, largest, many.sum()) if share else 0
+    top = rng.choice(V, 6, replace=False)
+    deg[top] = [largest, largest - 1, largest // 2, 4097, 256, 255]
+    src = np.repeat(np.arange(V), deg).astype(np.int32)
+    dst = np.where(rng.random(len(src)) < 0.2, rng.choice(top, len(src)), rng.integers(0, V, len(src))).astype(np.int32)
+    hg = ndo.csr_from_records(src, dst, np.ones(len(src), np.float32), V=V)
+    S, L, steps = 40, 32, 2 if largest < 1 << 20 else 1
+    initial = rng.integers(0, V, S * batch).astype(np.int32)
+    if steps == 1:
+        initial[deg[initial] > 2] = int(np.argmax(deg == 2))   # (lists of millions take the oracle long)
+    s = nd.Sampler(nd.Graph.from_csr(hg.row_ptr, hg.col, hg.w, hg.max_w), nd.app_params(8, steps=steps, fanout=L, batch=batch, seed=3), num_samples=S, initial=initial)
+    s.sample()
+    exp = ndo.sample(hg, ndo.make_params(8, steps=steps, fanout=L, batch=batch, seed=3), S, initial=initial)
+    aux = s.aux()
+    assert np.array_equal(s.final_samples(), exp["out"])   # whole numbers below 2^53: the sums are exact
+    assert np.array_equal(aux["prob"].reshape(-1), exp["prob"].reshape(-1))
+    assert np.array_equal(aux["adj_row"], exp["adj_row"]) and np.array_equal(aux["adj_col"], exp["adj_col"])
+    assert s.stats()["union_unique"] == exp["counters"]["union_unique"]
