@@ -7,7 +7,7 @@
 // integer weights sum exactly).
 //
 // What bounds it, and what is done about it (2^20 vertices, 1024 batches of 64, 2 layers of 64: FastGCN
-// 4.8 -> 0.74 ms, LADIES 5.7 -> 0.80 ms).  One CTA fills an SM, and neither memory nor issue slots are full: FastGCN issued
+// 4.8 -> 0.70 ms, LADIES 5.7 -> 0.80 ms).  One CTA fills an SM, and neither memory nor issue slots are full: FastGCN issued
 // in 58 % of the cycles at 0.89 ms (5.5 GB out of the L2 at 18 % of its rate), LADIES in 57 % at 1.07 (610 M
 // instructions for 131 M list entries, the distinct ones of 313 M), its shared memory busy in half of them; the warps
 // wait for barriers between the phases, for shared memory and for loads:
@@ -26,7 +26,10 @@
 //    entries to a thread, instead of looking through 2^20 vertices for them (390 -> 100 thousand cycles an SM with the lists
 //    a warp each before; V / FEW: 64 0.755, 16 0.79 ms).  Groups' sums are two 32-bit words until they are scanned: a 64-bit
 //    add in shared memory is a loop.  0.89 -> 0.74 ms, 256 batches on 2^21 0.56 -> 0.46, 700 of 100 on 100 K 0.50 -> 0.46.
-//  * A draw of FastGCN asks for all row offsets of its group at once (0.98 -> 0.89 ms).
+//  * FastGCN's draws: the groups are found a thread a draw (a warp each took as long twice, for two draws); then a warp sums the
+//    group's weights, sixteen vertices a lane, and goes to the vertices of the one lane that reaches the target, one scan each
+//    instead of one for every 128 vertices.  0.74 -> 0.70 ms, 0.46 -> 0.45, 0.46 -> 0.41.  (Weights as whole numbers: 0.75, the
+//    few of them that are not below 2^24 diverge.)
 //  * LADIES' terms (w / rowsum)^2 depend on the edge alone: an array, built once per graph, instead of a pass over
 //    the weights and a division per entry and sample.  One pass over the lists sets the union's bits and adds the terms
 //    up per group; then the groups that the draws fall into get an accumulator per vertex, where the union was,
@@ -59,7 +62,7 @@ constexpr int LADIES_GROUP_BITS = 7;   // LADIES: 2^7 vertices, more where the s
 constexpr int RUN = 4;            // listed vertices a thread takes at a time
 constexpr int BIG_DEGREE = 2048;  // from here a vertex is listed and its code is 0: 512 * 2047^2 < 2^31
 constexpr int LISTED = 32;        // degrees are codes of a byte where fewer than V / LISTED vertices do not fit one
-constexpr int FLIGHT = 6;         // groups a warp sums at a time (2^20 vertices 3: 0.74, 4: 0.73, 6: 0.73 ms; 2^21 0.49, 0.48, 0.46)
+constexpr int FLIGHT = 6;         // groups a warp sums at a time (2^20 vertices 4: 0.71, 6: 0.70, 8: 0.72 ms; 2^21 0.48, 0.45, 0.45)
 constexpr int HUB = 128;          // a vertex with at least V / HUB neighbours has a bitmap of them
 constexpr int FEW = 64;           // lists with fewer than V / FEW entries in all are weighed entry by entry
 constexpr int OCT = 8;            // list entries a thread takes at a time: 32 aligned bytes (LADIES)
@@ -709,79 +712,68 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
           }
         }
       }
+      if (!LADIES) {
+        for (int j = tid; j < cp.L; j += blockDim.x) {
+          Rng rng(cp.seed, (uint32_t)(cp.first_sample + s), (uint32_t)cp.step, (uint32_t)j);
+          const double target = (double)rng.uniform() * total;
+          sh_target[j] = target;
+          sh_group[j] = first_reaching(gcdf, groups, target);
+        }
+        __syncthreads();
+      }
       for (int j = LADIES ? cp.L : warp; j < cp.L; j += warps) {   // FastGCN: a warp each
         int32_t pick = cp.V;
         float pr = 0.f;
         if (U > 0 && total > 0.0) {
-          Rng rng(cp.seed, (uint32_t)(cp.first_sample + s), (uint32_t)cp.step, (uint32_t)j);
-          const double target = (double)rng.uniform() * total;
-          int lo = 0, hi = groups - 1;  // first group whose prefix reaches the target (rounding: the last one takes what is above all)
-          while (lo < hi) {
-            const int mid = lo + (hi - lo) / 2;
-            if (gcdf[mid] >= target) hi = mid; else lo = mid + 1;
-          }
+          const double target = sh_target[j];
+          int lo = sh_group[j];
           // (a target of zero takes the first candidate of all, whatever its weight)
           if (target <= 0.0) while (!__any_sync(0xffffffffu, bm[lo * GROUP_WORDS + (lane & (GROUP_WORDS - 1))])) lo++;
           const double before = lo > 0 ? gcdf[lo - 1] : 0.0;
-          // the group in four blocks of 128 vertices, a lane holding four of each: the first (block,
-          // lane) that reaches the target, then the first of its candidates that does
-          float x[4][4];
-          uint32_t there = 0;   // which of the lane's sixteen are candidates
-          int32_t at[4][5];
+          // the first lane, of sixteen vertices each, in which a candidate reaches the target, then the candidate; by rounding
+          // nobody reaches it: the last ones
+          const int64_t r = (int64_t)lo * GROUP + lane * 16;
+          const uint32_t mine = reinterpret_cast<const uint16_t *>(bm)[lo * 32 + lane];
+          double sum = 0.0;
+          if (mine) {
+            int32_t at[17];
+            if (r + 16 <= cp.V) {
 #pragma unroll
-          for (int q = 0; q < 4; q++) {   // the degrees from the row offsets, all of them asked for at once
-            const int64_t r = (int64_t)lo * GROUP + q * 128 + lane * 4;
-            there |= ((bm[r >> 5] >> (r & 31)) & 15u) << (4 * q);
+              for (int q = 0; q < 4; q++) {
+                const int4 f = __ldg(reinterpret_cast<const int4 *>(a.g.row_ptr + r) + q);
+                at[4 * q] = f.x; at[4 * q + 1] = f.y; at[4 * q + 2] = f.z; at[4 * q + 3] = f.w;
+              }
+              at[16] = __ldg(a.g.row_ptr + r + 16);
+            } else {
 #pragma unroll
-            for (int k = 0; k < 5; k++) at[q][k] = __ldg(a.g.row_ptr + (r + k < cp.V ? r + k : (int64_t)cp.V));
+              for (int k = 0; k < 17; k++) at[k] = __ldg(a.g.row_ptr + (r + k < cp.V ? r + k : (int64_t)cp.V));
+            }
+            double part[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int k = 0; k < 16; k++) part[k & 3] += (mine >> k) & 1u ? (double)square(at[k + 1] - at[k]) : 0.0;
+            sum = (part[0] + part[1]) + (part[2] + part[3]);
           }
-#pragma unroll
-          for (int q = 0; q < 4; q++)
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-              const float d = (there >> (4 * q + k)) & 1u ? __int2float_rn(at[q][k + 1] - at[q][k]) : 0.f;
-              x[q][k] = __fmul_rn(d, d);
-            }
-          double at_block = before, lane_before = 0.0;
-          bool found = false;
-          int bq = -1, bl = 0;
-#pragma unroll
-          for (int q = 0; q < 4; q++) {
-            if (found) break;
-            const double mine = ((double)x[q][0] + (double)x[q][1]) + ((double)x[q][2] + (double)x[q][3]);
-            double run = mine;
-            for (int o = 1; o < 32; o <<= 1) {
-              const double t = __shfl_up_sync(0xffffffffu, run, o);
-              if (lane >= o) run += t;
-            }
-            const bool some = (there >> (4 * q)) & 15u;
-            const uint32_t reach = __ballot_sync(0xffffffffu, some && at_block + run >= target), any = __ballot_sync(0xffffffffu, some);
-            // (nobody reaches it, by rounding: the last candidates of the group)
-            if (any) {
-              bq = q;
-              bl = reach ? __ffs(reach) - 1 : 31 - __clz(any);
-              lane_before = at_block + __shfl_sync(0xffffffffu, run - mine, bl);
-              found = reach != 0u;
-            }
-            at_block += __shfl_sync(0xffffffffu, run, 31);
+          double run = sum;
+          for (int o = 1; o < 32; o <<= 1) {
+            const double t = __shfl_up_sync(0xffffffffu, run, o);
+            if (lane >= o) run += t;
           }
-          const uint32_t first = (uint32_t)(lo * GROUP + bq * 128 + bl * 4);
-          uint32_t rank = first;
-          float wt = 0.f;
-          double run = lane_before;
-          bool hit = false;
-          const uint32_t its = __shfl_sync(0xffffffffu, there, bl) >> (4 * bq);
-#pragma unroll
-          for (int k = 0; k < 4; k++) {
-            const float own = bq == 0 ? x[0][k] : bq == 1 ? x[1][k] : bq == 2 ? x[2][k] : x[3][k];
-            const float t = __shfl_sync(0xffffffffu, own, bl);
-            run += (double)t;
-            if (!hit && ((its >> k) & 1u)) {
-              rank = first + k;
-              wt = t;
-              hit = run >= target;
-            }
+          const uint32_t reach = __ballot_sync(0xffffffffu, mine && before + run >= target), any = __ballot_sync(0xffffffffu, mine != 0u);
+          const int l = reach ? __ffs(reach) - 1 : 31 - __clz(any | 1u);
+          const double at_lane = before + __shfl_sync(0xffffffffu, run - sum, l);
+          const uint32_t its = __shfl_sync(0xffffffffu, mine, l);
+          const int32_t v = lo * GROUP + l * 16 + (lane & 15);
+          const bool there = (its >> (lane & 15)) & 1u;
+          const float own = there ? square(__ldg(a.g.row_ptr + v + 1) - __ldg(a.g.row_ptr + v)) : 0.f;
+          run = (double)own;
+          for (int o = 1; o < 16; o <<= 1) {
+            const double t = __shfl_up_sync(0xffffffffu, run, o, 16);
+            if ((lane & 15) >= o) run += t;
           }
+          const uint32_t hits = __ballot_sync(0xffffffffu, there && at_lane + run >= target) & 0xffffu;
+          const int k = hits ? __ffs(hits) - 1 : 31 - __clz(its | 1u);
+          const float wt = __shfl_sync(0xffffffffu, own, k);
+          const int32_t rank = lo * GROUP + l * 16 + k;
           pick = (int32_t)rank;
           pr = (float)((double)wt / total);
         }
