@@ -493,6 +493,56 @@ __device__ __forceinline__ void sum_listed(const uint32_t *bm, const Degrees &d,
   }
 }
 
+// The adjacency of a batch's lists, a row of bits each: bit j of row i, the layer's vertex j is in list i.  A list with a bitmap is
+// asked by a bit test, the others are bisected; a warp takes 32 vertices of a row, a few side by side, as every step of a search
+// waits for the one before.  (Three places a step instead of one take half of the steps and more time, 0.69 -> 0.71 ms; going
+// through short lists once more with a filter of the layer's vertices too, 0.74: a layer holds a hub many times, and
+// graphs repeat edges.)  `apart`: the places between the hubs in ut and the other lists.
+__device__ __forceinline__ void probe_rows(const int32_t *__restrict__ col, const uint32_t *__restrict__ hub_bits, int words, int32_t V, const Transit *ut,
+                                           int apart, int nh, int rows, const int32_t *layer, int L, uint32_t *out) {
+  constexpr int SIDE = 4;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, row_words = (L + 31) / 32, n = rows * row_words;
+  for (int i0 = warp; i0 < n; i0 += SIDE * warps) {
+    int32_t v[SIDE], l[SIDE], r[SIDE];   // searched for in [l, r)
+    bool edge[SIDE];
+    uint32_t word[SIDE];
+#pragma unroll
+    for (int k = 0; k < SIDE; k++) {
+      const int i = i0 + k * warps, row = i / row_words, j = (i - row * row_words) * 32 + lane;
+      v[k] = i < n && j < L ? layer[j] : V;
+      l[k] = r[k] = 0; edge[k] = false; word[k] = 0u;
+      if (v[k] < 0 || v[k] >= V) continue;
+      const Transit &t = ut[row < nh ? row : row + apart];
+      if (t.slot >= 0) word[k] = __ldg(hub_bits + (size_t)t.slot * words + ((uint32_t)v[k] >> 5));
+      else { l[k] = t.rs; r[k] = t.rs + t.deg; }
+    }
+#pragma unroll
+    for (int k = 0; k < SIDE; k++) edge[k] = (word[k] >> (v[k] & 31)) & 1u;
+    for (bool more = rows > nh; __any_sync(0xffffffffu, more);) {
+      more = false;
+      int32_t m[SIDE], c[SIDE];
+#pragma unroll
+      for (int k = 0; k < SIDE; k++) {
+        m[k] = l[k] + (r[k] - l[k]) / 2;
+        c[k] = l[k] < r[k] ? __ldg(col + m[k]) : 0;
+      }
+#pragma unroll
+      for (int k = 0; k < SIDE; k++) {
+        if (l[k] >= r[k]) continue;
+        if (c[k] == v[k]) { edge[k] = true; l[k] = r[k]; }
+        else if (c[k] < v[k]) l[k] = m[k] + 1;
+        else r[k] = m[k];
+        more |= l[k] < r[k];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < SIDE; k++) {
+      const uint32_t answers = __ballot_sync(0xffffffffu, edge[k]);
+      if (lane == 0 && i0 + k * warps < n) out[i0 + k * warps] = answers;
+    }
+  }
+}
+
 // SUMS_FAR: LADIES' group sums are in the big part.
 template <bool LADIES, bool SUMS_FAR>
 __global__ void __launch_bounds__(1024, 1)
@@ -786,28 +836,24 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
       if (tid == 0) { if (U > 0 && total > 0.0) draws += (unsigned long long)cp.L; }
       __syncthreads();
       uint32_t *adj = a.adj + (s * a.steps + cp.step) * (int64_t)adj_words(cp.stride);
-      if (nu < cp.ntr && (int64_t)nu * cp.L <= (int64_t)lay.words * 32) {
-        // repeated transits have the same entries: each list is asked once, where the union was, and the answers copied
-        probe_pairs(a.g.col, a.hub_bits, lay.words, nu * cp.L, bm, [&](int e, PairList &list, int32_t &v) {
-          const int d = e / cp.L;
-          const Transit &t = ut[d < nh ? d : cp.ntr - 1 - (d - nh)];
-          list = PairList{t.rs, t.deg, t.slot};
-          v = sh_layer[e - d * cp.L];
-          return v >= 0 && v < cp.V;
-        });
+      const int row_words = (cp.L + 31) / 32;
+      if ((int64_t)nu * row_words <= lay.words) {
+        // a row of answers for every list, where the union was; repeated transits have the same
+        probe_rows(a.g.col, a.hub_bits, lay.words, cp.V, ut, cp.ntr - nu, nh, nu, sh_layer, cp.L, bm);
         __syncthreads();
-        for (int e0 = tid - lane; e0 < cp.stride; e0 += blockDim.x) {
-          const int e = e0 + lane, i = e / cp.L;
-          bool edge = false;
-          if (e < cp.stride && i < cp.ntr) {
-            const int place = sh_mult[sh_same[i]];
+        for (int w = tid; w < adj_words(cp.stride); w += blockDim.x) {
+          uint32_t word = 0;
+          for (int e = 32 * w, end = min(e + 32, cp.ntr * cp.L); e < end;) {
+            const int i = e / cp.L, j = e - i * cp.L, n = min(cp.L - j, end - e), place = sh_mult[sh_same[i]];
             if (place >= 0) {
-              const int at = (place < nh ? place : nh + (cp.ntr - 1 - place)) * cp.L + (e - i * cp.L);
-              edge = (bm[at >> 5] >> (at & 31)) & 1u;
+              const uint32_t *at = bm + (place < nh ? place : place - (cp.ntr - nu)) * row_words + j / 32;
+              uint32_t bits = at[0] >> (j & 31);
+              if ((j & 31) + n > 32) bits |= at[1] << (32 - (j & 31));
+              word |= (n < 32 ? bits & ((1u << n) - 1u) : bits) << (e & 31);
             }
+            e += n;
           }
-          const uint32_t word = __ballot_sync(0xffffffffu, edge);
-          if (lane == 0) adj[e0 / 32] = word;
+          adj[w] = word;
         }
       } else {
         emit_adjacency(a.g, cp, sh_tr, sh_layer, adj, a.hub_slot, a.hub_bits, lay.words);
