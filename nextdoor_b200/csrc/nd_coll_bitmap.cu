@@ -65,6 +65,7 @@ constexpr int LISTED = 32;        // degrees are codes of a byte where fewer tha
 constexpr int FLIGHT = 6;         // groups a warp sums at a time (2^20 vertices 4: 0.71, 6: 0.70, 8: 0.72 ms; 2^21 0.48, 0.45, 0.45)
 constexpr int HUB = 128;          // a vertex with at least V / HUB neighbours has a bitmap of them
 constexpr int FEW = 64;           // lists with fewer than V / FEW entries in all are weighed entry by entry
+constexpr int SUB = 16;           // LADIES: lanes that add up a group of a hub (100 K vertices: 32 0.62, 16 0.595, 8 0.595, 4 0.60 ms; 2^20: 0.77, 0.77, 0.78, 0.80)
 constexpr int OCT = 8;            // list entries a thread takes at a time: 32 aligned bytes (LADIES)
 
 // The bitmap and FastGCN's CDF make the "big" part (V/8 + V/64 bytes).  It lives in shared memory when the whole layout
@@ -738,12 +739,12 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
             }
             __syncthreads();
             add_candidates(a.g, a.term, ut, cp.ntr, nh, nu, pre, octs, slot, acc, lay.group_bits);
-            for (int q = warp; q < here * nh; q += warps) {   // hubs: a warp goes to a group of one
+            for (int q = tid / SUB; q < here * nh; q += blockDim.x / SUB) {   // hubs: a few lanes go to a group of one
               const int k = q / nh;
               const Transit t = ut[q - k * nh];
               const int32_t *at = a.hub_starts + (size_t)t.slot * (groups + 1) + sh_slot_group[k];
               const int32_t end = __ldg(at + 1);
-              for (int32_t e = __ldg(at) + lane; e < end; e += 32)
+              for (int32_t e = __ldg(at) + tid % SUB; e < end; e += SUB)
                 atomicAdd(acc + ((size_t)k << lay.group_bits) + (__ldg(a.hub_ids + e) & (n - 1)), __ldg(a.hub_terms + e) * (double)t.mult);
             }
             __syncthreads();
