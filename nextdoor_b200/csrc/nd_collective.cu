@@ -40,7 +40,7 @@ constexpr int CTHREADS = 256;
 // first and all their (transit, layer) pairs are probed together: the transits' lists are flattened over the
 // CTA, every entry asks a filter of the layer's ids in shared memory, and the few that pass look for the id.
 // A list longer than PROBE_RATIO times the layer is bisected for every id instead.  (One bisection per
-// (transit, slot) pair, 205 M of them for 10,000 samples of 5 x 64 x 64 on 57 K vertices: 1.04 ms, the kernel now 0.24.)
+// (transit, slot) pair, 205 M of them for 10,000 samples of 5 x 64 x 64 on 57 K vertices: 1.04 ms, the kernel now 0.20.)
 // The flags of the edges that were found are the adjacency as it is kept: a bit per entry (the two arrays of the
 // reference's form, 1.6 GB for those samples, took 0.1 ms of 0.54).
 constexpr int FILTER_WORDS = 256;   // 8192 bits per layer
@@ -48,25 +48,27 @@ constexpr int PROBE_RATIO = 8;
 
 struct RefLayout {
   int per_pass;                                                        // layers drawn and probed together
-  uint32_t off_ids, off_tr, off_rs, off_deg, off_pre, off_filter, off_flags;    // bytes
+  uint32_t off_red, off_rec, off_ids, off_pre, off_filter, off_flags;           // bytes
   uint32_t bytes;
   int flag_words;                                                      // per transit
-  uint32_t inv_L;                                                      // 2^32 / L, rounded up (L > 1): x / L is the high half of x * inv_L below 2^16
+  int words;                                                           // of a layer's adjacency
+  uint32_t inv_L, inv_words;                                           // 2^32 / L, rounded up: x / L is the high half of x * inv_L below 2^16
 };
 
 static RefLayout ref_layout(int steps, int B, int L) {
   RefLayout r;
   const int ntr = B > L ? B : L;
   r.flag_words = (L + 31) / 32;
-  r.inv_L = L > 1 ? (uint32_t)((((uint64_t)1 << 32) + (uint32_t)L - 1) / (uint32_t)L) : 0u;
+  r.words = adj_words(ntr * L);
+  r.inv_L = (uint32_t)((((uint64_t)1 << 32) + (uint32_t)L - 1) / (uint32_t)L);
+  r.inv_words = (uint32_t)((((uint64_t)1 << 32) + (uint32_t)r.words - 1) / (uint32_t)r.words);
   // (a layer's filter is a kilobyte: no more than 24 of them fit, and the sums below stay in 32 bits)
   for (r.per_pass = std::min(steps, 24);; r.per_pass--) {
     const uint32_t k = (uint32_t)r.per_pass, nt = k * (uint32_t)ntr;
     uint32_t off = 0;
+    r.off_red = off; off += 8u * (CTHREADS / 32);
+    r.off_rec = off; off += 8u * (nt + 1u);
     r.off_ids = off; off += 4u * (k + 1u) * (uint32_t)L;   // the layer before the pass too: its transits
-    r.off_tr = off; off += 4u * nt;
-    r.off_rs = off; off += 4u * nt;
-    r.off_deg = off; off += 4u * nt;
     r.off_pre = off; off += 4u * (nt + 1u);
     r.off_filter = off; off += 4u * k * FILTER_WORDS;
     r.off_flags = off; off += 4u * nt * (uint32_t)r.flag_words;
@@ -74,6 +76,9 @@ static RefLayout ref_layout(int steps, int B, int L) {
     if (r.per_pass == 1 || off <= 24u * 1024u) return r;
   }
 }
+
+// x / n of a kernel's RefLayout, inv = 2^32 / n rounded up (0: n is 1): x below 2^16, or 0 is the only quotient
+__device__ __forceinline__ int quotient(int x, uint32_t inv) { return inv ? (int)__umulhi((uint32_t)x, inv) : x; }
 
 // the last i of [lo, hi] with pre[i] <= f, lo if there is none
 __device__ __forceinline__ int last_at_most(const uint32_t *pre, int lo, int hi, uint32_t f) {
@@ -85,13 +90,16 @@ __device__ __forceinline__ int last_at_most(const uint32_t *pre, int lo, int hi,
 }
 
 __global__ void __launch_bounds__(CTHREADS)
-coll_ref_kernel(NdGraphView g, CollParams cp, RefLayout lay, int steps, int64_t S, const int32_t *__restrict__ initial, int32_t *__restrict__ out,
+coll_ref_kernel(NdGraphView g, CollParams cp, const __grid_constant__ ndrng::RoundKeys keys, RefLayout lay, int steps, int64_t S, const int32_t *__restrict__ initial, int32_t *__restrict__ out,
                 uint32_t *__restrict__ adj, unsigned long long *__restrict__ stats) {
   extern __shared__ __align__(16) unsigned char sm[];
-  __shared__ uint32_t red[CTHREADS / 32];
+  uint2 *red = reinterpret_cast<uint2 *>(sm + lay.off_red);
+  // The transits whose lists are streamed, those without neighbours left out: pre[l] entries come before the list, and entry f
+  // of all of them is rec[l].x + f of the graph's, of transit rec[l].y & 0xffff and layer rec[l].y >> 16.  Those whose lists are
+  // bisected come from the arrays' ends: rec (row start, as above), pre the length.
+  int2 *rec = reinterpret_cast<int2 *>(sm + lay.off_rec);
   int32_t *ids = reinterpret_cast<int32_t *>(sm + lay.off_ids);
-  int32_t *tr = reinterpret_cast<int32_t *>(sm + lay.off_tr), *rs = reinterpret_cast<int32_t *>(sm + lay.off_rs), *deg_of = reinterpret_cast<int32_t *>(sm + lay.off_deg);
-  __shared__ int heavy;   // transits whose lists are bisected: the first entries of tr
+  __shared__ int heavy;
   uint32_t *pre = reinterpret_cast<uint32_t *>(sm + lay.off_pre);
   uint32_t *filter = reinterpret_cast<uint32_t *>(sm + lay.off_filter), *flags = reinterpret_cast<uint32_t *>(sm + lay.off_flags);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, L = cp.L;
@@ -107,82 +115,93 @@ coll_ref_kernel(NdGraphView g, CollParams cp, RefLayout lay, int steps, int64_t 
       for (int i = tid; i < nt * lay.flag_words; i += CTHREADS) flags[i] = 0u;
       __syncthreads();
       for (int q = tid; q < kn * L; q += CTHREADS) {
-        const int k = q / L, j = q - k * L;
-        Rng rng(cp.seed, (uint32_t)(cp.first_sample + s), (uint32_t)(k0 + k), (uint32_t)j);
-        const int32_t id = rng.rand_int(cp.V);
+        const int k = quotient(q, lay.inv_L), j = q - k * L;
+        uint32_t o[4];
+        ndrng::philox4x32_10((uint32_t)(cp.first_sample + s), (uint32_t)(k0 + k), (uint32_t)j, 0u, keys, o);
+        const int32_t id = ndrng::rand_int_from(ndrng::u32_to_uniform(o[0]), cp.V);
         ids[L + q] = id;
         out[s * cp.fs + (int64_t)k0 * L + q] = id;
         atomicOr(filter + k * FILTER_WORDS + (((uint32_t)id >> 5) & (FILTER_WORDS - 1)), 1u << (id & 31));
       }
       __syncthreads();
-      // rows of the transits; exclusive prefix of the lengths that are streamed
+      // rows of the transits; their places in the list, and how many entries come before them
       uint32_t carry = 0;
+      int n_live = 0;
       for (int i0 = 0; i0 < nt; i0 += CTHREADS) {
         const int i = i0 + tid;
         uint32_t n = 0;
+        int2 r = make_int2(0, i);
         if (i < nt) {
           const int32_t t = i < n0 ? (k0 == 0 ? initial[s * cp.B + i] : ids[i]) : ids[L + (i - n0)];
-          int32_t at = 0, deg = 0;
-          if (t >= 0 && t < cp.V) { at = __ldg(g.row_ptr + t); deg = __ldg(g.row_ptr + t + 1) - at; }
+          int32_t deg = 0;
+          if (t >= 0 && t < cp.V) { r.x = __ldg(g.row_ptr + t); deg = __ldg(g.row_ptr + t + 1) - r.x; }
+          if (i >= n0) r.y |= (1 + quotient(i - n0, lay.inv_L)) << 16;
           if (deg > PROBE_RATIO * L) {   // bisected
-            const int h = atomicAdd(&heavy, 1);
-            tr[h] = i;
+            const int h = nt - atomicAdd(&heavy, 1);
+            rec[h] = r;
+            pre[h] = (uint32_t)deg;
+          } else {
+            n = (uint32_t)deg;
           }
-          rs[i] = at;
-          deg_of[i] = deg;
-          n = deg > PROBE_RATIO * L ? 0u : (uint32_t)deg;
         }
         uint32_t inc = n;
         for (int o = 1; o < 32; o <<= 1) {
           const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
           if (lane >= o) inc += t;
         }
-        if (lane == 31) red[warp] = inc;
+        const uint32_t live = __ballot_sync(0xffffffffu, n > 0);
+        if (lane == 31) red[warp] = make_uint2(inc, __popc(live));
         __syncthreads();
-        uint32_t before = carry + inc - n, all = 0;
+        uint32_t before = carry + inc - n;
+        int at = n_live + __popc(live & ((1u << lane) - 1u));
         for (int w = 0; w < CTHREADS / 32; w++) {
-          if (w < warp) before += red[w];
-          all += red[w];
+          const uint2 x = red[w];
+          if (w < warp) { before += x.x; at += (int)x.y; }
+          carry += x.x;
+          n_live += (int)x.y;
         }
-        if (i < nt) pre[i] = before;
-        carry += all;
+        if (n > 0) {
+          pre[at] = before;
+          rec[at] = make_int2(r.x - (int32_t)before, r.y);
+        }
+        if (i0 + CTHREADS >= nt && tid == 0) pre[n_live] = carry;
         __syncthreads();
       }
       // the entries of the short lists: a warp takes a run of them, a lane four neighbouring ones at a time
       constexpr int LOADS = 4;
       const uint32_t chunks = (carry + 32 * LOADS - 1) / (32 * LOADS), each = (chunks + CTHREADS / 32 - 1) / (CTHREADS / 32) * (32 * LOADS);
       const uint32_t run_end = min(((uint32_t)warp + 1u) * each, carry);
-      int from = 0;   // transit of the chunk's first entry: the last with pre <= c0
-      if (warp * each < run_end) from = last_at_most(pre, 0, nt - 1, warp * each);
+      int from = 0;   // list of the chunk's first entry: the last with pre <= c0
+      if (warp * each < run_end) from = last_at_most(pre, 0, n_live - 1, warp * each);
       for (uint32_t c0 = warp * each; c0 < run_end; c0 += 32 * LOADS) {
-        int32_t v[LOADS];
-        int at[LOADS];
+        int32_t v[LOADS], who[LOADS];
         const uint32_t c1 = min(c0 + 32 * LOADS, run_end) - 1;
-        int to;   // transit of its last entry: seldom 32 further on
-        const uint32_t within = __ballot_sync(0xffffffffu, from + 1 + lane < nt && pre[from + 1 + lane] <= c1);
-        if (within == 0xffffffffu) to = last_at_most(pre, from + 32, nt - 1, c1);
+        int to;   // list of its last entry: seldom 32 further on
+        const uint32_t within = __ballot_sync(0xffffffffu, from + 1 + lane < n_live && pre[from + 1 + lane] <= c1);
+        if (within == 0xffffffffu) to = last_at_most(pre, from + 32, n_live - 1, c1);
         else to = from + __popc(within);
         const uint32_t f0 = c0 + (uint32_t)(LOADS * lane);
         int lo = f0 <= c1 ? last_at_most(pre, from, to, f0) : to;
+        int2 r = rec[lo];
+        uint32_t end = pre[lo + 1];
 #pragma unroll
         for (int j = 0; j < LOADS; j++) {
           const uint32_t f = f0 + j;
           v[j] = -1;
           if (f <= c1) {
-            while (lo < to && pre[lo + 1] <= f) lo++;
-            v[j] = __ldg(g.col + rs[lo] + (int32_t)(f - pre[lo]));
+            if (f == end) { lo++; r = rec[lo]; end = pre[lo + 1]; }
+            v[j] = __ldg(g.col + (r.x + (int32_t)f));
           }
-          at[j] = lo;
+          who[j] = r.y;
         }
         from = to;
 #pragma unroll
         for (int j = 0; j < LOADS; j++) {
-          const int x = at[j] - n0, k = x < 0 ? 0 : 1 + (L > 1 ? (int)__umulhi((uint32_t)x, lay.inv_L) : x);
-          const bool may = v[j] >= 0 && ((filter[k * FILTER_WORDS + (((uint32_t)v[j] >> 5) & (FILTER_WORDS - 1))] >> (v[j] & 31)) & 1u);
+          const bool may = v[j] >= 0 && ((filter[(who[j] >> 16) * FILTER_WORDS + (((uint32_t)v[j] >> 5) & (FILTER_WORDS - 1))] >> (v[j] & 31)) & 1u);
           for (uint32_t left = __ballot_sync(0xffffffffu, may); left; left &= left - 1) {   // the warp looks for each of them
             const int src = __ffs(left) - 1;
             const int32_t id = __shfl_sync(0xffffffffu, v[j], src);
-            const int i = __shfl_sync(0xffffffffu, at[j], src), layer = __shfl_sync(0xffffffffu, k, src);
+            const int w_i = __shfl_sync(0xffffffffu, who[j], src), i = w_i & 0xffff, layer = w_i >> 16;
             for (int w = 0; w < lay.flag_words; w++) {
               const int q = 32 * w + lane;
               const uint32_t found = __ballot_sync(0xffffffffu, q < L && ids[L + layer * L + q] == id);
@@ -193,24 +212,26 @@ coll_ref_kernel(NdGraphView g, CollParams cp, RefLayout lay, int steps, int64_t 
       }
       const int nheavy = heavy;
       for (int q = tid; q < nheavy * L; q += CTHREADS) {
-        const int i = tr[q / L], j = q % L, k = i < n0 ? 0 : 1 + (i - n0) / L;
-        const int32_t id = ids[L + k * L + j];
-        int32_t lo = rs[i], hi = rs[i] + deg_of[i];
+        const int h = nt - q / L, j = q % L;
+        const int2 r = rec[h];
+        const int i = r.y & 0xffff;
+        const int32_t id = ids[L + (r.y >> 16) * L + j], end = r.x + (int32_t)pre[h];
+        int32_t lo = r.x, hi = end;
         while (lo < hi) {
           const int32_t m = lo + ((hi - lo) >> 1);
           if (__ldg(g.col + m) < id) lo = m + 1; else hi = m;
         }
-        if (lo < rs[i] + deg_of[i] && __ldg(g.col + lo) == id) atomicOr(flags + i * lay.flag_words + (j >> 5), 1u << (j & 31));
+        if (lo < end && __ldg(g.col + lo) == id) atomicOr(flags + i * lay.flag_words + (j >> 5), 1u << (j & 31));
       }
       __syncthreads();
       // the layers' adjacency: the flags are the bits where a transit's are whole words
-      const int words = adj_words(cp.stride);
+      const int words = lay.words;
       for (int q = tid; q < kn * words; q += CTHREADS) {
-        const int k = q / words, w = q - k * words;
+        const int k = kn == 1 ? 0 : quotient(q, lay.inv_words), w = q - k * words;
         const int first = k == 0 ? 0 : n0 + (k - 1) * L, n = k == 0 ? n0 : L;
         uint32_t bits = 0u;
         if ((L & 31) == 0) {
-          if (w / lay.flag_words < n) bits = flags[first * lay.flag_words + w];
+          if (w < n * lay.flag_words) bits = flags[first * lay.flag_words + w];
         } else {
           for (int e = 32 * w; e < 32 * w + 32;) {   // up to the end of the word, of the transit's flags' word or of its row
             const int i = e / L, j = e - i * L, len = min(min(32 * w + 32 - e, L - j), 32 - (j & 31));
@@ -463,7 +484,7 @@ int nd_collective_sample(nd_sampler *s, int mode) {
     const int per_sm = lay.bytes <= 24u * 1024u ? 8 : 1;
     nd_phase_begin(s, ND_PHASE_NEXT);
     coll_ref_kernel<<<(int)std::min<int64_t>(S, (int64_t)s->dev.sms * per_sm), CTHREADS, lay.bytes, st>>>(
-        gv, cp, lay, p.steps, S, s->d_initial, s->d_out, s->d_adj, s->d_stats);
+        gv, cp, ndrng::RoundKeys(p.seed), lay, p.steps, S, s->d_initial, s->d_out, s->d_adj, s->d_stats);
     nd_phase_end(s);
     nd_count_launches(1);
     ND_CUDA(cudaGetLastError());
