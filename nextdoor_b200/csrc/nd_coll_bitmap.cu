@@ -64,6 +64,7 @@ constexpr int BIG_DEGREE = 2048;  // from here a vertex is listed and its code i
 constexpr int LISTED = 32;        // degrees are codes of a byte where fewer than V / LISTED vertices do not fit one
 constexpr int FLIGHT = 6;         // groups a warp sums at a time (2^20 vertices 4: 0.71, 6: 0.70, 8: 0.72 ms; 2^21 0.48, 0.45, 0.45)
 constexpr int HUB = 128;          // a vertex with at least V / HUB neighbours has a bitmap of them
+constexpr int32_t SHARED_V = 1 << 18;   // see plan_of()
 constexpr int FEW = 64;           // lists with fewer than V / FEW entries in all are weighed entry by entry
 constexpr int SUB = 16;           // LADIES: lanes that add up a group of a hub (100 K vertices: 32 0.62, 16 0.595, 8 0.595, 4 0.60 ms; 2^20: 0.77, 0.77, 0.78, 0.80)
 constexpr int OCT = 8;            // list entries a thread takes at a time: 32 aligned bytes (LADIES)
@@ -1250,7 +1251,7 @@ struct Plan {
   int threads, per_sm;
 };
 
-// Two CTAs of 512 threads per SM where both layouts fit, else one of 1024.
+// Two CTAs of 512 threads per SM where both layouts fit, or one, three or four by the number of samples, else one of 1024.
 Plan plan_of(const nd_sampler *s) {
   const int32_t V = s->g->V;
   const int L = s->p.fanout[0], B = s->p.batch, ntr = B > L ? B : L;
@@ -1303,9 +1304,32 @@ Plan plan_of(const nd_sampler *s) {
     fits(LADIES_GROUP_BITS, true, optin);
     if (ladies && l.slots < 1) { l.slots = 1; l.bytes += 8u << LADIES_GROUP_BITS; }
   }
+  // Where two fit an SM: with no more samples than SMs a sample has one for itself (140 batches of 64, 2 layers of 64: 70 K
+  // vertices, FastGCN 67 -> 63 us, LADIES 95 -> 82; 330 K: 91 -> 82, 120 -> 94; but 56 -> 58 where FastGCN's batches, layers and graph
+  // are all small: 32, 120 K).  With many samples, three or four smaller CTAs
+  // overlap better while the graph is small (70 K, 1024 batches, two, three, four an SM: 215, 206, 187; 322, 314, 290; 500 K,
+  // 640: 412, 448 with three), unless their last round would be nearly empty (700: 166, 155, 158) or, LADIES, there were not
+  // accumulators for half of the draws at a time (batches and layers of 100, 100 K, 520: 475, 533), for three quarters on larger
+  // graphs (200 K, 64, 1024: 348, 356; but layers of 32 on 250 K 289, 251).  The groups stay: tables of
+  // the graph go by them.
   Plan p;
-  p.threads = two ? 512 : 1024;
   p.per_sm = two ? 2 : 1;
+  const bool small = V <= SHARED_V / 2;
+  if (two && s->S <= s->dev.sms) {
+    if (ladies || !small || ntr > 32) p.per_sm = 1;
+  }
+  if (two && p.per_sm == 1) {
+    fits(l.group_bits, false, optin);
+  } else if (two && s->S > 2 * s->dev.sms && V <= SHARED_V) {
+    for (int k = 4; k > 2 && p.per_sm == 2; k--) {
+      const int64_t round = (int64_t)k * s->dev.sms, rounds = (s->S + round - 1) / round;
+      if (10 * s->S < 7 * rounds * round) continue;
+      const Layout with_two = l;
+      if (fits(l.group_bits, false, optin / (uint32_t)k - 1024u) && (!ladies || 4 * l.slots >= (small ? 2 * L : 3 * L))) p.per_sm = k;
+      else l = with_two;
+    }
+  }
+  p.threads = 1024 / p.per_sm / 32 * 32;
   p.lay = l;
   return p;
 }

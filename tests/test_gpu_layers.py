@@ -293,3 +293,23 @@ def test_fastgcn_weights_of_listed_vertices(nd, ndo, monkeypatch, V, share, larg
     assert np.array_equal(aux["prob"].reshape(-1), exp["prob"].reshape(-1))
     assert np.array_equal(aux["adj_row"], exp["adj_row"]) and np.array_equal(aux["adj_col"], exp["adj_col"])
     assert s.stats()["union_unique"] == exp["counters"]["union_unique"]
+
+
+@pytest.mark.parametrize("V,B,L", [(3000, 24, 33), (70_000, 64, 64)])
+@pytest.mark.parametrize("app", [8, 9])
+def test_layers_by_number_of_samples(nd, app, V, B, L):
+    """One to four samples share an SM by how many there are (148 SMs); a sample's layers do not depend on it."""
+    g = nd.Graph.rmat(V, 10 * V, seed=1)
+    init = np.random.default_rng(V).integers(0, V, 600 * B).astype(np.int32)
+
+    def job(first, S):
+        s = nd.Sampler(g, nd.app_params(app, steps=2, fanout=L, batch=B, seed=3), num_samples=S, first_sample=first, initial=init[first * B:(first + S) * B])
+        s.sample()
+        aux = s.aux()
+        return [x.reshape(S, -1) for x in (s.final_samples(), aux["adj_row"], aux["adj_col"], aux["prob"])]
+
+    one = [np.concatenate(x) for x in zip(*(job(first, 120) for first in range(0, 600, 120)))]
+    for first, S in [(0, 600), (600 - 148, 148), (7, 149), (150, 296), (0, 312), (3, 444), (100, 445)]:
+        for got, exp in zip(job(first, S)[:3], one):
+            assert np.array_equal(got, exp[first:first + S])
+        assert np.allclose(job(first, S)[3], one[3][first:first + S], rtol=1e-6, atol=0)   # 32-bit results of 64-bit sums in another order
