@@ -7,7 +7,7 @@
 // integer weights sum exactly).
 //
 // What bounds it, and what is done about it (2^20 vertices, 1024 batches of 64, 2 layers of 64: FastGCN
-// 4.8 -> 0.70 ms, LADIES 5.7 -> 0.80 ms).  One CTA fills an SM, and neither memory nor issue slots are full: FastGCN issued
+// 4.8 -> 0.665 ms, LADIES 5.7 -> 0.725 ms).  One CTA fills an SM, and neither memory nor issue slots are full: FastGCN issued
 // in 58 % of the cycles at 0.89 ms (5.5 GB out of the L2 at 18 % of its rate), LADIES in 57 % at 1.07 (610 M
 // instructions for 131 M list entries, the distinct ones of 313 M), its shared memory busy in half of them; the warps
 // wait for barriers between the phases, for shared memory and for loads:
@@ -125,10 +125,28 @@ struct Transit { int32_t rs, deg, mult, slot; };
 
 constexpr uint32_t NO_SLOT = 255u;
 
-// exclusive (uint32) or inclusive (double) scan of an array by the whole CTA: every thread owns a contiguous
-// chunk, the chunk totals are scanned through warp shuffles
+// exclusive scan of an array by the whole CTA; its sum.  A few words are one warp's (every thread adding up all warps' sums takes a
+// thousand cycles); else every thread owns a contiguous chunk and the chunks' sums are scanned through shuffles.
 __device__ __forceinline__ uint32_t scan_u32(uint32_t *a, int n, uint32_t *red) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  if (n <= 128) {
+    if (warp == 0) {
+      uint32_t carry = 0;
+      for (int i0 = 0; i0 < n; i0 += 32) {
+        const uint32_t own = i0 + lane < n ? a[i0 + lane] : 0u;
+        uint32_t inc = own;
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= o) inc += t;
+        }
+        if (i0 + lane < n) a[i0 + lane] = carry + inc - own;
+        carry += __shfl_sync(0xffffffffu, inc, 31);
+      }
+      if (lane == 0) red[0] = carry;
+    }
+    __syncthreads();
+    return red[0];
+  }
   const int per = (n + blockDim.x - 1) / blockDim.x;
   const int b = min((int)threadIdx.x * per, n), e = min(b + per, n);
   uint32_t sum = 0;
@@ -150,34 +168,81 @@ __device__ __forceinline__ uint32_t scan_u32(uint32_t *a, int n, uint32_t *red) 
   return total;
 }
 
-// (a warp takes whole rows of 32, so that neighbouring lanes read neighbouring words.  The adds that lead to two
-// neighbouring sums come in different orders, so the sums may differ by a rounding where nothing lies between them: an
-// element of zero takes over the sum before it, and the first sum to reach a target is never one of those.)
-__device__ __forceinline__ void scan_f64(double *a, int n, double *red) {
+// Inclusive scan of n doubles by the whole CTA, get(i) gives the i-th to be added (in place is fine).  A thread owns P neighbouring
+// ones, read and written two at a time; of eight each second thread starts at another pair, or the accesses of a quarter
+// of a warp would meet in two banks' places (rows of 32 scanned by shuffles and every warp's base added up from memory, with the
+// counts' sums and the lists' scan done likewise by all threads: 1024 batches on 2^20 vertices FastGCN 0.69 -> 0.665 ms, LADIES
+// 0.775 -> 0.725; 600 of 32, layers of 100, on 900 K 0.43 -> 0.40).  The adds that lead to two neighbouring sums come in different orders,
+// so the sums may differ by a rounding where nothing lies between them: an element of zero takes over the sum before it,
+// and the first sum to reach a target is never one of those.  (Values are made relative to the warp first; the warps' bases are
+// added up in order from what their last elements become, so what is equal stays equal.)
+template <int P, class Get>
+__device__ __forceinline__ void scan_f64(double *a, int n, double *red, Get get) {
+  constexpr int PAIRS = P / 2;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  const int per = ((n + 31) / 32 + warps - 1) / warps * 32, b = warp * per;
-  double carry = 0.0;
-  for (int i0 = b; i0 < b + per && i0 < n; i0 += 32) {
-    const int i = i0 + lane;
-    const double own = i < n ? a[i] : 0.0;
-    double run = own;
-    for (int o = 1; o < 32; o <<= 1) {
-      const double t = __shfl_up_sync(0xffffffffu, run, o);
-      if (lane >= o) run += t;
+  const int turn = PAIRS == 4 ? (threadIdx.x >> 1) & 3 : 0;
+  double start = 0.0;   // the sum before the block
+  for (int b0 = 0; b0 < n; b0 += P * (int)blockDim.x) {
+    const int b = b0 + P * (int)threadIdx.x;
+    double2 d[PAIRS];
+#pragma unroll
+    for (int k = 0; k < PAIRS; k++) {
+      const int i = b + 2 * ((k + turn) & (PAIRS - 1));
+      d[k] = i + 1 < n ? get.two(i) : make_double2(i < n ? get.one(i) : 0.0, 0.0);
     }
-    run += carry;
-    const uint32_t upto = __ballot_sync(0xffffffffu, own != 0.0) & (0xffffffffu >> (31 - lane));
-    const double last = __shfl_sync(0xffffffffu, run, upto ? 31 - __clz(upto) : 0);
-    run = upto ? last : carry;
-    if (i < n) a[i] = run;
-    carry = __shfl_sync(0xffffffffu, run, 31);
+    if (PAIRS == 4) {   // pair k is at (k - turn) & 3
+      if (turn & 1) { const double2 x = d[3]; d[3] = d[2]; d[2] = d[1]; d[1] = d[0]; d[0] = x; }
+      if (turn & 2) { double2 x = d[0]; d[0] = d[2]; d[2] = x; x = d[1]; d[1] = d[3]; d[3] = x; }
+    }
+    double sum = 0.0;
+#pragma unroll
+    for (int k = 0; k < PAIRS; k++) { sum += d[k].x; sum += d[k].y; }
+    double before = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+      const double t = __shfl_up_sync(0xffffffffu, before, o);
+      if (lane >= o) before += t;
+    }
+    before = __shfl_up_sync(0xffffffffu, before, 1);
+    if (lane == 0) before = 0.0;
+    const bool some = sum != 0.0;
+    double last = before;
+#pragma unroll
+    for (int k = 0; k < PAIRS; k++) { last += d[k].x; last += d[k].y; }
+    const uint32_t those = __ballot_sync(0xffffffffu, some), left = those & ((1u << lane) - 1u);
+    const double taken = __shfl_sync(0xffffffffu, last, left ? 31 - __clz(left) : 0);   // what elements of zero take over
+    double take = left ? taken : 0.0;
+    const double end = __shfl_sync(0xffffffffu, last, those ? 31 - __clz(those) : 0);
+    if (lane == 0) red[warp] = those ? end : 0.0;
+    __syncthreads();
+    double base = start, next = start;
+#pragma unroll 8
+    for (int w = 0; w < warps; w++) {
+      next += red[w];
+      if (w + 1 == warp) base = next;
+    }
+    start = next;
+    double run = before;
+#pragma unroll
+    for (int k = 0; k < PAIRS; k++) {
+      run += d[k].x;
+      if (d[k].x != 0.0) take = run;
+      d[k].x = base + take;
+      run += d[k].y;
+      if (d[k].y != 0.0) take = run;
+      d[k].y = base + take;
+    }
+    if (PAIRS == 4) {
+      if (turn & 1) { const double2 x = d[0]; d[0] = d[1]; d[1] = d[2]; d[2] = d[3]; d[3] = x; }
+      if (turn & 2) { double2 x = d[0]; d[0] = d[2]; d[2] = x; x = d[1]; d[1] = d[3]; d[3] = x; }
+    }
+#pragma unroll
+    for (int k = 0; k < PAIRS; k++) {
+      const int i = b + 2 * ((k + turn) & (PAIRS - 1));
+      if (i + 1 < n) *reinterpret_cast<double2 *>(a + i) = d[k];
+      else if (i < n) a[i] = d[k].x;
+    }
+    __syncthreads();
   }
-  if (lane == 0) red[warp] = carry;
-  __syncthreads();
-  double base = 0.0;
-  for (int w = 0; w < warp; w++) base += red[w];
-  for (int i = b + lane; i < b + per && i < n; i += 32) a[i] += base;
-  __syncthreads();
 }
 
 // eight consecutive words at an address that is a multiple of 32
@@ -233,6 +298,26 @@ struct Sum {
   }
   static __device__ __forceinline__ double value(const uint2 &s) { return (double)s.x + (double)(1 << SUM_BITS) * (double)s.y; }
 };
+
+struct Doubles {
+  const double *a;
+  __device__ __forceinline__ double one(int i) const { return a[i]; }
+  __device__ __forceinline__ double2 two(int i) const { return *reinterpret_cast<const double2 *>(a + i); }
+};
+struct Sums {
+  const uint2 *a;
+  __device__ __forceinline__ double one(int i) const { return Sum::value(a[i]); }
+  __device__ __forceinline__ double2 two(int i) const {
+    const uint4 s = *reinterpret_cast<const uint4 *>(a + i);
+    return make_double2(Sum::value(make_uint2(s.x, s.y)), Sum::value(make_uint2(s.z, s.w)));
+  }
+};
+// few elements: two a thread
+template <class Get>
+__device__ __forceinline__ void scan_groups(double *a, int n, double *red, Get get) {
+  if (n <= 2 * (int)blockDim.x) scan_f64<2>(a, n, red, get);
+  else scan_f64<8>(a, n, red, get);
+}
 
 // FastGCN: the entries of the lists without bitmaps into the union; with WEIGHTS what they add to it goes to the groups' sums
 // and is counted (the number the thread has added).
@@ -573,16 +658,23 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
   uint32_t *sh_firsts = reinterpret_cast<uint32_t *>(sh_slot_group + cp.L);   // draws that are the first of their group, as bits
   uint8_t *slot = (LADIES && !SUMS_FAR ? smem : big) + lay.off_slot;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
-  unsigned long long ids_sum = 0, uniq_sum = 0, draws = 0;   // thread 0
+  unsigned long long ids_sum = 0, uniq_sum = 0, draws = 0;   // the thread's; draws: thread 0's
   for (int64_t s = blockIdx.x; s < a.S;) {
     for (int step = 0; step < a.steps; step++) {
       cp.step = step;
       cp.ntr = step == 0 ? cp.B : cp.L;
       const int32_t *tr = transits_of(cp, a.initial, a.out, s);
       if (tid == 0) { sh_hubs = 0; sh_rest = 0; }
+      int32_t rs0 = 0, end0 = 0, slot0 = -1;   // row and slot of the thread's first transit, asked for before the repeated ones are found
       for (int i = tid; i < cp.ntr; i += blockDim.x) {
-        sh_tr[i] = step == 0 ? tr[i] : sh_layer[i];
+        const int32_t t = step == 0 ? tr[i] : sh_layer[i];
+        sh_tr[i] = t;
         sh_mult[i] = 1;
+        if (i == tid && t >= 0 && t < cp.V) {
+          rs0 = __ldg(a.g.row_ptr + t);
+          end0 = __ldg(a.g.row_ptr + t + 1);
+          slot0 = __ldg(a.hub_slot + t);
+        }
       }
       __syncthreads();
       // ---- the batch's transits, each once: the hubs from the front of the list, the others from its end
@@ -595,27 +687,23 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
         if (first != j) atomicAdd(sh_mult + first, 1);
       }
       __syncthreads();
-      unsigned long long ids = 0;
       for (int i = tid; i < cp.ntr; i += blockDim.x) {
         const int32_t t = sh_tr[i];
         const bool valid = t >= 0 && t < cp.V, first = sh_same[i] == i;
         int place = -1;
         if (valid) {
-          const int32_t rs = __ldg(a.g.row_ptr + t), deg = __ldg(a.g.row_ptr + t + 1) - rs;
-          ids += (unsigned long long)deg;
+          const int32_t rs = i == tid ? rs0 : __ldg(a.g.row_ptr + t), deg = (i == tid ? end0 : __ldg(a.g.row_ptr + t + 1)) - rs;
+          ids_sum += (unsigned long long)deg;
           if (first) {
-            const int32_t slot = __ldg(a.hub_slot + t);
+            const int32_t slot = i == tid ? slot0 : __ldg(a.hub_slot + t);
             place = slot >= 0 && (!LADIES || a.hub_sums) ? atomicAdd(&sh_hubs, 1) : cp.ntr - 1 - atomicAdd(&sh_rest, 1);
             ut[place] = Transit{rs, deg, sh_mult[i], slot};
           }
         }
         if (first) sh_mult[i] = place;
       }
-      for (int o = 16; o > 0; o >>= 1) ids += __shfl_xor_sync(0xffffffffu, ids, o);
-      if (lane == 0) reinterpret_cast<unsigned long long *>(red)[warp] = ids;
       __syncthreads();
       const int nh = sh_hubs, nu = nh + sh_rest;
-      if (tid == 0) for (int w = 0; w < warps; w++) ids_sum += reinterpret_cast<unsigned long long *>(red)[w];
       // ---- the union: hubs' bitmaps, then the other lists
       for (int w4 = tid; w4 < lay.words / 4; w4 += blockDim.x) {
         uint4 u = make_uint4(0u, 0u, 0u, 0u);
@@ -669,28 +757,28 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
           seen += __popc(u.x) + __popc(u.y) + __popc(u.z) + __popc(u.w);
         }
       }
-      seen = __reduce_add_sync(0xffffffffu, seen);
-      if (lane == 0) red_u[warp] = seen;
-      __syncthreads();
-      uint32_t U = 0;
-      for (int w = 0; w < warps; w++) U += red_u[w];
-      if (tid == 0) uniq_sum += U;
-      if (!LADIES) {
+      uniq_sum += seen;
+      const bool candidates = __syncthreads_or(seen != 0u);
+      if (LADIES) {
+        scan_groups(gcdf, groups, red, Doubles{gcdf});
+      } else if (!a.n_huge) {
+        scan_groups(gcdf, groups, red, Sums{gsum});
+      } else {
         for (int k = tid; k < groups; k += blockDim.x) gcdf[k] = Sum::value(gsum[k]);   // (in its place)
         __syncthreads();
-        if (a.n_huge) {
+        {
           for (int i = tid; i < a.n_huge; i += blockDim.x) {
             const NdBigVertex v = a.huge[i];
             if ((bm[v.v >> 5] >> (v.v & 31)) & 1u) atomicAdd(gcdf + v.v / GROUP, (double)v.weight);
           }
           __syncthreads();
         }
+        scan_groups(gcdf, groups, red, Doubles{gcdf});
       }
-      scan_f64(gcdf, groups, red);
       const double total = groups > 0 ? gcdf[groups - 1] : 0.0;
       // ---- the layer's draws
       if (LADIES) {
-        const bool any = U > 0 && total > 0.0;
+        const bool any = candidates && total > 0.0;
         const int n = 1 << lay.group_bits;
         for (int j = tid; j < cp.L; j += blockDim.x) {
           if (!any) {
@@ -776,7 +864,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
       for (int j = LADIES ? cp.L : warp; j < cp.L; j += warps) {   // FastGCN: a warp each
         int32_t pick = cp.V;
         float pr = 0.f;
-        if (U > 0 && total > 0.0) {
+        if (candidates && total > 0.0) {
           const double target = sh_target[j];
           int lo = sh_group[j];
           // (a target of zero takes the first candidate of all, whatever its weight)
@@ -835,7 +923,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
           a.prob[s * cp.fs + (int64_t)cp.step * cp.L + j] = pr;
         }
       }
-      if (tid == 0) { if (U > 0 && total > 0.0) draws += (unsigned long long)cp.L; }
+      if (tid == 0) { if (candidates && total > 0.0) draws += (unsigned long long)cp.L; }
       __syncthreads();
       uint32_t *adj = a.adj + (s * a.steps + cp.step) * (int64_t)adj_words(cp.stride);
       const int row_words = (cp.L + 31) / 32;
@@ -866,10 +954,18 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
     __syncthreads();
     s = sh_sample;
   }
-  if (tid == 0) {
-    atomicAdd(&a.acc[0], draws);
+  for (int o = 16; o > 0; o >>= 1) {
+    ids_sum += __shfl_xor_sync(0xffffffffu, ids_sum, o);
+    uniq_sum += __shfl_xor_sync(0xffffffffu, uniq_sum, o);
+  }
+  if (lane == 0) {
     atomicAdd(&a.acc[5], ids_sum);
     atomicAdd(&a.acc[6], uniq_sum);
+    __threadfence();
+  }
+  __syncthreads();
+  if (tid == 0) {
+    atomicAdd(&a.acc[0], draws);
     __threadfence();
     if (atomicAdd(&a.acc[10], 1ull) == (unsigned long long)gridDim.x - 1ull) {   // the last CTA
       __threadfence();
