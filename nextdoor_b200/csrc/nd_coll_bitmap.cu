@@ -7,7 +7,7 @@
 // integer weights sum exactly).
 //
 // What bounds it, and what is done about it (2^20 vertices, 1024 batches of 64, 2 layers of 64: FastGCN
-// 4.8 -> 0.665 ms, LADIES 5.7 -> 0.725 ms).  One CTA fills an SM, and neither memory nor issue slots are full: FastGCN issued
+// 4.8 -> 0.64 ms, LADIES 5.7 -> 0.69 ms).  One CTA fills an SM, and neither memory nor issue slots are full: FastGCN issued
 // in 58 % of the cycles at 0.89 ms (5.5 GB out of the L2 at 18 % of its rate), LADIES in 57 % at 1.07 (610 M
 // instructions for 131 M list entries, the distinct ones of 313 M), its shared memory busy in half of them; the warps
 // wait for barriers between the phases, for shared memory and for loads:
@@ -705,14 +705,19 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
       __syncthreads();
       const int nh = sh_hubs, nu = nh + sh_rest;
       // ---- the union: hubs' bitmaps, then the other lists
-      for (int w4 = tid; w4 < lay.words / 4; w4 += blockDim.x) {
-        uint4 u = make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll 8
+      // (32 bytes a load: with 16, eight of them in flight, FastGCN 0.661 ms and not 0.642, LADIES 0.725 and 0.71; lanes that know from
+      // flags that their 16 bytes are zero, as half of them are, and do not ask for them: 0.744)
+      for (int w8 = tid; w8 < lay.words / 8; w8 += blockDim.x) {
+        uint32_t u[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+#pragma unroll 4
         for (int i = 0; i < nh; i++) {
-          const uint4 h = __ldg(reinterpret_cast<const uint4 *>(a.hub_bits + (size_t)ut[i].slot * lay.words) + w4);
-          u.x |= h.x; u.y |= h.y; u.z |= h.z; u.w |= h.w;
+          int32_t h[8];
+          load8(reinterpret_cast<const int32_t *>(a.hub_bits + (size_t)ut[i].slot * lay.words) + 8 * w8, h);
+#pragma unroll
+          for (int k = 0; k < 8; k++) u[k] |= (uint32_t)h[k];
         }
-        reinterpret_cast<uint4 *>(bm)[w4] = u;
+        reinterpret_cast<uint4 *>(bm)[2 * w8] = make_uint4(u[0], u[1], u[2], u[3]);
+        reinterpret_cast<uint4 *>(bm)[2 * w8 + 1] = make_uint4(u[4], u[5], u[6], u[7]);
       }
       const int groups = lay.groups;
       uint32_t seen = 0, octs = 0;
@@ -738,11 +743,19 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
         }
       } else {
         // ---- the groups' weights and the rest of the union, then the number of candidates
-        for (int k = tid; k < groups; k += blockDim.x) {
-          double sum = 0.0;
-#pragma unroll 4
-          for (int i = 0; i < nh; i++) sum += __ldg(a.hub_sums + (size_t)ut[i].slot * groups + k) * (double)ut[i].mult;
-          gcdf[k] = sum;
+        constexpr int AT_ONCE = 4;   // groups a thread has in flight (one at a time: LADIES 0.71 ms, four 0.69)
+        for (int k = tid; k < groups; k += AT_ONCE * blockDim.x) {
+          double sum[AT_ONCE] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+          for (int i = 0; i < nh; i++) {
+            const double *from = a.hub_sums + (size_t)ut[i].slot * groups + k;
+            const double mult = (double)ut[i].mult;
+#pragma unroll
+            for (int q = 0; q < AT_ONCE; q++) sum[q] += (k + q * (int)blockDim.x < groups ? __ldg(from + q * blockDim.x) : 0.0) * mult;
+          }
+#pragma unroll
+          for (int q = 0; q < AT_ONCE; q++)
+            if (k + q * (int)blockDim.x < groups) gcdf[k + q * blockDim.x] = sum[q];
         }
         for (int i = tid; i < nu; i += blockDim.x) {
           const Transit &t = ut[i < nh ? i : cp.ntr - nu + i];
