@@ -581,8 +581,10 @@ __device__ __forceinline__ void sum_listed(const uint32_t *bm, const Degrees &d,
 }
 
 // The adjacency of a batch's lists, a row of bits each: bit j of row i, the layer's vertex j is in list i.  A list with a bitmap is
-// asked by a bit test, the others are bisected; a warp takes 32 vertices of a row, a few side by side, as every step of a search
-// waits for the one before.  (Three places a step instead of one take half of the steps and more time, 0.69 -> 0.71 ms; going
+// asked by a bit test, of the others the warp, which has 32 vertices of a row, first gets 32 entries, the last ones of as many parts
+// of the list, from which a lane finds its part without a read, and then bisects that: two or three reads that wait for one
+// another instead of up to thirteen (FastGCN 2^20 vertices 0.644 -> 0.636 ms, LADIES 0.689 -> 0.68); a few lists side by side.
+// (Three places a step instead of one take half of the steps and more time, 0.69 -> 0.71 ms; going
 // through short lists once more with a filter of the layer's vertices too, 0.74: a layer holds a hub many times, and
 // graphs repeat edges.)  `apart`: the places between the hubs in ut and the other lists.
 __device__ __forceinline__ void probe_rows(const int32_t *__restrict__ col, const uint32_t *__restrict__ hub_bits, int words, int32_t V, const Transit *ut,
@@ -592,20 +594,45 @@ __device__ __forceinline__ void probe_rows(const int32_t *__restrict__ col, cons
   for (int i0 = warp; i0 < n; i0 += SIDE * warps) {
     int32_t v[SIDE], l[SIDE], r[SIDE];   // searched for in [l, r)
     bool edge[SIDE];
-    uint32_t word[SIDE];
+    uint32_t got[SIDE];                  // a word of the bitmap, or the last entry of the lane's part of the list
 #pragma unroll
     for (int k = 0; k < SIDE; k++) {
       const int i = i0 + k * warps, row = i / row_words, j = (i - row * row_words) * 32 + lane;
       v[k] = i < n && j < L ? layer[j] : V;
-      l[k] = r[k] = 0; edge[k] = false; word[k] = 0u;
-      if (v[k] < 0 || v[k] >= V) continue;
+      l[k] = r[k] = 0; edge[k] = false; got[k] = 0u;
+      if (i >= n) continue;
       const Transit &t = ut[row < nh ? row : row + apart];
-      if (t.slot >= 0) word[k] = __ldg(hub_bits + (size_t)t.slot * words + ((uint32_t)v[k] >> 5));
-      else { l[k] = t.rs; r[k] = t.rs + t.deg; }
+      if (t.slot >= 0) {
+        if (v[k] >= 0 && v[k] < V) got[k] = __ldg(hub_bits + (size_t)t.slot * words + ((uint32_t)v[k] >> 5));
+      } else {
+        const int part = (t.deg + 31) / 32, last = (lane + 1) * part - 1;
+        got[k] = t.deg > 0 && lane * part < t.deg ? (uint32_t)__ldg(col + t.rs + min(last, t.deg - 1)) : 0x7fffffffu;
+        l[k] = t.rs; r[k] = t.rs + t.deg;
+      }
     }
+    bool more = false;
 #pragma unroll
-    for (int k = 0; k < SIDE; k++) edge[k] = (word[k] >> (v[k] & 31)) & 1u;
-    for (bool more = rows > nh; __any_sync(0xffffffffu, more);) {
+    for (int k = 0; k < SIDE; k++) {
+      const int i = i0 + k * warps, row = i / row_words;
+      if (i >= n) continue;                // (the warp is of one mind here: a list is the warp's)
+      const Transit &t = ut[row < nh ? row : row + apart];
+      if (t.slot >= 0) {
+        edge[k] = v[k] >= 0 && v[k] < V && ((got[k] >> (v[k] & 31)) & 1u);
+        continue;
+      }
+      int at = 0;                          // the first part whose last entry is not below the vertex
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1)
+        if ((int32_t)__shfl_sync(0xffffffffu, got[k], at + step - 1) < v[k]) at += step;
+      const int32_t last = (int32_t)__shfl_sync(0xffffffffu, got[k], at);
+      const int part = (t.deg + 31) / 32;
+      r[k] = min(r[k], l[k] + (at + 1) * part) - 1;   // (it has been compared with)
+      l[k] += at * part;
+      edge[k] = last == v[k] && v[k] >= 0 && v[k] < V;
+      if (last <= v[k] || v[k] < 0 || v[k] >= V) r[k] = l[k];
+      more |= l[k] < r[k];
+    }
+    while (__any_sync(0xffffffffu, more)) {
       more = false;
       int32_t m[SIDE], c[SIDE];
 #pragma unroll
