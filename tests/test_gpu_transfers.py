@@ -217,3 +217,21 @@ def test_loader_of_ids_before_weights(nd, n, V, weights, repeats):
         nd.Graph.from_edge_records(src, dst, w)
     dst[n // 2] = 3
     assert nd.Graph.from_edge_records(src, dst, w).E == n
+
+
+@pytest.mark.parametrize("nbytes", [(256 << 10) - 4, 256 << 10, (256 << 10) + 4])
+def test_results_of_the_smallest_size_that_is_kept(nd, small_graph, nbytes):
+    """New memory, lent again, pinned: every result is the job's, and one that a caller holds stays as it is."""
+    g = nd.Graph.from_csr(small_graph.row_ptr, small_graph.col, small_graph.w, small_graph.max_w)
+    jobs = [nd.Sampler(g, nd.app_params(0, steps=1, seed=seed), num_samples=nbytes // 4) for seed in (2, 3)]
+    exp = []
+    for s in jobs:
+        s.sample()
+        out = np.full(nbytes // 4, -9, np.int32)
+        s.final_samples(out)
+        exp.append(out.reshape(-1, 1))
+    held = jobs[0].final_samples()
+    for _ in range(4):
+        for s, e in zip(jobs, exp):
+            assert np.array_equal(s.final_samples(), e)
+    assert np.array_equal(held, exp[0]) and not np.array_equal(exp[0], exp[1])
