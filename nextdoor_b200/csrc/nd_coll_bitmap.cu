@@ -581,80 +581,102 @@ __device__ __forceinline__ void sum_listed(const uint32_t *bm, const Degrees &d,
 }
 
 // The adjacency of a batch's lists, a row of bits each: bit j of row i, the layer's vertex j is in list i.  A list with a bitmap is
-// asked by a bit test, of the others the warp, which has 32 vertices of a row, first gets 32 entries, the last ones of as many parts
-// of the list, from which a lane finds its part without a read, and then bisects that: two or three reads that wait for one
-// another instead of up to thirteen (FastGCN 2^20 vertices 0.644 -> 0.636 ms, LADIES 0.689 -> 0.68); a few lists side by side.
-// (Three places a step instead of one take half of the steps and more time, 0.69 -> 0.71 ms; going
-// through short lists once more with a filter of the layer's vertices too, 0.74: a layer holds a hub many times, and
-// graphs repeat edges.)  `apart`: the places between the hubs in ut and the other lists.
-__device__ __forceinline__ void probe_rows(const int32_t *__restrict__ col, const uint32_t *__restrict__ hub_bits, int words, int32_t V, const Transit *ut,
-                                           int apart, int nh, int rows, const int32_t *layer, int L, uint32_t *out) {
-  constexpr int SIDE = 4;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, row_words = (L + 31) / 32, n = rows * row_words;
-  for (int i0 = warp; i0 < n; i0 += SIDE * warps) {
-    int32_t v[SIDE], l[SIDE], r[SIDE];   // searched for in [l, r)
-    bool edge[SIDE];
-    uint32_t got[SIDE];                  // a word of the bitmap, or the last entry of the lane's part of the list
+// asked by a bit test.  Of the others the warp, which has a row or a few side by side, first gets 32 entries, the last ones of as
+// many parts of the list, from which a lane finds the part of its vertex without a read, and then bisects that: two or three
+// reads that wait for one another instead of up to thirteen (FastGCN 2^20 vertices 0.644 -> 0.636 ms, LADIES 0.689 -> 0.68).
+// WORDS: the words of a row that are side by side, which share the list and its 32 entries (a word of any row each, with a division
+// to find it, before: layers of 100 on 100 K, 700 batches, FastGCN 360 -> 323 us, LADIES 592 -> 549; of 64 on 70 K, 1024:
+// 190 -> 180).  (Three places a step instead of one take half of the steps and more time; going through short lists once more with a
+// filter of the layer's vertices too: a layer holds a hub many times, and graphs repeat edges.)  `apart`: the places between the
+// hubs in ut and the other lists.
+template <int ROWS, int WORDS>
+__device__ __forceinline__ void probe_rows_as(const int32_t *__restrict__ col, const uint32_t *__restrict__ hub_bits, int words, int32_t V, const Transit *ut,
+                                              int apart, int nh, int rows, const int32_t *layer, int L, uint32_t *out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, row_words = (L + 31) / 32;
+  for (int row0 = warp; row0 < rows; row0 += ROWS * warps) {
+    int32_t rs[ROWS], deg[ROWS], slot[ROWS], last[ROWS];   // last: the last entry of the lane's part of the list
 #pragma unroll
-    for (int k = 0; k < SIDE; k++) {
-      const int i = i0 + k * warps, row = i / row_words, j = (i - row * row_words) * 32 + lane;
-      v[k] = i < n && j < L ? layer[j] : V;
-      l[k] = r[k] = 0; edge[k] = false; got[k] = 0u;
-      if (i >= n) continue;
-      const Transit &t = ut[row < nh ? row : row + apart];
-      if (t.slot >= 0) {
-        if (v[k] >= 0 && v[k] < V) got[k] = __ldg(hub_bits + (size_t)t.slot * words + ((uint32_t)v[k] >> 5));
-      } else {
-        const int part = (t.deg + 31) / 32, last = (lane + 1) * part - 1;
-        got[k] = t.deg > 0 && lane * part < t.deg ? (uint32_t)__ldg(col + t.rs + min(last, t.deg - 1)) : 0x7fffffffu;
-        l[k] = t.rs; r[k] = t.rs + t.deg;
-      }
-    }
-    bool more = false;
-#pragma unroll
-    for (int k = 0; k < SIDE; k++) {
-      const int i = i0 + k * warps, row = i / row_words;
-      if (i >= n) continue;                // (the warp is of one mind here: a list is the warp's)
-      const Transit &t = ut[row < nh ? row : row + apart];
-      if (t.slot >= 0) {
-        edge[k] = v[k] >= 0 && v[k] < V && ((got[k] >> (v[k] & 31)) & 1u);
-        continue;
-      }
-      int at = 0;                          // the first part whose last entry is not below the vertex
-#pragma unroll
-      for (int step = 16; step > 0; step >>= 1)
-        if ((int32_t)__shfl_sync(0xffffffffu, got[k], at + step - 1) < v[k]) at += step;
-      const int32_t last = (int32_t)__shfl_sync(0xffffffffu, got[k], at);
+    for (int q = 0; q < ROWS; q++) {
+      const int row = row0 + q * warps;
+      const Transit t = ut[row < rows ? row < nh ? row : row + apart : row0 < nh ? row0 : row0 + apart];
+      rs[q] = t.rs; deg[q] = t.deg; slot[q] = t.slot;
       const int part = (t.deg + 31) / 32;
-      r[k] = min(r[k], l[k] + (at + 1) * part) - 1;   // (it has been compared with)
-      l[k] += at * part;
-      edge[k] = last == v[k] && v[k] >= 0 && v[k] < V;
-      if (last <= v[k] || v[k] < 0 || v[k] >= V) r[k] = l[k];
-      more |= l[k] < r[k];
+      last[q] = 0x7fffffff;
+      if (t.slot < 0 && lane * part < t.deg) last[q] = __ldg(col + t.rs + min((lane + 1) * part, t.deg) - 1);
     }
-    while (__any_sync(0xffffffffu, more)) {
-      more = false;
-      int32_t m[SIDE], c[SIDE];
+    for (int j0 = 0; j0 < L; j0 += 32 * WORDS) {
+      int32_t v[WORDS], l[ROWS][WORDS], r[ROWS][WORDS];   // searched for in [l, r)
+      uint32_t word[ROWS][WORDS];
+      bool edge[ROWS][WORDS], more = false;
 #pragma unroll
-      for (int k = 0; k < SIDE; k++) {
-        m[k] = l[k] + (r[k] - l[k]) / 2;
-        c[k] = l[k] < r[k] ? __ldg(col + m[k]) : 0;
+      for (int w = 0; w < WORDS; w++) {
+        const int j = j0 + 32 * w + lane;
+        v[w] = j < L ? layer[j] : V;
+        if (v[w] < 0 || v[w] >= V) v[w] = -1;   // in no list
       }
 #pragma unroll
-      for (int k = 0; k < SIDE; k++) {
-        if (l[k] >= r[k]) continue;
-        if (c[k] == v[k]) { edge[k] = true; l[k] = r[k]; }
-        else if (c[k] < v[k]) l[k] = m[k] + 1;
-        else r[k] = m[k];
-        more |= l[k] < r[k];
-      }
-    }
+      for (int q = 0; q < ROWS; q++)
 #pragma unroll
-    for (int k = 0; k < SIDE; k++) {
-      const uint32_t answers = __ballot_sync(0xffffffffu, edge[k]);
-      if (lane == 0 && i0 + k * warps < n) out[i0 + k * warps] = answers;
+        for (int w = 0; w < WORDS; w++) word[q][w] = slot[q] >= 0 && v[w] >= 0 ? __ldg(hub_bits + (size_t)slot[q] * words + ((uint32_t)v[w] >> 5)) : 0u;
+#pragma unroll
+      for (int q = 0; q < ROWS; q++) {
+        const int part = (deg[q] + 31) / 32;
+#pragma unroll
+        for (int w = 0; w < WORDS; w++) {
+          l[q][w] = r[q][w] = 0;
+          if (slot[q] >= 0) {   // (the warp is of one mind: a list is the warp's)
+            edge[q][w] = v[w] >= 0 && ((word[q][w] >> (v[w] & 31)) & 1u);
+            continue;
+          }
+          int at = 0;           // the first part whose last entry is not below the vertex
+#pragma unroll
+          for (int step = 16; step > 0; step >>= 1)
+            if (__shfl_sync(0xffffffffu, last[q], at + step - 1) < v[w]) at += step;
+          const int32_t its = __shfl_sync(0xffffffffu, last[q], at);
+          edge[q][w] = its == v[w];
+          if (its > v[w] && v[w] >= 0) {
+            l[q][w] = rs[q] + at * part;
+            r[q][w] = min(rs[q] + deg[q], l[q][w] + part) - 1;   // (the last one has been compared with)
+            more |= l[q][w] < r[q][w];
+          }
+        }
+      }
+      while (__any_sync(0xffffffffu, more)) {
+        more = false;
+        int32_t m[ROWS][WORDS], c[ROWS][WORDS];
+#pragma unroll
+        for (int q = 0; q < ROWS; q++)
+#pragma unroll
+          for (int w = 0; w < WORDS; w++) {
+            m[q][w] = l[q][w] + (r[q][w] - l[q][w]) / 2;
+            c[q][w] = l[q][w] < r[q][w] ? __ldg(col + m[q][w]) : 0;
+          }
+#pragma unroll
+        for (int q = 0; q < ROWS; q++)
+#pragma unroll
+          for (int w = 0; w < WORDS; w++) {
+            if (l[q][w] >= r[q][w]) continue;
+            if (c[q][w] == v[w]) { edge[q][w] = true; l[q][w] = r[q][w]; }
+            else if (c[q][w] < v[w]) l[q][w] = m[q][w] + 1;
+            else r[q][w] = m[q][w];
+            more |= l[q][w] < r[q][w];
+          }
+      }
+#pragma unroll
+      for (int q = 0; q < ROWS; q++)
+#pragma unroll
+        for (int w = 0; w < WORDS; w++) {
+          const uint32_t answers = __ballot_sync(0xffffffffu, edge[q][w]);
+          if (lane == 0 && row0 + q * warps < rows && j0 + 32 * w < L) out[(row0 + q * warps) * row_words + j0 / 32 + w] = answers;
+        }
     }
   }
+}
+__device__ __forceinline__ void probe_rows(const int32_t *__restrict__ col, const uint32_t *__restrict__ hub_bits, int words, int32_t V, const Transit *ut,
+                                           int apart, int nh, int rows, const int32_t *layer, int L, uint32_t *out) {
+  if (L <= 32) probe_rows_as<4, 1>(col, hub_bits, words, V, ut, apart, nh, rows, layer, L, out);
+  else if (L <= 64) probe_rows_as<2, 2>(col, hub_bits, words, V, ut, apart, nh, rows, layer, L, out);
+  else probe_rows_as<1, 4>(col, hub_bits, words, V, ut, apart, nh, rows, layer, L, out);
 }
 
 // SUMS_FAR: LADIES' group sums are in the big part.

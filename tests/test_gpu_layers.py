@@ -313,3 +313,28 @@ def test_layers_by_number_of_samples(nd, app, V, B, L):
         for got, exp in zip(job(first, S)[:3], one):
             assert np.array_equal(got, exp[first:first + S])
         assert np.allclose(job(first, S)[3], one[3][first:first + S], rtol=1e-6, atol=0)   # 32-bit results of 64-bit sums in another order
+
+
+@pytest.mark.parametrize("app,B,L", [(8, 40, 1), (8, 40, 32), (9, 70, 33), (9, 70, 64), (8, 70, 65), (9, 40, 100), (8, 40, 129), (9, 70, 300)])
+def test_adjacency_by_length_of_the_lists(nd, ndo, app, B, L):
+    """Lists around the 32 parts in which they are looked through, none, short, with repeated edges; hubs (V / 128 neighbours)."""
+    V = 40_000
+    rng = np.random.default_rng(L)
+    deg = rng.choice([0, 1, 2, 3, 31, 32, 33, 63, 64, 65, 95, 97, 255, 311, 312, 313, 900], V, p=[.3, .1, .1, .1, .05, .05, .05] + [.025] * 9 + [.025])
+    src = np.repeat(np.arange(V), deg).astype(np.int32)
+    dst = np.where(rng.random(len(src)) < 0.5, rng.integers(0, 60, len(src)) * 661, rng.integers(0, V, len(src))).astype(np.int32)   # (the 60 are drawn again and again)
+    hg = ndo.csr_from_records(src, dst, np.ones(len(src), np.float32), V=V)
+    g = nd.Graph.from_csr(hg.row_ptr, hg.col, hg.w, hg.max_w)
+    S, steps = 30, 2
+    init = rng.integers(0, V, S * B).astype(np.int32)
+    s = nd.Sampler(g, nd.app_params(app, steps=steps, fanout=L, batch=B, seed=3), num_samples=S, initial=init)
+    s.sample()
+    out, aux = s.final_samples().reshape(S, steps, L), s.aux()
+    rows, found = aux["adj_row"].reshape(S, steps, -1), 0
+    for k in range(S):
+        for step in range(steps):
+            transits = init.reshape(S, B)[k] if step == 0 else out[k, 0]
+            exp = np.concatenate([np.isin(out[k, step], hg.col[hg.row_ptr[t]:hg.row_ptr[t + 1]]) for t in transits])
+            assert np.array_equal(rows[k, step, :len(exp)] >= 0, exp) and (rows[k, step, len(exp):] == -1).all()
+            found += exp.sum()
+    assert found > S * L
