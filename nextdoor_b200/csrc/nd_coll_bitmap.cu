@@ -7,10 +7,9 @@
 // integer weights sum exactly).
 //
 // What bounds it, and what is done about it (2^20 vertices, 1024 batches of 64, 2 layers of 64: FastGCN
-// 4.8 -> 0.64 ms, LADIES 5.7 -> 0.69 ms).  One CTA fills an SM, and neither memory nor issue slots are full: FastGCN issued
-// in 58 % of the cycles at 0.89 ms (5.5 GB out of the L2 at 18 % of its rate), LADIES in 57 % at 1.07 (610 M
-// instructions for 131 M list entries, the distinct ones of 313 M), its shared memory busy in half of them; the warps
-// wait for barriers between the phases, for shared memory and for loads:
+// 4.8 -> 0.64 ms, LADIES 5.7 -> 0.69 ms).  One CTA fills an SM there, and neither memory nor issue slots are full:
+// FastGCN issues in 48 % of the cycles (322 M instructions, 5.0 GB out of the L2), LADIES in 43 % (304 M instructions for 131 M
+// list entries, the distinct ones of 313 M); the warps wait for barriers between the phases, for loads and for shared memory:
 //  * The second layer's transits are hubs (FastGCN draws them with the square of their degree), many of them the
 //    same one: repeated transits of a batch are taken once (LADIES with their multiplicity).
 //  * A hub's list (up to 140 K ids; FastGCN's second layer has 28 distinct hubs a sample) costs a shared-memory test per id.  Vertices with at least V/128 neighbours

@@ -8,9 +8,10 @@
 // (src/apps/khop/khop.cu:10-23); ND_APP_KHOP_DISTINCT without replacement, every hop sorted and made unique at
 // the end (src/distinct.cuh:1-111).  A warp writes its row at the end.
 // What bounds it: with replacement, gathers of 4 bytes from the adjacency array at the rate of random DRAM
-// reads (262,144 seeds, 25 x 10, 2^21 vertices: 0.89 ms transit-parallel -> 0.36); without (1.15 -> 0.49 ms), the
-// instructions: 341 M of a warp, 0.29 ms at one per cycle and scheduler, and of the 18 cycles from one to the next 5.5 are
-// spent waiting for the next instruction to be fetched, 2.6 for memory and 2.5 for shared memory (DRAM 34 %); a mini-batch
+// reads (262,144 seeds, 25 x 10, 2^21 vertices: 0.89 ms transit-parallel -> 0.36); without (1.15 -> 0.475 ms), the
+// instructions: 341 M of a warp, 0.29 ms at one per cycle and scheduler, and of the 18 cycles from one to the next 4.8 are
+// spent waiting for the next instruction to be fetched, 2.5 for memory and 2.4 for shared memory (DRAM 35 %); without its sorts
+// 0.375 ms, without the resolution of picks taken twice 0.43, without the gathers 0.46, with a cheap hash for the draws 0.46; a mini-batch
 // of 1024, the chain seed -> row -> neighbours -> rows -> neighbours (74 -> 12 us with the seeds' copy).
 #include "nd_common.cuh"
 #include "nd_khop_rows.cuh"

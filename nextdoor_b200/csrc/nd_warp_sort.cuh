@@ -4,8 +4,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-// The smaller of both where `lower`, else the larger.  The networks are bound by these: two predicated instructions, where the
-// compiler's choice between two results is three (262,144 samples, 25 x 10: 488 -> 478 us; no gain in networks of 64 and 32 ids).
+// The smaller of both where `lower`, else the larger.  Written as two predicated instructions in networks of 128 ids and more: no
+// fewer instructions than the choice between two results (341 M for 262,144 samples, 25 x 10), but 4.8 instead of 5.4 of the 18
+// cycles between two of a warp's are spent on fetching the next one, 488 -> 475 us; no gain in networks of 64 and 32 ids.
 template <int E>
 __device__ __forceinline__ int32_t smaller_if(bool lower, int32_t a, int32_t b) {
   if (E < 4) return lower ? min(a, b) : max(a, b);
