@@ -7,7 +7,7 @@
 // integer weights sum exactly).
 //
 // What bounds it, and what is done about it (2^20 vertices, 1024 batches of 64, 2 layers of 64: FastGCN
-// 4.8 -> 0.64 ms, LADIES 5.7 -> 0.69 ms).  One CTA fills an SM there, and neither memory nor issue slots are full:
+// 4.8 -> 0.62 ms, LADIES 5.7 -> 0.68 ms).  One CTA fills an SM there, and neither memory nor issue slots are full:
 // FastGCN issues in 48 % of the cycles (322 M instructions, 5.0 GB out of the L2), LADIES in 43 % (304 M instructions for 131 M
 // list entries, the distinct ones of 313 M); the warps wait for barriers between the phases, for loads and for shared memory:
 //  * The second layer's transits are hubs (FastGCN draws them with the square of their degree), many of them the
@@ -86,10 +86,12 @@ struct Layout {
 
 // The degrees in vertex order, FastGCN.  Codes: the low bytes of sixteen vertices' each, then the high ones; a listed
 // vertex's is zero.
+__host__ __device__ inline int64_t listed_room(int64_t n) { return (n + 7) / 8 * 8 + 8; }
 struct Degrees {
   const uint4 *__restrict__ codes;
   const uint32_t *__restrict__ wide;        // a bit per group: it has high bytes that are not zero; null: none has
-  const int2 *__restrict__ listed;          // [n_listed] (vertex, degree) in order, read in whole runs
+  const int32_t *__restrict__ listed;       // [listed_room(n_listed)] vertices in order, read in whole runs, beyond n_listed 0 without a weight
+  const uint2 *__restrict__ weights;        // ... their weights as the words of a Sum
   int n_listed;
 };
 
@@ -552,18 +554,18 @@ __device__ __forceinline__ uint32_t sum_groups(const uint32_t *bm, const Degrees
   return seen;
 }
 
-// ... and over the listed vertices; neighbours on the list mostly share a group
+// ... and over the listed vertices; neighbours on the list mostly share a group.  Their weights come as the two words that are added
+// (from degrees, with a case for each size and 64-bit conversions for the large: 1024 batches on 2^20 vertices 0.631 ms, so 0.622;
+// 100 of 100 on 600 K 84.4 and 82.6 us).
 __device__ __forceinline__ void sum_listed(const uint32_t *bm, const Degrees &d, uint2 *sums) {
   for (int i0 = threadIdx.x * RUN; i0 < d.n_listed; i0 += blockDim.x * RUN) {
-    int32_t v[RUN], deg[RUN];
+    const int4 four = __ldg(reinterpret_cast<const int4 *>(d.listed + i0));
+    const int32_t v[RUN] = {four.x, four.y, four.z, four.w};
+    int32_t weight[2 * RUN];
+    load8(reinterpret_cast<const int32_t *>(d.weights + i0), weight);
     uint32_t word[RUN];
 #pragma unroll
-    for (int k = 0; k < RUN; k += 2) {
-      const int4 two = __ldg(reinterpret_cast<const int4 *>(d.listed + i0 + k));
-      v[k] = two.x; deg[k] = two.y; v[k + 1] = two.z; deg[k + 1] = two.w;
-    }
-#pragma unroll
-    for (int k = 0; k < RUN; k++) word[k] = i0 + k < d.n_listed ? bm[v[k] >> 5] : 0u;
+    for (int k = 0; k < RUN; k++) word[k] = bm[v[k] >> 5];
     int at = v[0] / GROUP;
     Sum sum;
 #pragma unroll
@@ -573,7 +575,9 @@ __device__ __forceinline__ void sum_listed(const uint32_t *bm, const Degrees &d,
         at = v[k] / GROUP;
         sum = Sum();
       }
-      if ((word[k] >> (v[k] & 31)) & 1u) sum.add(deg[k]);
+      const bool in = (word[k] >> (v[k] & 31)) & 1u;
+      sum.low += in ? (uint32_t)weight[2 * k] : 0u;
+      sum.high += in ? (uint32_t)weight[2 * k + 1] : 0u;
     }
     sum.to(sums, at);
   }
@@ -1078,7 +1082,7 @@ deg_build_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int64_t units, 
 }
 
 __global__ void __launch_bounds__(256)
-deg_list_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int64_t units, int32_t least, const int32_t *__restrict__ listed_at, int2 *__restrict__ listed,
+deg_list_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int64_t units, int32_t least, const int32_t *__restrict__ listed_at, int32_t *__restrict__ listed, uint2 *__restrict__ weights,
                 NdBigVertex *__restrict__ huge, int32_t *__restrict__ n_huge) {
   const int lane = threadIdx.x & 31;
   for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < units; u += (int64_t)gridDim.x * blockDim.x) {
@@ -1099,7 +1103,12 @@ deg_list_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int64_t units, i
 #pragma unroll
     for (int k = 0; k < 16; k++) {
       if (d[k] < least) continue;
-      if (d[k] < HUGE_DEGREE) listed[at++] = make_int2((int32_t)(16 * u + k), d[k]);
+      if (d[k] < HUGE_DEGREE) {
+        Sum sum;
+        sum.add(d[k]);
+        weights[at] = make_uint2(sum.low, sum.high);
+        listed[at++] = (int32_t)(16 * u + k);
+      }
       else huge[atomicAdd(n_huge, 1)] = NdBigVertex{(int32_t)(16 * u + k), square(d[k])};
     }
   }
@@ -1285,7 +1294,7 @@ int ensure_degrees(const nd_graph *g, int grid) {
   const size_t groups = (size_t)units / (GROUP / 16), flags = (groups + 31) / 32 + 1;
   NdDevMem<uint4> deg;
   NdDevMem<int32_t> at;
-  NdDevMem<int2> listed;
+  NdDevMem<uint2> listed;     // weights, then vertices
   NdDevMem<NdBigVertex> huge;
   int32_t n[3] = {0, 0, 0};   // vertices with at least 256, BIG_DEGREE, HUGE_DEGREE neighbours
   ND_TRY(deg.alloc((size_t)(2 * units) + (flags + 3) / 4));
@@ -1297,9 +1306,9 @@ int ensure_degrees(const nd_graph *g, int grid) {
   ND_CUDA(cudaMemcpy(n, count, sizeof(n), cudaMemcpyDeviceToHost));
   const bool few = (int64_t)n[0] * LISTED <= g->V;
   const int32_t least = few ? 256 : BIG_DEGREE;
-  const size_t n_listed = (size_t)(n[few ? 0 : 1] - n[2]), room = n_listed + RUN;
-  ND_TRY(listed.alloc(room));
-  ND_CUDA(cudaMemset(listed.p, 0, sizeof(int2) * room));
+  const size_t n_listed = (size_t)(n[few ? 0 : 1] - n[2]), room = (size_t)listed_room((int64_t)n_listed);
+  ND_TRY(listed.alloc(room + room / 2));
+  ND_CUDA(cudaMemset(listed.p, 0, sizeof(uint2) * (room + room / 2)));
   ND_TRY(huge.alloc((size_t)n[2] + 1));
   deg_build_kernel<<<grid, 256>>>(g->row_ptr, g->V, units, least, deg.p, reinterpret_cast<uint32_t *>(deg.p + 2 * units), at.p);
   std::vector<int32_t> starts(groups + 1);
@@ -1311,7 +1320,7 @@ int ensure_degrees(const nd_graph *g, int grid) {
     all += own;
   }
   ND_CUDA(cudaMemcpy(at.p, starts.data(), sizeof(int32_t) * (groups + 1), cudaMemcpyHostToDevice));
-  deg_list_kernel<<<grid, 256>>>(g->row_ptr, g->V, units, least, at.p, listed.p, huge.p, count + 3);
+  deg_list_kernel<<<grid, 256>>>(g->row_ptr, g->V, units, least, at.p, reinterpret_cast<int32_t *>(listed.p + room), listed.p, huge.p, count + 3);
   ND_CUDA(cudaDeviceSynchronize());
   g->n_huge = n[2];
   g->deg_wide = !few;
@@ -1518,7 +1527,8 @@ int nd_coll_bitmap_launch(nd_sampler *s, const CollParams &cp, unsigned long lon
   const Plan p = plan_of(s);
   const nd_graph *g = s->g;
   const Args a{nd_view(g), cp, s->p.steps, s->S, p.lay, s->d_bm, s->d_initial, s->d_out, s->d_adj, s->d_prob,
-               Degrees{g->deg_codes, g->deg_wide ? reinterpret_cast<const uint32_t *>(g->deg_codes + 4 * (int64_t)p.lay.words) : nullptr, g->listed, g->n_listed},
+               Degrees{g->deg_codes, g->deg_wide ? reinterpret_cast<const uint32_t *>(g->deg_codes + 4 * (int64_t)p.lay.words) : nullptr,
+                       reinterpret_cast<const int32_t *>(g->listed + listed_room(g->n_listed)), g->listed, g->n_listed},
                g->huge, g->n_huge, g->term, g->hub_slot, g->hub_bits, s->hub_table.sums, s->hub_table.starts, g->hub_ids, g->hub_terms, s->d_rows_acc, s->d_stats, pairs};
   if (ladies && p.lay.sums_far) coll_bitmap_kernel<true, true><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);
   else if (ladies) coll_bitmap_kernel<true, false><<<s->coll_grid, p.threads, p.lay.bytes, s->stream>>>(a);

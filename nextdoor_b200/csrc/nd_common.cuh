@@ -131,7 +131,7 @@ struct nd_graph {
   mutable int32_t *adjset = nullptr;   // node2vec membership: per-vertex hash sets of the neighbour ids, 8-slot buckets
   mutable uint32_t *adjsign = nullptr; // ... and the filter in front of them
   mutable uint4 *deg_codes = nullptr;  // degrees of sixteen vertices each, low bytes, high bytes, flags (FastGCN)
-  mutable int2 *listed = nullptr;          // [n_listed] vertices whose degrees the codes do not hold, and those, except
+  mutable uint2 *listed = nullptr;         // [n_listed] weights and vertices whose degrees the codes do not hold, and those, except
   mutable NdBigVertex *huge = nullptr;     // ... [n_huge], whose weights the groups' sums do not hold
   mutable int n_listed = 0, n_huge = 0;
   mutable bool deg_wide = false;           // the codes have high bytes
