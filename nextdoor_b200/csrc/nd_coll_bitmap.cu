@@ -7,7 +7,7 @@
 // integer weights sum exactly).
 //
 // What bounds it, and what is done about it (2^20 vertices, 1024 batches of 64, 2 layers of 64: FastGCN
-// 4.8 -> 0.62 ms, LADIES 5.7 -> 0.68 ms).  One CTA fills an SM there, and neither memory nor issue slots are full:
+// 4.8 -> 0.59 ms, LADIES 5.7 -> 0.68 ms).  One CTA fills an SM there, and neither memory nor issue slots are full:
 // FastGCN issues in 48 % of the cycles (322 M instructions, 5.0 GB out of the L2), LADIES in 43 % (304 M instructions for 131 M
 // list entries, the distinct ones of 313 M); the warps wait for barriers between the phases, for loads and for shared memory:
 //  * The second layer's transits are hubs (FastGCN draws them with the square of their degree), many of them the
@@ -16,9 +16,9 @@
 //    have their neighbourhood as a bitmap, built once per graph: V/8 bytes that are ORed in registers, word by
 //    word, and stored to the union once; and an adjacency probe of such a transit is a bit test.
 //  * FastGCN's weights are summed without a list of candidates (writing that and fetching deg^2 one by one took more
-//    than half of the time).  The degrees lie in vertex order, a byte each: a lane takes sixteen vertices with one load, masks
-//    them with its half word of the bitmap and squares and sums them with dp4a.  That is bound by the products (four cycles
-//    each): the two bytes that hold degrees up to 2047 take three times as many, so that from 256 on, where few vertices have
+//    than half of the time).  The degrees lie in the order of the bitmap, a byte each: a lane takes the 32 vertices of a word with one load,
+//    masks them with it and squares and sums them with dp4a (byte b of code word j is vertex j + 8 b: a mask is a shift and a
+//    byte permutation; sixteen vertices a lane in their own order, with a multiplication a mask, 0.622 ms, now 0.588).  The two bytes that hold degrees up to 2047 take three times as many, so that from 256 on, where few vertices have
 //    as many, they are a list (20 K of 2^20, 65 against 160 thousand cycles an SM); where they are not few the codes have a
 //    second byte, for the groups that need it.  Groups without a candidate are passed over, and the lists beside the hubs',
 //    where they are short (a first layer's: 2 K entries), are weighed entry by entry as they come into the union, an eight of
@@ -61,7 +61,7 @@ constexpr int LADIES_GROUP_BITS = 7;   // LADIES: 2^7 vertices, more where the s
 constexpr int RUN = 4;            // listed vertices a thread takes at a time
 constexpr int BIG_DEGREE = 2048;  // from here a vertex is listed and its code is 0: 512 * 2047^2 < 2^31
 constexpr int LISTED = 32;        // degrees are codes of a byte where fewer than V / LISTED vertices do not fit one
-constexpr int FLIGHT = 6;         // groups a warp sums at a time (2^20 vertices 4: 0.71, 6: 0.70, 8: 0.72 ms; 2^21 0.48, 0.45, 0.45)
+constexpr int FLIGHT = 4;         // pairs of groups a warp sums at a time (2^20 vertices 2: 0.595, 3: 0.589, 4: 0.588 ms; 600 K, 100 batches 77.7, 76.7, 76.3 us)
 constexpr int HUB = 128;          // a vertex with at least V / HUB neighbours has a bitmap of them
 constexpr int32_t SHARED_V = 1 << 18;   // see plan_of()
 constexpr int FEW = 64;           // lists with fewer than V / FEW entries in all are weighed entry by entry
@@ -84,9 +84,11 @@ struct Layout {
   uint32_t glob_bytes;                                 // per-CTA slice of the global scratch, 0 = big part in shared memory
 };
 
-// The degrees in vertex order, FastGCN.  Codes: the low bytes of sixteen vertices' each, then the high ones; a listed
-// vertex's is zero.
+// vertices there is room for on a list of n
 __host__ __device__ inline int64_t listed_room(int64_t n) { return (n + 7) / 8 * 8 + 8; }
+
+// The degrees, FastGCN.  Codes: the low bytes of 32 vertices' each in two (squares() says in which order), then the high ones; a
+// listed vertex's is zero.
 struct Degrees {
   const uint4 *__restrict__ codes;
   const uint32_t *__restrict__ wide;        // a bit per group: it has high bytes that are not zero; null: none has
@@ -499,56 +501,61 @@ __device__ __forceinline__ void pick_in_group(const double *acc, int n, double b
   }
 }
 
-// bits 0..3 (no others) -> 0xff in bytes 0..3
-__device__ __forceinline__ uint32_t byte_mask(uint32_t bits) {
-  uint32_t m;
-  asm("prmt.b32 %0, %1, 0, 0xba98;" : "=r"(m) : "r"(bits * 0x10204080u));   // each to the top of its byte, which is filled with it
-  return m;
-}
-
-// The sum of deg^2 over the vertices of `bits` (sixteen, low and high bytes of their degrees as in Args::deg), in products of
-// low, low and high, and high bytes.
+// The sum of deg^2 over the vertices of a bitmap's word (32, low and high bytes of their degrees as in Degrees::codes), in products
+// of low, low and high, and high bytes.  Byte b of code word j is vertex j + 8 b, so that a shift brings its bit to the top of the
+// byte, which is then filled with it.
 template <bool WIDE>
-__device__ __forceinline__ uint32_t squares(uint32_t bits, const uint4 &low, const uint4 &high) {
-  const uint32_t m0 = byte_mask(bits & 15u), m1 = byte_mask((bits >> 4) & 15u), m2 = byte_mask((bits >> 8) & 15u), m3 = byte_mask(bits >> 12);
-  const uint32_t l0 = low.x & m0, l1 = low.y & m1, l2 = low.z & m2, l3 = low.w & m3;
-  const uint32_t ll = __dp4a(l3, l3, __dp4a(l2, l2, __dp4a(l1, l1, __dp4a(l0, l0, 0u))));
-  if (!WIDE) return ll;
-  const uint32_t lh = __dp4a(l3, high.w, __dp4a(l2, high.z, __dp4a(l1, high.y, __dp4a(l0, high.x, 0u))));
-  const uint32_t hh = __dp4a(high.w & m3, high.w, __dp4a(high.z & m2, high.z, __dp4a(high.y & m1, high.y, __dp4a(high.x & m0, high.x, 0u))));
-  return ll + (lh << 9) + (hh << 16);
+__device__ __forceinline__ uint32_t squares(uint32_t bits, const int32_t (&low)[8], const int32_t (&high)[8]) {
+  uint32_t ll = 0, lh = 0, hh = 0;
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    uint32_t m;
+    asm("prmt.b32 %0, %1, 0, 0xba98;" : "=r"(m) : "r"(bits << (7 - j)));
+    const uint32_t l = (uint32_t)low[j] & m;
+    ll = __dp4a(l, l, ll);
+    if (WIDE) {
+      lh = __dp4a(l, (uint32_t)high[j], lh);
+      hh = __dp4a((uint32_t)high[j] & m, (uint32_t)high[j], hh);
+    }
+  }
+  return WIDE ? ll + (lh << 9) + (hh << 16) : ll;
 }
 
-// FastGCN: the groups' weights, without HUGE_DEGREE ones; the candidates the thread has seen.  A warp takes FLIGHT groups at a
-// time: a lane sixteen vertices' codes, then the group's listed vertices side by side.  WIDE: the codes have high bytes.
+// FastGCN: the groups' weights, without HUGE_DEGREE ones; the candidates the thread has seen.  A warp takes FLIGHT times two
+// groups at a time, a lane a word of the bitmap and its 32 bytes of codes.  WIDE: the codes have high bytes.
 template <bool WIDE>
 __device__ __forceinline__ uint32_t sum_groups(const uint32_t *bm, const Degrees &d, int words, int groups, uint2 *sums) {
+  constexpr int AT_ONCE = WIDE ? FLIGHT / 2 : FLIGHT;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  const uint16_t *half = reinterpret_cast<const uint16_t *>(bm);
-  const uint4 *__restrict__ high_bytes = d.codes + (int64_t)words * 2;
+  const int32_t *__restrict__ low_bytes = reinterpret_cast<const int32_t *>(d.codes), *__restrict__ high_bytes = low_bytes + (int64_t)words * 8;
   uint32_t seen = 0;
-  for (int g0 = warp * FLIGHT; g0 < groups; g0 += warps * FLIGHT) {
-    uint32_t bits[FLIGHT], some = 0u;
-    bool wide[FLIGHT];
-    uint4 lo[FLIGHT], hi[FLIGHT];
+  for (int w0 = warp * AT_ONCE * 32; w0 < words; w0 += warps * AT_ONCE * 32) {
+    uint32_t bits[AT_ONCE], some = 0u;
+    bool wide[AT_ONCE];
+    int32_t lo[AT_ONCE][8], hi[AT_ONCE][8];
 #pragma unroll
-    for (int k = 0; k < FLIGHT; k++) {
-      bits[k] = g0 + k < groups ? half[(g0 + k) * 32 + lane] : 0u;
-      wide[k] = WIDE && g0 + k < groups && ((__ldg(d.wide + (g0 + k) / 32) >> ((g0 + k) & 31)) & 1u);
+    for (int k = 0; k < AT_ONCE; k++) {
+      const int w = w0 + 32 * k + lane, g = w / GROUP_WORDS;
+      bits[k] = w < words ? bm[w] : 0u;
+      wide[k] = WIDE && w < words && ((__ldg(d.wide + g / 32) >> (g & 31)) & 1u);
       some |= bits[k];
     }
     if (!__any_sync(0xffffffffu, some)) continue;   // (a first layer's thousand candidates leave most groups empty)
 #pragma unroll
-    for (int k = 0; k < FLIGHT; k++) {
-      const int unit = (g0 + k) * 32 + lane;
-      lo[k] = bits[k] ? __ldg(d.codes + unit) : make_uint4(0u, 0u, 0u, 0u);
-      if (WIDE) hi[k] = wide[k] && bits[k] ? __ldg(high_bytes + unit) : make_uint4(0u, 0u, 0u, 0u);
+    for (int k = 0; k < AT_ONCE; k++) {
+      const int w = w0 + 32 * k + lane;
+#pragma unroll
+      for (int j = 0; j < 8; j++) lo[k][j] = hi[k][j] = 0;
+      if (bits[k]) load8(low_bytes + 8 * (int64_t)w, lo[k]);
+      if (WIDE && wide[k] && bits[k]) load8(high_bytes + 8 * (int64_t)w, hi[k]);
     }
 #pragma unroll
-    for (int k = 0; k < FLIGHT; k++) {
+    for (int k = 0; k < AT_ONCE; k++) {
       seen += __popc(bits[k]);
-      const uint32_t low = __reduce_add_sync(0xffffffffu, squares<WIDE>(bits[k], lo[k], hi[k]));
-      if (lane == 0 && low) atomicAdd(&sums[g0 + k].x, low);
+      const uint32_t sum = squares<WIDE>(bits[k], lo[k], hi[k]);
+      const uint32_t first = __reduce_add_sync(0xffffffffu, lane < GROUP_WORDS ? sum : 0u), second = __reduce_add_sync(0xffffffffu, sum) - first;
+      const uint32_t low = lane == 0 ? first : second;
+      if (lane < 2 && low) atomicAdd(&sums[w0 / GROUP_WORDS + 2 * k + lane].x, low);
     }
   }
   return seen;
@@ -1062,20 +1069,22 @@ deg_build_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int64_t units, 
                  int32_t *__restrict__ count) {
   const int lane = threadIdx.x & 31;
   for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < units; u += (int64_t)gridDim.x * blockDim.x) {   // (whole warps)
-    uint32_t low[4] = {0u, 0u, 0u, 0u}, high[4] = {0u, 0u, 0u, 0u};
+    uint32_t low[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u}, high[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u}, any = 0u;   // two bytes of each of eight words
     int listed = 0;
 #pragma unroll
     for (int k = 0; k < 16; k++) {
       const int64_t v = 16 * u + k;
       const int32_t d = v < V ? row_ptr[v + 1] - row_ptr[v] : 0;
       if (d >= least) { listed += d < HUGE_DEGREE ? 1 : 0; continue; }
-      low[k >> 2] |= (uint32_t)(d & 255) << (8 * (k & 3));
-      high[k >> 2] |= (uint32_t)(d >> 8) << (8 * (k & 3));
+      low[k & 7] |= (uint32_t)(d & 255) << (8 * (k >> 3));
+      high[k & 7] |= (uint32_t)(d >> 8) << (8 * (k >> 3));
+      any |= (uint32_t)(d >> 8);
     }
-    deg[u] = make_uint4(low[0], low[1], low[2], low[3]);
-    deg[units + u] = make_uint4(high[0], high[1], high[2], high[3]);
+    uint16_t *to = reinterpret_cast<uint16_t *>(deg + (u & ~(int64_t)1)) + (u & 1);   // (see squares())
+#pragma unroll
+    for (int j = 0; j < 8; j++) { to[2 * j] = (uint16_t)low[j]; to[8 * units + 2 * j] = (uint16_t)high[j]; }
     const int64_t group = 16 * u / GROUP;
-    if (__any_sync(0xffffffffu, (high[0] | high[1] | high[2] | high[3]) != 0u) && lane == 0) atomicOr(wide + group / 32, 1u << (group & 31));
+    if (__any_sync(0xffffffffu, any != 0u) && lane == 0) atomicOr(wide + group / 32, 1u << (group & 31));
     listed = __reduce_add_sync(0xffffffffu, listed);
     if (lane == 0) count[group] = listed;
   }
