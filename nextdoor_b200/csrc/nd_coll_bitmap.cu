@@ -8,7 +8,7 @@
 //
 // What bounds it, and what is done about it (2^20 vertices, 1024 batches of 64, 2 layers of 64: FastGCN
 // 4.8 -> 0.59 ms, LADIES 5.7 -> 0.68 ms).  One CTA fills an SM there, and neither memory nor issue slots are full:
-// FastGCN issues in 48 % of the cycles (322 M instructions, 5.0 GB out of the L2), LADIES in 43 % (304 M instructions for 131 M
+// FastGCN issues in 43 % of the cycles (270 M instructions, 5.2 GB out of the L2), LADIES in 43 % (304 M instructions for 131 M
 // list entries, the distinct ones of 313 M); the warps wait for barriers between the phases, for loads and for shared memory:
 //  * The second layer's transits are hubs (FastGCN draws them with the square of their degree), many of them the
 //    same one: repeated transits of a batch are taken once (LADIES with their multiplicity).
