@@ -166,8 +166,8 @@ int nd_sampler_host_update_fetch(nd_sampler *s);
 int nd_sampler_host_update_finish(nd_sampler *s, int64_t *values_copied);
 /* dst[0..n) = value with the same host threads (first fill of a result array) */
 int nd_host_fill_int32(int32_t *dst, int64_t n, int32_t value);
-/* Host memory for result arrays (contents undefined).  While graphs or samplers are alive up to 256 MB of what is freed are kept for
- * the next one, and pinned when they are used again, so that a caller with a new array for every call neither faults its pages in again
+/* Host memory for result arrays (contents undefined).  While graphs or samplers are alive up to 256 MB of what is freed (and 64 MB of
+ * blocks below 2 MB) are kept for the next one, and pinned when they are used again, so that a caller with a new array for every call neither faults its pages in again
  * nor copies through a staging buffer. */
 int nd_result_alloc(int device, int64_t bytes, void **p);
 int nd_result_free(void *p);

@@ -55,14 +55,16 @@ class _PinnedMemory:
             self._free(self._p)
 
 
-# From here on (bytes) a result lies in memory that is kept and pinned: a copy into np.empty, page by page and through the
-# driver's buffer, takes 60 us more at 0.5 MB and 80 to 100 at 1 to 2 (module walks of 16 and 30 steps on 16 K vertices
-# 117 -> 61 and 180 -> 83 us, 2000 samples of 3 reference layers 167 -> 81).
+# From here on (bytes) a result lies in memory of the library's: new for a caller that holds its results, and then of their size;
+# lent again, and from then on pinned, for one that drops them.  A copy into pinned memory instead of np.empty, which goes through
+# the driver's buffer, takes 28 us less at 0.5 MB and 55 to 100 at 1 to 2 (module walks of 16 and 30 steps on 16 K vertices 117 -> 61
+# and 180 -> 83 us, 2000 samples of 3 reference layers 167 -> 81); 300 results held take 106 us each at 256 KB (145 in np.empty),
+# 187 at 0.5 MB (266), 345 at 1 MB (500).
 KEPT_RESULT = 256 << 10
 
 
 def _result_array(count, dtype, device):
-    """np.empty for results; large ones in memory that is not faulted in again for every call."""
+    """np.empty for results; from KEPT_RESULT bytes on in memory that is not faulted in again for every call."""
     large = KEPT_RESULT <= count * np.dtype(dtype).itemsize <= 128 << 20
     return np.asarray(_ResultMemory(count, dtype, device)) if large else np.empty(count, dtype)
 

@@ -473,64 +473,80 @@ void nd_block_free(int device, void *p, size_t bytes) {
 // ---------------------------------------------------------------- host memory of results that is kept
 
 namespace {
-constexpr size_t KEEP_RESULT = (size_t)128 << 20, KEEP_RESULTS = (size_t)256 << 20, HUGE_PAGE = (size_t)2 << 20;
+constexpr size_t KEEP_RESULT = (size_t)128 << 20, HUGE_PAGE = (size_t)2 << 20, SMALL_STEP = (size_t)64 << 10;
 struct HostBlock {
   void *p;
   size_t bytes;
   bool pinned;
 };
+// Blocks of less than a huge page are kept and pinned on an account of their own: a queue of small results, held and dropped,
+// neither pushes the large blocks out nor takes the pinned memory that they are to get.
+struct ResultPool {
+  size_t most;                           // of `bytes`, and of `pinned`
+  std::vector<HostBlock> free;           // oldest first
+  size_t bytes = 0, pinned = 0;          // of the free ones; of all that are pinned, lent ones too
+};
 std::mutex g_results_mutex;
-std::vector<HostBlock> g_results;   // free blocks, oldest first
-std::vector<HostBlock> g_lent;      // blocks that callers have
-size_t g_results_bytes = 0, g_pinned_bytes = 0;   // of the free ones; of all that are pinned
+ResultPool g_large{(size_t)256 << 20, {}}, g_small{(size_t)64 << 20, {}};
+std::vector<HostBlock> g_lent;           // blocks that callers have
+
+ResultPool &pool_of(size_t bytes) { return bytes < HUGE_PAGE ? g_small : g_large; }
 
 void unmap(const HostBlock &b) {   // under the lock
   if (b.pinned) {
     if (!g_exiting.load()) cudaHostUnregister(b.p);
-    g_pinned_bytes -= b.bytes;
+    pool_of(b.bytes).pinned -= b.bytes;
   }
   munmap(b.p, b.bytes);
 }
-void drop_results(size_t keep) {   // under the lock
-  while (g_results_bytes > keep) {
-    g_results_bytes -= g_results.front().bytes;
-    unmap(g_results.front());
-    g_results.erase(g_results.begin());
+void drop_results(ResultPool &pool, size_t keep) {   // under the lock
+  while (pool.bytes > keep) {
+    pool.bytes -= pool.free.front().bytes;
+    unmap(pool.free.front());
+    pool.free.erase(pool.free.begin());
   }
 }
 }  // namespace
 
 // Memory for a result array of a caller that makes a new one for every call: faulting 23 MB in takes as long as copying
 // them, and a copy into pageable memory 0.64 ms (35 GB/s, through the ring) instead of 0.44 (52).  So what is freed is
-// kept, and pinned when it is lent again -- a caller that keeps its results never gets there.  Contents undefined.
+// kept, and pinned when it is lent again -- a caller that keeps its results never gets there.  From 2 MB on blocks are whole
+// huge pages; below, where a caller may hold hundreds, steps of 64 KB whose pages are asked for at once, and one that is lent
+// again is a quarter larger at most (300 results of 256 KB held: 73 MB and 106 us each; a huge page each 582 MB and 275 us; faulted
+// in one by one 142 us, as in malloc's memory; of 1 MB 345, 370 and 490 us).  Contents undefined.
 extern "C" int nd_result_alloc(int device, int64_t bytes, void **p) {
   ND_REQUIRE(p && bytes > 0, ND_ERR_ARG, "nd_result_alloc: bad argument");
-  const size_t n = ((size_t)bytes + HUGE_PAGE - 1) / HUGE_PAGE * HUGE_PAGE;
-  std::lock_guard<std::mutex> lock(g_results_mutex);
-  size_t best = g_results.size();
-  for (size_t k = 0; k < g_results.size(); k++)   // (the last one freed of the smallest that fit)
-    if (g_results[k].bytes >= n && g_results[k].bytes / 2 <= n && (best == g_results.size() || g_results[k].bytes <= g_results[best].bytes)) best = k;
+  size_t n = ((size_t)bytes + SMALL_STEP - 1) / SMALL_STEP * SMALL_STEP;
+  if (n >= HUGE_PAGE) n = (n + HUGE_PAGE - 1) / HUGE_PAGE * HUGE_PAGE;
+  const size_t largest = n < HUGE_PAGE ? n + n / 4 : 2 * n;
+  std::unique_lock<std::mutex> lock(g_results_mutex);
+  ResultPool &pool = pool_of(n);
+  size_t best = pool.free.size();
+  for (size_t k = 0; k < pool.free.size(); k++)   // (the last one freed of the smallest that fit)
+    if (pool.free[k].bytes >= n && pool.free[k].bytes <= largest && (best == pool.free.size() || pool.free[k].bytes <= pool.free[best].bytes)) best = k;
   HostBlock b{nullptr, n, false};
-  if (best < g_results.size()) {
-    b = g_results[best];
-    g_results_bytes -= b.bytes;
-    g_results.erase(g_results.begin() + (long)best);
-    if (!b.pinned && g_pinned_bytes + b.bytes <= KEEP_RESULTS && !g_exiting.load()) {
+  if (best < pool.free.size()) {
+    b = pool.free[best];
+    pool.bytes -= b.bytes;
+    pool.free.erase(pool.free.begin() + (long)best);
+    if (!b.pinned && pool.pinned + b.bytes <= pool.most && !g_exiting.load()) {
       b.pinned = cudaSetDevice(device) == cudaSuccess && cudaHostRegister(b.p, b.bytes, cudaHostRegisterPortable) == cudaSuccess;
-      if (b.pinned) g_pinned_bytes += b.bytes;
+      if (b.pinned) pool.pinned += b.bytes;
       else cudaGetLastError();
     }
   } else {
-    b.p = mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    lock.unlock();
+    b.p = mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | (n < HUGE_PAGE ? MAP_POPULATE : 0), -1, 0);
     ND_REQUIRE(b.p != MAP_FAILED, ND_ERR_RANGE, "no memory for a result of %lld bytes", (long long)bytes);
-    madvise(b.p, n, MADV_HUGEPAGE);
+    if (n >= HUGE_PAGE) madvise(b.p, n, MADV_HUGEPAGE);
+    lock.lock();
   }
   g_lent.push_back(b);
   *p = b.p;
   return ND_OK;
 }
 
-// kept for the next result while graphs or samplers are alive, 256 MB in all
+// kept for the next result while graphs or samplers are alive, 256 MB in all and 64 MB of small ones
 extern "C" int nd_result_free(void *p) {
   std::lock_guard<std::mutex> objects(g_objects_mutex);
   std::lock_guard<std::mutex> lock(g_results_mutex);
@@ -539,9 +555,10 @@ extern "C" int nd_result_free(void *p) {
     const HostBlock b = g_lent[k];
     g_lent.erase(g_lent.begin() + (long)k);
     if (b.bytes > KEEP_RESULT || g_objects <= 0) { unmap(b); return ND_OK; }
-    g_results.push_back(b);
-    g_results_bytes += b.bytes;
-    drop_results(KEEP_RESULTS);
+    ResultPool &pool = pool_of(b.bytes);
+    pool.free.push_back(b);
+    pool.bytes += b.bytes;
+    drop_results(pool, pool.most);
     return ND_OK;
   }
   ND_REQUIRE(!p, ND_ERR_ARG, "nd_result_free: not a result's memory");
@@ -569,7 +586,8 @@ void nd_objects_add(int n) {
   if (g_objects > 0) return;
   {
     std::lock_guard<std::mutex> results(g_results_mutex);
-    drop_results(0);
+    drop_results(g_large, 0);
+    drop_results(g_small, 0);
   }
   std::lock_guard<std::mutex> blocks(g_blocks_mutex);
   int now = 0;

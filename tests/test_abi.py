@@ -102,3 +102,25 @@ def test_host_fill_of_any_words(offset, n):
     a = np.full(n + 16, -5, np.int32)
     api.host_fill(a[offset:offset + n], 7)
     assert (a[offset:offset + n] == 7).all() and (a[:offset] == -5).all() and (a[offset + n:] == -5).all()
+
+
+@pytest.mark.parametrize("nbytes", [256 << 10, (256 << 10) + 4, (1 << 20) - 4, 1 << 20, 3 << 19])
+def test_results_that_a_caller_holds_take_their_size(lib, nbytes):
+    """A hundred results: memory of their size, in steps of 64 KB below 2 MB, all of it the caller's."""
+    def held():
+        return int(open("/proc/self/statm").read().split()[0]) * os.sysconf("SC_PAGE_SIZE")
+
+    def result():
+        p = C.c_void_p()
+        assert lib.lib.nd_result_alloc(0, nbytes, C.byref(p)) == 0
+        return p
+
+    before, step = held(), 64 << 10
+    results = [result() for _ in range(100)]
+    assert held() - before <= 100 * ((nbytes + step - 1) // step * step) + (8 << 20)
+    for i, p in enumerate(results):
+        C.memset(p, i, nbytes)
+    for i, p in enumerate(results):
+        assert C.string_at(p, nbytes) == bytes([i]) * nbytes
+        assert lib.lib.nd_result_free(p) == 0
+    assert held() - before <= 8 << 20

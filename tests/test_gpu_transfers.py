@@ -235,3 +235,29 @@ def test_results_of_the_smallest_size_that_is_kept(nd, small_graph, nbytes):
         for s, e in zip(jobs, exp):
             assert np.array_equal(s.final_samples(), e)
     assert np.array_equal(held, exp[0]) and not np.array_equal(exp[0], exp[1])
+
+
+def test_small_results_leave_the_large_ones_their_memory(nd):
+    """A queue of results below 2 MB, held and dropped again and again, and a large one that is lent, pinned, kept."""
+    import torch
+    large = nd.Sampler(nd.Graph.rmat(5000, 40_000, seed=1), nd.app_params(0, steps=100, seed=1), num_samples=50_000)
+    small = nd.Sampler(large.graph, nd.app_params(0, steps=1, seed=2), num_samples=1 << 16)
+    large.sample()
+    small.sample()
+    exp_large, exp = np.zeros((50_000, 100), np.int32), np.zeros((1 << 16, 1), np.int32)
+    large.final_samples(exp_large)
+    small.final_samples(exp)
+    for _ in range(3):
+        queue = [small.final_samples() for _ in range(300)]
+        assert all(np.array_equal(a, exp) for a in queue)
+        del queue
+    for turn in range(3):
+        result = large.final_samples()
+        assert np.array_equal(result, exp_large)
+        assert turn == 0 or torch.from_numpy(result).is_pinned()
+        del result
+    at = large.final_samples().ctypes.data
+    queue = [small.final_samples() for _ in range(300)]
+    del queue
+    result = large.final_samples()
+    assert result.ctypes.data == at and torch.from_numpy(result).is_pinned() and np.array_equal(result, exp_large)
