@@ -87,8 +87,8 @@ struct Layout {
 // vertices there is room for on a list of n
 __host__ __device__ inline int64_t listed_room(int64_t n) { return (n + 7) / 8 * 8 + 8; }
 
-// The degrees, FastGCN.  Codes: the low bytes of 32 vertices' each in two (squares() says in which order), then the high ones; a
-// listed vertex's is zero.
+// The degrees, FastGCN.  Codes: the low bytes of 32 vertices' each in two (squares() says in which order), then the high ones if
+// there are any; a listed vertex's is zero.
 struct Degrees {
   const uint4 *__restrict__ codes;
   const uint32_t *__restrict__ wide;        // a bit per group: it has high bytes that are not zero; null: none has
@@ -1049,66 +1049,99 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
 
 // ---------------------------------------------------------------- arrays built once per graph
 
-// vertices with at least 256, BIG_DEGREE, HUGE_DEGREE neighbours
-__global__ void __launch_bounds__(256) deg_count_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int32_t *__restrict__ count) {
-  int32_t n[3] = {0, 0, 0};
-  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V; v += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t d = row_ptr[v + 1] - row_ptr[v];
-    n[0] += d >= 256 ? 1 : 0; n[1] += d >= BIG_DEGREE ? 1 : 0; n[2] += d >= HUGE_DEGREE ? 1 : 0;
-  }
-  for (int k = 0; k < 3; k++) {
-    n[k] = __reduce_add_sync(0xffffffffu, n[k]);
-    if ((threadIdx.x & 31) == 0 && n[k]) atomicAdd(count + k, n[k]);
-  }
-}
-
-// A warp per group, a lane per sixteen vertices: codes, flags, and how many of the group's vertices have `least` neighbours or
-// more; then those onto their list, and the ones for `huge` onto theirs, in any order.
-__global__ void __launch_bounds__(256)
-deg_build_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int64_t units, int32_t least, uint4 *__restrict__ deg, uint32_t *__restrict__ wide,
-                 int32_t *__restrict__ count) {
-  const int lane = threadIdx.x & 31;
+// The degrees of a lane's sixteen vertices, a warp per group: f(group, u, d).
+template <class F>
+__device__ __forceinline__ void for_groups(const int32_t *__restrict__ row_ptr, int32_t V, int64_t units, F f) {
   for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < units; u += (int64_t)gridDim.x * blockDim.x) {   // (whole warps)
-    uint32_t low[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u}, high[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u}, any = 0u;   // two bytes of each of eight words
-    int listed = 0;
-#pragma unroll
-    for (int k = 0; k < 16; k++) {
-      const int64_t v = 16 * u + k;
-      const int32_t d = v < V ? row_ptr[v + 1] - row_ptr[v] : 0;
-      if (d >= least) { listed += d < HUGE_DEGREE ? 1 : 0; continue; }
-      low[k & 7] |= (uint32_t)(d & 255) << (8 * (k >> 3));
-      high[k & 7] |= (uint32_t)(d >> 8) << (8 * (k >> 3));
-      any |= (uint32_t)(d >> 8);
-    }
-    uint16_t *to = reinterpret_cast<uint16_t *>(deg + (u & ~(int64_t)1)) + (u & 1);   // (see squares())
-#pragma unroll
-    for (int j = 0; j < 8; j++) { to[2 * j] = (uint16_t)low[j]; to[8 * units + 2 * j] = (uint16_t)high[j]; }
-    const int64_t group = 16 * u / GROUP;
-    if (__any_sync(0xffffffffu, any != 0u) && lane == 0) atomicOr(wide + group / 32, 1u << (group & 31));
-    listed = __reduce_add_sync(0xffffffffu, listed);
-    if (lane == 0) count[group] = listed;
-  }
-}
-
-__global__ void __launch_bounds__(256)
-deg_list_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int64_t units, int32_t least, const int32_t *__restrict__ listed_at, int32_t *__restrict__ listed, uint2 *__restrict__ weights,
-                NdBigVertex *__restrict__ huge, int32_t *__restrict__ n_huge) {
-  const int lane = threadIdx.x & 31;
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < units; u += (int64_t)gridDim.x * blockDim.x) {
     int32_t d[16];
-    int mine = 0;
 #pragma unroll
     for (int k = 0; k < 16; k++) {
       const int64_t v = 16 * u + k;
       d[k] = v < V ? row_ptr[v + 1] - row_ptr[v] : 0;
-      mine += d[k] >= least && d[k] < HUGE_DEGREE ? 1 : 0;
+    }
+    f(16 * u / GROUP, u, d);
+  }
+}
+
+// Vertices with at least 256, BIG_DEGREE, HUGE_DEGREE neighbours; of a group, those of the first two kinds that are not of the third,
+// in the low and the high half of a word.
+__global__ void __launch_bounds__(256) deg_count_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int64_t units, int32_t *__restrict__ count,
+                                                        uint32_t *__restrict__ of_group) {
+  int32_t all[3] = {0, 0, 0};
+  for_groups(row_ptr, V, units, [&](int64_t group, int64_t, const int32_t (&d)[16]) {
+    int32_t n[3] = {0, 0, 0};
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+      n[0] += d[k] >= 256 ? 1 : 0; n[1] += d[k] >= BIG_DEGREE ? 1 : 0; n[2] += d[k] >= HUGE_DEGREE ? 1 : 0;
+    }
+    const uint32_t both = __reduce_add_sync(0xffffffffu, (uint32_t)(n[0] - n[2]) | (uint32_t)(n[1] - n[2]) << 16);
+    if ((threadIdx.x & 31) == 0) of_group[group] = both;
+    for (int k = 0; k < 3; k++) all[k] += n[k];
+  });
+  for (int k = 0; k < 3; k++) {
+    all[k] = __reduce_add_sync(0xffffffffu, all[k]);
+    if ((threadIdx.x & 31) == 0 && all[k]) atomicAdd(count + k, all[k]);
+  }
+}
+
+// where a group's vertices begin on the list, in the place of its counts (the half `shift` says), by one CTA
+constexpr int STARTS_THREADS = 1024;
+__global__ void __launch_bounds__(STARTS_THREADS) deg_starts_kernel(uint32_t *__restrict__ of_group, int groups, int shift) {
+  __shared__ uint32_t sums[STARTS_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t before = 0;
+  for (int g0 = 0; g0 < groups; g0 += STARTS_THREADS) {
+    const int g = g0 + (int)threadIdx.x;
+    const uint32_t own = g < groups ? (of_group[g] >> shift) & 0xffffu : 0u;
+    uint32_t upto = own;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += t;
+    }
+    if (lane == 31) sums[warp] = upto;
+    __syncthreads();
+    uint32_t start = before + upto - own;
+    for (int w = 0; w < STARTS_THREADS / 32; w++) {
+      if (w < warp) start += sums[w];
+      before += sums[w];
+    }
+    if (g < groups) of_group[g] = start;
+    __syncthreads();
+  }
+}
+
+// Codes, with `high` the high bytes and a flag per group, and the vertices with `least` neighbours and more: onto the list, or onto
+// the one of the huge ones, in any order.
+__global__ void __launch_bounds__(256)
+deg_build_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int64_t units, int32_t least, uint4 *__restrict__ low_bytes, uint4 *__restrict__ high_bytes,
+                 uint32_t *__restrict__ wide, const uint32_t *__restrict__ starts, int32_t *__restrict__ listed, uint2 *__restrict__ weights,
+                 NdBigVertex *__restrict__ huge, int32_t *__restrict__ n_huge) {
+  const int lane = threadIdx.x & 31;
+  for_groups(row_ptr, V, units, [&](int64_t group, int64_t u, const int32_t (&d)[16]) {
+    uint32_t low[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u}, high[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u}, any = 0u;   // two bytes of each of eight words
+    int mine = 0;
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+      if (d[k] >= least) { mine += d[k] < HUGE_DEGREE ? 1 : 0; continue; }
+      low[k & 7] |= (uint32_t)(d[k] & 255) << (8 * (k >> 3));
+      high[k & 7] |= (uint32_t)(d[k] >> 8) << (8 * (k >> 3));
+      any |= (uint32_t)(d[k] >> 8);
+    }
+    uint16_t *to = reinterpret_cast<uint16_t *>(low_bytes + (u & ~(int64_t)1)) + (u & 1);   // (see squares())
+#pragma unroll
+    for (int j = 0; j < 8; j++) to[2 * j] = (uint16_t)low[j];
+    if (high_bytes) {
+      to = reinterpret_cast<uint16_t *>(high_bytes + (u & ~(int64_t)1)) + (u & 1);
+#pragma unroll
+      for (int j = 0; j < 8; j++) to[2 * j] = (uint16_t)high[j];
+      if (__any_sync(0xffffffffu, any != 0u) && lane == 0) atomicOr(wide + group / 32, 1u << (group & 31));
     }
     int upto = mine;
     for (int o = 1; o < 32; o <<= 1) {
       const int t = __shfl_up_sync(0xffffffffu, upto, o);
       if (lane >= o) upto += t;
     }
-    int32_t at = listed_at[16 * u / GROUP] + upto - mine;
+    uint32_t at = starts[group] + (uint32_t)(upto - mine);
 #pragma unroll
     for (int k = 0; k < 16; k++) {
       if (d[k] < least) continue;
@@ -1117,10 +1150,11 @@ deg_list_kernel(const int32_t *__restrict__ row_ptr, int32_t V, int64_t units, i
         sum.add(d[k]);
         weights[at] = make_uint2(sum.low, sum.high);
         listed[at++] = (int32_t)(16 * u + k);
+      } else {
+        huge[atomicAdd(n_huge, 1)] = NdBigVertex{(int32_t)(16 * u + k), square(d[k])};
       }
-      else huge[atomicAdd(n_huge, 1)] = NdBigVertex{(int32_t)(16 * u + k), square(d[k])};
     }
-  }
+  });
 }
 
 // fp64 sums of the rows' weights (the order of the adds does not matter)
@@ -1296,47 +1330,38 @@ int ensure_hubs(const nd_graph *g, int grid) {
 }
 
 // FastGCN: the packed degrees and the vertices whose degrees they do not hold, listed: from 256 on where those are few, else
-// from BIG_DEGREE on.
+// from BIG_DEGREE on, with a second byte per vertex.  In one allocation: low bytes, high bytes and flags, the listed ones' weights
+// and ids, the huge ones.
 int ensure_degrees(const nd_graph *g, int grid) {
   if (g->deg_codes) return ND_OK;
-  const int64_t units = 2 * (int64_t)words_of(g->V);
-  const size_t groups = (size_t)units / (GROUP / 16), flags = (groups + 31) / 32 + 1;
-  NdDevMem<uint4> deg;
-  NdDevMem<int32_t> at;
-  NdDevMem<uint2> listed;     // weights, then vertices
-  NdDevMem<NdBigVertex> huge;
+  const int64_t words = words_of(g->V), units = 2 * words;
+  const int groups = (int)(words / GROUP_WORDS);
+  NdDevMem<int32_t> counts;   // of n, of the huge ones that are listed, of the groups
+  ND_TRY(counts.alloc((size_t)groups + 4));
+  uint32_t *const of_group = reinterpret_cast<uint32_t *>(counts.p + 4);
+  ND_CUDA(cudaMemset(counts.p, 0, sizeof(int32_t) * 4));
+  deg_count_kernel<<<grid, 256>>>(g->row_ptr, g->V, units, counts.p, of_group);
   int32_t n[3] = {0, 0, 0};   // vertices with at least 256, BIG_DEGREE, HUGE_DEGREE neighbours
-  ND_TRY(deg.alloc((size_t)(2 * units) + (flags + 3) / 4));
-  ND_TRY(at.alloc(groups + 5));
-  int32_t *const count = at.p + groups + 1;   // of n, then of the huge ones listed
-  ND_CUDA(cudaMemset(at.p, 0, sizeof(int32_t) * (groups + 5)));
-  ND_CUDA(cudaMemset(deg.p + 2 * units, 0, sizeof(uint32_t) * flags));
-  deg_count_kernel<<<grid, 256>>>(g->row_ptr, g->V, count);
-  ND_CUDA(cudaMemcpy(n, count, sizeof(n), cudaMemcpyDeviceToHost));
+  ND_CUDA(cudaMemcpy(n, counts.p, sizeof(n), cudaMemcpyDeviceToHost));
   const bool few = (int64_t)n[0] * LISTED <= g->V;
-  const int32_t least = few ? 256 : BIG_DEGREE;
-  const size_t n_listed = (size_t)(n[few ? 0 : 1] - n[2]), room = (size_t)listed_room((int64_t)n_listed);
-  ND_TRY(listed.alloc(room + room / 2));
-  ND_CUDA(cudaMemset(listed.p, 0, sizeof(uint2) * (room + room / 2)));
-  ND_TRY(huge.alloc((size_t)n[2] + 1));
-  deg_build_kernel<<<grid, 256>>>(g->row_ptr, g->V, units, least, deg.p, reinterpret_cast<uint32_t *>(deg.p + 2 * units), at.p);
-  std::vector<int32_t> starts(groups + 1);
-  ND_CUDA(cudaMemcpy(starts.data(), at.p, sizeof(int32_t) * groups, cudaMemcpyDeviceToHost));
-  int32_t all = 0;
-  for (int32_t &s : starts) {
-    const int32_t own = s;
-    s = all;
-    all += own;
-  }
-  ND_CUDA(cudaMemcpy(at.p, starts.data(), sizeof(int32_t) * (groups + 1), cudaMemcpyHostToDevice));
-  deg_list_kernel<<<grid, 256>>>(g->row_ptr, g->V, units, least, at.p, reinterpret_cast<int32_t *>(listed.p + room), listed.p, huge.p, count + 3);
+  const size_t plane = 32 * (size_t)words, high = few ? 0 : plane, flags = few ? 0 : ((size_t)groups + 255) / 256 * 32;
+  const size_t n_listed = (size_t)(n[few ? 0 : 1] - n[2]), room = (size_t)listed_room((int64_t)n_listed), lists = 12 * room;
+  NdDevMem<unsigned char> deg;
+  ND_TRY(deg.alloc(plane + high + flags + lists + sizeof(NdBigVertex) * ((size_t)n[2] + 1)));
+  unsigned char *const at_high = deg.p + plane, *const at_flags = at_high + high, *const at_lists = at_flags + flags;
+  uint2 *const weights = reinterpret_cast<uint2 *>(at_lists);
+  NdBigVertex *const huge = reinterpret_cast<NdBigVertex *>(at_lists + lists);
+  ND_CUDA(cudaMemset(at_flags, 0, flags + lists));
+  deg_starts_kernel<<<1, STARTS_THREADS>>>(of_group, groups, few ? 0 : 16);
+  deg_build_kernel<<<grid, 256>>>(g->row_ptr, g->V, units, few ? 256 : BIG_DEGREE, reinterpret_cast<uint4 *>(deg.p), few ? nullptr : reinterpret_cast<uint4 *>(at_high),
+                                  reinterpret_cast<uint32_t *>(at_flags), of_group, reinterpret_cast<int32_t *>(weights + room), weights, huge, counts.p + 3);
   ND_CUDA(cudaDeviceSynchronize());
   g->n_huge = n[2];
   g->deg_wide = !few;
-  g->huge = huge.release();
-  g->listed = listed.release();
+  g->huge = huge;
+  g->listed = weights;
   g->n_listed = (int)n_listed;
-  g->deg_codes = deg.release();
+  g->deg_codes = reinterpret_cast<uint4 *>(deg.release());
   return ND_OK;
 }
 

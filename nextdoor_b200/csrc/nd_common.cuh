@@ -130,11 +130,11 @@ struct nd_graph {
   mutable int odd_max = -1;            // some row's maximum weight rules `pack` and `codes` out (-1: not asked yet)
   mutable int32_t *adjset = nullptr;   // node2vec membership: per-vertex hash sets of the neighbour ids, 8-slot buckets
   mutable uint32_t *adjsign = nullptr; // ... and the filter in front of them
-  mutable uint4 *deg_codes = nullptr;  // degrees of 32 vertices in two each, low bytes, high bytes, flags (FastGCN)
-  mutable uint2 *listed = nullptr;         // [n_listed] weights and vertices whose degrees the codes do not hold, and those, except
-  mutable NdBigVertex *huge = nullptr;     // ... [n_huge], whose weights the groups' sums do not hold
+  mutable uint4 *deg_codes = nullptr;  // degrees of 32 vertices in two each: low bytes, if deg_wide high bytes and flags (FastGCN); in the same allocation
+  mutable uint2 *listed = nullptr;     // [n_listed] weights and vertices whose degrees the codes do not hold, and those, except
+  mutable NdBigVertex *huge = nullptr; // ... [n_huge], whose weights the groups' sums do not hold
   mutable int n_listed = 0, n_huge = 0;
-  mutable bool deg_wide = false;           // the codes have high bytes
+  mutable bool deg_wide = false;       // the codes have high bytes
   mutable float *term = nullptr;       // [E] (w / rowsum)^2 (LADIES)
   mutable int32_t *hub_slot = nullptr; // [V] slot of the vertex's neighbourhood as a bitmap, -1: none
   mutable uint32_t *hub_bits = nullptr;

@@ -496,7 +496,7 @@ static void free_graph(nd_graph *g) {
   if (g->block) nd_block_free(g->device, g->block, g->block_bytes);
   else { cudaFree(g->row_ptr); cudaFree(g->col); cudaFree(g->w); cudaFree(g->max_w); }
   cudaFree(g->colw); cudaFree(g->vrec); cudaFree(g->vrow); cudaFree(g->erec); cudaFree(g->pack); cudaFree(g->codes); cudaFree(g->col3); cudaFree(g->adjset); cudaFree(g->adjsign);
-  cudaFree(g->deg_codes); cudaFree(g->listed); cudaFree(g->huge); cudaFree(g->term); cudaFree(g->hub_slot); cudaFree(g->hub_bits); cudaFree(g->hubs); cudaFree(g->hub_ids); cudaFree(g->hub_terms); cudaFree(g->hub_offs);
+  cudaFree(g->deg_codes); cudaFree(g->term); cudaFree(g->hub_slot); cudaFree(g->hub_bits); cudaFree(g->hubs); cudaFree(g->hub_ids); cudaFree(g->hub_terms); cudaFree(g->hub_offs);
   for (const NdHubTable &t : g->hub_tables) { cudaFree(t.sums); cudaFree(t.starts); }
   delete g;
 }

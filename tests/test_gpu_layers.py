@@ -338,3 +338,22 @@ def test_adjacency_by_length_of_the_lists(nd, ndo, app, B, L):
             assert np.array_equal(rows[k, step, :len(exp)] >= 0, exp) and (rows[k, step, len(exp):] == -1).all()
             found += exp.sum()
     assert found > S * L
+
+
+@pytest.mark.parametrize("many", [False, True])
+def test_fastgcn_tables_of_a_graph(nd, many):
+    """A byte of degree per vertex, two where many have 256 neighbours and more, beside the hubs' slots and one bitmap at least."""
+    import torch
+    V = 1 << 23
+    deg = np.zeros(V, np.int64)
+    deg[::31 if many else 4096] = 256 if many else 3
+    row_ptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    col = (np.arange(row_ptr[-1]) % V).astype(np.int32)
+    g = nd.Graph.from_csr(row_ptr, col, np.ones(len(col), np.float32), None)
+    torch.cuda.synchronize()
+    free, samplers = [torch.cuda.mem_get_info()[0]], []
+    for _ in range(3):
+        samplers.append(nd.Sampler(g, nd.app_params(8, steps=1, fanout=8, batch=8, seed=3), num_samples=4))
+        free.append(torch.cuda.mem_get_info()[0])
+    tables = (free[0] - free[1]) - (free[2] - free[3])
+    assert tables <= 4 * V + V // 8 + (2 * V + V // 4096 if many else V) + (6 << 20)   # memory comes in pieces of 2 MB
