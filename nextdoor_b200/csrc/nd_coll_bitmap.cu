@@ -690,12 +690,17 @@ __device__ __forceinline__ void probe_rows(const int32_t *__restrict__ col, cons
 }
 
 // SUMS_FAR: LADIES' group sums are in the big part.
+// 64 registers a thread.  Counters that only one thread needs are in shared memory: in registers they had FastGCN store 48 bytes a
+// thread in local memory and load 32 (-Xptxas -v; now none), LADIES 36 and 24 (now 24 and 16, which scan_f64's eight elements take;
+// two a thread take none, but leave more to add up).  1024 batches on 2^20 vertices FastGCN 718 -> 705 us, LADIES 1184 -> 1170 (edges 32 a vertex);
+// on 70 K FastGCN 165 -> 163.
 template <bool LADIES, bool SUMS_FAR>
 __global__ void __launch_bounds__(1024, 1)
 coll_bitmap_kernel(const __grid_constant__ Args a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ long long sh_sample;
   __shared__ int sh_hubs, sh_rest;
+  __shared__ uint32_t sh_drawn;   // layers with draws; thread 0's
   const Layout &lay = a.lay;
   CollParams cp = a.cp;
   unsigned char *big = lay.glob_bytes ? a.gscratch + (size_t)blockIdx.x * lay.glob_bytes : smem;
@@ -717,7 +722,8 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
   uint32_t *sh_firsts = reinterpret_cast<uint32_t *>(sh_slot_group + cp.L);   // draws that are the first of their group, as bits
   uint8_t *slot = (LADIES && !SUMS_FAR ? smem : big) + lay.off_slot;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
-  unsigned long long ids_sum = 0, uniq_sum = 0, draws = 0;   // the thread's; draws: thread 0's
+  unsigned long long ids_sum = 0, uniq_sum = 0;   // the thread's
+  if (tid == 0) sh_drawn = 0;
   for (int64_t s = blockIdx.x; s < a.S;) {
     for (int step = 0; step < a.steps; step++) {
       cp.step = step;
@@ -995,7 +1001,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
           a.prob[s * cp.fs + (int64_t)cp.step * cp.L + j] = pr;
         }
       }
-      if (tid == 0) { if (candidates && total > 0.0) draws += (unsigned long long)cp.L; }
+      if (tid == 0) { if (candidates && total > 0.0) sh_drawn++; }
       __syncthreads();
       uint32_t *adj = a.adj + (s * a.steps + cp.step) * (int64_t)adj_words(cp.stride);
       const int row_words = (cp.L + 31) / 32;
@@ -1037,7 +1043,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
   }
   __syncthreads();
   if (tid == 0) {
-    atomicAdd(&a.acc[0], draws);
+    atomicAdd(&a.acc[0], (unsigned long long)sh_drawn * (unsigned long long)cp.L);
     __threadfence();
     if (atomicAdd(&a.acc[10], 1ull) == (unsigned long long)gridDim.x - 1ull) {   // the last CTA
       __threadfence();
