@@ -1519,8 +1519,11 @@ Plan plan_of(const nd_sampler *s) {
     if (ladies && l.slots < 1) { l.slots = 1; l.bytes += 8u << LADIES_GROUP_BITS; }
   }
   // Where two fit an SM: with no more samples than SMs a sample has one for itself (140 batches of 64, 2 layers of 64: 70 K
-  // vertices, FastGCN 67 -> 63 us, LADIES 95 -> 82; 330 K: 91 -> 82, 120 -> 94; but 56 -> 58 where FastGCN's batches, layers and graph
-  // are all small: 32, 120 K).  With many samples, three or four smaller CTAs
+  // vertices, FastGCN 67 -> 63 us, LADIES 95 -> 82; 330 K: 91 -> 82, 120 -> 94), except where batch, layer and graph are so small that
+  // 32 warps wait for one another longer than 16 work (up to 131 K vertices, 20 and 148 batches; FastGCN on 3, 30, 70, 125 K vertices of 8: 33 -> 27,
+  // 34.7 -> 30.9, 38.7 -> 35.3, 38.3 -> 36.9, of 40 40.2 -> 35.1, 41.3 -> 39.2, 47.0 -> 45.5, 47.1 -> 47.3, but of 64 43.4, 45.2, 52 and 54 us instead of
+  // 43.3, 43.4, 51.5 and 51.6; LADIES on 3, 30, 70, 125 K of 8 41 -> 37, 39.2 -> 37.1, 41.9 -> 40.7, 41.6 -> 39.1, on 5 to 30 K of 12 39.2 .. 46.3 -> 37.5 .. 45,
+  // of 16 on 3 and 8 K 44.7 -> 41.5, 43.2 -> 41.4, but 53.5 -> 55.6 on 70 K).  With many samples, three or four smaller CTAs
   // overlap better while the graph is small (70 K, 1024 batches, two, three, four an SM: 215, 206, 187; 322, 314, 290; 500 K,
   // 640: 412, 448 with three), unless their last round would be nearly empty (700: 166, 155, 158) or, LADIES, there were not
   // accumulators for half of the draws at a time (batches and layers of 100, 100 K, 520: 475, 533), for three quarters on larger
@@ -1530,7 +1533,7 @@ Plan plan_of(const nd_sampler *s) {
   p.per_sm = two ? 2 : 1;
   const bool small = V <= SHARED_V / 2;
   if (two && s->S <= s->dev.sms) {
-    if (ladies || !small || ntr > 32) p.per_sm = 1;
+    if (!small || ntr > (!ladies ? 40 : V <= SHARED_V / 32 ? 16 : 12)) p.per_sm = 1;
   }
   if (two && p.per_sm == 1) {
     fits(l.group_bits, false, optin);

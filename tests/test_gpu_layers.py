@@ -357,3 +357,26 @@ def test_fastgcn_tables_of_a_graph(nd, many):
         free.append(torch.cuda.mem_get_info()[0])
     tables = (free[0] - free[1]) - (free[2] - free[3])
     assert tables <= 4 * V + V // 8 + (2 * V + V // 4096 if many else V) + (6 << 20)   # memory comes in pieces of 2 MB
+
+
+@pytest.mark.parametrize("app,V,B,L", [(8, 20_000, 8, 8), (9, 20_000, 8, 8), (9, 5000, 16, 16), (8, 5000, 40, 33), (8, 5000, 41, 33), (8, 200_000, 32, 32), (9, 200_000, 32, 32),
+                                       (9, 200_000, 64, 64), (8, 260_000, 32, 48), (8, 400_000, 64, 64), (9, 400_000, 48, 32)])
+def test_layers_by_number_of_samples_and_size(nd, app, V, B, L):
+    """Samples share an SM by how many there are, by the layers' size and by the graph's; a sample's layers depend on none of it."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    g = nd.Graph.rmat(V, 10 * V, seed=1)
+    init = np.random.default_rng(V).integers(0, V, (4 * sms + 8) * B).astype(np.int32)
+
+    def job(first, S):
+        s = nd.Sampler(g, nd.app_params(app, steps=2, fanout=L, batch=B, seed=3), num_samples=S, first_sample=first, initial=init[first * B:(first + S) * B])
+        s.sample()
+        aux = s.aux()
+        return [x.reshape(S, -1) for x in (s.final_samples(), aux["adj_row"], aux["adj_col"], aux["prob"])]
+
+    one = [np.concatenate(x) for x in zip(*(job(first, sms) for first in range(0, 4 * sms, sms)))]
+    for first, S in [(5, sms + 1), (0, 2 * sms), (sms, 2 * sms + sms // 2), (0, 3 * sms), (0, 4 * sms)]:
+        got = job(first, S)
+        for x, exp in zip(got[:3], one):
+            assert np.array_equal(x, exp[first:first + S])
+        assert np.allclose(got[3], one[3][first:first + S], rtol=1e-6, atol=0)   # 32-bit results of 64-bit sums in another order
