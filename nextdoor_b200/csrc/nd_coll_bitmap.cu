@@ -65,6 +65,10 @@ constexpr int FLIGHT = 4;         // pairs of groups a warp sums at a time (2^20
 constexpr int HUB = 128;          // a vertex with at least V / HUB neighbours has a bitmap of them
 constexpr int32_t SHARED_V = 1 << 18;   // see plan_of()
 constexpr int FEW = 64;           // lists with fewer than V / FEW entries in all are weighed entry by entry
+// Entries a thread, up to which lists that are weighed entry by entry are taken an entry at a time, and not eight (148 batches of 4, layers
+// of 4, 30 K vertices: 29.9 us, one 26.3, two 26.2, four 26.3; 125 K: 33.7, 33.1, 30.9, 30.9; 1000 of 64 on 1 M: 527, 523, 521, 521, without a
+// limit 533; 148 of 16, 40 edges a vertex, 106, 106, 106, 106, 115).
+constexpr int ENTRIES = 4;
 constexpr int SUB = 16;           // LADIES: lanes that add up a group of a hub (100 K vertices: 32 0.62, 16 0.595, 8 0.595, 4 0.60 ms; 2^20: 0.77, 0.77, 0.78, 0.80)
 constexpr int OCT = 8;            // list entries a thread takes at a time: 32 aligned bytes (LADIES)
 
@@ -377,6 +381,28 @@ __device__ __forceinline__ uint32_t add_lists(const NdGraphView &g, const Transi
       sum.add(deg[j]);
     }
     sum.to(sums, at);
+  }
+  return added;
+}
+
+// ... with WEIGHTS, an entry to a thread: eight are one after another, which lists that leave most of the CTA idle need not wait for.
+__device__ __forceinline__ uint32_t add_entries(const NdGraphView &g, const Transit *rest, int n, const uint32_t *pre, uint32_t total, uint32_t *bm, uint2 *sums) {
+  uint32_t added = 0;
+  for (uint32_t x = threadIdx.x; x < total * OCT; x += blockDim.x) {
+    const uint32_t o = x / OCT;
+    const int i = list_of_oct(pre, n, o);
+    const Transit t = rest[i];
+    const int64_t e = ((int64_t)((uint32_t)t.rs / OCT) + (int64_t)(o - pre[i])) * OCT + x % OCT;
+    if (e < t.rs || e >= (int64_t)t.rs + t.deg) continue;
+    const int32_t v = __ldg(g.col + e);
+    const uint32_t bit = 1u << (v & 31);
+    if (bm[(uint32_t)v >> 5] & bit) continue;
+    const int32_t from = __ldg(g.row_ptr + v), to = __ldg(g.row_ptr + v + 1);
+    if (atomicOr(bm + ((uint32_t)v >> 5), bit) & bit) continue;
+    added++;
+    Sum sum;
+    sum.add(to - from);
+    sum.to(sums, v / GROUP);
   }
   return added;
 }
@@ -818,7 +844,7 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
         }
         if (few) {
           if (nh > 0) __syncthreads();
-          seen += add_lists<true>(a.g, rest, nu - nh, pre, octs, bm, gsum);
+          seen += octs * OCT <= ENTRIES * blockDim.x ? add_entries(a.g, rest, nu - nh, pre, octs, bm, gsum) : add_lists<true>(a.g, rest, nu - nh, pre, octs, bm, gsum);
         }
       } else {
         // ---- the groups' weights and the rest of the union, then the number of candidates

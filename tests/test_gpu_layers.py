@@ -380,3 +380,26 @@ def test_layers_by_number_of_samples_and_size(nd, app, V, B, L):
         for x, exp in zip(got[:3], one):
             assert np.array_equal(x, exp[first:first + S])
         assert np.allclose(got[3], one[3][first:first + S], rtol=1e-6, atol=0)   # 32-bit results of 64-bit sums in another order
+
+
+@pytest.mark.parametrize("V,B,L", [(3000, 1, 1), (70_000, 1, 1), (70_000, 4, 16), (70_000, 40, 16), (300_000, 60, 32), (300_000, 150, 32), (300_000, 230, 32)])
+@pytest.mark.parametrize("scratch", ["0", "1"])
+def test_fastgcn_few_entries(nd, ndo, monkeypatch, V, B, L, scratch):
+    """Lists of 0 to 25 entries that begin and end anywhere in eight, with repeated entries, up to and beyond four entries a thread."""
+    monkeypatch.setenv("ND_COLLECTIVE_BITMAP_GLOBAL", scratch)
+    rng = np.random.default_rng(V + B)
+    deg = rng.integers(0, 26, V)
+    deg[rng.choice(V, 5, replace=False)] = [V // 100, V // 200, 300, 2100, 255]
+    src = np.repeat(np.arange(V), deg).astype(np.int32)
+    dst = np.where(rng.random(len(src)) < 0.1, src // 2, rng.integers(0, V, len(src))).astype(np.int32)
+    hg = ndo.csr_from_records(src, dst, np.ones(len(src), np.float32), V=V)
+    S = 20
+    initial = rng.integers(-1, V, S * B).astype(np.int32)
+    s = nd.Sampler(nd.Graph.from_csr(hg.row_ptr, hg.col, hg.w, hg.max_w), nd.app_params(8, steps=2, fanout=L, batch=B, seed=3), num_samples=S, initial=initial)
+    s.sample()
+    exp = ndo.sample(hg, ndo.make_params(8, steps=2, fanout=L, batch=B, seed=3), S, initial=initial)
+    aux = s.aux()
+    assert np.array_equal(s.final_samples(), exp["out"])   # whole numbers: the sums are exact
+    assert np.array_equal(aux["prob"].reshape(-1), exp["prob"].reshape(-1))
+    assert np.array_equal(aux["adj_row"], exp["adj_row"]) and np.array_equal(aux["adj_col"], exp["adj_col"])
+    assert s.stats()["union_unique"] == exp["counters"]["union_unique"]
