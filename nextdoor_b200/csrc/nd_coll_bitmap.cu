@@ -7,8 +7,8 @@
 // integer weights sum exactly).
 //
 // What bounds it, and what is done about it (2^20 vertices, 1024 batches of 64, 2 layers of 64: FastGCN
-// 4.8 -> 0.59 ms, LADIES 5.7 -> 0.68 ms).  One CTA fills an SM there, and neither memory nor issue slots are full:
-// FastGCN issues in 43 % of the cycles (270 M instructions, 5.2 GB out of the L2), LADIES in 43 % (304 M instructions for 131 M
+// 4.8 -> 0.58 ms, LADIES 5.7 -> 0.67 ms).  One CTA fills an SM there, and neither memory nor issue slots are full:
+// FastGCN issues in 45 % of the cycles (270 M instructions, 5.1 GB out of the L2), LADIES in 44 % (303 M instructions for 131 M
 // list entries, the distinct ones of 313 M); the warps wait for barriers between the phases, for loads and for shared memory:
 //  * The second layer's transits are hubs (FastGCN draws them with the square of their degree), many of them the
 //    same one: repeated transits of a batch are taken once (LADIES with their multiplicity).
@@ -21,7 +21,7 @@
 //    byte permutation; sixteen vertices a lane in their own order, with a multiplication a mask, 0.622 ms, now 0.588).  The two bytes that hold degrees up to 2047 take three times as many, so that from 256 on, where few vertices have
 //    as many, they are a list (20 K of 2^20, 65 against 160 thousand cycles an SM); where they are not few the codes have a
 //    second byte, for the groups that need it.  Groups without a candidate are passed over, and the lists beside the hubs',
-//    where they are short (a first layer's: 2 K entries), are weighed entry by entry as they come into the union, an eight of
+//    where they are short (a first layer's: 2 K entries), are weighed entry by entry as they come into the union, one or an eight of
 //    entries to a thread, instead of looking through 2^20 vertices for them (390 -> 100 thousand cycles an SM with the lists
 //    a warp each before; V / FEW: 64 0.755, 16 0.79 ms).  Groups' sums are two 32-bit words until they are scanned: a 64-bit
 //    add in shared memory is a loop.  0.89 -> 0.74 ms, 256 batches on 2^21 0.56 -> 0.46, 700 of 100 on 100 K 0.50 -> 0.46.
@@ -60,7 +60,7 @@ constexpr int GROUP = 512;        // FastGCN: vertices (GROUP_WORDS words) whose
 constexpr int LADIES_GROUP_BITS = 7;   // LADIES: 2^7 vertices, more where the sums of the groups would not fit shared memory
 constexpr int RUN = 4;            // listed vertices a thread takes at a time
 constexpr int BIG_DEGREE = 2048;  // from here a vertex is listed and its code is 0: 512 * 2047^2 < 2^31
-constexpr int LISTED = 32;        // degrees are codes of a byte where fewer than V / LISTED vertices do not fit one
+constexpr int LISTED = 32;        // degrees are codes of a byte where no more than V / LISTED vertices do not fit one
 constexpr int FLIGHT = 4;         // pairs of groups a warp sums at a time (2^20 vertices 2: 0.595, 3: 0.589, 4: 0.588 ms; 600 K, 100 batches 77.7, 76.7, 76.3 us)
 constexpr int HUB = 128;          // a vertex with at least V / HUB neighbours has a bitmap of them
 constexpr int32_t SHARED_V = 1 << 18;   // see plan_of()
@@ -70,7 +70,7 @@ constexpr int FEW = 64;           // lists with fewer than V / FEW entries in al
 // limit 533; 148 of 16, 40 edges a vertex, 106, 106, 106, 106, 115).
 constexpr int ENTRIES = 4;
 constexpr int SUB = 16;           // LADIES: lanes that add up a group of a hub (100 K vertices: 32 0.62, 16 0.595, 8 0.595, 4 0.60 ms; 2^20: 0.77, 0.77, 0.78, 0.80)
-constexpr int OCT = 8;            // list entries a thread takes at a time: 32 aligned bytes (LADIES)
+constexpr int OCT = 8;            // list entries a thread takes at a time: 32 aligned bytes
 
 // The bitmap and FastGCN's CDF make the "big" part (V/8 + V/64 bytes).  It lives in shared memory when the whole layout
 // fits the CTA's opt-in shared memory (graphs up to about 1.2 M vertices) and otherwise in a per-CTA slice of a global
@@ -82,7 +82,7 @@ struct Layout {
   uint32_t off_gcdf;                                   // FastGCN: inside the big part (the bitmap is at 0); LADIES: inside shared memory, unless sums_far
   bool sums_far;
   uint32_t off_red, off_tr, off_layer, off_ut, off_mult, off_same, off_pre;   // inside shared memory
-  uint32_t off_draw, off_acc;                           // LADIES: the same; the accumulators may be where the bitmap is
+  uint32_t off_draw, off_acc;                           // the same; LADIES' accumulators, which may be where the bitmap is
   uint32_t off_slot;                                   // LADIES: with the groups' sums
   uint32_t bytes;                                      // dynamic shared memory of the launch
   uint32_t glob_bytes;                                 // per-CTA slice of the global scratch, 0 = big part in shared memory
@@ -561,7 +561,7 @@ __device__ __forceinline__ uint32_t squares(uint32_t bits, const int32_t (&low)[
   return WIDE ? ll + (lh << 9) + (hh << 16) : ll;
 }
 
-// FastGCN: the groups' weights, without HUGE_DEGREE ones; the candidates the thread has seen.  A warp takes FLIGHT times two
+// FastGCN: the groups' weights, without the listed and the huge vertices' (their codes are zero); the candidates the thread has seen.  A warp takes FLIGHT times two
 // groups at a time, a lane a word of the bitmap and its 32 bytes of codes.  WIDE: the codes have high bytes.
 template <bool WIDE>
 __device__ __forceinline__ uint32_t sum_groups(const uint32_t *bm, const Degrees &d, int words, int groups, uint2 *sums) {
@@ -632,8 +632,8 @@ __device__ __forceinline__ void sum_listed(const uint32_t *bm, const Degrees &d,
 
 // The adjacency of a batch's lists, a row of bits each: bit j of row i, the layer's vertex j is in list i.  A list with a bitmap is
 // asked by a bit test.  Of the others the warp, which has a row or a few side by side, first gets 32 entries, the last ones of as
-// many parts of the list, from which a lane finds the part of its vertex without a read, and then bisects that: two or three
-// reads that wait for one another instead of up to thirteen (FastGCN 2^20 vertices 0.644 -> 0.636 ms, LADIES 0.689 -> 0.68).
+// many parts of the list, from which a lane finds the part of its vertex without a read, and then bisects that: of 32, 64, 1024 and 8191
+// entries (the longest list without a bitmap on 2^20 vertices) 1, 2, 6 and 9 reads that wait for one another instead of up to 6, 7, 11 and 13 (FastGCN 2^20 vertices 0.644 -> 0.636 ms, LADIES 0.689 -> 0.68).
 // WORDS: the words of a row that are side by side, which share the list and its 32 entries (a word of any row each, with a division
 // to find it, before: layers of 100 on 100 K, 700 batches, FastGCN 360 -> 323 us, LADIES 592 -> 549; of 64 on 70 K, 1024:
 // 190 -> 180).  (Three places a step instead of one take half of the steps and more time; going through short lists once more with a

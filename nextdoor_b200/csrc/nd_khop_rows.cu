@@ -12,7 +12,8 @@
 // instructions: 341 M of a warp, 0.29 ms at one per cycle and scheduler, and of the 18 cycles from one to the next 4.8 are
 // spent waiting for the next instruction to be fetched, 2.5 for memory and 2.4 for shared memory (DRAM 35 %); without its sorts
 // 0.375 ms, without the resolution of picks taken twice 0.43, without the gathers 0.46, with a cheap hash for the draws 0.46; a mini-batch
-// of 1024, the chain seed -> row -> neighbours -> rows -> neighbours (74 -> 12 us with the seeds' copy).
+// of 1024 (74 -> 12 us with the seeds' copy), the hand-over from the copy to the kernel and the caller (100 seeds take 12.4 us too), and of the
+// kernel's 10 us one warp's instructions: a thousand for a sample, 15.7 cycles each, 4.6 of them for memory and 4.6 at barriers, 10 % of the warps in use.
 #include "nd_common.cuh"
 #include "nd_khop_rows.cuh"
 #include "nd_philox.cuh"
