@@ -69,6 +69,7 @@ constexpr int FEW = 64;           // lists with fewer than V / FEW entries in al
 // of 4, 30 K vertices: 29.9 us, one 26.3, two 26.2, four 26.3; 125 K: 33.7, 33.1, 30.9, 30.9; 1000 of 64 on 1 M: 527, 523, 521, 521, without a
 // limit 533; 148 of 16, 40 edges a vertex, 106, 106, 106, 106, 115).
 constexpr int ENTRIES = 4;
+constexpr int PAIRS = 8, PAIR_ROWS = 8;   // longest layer and fewest lists that are probed pair by pair, see the kernel's adjacency
 constexpr int SUB = 16;           // LADIES: lanes that add up a group of a hub (100 K vertices: 32 0.62, 16 0.595, 8 0.595, 4 0.60 ms; 2^20: 0.77, 0.77, 0.78, 0.80)
 constexpr int OCT = 8;            // list entries a thread takes at a time: 32 aligned bytes
 
@@ -1048,7 +1049,19 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
       __syncthreads();
       uint32_t *adj = a.adj + (s * a.steps + cp.step) * (int64_t)adj_words(cp.stride);
       const int row_words = (cp.L + 31) / 32;
-      if ((int64_t)nu * row_words <= lay.words) {
+      if ((int64_t)nu * row_words > lay.words || (nu > PAIR_ROWS && cp.L <= (nu > 2 * warps ? PAIRS : PAIRS / 2))) {
+        // A thread a pair: where the rows do not fit, and for layers so short that a warp to a row leaves most of its lanes idle (167 batches
+        // of 250, layers of 1, 20 K vertices: rows, as below, FastGCN 47.5 us, LADIES 77, pairs 35.6 and 67; 1 M, FastGCN 174, 162; of 4 20 K LADIES 87, 80.6;
+        // of 8 49.4, 43.2.  Of 4 or 8 lists rows are faster, 0.885 to 0.91 in units of either, of 30 lists from layers of 8 on).
+        probe_pairs(a.g.col, a.hub_bits, lay.words, cp.stride, adj, [&](int e, PairList &list, int32_t &v) {
+          const int i = e / cp.L, place = i < cp.ntr ? sh_mult[sh_same[i]] : -1;
+          if (place < 0) return false;
+          const Transit &t = ut[place];
+          list = PairList{t.rs, t.deg, t.slot};
+          v = sh_layer[e - i * cp.L];
+          return v >= 0 && v < cp.V;
+        });
+      } else {
         // a row of answers for every list, where the union was; repeated transits have the same
         probe_rows(a.g.col, a.hub_bits, lay.words, cp.V, ut, cp.ntr - nu, nh, nu, sh_layer, cp.L, bm);
         __syncthreads();
@@ -1066,8 +1079,6 @@ coll_bitmap_kernel(const __grid_constant__ Args a) {
           }
           adj[w] = word;
         }
-      } else {
-        emit_adjacency(a.g, cp, sh_tr, sh_layer, adj, a.hub_slot, a.hub_bits, lay.words);
       }
       __syncthreads();
     }

@@ -403,3 +403,29 @@ def test_fastgcn_few_entries(nd, ndo, monkeypatch, V, B, L, scratch):
     assert np.array_equal(aux["prob"].reshape(-1), exp["prob"].reshape(-1))
     assert np.array_equal(aux["adj_row"], exp["adj_row"]) and np.array_equal(aux["adj_col"], exp["adj_col"])
     assert s.stats()["union_unique"] == exp["counters"]["union_unique"]
+
+
+@pytest.mark.parametrize("V,B,L", [(2000, 9, 1), (3000, 8, 4), (3000, 9, 4), (3000, 9, 5), (70_000, 65, 5), (70_000, 300, 8), (70_000, 300, 9), (300_000, 700, 3)])
+@pytest.mark.parametrize("app", [8, 9])
+def test_adjacency_of_short_layers(nd, ndo, app, V, B, L):
+    """Few vertices and many lists, repeated ones and ones that are none among them: bit for bit what the lists hold."""
+    rng = np.random.default_rng(B + L)
+    hg = ndo.rmat_graph(V, 20 * V, seed=3)
+    S, steps = 30, 2
+    initial = rng.integers(-1, V, S * B).astype(np.int32)
+    initial[::7] = initial[3]
+    s = nd.Sampler(nd.Graph.from_csr(hg.row_ptr, hg.col, hg.w, hg.max_w), nd.app_params(app, steps=steps, fanout=L, batch=B, seed=3), num_samples=S, initial=initial)
+    s.sample()
+    out, aux = s.final_samples().reshape(S, steps, L), s.aux()
+    rows, cols = aux["adj_row"].reshape(S, steps, -1), aux["adj_col"].reshape(S, steps, -1)
+    for k in range(S):
+        for step in range(steps):
+            transits = initial[k * B:(k + 1) * B] if step == 0 else out[k, step - 1]
+            exp = np.zeros((len(transits), L), bool)
+            for i, t in enumerate(transits):
+                if 0 <= t < V:
+                    exp[i] = np.isin(out[k, step], hg.col[hg.row_ptr[t]:hg.row_ptr[t + 1]])
+            exp = exp.reshape(-1)
+            i, j = np.divmod(np.arange(len(exp)), L)
+            assert np.array_equal(rows[k, step, :len(exp)], np.where(exp, i, -1)) and np.array_equal(cols[k, step, :len(exp)], np.where(exp, j, -1))
+            assert (rows[k, step, len(exp):] == -1).all()
