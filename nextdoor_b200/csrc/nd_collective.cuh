@@ -71,9 +71,8 @@ __device__ __forceinline__ void probe_pairs(const int32_t *__restrict__ col, con
 }
 
 // the adjacency of one layer of one sample
-__device__ __forceinline__ void emit_adjacency(const NdGraphView &g, const CollParams &cp, const int32_t *tr, const int32_t *layer, uint32_t *adj,
-                                               const int32_t *hub_slot = nullptr, const uint32_t *hub_bits = nullptr, int words = 0) {
-  probe_pairs(g.col, hub_bits, words, cp.stride, adj, [&](int e, PairList &list, int32_t &v) {
+__device__ __forceinline__ void emit_adjacency(const NdGraphView &g, const CollParams &cp, const int32_t *tr, const int32_t *layer, uint32_t *adj) {
+  probe_pairs(g.col, nullptr, 0, cp.stride, adj, [&](int e, PairList &list, int32_t &v) {
     const int i = e / cp.L, j = e - i * cp.L;
     if (i >= cp.ntr) return false;
     const int32_t t = tr[i];
@@ -81,7 +80,7 @@ __device__ __forceinline__ void emit_adjacency(const NdGraphView &g, const CollP
     if (t < 0 || t >= cp.V || v < 0 || v >= cp.V) return false;
     list.rs = __ldg(g.row_ptr + t);
     list.deg = __ldg(g.row_ptr + t + 1) - list.rs;
-    list.slot = hub_slot ? __ldg(hub_slot + t) : -1;
+    list.slot = -1;
     return true;
   });
 }
